@@ -306,12 +306,17 @@ int qmm_poll_status_static(int* status_out);
  * seconds; at least 1000). Process-wide. No counterpart in the reference. */
 int qmm_set_wait_limit(long long clocks);
 
+/* The split products' scratch comes from a memory pool of the library, one per device, which keeps
+ * up to 64 MiB between calls. Returns what the current device's pool holds unused to the driver.
+ * No counterpart in the reference. */
+int qmm_release_scratch(void);
+
 /* Number of kernels this library has launched on the calling process since load
  * (monotonic; used by benchmarks to report their launch count). */
 uint64_t qmm_launch_count(void);
 
-/* Number of device-memory allocations (cudaMalloc / cudaMallocAsync) the library itself has
- * made since load: the per-device status word on first use, and the float32 partial-sum
+/* Number of device-memory allocations (cudaMalloc, or a request from its scratch pool) the library
+ * itself has made since load: the per-device status word on first use, and the float32 partial-sum
  * scratch of a split tensor-core product. `qmm_quantized_matmul_static` never raises it once
  * the device has been used. No counterpart in the reference. */
 uint64_t qmm_alloc_count(void);

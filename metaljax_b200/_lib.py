@@ -8,11 +8,14 @@ this file; it is never built implicitly and there is no fallback when it is miss
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
+NATIVE_PATH = os.path.join(_HERE, "_native.so")
 LIB_PATH = os.environ.get("QMM_LIBRARY") or os.path.join(_HERE, "libqmm.so")     # (a development build can be named)
 
 MODE = {"affine": 0, "mxfp4": 1}
@@ -88,6 +91,7 @@ _SIGNATURES = {
     "qmm_alloc_count": (ctypes.c_uint64, []),
     "qmm_poll_status": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int)]),
     "qmm_poll_status_static": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int)]),
+    "qmm_release_scratch": (ctypes.c_int, []),
     "qmm_set_wait_limit": (ctypes.c_int, [ctypes.c_longlong]),
     "qmm_set_route_override": (ctypes.c_int, [ctypes.c_int]),
     "qmm_quantized_matmul": (ctypes.c_int, [_T, _T, _T, _T, _T, ctypes.c_int, ctypes.c_int,
@@ -164,6 +168,23 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The calls that build their views natively (csrc/torch_call.cpp), bound to the loaded libqmm."""
+    global _native
+    if _native is None:
+        if not os.path.exists(NATIVE_PATH):
+            raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m metaljax_b200.build`.")
+        loader = importlib.machinery.ExtensionFileLoader("_native", NATIVE_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
+        loader.exec_module(module)
+        module.bind(*(ctypes.cast(getattr(lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul",)))
+        _native = module
+    return _native
+
+
 def check(status: int) -> None:
     if status:
         raise QmmError(status, lib().qmm_last_error().decode(errors="replace"))
@@ -222,6 +243,11 @@ def poll_status_static() -> int:
     st = ctypes.c_int(0)
     check(lib().qmm_poll_status_static(ctypes.byref(st)))
     return int(st.value)
+
+
+def release_scratch() -> None:
+    """Gives the scratch that the library's pool keeps between calls back to the driver."""
+    check(lib().qmm_release_scratch())
 
 
 def launch_count() -> int:

@@ -389,6 +389,8 @@ int qmm_set_wait_limit(long long clocks) {
   return QMM_OK;
 }
 
+int qmm_release_scratch(void) { return release_scratch(); }
+
 uint64_t qmm_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
 uint64_t qmm_alloc_count(void) { return g_allocs.load(std::memory_order_relaxed); }

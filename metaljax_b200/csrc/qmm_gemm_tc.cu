@@ -967,15 +967,9 @@ int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
                     block->bytes);
       tp.partial = static_cast<float*>(block->ptr);
     } else {
-      void* ptr = nullptr;
-      if (cudaMallocAsync(&ptr, need, stream) == cudaSuccess) {
-        count_alloc();
-        tp.partial = static_cast<float*>(ptr);
-        scratch_async = true;
-      } else {
-        cudaGetLastError();
-        splits = 1;
-      }
+      tp.partial = static_cast<float*>(scratch_alloc(need, stream));
+      scratch_async = tp.partial != nullptr;
+      if (!scratch_async) splits = 1;
     }
   }
   tp.splits = splits;
@@ -1000,14 +994,8 @@ int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
       if (block) {
         if (need <= block->bytes) part = static_cast<float*>(block->ptr);
       } else {
-        void* ptr = nullptr;
-        if (cudaMallocAsync(&ptr, need, stream) == cudaSuccess) {
-          count_alloc();
-          part = static_cast<float*>(ptr);
-          part_async = true;
-        } else {
-          cudaGetLastError();
-        }
+        part = static_cast<float*>(scratch_alloc(need, stream));
+        part_async = part != nullptr;
       }
       if (part) {
         TcParams head = tp, tail = tp;
@@ -1027,7 +1015,7 @@ int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
         launch_dependent(splitk_tail_reduce_kernel, static_cast<unsigned>(blocks), 256, 0, stream, part, p.y, p.y_dtype, p.M, p.N,
                          ftiles, max_tiles - rem, rem, BT, static_cast<int>(s));
         count_launch(3);
-        if (part_async) cudaFreeAsync(part, stream);
+        if (part_async) scratch_free(part, stream);
         return check_launch("qmm_gemm_tc_kernel");
       }
     }
@@ -1041,7 +1029,7 @@ int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
     if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
     launch_dependent(splitk_reduce_kernel, static_cast<unsigned>(blocks), 256, 0, stream, tp.partial, p.y, p.y_dtype, total, splits);
     count_launch();
-    if (scratch_async) cudaFreeAsync(tp.partial, stream);
+    if (scratch_async) scratch_free(tp.partial, stream);
   }
 #if QMM_TC_TRACING
   if (trace_on) {   // development aid: average cycles per wait site over the CTAs

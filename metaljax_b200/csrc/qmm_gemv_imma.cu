@@ -897,7 +897,7 @@ int launch_fused(const CUtensorMap& wm, const ImmaParams& ip, const ImmaPlan& pl
 // warps, and the successor's CTAs can become resident early), else sixteen warps in one CTA.
 ImmaPlan make_plan(const qmm_problem& p, int nchunks, int plane_bytes, int groups, bool mx, bool fused) {
   const int sms = device_sm_count();
-  const int force_r = env_int("QMM_IMMA_R", 0), force_ring = env_int("QMM_IMMA_RING", 0), force_nw = env_int("QMM_IMMA_NW", 0);
+  static const int force_r = env_int("QMM_IMMA_R", 0), force_ring = env_int("QMM_IMMA_RING", 0), force_nw = env_int("QMM_IMMA_NW", 0);
   const size_t kTwoPerSm = 113 * 1024;     // an SM has 228 KiB, of which every resident CTA also takes 1 KiB
   const size_t kOnePerSm = 226 * 1024;
   const bool small = (p.N + 31) / 32 <= sms;

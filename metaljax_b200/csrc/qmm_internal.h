@@ -40,6 +40,12 @@ struct ScratchBlock {
 const ScratchBlock* scratch_override();
 void set_scratch_override(const ScratchBlock* block);
 
+// Stream-ordered device memory from the library's pool (NULL: none to be had); counted by
+// qmm_alloc_count(). `release_scratch` returns what the pool holds unused to the driver.
+void* scratch_alloc(size_t bytes, cudaStream_t stream);
+void scratch_free(void* ptr, cudaStream_t stream);
+int release_scratch();
+
 int launch_gemv(const qmm_problem& p, cudaStream_t stream);
 bool gemv_supports(const qmm_problem& p);
 // What a decode step fuses into a single-row linear: how its activation row is made from the
