@@ -21,7 +21,7 @@ LIB_PATH = os.environ.get("QMM_LIBRARY") or os.path.join(_HERE, "libqmm.so")    
 MODE = {"affine": 0, "mxfp4": 1}
 ROUTES = {0: "none", 1: "gemv", 2: "gemm_tc", 3: "simt", 4: "gemv_fmma"}
 ELEM = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2, torch.uint8: 3,
-        torch.uint32: 4, torch.int32: 5}
+        torch.uint32: 4, torch.int32: 5, torch.int8: 6}
 
 
 class QmmError(RuntimeError):
@@ -108,6 +108,10 @@ _SIGNATURES = {
     "qmm_dequantize": (ctypes.c_int, [_T, _T, _T, _T, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                       ctypes.c_void_p]),
     "qmm_pack_codes": (ctypes.c_int, [_T, _T, ctypes.c_int, ctypes.c_void_p]),
+    "qmm_pack_dense_codes": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_int64] * 2 + [ctypes.c_void_p] * 2),
+    "qmm_pack_dense_facts": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_int] * 2 + [ctypes.c_int64] * 3 + [ctypes.c_void_p] * 2),
+    "qmm_pack_dense_tables": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2 + [ctypes.c_int]
+                              + [ctypes.c_int64] * 3 + [ctypes.c_int, ctypes.c_void_p]),
     "qmm_moe_silu_mul": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
                                         ctypes.c_int, ctypes.c_void_p]),
     "qmm_moe_routed_sum": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,

@@ -1,0 +1,231 @@
+// Packing a quantized Dense layer's stored arrays on the device (keras' int4 layout: two output columns per byte,
+// tables per group of input rows; tests/test_qmm.py:179-199): the code transpose and the table transpose as one
+// pass each, with the facts the packer decides from (src/metaljax/qmm.py:206-286, 1204-1247) gathered on the way.
+//
+// Through generic tensor passes (unpack to int16, transpose, widen to int64, minimum and maximum, repack, expanded
+// scale and zero maps, ...) a [4096, 14336] layer took 2.8 ms and a dozen waits for the device; the bytes that have to move
+// are 69 MB, 11 us of HBM. Three kernels and one wait: 96 us, most of it the host's and the wait's.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <type_traits>
+
+#include "../../include/qmm.h"
+#include "qmm_internal.h"
+
+namespace qmm {
+namespace {
+
+constexpr int kTileN = 64, kTileK = 256;           // output rows and codes of a CTA's tile: 32-byte input sectors, 128-byte output lines
+constexpr uint32_t kMix = 2246822519u;
+
+// packed int8 [K, bytes] (byte j of row k: columns 2j, 2j + 1, two's complement nibbles) -> out words [N, K / 8], codes + 8.
+// A thread owns 4 bytes (8 columns) x 8 rows: eight 4-byte reads, a byte transpose, a nibble squeeze, eight words.
+// `digest` accumulates the content digest of the words (the sharing table's key).
+__global__ void __launch_bounds__(256)
+transpose_pack_kernel(const uint8_t* __restrict__ packed, uint32_t* __restrict__ out, int K, int N, int bytes, bool words4, unsigned long long* digest) {
+  __shared__ uint32_t tile[kTileN][kTileK / 8 + 1];
+  __shared__ unsigned long long warp_sum[8];
+  const int n0 = blockIdx.x * kTileN, k0 = blockIdx.y * kTileK;
+  const int q = threadIdx.x & 7, o = threadIdx.x >> 3;                 // which 4 bytes, which 8 rows
+  const int byte0 = n0 / 2 + q * 4, row0 = k0 + o * 8;
+  uint32_t r[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    r[i] = 0u;
+    if (row0 + i < K) {
+      const uint8_t* src = packed + static_cast<int64_t>(row0 + i) * bytes + byte0;
+      if (words4 && byte0 + 4 <= bytes) {
+        r[i] = __ldcs(reinterpret_cast<const uint32_t*>(src));
+      } else {
+        for (int b = 0; b < 4; ++b)
+          if (byte0 + b < bytes) r[i] |= static_cast<uint32_t>(src[b]) << (8 * b);
+      }
+    }
+  }
+  // column c of four rows as one word: bytes transposed
+  auto transpose = [](uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&t)[4]) {
+    const uint32_t x0 = __byte_perm(a, b, 0x5140), x1 = __byte_perm(a, b, 0x7362), y0 = __byte_perm(c, d, 0x5140), y1 = __byte_perm(c, d, 0x7362);
+    t[0] = __byte_perm(x0, y0, 0x5410); t[1] = __byte_perm(x0, y0, 0x7632);
+    t[2] = __byte_perm(x1, y1, 0x5410); t[3] = __byte_perm(x1, y1, 0x7632);
+  };
+  auto squeeze = [](uint32_t v) -> uint32_t {      // the low nibbles of four bytes as 16 bits
+    v &= 0x0F0F0F0Fu;
+    v = (v | (v >> 4)) & 0x00FF00FFu;
+    return (v | (v >> 8)) & 0xFFFFu;
+  };
+  uint32_t lo[4], hi[4];
+  transpose(r[0], r[1], r[2], r[3], lo);
+  transpose(r[4], r[5], r[6], r[7], hi);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {                    // two's complement + 8 is an exclusive or with 8
+    tile[q * 8 + 2 * c][o] = (squeeze(lo[c]) | (squeeze(hi[c]) << 16)) ^ 0x88888888u;
+    tile[q * 8 + 2 * c + 1][o] = (squeeze(lo[c] >> 4) | (squeeze(hi[c] >> 4) << 16)) ^ 0x88888888u;
+  }
+  __syncthreads();
+  const int words = K / 8, w = threadIdx.x & 31, wk = k0 / 8 + w;
+  unsigned long long sum = 0;
+  for (int i = threadIdx.x >> 5; i < kTileN; i += 8) {
+    const int n = n0 + i;
+    if (n < N && wk < words) {
+      const uint32_t v = tile[i][w];
+      const int64_t at = static_cast<int64_t>(n) * words + wk;
+      __stcs(out + at, v);
+      uint32_t m = (v ^ (static_cast<uint32_t>(at) * 2654435761u)) * kMix;
+      m ^= m >> 15;
+      sum += m;
+    }
+  }
+  for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; ++i) sum += warp_sum[i];
+    atomicAdd(digest, sum);
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ float as_float(T v) { return static_cast<float>(v); }
+template <>
+__device__ __forceinline__ float as_float(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <>
+__device__ __forceinline__ float as_float(__half v) { return __half2float(v); }
+
+template <typename T>
+__device__ __forceinline__ T to_table(float v) {
+  if constexpr (sizeof(T) == 4) return v;
+  else if constexpr (std::is_same<T, __nv_bfloat16>::value) return __float2bfloat16_rn(v);
+  else return __float2half_rn(v);
+}
+
+// Facts about scale / zero [G, N] (group = K / G rows): bit 0 not constant within 128 codes, 1 within 64, 2 the biases do not narrow
+// to the scales' type exactly, 3 something the packer has to look at itself (a NaN, a zero point that is no integer or out of range).
+template <typename S, typename Z>
+__global__ void table_facts_kernel(const S* __restrict__ scale, const Z* __restrict__ zero, int G, int N, int K, unsigned* __restrict__ facts) {
+  const int group = K / G;
+  unsigned f = 0;
+  const int64_t total = static_cast<int64_t>(G) * N;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int j = static_cast<int>(i / N), n = static_cast<int>(i - static_cast<int64_t>(j) * N);
+    const float s = as_float(scale[i]), z = zero ? as_float(zero[i]) : 0.0f;
+    if (!(s == s) || !(z == z) || rintf(z) != z || fabsf(z) > 32768.0f) f |= 8u;
+    const float b = -(s * (z + 8.0f));
+    if (as_float(to_table<S>(b)) != b) f |= 4u;
+    // blocks of 128 and of 64 codes that this group's first code is not the start of: the same entries as their first group's?
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int g = t ? 64 : 128;
+      const int64_t at = static_cast<int64_t>(j) * group;
+      const int64_t first = at / g * g / group;    // group of the block's first code
+      if (at % g != 0 && first != j) {
+        const float s0 = as_float(scale[first * N + n]), z0 = zero ? as_float(zero[first * N + n]) : 0.0f;
+        if (!(s == s0) || !(z == z0)) f |= 1u << t;
+      }
+    }
+  }
+  f = __reduce_or_sync(0xffffffffu, f);
+  if ((threadIdx.x & 31) == 0 && f) atomicOr(facts, f);
+}
+
+// scale, zero [G, N] -> scales, biases = -scale (zero + 8) [N, K / g], transposed through shared memory.
+template <typename S, typename Z, typename T>
+__global__ void __launch_bounds__(256)
+tables_kernel(const S* __restrict__ scale, const Z* __restrict__ zero, T* __restrict__ scales, T* __restrict__ biases, int G, int N, int K, int g) {
+  __shared__ float ts[32][33], tb[32][33];
+  const int groups = K / g, group = K / G;
+  const int n0 = blockIdx.x * 32, j0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int i = ty; i < 32; i += 8) {
+    const int j = j0 + i, n = n0 + tx;
+    if (j < groups && n < N) {
+      const int64_t at = static_cast<int64_t>(static_cast<int64_t>(j) * g / group) * N + n;
+      const float s = as_float(scale[at]), z = zero ? as_float(zero[at]) : 0.0f;
+      ts[i][tx] = s;
+      tb[i][tx] = -(s * (z + 8.0f));
+    }
+  }
+  __syncthreads();
+  for (int i = ty; i < 32; i += 8) {
+    const int n = n0 + i, j = j0 + tx;
+    if (j < groups && n < N) {
+      const int64_t at = static_cast<int64_t>(n) * groups + j;
+      scales[at] = to_table<T>(ts[tx][i]);
+      biases[at] = to_table<T>(tb[tx][i]);
+    }
+  }
+}
+
+// f(S(), Z()) for a scale and a zero type.
+template <typename F>
+int with_types(int scale_dtype, int zero_dtype, F&& f) {
+  auto z = [&](auto s) -> int {
+    switch (zero_dtype) {
+      case QMM_BF16: return f(s, __nv_bfloat16());
+      case QMM_F16: return f(s, __half());
+      case QMM_F32: return f(s, float());
+      case QMM_U8: return f(s, uint8_t());
+      case QMM_I8: return f(s, int8_t());
+    }
+    return fail(QMM_ERR_DTYPE, "pack_dense: zero points are bf16, f16, f32, int8 or uint8");
+  };
+  switch (scale_dtype) {
+    case QMM_BF16: return z(__nv_bfloat16());
+    case QMM_F16: return z(__half());
+    case QMM_F32: return z(float());
+  }
+  return fail(QMM_ERR_DTYPE, "pack_dense: scales are bf16, f16 or f32");
+}
+
+}  // namespace
+}  // namespace qmm
+
+using namespace qmm;
+
+extern "C" int qmm_pack_dense_codes(const void* packed, uint32_t* words, int64_t K, int64_t N, uint64_t* digest, void* stream) {
+  if (!packed || !words || !digest) return fail(QMM_ERR_NULL, "pack_dense_codes: null pointer");
+  if (K < 32 || K % 32 || N < 1 || K >= (1LL << 24) || N >= (1LL << 30)) return fail(QMM_ERR_SHAPE, "pack_dense_codes: K is a multiple of 32");
+  const int64_t bytes = (N + 1) / 2;
+  const dim3 grid(static_cast<unsigned>((N + kTileN - 1) / kTileN), static_cast<unsigned>((K + kTileK - 1) / kTileK));
+  if (grid.y > 65535) return fail(QMM_ERR_SHAPE, "pack_dense_codes: K is too long");
+  const bool words4 = bytes % 4 == 0 && reinterpret_cast<uintptr_t>(packed) % 4 == 0;
+  transpose_pack_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint8_t*>(packed), words, static_cast<int>(K), static_cast<int>(N),
+                                                                             static_cast<int>(bytes), words4, reinterpret_cast<unsigned long long*>(digest));
+  count_launch();
+  return check_launch("transpose_pack_kernel");
+}
+
+extern "C" int qmm_pack_dense_facts(const void* scale, const void* zero, int scale_dtype, int zero_dtype, int64_t G, int64_t N, int64_t K, uint32_t* facts, void* stream) {
+  if (!scale || !facts) return fail(QMM_ERR_NULL, "pack_dense_facts: null pointer");
+  if (G < 1 || N < 1 || K % G || (K / G) % 32 || G >= (1LL << 30) || N >= (1LL << 30) || K >= (1LL << 30)) return fail(QMM_ERR_SHAPE, "pack_dense_facts: groups are multiples of 32 codes");
+  const int64_t total = G * N, cap = static_cast<int64_t>(device_sm_count()) * 8;
+  const int64_t blocks = (total + 255) / 256 < cap ? (total + 255) / 256 : cap;
+  return with_types(scale_dtype, zero ? zero_dtype : QMM_U8, [&](auto s, auto z) -> int {
+    using S = decltype(s);
+    using Z = decltype(z);
+    table_facts_kernel<S, Z><<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const S*>(scale), static_cast<const Z*>(zero), static_cast<int>(G), static_cast<int>(N), static_cast<int>(K), facts);
+    count_launch();
+    return check_launch("table_facts_kernel");
+  });
+}
+
+extern "C" int qmm_pack_dense_tables(const void* scale, const void* zero, int scale_dtype, int zero_dtype, void* scales, void* biases, int narrow, int64_t G, int64_t N,
+                                     int64_t K, int group_size, void* stream) {
+  if (!scale || !scales || !biases) return fail(QMM_ERR_NULL, "pack_dense_tables: null pointer");
+  if (G < 1 || N < 1 || K % G || group_size < 32 || K % group_size || N >= (1LL << 30) || K >= (1LL << 30)) return fail(QMM_ERR_SHAPE, "pack_dense_tables: bad shape");
+  const dim3 grid(static_cast<unsigned>((N + 31) / 32), static_cast<unsigned>((K / group_size + 31) / 32));
+  if (grid.y > 65535) return fail(QMM_ERR_SHAPE, "pack_dense_tables: K is too long");
+  return with_types(scale_dtype, zero ? zero_dtype : QMM_U8, [&](auto s, auto z) -> int {
+    using S = decltype(s);
+    using Z = decltype(z);
+    if (narrow && scale_dtype != QMM_F32)
+      tables_kernel<S, Z, S><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const S*>(scale), static_cast<const Z*>(zero), static_cast<S*>(scales),
+                                                                                  static_cast<S*>(biases), static_cast<int>(G), static_cast<int>(N), static_cast<int>(K), group_size);
+    else
+      tables_kernel<S, Z, float><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const S*>(scale), static_cast<const Z*>(zero), static_cast<float*>(scales),
+                                                                                      static_cast<float*>(biases), static_cast<int>(G), static_cast<int>(N), static_cast<int>(K), group_size);
+    count_launch();
+    return check_launch("tables_kernel");
+  });
+}

@@ -24,6 +24,7 @@ from __future__ import annotations
 
 import math
 import os
+import threading
 import weakref
 
 import numpy as np
@@ -528,8 +529,8 @@ def build_pack(m: Match, codes, scale_map, zero_map=None, leaves=()) -> _Pack:
     return _record_pack(m, pack)
 
 
-def _record_pack(m: Match, pack: _Pack) -> _Pack:
-    pack = _share(pack)
+def _record_pack(m: Match, pack: _Pack, digest=None) -> _Pack:
+    pack = _share(pack, digest)
     m.gs, m.bits, m.has_perm = pack.gs, pack.bits, pack.perm is not None
     m.nvals = len(pack.arrays())
     m.packs.insert(0, pack)
@@ -562,13 +563,13 @@ def _digest(a: torch.Tensor) -> int:
     return int(mixed.sum().item()) & 0xFFFFFFFFFFFF
 
 
-def _share(pk: _Pack) -> _Pack:
+def _share(pk: _Pack, digest=None) -> _Pack:
     """Alias `pk`'s arrays onto an identical earlier pack's, if one is alive. Content-addressed:
     nothing is aliased until the arrays compare equal element for element, so two chains that
     reconstruct the same weight share one copy and two that do not can never be confused."""
     arrays = pk.arrays()
     key = (pk.mode, pk.gs, pk.bits, len(arrays), str(arrays[0].device),
-           tuple((tuple(a.shape), a.dtype) for a in arrays), _digest(arrays[0]))
+           tuple((tuple(a.shape), a.dtype) for a in arrays), _digest(arrays[0]) if digest is None else digest)
     bucket = _SHARED.get(key)
     if bucket is not None:
         for i, refs in enumerate(bucket):
@@ -722,6 +723,50 @@ def unpack_keras_int4(packed: torch.Tensor, columns: int) -> torch.Tensor:
     return ((both ^ 8) - 8).to(torch.int8)
 
 
+_PINNED = threading.local()       # a few bytes of page-locked memory per thread: where a packer's facts arrive
+
+
+def _pack_dense(packed, scale, zero, k, n, out_dtype):
+    """`from_keras_int4` on the GPU for consecutive groups of a multiple of 32 rows: codes and tables in one
+    kernel each and one wait for the device (which group size the tables allow, and whether the biases narrow, is in the data).
+    None where the general way has to look (host arrays, other layouts, zero points it may reject)."""
+    tables = (scale,) if zero is None else (scale, zero)
+    if not all(t.is_cuda and t.is_contiguous() and t.dim() == 2 and t.device == packed.device for t in (packed, *tables)):
+        return None
+    g = scale.shape[0]
+    if packed.dtype != torch.int8 or packed.shape[1] != -(-n // 2) or any(tuple(t.shape) != (g, n) for t in tables) or n == 0:
+        return None
+    if k % g or (k // g) % 32 or scale.dtype not in _FLOATS or (zero is not None and zero.dtype not in (*_FLOATS, torch.int8, torch.uint8)):
+        return None
+    if _SCALE_WIDTH not in ("auto", "source", "f32"):
+        return None
+    lib, stream, dev = _lib.lib(), _lib.stream_ptr(packed), packed.device
+    with torch.cuda.device(dev):
+        facts = torch.zeros(2, dtype=torch.int64, device=dev)               # [digest, flags]
+        at = facts.data_ptr()
+        words = torch.empty((n, k // 8), dtype=torch.uint32, device=dev)
+        args = (scale.data_ptr(), None if zero is None else zero.data_ptr(), _lib.ELEM[scale.dtype], 0 if zero is None else _lib.ELEM[zero.dtype])
+        _lib.check(lib.qmm_pack_dense_facts(*args, g, n, k, at + 8, stream))
+        _lib.check(lib.qmm_pack_dense_codes(packed.data_ptr(), words.data_ptr(), k, n, at, stream))
+        host = getattr(_PINNED, "facts", None)
+        if host is None:
+            host = _PINNED.facts = torch.empty(2, dtype=torch.int64).pin_memory()
+        host.copy_(facts, non_blocking=True)
+        torch.cuda.current_stream(dev).synchronize()
+        digest, flags = int(host[0]), int(host[1])
+        if flags & 8:
+            return None
+        group = next(s for s in _GROUP_SIZES if k % s == 0 and not (flags & {128: 1, 64: 2, 32: 0}[s]))
+        narrow = scale.dtype != torch.float32 and _SCALE_WIDTH != "f32" and (_SCALE_WIDTH == "source" or not flags & 4)
+        scales = torch.empty((n, k // group), dtype=scale.dtype if narrow else torch.float32, device=dev)
+        biases = torch.empty_like(scales)
+        _lib.check(lib.qmm_pack_dense_tables(*args, scales.data_ptr(), biases.data_ptr(), int(narrow), g, n, k, group, stream))
+    m = Match()
+    m.mode, m.N, m.K = "affine", n, k
+    m.out_dtype = out_dtype or scale.dtype
+    return _record_pack(m, _Pack((packed, scale), words, scales, biases, None, group, 4, "affine"), digest & 0xFFFFFFFFFFFF)
+
+
 def from_keras_int4(packed, scale, zero=None, g_idx=None, columns=None, out_dtype=None):
     """A keras int4 `Dense` kernel as the fused op's operands (`Dense._int4_call`,
     tests/test_qmm.py:193-199): `packed` int8 `[K, ceil(N/2)]` (two OUTPUT columns per byte),
@@ -731,6 +776,10 @@ def from_keras_int4(packed, scale, zero=None, g_idx=None, columns=None, out_dtyp
     the activations. The same checks as the recognizer's pack prologue (`build_pack`)."""
     k = packed.shape[0]
     n = int(columns if columns is not None else scale.shape[-1])
+    if g_idx is None:
+        pack = _pack_dense(packed, scale, zero, k, n, out_dtype)
+        if pack is not None:
+            return pack
     codes = unpack_keras_int4(packed, n).t().contiguous()                      # [N, K]
     groups = scale.shape[0]
     if g_idx is None:

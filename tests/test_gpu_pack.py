@@ -1,0 +1,43 @@
+"""A stored int4 Dense layer packed on the device against the same call on host arrays (the general way):
+every word and table entry the same, at the edges of the 64 x 256 tile, odd column counts, group sizes that
+allow 128, 64 and 32 codes per table entry, and tables that have to stay float32. Needs a B200."""
+
+import pytest
+import torch
+
+from metaljax_b200 import qmm
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("k,n,groups,sdt,zdt,constant", [
+    (32, 1, 1, torch.bfloat16, torch.bfloat16, False), (256, 64, 2, torch.bfloat16, torch.int8, False),
+    (288, 65, 3, torch.float16, torch.float16, False), (320, 63, 5, torch.float32, torch.float32, False),
+    (1024, 130, 32, torch.bfloat16, None, False), (1024, 130, 32, torch.bfloat16, torch.uint8, True),
+    (512, 7, 8, torch.float16, None, False), (4096, 200, 32, torch.bfloat16, torch.bfloat16, False),
+])
+def test_device_pack_is_the_host_pack(k, n, groups, sdt, zdt, constant):
+    g = torch.Generator().manual_seed(k + n)
+    packed = torch.randint(-128, 128, (k, -(-n // 2)), generator=g, dtype=torch.int8)
+    if n % 2:
+        packed[:, -1] &= 15                                   # (the column past the last one is zero)
+    rows = 1 if constant else groups
+    scale = (torch.rand((rows, n), generator=g) * 0.02 + 0.01).to(sdt).expand(groups, n).contiguous()
+    zero = None
+    if zdt is not None:
+        zero = torch.randint(0, 5, (rows, n), generator=g).to(zdt).expand(groups, n).contiguous()
+    want = qmm.from_keras_int4(packed, scale, zero, columns=n)
+    got = qmm.from_keras_int4(packed.to(DEV), scale.to(DEV), None if zero is None else zero.to(DEV), columns=n)
+    assert (got.gs, got.bits, got.mode, got.scales.dtype) == (want.gs, want.bits, want.mode, want.scales.dtype)
+    assert torch.equal(got.w.cpu().view(torch.int32), want.w.view(torch.int32))
+    assert torch.equal(got.scales.cpu(), want.scales) and torch.equal(got.biases.cpu(), want.biases)
+
+
+def test_device_pack_rejects_what_the_host_pack_rejects():
+    packed = torch.zeros((256, 3), dtype=torch.int8, device=DEV)
+    scale = torch.full((4, 6), 0.5, device=DEV)
+    zero = torch.full((4, 6), 0.5, device=DEV)                # no integer
+    with pytest.raises(qmm._Reject):
+        qmm.from_keras_int4(packed, scale, zero, columns=6)
