@@ -186,10 +186,8 @@ int route_of(const qmm_problem& p) {
   if (forced == QMM_ROUTE_GEMV || forced == QMM_ROUTE_GEMV_FMMA) return gemv_supports(p) ? QMM_ROUTE_GEMV : -QMM_ERR_UNSUPPORTED;
   if (forced == QMM_ROUTE_GEMM_TC) return gemm_tc_supports(p) ? forced : -QMM_ERR_UNSUPPORTED;
   if (forced == QMM_ROUTE_SIMT) return forced;
-  // More than 8 rows against a long K (the activations no longer fit next to the decode
-  // kernel's rings) go to the tensor-core kernel, whose K split then fills the machine.
-  const bool long_k = p.M > 8 && p.K >= 8192 && p.batch == 1 && !p.lhs_idx && gemm_tc_supports(p);
-  if (gemv_supports(p) && !long_k) return QMM_ROUTE_GEMV;
+  if (gemv_supports(p)) return QMM_ROUTE_GEMV;
+  if (p.group_sizes && p.x_dtype != QMM_F32 && rows_grouped_pays(p)) return QMM_ROUTE_GEMV;
   if (gemm_tc_supports(p)) return QMM_ROUTE_GEMM_TC;
   return QMM_ROUTE_SIMT;
 }
@@ -210,9 +208,11 @@ int launch_problem(const qmm_problem& p, cudaStream_t stream) {
   if (route < 0) return fail(-route, "the forced kernel family does not support this problem");
   switch (route) {
     case QMM_ROUTE_NONE: return QMM_OK;
-    case QMM_ROUTE_GEMV: return launch_gemv(p, stream);
+    case QMM_ROUTE_GEMV: return p.group_sizes ? launch_rows(p, stream) : launch_gemv(p, stream);
     case QMM_ROUTE_GEMM_TC: return launch_gemm_tc(p, stream);
-    default: return launch_simt(p, stream);
+    // Float32 activations and what the others decline (unsorted gathers of more than 16 rows, K below 64): the
+    // few-rows kernel takes them as columns of its MMAs; the plain SIMT kernel is what a forced route cross-checks with.
+    default: return route_override() != QMM_ROUTE_SIMT && rows_supports(p) ? launch_rows(p, stream) : launch_simt(p, stream);
   }
 }
 
@@ -274,6 +274,8 @@ int build_dense(const qmm_tensor* x, const qmm_tensor* w, const qmm_tensor* scal
 
 namespace qmm {
 int check_problem(const qmm_problem& p) { return validate_problem(p, true); }
+int run_problem(const qmm_problem& p, cudaStream_t stream) { return launch_problem(p, stream); }
+bool grouped_takes_rows(const qmm_problem& p) { return route_of(p) == QMM_ROUTE_GEMV; }
 }  // namespace qmm
 
 using namespace qmm;

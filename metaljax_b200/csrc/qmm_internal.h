@@ -48,6 +48,17 @@ int release_scratch();
 
 int launch_gemv(const qmm_problem& p, cudaStream_t stream);
 bool gemv_supports(const qmm_problem& p);
+// The few-rows kernel: everything launch_gemv takes, grouped products and float32 activations.
+struct RowsGather {            // grouped products whose rows of x are picked by index
+  const int32_t* x_rows;       // [M] row of x behind each row of the product
+  int64_t total_x_rows;
+};
+int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr);
+bool rows_supports(const qmm_problem& p);
+bool rows_grouped_pays(const qmm_problem& p);
+// A checked problem on the kernel its route names; and whether that is the few-rows kernel for a grouped one.
+int run_problem(const qmm_problem& p, cudaStream_t stream);
+bool grouped_takes_rows(const qmm_problem& p);
 // What a decode step fuses into a single-row linear: how its activation row is made from the
 // previous kernels' outputs, and the exchange of its input and output rows over peer memory.
 struct DecodeFusion {
@@ -124,6 +135,23 @@ int launch_pack_codes(const uint8_t* codes, uint32_t* out, int64_t rows, int64_t
                       cudaStream_t stream);
 
 #ifdef __CUDACC__
+// Launches with programmatic stream serialization: a kernel that begins with griddepcontrol.wait is scheduled while the one
+// before it drains. A failure stays as the last error (check_launch reports it).
+template <typename... Params, typename... Args>
+void launch_early(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // Raw bits of element i of a 16-bit (`wide` false) or 32-bit (`wide` true) table, zero-extended.
 // Nothing here depends on the loaded value, so a caller can request many elements before it
 // uses the first; callers keep `wide` loop-invariant so that the loads of a batch do not end

@@ -1,0 +1,171 @@
+// The few-rows kernel's plan and entry points (the kernel itself: qmm_rows.cuh; its instantiations: qmm_rows_*.cu).
+#include "qmm_rows.cuh"
+
+namespace qmm {
+
+using namespace rows;
+
+namespace rows {
+#define QMM_ROWS_EXTERN(QK, XT) \
+  extern template int launch_rows_kernel<QK, XT>(const CUtensorMap&, RowsParams&, RowsPlan&, const RowsShape&, bool, cudaStream_t);
+QMM_ROWS_EXTERN(kAff4, __nv_bfloat16)
+QMM_ROWS_EXTERN(kAff4, __half)
+QMM_ROWS_EXTERN(kAff4, float)
+QMM_ROWS_EXTERN(kAff8, __nv_bfloat16)
+QMM_ROWS_EXTERN(kAff8, __half)
+QMM_ROWS_EXTERN(kAff8, float)
+QMM_ROWS_EXTERN(kMx4, __nv_bfloat16)
+QMM_ROWS_EXTERN(kMx4, __half)
+QMM_ROWS_EXTERN(kMx4, float)
+}  // namespace rows
+
+namespace {
+
+size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
+  const size_t shares = static_cast<size_t>(pl.blocks) * 512;
+  return 1024 + kHeadBytes +
+         static_cast<size_t>(pl.warps) * (pl.ring * (pl.blocks * sh.stage + table_stage_bytes(pl.blocks, sh.groups, sh.tt)) + pl.red_bufs * shares + sums_bytes(sh.groups) + more_x_bytes(sh.tokens)) +
+         (pl.cluster > 1 ? kExchangeSlots * pl.cluster * shares : 0) + (segs ? (2 * static_cast<size_t>(segs) + 1) * 4 : 0);
+}
+
+// How K and the tiles are shared out. An SM's time is the slices it works through, so the plan with the fewest
+// slices on the busiest SM wins: tiles per cluster x warps per CTA x CTAs per SM (a tile's fixed costs count
+// as half a slice of 32 rows per warp, meeting in a cluster as two slices). More CTAs per tile (a larger cluster) is
+// what fills the machine when a weight has few tiles, and what keeps K within 8 warps x 512 codes of registers when K is
+// long. Tiles of one block cost more per row, but an SM that has one tile or two waits less for them (8 rows, mxfp4
+// 5760 x 2880: 2.4 tiles of 16 rows per SM instead of 1.2 -> 2 of 32).
+RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh, int segs) {
+  const int sms = device_sm_count();
+  RowsPlan best = {};
+  double best_load = 0.0;
+  for (int blocks = kMaxBlocks; blocks >= 1; --blocks) {
+    const int64_t items = chunks * ((rows + kBlockRows * blocks - 1) / (kBlockRows * blocks));
+    for (int c = 1; c <= kMaxCluster; c *= 2) {
+      if (c > slices && c > 1) break;
+      RowsPlan pl = {};
+      pl.blocks = blocks;
+      pl.cluster = c;
+      pl.slices_per_cta = (slices + c - 1) / c;
+      pl.slices_per_warp = (pl.slices_per_cta + kMaxWarps - 1) / kMaxWarps;
+      if (pl.slices_per_warp > 1 && c < kMaxCluster) continue;        // (reloading activations per tile: only where nothing else is left)
+      pl.warps = (pl.slices_per_cta + pl.slices_per_warp - 1) / pl.slices_per_warp;
+      pl.slices_per_cta = pl.warps * pl.slices_per_warp;
+      int per_sm = kMaxWarps / pl.warps;
+      if (per_sm > 4) per_sm = 4;
+      pl.ring = kMaxRing;
+      pl.red_bufs = 4;
+      const size_t budget = static_cast<size_t>(kSmemLimit) / per_sm - 1024;
+      while (pl.red_bufs > 3 && smem_of(pl, sh, segs) > budget) --pl.red_bufs;
+      while (pl.ring > 2 && smem_of(pl, sh, segs) > budget) --pl.ring;
+      while (pl.ring > 1 && smem_of(pl, sh, segs) > static_cast<size_t>(kSmemLimit)) --pl.ring;
+      pl.smem = smem_of(pl, sh, segs);
+      if (pl.smem > static_cast<size_t>(kSmemLimit)) continue;
+      while (per_sm > 1 && pl.smem > static_cast<size_t>(kSmemLimit) / per_sm - 1024) --per_sm;
+      int64_t clusters = static_cast<int64_t>(sms) * per_sm / c;
+      if (clusters > items) clusters = items;
+      if (clusters < 1) clusters = 1;
+      pl.grid = static_cast<int>(clusters * c);
+      const int64_t tiles = (items + clusters - 1) / clusters;
+      const int64_t resident = (clusters * c + sms - 1) / sms;
+      const int64_t busy = resident * pl.warps > 6 ? resident * pl.warps : 6;      // (fewer warps leave an SM waiting)
+      const double tile = blocks == 2 ? pl.slices_per_warp + (c > 1 ? 0.55 : 0.5) : 0.5 * pl.slices_per_warp + (c > 1 ? 0.4 : 0.35);
+      double load = static_cast<double>(tiles) * busy * tile + (c > 1 ? 4.0 : 0.0);
+      if (pl.ring == 1) load *= 100.0;               // (nothing is loaded while a box is worked on: where nothing else fits)
+      if (!best.warps || load < best_load) {
+        best = pl;
+        best_load = load;
+      }
+    }
+  }
+  return best;
+}
+
+}  // namespace
+
+bool rows_supports(const qmm_problem& p) {
+  if (p.mode == QMM_MODE_FLOAT || p.K < 32 || p.K % 32 || p.K >= (1LL << 30) || p.N < 1 || p.M < 1 || p.batch < 1) return false;
+  if (p.M >= (1LL << 31) || p.batch >= (1LL << 31)) return false;
+  if (p.group_sizes && p.batch > kMaxSegments) return false;
+  const int64_t nw = p.num_weights > 0 ? p.num_weights : (p.w_batch_stride ? p.batch : 1);
+  if (p.batch * ((p.M + 3) / 4) * ((p.N + 15) / 16) >= (1LL << 31)) return false;       // items are counted in 32 bits
+  return nw * p.N < (1LL << 31);                    // TMA row coordinates are 32-bit
+}
+
+// A grouped product of at most this many rows per expert on average streams its experts' weights here; above it
+// the tensor-core kernel's wide token tiles win. (Experts' shares are only known on the device: an expert
+// of more than 8 rows passes its weight once per 8.)
+bool rows_grouped_pays(const qmm_problem& p) { return rows_supports(p) && p.M <= 16 * p.batch; }
+
+// The decode family as callers may force it: dense or gathered products of up to 16 rows of 16-bit activations.
+bool gemv_supports(const qmm_problem& p) {
+  return (p.x_dtype == QMM_BF16 || p.x_dtype == QMM_F16) && !p.group_sizes && p.M <= 16 && p.batch <= 65535 && rows_supports(p);
+}
+
+int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather) {
+  RowsParams rp = {};
+  rp.x = p.x; rp.scales = p.scales; rp.biases = p.biases; rp.y = p.y;
+  rp.lhs_idx = p.lhs_idx; rp.rhs_idx = p.rhs_idx; rp.group_sizes = p.group_sizes;
+  if (gather) {
+    rp.x_rows = gather->x_rows;
+    rp.total_x_rows = gather->total_x_rows;
+  }
+  rp.status = device_status_word();
+  if (!rp.status) return fail(QMM_ERR_CUDA, "could not allocate the device status word");
+  const bool mx = p.mode == QMM_MODE_MXFP4;
+  const int bits = (!mx && p.bits == 8) ? 8 : 4;
+  const int group = mx ? 32 : p.group_size;
+  rp.x_batch_stride = p.x_batch_stride; rp.y_batch_stride = p.y_batch_stride;
+  rp.num_weights = p.num_weights > 0 ? p.num_weights : 1;
+  rp.x_batches = p.x_batches;
+  rp.M = p.M; rp.K = static_cast<int>(p.K); rp.N = static_cast<int>(p.N); rp.segs = static_cast<int>(p.batch);
+  rp.groups = rp.K / group;
+  rp.weight_rows = (p.rhs_idx || p.group_sizes || p.w_batch_stride) ? rp.N : 0;
+  rp.table_dtype = p.table_dtype; rp.y_dtype = p.y_dtype;
+  const int slices = (rp.K + kSliceK - 1) / kSliceK;
+  // Rows of a chunk: what the registers take. Nine to sixteen rows are two chunks: the CTAs that work on either half pass over
+  // the weight side by side, so that the second reads it from L2 (16 rows of 4096 x 4096: 9.2 us; as one chunk of 16, half of whose activations
+  // live in shared memory, 14.2; 14336 x 4096 25.0 against 30.5 on the tensor cores, 8-bit 14336 x 4096 31 against 51).
+  const int chunk = p.x_dtype == QMM_F32 ? 4 : 8;
+  const int64_t per_seg = p.group_sizes ? (p.M + p.batch - 1) / p.batch : p.M;      // grouped: of an average expert
+  const int64_t live = p.group_sizes ? (p.batch < p.M ? p.batch : p.M) : p.batch;
+  const int entry = mx ? 1 : (p.table_dtype == QMM_F32 ? 4 : 2);
+  const RowsShape sh = {chunk, kSliceK / group, mx ? kTabE8 : (p.table_dtype == QMM_BF16 ? kTabBf16 : (p.table_dtype == QMM_F16 ? kTabF16 : kTabF32)),
+                        kBlockRows * kSliceK * bits / 8};
+  const int64_t nweights = p.num_weights > 0 ? p.num_weights : (p.w_batch_stride ? p.batch : 1);
+  rp.table_bytes = nweights * p.N * rp.groups * entry;
+  // (a slice's entries start on the units that its own row of entries and a row of the table are multiples of)
+  const int slice_bytes = sh.groups * entry, row_bytes_t = rp.groups * entry;
+  rp.table_unit = (row_bytes_t | slice_bytes) % 8 == 0 && row_bytes_t % slice_bytes == 0 ? 8 : (row_bytes_t | slice_bytes) % 4 == 0 ? 4 : 1;
+  RowsPlan pl = plan_rows(live * ((per_seg + chunk - 1) / chunk), rp.N, slices, sh, p.group_sizes ? rp.segs : 0);
+  if (!pl.warps) return fail(QMM_ERR_UNSUPPORTED, "few-rows kernel: no plan fits shared memory");
+  const int tile_rows = kBlockRows * pl.blocks;
+  rp.tiles = (rp.N + tile_rows - 1) / tile_rows;
+  pl.items = p.batch * ((p.M + chunk - 1) / chunk) * rp.tiles;
+  rp.cluster = pl.cluster; rp.slices_per_cta = pl.slices_per_cta; rp.slices_per_warp = pl.slices_per_warp;
+  rp.ring = pl.ring; rp.red_bufs = pl.red_bufs;
+
+  // The packed weight as a 2-D byte tensor [rows, K*bits/8] over every weight matrix behind `w`; what a box
+  // reaches past the last row or the end of a row is zero-filled by the TMA unit.
+  const uint64_t row_bytes = static_cast<uint64_t>(p.K) * bits / 8;
+  CUtensorMap wm;
+  const int rc = tensor_map_2d(&wm, QMM_U8, p.w, row_bytes, static_cast<uint64_t>(p.N) * nweights, row_bytes, kBoxBytes, tile_rows, 1);
+  if (rc) return rc;
+  // A gather's indices decide which weight the first boxes come from: it is serialized in the ordinary way.
+  const bool early = !p.lhs_idx;
+  auto launch = [&](auto kind) {
+    constexpr int QK = decltype(kind)::value;
+    if (p.x_dtype == QMM_BF16) return launch_rows_kernel<QK, __nv_bfloat16>(wm, rp, pl, sh, early, stream);
+    if (p.x_dtype == QMM_F16) return launch_rows_kernel<QK, __half>(wm, rp, pl, sh, early, stream);
+    return launch_rows_kernel<QK, float>(wm, rp, pl, sh, early, stream);
+  };
+  if (mx) return launch(std::integral_constant<int, kMx4>());
+  if (bits == 8) return launch(std::integral_constant<int, kAff8>());
+  return launch(std::integral_constant<int, kAff4>());
+}
+
+int launch_gemv(const qmm_problem& p, cudaStream_t stream) {
+  if (route_override() != QMM_ROUTE_GEMV_FMMA && gemv_imma_supports(p)) return launch_gemv_imma(p, stream);
+  return launch_rows(p, stream);
+}
+
+}  // namespace qmm

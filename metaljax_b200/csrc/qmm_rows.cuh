@@ -1,0 +1,1140 @@
+// The few-rows kernel of the fused dequantize-and-matmul (`y = x . deq(w)^T`,
+// src/metaljax/qmm.py:2491): 2..16 rows of 16-bit activations against a streamed weight (and one row
+// where the single-row integer kernel declines), unsorted expert gathers, grouped products of a few rows
+// per expert, and every product of float32 activations.
+//
+// What bounds it. An SM's share of HBM is 23 bytes a clock, 46 4-bit codes: at four instructions a
+// clock that leaves 22 warp instructions per 256 codes, two thirds of what a dequantization element by
+// element takes, so the budget decides the layout: nothing may be done twice for a code, and nothing that
+// belongs to the activations may be done per tile of weights.
+//
+// Split. A warp owns ONE slice of 512 codes of K for as long as it lives and holds its slice of the
+// activations as MMA fragments in registers (64 registers per 8 columns); the warps of a CTA
+// (up to 8) are consecutive slices, the CTAs of a cluster (up to 8) consecutive stretches of K. Weight tiles
+// of 16 rows pass by: 16 x 128-byte boxes by TMA (128-byte swizzle) through a ring of its own per warp,
+// a few boxes ahead across tiles, so the HBM stream never waits for a barrier of the CTA. The warps'
+// partial sums of a tile meet in shared memory, one warp (in turn) adds them up in warp order; in
+// a cluster the CTAs' sums travel to the tile's leader (in turn) by st.async and are added in rank order.
+// No global scratch, no atomics, fixed order of summation.
+//
+// Arithmetic. The codes are never dequantized: a nibble pair under a magic exponent is an exact bf16 (128 + q) or f16 (1024 + q) A
+// fragment of `mma.sync.m16n8k16`, an 8-bit pair an f16 one (a byte permute), an E2M1 pair an exact f16 times 2^-14; scale and bias
+// meet the float32 accumulators once per group (the 16 K slots of an MMA lie in one group; the accumulators start at -C sum x, which takes the
+// magic number out again). The bias term is an MMA of its own per 16 rows and slice: the bf16 bias entries against the groups' sums of x
+// in three bf16 pieces. Activations that the element type cannot hold as they are become several columns or carry a power of two: float32 is
+// three columns (8 + 8 + 8 bits of bf16, or 11 + 11 + 11 of f16) that are added at the end; for f16 fragments of bf16 or float32 activations
+// each row of each slice is scaled to [2^14, 2^15) by its largest magnitude, and back in its partial sums. The K order inside a group is
+// free as long as codes and activations agree: lane t takes 16 consecutive codes (8 in groups of 32), in the pair order one LOP3 extracts.
+// (8-bit float MMAs would take the codes with a third of the instructions, but `mma.sync` on e4m3 is emulated here with
+// conversions to f16: 88 against 67 us for 8 rows of 128256 x 4096.)
+//
+// Measured (device time, weights from HBM; before: the kernel that dequantized in registers and staged its
+// activations in shared memory; float32: the SIMT kernel), int4 group 64: 8 rows 28672 x 4096 27.1 -> 21.4 us (3.1 TB/s), 128256 x 4096
+// 99.5 -> 66.6 (4.4 TB/s), 4096 x 14336 26.8 -> 16.8, 16 rows 128256 x 4096 170 -> 128, 16 rows 4096 x 4096 12.2 -> 9.2; 8-bit 14336 x 4096 22.6
+// -> 15.5 (3.9 TB/s); float32 33 rows 4096 x 4096 323 -> 36. At the small end (2 rows 4096 x 4096 6.3 -> 7.1 us) it is the chain launch, activations,
+// one tile, sum that counts, not a stream.
+//
+// Every wait on an mbarrier is bounded. The kernel is launched with programmatic stream
+// serialization: it lets the next kernel of the stream start early and touches only weights and
+// tables before `griddepcontrol.wait` (a gather or grouped product waits first: indices decide what it reads).
+#pragma once
+
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+
+
+#include <mutex>
+#include <type_traits>
+
+#include "qmm_internal.h"
+#include "qmm_ptx.cuh"
+
+namespace qmm {
+namespace rows {
+
+using namespace ptx;
+
+constexpr int kMaxWarps = 8;
+constexpr int kSliceK = 512;            // codes of K per warp
+constexpr int kBlockRows = 16;          // weight rows of an MMA; a tile is one or two blocks (see tile_blocks)
+constexpr int kBoxBytes = 128;          // bytes of a weight row in a TMA box
+constexpr int kMaxRing = 6;
+constexpr int kMaxCluster = 8;
+constexpr int kExchangeSlots = 2;       // tiles a leader may have on the way from its peers
+constexpr int kMaxSegments = 1024;      // experts of a grouped product
+constexpr int kSmemLimit = 226 * 1024;
+
+enum { kAff4 = 0, kAff8 = 1, kMx4 = 2 };
+enum { kTabBf16 = 0, kTabF16 = 1, kTabF32 = 2, kTabE8 = 3 };           // table entries
+constexpr int entry_bytes(int tt) { return tt == kTabF32 ? 4 : tt == kTabE8 ? 1 : 2; }
+
+struct RowsParams {
+  const void* x;
+  const void* scales;
+  const void* biases;
+  void* y;
+  const int32_t* lhs_idx;        // gather: x batch and weight of segment s
+  const int32_t* rhs_idx;
+  const int32_t* group_sizes;    // grouped: rows of segment s (they follow one another in x and y)
+  const int32_t* x_rows;         // grouped: the row of x behind row r of the product (NULL: r)
+  int* status;
+  int64_t x_batch_stride, y_batch_stride, num_weights, x_batches, M;
+  int K, N, segs, groups;        // groups = K / group_size
+  int weight_rows;               // weight rows between segments (N, or 0: one weight)
+  int table_dtype, y_dtype;
+  int tiles;                     // tiles per weight
+  int cluster, slices_per_cta, slices_per_warp;
+  unsigned share, share_more;    // dense: (chunk, tile) items of every cluster, and how many clusters have one more
+  int ring, red_bufs;
+  int table_unit;                // bytes on which every row's table entries of every slice start: 8, 4, or less
+  int64_t table_bytes;           // of a whole table
+  int64_t total_x_rows;          // grouped: rows of x that x_rows may name
+};
+
+// d (+)= A (16 rows of weights) * B (8 columns of activations), K 16.
+template <typename AT>
+struct Mma;
+template <>
+struct Mma<__nv_bfloat16> {
+  static constexpr uint32_t kMagic = 0x43004300u;
+  static constexpr float kMagicValue = 128.0f;
+  static __device__ __forceinline__ void run(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  }
+  // ... starting from c0, c1 (its two columns) in both rows
+  static __device__ __forceinline__ void first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0, float c1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1));
+  }
+};
+template <>
+struct Mma<__half> {
+  static constexpr uint32_t kMagic = 0x64006400u;
+  static constexpr float kMagicValue = 1024.0f;
+  static __device__ __forceinline__ void run(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  }
+  static __device__ __forceinline__ void first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0, float c1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1));
+  }
+};
+
+// (a & b) | c in one LOP3 with all three operands in registers.
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+// y0, y1 += s * a0, s * a1 in one instruction.
+__device__ __forceinline__ void fma2(float& y0, float& y1, float s, float a0, float a1) {
+  asm("{ .reg .b64 y, s, a; mov.b64 y, {%0, %1}; mov.b64 s, {%2, %2}; mov.b64 a, {%3, %4}; fma.rn.f32x2 y, s, a, y; mov.b64 {%0, %1}, y; }"
+      : "+f"(y0), "+f"(y1) : "f"(s), "f"(a0), "f"(a1));
+}
+
+__device__ __forceinline__ void store_y(void* p, int dtype, int64_t i, float v) {
+  if (dtype == QMM_BF16) reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
+  else if (dtype == QMM_F16) reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
+  else reinterpret_cast<float*>(p)[i] = v;
+}
+
+template <int N, int I = 0, typename F>
+__device__ __forceinline__ void static_for(F&& f) {
+  if constexpr (I < N) {
+    f(std::integral_constant<int, I>{});
+    static_for<N, I + 1>(f);
+  }
+}
+
+// Two floats as a pair of AT, and the floats the pair stands for.
+template <typename AT>
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  if constexpr (std::is_same<AT, __nv_bfloat16>::value) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __half2 v = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+template <typename AT>
+__device__ __forceinline__ float2 unpack2(uint32_t u) {
+  if constexpr (std::is_same<AT, __nv_bfloat16>::value) return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+  else return __half22float2(*reinterpret_cast<const __half2*>(&u));
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t remote(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void remote_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// mbar_wait for a barrier that another CTA of the cluster arrives on (its reads happened before our writes).
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t abort_flag, int where) {
+  const long long t0 = clock64();
+  for (int spins = 1;; ++spins) {
+    uint32_t done;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return true;
+    if ((spins & 255) == 0) {
+      uint32_t gave_up;
+      asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(gave_up) : "r"(abort_flag) : "memory");
+      if (gave_up) return false;
+      if (clock64() - t0 > kSpinLimit) {
+        asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_flag), "r"(where) : "memory");
+        return false;
+      }
+    }
+  }
+}
+__device__ __forceinline__ void st_async4(uint32_t addr, uint32_t bar, const float (&v)[4]) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(v[0]),
+               "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar)
+               : "memory");
+}
+
+// Shared memory, from the (1024-byte aligned) start: barriers and small state, then per warp its ring, then
+// what the CTA shares. Fixed places first: an address that is a constant costs no register.
+constexpr int kFullAt = 0;                                             // [16 warps][kMaxRing] a box has landed
+constexpr int kRedFullAt = kMaxWarps * kMaxRing * 8;                   // [4] every warp's share of a tile is there
+constexpr int kRedEmptyAt = kRedFullAt + 4 * 8;                        // [4] ... and has been added up
+constexpr int kXFullAt = kRedEmptyAt + 4 * 8;                          // [kExchangeSlots] the peers' sums of a tile this CTA leads
+constexpr int kXFreeAt = kXFullAt + kExchangeSlots * 8;                // [kMaxCluster][kExchangeSlots] leader r has read slot s
+constexpr int kAbortAt = kXFreeAt + kMaxCluster * kExchangeSlots * 8;  // the abort flag, the number of chunks of a grouped product
+constexpr int kStateAt = kAbortAt + 16;                                // [16 warps][2] where a warp's consumer is
+constexpr int kStateBytes = 32;
+constexpr int kAheadAt = kStateAt + kMaxWarps * 2 * kStateBytes;       // [16 warps] where its requests are: segment, chunk
+constexpr int kHeadBytes = (kAheadAt + kMaxWarps * 8 + 1023) / 1024 * 1024;
+
+struct Place {            // one chunk of the walk: 8 NT columns against every row of one weight
+  int64_t y0;             // element of y that its first column's first weight row goes to
+  int seg, chunk;
+  int rows_left;          // activation rows of it that exist
+  int weight_row;         // first row of its weight
+};
+static_assert(sizeof(Place) <= kStateBytes, "");
+
+// 16-row blocks of a tile: two halve what a tile costs apart from its codes, one halves the wait for a lone tile (plan_rows).
+constexpr int kMaxBlocks = 2;
+
+// A tile's table entries travel with its codes: per weight row the slice's entries as they are in memory, at a pitch
+// that 8-byte copies and conflict-free 4-byte reads allow, with a word to spare for entries that do not start
+// on a word.
+constexpr int table_row_bytes(int groups, int tt) { return groups * entry_bytes(tt); }
+constexpr int table_pitch(int groups, int tt) { return table_row_bytes(groups, tt) == 4 ? 8 : table_row_bytes(groups, tt) == 8 ? 16 : table_row_bytes(groups, tt) + 8; }
+constexpr int table_stage_bytes(int blocks, int groups, int tt) { return kBlockRows * blocks * table_pitch(groups, tt) * (tt == kTabE8 ? 1 : 2); }
+constexpr int sums_bytes(int groups) { return groups * 32; }
+// Fragments of a second column group (the third piece of float32): they would not fit the registers.
+constexpr int more_x_bytes(int tokens) { return tokens == 8 ? 0 : kSliceK * 16; }
+
+// QK: quantization kind. XT: activation type in memory. T: activation rows (tokens) of a chunk, 8 (16-bit) or 4 (float32). SPG: 32-code
+// steps per quantization group (1, 2, 4). TT: what the table entries are. R: 16-row blocks of a tile.
+template <int QK, typename XT, int T, int SPG, int TT, int R>
+__global__ void __launch_bounds__(kMaxWarps * 32, 1)
+qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
+  using AT = typename std::conditional<QK == kAff4, typename std::conditional<std::is_same<XT, float>::value, __nv_bfloat16, XT>::type, __half>::type;
+  constexpr bool kScaled = std::is_same<AT, __half>::value && !std::is_same<XT, __half>::value;
+  // Columns: piece i of the tokens of octet q is column group q * kPieces + i, its column c token 8 q + c. With 4 tokens two pieces share
+  // a group: column c is token c & 3 of piece 2 h + (c >> 2).
+  constexpr int kPieces = std::is_same<XT, float>::value ? 3 : 1;
+  constexpr bool kHalf = T == 4;
+  constexpr int Q = 1;                                                // groups of 8 output columns
+  constexpr int NT = kHalf ? (kPieces + 1) / 2 : Q * kPieces;
+  constexpr int kBits = QK == kAff8 ? 8 : 4;
+  constexpr int kTileRows = kBlockRows * R;
+  constexpr int kBoxSmem = kTileRows * kBoxBytes;
+  constexpr int kBoxes = kSliceK * kBits / 8 / kBoxBytes;             // boxes side by side in a slice
+  constexpr int kStage = kBoxes * kBoxSmem;
+  constexpr int kBlk = SPG == 1 ? 32 : 64;                            // codes that four lanes read together
+  constexpr int kBlocks = kSliceK / kBlk;
+  constexpr int kLane = kBlk / 4;                                     // consecutive codes of a lane in a block
+  constexpr int kMmas = kBlk / 16;
+  constexpr int kGroups = kSliceK / (32 * SPG);                       // groups of a slice
+  constexpr int kBlocksPerGroup = kBlocks / kGroups;
+  constexpr bool kBiasMma = TT == kTabBf16;                           // the bias term is an MMA of its own (see load_x)
+  constexpr int kBiasMmas = kGroups == 16 ? 3 : kGroups == 8 ? 2 : 1;
+  constexpr int kEntry = entry_bytes(TT);
+  constexpr int kRowBytes = table_row_bytes(kGroups, TT);             // a weight row's table entries in a slice
+  constexpr int kPitch = table_pitch(kGroups, TT);
+  constexpr int kTable = kTileRows * kPitch;                          // one table of a tile
+  constexpr int kSlot = kStage + table_stage_bytes(R, kGroups, TT);   // codes, scales, biases: a place of the ring
+  constexpr float kUnit = QK == kMx4 ? 16384.0f : 1.0f;               // (the E2M1 fragments are the values times 2^-14)
+
+  extern __shared__ uint8_t rows_smem_raw[];
+  const uint32_t smem = (smem_u32(rows_smem_raw) + 1023) & ~1023u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int rho = ((g & 1) << 2) | (g & 2) | (g >> 2);                // weight row of MMA row g: bit-reversed, which makes the
+                                                                      // swizzled reads of 4, 8 and 16 bytes free of bank conflicts
+  const int csize = p.cluster;
+  const int rank = csize > 1 ? static_cast<int>(cluster_rank()) : 0;
+
+  // (every access below goes through 32-bit shared addresses)
+  const uint32_t ring_at = smem + kHeadBytes + warp * p.ring * kStage;
+  const uint32_t tables_at = smem + kHeadBytes + warps * p.ring * kStage + warp * p.ring * (kSlot - kStage);
+  const uint32_t red_at = smem + kHeadBytes + warps * p.ring * kSlot;                           // [bufs][warps][R Q][32] float4
+  const uint32_t xbuf_at = red_at + p.red_bufs * warps * R * Q * 512;                          // [slots][cluster][R Q][32] float4
+  const uint32_t own_at = xbuf_at + (csize > 1 ? kExchangeSlots * csize * R * Q * 512 : 0);
+  const uint32_t sums_at = own_at + warp * sums_bytes(kGroups);                              // [warps] sums of x
+  const uint32_t more_x_at = own_at + warps * sums_bytes(kGroups) + warp * more_x_bytes(T) + lane * 16;      // [warps][MMA pairs][32] 16 bytes
+  const uint32_t segs_at = own_at + warps * (sums_bytes(kGroups) + more_x_bytes(T));         // grouped: [segs] chunks, [segs + 1] first rows
+  int* seg_chunks = reinterpret_cast<int*>(rows_smem_raw + (segs_at - smem_u32(rows_smem_raw)));
+  int* seg_row = seg_chunks + p.segs;
+  uint8_t* head = rows_smem_raw + (smem - smem_u32(rows_smem_raw));
+  const uint32_t my_full = smem + kFullAt + warp * kMaxRing * 8, abort_at = smem + kAbortAt;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(head + kAbortAt);
+  Place* place = reinterpret_cast<Place*>(head + kStateAt + warp * 2 * kStateBytes);
+  int* ahead_at = reinterpret_cast<int*>(head + kAheadAt) + warp * 2;
+
+  if (lane == 0) {
+    auto init = [](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n)); };
+    if (warp == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&w_map)) : "memory");
+    for (int i = 0; i < p.ring; ++i) init(my_full + i * 8, 1 + 32);    // the boxes, and every lane's table entries
+    if (warp == 0) {
+      for (int i = 0; i < 4; ++i) {
+        init(smem + kRedFullAt + i * 8, warps);
+        init(smem + kRedEmptyAt + i * 8, 1);
+      }
+      for (int i = 0; i < kExchangeSlots; ++i) init(smem + kXFullAt + i * 8, 1);
+      for (int i = 0; i < kMaxCluster * kExchangeSlots; ++i) init(smem + kXFreeAt + i * 8, 1);
+      *abort_flag = 0;
+    }
+    mbar_init_fence();
+  }
+  __syncwarp();
+
+  // ---- which work is this CTA's: a contiguous share of (chunk, tile), tiles fastest ----
+  const bool grouped = p.group_sizes != nullptr;
+  const int dense_chunks = static_cast<int>((p.M + T - 1) / T);
+  if (grouped || p.lhs_idx) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (grouped) {
+    // chunks of every expert and the rows before it (at most p.M in all, as if the sizes were cut off there)
+    for (int s = threadIdx.x; s < p.segs; s += blockDim.x) seg_row[s + 1] = p.group_sizes[s] > 0 ? p.group_sizes[s] : 0;
+    __syncthreads();
+    if (warp == 0) {
+      int64_t before = 0;
+      int chunks_before = 0;
+      for (int s0 = 0; s0 < p.segs; s0 += 32) {
+        const int s = s0 + lane;
+        const int64_t own = s < p.segs ? seg_row[s + 1] : 0;
+        int64_t run = own;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int64_t v = __shfl_up_sync(0xffffffffu, run, o);
+          if (lane >= o) run += v;
+        }
+        const int64_t lo = before + run - own < p.M ? before + run - own : p.M, hi = before + run < p.M ? before + run : p.M;
+        const int c = static_cast<int>((hi - lo + T - 1) / T);
+        __syncwarp();
+        if (s < p.segs) {
+          seg_chunks[s] = c;
+          seg_row[s] = static_cast<int>(lo);
+          if (s == p.segs - 1) seg_row[p.segs] = static_cast<int>(hi);
+        }
+        chunks_before += __reduce_add_sync(0xffffffffu, c);
+        before += __shfl_sync(0xffffffffu, run, 31);
+      }
+      if (lane == 0) abort_flag[1] = chunks_before;
+    }
+    __syncthreads();
+  }
+  auto chunks_of = [&](int seg) -> int { return grouped ? seg_chunks[seg] : dense_chunks; };
+  auto weight_row_of = [&](int seg) -> int {
+    int64_t r = p.weight_rows ? seg : 0;
+    if (p.rhs_idx) {
+      r = p.rhs_idx[seg];
+      if (r < 0 || r >= p.num_weights) {
+        if (lane == 0) atomicCAS(p.status, 0, QMM_DEVICE_BAD_INDEX);
+        r = 0;
+      }
+    }
+    return static_cast<int>(r * p.N);
+  };
+  int left, tile0, seg0 = 0, chunk0;
+  {
+    const unsigned cluster = csize > 1 ? blockIdx.x / csize : blockIdx.x;
+    unsigned share = p.share, more = p.share_more;                     // (32 bits all the way: a 64-bit division is a hundred instructions)
+    if (grouped) {
+      const unsigned total = static_cast<unsigned>(abort_flag[1]) * p.tiles, clusters = csize > 1 ? gridDim.x / csize : gridDim.x;
+      share = total / clusters;
+      more = total - share * clusters;
+    }
+    const unsigned lo = cluster * share + min(cluster, more);
+    left = static_cast<int>(share + (cluster < more ? 1u : 0u));
+    unsigned c = lo / p.tiles;
+    tile0 = static_cast<int>(lo - c * p.tiles);
+    if (grouped) {
+      while (seg0 + 1 < p.segs && c >= static_cast<unsigned>(seg_chunks[seg0])) c -= seg_chunks[seg0++];
+    } else if (p.segs > 1) {
+      seg0 = static_cast<int>(c / dense_chunks);
+      c -= static_cast<unsigned>(seg0) * dense_chunks;
+    }
+    chunk0 = static_cast<int>(c);
+  }
+  // the chunk after (seg, chunk); only asked while there is one
+  auto next_chunk = [&](int& seg, int& chunk) {
+    if (++chunk < chunks_of(seg)) return;
+    chunk = 0;
+    do { ++seg; } while (seg + 1 < p.segs && chunks_of(seg) == 0);
+  };
+
+  // ---- the ring: boxes in the order they are consumed, a few ahead ----
+  const int first_slice = rank * p.slices_per_cta + warp * p.slices_per_warp;
+  int ahead_left = left * p.slices_per_warp, ahead_row = 0, ahead_last = 0, ahead_tiles = p.tiles - tile0, ahead_sub = 0;
+  uint32_t ahead_slot = 0;
+  if (left > 0) {
+    ahead_row = weight_row_of(seg0);
+    ahead_last = ahead_row + p.N - 1;
+    ahead_row += tile0 * kTileRows;
+    if (lane == 0) { ahead_at[0] = seg0; ahead_at[1] = chunk0; }
+    __syncwarp();
+  }
+  // (a slice past the end of K is given the row's first entries: what they multiply is zero)
+  auto first_entry = [&](int slice) -> int { return slice * kGroups < p.groups ? slice * kGroups : 0; };
+  auto request = [&]() {               // the whole warp; ahead_left > 0
+    const uint32_t bar = my_full + ahead_slot * 8;
+    const int slice = first_slice + ahead_sub;
+    if (lane == 0) {
+      const uint32_t dst = ring_at + ahead_slot * kStage;
+      mbar_expect_tx(bar, kStage);
+#pragma unroll
+      for (int b = 0; b < kBoxes; ++b) tma_load_2d(&w_map, dst + b * kBoxSmem, bar, (slice * kBoxes + b) * kBoxBytes, ahead_row);
+    }
+    {
+      // a lane's share of the tables: a weight row of one table, or (two blocks) of both. Entries past the end of a row are
+      // some other entry of it: what they multiply is zero.
+      constexpr bool kBoth = R == 2 || TT == kTabE8;
+      const int row = kTileRows == 32 ? lane : lane & 15;
+      const int64_t at = (static_cast<int64_t>(min(ahead_row + row, ahead_last)) * p.groups + first_entry(slice)) * kEntry;
+      const uint32_t dst = tables_at + ahead_slot * (kSlot - kStage) + row * kPitch;
+      auto copy = [&](const void* table, uint32_t to) {
+        const uint8_t* src = static_cast<const uint8_t*>(table) + at;
+        if (p.table_unit == 8 && kRowBytes >= 8) {
+#pragma unroll
+          for (int i = 0; i < kRowBytes; i += 8) cp_async8(to + i, src + i);
+        } else if (p.table_unit >= 4) {
+#pragma unroll
+          for (int i = 0; i < kRowBytes; i += 4) cp_async4(to + i, slice * kGroups * kEntry + i < p.groups * kEntry ? src + i : src);
+        } else {                         // from the word the first entry lies in; nothing past the table's end is read
+          const int skew = static_cast<int>(at & 3);
+#pragma unroll
+          for (int i = 0; i <= kRowBytes; i += 4) {
+            const int64_t room = p.table_bytes - (at - skew + i);
+            cp_async4(to + i, room > 0 ? src - skew + i : src - skew, room >= 4 ? 4 : room > 0 ? static_cast<int>(room) : 0);
+          }
+        }
+      };
+      if (kBoth) {
+        if (kTileRows == 32 || lane < 16) copy(p.scales, dst);
+        if (TT != kTabE8) copy(p.biases, dst + kTable);
+      } else {
+        copy(lane < 16 ? p.scales : p.biases, dst + (lane < 16 ? 0 : kTable));
+      }
+      cp_async_arrive(bar);
+    }
+    --ahead_left;
+    if (++ahead_slot == static_cast<uint32_t>(p.ring)) ahead_slot = 0;
+    if (p.slices_per_warp > 1) {
+      if (++ahead_sub < p.slices_per_warp) return;
+      ahead_sub = 0;
+    }
+    ahead_row += kTileRows;
+    if (--ahead_tiles == 0) {
+      ahead_tiles = p.tiles;
+      if (ahead_left > 0) {
+        int seg = ahead_at[0], chunk = ahead_at[1];
+        next_chunk(seg, chunk);
+        ahead_row = weight_row_of(seg);
+        ahead_last = ahead_row + p.N - 1;
+        __syncwarp();
+        if (lane == 0) { ahead_at[0] = seg; ahead_at[1] = chunk; }
+        __syncwarp();
+      }
+    }
+  };
+  // (a warp past the end of K computes on zeros: its boxes are zero-filled)
+  for (int i = 0; i < p.ring && ahead_left > 0; ++i) request();
+
+  auto set_place = [&](int which, int seg, int chunk) {               // the whole warp
+    const int rows = grouped ? seg_row[seg + 1] - seg_row[seg] : static_cast<int>(p.M);
+    const int weight_row = weight_row_of(seg);
+    __syncwarp();
+    if (lane == 0) {
+      Place pl;
+      const int64_t m0 = static_cast<int64_t>(chunk) * T;
+      pl.y0 = grouped ? (seg_row[seg] + m0) * p.N : seg * p.y_batch_stride + m0 * p.N;
+      pl.seg = seg;
+      pl.chunk = chunk;
+      pl.rows_left = rows - chunk * T;
+      pl.weight_row = weight_row;
+      place[which] = pl;
+    }
+    __syncwarp();
+  };
+  if (left > 0) set_place(0, seg0, chunk0);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!grouped && !p.lhs_idx) asm volatile("griddepcontrol.wait;" ::: "memory");
+  __syncthreads();                                 // the shared barriers are initialised
+  if (csize > 1) {                                 // ... in every CTA of the cluster
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+
+  // ---- activations: this warp's slice as MMA fragments ----
+  static_assert(NT <= 2, "one column group in registers, one in shared memory");
+  uint32_t xf[kSliceK / 8];                        // column group 0: two registers per MMA of the slice
+  // The bias term sum_g bias[n, g] sum x_g of a slice is an MMA of 16 K slots: bias entries as they are in the table
+  // (bf16) against the groups' sums of x, each split into three bf16 pieces (24 bits) that take a slot of their own.
+  [[maybe_unused]] uint32_t bf[Q][kBiasMmas][2];
+  float back[Q][2];                                // what a unit of the scaled activations of output columns 2t, 2t + 1 is worth
+#pragma unroll
+  for (int q = 0; q < Q; ++q) back[q][0] = back[q][1] = 1.0f;
+  [[maybe_unused]] uint32_t least_e[Q];
+  auto load_x = [&](const Place& pl, int slice, int sub) {
+    int64_t base = 0;
+    if (!grouped) {
+      int64_t b = pl.seg;
+      if (p.lhs_idx) {
+        b = p.lhs_idx[pl.seg];
+        if (b < 0 || (p.x_batches > 0 && b >= p.x_batches)) {
+          if (lane == 0) atomicCAS(p.status, 0, QMM_DEVICE_BAD_INDEX);
+          b = 0;
+        }
+      }
+      base = b * p.x_batch_stride;
+    }
+    __syncwarp();                                  // (the sums below may still be read)
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int m = kHalf ? g & 3 : q * 8 + g;
+      const bool live = m < pl.rows_left;
+      int64_t xr = pl.chunk * T + m;
+      if (grouped && live) {
+        xr += seg_row[pl.seg];
+        if (p.x_rows) {
+          xr = p.x_rows[xr];
+          if (xr < 0 || xr >= p.total_x_rows) {
+            if (t == 0) atomicCAS(p.status, 0, QMM_DEVICE_BAD_INDEX);
+            xr = 0;
+          }
+        }
+      }
+      const XT* src = reinterpret_cast<const XT*>(p.x) + base + (live ? xr : 0) * p.K;
+      const int k0 = slice * kSliceK + t * kLane;
+      // The lane's c-th eight elements. Where they are looked at twice (scaled) and are the ones that end up in xf,
+      // they wait there as they are: one trip to memory instead of two (8 rows, mxfp4 5760 x 2880: see below).
+      constexpr bool kMayStay = kScaled && sizeof(XT) == 2;
+      const bool stays = kMayStay && q == 0;
+      auto element_of = [&](int c) -> int { return k0 + (c / (kLane / 8)) * kBlk + (c % (kLane / 8)) * 8; };
+      if (stays) {
+#pragma unroll
+        for (int c = 0; c < kSliceK / 32; ++c) {
+          const int k = element_of(c);
+          const uint4 v = live && k < p.K ? __ldg(reinterpret_cast<const uint4*>(src + k)) : make_uint4(0u, 0u, 0u, 0u);
+          xf[c * 4] = v.x; xf[c * 4 + 1] = v.y; xf[c * 4 + 2] = v.z; xf[c * 4 + 3] = v.w;
+        }
+      }
+      auto load8 = [&](int c, float (&f)[8]) {
+        const int k = element_of(c);
+        if (stays) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 w = unpack2<XT>(xf[c * 4 + i]);
+            f[2 * i] = w.x; f[2 * i + 1] = w.y;
+          }
+        } else if (live && k < p.K) {
+          if constexpr (sizeof(XT) == 4) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(src + k)), b = __ldg(reinterpret_cast<const float4*>(src + k) + 1);
+            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+          } else {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + k));
+            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 w = unpack2<XT>(u[i]);
+              f[2 * i] = w.x; f[2 * i + 1] = w.y;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[i] = 0.0f;
+        }
+      };
+      float up = 1.0f;
+      if constexpr (kScaled) {
+        float big = 0.0f;
+        bool bad = false;                                              // a NaN or an infinity: the row's results are NaN
+#pragma unroll
+        for (int c = 0; c < kSliceK / 32; ++c) {
+          float f[8];
+          load8(c, f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            big = fmaxf(big, fabsf(f[i]));
+            bad |= !(fabsf(f[i]) <= 3.402823466e38f);
+          }
+        }
+        big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
+        big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
+        bad = __ballot_sync(0xffffffffu, bad) & (0xfu << (lane & ~3));
+        // largest magnitude to [2^14, 2^15); a warp's later slices no finer than its earlier ones, whose sums are brought to their units
+        const uint32_t e = min(max(__float_as_uint(big) >> 23, sub > 0 ? least_e[q] : 15u), 253u);
+        least_e[q] = e;
+        up = __uint_as_float((268u - e) << 23);
+        const float down = bad ? __uint_as_float(0x7fc00000u) : __uint_as_float((e - 14u) << 23);
+        back[q][0] = __shfl_sync(0xffffffffu, down, 8 * t);
+        back[q][1] = __shfl_sync(0xffffffffu, down, 8 * t + 4);
+      }
+      float sum = 0.0f;
+      [[maybe_unused]] float group_sum[kGroups];
+#pragma unroll
+      for (int c = 0; c < kSliceK / 32; ++c) {
+        float f[8];
+        load8(c, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if constexpr (kScaled) f[i] *= up;
+          sum += f[i];
+        }
+        if constexpr (QK != kMx4) {
+          constexpr int kPer = kSliceK / 32 / kGroups;                 // eights per group
+          if (c % kPer == kPer - 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            // (kept as -C sum x: where the group's accumulators start)
+            if (t == 0) sts32(sums_at + ((q * kGroups + c / kPer) * 8 + g) * 4, -Mma<AT>::kMagicValue * sum);
+            if constexpr (kBiasMma) group_sum[c / kPer] = kHalf && g >= 4 ? 0.0f : sum;
+            sum = 0.0f;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+          const int h = kHalf ? i / 2 : q * kPieces + i;
+          const bool here = !kHalf || (g >> 2) == (i & 1);             // (4 tokens: which of the two pieces this lane's column is)
+          uint32_t u[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) u[j] = pack2<AT>(f[2 * j], f[2 * j + 1]);
+          if (i + 1 < kPieces) {                                       // what this piece leaves over (exact)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 got = unpack2<AT>(u[j]);
+              f[2 * j] -= got.x; f[2 * j + 1] -= got.y;
+            }
+          }
+          if constexpr (QK != kAff8) {                                 // 4-bit codes: (0,4) (1,5) (2,6) (3,7); 8-bit ones in order, (0,1) (2,3)
+            const uint32_t v[4] = {u[0], u[1], u[2], u[3]};
+            u[0] = __byte_perm(v[0], v[2], 0x5410); u[1] = __byte_perm(v[0], v[2], 0x7632);
+            u[2] = __byte_perm(v[1], v[3], 0x5410); u[3] = __byte_perm(v[1], v[3], 0x7632);
+          }
+          if (h == 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (!kHalf || i % 2 == 0 || here) xf[c * 4 + j] = u[j];
+          } else {
+            const bool empty = kHalf && !here;                         // (the half of the last group that no piece is left for)
+            sts128(more_x_at + c * 512, __uint_as_float(empty ? 0u : u[0]), __uint_as_float(empty ? 0u : u[1]), __uint_as_float(empty ? 0u : u[2]),
+                   __uint_as_float(empty ? 0u : u[3]));
+          }
+        }
+      }
+      if constexpr (kBiasMma) {
+        // K slots of the bias MMAs: 16 groups -- one MMA per piece of the sums (lane t: groups 2t, 2t + 1, 2t + 8, 2t + 9);
+        // 8 groups -- (hi | mid) and (lo | 0) with lane t's groups 2t, 2t + 1; 4 groups -- lanes t < 2 (hi | mid), t >= 2 (lo | 0)
+        // with groups 2 (t & 1), 2 (t & 1) + 1
+        auto pick = [&](int first) -> float {        // group_sum[first + 2 t], without indexing registers
+          float v = group_sum[first];
+#pragma unroll
+          for (int i = 1; i < (kGroups == 4 ? 2 : 4); ++i)
+            if ((kGroups == 4 ? t & 1 : t) == i) v = group_sum[first + 2 * i];
+          return v;
+        };
+        using B16 = __nv_bfloat16;
+        auto split = [&](float a, float b, uint32_t (&piece)[3]) {
+          piece[0] = pack2<B16>(a, b);
+          const float2 f0 = unpack2<B16>(piece[0]);
+          piece[1] = pack2<B16>(a - f0.x, b - f0.y);
+          const float2 f1 = unpack2<B16>(piece[1]);
+          piece[2] = pack2<B16>((a - f0.x) - f1.x, (b - f0.y) - f1.y);
+        };
+        uint32_t lower[3];
+        split(pick(0), pick(1), lower);
+        if constexpr (kGroups == 16) {
+          uint32_t upper[3];
+          split(pick(8), pick(9), upper);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) { bf[q][i][0] = lower[i]; bf[q][i][1] = upper[i]; }
+        } else if constexpr (kGroups == 8) {
+          bf[q][0][0] = lower[0]; bf[q][0][1] = lower[1];
+          bf[q][kBiasMmas - 1][0] = lower[2]; bf[q][kBiasMmas - 1][1] = 0u;
+        } else {
+          bf[q][0][0] = t < 2 ? lower[0] : lower[2]; bf[q][0][1] = t < 2 ? lower[1] : 0u;
+        }
+      }
+    }
+    __syncwarp();
+  };
+
+  // (4 tokens: only the columns of the first piece start at -C sum x, which is of the whole value)
+  [[maybe_unused]] auto half_start = [&](float c) -> float { return t < 2 ? c : 0.0f; };
+
+  // ---- the tiles ----
+  // A lane's bytes of block 0 of row rho in a slot; block j is at this address XOR its chunk term.
+  const uint32_t wthread = ring_at + rho * kBoxBytes +
+                           (QK == kAff8 ? (SPG == 1 ? ((((t >> 1) ^ rho) << 4) + (t & 1) * 8) : ((t ^ rho) << 4))
+                                        : (SPG == 1 ? ((rho << 4) + t * 4) : ((((t >> 1) ^ rho) << 4) + (t & 1) * 8)));
+  uint32_t nib_mask = 0x000F000Fu, magic = Mma<AT>::kMagic;
+  asm volatile("" : "+r"(nib_mask), "+r"(magic));                      // constants in registers: one LOP3 per use
+  const uint32_t tthread = tables_at + rho * kPitch, scol = sums_at + 8 * t;
+  int turn = 0, which = 0, tile = tile0, sub = 0, count = 0;
+  uint32_t slot = 0, slot_phase = 0, buf = 0, buf_phase = 0;
+  // the tile that is to be added up next
+  int done_tile = 0, done_which = 0, lap = 0, leader = 0;
+  uint32_t done_buf = 0, done_phase = 0;
+  auto add_up = [&]() -> bool {
+    // ---- the warps' shares, in warp order ----
+    const uint32_t shares = red_at + done_buf * warps * (R * Q * 512) + lane * 16;
+    if (!mbar_wait(smem + kRedFullAt + done_buf * 8, done_phase, abort_at, 13)) return false;
+    __syncwarp();
+    float v[R * Q][4];
+#pragma unroll
+    for (int h = 0; h < R * Q; ++h) v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0.0f;
+#pragma unroll 4
+    for (int i = 0; i < warps; ++i)
+#pragma unroll
+      for (int h = 0; h < R * Q; ++h) {
+        const float4 f = ldsf128<0>(shares + (i * R * Q + h) * 512);
+        v[h][0] += f.x; v[h][1] += f.y; v[h][2] += f.z; v[h][3] += f.w;
+      }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem + kRedEmptyAt + done_buf * 8);
+    bool mine = true;
+    if (csize > 1) {
+      // ---- the CTAs' sums meet at the tile's leader (in turn; `lap` counts its tiles), in rank order ----
+      const int xs = lap % kExchangeSlots;
+      const uint32_t xphase = static_cast<uint32_t>(lap / kExchangeSlots) & 1u;
+      const uint32_t xslot = xbuf_at + xs * csize * (R * Q * 512) + lane * 16;
+      mine = leader == rank;
+      if (!mine) {
+        if (!mbar_wait_cluster(smem + kXFreeAt + (leader * kExchangeSlots + xs) * 8, xphase ^ 1u, abort_at, 14)) return false;
+        __syncwarp();
+        const uint32_t bar = remote(smem + kXFullAt + xs * 8, leader), to = remote(xslot + rank * (R * Q * 512), leader);
+#pragma unroll
+        for (int h = 0; h < R * Q; ++h) st_async4(to + h * 512, bar, v[h]);
+      } else {
+        if (lane == 0) mbar_expect_tx(smem + kXFullAt + xs * 8, (csize - 1) * R * Q * 512);
+        if (!mbar_wait_cluster(smem + kXFullAt + xs * 8, xphase, abort_at, 15)) return false;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < R * Q; ++h) {
+          sts128(xslot + rank * (R * Q * 512) + h * 512, v[h][0], v[h][1], v[h][2], v[h][3]);
+          v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0.0f;
+        }
+        for (int r = 0; r < csize; ++r)
+#pragma unroll
+          for (int h = 0; h < R * Q; ++h) {
+            const float4 f = ldsf128<0>(xslot + (r * R * Q + h) * 512);
+            v[h][0] += f.x; v[h][1] += f.y; v[h][2] += f.z; v[h][3] += f.w;
+          }
+        __syncwarp();
+        if (lane < csize && lane != rank) remote_arrive(remote(smem + kXFreeAt + (rank * kExchangeSlots + xs) * 8, lane));
+      }
+    }
+    if (mine) {
+      const int rows_left = place[done_which].rows_left;
+      const int64_t y0 = place[done_which].y0;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int col = q * 8 + 2 * t + (i & 1), n = done_tile * kTileRows + r * kBlockRows + rho + (i >> 1) * 8;
+            if (col < rows_left && col < T && n < p.N) store_y(p.y, p.y_dtype, y0 + static_cast<int64_t>(col) * p.N + n, v[r * Q + q][i]);
+          }
+    }
+    return true;
+  };
+  bool ok = true, stale = true;
+  float y[R][NT][4];                               // per column group: sums of scale * codes * digits
+  [[maybe_unused]] float yb[R][Q][4];              // ... and, where it is no MMA, the bias term per output column
+  while (left > 0) {
+    if (stale) {
+      float unit[Q][2];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) { unit[q][0] = back[q][0]; unit[q][1] = back[q][1]; }
+      load_x(place[which], first_slice + sub, sub);
+      if (kScaled && sub > 0) {                    // the sums so far in the new slice's units (a power of two)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int h = 0; h < NT; ++h) {
+              // (with 4 tokens the upper lanes' columns are the lower lanes' tokens)
+              float u0 = unit[kHalf ? 0 : h / kPieces][i & 1] / back[kHalf ? 0 : h / kPieces][i & 1];
+              if (kHalf) u0 = __shfl_sync(0xffffffffu, u0, lane & ~2);
+              y[r][h][i] *= u0;
+            }
+            if constexpr (QK != kMx4)
+#pragma unroll
+              for (int q = 0; q < Q; ++q) yb[r][q][i] *= unit[q][i & 1] / back[q][i & 1];
+          }
+      }
+      stale = p.slices_per_warp > 1;
+    }
+    if (sub == 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int h = 0; h < NT; ++h) y[r][h][0] = y[r][h][1] = y[r][h][2] = y[r][h][3] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) yb[r][q][0] = yb[r][q][1] = yb[r][q][2] = yb[r][q][3] = 0.0f;
+      }
+    }
+    // where this warp goes next
+    const bool last_sub = sub + 1 == p.slices_per_warp;
+    const bool wraps = last_sub && tile + 1 == p.tiles;
+    const int next_tile = !last_sub ? tile : (wraps ? 0 : tile + 1);
+
+    if (!(ok = mbar_wait(my_full + slot * 8, slot_phase, abort_at, 11))) break;
+    __syncwarp();
+    const uint32_t wrow = wthread + slot * kStage, trow = tthread + slot * (kSlot - kStage);
+    if (kEntry < 4 && p.table_unit < 4) {          // entries that do not start on words: shifted to where they would, once per tile
+      const int row = kTileRows == 32 ? lane : lane & 15;
+      auto straighten = [&](uint32_t at) {
+        const int wr = place[which].weight_row + min(tile * kTileRows + row, p.N - 1);
+        const uint32_t skew = ((static_cast<uint32_t>(wr) * static_cast<uint32_t>(p.groups) + first_entry(first_slice + sub)) * kEntry & 3u) * 8;
+        uint32_t word = lds32<0>(at);
+#pragma unroll
+        for (int i = 0; i < kRowBytes; i += 4) {
+          const uint32_t next = lds32<0>(at + i + 4);
+          sts32(at + i, __uint_as_float(__funnelshift_r(word, next, skew)));
+          word = next;
+        }
+      };
+      const uint32_t at = tables_at + slot * (kSlot - kStage) + row * kPitch;
+      if (R == 2 || TT == kTabE8) {
+        if (kTileRows == 32 || lane < 16) straighten(at);
+        if (TT != kTabE8) straighten(at + kTable);
+      } else {
+        straighten(at + (lane < 16 ? 0 : kTable));
+      }
+      __syncwarp();
+    }
+    if constexpr (kBiasMma) {
+      static_for<R>([&](auto rc) {
+        constexpr int r = decltype(rc)::value, kAt = kTable + r * kBlockRows * kPitch;
+        const uint32_t at = trow + (kGroups == 4 ? t & 1 : t) * 4;
+        const uint32_t b0 = lds32<kAt>(at), b1 = lds32<kAt + 8 * kPitch>(at);
+        uint32_t a[4] = {b0, b1, b0, b1};
+        if constexpr (kGroups == 16) { a[2] = lds32<kAt + 16>(at); a[3] = lds32<kAt + 8 * kPitch + 16>(at); }
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+          for (int i = 0; i < kBiasMmas; ++i) Mma<__nv_bfloat16>::run(yb[r][q], a, bf[q][i][0], bf[q][i][1]);
+      });
+    }
+    static_for<kGroups>([&](auto gc) {
+      constexpr int gi = decltype(gc)::value;
+      float acc[R][NT][4];
+      float start[Q][2];                           // -C sum x of the group
+#pragma unroll
+      for (int q = 0; q < Q; ++q) start[q][0] = start[q][1] = 0.0f;
+      if constexpr (QK != kMx4)
+        static_for<Q>([&](auto qc) {
+          constexpr int q = decltype(qc)::value;
+          const uint2 sr = lds64<(q * kGroups + gi) * 32>(scol);
+          start[q][0] = __uint_as_float(sr.x); start[q][1] = __uint_as_float(sr.y);
+        });
+      static_for<kBlocksPerGroup>([&](auto bc) {
+        constexpr int jj = decltype(bc)::value, j = gi * kBlocksPerGroup + jj;      // block of the slice
+        constexpr int kLaneWords = kLane * kBits / 32;
+        constexpr int kPerBox = kBoxBytes * 8 / kBits / kBlk, kChunk = kBlk * kBits / 8;      // blocks of a box, bytes of a row in a block
+        const uint32_t a0 = (wrow ^ ((j % kPerBox) * kChunk)) + (j / kPerBox) * kBoxSmem;
+        static_for<R>([&](auto rc) {
+          constexpr int r = decltype(rc)::value, kRow = r * kBlockRows * kBoxBytes;
+          uint32_t u[2][kLaneWords];               // words of this lane, rows rho and rho + 8 of block r
+          [[maybe_unused]] uint4 more = make_uint4(0u, 0u, 0u, 0u);
+          if constexpr (kLaneWords == 1) {
+            u[0][0] = lds32<kRow>(a0);
+            u[1][0] = lds32<kRow + 8 * kBoxBytes>(a0);
+          } else if constexpr (kLaneWords == 2) {
+            const uint2 v0 = lds64<kRow>(a0), v1 = lds64<kRow + 8 * kBoxBytes>(a0);
+            u[0][0] = v0.x; u[0][1] = v0.y; u[1][0] = v1.x; u[1][1] = v1.y;
+          } else {
+            const uint4 v0 = lds128<kRow>(a0), v1 = lds128<kRow + 8 * kBoxBytes>(a0);
+            u[0][0] = v0.x; u[0][1] = v0.y; u[0][2] = v0.z; u[0][3] = v0.w;
+            u[1][0] = v1.x; u[1][1] = v1.y; u[1][2] = v1.z; u[1][3] = v1.w;
+          }
+          static_for<kMmas>([&](auto mc) {
+            constexpr int mi = decltype(mc)::value, x0 = (j * kMmas + mi) * 2;
+            if constexpr (NT > 1 && mi % 2 == 0) more = lds128<(x0 / 4) * 512>(more_x_at);
+            uint32_t a[4];
+            if constexpr (QK == kAff8) {                                  // one word: codes (0,1) and (2,3)
+              a[0] = __byte_perm(u[0][mi], 0x64646464u, 0x4140); a[1] = __byte_perm(u[1][mi], 0x64646464u, 0x4140);
+              a[2] = __byte_perm(u[0][mi], 0x64646464u, 0x4342); a[3] = __byte_perm(u[1][mi], 0x64646464u, 0x4342);
+            } else {                                                      // half a word: nibbles (0,4) (1,5), or (2,6) (3,7)
+              const uint32_t v0 = u[0][mi / 2], v1 = u[1][mi / 2];
+              if constexpr (QK == kAff4) {
+                constexpr int sh = (mi & 1) * 8;
+                a[0] = and_or(v0 >> sh, nib_mask, magic);       a[1] = and_or(v1 >> sh, nib_mask, magic);
+                a[2] = and_or(v0 >> (sh + 4), nib_mask, magic); a[3] = and_or(v1 >> (sh + 4), nib_mask, magic);
+              } else {
+                // magnitude bits of an E2M1 code at f16's exponent / mantissa boundary (the value times 2^-14,
+                // the subnormal 0.5 included), its sign at the sign
+                auto place_bits = [](uint32_t v, int nib) -> uint32_t {
+                  const uint32_t m = nib == 3 ? v >> 3 : v << (9 - 4 * nib);
+                  return (m & 0x0E000E00u) | ((v << (12 - 4 * nib)) & 0x80008000u);
+                };
+                constexpr int n0 = (mi & 1) * 2;
+                a[0] = place_bits(v0, n0); a[1] = place_bits(v1, n0); a[2] = place_bits(v0, n0 + 1); a[3] = place_bits(v1, n0 + 1);
+              }
+            }
+#pragma unroll
+            for (int h = 0; h < NT; ++h) {
+              // (all pieces but the first start from zero: -C sum x is of the whole value)
+              const bool of_first = kHalf ? h == 0 : h % kPieces == 0;
+              const int q = kHalf ? 0 : h / kPieces;
+              if constexpr (jj == 0 && mi == 0)
+                Mma<AT>::first(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1], of_first ? (kHalf ? half_start(start[q][0]) : start[q][0]) : 0.0f,
+                               of_first ? (kHalf ? half_start(start[q][1]) : start[q][1]) : 0.0f);
+              else
+                Mma<AT>::run(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1]);
+            }
+          });
+        });
+      });
+      // fold the group: rows rho (acc 0, 1) and rho + 8 (acc 2, 3), columns 2t and 2t + 1
+      static_for<R>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        constexpr int kWord = gi * kEntry / 4;
+        [[maybe_unused]] constexpr int kIn = gi * kEntry % 4;
+        constexpr int kAt = r * kBlockRows * kPitch + kWord * 4, kAt8 = kAt + 8 * kPitch;      // rows rho and rho + 8
+        auto value = [](uint32_t w) -> float {
+          if constexpr (TT == kTabE8) return __uint_as_float(max(((w >> (8 * kIn)) & 0xffu) << 23, 0x00400000u));      // 2^(e8 - 127)
+          else if constexpr (TT == kTabF32) return __uint_as_float(w);
+          else if constexpr (TT == kTabBf16) return __uint_as_float(kIn ? (w & 0xffff0000u) : (w << 16));
+          else return table_value(kIn ? w >> 16 : w & 0xffffu, QMM_F16);
+        };
+        const float s0 = value(lds32<kAt>(trow)), s1 = value(lds32<kAt8>(trow));
+#pragma unroll
+        for (int h = 0; h < NT; ++h) {
+          fma2(y[r][h][0], y[r][h][1], s0, acc[r][h][0], acc[r][h][1]);
+          fma2(y[r][h][2], y[r][h][3], s1, acc[r][h][2], acc[r][h][3]);
+        }
+        if constexpr (QK != kMx4 && !kBiasMma) {
+          constexpr float kPer = -1.0f / Mma<AT>::kMagicValue;
+          const float b0 = kPer * value(lds32<kTable + kAt>(trow)), b1 = kPer * value(lds32<kTable + kAt8>(trow));
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            fma2(yb[r][q][0], yb[r][q][1], b0, start[q][0], start[q][1]);
+            fma2(yb[r][q][2], yb[r][q][3], b1, start[q][0], start[q][1]);
+          }
+        }
+      });
+    });
+    // every read of the slot has been consumed above: the warp's next box may land in it
+    __syncwarp();
+    if (ahead_left > 0) request();
+    if (++slot == static_cast<uint32_t>(p.ring)) { slot = 0; slot_phase ^= 1u; }
+    if (!last_sub) {
+      ++sub;
+      continue;
+    }
+    sub = 0;
+
+    // ---- this warp's share of the tile ----
+    if (!(ok = mbar_wait(smem + kRedEmptyAt + buf * 8, buf_phase ^ 1u, abort_at, 12))) break;
+    // the pieces of a column together, the bias term, the scale
+    const uint32_t rbuf = red_at + (buf * warps + warp) * (R * Q * 512) + lane * 16;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if constexpr (kHalf) {
+            float s = y[r][NT - 1][i];
+#pragma unroll
+            for (int h = NT - 2; h >= 0; --h) s += y[r][h][i];
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            v[i] = s;
+          } else {
+            float s = y[r][q * kPieces + kPieces - 1][i];
+#pragma unroll
+            for (int h = kPieces - 2; h >= 0; --h) s += y[r][q * kPieces + h][i];
+            v[i] = s;
+          }
+          v[i] = fmaf(v[i], kUnit, yb[r][q][i]) * back[q][i & 1];
+        }
+        sts128(rbuf + (r * Q + q) * 512, v[0], v[1], v[2], v[3]);
+      }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem + kRedFullAt + buf * 8);
+    // the tile before this one: its shares have all been written by now, or nearly (adding up this very tile would make each adder wait
+    // for the warp that has just been one: a tile then costs its codes plus the adding up)
+    if (warp == turn && count > 0 && !(ok = add_up())) break;
+    done_tile = tile;
+    done_which = which;
+    if (count > 0) {
+      if (++turn == warps) turn = 0;
+      if (++done_buf == static_cast<uint32_t>(p.red_bufs)) { done_buf = 0; done_phase ^= 1u; }
+      if (++leader == csize) { leader = 0; ++lap; }
+    }
+    ++count;
+    if (++buf == static_cast<uint32_t>(p.red_bufs)) { buf = 0; buf_phase ^= 1u; }
+    --left;
+    tile = next_tile;
+    if (wraps && left > 0) {
+      int seg = place[which].seg, chunk = place[which].chunk;
+      next_chunk(seg, chunk);
+      which ^= 1;
+      set_place(which, seg, chunk);
+      stale = true;
+    }
+  }
+
+  if (ok && count > 0 && warp == turn) ok = add_up();      // the last tile
+
+  // ---- rows past the last expert's are zero ----
+  if (grouped) {
+    const int64_t used = static_cast<int64_t>(seg_row[p.segs]) * p.N, all = p.M * p.N;
+    for (int64_t i = used + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < all; i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+      store_y(p.y, p.y_dtype, i, 0.0f);
+  }
+  if (!ok && lane == 0) atomicCAS(p.status, 0, *abort_flag);
+  if (csize > 1) {                                 // nobody leaves while a peer may still write to its shared memory
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+// ---- host side ---------------------------------------------------------------------------
+
+struct RowsPlan {
+  int blocks, cluster, warps, slices_per_cta, slices_per_warp, ring, red_bufs, grid;
+  int64_t items;                 // (chunk, tile) items of a dense product
+  size_t smem;
+};
+
+struct RowsShape {
+  int tokens, groups, tt, stage;         // rows of a chunk; groups per slice; bytes of codes of a 16-row block and slice
+};
+
+// Clusters of this shape that fit the device at once (a GPC's SMs do not always divide by the cluster
+// size): more of them than that would be a second wave of persistent CTAs. Asked once per shape.
+template <typename Kernel>
+inline int max_clusters(Kernel kernel, const cudaLaunchConfig_t& cfg, int cluster, int warps, int ring) {
+  static std::mutex mutex;
+  static int known[kMaxDevices][4][kMaxWarps + 1][kMaxRing + 1] = {};
+  const int dev = current_device();
+  const int ci = cluster == 8 ? 3 : cluster == 4 ? 2 : cluster == 2 ? 1 : 0;
+  std::lock_guard<std::mutex> lock(mutex);
+  int& n = known[dev][ci][warps][ring];
+  if (!n && (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1)) {
+    cudaGetLastError();
+    n = 1;
+  }
+  return n;
+}
+
+template <int QK, typename XT, int T, int SPG, int TT, int R>
+int launch_kernel_of(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool early, cudaStream_t stream) {
+  auto kernel = qmm_rows_kernel<QK, XT, T, SPG, TT, R>;
+  static bool configured[kMaxDevices] = {};     // the attribute is per device
+  const int dev = current_device();
+  if (dev < 0) return QMM_ERR_DEVICE;
+  if (!configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e != cudaSuccess) return fail(QMM_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(pl.warps * 32);
+  cfg.dynamicSmemBytes = pl.smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  cfg.numAttrs = 0;
+  if (pl.cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = pl.cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+    cfg.gridDim = dim3(pl.grid);
+    const int most = max_clusters(kernel, cfg, pl.cluster, pl.warps, pl.ring);
+    if (pl.grid > most * pl.cluster) pl.grid = most * pl.cluster;
+  }
+  cfg.gridDim = dim3(pl.grid);
+  const unsigned clusters = static_cast<unsigned>(pl.grid / pl.cluster);
+  rp.share = static_cast<unsigned>(pl.items / clusters);
+  rp.share_more = static_cast<unsigned>(pl.items - static_cast<int64_t>(rp.share) * clusters);
+  if (early) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, wm, rp);
+  if (e != cudaSuccess) return fail(QMM_ERR_CUDA, "qmm_rows_kernel launch: %s", cudaGetErrorString(e));
+  count_launch();
+  return check_launch("qmm_rows_kernel");
+}
+
+template <int QK, typename XT, int T, int SPG, int TT>
+int launch_kernel(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool early, cudaStream_t stream) {
+  if (pl.blocks == 1) return launch_kernel_of<QK, XT, T, SPG, TT, 1>(wm, rp, pl, early, stream);
+  return launch_kernel_of<QK, XT, T, SPG, TT, kMaxBlocks>(wm, rp, pl, early, stream);
+}
+
+// (QK, XT) by T, group size and table type.
+template <int QK, typename XT, int T, int SPG>
+int launch_tt(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, int tt, bool early, cudaStream_t stream) {
+  if constexpr (QK == kMx4) {
+    return launch_kernel<QK, XT, T, SPG, kTabE8>(wm, rp, pl, early, stream);
+  } else {
+    if (tt == kTabBf16) return launch_kernel<QK, XT, T, SPG, kTabBf16>(wm, rp, pl, early, stream);
+    if (tt == kTabF16) return launch_kernel<QK, XT, T, SPG, kTabF16>(wm, rp, pl, early, stream);
+    return launch_kernel<QK, XT, T, SPG, kTabF32>(wm, rp, pl, early, stream);
+  }
+}
+
+template <int QK, typename XT, int T>
+int launch_spg(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, int groups, int tt, bool early, cudaStream_t stream) {
+  if constexpr (QK == kMx4) {
+    return launch_tt<QK, XT, T, 1>(wm, rp, pl, tt, early, stream);
+  } else {
+    if (groups == kSliceK / 32) return launch_tt<QK, XT, T, 1>(wm, rp, pl, tt, early, stream);
+    if (groups == kSliceK / 64) return launch_tt<QK, XT, T, 2>(wm, rp, pl, tt, early, stream);
+    return launch_tt<QK, XT, T, 4>(wm, rp, pl, tt, early, stream);
+  }
+}
+
+template <int QK, typename XT>
+int launch_rows_kernel(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
+  if constexpr (sizeof(XT) == 4) {
+    return launch_spg<QK, XT, 4>(wm, rp, pl, sh.groups, sh.tt, early, stream);
+  } else {
+    return launch_spg<QK, XT, 8>(wm, rp, pl, sh.groups, sh.tt, early, stream);
+  }
+}
+
+}  // namespace rows
+}  // namespace qmm

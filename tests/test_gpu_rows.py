@@ -1,0 +1,72 @@
+"""The few-rows kernel at the sizes where its split can go wrong -- chunks of 4, 8 and 16 rows, slices and clusters
+along K and their remainders, tables whose rows start on no word, experts of nought to twenty rows --
+against the exact product of the oracle. Needs a B200.
+
+Tolerances are the parity gates of the package: 1e-2 of the largest result for 16-bit activations (the output
+is rounded to 8 bits: 2^-9 of each value; everything before it is kept in 21 bits or more), 1e-5 for
+float32 (sums of K terms in float32, in pieces of 512: below 2^-24 * 512)."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import activations, affine_case, mxfp4_case, to_numpy, to_torch
+from metaljax_b200 import _lib, moe, qmm
+from oracle import qmm_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+DT = {"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}
+TOL = {"bf16": 1e-2, "f16": 1e-2, "f32": 1e-5}
+
+
+def _case(rng, kind, n, k, gs, tdt, lead=()):
+    if kind == "mxfp4":
+        out = mxfp4_case(rng, n, k, lead=lead)
+        return (*out[-2:], None), dict(group_size=32, bits=4, mode="mxfp4")
+    return affine_case(rng, n, k, gs, int(kind[3:]), tdt, lead=lead)[1:], dict(group_size=gs, bits=int(kind[3:]))
+
+
+@pytest.fixture(autouse=True)
+def _no_wait_ran_out():
+    yield
+    assert _lib.poll_status() == 0
+
+
+@pytest.mark.parametrize("kind,gs,x,tdt", [
+    ("int4", 64, "bf16", "bf16"), ("int4", 32, "bf16", "f32"), ("int4", 128, "f16", "f16"), ("int8", 32, "f16", "f16"),
+    ("int8", 64, "bf16", "bf16"), ("mxfp4", 32, "bf16", None), ("int4", 64, "f32", "f32"), ("int8", 128, "f32", "bf16"), ("mxfp4", 32, "f32", None),
+])
+@pytest.mark.parametrize("m,k,n", [
+    (2, 128, 1), (7, 384, 33), (8, 512, 300), (9, 640, 31), (16, 1152, 65), (5, 4480, 130), (3, 16384, 48), (12, 34048, 20), (17, 2176, 100),
+])
+def test_rows_at_the_edges(kind, gs, x, tdt, m, k, n):
+    if m > 16 and x != "f32":
+        pytest.skip("more rows of 16-bit activations are the tensor-core kernel's")
+    rng = np.random.default_rng(m * k + n)
+    (w, s, b), kw = _case(rng, kind, n, k, gs, tdt)
+    xs = activations(rng, (m, k), x)
+    args = [to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV)]
+    if x == "f32":
+        y = qmm.quantized_matmul(*args, **kw)
+    else:
+        with _lib.force_route("gemv_fmma"):                   # (a long K has the tensor-core kernel by default)
+            y = qmm.quantized_matmul(*args, **kw)
+    exact = O.qmm_exact(xs, w, s, b, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
+    assert O.rel_err(to_numpy(y).astype(np.float32), exact) <= TOL[x]
+
+
+@pytest.mark.parametrize("sizes", [[1], [0, 3, 0, 1], [20, 0, 17, 8, 9, 1, 0, 2], [0, 0, 0], [1] * 40])
+@pytest.mark.parametrize("kind,x", [("int4", "bf16"), ("int8", "f16"), ("mxfp4", "bf16")])
+def test_few_rows_per_expert(kind, x, sizes):
+    rng = np.random.default_rng(len(sizes) + sum(sizes))
+    k, n, total = 672 if kind == "mxfp4" else 704, 90, sum(sizes) + 1
+    (w, s, b), kw = _case(rng, kind, n, k, 64, x, lead=(len(sizes),))
+    xs = activations(rng, (total, k), x)
+    gsz = np.array(sizes, np.int32)
+    y = moe.ragged_dot(to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV), torch.from_numpy(gsz).to(DEV), **kw)
+    got = to_numpy(y).astype(np.float32)
+    assert not got[sum(sizes):].any()
+    if sum(sizes):
+        assert O.rel_err(got, O.ragged_qmm_exact(xs, w, s, b, gsz, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))) <= 1e-2
