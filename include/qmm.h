@@ -196,6 +196,35 @@ int qmm_moe_silu_mul(const void* gate, const void* up, void* out, int64_t elemen
 int qmm_moe_routed_sum(const void* rows, const int64_t* row_of_pair, const float* weights, void* out,
                        int64_t tokens, int k, int64_t width, int64_t total_rows, int dtype, void* stream);
 
+/* The whole gathered SwiGLU expert block of a mixture-of-experts layer (src/metaljax/moe.py:1283-1461):
+ *   out[t] = sum_j weights[t, j] * down_e(silu(gate_e(x[t])) * up_e(x[t])),  e = indices[t, j],
+ * as one sort of the pairs by expert, three grouped products, SwiGLU and the routed sum, all enqueued on
+ * `stream`; nothing is read back. x, out [tokens, d] bf16 | f16; indices [tokens, k] 32- or 64-bit; weights
+ * [tokens, k] float32; w1 (gate), w3 (up) [experts, ffn, d], w2 (down) [experts, d, ffn] packed, tables as in
+ * qmm_ragged_dot. `workspace` is qmm_moe_workspace_bytes of device memory (16-byte aligned; -1: bad shape).
+ * An expert index outside [0, experts) is reported (QMM_ERR_SHAPE from qmm_poll_status), never followed. */
+typedef struct {
+  const void* w;
+  const void* scales;
+  const void* biases;      /* NULL for mxfp4 */
+} qmm_moe_weight;
+typedef struct {
+  uint32_t struct_size;    /* sizeof(qmm_moe_block) */
+  int32_t mode, bits, group_size;
+  int32_t x_dtype, table_dtype;
+  int32_t k, experts, index_bytes;
+  int64_t tokens, d, ffn;
+  const void* x;
+  const void* indices;
+  const float* weights;
+  qmm_moe_weight w1, w3, w2;
+  void* out;
+  void* workspace;
+  int64_t workspace_bytes;
+} qmm_moe_block;
+int64_t qmm_moe_workspace_bytes(const qmm_moe_block* block);
+int qmm_moe_experts(const qmm_moe_block* block, void* stream);
+
 /* Replaces `mx.dequantize(w, scales, biases, group_size, bits[, mode])`, which the
  * reference uses to pin the packed layout (tests/test_qmm.py:121,
  * tests/test_qmm_mxfp4.py:192): out [.., N, K] bf16 | f16 | f32, each element one

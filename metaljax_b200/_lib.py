@@ -117,6 +117,8 @@ _SIGNATURES = {
     "qmm_moe_routed_sum": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                           ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int,
                                           ctypes.c_void_p]),
+    "qmm_moe_workspace_bytes": (ctypes.c_int64, [_T]),
+    "qmm_moe_experts": (ctypes.c_int, [_T, ctypes.c_void_p]),
     "qmm_launch": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.c_void_p]),
     # include/qmm_decode.h
     "qmm_decode_add_rmsnorm": (ctypes.c_int, [ctypes.c_void_p] * 5 + [ctypes.c_int64, ctypes.c_int64,
@@ -184,7 +186,8 @@ def native():
         loader = importlib.machinery.ExtensionFileLoader("_native", NATIVE_PATH)
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
         loader.exec_module(module)
-        module.bind(*(ctypes.cast(getattr(lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul",)))
+        module.bind(*(ctypes.cast(getattr(lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul", "qmm_moe_workspace_bytes",
+                                                                                             "qmm_moe_experts")))
         _native = module
     return _native
 

@@ -49,8 +49,11 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // out = silu(gate) * up, the product rounded as the two-step form rounds it: silu to T, then
 // the product to T.
 template <typename T>
-__global__ void silu_mul_kernel(const uint4* __restrict__ gate, const uint4* __restrict__ up, uint4* __restrict__ out,
+__global__ void silu_mul_kernel(const uint4* gate, const uint4* up, uint4* out,   // (out may be gate)
+                               
                                 int64_t pieces) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < pieces; i += stride) {
     float g[8], u[8];
@@ -71,6 +74,8 @@ template <typename T>
 __global__ void routed_sum_kernel(const uint4* __restrict__ rows, const int64_t* __restrict__ row_of_pair,
                                   const float* __restrict__ weights, uint4* __restrict__ out, int64_t tokens, int k,
                                   int64_t pieces, int64_t total_rows, int* status) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int64_t t = blockIdx.x; t < tokens; t += gridDim.x) {
     for (int64_t pc = threadIdx.x; pc < pieces; pc += blockDim.x) {
       float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -110,11 +115,11 @@ extern "C" int qmm_moe_silu_mul(const void* gate, const void* up, void* out, int
   if (blocks > cap) blocks = cap;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == QMM_BF16)
-    silu_mul_kernel<__nv_bfloat16><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
-        static_cast<const uint4*>(gate), static_cast<const uint4*>(up), static_cast<uint4*>(out), pieces);
+    launch_early(silu_mul_kernel<__nv_bfloat16>, static_cast<unsigned>(blocks), 256, 0, st, static_cast<const uint4*>(gate), static_cast<const uint4*>(up),
+                 static_cast<uint4*>(out), pieces);
   else
-    silu_mul_kernel<__half><<<static_cast<unsigned>(blocks), 256, 0, st>>>(
-        static_cast<const uint4*>(gate), static_cast<const uint4*>(up), static_cast<uint4*>(out), pieces);
+    launch_early(silu_mul_kernel<__half>, static_cast<unsigned>(blocks), 256, 0, st, static_cast<const uint4*>(gate), static_cast<const uint4*>(up),
+                 static_cast<uint4*>(out), pieces);
   count_launch();
   return check_launch("moe silu_mul_kernel");
 }
@@ -138,11 +143,11 @@ extern "C" int qmm_moe_routed_sum(const void* rows, const int64_t* row_of_pair, 
   const int threads = pieces >= 256 ? 256 : (pieces >= 128 ? 128 : 64);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == QMM_BF16)
-    routed_sum_kernel<__nv_bfloat16><<<static_cast<unsigned>(blocks), threads, 0, st>>>(
-        static_cast<const uint4*>(rows), row_of_pair, weights, static_cast<uint4*>(out), tokens, k, pieces, total_rows, status);
+    launch_early(routed_sum_kernel<__nv_bfloat16>, static_cast<unsigned>(blocks), threads, 0, st, static_cast<const uint4*>(rows), row_of_pair, weights,
+                 static_cast<uint4*>(out), tokens, k, pieces, total_rows, status);
   else
-    routed_sum_kernel<__half><<<static_cast<unsigned>(blocks), threads, 0, st>>>(
-        static_cast<const uint4*>(rows), row_of_pair, weights, static_cast<uint4*>(out), tokens, k, pieces, total_rows, status);
+    launch_early(routed_sum_kernel<__half>, static_cast<unsigned>(blocks), threads, 0, st, static_cast<const uint4*>(rows), row_of_pair, weights,
+                 static_cast<uint4*>(out), tokens, k, pieces, total_rows, status);
   count_launch();
   return check_launch("moe routed_sum_kernel");
 }

@@ -21,9 +21,14 @@ namespace {
 typedef int (*QuantizedMatmul)(const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, qmm_tensor*, int,
                                int, int, int, void*);
 
+typedef int64_t (*MoeWorkspace)(const qmm_moe_block*);
+typedef int (*MoeExperts)(const qmm_moe_block*, void*);
+
 // Entry points of the library that is loaded (ctypes hands their addresses over: one library per
 // process, whichever file it was loaded from).
 QuantizedMatmul g_quantized_matmul = nullptr;
+MoeWorkspace g_moe_workspace = nullptr;
+MoeExperts g_moe_experts = nullptr;
 
 bool dtype_of(at::ScalarType t, qmm_dtype* d) {
   d->lanes = 1;
@@ -128,13 +133,82 @@ PyObject* quantized_matmul(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(y));
 }
 
-// bind(address of qmm_quantized_matmul)
+int elem_of(at::ScalarType t) {
+  switch (t) {
+    case at::kBFloat16: return QMM_BF16;
+    case at::kHalf: return QMM_F16;
+    case at::kFloat: return QMM_F32;
+    case at::kByte: return QMM_U8;
+    default: return -1;
+  }
+}
+
+// moe_experts(x, indices, weights, (w, scales, biases | None) x 3: gate, up, down, group_size, bits, mode)
+// -> the result, a status code, or None (declined: what is not the plain block takes the step by step way)
+PyObject* moe_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 15 || !g_moe_experts) Py_RETURN_NONE;
+  const at::Tensor *x = plain_tensor(a[0]), *idx = plain_tensor(a[1]), *wts = plain_tensor(a[2]);
+  if (!x || !idx || !wts || x->dim() != 2 || idx->dim() != 2 || !x->is_contiguous() || !idx->is_contiguous()) Py_RETURN_NONE;
+  const long gs = PyLong_AsLong(a[12]), bits = PyLong_AsLong(a[13]), mode = PyLong_AsLong(a[14]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
+  if ((bits != 4 && bits != 8) || gs < 32 || wts->numel() != idx->numel() || idx->size(0) != x->size(0)) Py_RETURN_NONE;
+  qmm_moe_block b = {};
+  b.struct_size = sizeof(b);
+  b.mode = static_cast<int32_t>(mode); b.bits = static_cast<int32_t>(bits); b.group_size = static_cast<int32_t>(gs);
+  b.x_dtype = elem_of(x->scalar_type());
+  if (b.x_dtype != QMM_BF16 && b.x_dtype != QMM_F16) Py_RETURN_NONE;
+  if (idx->scalar_type() != at::kLong && idx->scalar_type() != at::kInt) Py_RETURN_NONE;
+  b.index_bytes = idx->scalar_type() == at::kLong ? 8 : 4;
+  b.tokens = x->size(0); b.d = x->size(1); b.k = static_cast<int32_t>(idx->size(1));
+  qmm_moe_weight* ws[3] = {&b.w1, &b.w3, &b.w2};
+  for (int i = 0; i < 3; ++i) {
+    const at::Tensor *w = plain_tensor(a[3 + 3 * i]), *s = plain_tensor(a[4 + 3 * i]);
+    const at::Tensor* z = a[5 + 3 * i] == Py_None ? nullptr : plain_tensor(a[5 + 3 * i]);
+    if (!w || !s || (!z && a[5 + 3 * i] != Py_None) || w->dim() != 3 || s->dim() != 3 || !w->is_contiguous() || !s->is_contiguous() || (z && !z->is_contiguous()))
+      Py_RETURN_NONE;
+    if ((w->scalar_type() != at::kUInt32 && w->scalar_type() != at::kInt) || w->device() != x->device() || s->device() != x->device()) Py_RETURN_NONE;
+    if (i == 0) {
+      b.experts = static_cast<int32_t>(w->size(0));
+      b.ffn = w->size(1);
+      b.table_dtype = elem_of(s->scalar_type());
+    }
+    const int64_t rows = i < 2 ? b.ffn : b.d, k = i < 2 ? b.d : b.ffn;
+    if (w->size(0) != b.experts || w->size(1) != rows || w->size(2) * 32 != k * bits || k % gs || s->size(0) != b.experts || s->size(1) != rows || s->size(2) != k / gs ||
+        elem_of(s->scalar_type()) != b.table_dtype || (z && (z->sizes() != s->sizes() || z->scalar_type() != s->scalar_type() || z->device() != x->device())))
+      Py_RETURN_NONE;
+    *ws[i] = {w->const_data_ptr(), s->const_data_ptr(), z ? z->const_data_ptr() : nullptr};
+  }
+  if (idx->device() != x->device() || wts->device() != x->device()) Py_RETURN_NONE;
+  const int64_t need = g_moe_workspace(&b);
+  if (need < 0) Py_RETURN_NONE;
+  at::Tensor y, work, w32;
+  try {
+    w32 = wts->scalar_type() == at::kFloat && wts->is_contiguous() ? *wts : wts->to(at::kFloat).contiguous();
+    y = at::detail::empty_cuda({b.tokens, b.d}, x->scalar_type(), x->device(), std::nullopt);
+    work = at::detail::empty_cuda({need}, at::kByte, x->device(), std::nullopt);
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+  b.x = x->const_data_ptr(); b.indices = idx->const_data_ptr(); b.weights = w32.const_data_ptr<float>();
+  b.out = y.data_ptr(); b.workspace = work.data_ptr(); b.workspace_bytes = need;
+  const int rc = g_moe_experts(&b, c10::cuda::getCurrentCUDAStream(x->get_device()).stream());
+  if (rc) return PyLong_FromLong(rc);
+  return THPVariable_Wrap(std::move(y));
+}
+
+// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts)
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 1) {
+  if (n != 3) {
     PyErr_SetString(PyExc_TypeError, "bind takes the entry points' addresses");
     return nullptr;
   }
   g_quantized_matmul = reinterpret_cast<QuantizedMatmul>(PyLong_AsVoidPtr(a[0]));
+  g_moe_workspace = reinterpret_cast<MoeWorkspace>(PyLong_AsVoidPtr(a[1]));
+  g_moe_experts = reinterpret_cast<MoeExperts>(PyLong_AsVoidPtr(a[2]));
   if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }
@@ -142,6 +216,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef kMethods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(bind)), METH_FASTCALL, nullptr},
     {"quantized_matmul", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(quantized_matmul)), METH_FASTCALL, nullptr},
+    {"moe_experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(moe_experts)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -115,6 +115,13 @@ def moe_experts(x, indices, weights, w1, w3, w2, group_size=64, bits=4, mode="af
     weights are applied and the K terms summed in `sum_dtype` as the reference does
     after its gathered dots (src/metaljax/moe.py:1446-1453).
     """
+    if sum_dtype == torch.float32:           # the whole block in one native call
+        done = _lib.native().moe_experts(x, indices, weights, *w1, *w3, *w2, group_size, bits, _mode_id(mode))
+        if done.__class__ is int:
+            _lib.check(done)
+        if done is not None:
+            STATS["ragged_dot"] += 3
+            return done
     t, k = indices.shape
     e = w1[0].shape[0]
     order, tok, group_sizes = sort_pairs(indices, e)

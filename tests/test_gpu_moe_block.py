@@ -1,0 +1,46 @@
+"""The expert block in one native call against its steps one by one, at the edges of the pair sort (one pair, experts
+without a pair, more pairs than a warp, more than a block's warps) and on either product kernel. Needs a B200."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import activations, affine_case, mxfp4_case, to_numpy, to_torch
+from metaljax_b200 import _lib, moe
+from oracle import qmm_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def _case(rng, kind, n, k, tdt, lead):
+    if kind == "mxfp4":
+        return (*mxfp4_case(rng, n, k, lead=lead)[1:], None), dict(group_size=32, bits=4, mode="mxfp4")
+    return affine_case(rng, n, k, 64, 4, tdt, lead=lead)[1:], dict(group_size=64, bits=4)
+
+
+@pytest.mark.parametrize("tokens,experts,k", [(1, 4, 1), (3, 8, 2), (33, 40, 4), (150, 4, 2)])
+@pytest.mark.parametrize("kind,x,index", [("int4", "bf16", torch.int64), ("mxfp4", "f16", torch.int32)])
+def test_expert_block_in_one_call(kind, x, index, tokens, experts, k):
+    """Against the block's steps one by one: the same kernels on either side of the same 16-bit hand-offs, so
+    what differs is the order of float32 sums (a chunk of rows may be another width) and what 8 bits make of that: the parity gate."""
+    rng = np.random.default_rng(tokens + experts)
+    d, f = 192, 320
+    packs, kw = [], None
+    for n, kk in ((f, d), (f, d), (d, f)):
+        arrays, kw = _case(rng, kind, n, kk, x, lead=(experts,))
+        packs.append(tuple(None if a is None else to_torch(a, DEV) for a in arrays))
+    xs = to_torch(activations(rng, (tokens, d), x, 0.5), DEV)
+    idx = torch.from_numpy(np.stack([rng.permutation(experts)[:k] for _ in range(tokens)])).to(index).to(DEV)
+    wts = torch.from_numpy(rng.random((tokens, k)).astype(np.float32)).to(DEV)
+    got = moe.moe_experts(xs, idx, wts, *packs, **kw)
+    order, tok, sizes = moe.sort_pairs(idx.to(torch.int64), experts)
+    rows = xs.index_select(0, tok)
+    act = moe.silu_mul(moe.ragged_dot(rows, *packs[0], sizes, **kw), moe.ragged_dot(rows, *packs[1], sizes, **kw))
+    want = moe.routed_sum(moe.ragged_dot(act, *packs[2], sizes, **kw), order, wts, tokens, k)
+    assert O.rel_err(to_numpy(got).astype(np.float32), to_numpy(want).astype(np.float64)) <= 1e-2
+    idx[0, 0] = experts                                       # an index outside the experts: reported, never followed
+    moe.moe_experts(xs, idx, wts, *packs, **kw)
+    with pytest.raises(_lib.QmmError):
+        _lib.poll_status()
