@@ -3,24 +3,41 @@
 //   y[t, f] = sum_k x[t, k] * deq(w)[f, k]          (transpose=True of the reference's call,
 //                                                    src/metaljax/qmm.py:2491)
 //
-// The WEIGHT is the MMA's A operand and lives in tensor memory: a tile is 128 output
-// features (= 128 TMEM lanes) x 64 K-elements, so one dequantizing thread owns one weight
-// row, reads its 32 packed bytes (64 for 8-bit) from shared memory, applies its own
-// per-group scale and bias in registers, and writes the bf16/f16 result straight to TMEM
-// with tcgen05.st -- the dequantized weight never exists in shared or global memory. The
-// ACTIVATIONS are the B operand: TMA brings [BT tokens x 64 K] tiles into shared memory in
+// The WEIGHT is the MMA's A operand and lives in tensor memory: a CTA's tile is 128 output
+// features (= 128 TMEM lanes), so one dequantizing thread owns one weight row, reads its packed bytes of
+// 64 K-elements from shared memory, applies its own per-group scale and bias in registers, and writes the
+// bf16/f16 result straight to TMEM with tcgen05.st -- the dequantized weight never exists in shared or
+// global memory. The ACTIVATIONS are the B operand: TMA brings [tokens x 64 K] tiles into shared memory in
 // the 128-byte-swizzled K-major layout tcgen05.mma reads. The accumulator D[feature, token]
-// (float32) sits in TMEM; the epilogue reads it back with tcgen05.ld, casts and stores
-// y[token, feature].
+// (float32) sits in TMEM; the epilogue reads it back with tcgen05.ld, casts and stores y[token, feature].
 //
-// Warp roles (18 warps): 0 = TMA producer, 1 = MMA issuer (+ TMEM allocation),
-// 2..17 = sixteen dequant/epilogue warps in four teams of four (one warp per TMEM lane
-// quarter); the teams take K blocks round-robin.
+// Wide token tiles (256) are worked on by PAIRS of CTAs (`cta_group::2`): 256 features x 256 tokens, each CTA
+// dequantizes its own 128 features and holds half of the tokens' activations, so an SM reads 16 KB of activations per 64 K
+// instead of 32: a lone CTA's 36 KB per 64 K were what L2 could not deliver (42 bytes a clock and SM at 974 TFLOP/s).
 //
-// One persistent CTA per SM walks a list of tiles (segment, token tile, feature tile).
+// Scales and biases of a box travel with it (cp.async by the weights' producer, a few bytes a row): read by the dequantizing
+// threads from global memory, 2 bytes per row and 64 K, they thrashed what is left of L1 next to 200 KB of shared memory, and their
+// latency was the dequantization's. Packed weights come in boxes of 128 rows x 128 bytes (256 4-bit K-elements, 128 8-bit ones, 64 float ones) through a
+// ring of their own: a box of 32 bytes a row for 64 4-bit elements costs the TMA unit and L2 a request per 32 bytes.
+//
+// Warp roles (19 warps): 0 = activations' producer, 1 = MMA issuer (+ TMEM allocation), 2..17 = sixteen
+// dequant/epilogue warps in four teams of four (one warp per TMEM lane quarter) that take K blocks round-robin,
+// 18 = weights' producer.
+//
+// Persistent workers (a CTA or a pair) walk a list of tiles (segment, token tile, feature tile).
 // A segment is a run of x rows that meets one weight matrix: the whole of x for the plain
 // op, one batch of a batched weight, or one expert's rows of a ragged (grouped) product,
 // in which case the per-expert row offsets are prefix sums of `group_sizes` computed here.
+// Tiles that do not fill the workers evenly are shared out by weight boxes (every worker an equal, contiguous stretch of K over
+// consecutive tiles): a tile's pieces meet through float32 partial tiles in scratch, which the worker that holds the
+// tile's last piece adds up in K order. A worker walks its stretch from the end, so the piece another worker waits for is
+// the first that it makes, and waits only on lower-numbered workers, which were scheduled before it.
+//
+// Measured (device time, before: one CTA per tile at every width, 32-byte boxes, tables from global memory, an issuer behind a branch, split
+// products added up by a second kernel), int4 group 64: 2048 rows 14336 x 4096 248 -> 202 us, 4096 x 14336 219 -> 178; 512 rows 28672 x 4096
+// 130 -> 102; 64 rows 28672 x 4096 59.7 -> 41.6, 4096 x 4096 16.4 -> 11.6, 4096 x 14336 31.2 -> 21.7; 128 rows 4096 x 14336 47 -> 24.6; 8-bit
+// group 128, 45 rows 14336 x 4096 33 -> 24. What bounds it: at 64 rows the dequantizing warps (about 300 clocks a K block and SM), at 256 the tensor
+// cores' 514 clocks a block plus what the dequantization does not keep up with, under the power cap.
 //
 // Every wait is bounded: when a barrier does not flip within ~2 s of SM clock the kernel
 // records the place in a status word, stops issuing work and drains.
@@ -28,34 +45,25 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include <cstdio>
-#include <cstdlib>
+#include <atomic>
 #include <type_traits>
 
 #include "qmm_internal.h"
+#include "qmm_ptx.cuh"
 
 namespace qmm {
 namespace {
 
-constexpr int kBF = 128;        // features per tile (MMA M, TMEM lanes)
-constexpr int kBK = 64;         // K elements per pipeline stage
-// Dequant / epilogue teams of four warps (one per TMEM lane quarter): five for wide token tiles,
-// where the dequantization is what the issuer waits for (C2a 965 -> 1009 TFLOP/s, C2b 1106 -> 1199,
-// int8 891 -> 991 against four); four for narrow tiles (five lose there: fewer ring slots fit)
-// and for float weights (whose 16 KB slots leave room for four).
-template <int QK, int BT>
-struct Teams {
-#ifndef QMM_TC_WIDE_TEAMS
-#define QMM_TC_WIDE_TEAMS 5
-#endif
-  static constexpr int kTeams = (BT <= 64 || QK == 3 /* kFloat */) ? 4 : QMM_TC_WIDE_TEAMS;
-  static constexpr int kThreads = (2 + 4 * kTeams) * 32;
-};
+using namespace ptx;
+
+constexpr int kBF = 128;        // features of a CTA's tile (TMEM lanes)
+constexpr int kBK = 64;         // K elements of a K block
+constexpr int kTeams = 4;       // dequant / epilogue teams of four warps (one per TMEM lane quarter)
+constexpr int kDequantWarps = 4 * kTeams;
+constexpr int kWarps = 3 + kDequantWarps;
+constexpr int kThreads = kWarps * 32;
 constexpr int kMaxSegments = 256;
-constexpr long long kSpinLimit = 4000000000LL;  // SM clocks (~2 s)
-#ifndef QMM_TC_TRACING
-#define QMM_TC_TRACING 0        // development builds: cycles per wait site (-DQMM_TC_TRACING=1)
-#endif
+constexpr int kBoxBytes = 128;  // bytes of a weight row in a box
 
 enum { kAff4 = 0, kAff8 = 1, kMx4 = 2, kFloat = 3 };    // kFloat: the weight holds values of the activation type (nothing to dequantize)
 
@@ -65,76 +73,25 @@ struct TcParams {
   void* y;
   const int32_t* group_sizes;  // ragged: [segments]; else NULL
   int* status;                 // device status word (0 = ok)
-  long long* trace;            // development aid: per-CTA cycles spent in each wait site, or NULL
   int64_t M;                   // rows of x per segment (dense) or total rows (ragged)
-  int64_t K, N;
-  int64_t segments;            // weight matrices
+  int64_t N;
   int64_t w_seg_rows;          // rows of the packed weight between segments (N, or 0 = shared)
-  int group_size, table_dtype, y_dtype;
-  int splits;                  // > 1: the K blocks of a tile are divided among `splits` CTAs, each
-  float* partial;              // of which writes its float32 partial tile to partial[split][M][N]
-  int64_t item0, item_end;     // the work items [item0, item_end) of the persistent walk are this launch's
-  int64_t tail_tile0;          // >= 0: this launch splits only the tiles from here on, and partial is
-  int64_t tail_tiles;          //       compact: partial[split][tile - tail_tile0][BT][128]
+  int K, segments, group_shift, table_dtype, y_dtype;
+  int w_stages;                // places of the weight ring, and of the ring of table chunks
+  unsigned w_inverse;          // 2^32 / w_stages rounded up: counts are divided by a multiplication
+  int table_entry, table_pitch, table_unit;   // bytes of a table entry; of a row's entries in shared memory; on which every chunk's entries start (8, 4 or less)
+  int chunk_shift;             // weight boxes per table chunk (log2)
+  int64_t table_bytes;         // of a whole table
+  int split;                   // > 1: `split` consecutive workers share the K of each tile (and the walk is one tile long): a cluster that
+  int cluster_adds;            // adds up over distributed shared memory, or partial tiles for the kernel that follows
+  int shared_tiles;            // the first tiles of the walk are shared out by weight boxes ...
+  unsigned share, share_more;  // ... `share` to every worker, one more to the first `share_more`
+  float* partial;              // [CTA][tokens of a tile][128]: a CTA's partial tile
+  unsigned long long* ready;   // [CTA][dequant warps]: == epoch when that warp's part of the partial tile is there
+  unsigned long long epoch;    // a value that no earlier launch used
 };
 
 // ---- PTX wrappers ---------------------------------------------------------------------
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait. Returns false (and records `where`) when the barrier never flips or another
-// role has already given up.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          int where) {
-  if (mbar_try(bar, parity)) return true;
-  const long long t0 = clock64();
-  int spins = 0;
-  while (!mbar_try(bar, parity)) {
-    if ((++spins & 1023) == 0) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > kSpinLimit) {
-        *abort_flag = where;
-        return false;
-      }
-    }
-  }
-  return true;
-}
-
-__device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, void* dst, uint64_t* bar, int c0,
-                                            int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-      : "memory");
-}
 
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -143,40 +100,113 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 remote_ld128(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// `n` arrivals on a barrier of this CTA, or (cluster address) of another's. The latter releases nothing wider than the CTA either: what
+// it announces are tensor-memory stores (ordered by tcgen05's own fences) and TMA writes, and a cluster-wide release costs a memory barrier.
+__device__ __forceinline__ void arrive_n(uint32_t bar, uint32_t n) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(n) : "memory");
+}
+__device__ __forceinline__ void remote_arrive_n(uint32_t bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
+// Bounded wait for a phase of a barrier: false (with `where` recorded at abort_flag) when it does not flip within kSpinLimit clocks, or as
+// soon as another waiter of the CTA has given up. CLUSTER: the other CTA of a pair arrives on it. The hint (nanoseconds) lets the
+// hardware hold the thread, so that waiting warps do not poll away the issue slots of those that work.
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, uint32_t abort_flag, int where) {
+  auto poll = [&]() -> bool {
+    uint32_t done;
+    if constexpr (CLUSTER)
+      asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+                   : "=r"(done) : "r"(bar), "r"(parity), "r"(100000) : "memory");
+    else
+      asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+                   : "=r"(done) : "r"(bar), "r"(parity), "r"(100000) : "memory");
+    return done != 0;
+  };
+  if (poll()) return true;
+  const long long t0 = clock64();
+  while (!poll()) {
+    uint32_t gave_up;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(gave_up) : "r"(abort_flag) : "memory");
+    if (gave_up) return false;
+    if (clock64() - t0 > kSpinLimit) {
+      asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_flag), "r"(where) : "memory");
+      return false;
+    }
+  }
+  return true;
 }
 
-// D[tmem_d] (+)= A[tmem_a] * B[desc_b]; A from tensor memory, B from shared memory.
-__device__ __forceinline__ void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{ .reg .pred p; setp.ne.b32 p, %4, 0;"
-      "  tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
+// The tensor-core instructions are issued by one elected lane, chosen inside the instruction sequence: the warp around it stays
+// converged, so that descriptors and addresses are uniform registers (behind a branch on the lane, every operand of every MMA
+// was moved into one first: 80 to 110 cycles an MMA, above the 64 that it runs for).
+
+// Arrives on `bar` (of both CTAs of a pair: a mask of their ranks in the cluster) when the MMAs issued so far have completed.
+template <bool PAIR>
+__device__ __forceinline__ void tc_commit(uint32_t bar, [[maybe_unused]] uint16_t pair) {
+  if constexpr (PAIR)
+    asm volatile("{ .reg .pred e; elect.sync _|e, 0xffffffff;"
+                 "  @e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1; }" ::"r"(bar),
+                 "h"(pair) : "memory");
+  else
+    asm volatile("{ .reg .pred e; elect.sync _|e, 0xffffffff;"
+                 "  @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0]; }" ::"r"(bar) : "memory");
 }
 
-#define QMM_R32(a, o) a[o + 0], a[o + 1], a[o + 2], a[o + 3], a[o + 4], a[o + 5], a[o + 6], a[o + 7]
+// D[tmem_d] (+)= A[tmem_a] * B over a K block: A from tensor memory (8 columns per 16 K), B from shared memory (32 bytes per
+// 16 K; the descriptor's words).
+#define QMM_MMA(GROUP, COL, ADV, ACC)                                    \
+  "add.u32 a, %1, " COL "; add.u32 lo, %2, " ADV "; mov.b64 b, {lo, %3};" \
+  "@e tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], [a], b, %4, " ACC ";"
+template <bool PAIR>
+__device__ __forceinline__ void tc_mma_block(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (PAIR)
+    asm volatile("{ .reg .pred e, p, t; .reg .b32 a, lo; .reg .b64 b; elect.sync _|e, 0xffffffff; setp.ne.b32 p, %5, 0; setp.eq.b32 t, 0, 0;"
+                 QMM_MMA("2", "0", "0", "p") QMM_MMA("2", "8", "2", "t") QMM_MMA("2", "16", "4", "t") QMM_MMA("2", "24", "6", "t") "}"
+                 ::"r"(tmem_d), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+  else
+    asm volatile("{ .reg .pred e, p, t; .reg .b32 a, lo; .reg .b64 b; elect.sync _|e, 0xffffffff; setp.ne.b32 p, %5, 0; setp.eq.b32 t, 0, 0;"
+                 QMM_MMA("1", "0", "0", "p") QMM_MMA("1", "8", "2", "t") QMM_MMA("1", "16", "4", "t") QMM_MMA("1", "24", "6", "t") "}"
+                 ::"r"(tmem_d), "r"(tmem_a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+}
+
 #define QMM_ASM_R(o) "r"(r[o]), "r"(r[o + 1]), "r"(r[o + 2]), "r"(r[o + 3]), "r"(r[o + 4]), "r"(r[o + 5]), "r"(r[o + 6]), "r"(r[o + 7])
 #define QMM_ASM_W(o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
 
-// 32 lanes x 32 consecutive 32-bit columns: thread i of the warp owns lane (base + i).
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-      QMM_ASM_R(0), QMM_ASM_R(8), QMM_ASM_R(16), QMM_ASM_R(24)
-      : "memory");
+__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds8(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
 }
 
-// 32 lanes x 8 consecutive 32-bit columns.
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
-               QMM_ASM_R(0)
+// 32 lanes x 16 / 32 consecutive 32-bit columns: thread i of the warp owns lane (base + i).
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+               QMM_ASM_R(0), QMM_ASM_R(8)
                : "memory");
 }
 
@@ -264,8 +294,6 @@ __device__ __forceinline__ void dequant_aff4(const uint32_t (&w)[NW], float s, f
   }
 }
 
-// 8-bit affine, NW packed words -> NW*2 pairs: float32 FMA per element, rounded to the
-// 16-bit type in pairs.
 // The same for float32 tables (what the packer emits when a bias is not exactly
 // representable in the narrow type): the magic pair is widened to float32, one float32 FMA
 // per element with (s, b - C s), one rounding to the pair type.
@@ -294,6 +322,15 @@ __device__ __forceinline__ void dequant_aff4_wide(const uint32_t (&w)[NW], float
   }
 }
 
+// x0, x1 = s * (x0 - 2^23) + b, the same for x1: two elements per instruction.
+__device__ __forceinline__ void take_magic_and_scale(float& x0, float& x1, float s, float b) {
+  asm("{ .reg .b64 x, m, s, b; mov.b64 x, {%0, %1}; mov.b64 m, {%2, %2}; mov.b64 s, {%3, %3}; mov.b64 b, {%4, %4};"
+      "  add.rn.f32x2 x, x, m; fma.rn.f32x2 x, x, s, b; mov.b64 {%0, %1}, x; }"
+      : "+f"(x0), "+f"(x1) : "f"(-8388608.0f), "f"(s), "f"(b));
+}
+
+// 8-bit affine, NW packed words -> NW*2 pairs: float32 FMA per element, rounded to the
+// 16-bit type in pairs.
 template <typename XT, int NW>
 __device__ __forceinline__ void dequant_aff8(const uint32_t (&w)[NW], float s, float b, uint32_t* out) {
   using H = Half2Ops<XT>;
@@ -301,10 +338,11 @@ __device__ __forceinline__ void dequant_aff8(const uint32_t (&w)[NW], float s, f
   for (int j = 0; j < NW; ++j) {
     float q[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      q[e] = __uint_as_float(__byte_perm(w[j], 0x4B000000u, 0x7540u + e)) - 8388608.0f;
-    out[j * 2] = H::pack(fmaf(s, q[0], b), fmaf(s, q[1], b));
-    out[j * 2 + 1] = H::pack(fmaf(s, q[2], b), fmaf(s, q[3], b));
+    for (int e = 0; e < 4; ++e) q[e] = __uint_as_float(__byte_perm(w[j], 0x4B000000u, 0x7540u + e));
+    take_magic_and_scale(q[0], q[1], s, b);
+    take_magic_and_scale(q[2], q[3], s, b);
+    out[j * 2] = H::pack(q[0], q[1]);
+    out[j * 2 + 1] = H::pack(q[2], q[3]);
   }
 }
 
@@ -336,387 +374,482 @@ __device__ __forceinline__ void dequant_mx4(const uint32_t (&w)[NW], uint32_t e8
 
 // ---- UMMA descriptors ------------------------------------------------------------------
 
-// K-major operand in the 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);        // start address
-  d |= static_cast<uint64_t>(1) << 16;                        // leading byte offset (unused)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;                // stride byte offset
-  d |= static_cast<uint64_t>(1) << 46;                        // descriptor version (sm_100)
-  d |= static_cast<uint64_t>(2) << 61;                        // SWIZZLE_128B
-  return d;
-}
+// K-major operand in the 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart. Low word: start address, leading
+// byte offset (unused); high word: stride byte offset, descriptor version (sm_100), SWIZZLE_128B.
+__device__ __forceinline__ uint32_t desc_low(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
 
-// kind::f16, float32 accumulate, both operands K-major.
-__host__ __device__ constexpr uint32_t instr_desc(int fmt /*0 f16, 1 bf16*/, int m, int n) {
-  return (1u << 4) | (static_cast<uint32_t>(fmt) << 7) | (static_cast<uint32_t>(fmt) << 10) |
-         (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+// kind::f16, float32 accumulate, both operands K-major; N goes in with `<< 17` in eighths.
+__host__ __device__ constexpr uint32_t instr_desc(int fmt /*0 f16, 1 bf16*/, int m) {
+  return (1u << 4) | (static_cast<uint32_t>(fmt) << 7) | (static_cast<uint32_t>(fmt) << 10) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
 // ---- shared-memory plan -----------------------------------------------------------------
 
+// Rings of activation tiles (each with a 32-column slot of dequantized weights in tensor memory per K block) and of
+// weight boxes. A step is what a team dequantizes and the issuer waits for and commits at once: two K blocks, since the waits,
+// fences and arrivals around a step cost a team about as much as one block's arithmetic.
 template <int QK, int BT>
 struct Plan {
-  static constexpr int kTeams = Teams<QK, BT>::kTeams;
-  static constexpr int kThreads = Teams<QK, BT>::kThreads;
+  static constexpr bool kPair = BT == 256;
+  static constexpr int kCtas = kPair ? 2 : 1;
   static constexpr int kBits = (QK == kFloat) ? 16 : ((QK == kAff8) ? 8 : 4);
-  static constexpr int kWRowBytes = kBK * kBits / 8;          // 32, 64 or (float weights) 128
-  static constexpr int kXBytes = BT * kBK * 2;                // one activation stage
-  static constexpr int kWBytes = kBF * kWRowBytes;            // one packed-weight stage
-  static constexpr int kStageBytes = kXBytes + kWBytes;
-  // as many stages as fit next to the barriers and the tile tables (the dequantized-A ring in
-  // tensor memory has one 32-column slot per stage)
-  static constexpr int kFit = (232448 - 4200 - 2048) / kStageBytes;
-  // The depth is a multiple of the number of dequant teams, so that a ring slot is always
-  // handled by the same team: a waiter then never lags its barrier by two phases, which a
-  // parity wait could not tell from "ready".
-  // Narrow token tiles leave most of tensor memory to the A ring and stage little: twelve
-  // slots instead of eight cover the per-slot latency chain (TMA, one team's dequantization,
-  // MMA, commit) that bounds a CTA's rate at a few dozen rows.
-  static constexpr int kACol0 = (BT <= 64) ? 64 : (BT <= 128 ? 128 : 256);   // A ring starts here (D is columns [0, BT))
-  static constexpr int kTmemFit = (512 - kACol0) / 32;
-  static constexpr int kMost = kFit < kTmemFit ? kFit : kTmemFit;
-  // (at most three rounds of the teams: twelve slots for four teams, five for five at 256 tokens)
-  static constexpr int kStages = (kMost / kTeams >= 3 ? 3 : (kMost / kTeams >= 2 ? 2 : 1)) * kTeams;
-  static_assert(kMost >= kTeams, "one slot per team must fit");
+  static constexpr int kRowBytes = kBK * kBits / 8;           // of a weight row in a K block: 32, 64 or (float weights) 128
+  static constexpr int kPer = kBoxBytes / kRowBytes;          // K blocks of a box
+  static constexpr int kStep = QK == kFloat && BT > 64 ? 1 : 2;      // (float weights' boxes leave no room for four of two)
+  static constexpr int kStepsPerBox = kPer >= kStep ? kPer / kStep : 1;
+  static constexpr int kXBlock = (BT / kCtas) * kBK * 2;      // a K block of this CTA's activations
+  static constexpr int kXBytes = kStep * kXBlock;
+  static constexpr int kWBytes = kBF * kBoxBytes;
+  static constexpr int kACol0 = BT;                           // the A ring starts behind D's columns [0, BT)
+  static constexpr int kStages = kStep == 1 || (BT <= 64 && QK != kFloat) ? 6 : 4;
   static constexpr int kBarBytes = 1024;
-  static constexpr int kSmem = kStages * kStageBytes + kBarBytes + 1024 /* alignment slack */;
-  static constexpr int kDCols = BT;                           // accumulator columns
-  static constexpr int kTmemCols = 512;
+  static constexpr int kBudget = 227 * 1024 - 4608;           // dynamic shared memory (the tile tables are static)
+  static constexpr int kFixed = kStages * kXBytes + kBarBytes + 1024 /* alignment slack */;
+  static constexpr int kMostBoxes = 10;
+  static constexpr bool kMaySplit = kStages * kXBytes >= BT * kBF * 4;      // a cluster's partial tile goes where the activations were
+  // A team need not touch every box, and a parity wait cannot tell a box from the one two rounds before it: the team's wait for
+  // its A slot, which comes first, has to imply that the box before in the same place has been used up.
+  static constexpr int kLeastPlaces = (kStages * kStep + (kPer > kStep ? kPer - kStep : 0) + kPer - 1) / kPer;
+  // ... and a team that waits for its next A slot must not be able to lag that slot's barrier by two phases.
+  static_assert(kStages >= kTeams, "");
+  static_assert(kACol0 + kStages * kStep * 32 <= 512, "the A ring fits tensor memory");
+  static_assert(kFixed + kLeastPlaces * kWBytes <= kBudget, "");
+  static_assert((2 * kMostBoxes + 3 * kStages + 2) * 8 + 16 <= kBarBytes, "");
 };
 
-struct TileInfo {
-  int split, kb_lo, kb_hi;   // this work item's share of the tile's K blocks
-  int seg;
-  int64_t tile;      // index in the walk
-  int64_t row0;      // first x / y row of this tile
-  int rows;          // valid rows in the tile (<= BT)
-  int64_t f0;        // first feature
+// A piece of work: K blocks [kb_lo, kb_hi) of a tile.
+struct Piece {
+  int kb_lo, kb_hi, tile;
+  bool begins, ends;           // it holds the tile's first / last K block
+  int seg, rows;               // rows: token rows of the tile that exist
+  int64_t row0, f0;            // first x / y row, first feature (of the whole tile)
 };
 
-// Tile t of the persistent walk -> (segment, token tile, feature tile); feature tiles vary
-// fastest inside a token tile so that concurrently running CTAs share the activation tile
-// and stream disjoint weight rows.
-template <int BT>
-__device__ __forceinline__ bool tile_at(int64_t item, const int64_t* seg_tile0, const int64_t* seg_row0,
-                                        int nseg, int64_t ftiles, int64_t N, int splits, int num_kb,
-                                        TileInfo* out) {
-  // work item -> (tile, split): the splits of a tile are adjacent items, so they run together
-  int64_t t = item;
-  out->split = 0;
-  if (splits > 1) {                                   // (the common case divides nothing)
-    t = item / splits;
-    out->split = static_cast<int>(item - t * splits);
+// The walk of worker `w` of `workers`: its stretch of the shared tiles from the end, then every workers-th tile.
+template <int BT, int kPer>
+struct Walk {
+  int lo, hi, next, w, workers, boxes, num_kb, tiles;
+  __device__ __forceinline__ Walk(const TcParams& p, int w_, int workers_, int num_kb_, int tiles_) : w(w_), workers(workers_), num_kb(num_kb_), tiles(tiles_) {
+    boxes = (num_kb + kPer - 1) / kPer;
+    lo = hi = 0;
+    if (p.split > 1) {                             // one piece, its stretch of K of the cluster's tile
+      const int tile = w / p.split, part = w - tile * p.split;
+      lo = tile * boxes + boxes * part / p.split;
+      hi = tile * boxes + boxes * (part + 1) / p.split;
+      next = 0x7fffffff;
+      return;
+    }
+    if (p.shared_tiles) {
+      lo = first_box(p, w);
+      hi = lo + static_cast<int>(p.share) + (static_cast<unsigned>(w) < p.share_more ? 1 : 0);
+    }
+    next = p.shared_tiles + w;
   }
-  if (t >= seg_tile0[nseg]) return false;
-  out->tile = t;
-  out->kb_lo = static_cast<int>(static_cast<int64_t>(out->split) * num_kb / splits);
-  out->kb_hi = static_cast<int>(static_cast<int64_t>(out->split + 1) * num_kb / splits);
-  int s = 0;
-  while (t >= seg_tile0[s + 1]) ++s;
-  const int64_t local = t - seg_tile0[s];
-  const int64_t tt = local / ftiles, ft = local % ftiles;
-  const int64_t rows = seg_row0[s + 1] - seg_row0[s];
-  out->seg = s;
-  out->row0 = seg_row0[s] + tt * BT;
-  const int64_t left = rows - tt * BT;
-  out->rows = static_cast<int>(left < BT ? left : BT);
-  out->f0 = ft * kBF;
-  (void)N;
-  return true;
-}
+  static __device__ __forceinline__ int first_box(const TcParams& p, int w) {
+    return static_cast<int>(static_cast<unsigned>(w) * p.share + min(static_cast<unsigned>(w), p.share_more));
+  }
+  __device__ __forceinline__ bool take(Piece* out, const int* seg_tile0, const int64_t* seg_row0, int nseg, int ftiles, int features) {
+    int t, b0, b1;
+    if (hi > lo) {
+      t = static_cast<int>(static_cast<unsigned>(hi - 1) / static_cast<unsigned>(boxes));
+      const int base = t * boxes;
+      b0 = (lo > base ? lo : base) - base;
+      b1 = hi - base;
+      hi = base + b0;
+    } else {
+      t = next;
+      next = static_cast<int>(static_cast<unsigned>(next) + static_cast<unsigned>(workers));
+      if (static_cast<unsigned>(t) >= static_cast<unsigned>(tiles)) return false;
+      b0 = 0;
+      b1 = boxes;
+    }
+    out->tile = t;
+    out->begins = b0 == 0;
+    out->ends = b1 == boxes;
+    out->kb_lo = b0 * kPer;
+    out->kb_hi = b1 * kPer < num_kb ? b1 * kPer : num_kb;
+    int s = 0;
+    while (t >= seg_tile0[s + 1]) ++s;
+    const unsigned local = static_cast<unsigned>(t - seg_tile0[s]);
+    // feature tiles vary fastest inside a token tile, so that concurrently running workers share the activation
+    // tile and stream disjoint weight rows
+    const unsigned tt = local / static_cast<unsigned>(ftiles), ft = local - tt * static_cast<unsigned>(ftiles);
+    out->seg = s;
+    out->row0 = seg_row0[s] + static_cast<int64_t>(tt) * BT;
+    const int64_t left = seg_row0[s + 1] - out->row0;
+    out->rows = static_cast<int>(left < BT ? left : BT);
+    out->f0 = static_cast<int64_t>(ft) * features;
+    return true;
+  }
+};
 
-// SPLIT: the K blocks of a tile are shared among p.splits CTAs (float32 partial tiles). A
-// separate instantiation, so that the unsplit kernel keeps compile-time K bounds.
-template <int QK, typename XT, int BT, bool SPLIT>
-__global__ void __launch_bounds__((Teams<QK, BT>::kThreads), 1)
-qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
-                   const TcParams p) {
+template <int QK, typename XT, int BT>
+__global__ void __launch_bounds__(kThreads, 1)
+qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const TcParams p) {
   using P = Plan<QK, BT>;
-  constexpr int kTeams = P::kTeams;
+  constexpr bool kPair = P::kPair;
+  constexpr int kCtas = P::kCtas, kPer = P::kPer, kStep = P::kStep, kStages = P::kStages, kMostBoxes = P::kMostBoxes;
+  constexpr int kTables = QK == kMx4 ? 1 : 2;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* bar_base = smem + P::kStages * P::kStageBytes;
-  uint64_t* full = reinterpret_cast<uint64_t*>(bar_base);      // [kStages] TMA landed
-  uint64_t* empty = full + P::kStages;                         // [kStages] stage consumed
-  uint64_t* a_full = empty + P::kStages;                       // [kStages] dequantized A is in TMEM
-  uint64_t* d_full = a_full + P::kStages;                      // accumulator complete
-  uint64_t* d_empty = d_full + 1;                              // accumulator drained
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  __shared__ int64_t seg_tile0[kMaxSegments + 1];
+  __shared__ int seg_tile0[kMaxSegments + 1];
   __shared__ int64_t seg_row0[kMaxSegments + 1];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nseg = static_cast<int>(p.segments);
-  const int64_t ftiles = (p.N + kBF - 1) / kBF;
-  const int num_kb = static_cast<int>((p.K + kBK - 1) / kBK);
+  const uint32_t smem = (smem_u32(smem_raw) + 1023) & ~1023u;
+  const uint32_t x_at = smem, bars = smem + kStages * P::kXBytes, w_at = bars + P::kBarBytes, t_at = w_at + p.w_stages * P::kWBytes;
+  const uint32_t wfull = bars, wempty = wfull + 8 * kMostBoxes;         // a weight box and its table entries have landed / have been read
+  const uint32_t xfull = wempty + 8 * kMostBoxes;                         // a step's activations have landed
+  const uint32_t empty = xfull + 8 * kStages;                           // a step's MMAs are done: its activations and its A slot are free
+  const uint32_t a_full = empty + 8 * kStages;                          // (a pair's leader) a step's dequantized weights are in TMEM
+  const uint32_t d_full = a_full + 8 * kStages, d_empty = d_full + 8;   // accumulator complete / (leader) drained
+  const uint32_t tmem_slot = d_empty + 8, abort_at = tmem_slot + 4;
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int in_cluster = kPair || p.cluster_adds ? static_cast<int>(cluster_rank()) : 0;
+  const int rank = kPair ? in_cluster & 1 : 0, leader = in_cluster - rank;            // within the pair
+  [[maybe_unused]] const uint16_t pair_mask = static_cast<uint16_t>(3 << leader);
+  const int worker = static_cast<int>(blockIdx.x) / kCtas, workers = static_cast<int>(gridDim.x) / kCtas;
+  const int nseg = p.segments;
+  const int ftiles = static_cast<int>((p.N + kBF * kCtas - 1) / (kBF * kCtas));
+  const int num_kb = (p.K + kBK - 1) / kBK;
 
   // Programmatic dependent launch: the grid that follows may be scheduled as soon as every CTA
   // of this one has got here (it touches memory only after its own griddepcontrol.wait). This
   // grid sets itself up, and requests its first weight boxes, while the grid it depends on is
   // still running; what that grid produces -- the activations, the group sizes of a ragged
-  // product -- is read only after thread 0's griddepcontrol.wait, and everything this grid
-  // writes is downstream of those reads.
+  // product -- is read only after a griddepcontrol.wait, and everything this grid writes is
+  // downstream of those reads.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.group_sizes) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int s = threadIdx.x; s < nseg; s += kThreads) seg_row0[s + 1] = p.group_sizes[s] > 0 ? p.group_sizes[s] : 0;
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
-    if (p.group_sizes) asm volatile("griddepcontrol.wait;" ::: "memory");
-    int64_t tiles = 0, rows = 0;
+    int64_t rows = 0;
+    int tiles = 0;
+    seg_row0[0] = 0;
+    seg_tile0[0] = 0;
     for (int s = 0; s < nseg; ++s) {
-      seg_tile0[s] = tiles;
-      seg_row0[s] = rows;
-      int64_t r = p.group_sizes ? p.group_sizes[s] : p.M;
+      int64_t r = p.group_sizes ? seg_row0[s + 1] : p.M;
       if (p.group_sizes && rows + r > p.M) r = p.M - rows;
-      if (r < 0) r = 0;
       rows += r;
-      tiles += ((r + BT - 1) / BT) * ftiles;
+      tiles += static_cast<int>((r + BT - 1) / BT) * ftiles;
+      seg_tile0[s + 1] = tiles;
+      seg_row0[s + 1] = rows;
     }
-    seg_tile0[nseg] = tiles;
-    seg_row0[nseg] = rows;
-    for (int i = 0; i < P::kStages; ++i) {
-      mbar_init(&full[i], 1);
-      mbar_init(&empty[i], 1 + 4);
+    auto init = [](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n)); };
+    for (int i = 0; i < p.w_stages; ++i) {
+      init(wfull + 8 * i, QK == kFloat ? 1 : 1 + 32);
+      init(wempty + 8 * i, 4 * P::kStepsPerBox);
     }
-    for (int i = 0; i < P::kStages; ++i) mbar_init(&a_full[i], 4);
-    mbar_init(d_full, 1);
-    mbar_init(d_empty, 4 * kTeams);
-    *abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < kStages; ++i) {
+      init(xfull + 8 * i, 1);
+      init(empty + 8 * i, 1);
+      init(a_full + 8 * i, 4 * kCtas);
+    }
+    init(d_full, 1);
+    init(d_empty, kDequantWarps * kCtas);
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(abort_at), "r"(0) : "memory");
+    mbar_init_fence();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(P::kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (kPair) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (kPair) cluster_barrier();          // the partner's barriers and tensor memory are there
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  // Waits go through here so that a development build can account the cycles per wait site.
-  long long waited[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  const bool tracing = QMM_TC_TRACING && p.trace != nullptr;
-  long long trace_c0 = 0, trace_n0 = 0;
-  if (tracing && threadIdx.x == 0) {
-    trace_c0 = clock64();
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(trace_n0));
-  }
-  auto twait = [&](uint64_t* bar, uint32_t parity, volatile int* flag, int where) -> bool {
-    if (!tracing) return mbar_wait(bar, parity, flag, where);
-    const long long t0 = clock64();
-    const bool r = mbar_wait(bar, parity, flag, where);
-    waited[where] += clock64() - t0;
-    return r;
-  };
+  uint32_t tmem_base;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot) : "memory");
+  tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
+  const int tiles = seg_tile0[nseg];
+  Walk<BT, kPer> walk(p, worker, workers, num_kb, tiles);
+  Piece pc = {};
+  auto wait = [&](uint32_t bar, uint32_t parity, int where) -> bool { return wait_phase(bar, parity, abort_at, where); };
+  // Columns of the MMA: the token rows that exist, in the widths the instruction takes (a pair's CTAs hold half each).
+  auto columns = [&]() -> int { return kPair ? (pc.rows + 31) & ~31 : (pc.rows + 15) & ~15; };
 
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
+    // ---------------- activations ----------------
     if (lane == 0) {
-      uint32_t it = 0, early = 0;
-      TileInfo ti;
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      uint32_t s = 0, ph = 0;
       bool ok = true;
-      // The weight boxes of the first tile's first ring (the stages start out free) go out before
-      // the wait for the preceding grid; their activation boxes follow it.
-      const int64_t first = p.item0 + blockIdx.x;
-      if (first < p.item_end && tile_at<BT>(first, seg_tile0, seg_row0, nseg, ftiles, p.N, SPLIT ? p.splits : 1, num_kb, &ti)) {
-        const int64_t wrow = ti.seg * p.w_seg_rows + ti.f0;
-        for (int kb = ti.kb_lo; kb < ti.kb_hi && early < static_cast<uint32_t>(P::kStages); ++kb, ++early) {
-          mbar_expect_tx(&full[early], P::kStageBytes);
-          tma_load_2d(&w_map, smem + early * P::kStageBytes + P::kXBytes, &full[early], kb * P::kWRowBytes, static_cast<int>(wrow));
+      while (ok && walk.take(&pc, seg_tile0, seg_row0, nseg, ftiles, kBF * kCtas)) {
+        const int row = static_cast<int>(pc.row0) + (kPair ? rank * (columns() / 2) : 0);
+        for (int kb = pc.kb_lo; kb < pc.kb_hi; kb += kStep) {
+          if (!(ok = wait(empty + 8 * s, ph ^ 1u, 1))) break;
+          const uint32_t bar = xfull + 8 * s;
+          const int blocks = kStep == 1 || kb + 1 < pc.kb_hi ? kStep : 1;
+          mbar_expect_tx(bar, blocks * P::kXBlock);
+          for (int i = 0; i < blocks; ++i) tma_load_2d(&x_map, x_at + s * P::kXBytes + i * P::kXBlock, bar, (kb + i) * kBK, row);
+          if (++s == static_cast<uint32_t>(kStages)) { s = 0; ph ^= 1u; }
         }
       }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      for (int64_t t = first; ok && t < p.item_end && tile_at<BT>(t, seg_tile0, seg_row0, nseg, ftiles, p.N, SPLIT ? p.splits : 1, num_kb, &ti);
-           t += gridDim.x) {
-        const int64_t wrow = ti.seg * p.w_seg_rows + ti.f0;
-        for (int kb = ti.kb_lo; kb < ti.kb_hi; ++kb, ++it) {
-          const int s = it % P::kStages;
-          uint8_t* stage = smem + s * P::kStageBytes;
-          if (it < early) {              // armed above, its weight box is on the way
-            tma_load_2d(&x_map, stage, &full[s], kb * kBK, static_cast<int>(ti.row0));
-            continue;
-          }
-          const uint32_t ph = (it / P::kStages) & 1;
-          if (!(ok = twait(&empty[s], ph ^ 1, abort_flag, 1))) break;
-          mbar_expect_tx(&full[s], P::kStageBytes);
-          tma_load_2d(&x_map, stage, &full[s], kb * kBK, static_cast<int>(ti.row0));
-          tma_load_2d(&w_map, stage + P::kXBytes, &full[s], kb * P::kWRowBytes, static_cast<int>(wrow));
+    }
+  } else if (warp == kWarps - 1) {
+    // ---------------- weights and tables (nothing the grid before writes: they need not wait for it) ----------------
+    const int groups = QK == kFloat ? 1 : p.K >> p.group_shift;
+    int s = 0;
+    [[maybe_unused]] int ts = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    while (ok && walk.take(&pc, seg_tile0, seg_row0, nseg, ftiles, kBF * kCtas)) {
+      const int row = static_cast<int>(pc.seg * p.w_seg_rows + pc.f0) + rank * kBF;
+      const int last = static_cast<int>(p.N - pc.f0) - rank * kBF - 1;                  // the tile's last row of this weight (or before its first)
+      int64_t row_at[kBF / 32];                    // where the lane's rows start in a table
+#pragma unroll
+      for (int i = 0; i < kBF / 32; ++i) row_at[i] = static_cast<int64_t>(row + min(i * 32 + lane, last)) * groups * p.table_entry;
+      for (int kb = pc.kb_lo; kb < pc.kb_hi; kb += kPer) {
+        if (!(ok = wait(wempty + 8 * s, ph ^ 1u, 3))) break;
+        const uint32_t bar = wfull + 8 * s;
+        if (lane == 0) {
+          mbar_expect_tx(bar, P::kWBytes);
+          tma_load_2d(&w_map, w_at + s * P::kWBytes, bar, QK == kFloat ? kb * kBK : kb * P::kRowBytes, row);
         }
+        if constexpr (QK != kFloat) {
+          // A chunk of table entries with its first box (or the piece's). Every box's barrier gets the lanes' arrivals: they come
+          // when all of a lane's earlier copies have landed, so any box of a chunk answers for its entries.
+          const int box = kb / kPer, chunk = box >> p.chunk_shift;
+          if (kb == pc.kb_lo || (box & ((1 << p.chunk_shift) - 1)) == 0) {
+            const int g0 = ((chunk << p.chunk_shift) * (kPer * kBK)) >> p.group_shift, most = (kPer * kBK << p.chunk_shift) >> p.group_shift;
+            const int bytes = (groups - g0 < most ? groups - g0 : most) * p.table_entry;
+            const uint32_t slot = t_at + ts * (kTables * kBF * p.table_pitch) + lane * p.table_pitch;
+            if (++ts == p.w_stages) ts = 0;
+#pragma unroll
+            for (int i = 0; i < kBF / 32; ++i) {
+              const int64_t at = row_at[i] + g0 * p.table_entry;
+              const uint32_t dst = slot + i * 32 * p.table_pitch;
+              auto copy = [&](const void* table, uint32_t to) {
+                const uint8_t* src = static_cast<const uint8_t*>(table) + at;
+                if (p.table_unit == 8) {
+#pragma unroll 1
+                  for (int o = 0; o < bytes; o += 8) cp_async8(to + o, src + o);
+                } else {                           // from the word the first entry lies in; nothing past the table's end is read
+                  const int skew = static_cast<int>(at & 3);
+#pragma unroll 1
+                  for (int o = -skew; o < bytes; o += 4) {
+                    const int64_t room = p.table_bytes - (at + o);
+                    cp_async4(to + skew + o, src + o, room >= 4 ? 4 : static_cast<int>(room));
+                  }
+                }
+              };
+              copy(p.scales, dst);
+              if constexpr (QK != kMx4) copy(p.biases, dst + kBF * p.table_pitch);
+            }
+          }
+          cp_async_arrive(bar);
+        }
+        if (++s == p.w_stages) { s = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    // The whole warp walks the loop so that stage indices, descriptors and TMEM addresses
-    // are warp-uniform values; one lane issues the tensor-core instructions.
-    constexpr uint32_t idesc = instr_desc(std::is_same<XT, __nv_bfloat16>::value ? 1 : 0, kBF, BT);
-    uint32_t tile_n = 0, ph = 0;
-    int s = 0;
-    TileInfo ti;
-    bool ok = true;
-    for (int64_t t = p.item0 + blockIdx.x; ok && t < p.item_end && tile_at<BT>(t, seg_tile0, seg_row0, nseg, ftiles, p.N, SPLIT ? p.splits : 1, num_kb, &ti);
-         t += gridDim.x, ++tile_n) {
-      if (!(ok = twait(d_empty, (tile_n & 1) ^ 1, abort_flag, 2))) break;
-      tc_fence_after();
-      for (int kb = ti.kb_lo; kb < ti.kb_hi; ++kb) {
-        // The dequantized A of this K block sits in TMEM slot s, the slot of its shared-
-        // memory stage. Its writers waited for the stage's TMA barrier themselves, so
-        // their barrier also says that the activation tile has landed.
-        if (!(ok = twait(&a_full[s], ph, abort_flag, 4))) break;
-        const long long tf0 = tracing ? clock64() : 0;
-        tc_fence_after();
-        const long long ti0 = tracing ? clock64() : 0;
-        if (tracing) waited[3] += ti0 - tf0;         // cycles in the fence
-        const uint64_t bdesc = smem_desc_sw128(smem_u32(smem + s * P::kStageBytes));
-        const uint32_t acol = tmem_base + P::kACol0 + s * 32;
-        if (lane == 0) {
-#pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            tc_mma_ts(tmem_base, acol + k * 8, bdesc + static_cast<uint64_t>(k * 2), idesc,
-                      (kb > ti.kb_lo || k) ? 1u : 0u);
-          tc_commit(&empty[s]);     // frees the stage and its TMEM slot together
+    // ---------------- MMA issuer (of a pair: the leader's) ----------------
+    if (!kPair || rank == 0) {
+      constexpr uint32_t idesc0 = instr_desc(std::is_same<XT, __nv_bfloat16>::value ? 1 : 0, kBF * kCtas);
+      uint32_t s = 0, ph = 0, piece = 0;
+      for (; walk.take(&pc, seg_tile0, seg_row0, nseg, ftiles, kBF * kCtas); ++piece) {
+        const uint32_t idesc = __shfl_sync(0xffffffffu, idesc0 | (static_cast<uint32_t>(columns() >> 3) << 17), 0);
+        const int nkb = __shfl_sync(0xffffffffu, pc.kb_hi - pc.kb_lo, 0);
+        bool ok = kPair ? wait_phase<true>(d_empty, (piece & 1) ^ 1, abort_at, 2) : wait(d_empty, (piece & 1) ^ 1, 2);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        for (int j = 0; j < nkb; j += kStep) {
+          // (a pair's dequantizing warps answer for their own CTA's activations: see there)
+          if constexpr (kPair) ok = wait_phase<true>(a_full + 8 * s, ph, abort_at, 4);
+          else ok = wait(xfull + 8 * s, ph, 5) && wait(a_full + 8 * s, ph, 4);
+          if (!__all_sync(0xffffffffu, ok)) break;
+          tc_fence_after();
+          const uint32_t blo = desc_low(x_at + s * P::kXBytes), acol = tmem_base + P::kACol0 + s * (32 * kStep);
+          tc_mma_block<kPair>(tmem_base, acol, blo, kDescHigh, idesc, j ? 1u : 0u);
+          if (kStep == 2 && j + 1 < nkb) tc_mma_block<kPair>(tmem_base, acol + 32, blo + P::kXBlock / 16, kDescHigh, idesc, 1u);
+          tc_commit<kPair>(empty + 8 * s, pair_mask);
+          if (++s == static_cast<uint32_t>(kStages)) { s = 0; ph ^= 1u; }
         }
-        if (tracing) waited[0] += clock64() - ti0;   // cycles spent issuing
-        if (++s == P::kStages) { s = 0; ph ^= 1u; }
+        if (!__all_sync(0xffffffffu, ok)) break;
+        tc_commit<kPair>(d_full, pair_mask);
       }
-      if (ok && lane == 0) tc_commit(d_full);
     }
   } else {
     // ---------------- dequant + epilogue warps ----------------
-    const int team = (warp - 2) >> 2;            // takes K blocks with it % kTeams == team
+    const int team = (warp - 2) >> 2;            // takes steps i of a piece with i % kTeams == team
     const int quarter = warp & 3;                // TMEM lane quarter this warp may touch
-    const int frow = quarter * 32 + lane;        // feature row within the tile
+    const int frow = quarter * 32 + lane;        // feature row within the CTA's tile
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const int64_t groups = p.K / p.group_size;
-    uint32_t it = 0, tile_n = 0;
-    TileInfo ti;
+    const int groups = QK == kFloat ? 1 : p.K >> p.group_shift;
+    const bool twide = p.table_dtype == QMM_F32;
+    const uint32_t a_bar = kPair ? in_cta(a_full, leader) : a_full, d_bar = kPair ? in_cta(d_empty, leader) : d_empty;
+    const uint32_t wthread = w_at + frow * kBoxBytes;
+    uint32_t wbase = 0, sbase = 0, cbase = 0, piece = 0;    // boxes, steps and table chunks before this piece
     bool ok = true;
-    for (int64_t t = p.item0 + blockIdx.x; ok && t < p.item_end && tile_at<BT>(t, seg_tile0, seg_row0, nseg, ftiles, p.N, SPLIT ? p.splits : 1, num_kb, &ti);
-         t += gridDim.x, ++tile_n) {
-      int64_t feat = ti.f0 + frow;
+    for (; ok && walk.take(&pc, seg_tile0, seg_row0, nseg, ftiles, kBF * kCtas); ++piece) {
+      int64_t feat = pc.f0 + rank * kBF + frow;
       const bool feat_ok = feat < p.N;
       if (!feat_ok) feat = p.N - 1;
-      const int64_t trow = (ti.seg * p.w_seg_rows + feat) * groups;   // row of the scale tables
-      // The teams take the tile's K blocks round-robin (block kb belongs to the team whose
-      // number is the block's global iteration index modulo kTeams). The per-group constants
-      // of a block are requested one of the team's blocks ahead, so their global-memory
-      // latency hides behind the previous block's work.
-      const int tsize = (p.table_dtype == QMM_F32) ? 4 : 2;
-      const bool twide = p.table_dtype == QMM_F32;
-      auto fetch_tables = [&](int kbb, float (&fs)[2], float (&fb)[2], uint32_t (&fe)[2]) {
-        int64_t gidx[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          int64_t g = (kbb * kBK + h * 32) / p.group_size;
-          gidx[h] = trow + (g >= groups ? groups - 1 : g);
-          fs[h] = fb[h] = 0.0f;
-          fe[h] = 0u;
-        }
-        if constexpr (QK == kMx4) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) fe[h] = __ldg(reinterpret_cast<const uint8_t*>(p.scales) + gidx[h]);
-        } else if (twide) {          // raw bits until used; the width is decided outside the loads
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            fs[h] = __uint_as_float(table_raw(p.scales, true, gidx[h]));
-            fb[h] = __uint_as_float(table_raw(p.biases, true, gidx[h]));
-          }
-        } else {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            fs[h] = __uint_as_float(table_raw(p.scales, false, gidx[h]));
-            fb[h] = __uint_as_float(table_raw(p.biases, false, gidx[h]));
-          }
-        }
-      };
-      constexpr int kHalfWords = P::kWRowBytes / 8;                // packed words per 32 elements
-      const uint32_t it0 = it;
-      int kb = ti.kb_lo + static_cast<int>((static_cast<uint32_t>(team) + kTeams - (it0 % kTeams)) % kTeams);
-      const int kb_end = ti.kb_hi;
-      float sc[2], bi[2];
-      uint32_t e8[2];
-      if constexpr (QK == kFloat) { sc[0] = sc[1] = bi[0] = bi[1] = 0.0f; e8[0] = e8[1] = 0u; }
-      if (QK != kFloat && kb < kb_end) fetch_tables(kb, sc, bi, e8);
-      for (; kb < kb_end; kb += kTeams) {
-        it = it0 + static_cast<uint32_t>(kb - ti.kb_lo);
-        const int s = it % P::kStages;
-        float nsc[2] = {0.0f, 0.0f}, nbi[2] = {0.0f, 0.0f};
-        uint32_t ne8[2] = {0u, 0u};
-        if (QK != kFloat && kb + kTeams < kb_end) fetch_tables(kb + kTeams, nsc, nbi, ne8);
-        if (!(ok = twait(&full[s], (it / P::kStages) & 1, abort_flag, 5))) break;
-        const uint8_t* wsm = smem + s * P::kStageBytes + P::kXBytes + frow * P::kWRowBytes;
-        uint32_t packed[2][kHalfWords];
-#pragma unroll
-        for (int i = 0; i < P::kWRowBytes / 16; ++i) {
-          // float weights are 128-byte rows in the TMA unit's 128-byte swizzle (chunk i of row r
-          // sits at chunk i ^ (r & 7)): the lanes of a quarter-warp then read distinct banks
-          const int ci = (QK == kFloat) ? (i ^ (frow & 7)) : i;
-          const uint4 v = *reinterpret_cast<const uint4*>(wsm + ci * 16);
-          const uint32_t q4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) packed[(i * 4 + e) / kHalfWords][(i * 4 + e) % kHalfWords] = q4[e];
-        }
+      const uint32_t trow = static_cast<uint32_t>(pc.seg * p.w_seg_rows + feat) * static_cast<uint32_t>(groups);   // row of the tables (its low bits count)
+      const int nkb = pc.kb_hi - pc.kb_lo, steps = (nkb + kStep - 1) / kStep;
+      constexpr int kHalfBytes = P::kRowBytes / 2;                 // packed bytes of a half block
+      for (int i = team; i < steps; i += kTeams) {
+        const int j = i * kStep;                   // first K block of the step
+        const int halves = j + kStep <= nkb ? 2 * kStep : 2 * (nkb - j);
+        const uint32_t si = sbase + i, s = si % kStages, ph = (si / kStages) & 1u;
+        if (!(ok = wait(empty + 8 * s, ph ^ 1u, 7))) break;
+        uint32_t wi = wbase + j / kPer, wround = __umulhi(wi, p.w_inverse), ws = wi - wround * p.w_stages;
+        if (!(ok = wait(wfull + 8 * ws, wround & 1u, 6))) break;
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);     // this warp's share of the stage is in registers
-        uint32_t out[32];
+        tc_fence_after();
+        // This row's entries of the chunk: where the first is, and which is the last of the whole row
+        const int box = (pc.kb_lo + j) / kPer, chunk = box >> p.chunk_shift;
+        const int g0 = ((chunk << p.chunk_shift) * (kPer * kBK)) >> p.group_shift, glast = groups - 1 - g0;
+        const int k0 = (pc.kb_lo + j) * kBK - (chunk << p.chunk_shift) * (kPer * kBK);      // the step's first element in the chunk
+        const uint32_t ci = cbase + chunk - (pc.kb_lo / kPer >> p.chunk_shift), ts = ci - __umulhi(ci, p.w_inverse) * p.w_stages;
+        const uint32_t tbox = t_at + ts * (kTables * kBF * p.table_pitch) + frow * p.table_pitch + (p.table_unit < 4 ? ((trow + g0) * p.table_entry & 3u) : 0u);
+        auto half = [&](int q) {
+          // 16-byte chunk c of row r sits at chunk c ^ (r & 7) (the TMA unit's 128-byte swizzle): eight lanes read distinct banks
+          const uint32_t wrow = wthread + ws * P::kWBytes;
+          const int in_box = ((j % kPer) * 2 + q) % (2 * kPer);    // which 32 elements of the box
+          uint32_t packed[kHalfBytes / 4], out[16];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+          for (int c = 0; c < kHalfBytes / 16; ++c) {
+            const uint4 v = lds128<0>(wrow + (((in_box * (kHalfBytes / 16) + c) ^ (frow & 7)) << 4));
+            packed[c * 4] = v.x; packed[c * 4 + 1] = v.y; packed[c * 4 + 2] = v.z; packed[c * 4 + 3] = v.w;
+          }
           if constexpr (QK == kFloat) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) out[h * 16 + j] = packed[h][j];
-          } else if constexpr (QK == kAff4) {
-            if (twide)
-              dequant_aff4_wide<XT, kHalfWords>(packed[h], sc[h], bi[h], &out[h * 16]);
-            else
-              dequant_aff4<XT, kHalfWords>(packed[h], table_value(__float_as_uint(sc[h]), p.table_dtype),
-                                           table_value(__float_as_uint(bi[h]), p.table_dtype), &out[h * 16]);
-          } else if constexpr (QK == kAff8) {
-            dequant_aff8<XT, kHalfWords>(packed[h], table_value(__float_as_uint(sc[h]), p.table_dtype),
-                                         table_value(__float_as_uint(bi[h]), p.table_dtype), &out[h * 16]);
+            for (int e = 0; e < 16; ++e) out[e] = packed[e];
           } else {
-            dequant_mx4<XT, kHalfWords>(packed[h], e8[h], &out[h * 16]);
+            const int g = min((k0 + q * 32) >> p.group_shift, glast);
+            const uint32_t at = tbox + g * p.table_entry, bias_at = at + kBF * p.table_pitch;
+            if constexpr (QK == kMx4) {
+              dequant_mx4<XT>(packed, lds8(at), out);
+            } else {
+              const float fs = twide ? __uint_as_float(lds32<0>(at)) : table_value(lds16(at), p.table_dtype);
+              const float fb = twide ? __uint_as_float(lds32<0>(bias_at)) : table_value(lds16(bias_at), p.table_dtype);
+              if constexpr (QK == kAff8) dequant_aff8<XT>(packed, fs, fb, out);
+              else if (twide) dequant_aff4_wide<XT>(packed, fs, fb, out);
+              else dequant_aff4<XT>(packed, fs, fb, out);
+            }
           }
+          tmem_st16(tmem_base + lane_addr + P::kACol0 + s * (32 * kStep) + q * 16, out);
+        };
+        // (a block at a time, not the whole step unrolled: the sixteen warps are at sixteen places of this code, and much more of it
+        // no longer stays in the instruction caches)
+#pragma unroll 1
+        for (int q = 0; q < halves; q += 2) {
+          if (kPer == 1 && q == 2) {               // (float weights: a box is one block)
+            __syncwarp();
+            if (lane == 0) arrive_n(wempty + 8 * ws, 1);
+            ++wi;
+            wround = __umulhi(wi, p.w_inverse);
+            ws = wi - wround * p.w_stages;
+            if (!(ok = wait(wfull + 8 * ws, wround & 1u, 6))) break;
+            __syncwarp();
+          }
+          half(q);
+          half(q + 1);
         }
-        // TMEM slot s is free: the TMA for this stage was only issued after the MMAs that
-        // read the slot's previous contents had completed (the producer waited for them).
-        tc_fence_after();
-        const long long ts0 = tracing ? clock64() : 0;
-        tmem_st32(tmem_base + lane_addr + P::kACol0 + s * 32, out);
-        tmem_wait_st();
-        if (tracing) waited[0] += clock64() - ts0;   // cycles in tcgen05.st + wait
-        tc_fence_before();
+        if (!ok) break;
         __syncwarp();
-        if (lane == 0) mbar_arrive(&a_full[s]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) { sc[h] = nsc[h]; bi[h] = nbi[h]; e8[h] = ne8[h]; }
+        // this warp's share of the step's part of the box has been read (a piece's last box may have fewer steps than its barrier counts)
+        if (lane == 0) arrive_n(wempty + 8 * ws, kPer > 1 && i + 1 == steps ? P::kStepsPerBox - (j % kPer) / kStep : 1);
+        tmem_wait_st();
+        tc_fence_before();
+        if constexpr (kPair) {                     // ... and this CTA's activations of the step have landed
+          if (!(ok = wait(xfull + 8 * s, ph, 5))) break;
+        }
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (kPair) remote_arrive_n(a_bar + 8 * s, 1);
+          else arrive_n(a_bar + 8 * s, 1);
+        }
       }
-      it = it0 + static_cast<uint32_t>(kb_end - ti.kb_lo);
+      wbase += static_cast<uint32_t>(nkb + kPer - 1) / kPer;
+      sbase += static_cast<uint32_t>(nkb + kStep - 1) / kStep;
+      cbase += ((pc.kb_hi - 1) / kPer >> p.chunk_shift) - (pc.kb_lo / kPer >> p.chunk_shift) + 1;
       if (!ok) break;
       // ---- epilogue: the teams drain disjoint 32-column chunks of the accumulator ----
-      if (!(ok = twait(d_full, tile_n & 1, abort_flag, 7))) break;
+      if (!(ok = wait(d_full, piece & 1, 8))) break;
       __syncwarp();      // lanes leave the wait loop one by one; tcgen05.ld needs the whole warp
       tc_fence_after();
+      if (P::kMaySplit && p.cluster_adds) {        // this worker's share of the sums, over its activation ring (which is done with)
+#pragma unroll 1
+        for (int c0 = team * 32; c0 < pc.rows; c0 += 32 * kTeams) {
+          uint32_t r[32];
+          tmem_ld32(tmem_base + lane_addr + c0, r);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sts32(x_at + ((c0 + j) * kBF + frow) * 4, __uint_as_float(r[j]));
+        }
+        break;
+      }
+      const bool mine = team * 32 < pc.rows;
+      const bool whole = pc.begins && pc.ends, part_only = !pc.ends || p.split > 1;
+      if (mine && !part_only && !whole) {          // the tile's earlier pieces, made by the workers before this one
+        const int tile_box0 = pc.tile * walk.boxes;
+        for (int v = worker - 1; ok && v >= 0; --v) {
+          const unsigned long long* flag = p.ready + (static_cast<int64_t>(v) * kCtas + rank) * kDequantWarps + (warp - 2);
+          const long long t0 = clock64();
+          for (;;) {
+            unsigned long long got;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(got) : "l"(flag) : "memory");
+            if (got == p.epoch) break;
+            if (clock64() - t0 > kSpinLimit) {
+              asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_at), "r"(9) : "memory");
+              ok = false;
+              break;
+            }
+          }
+          if (Walk<BT, kPer>::first_box(p, v) <= tile_box0) break;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+      }
 #pragma unroll 1
       for (int c0 = team * 32; c0 < BT; c0 += 32 * kTeams) {
-        if (c0 >= ti.rows) break;                  // warp-uniform: no valid token rows left
+        if (c0 >= pc.rows) break;                  // warp-uniform: no valid token rows left
+        const int64_t in_partial = static_cast<int64_t>(c0) * kBF + frow;
+        float sum[32];
+        if (!part_only && !whole) {                // in K order: the workers' pieces, then this one
+          const int tile_box0 = pc.tile * walk.boxes;
+          int v = worker - 1;
+          while (Walk<BT, kPer>::first_box(p, v) > tile_box0) --v;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum[j] = 0.0f;
+          for (; v < worker; ++v) {
+            const float* part = p.partial + (static_cast<int64_t>(v) * kCtas + rank) * (BT * kBF) + in_partial;
+            float f[32];
+            // (volatile: all 32 requests go out before the first is waited for)
+#pragma unroll
+            for (int j = 0; j < 32; ++j) asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(f[j]) : "l"(part + j * kBF));
+#pragma unroll
+            for (int j = 0; j < 32; ++j) sum[j] += f[j];
+          }
+        }
         uint32_t r[32];
         tmem_ld32(tmem_base + lane_addr + c0, r);
         tmem_wait_ld();
-        if (SPLIT && p.tail_tile0 >= 0) {          // the last partial wave only: compact partial tiles
-          float* part = p.partial + ((static_cast<int64_t>(ti.split) * p.tail_tiles + (ti.tile - p.tail_tile0)) * BT + c0) * kBF + frow;
+        if (part_only) {
+          float* part = p.partial + static_cast<int64_t>(blockIdx.x) * (BT * kBF) + in_partial;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) part[j * kBF] = __uint_as_float(r[j]);
-        } else if (SPLIT && feat_ok) {             // a share of the tile's K: float32 partial sums
-          float* part = p.partial + static_cast<int64_t>(ti.split) * p.M * p.N;
+          for (int j = 0; j < 32; ++j) __stcg(part + j * kBF, __uint_as_float(r[j]));
+          continue;
+        }
+        if (!whole) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (c0 + j < ti.rows) part[(ti.row0 + c0 + j) * p.N + feat] = __uint_as_float(r[j]);
-        } else if (feat_ok) {
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[j] + __uint_as_float(r[j]));
+        }
+        if (feat_ok) {
+          const int64_t o0 = (pc.row0 + c0) * p.N + feat;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            if (c0 + j < ti.rows) {
-              const int64_t o = (ti.row0 + c0 + j) * p.N + feat;
+            if (c0 + j < pc.rows) {
+              const int64_t o = o0 + j * p.N;
               const float v = __uint_as_float(r[j]);
               if (p.y_dtype == QMM_BF16) reinterpret_cast<__nv_bfloat16*>(p.y)[o] = __float2bfloat16_rn(v);
               else if (p.y_dtype == QMM_F16) reinterpret_cast<__half*>(p.y)[o] = __float2half_rn(v);
@@ -727,13 +860,29 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(d_empty);
+      if (lane == 0) {
+        if constexpr (kPair) remote_arrive_n(d_bar, 1);
+        else arrive_n(d_bar, 1);
+      }
+      if (p.split > 1) break;
+      if (mine && part_only) {                     // this warp's part of the partial tile is there
+        if (lane == 0) {
+          __threadfence();
+          asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p.ready + static_cast<int64_t>(blockIdx.x) * kDequantWarps + (warp - 2)), "l"(p.epoch) : "memory");
+        }
+      } else if (mine && !whole) {                 // taken: a replay of this launch starts from flags that say nothing
+        const int tile_box0 = pc.tile * walk.boxes;
+        for (int v = worker - 1; v >= 0; --v) {
+          if (lane == 0) p.ready[(static_cast<int64_t>(v) * kCtas + rank) * kDequantWarps + (warp - 2)] = 0ull;
+          if (Walk<BT, kPer>::first_box(p, v) <= tile_box0) break;
+        }
+      }
     }
     // ragged: rows past the last group are zero
     if (p.group_sizes) {
       const int64_t used = seg_row0[nseg];
       const int64_t total = (p.M - used) * p.N;
-      const int64_t nth = 128 * kTeams;
+      constexpr int64_t nth = 32 * kDequantWarps;
       const int64_t tid = static_cast<int64_t>(blockIdx.x) * nth + (threadIdx.x - 64);
       for (int64_t i = tid; i < total; i += static_cast<int64_t>(gridDim.x) * nth) {
         const int64_t o = used * p.N + i;
@@ -745,153 +894,127 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
 
   tc_fence_before();
   __syncthreads();
+  __syncwarp();
+  if (p.cluster_adds) {
+    // ---- a cluster's workers add up their shares of the tile: each a stretch of the token rows, in K order ----
+    cluster_barrier();
+    if (warp >= 2 && warp < 2 + kDequantWarps && pc.rows > 0) {
+      const int part = in_cluster / kCtas, c0 = pc.rows * part / p.split, c1 = pc.rows * (part + 1) / p.split;
+      const int64_t feat = pc.f0 + rank * kBF + lane * 4;
+#pragma unroll 2
+      for (int c = c0 + warp - 2; c < c1; c += kDequantWarps) {
+        const uint32_t at = x_at + (c * kBF + lane * 4) * 4;
+        float4 sum = remote_ld128(in_cta(at, rank));
+        for (int v = 1; v < p.split; ++v) {
+          const float4 f = remote_ld128(in_cta(at, v * kCtas + rank));
+          sum.x += f.x; sum.y += f.y; sum.z += f.z; sum.w += f.w;
+        }
+        const int64_t o = (pc.row0 + c) * p.N + feat;
+        const float out[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (feat + i < p.N) {
+            if (p.y_dtype == QMM_BF16) reinterpret_cast<__nv_bfloat16*>(p.y)[o + i] = __float2bfloat16_rn(out[i]);
+            else if (p.y_dtype == QMM_F16) reinterpret_cast<__half*>(p.y)[o + i] = __float2half_rn(out[i]);
+            else reinterpret_cast<float*>(p.y)[o + i] = out[i];
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (kPair || p.cluster_adds) cluster_barrier();  // another CTA may still read or signal this one's memory until here
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(P::kTmemCols)
-                 : "memory");
+    if constexpr (kPair)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
   }
-  if (threadIdx.x == 0 && *abort_flag) atomicCAS(p.status, 0, *abort_flag);
-  if (tracing && threadIdx.x == 0) {
-    long long n1;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(n1));
-    p.trace[blockIdx.x * 16 + 14] = clock64() - trace_c0;
-    p.trace[blockIdx.x * 16 + 15] = n1 - trace_n0;
+  if (threadIdx.x == 0) {
+    int gave_up;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(gave_up) : "r"(abort_at) : "memory");
+    if (gave_up) atomicCAS(p.status, 0, gave_up);
   }
-  if (tracing && lane == 0 && (warp == 0 || warp == 1 || warp == 2 || warp == 6))
-    for (int i = 0; i < 8; ++i)
-      if (waited[i]) p.trace[blockIdx.x * 16 + (warp == 1 ? 8 : 0) + i] = waited[i];
+}
+
+// Adds up the partial tiles of a split product in K order and casts to y's type: a thread has four features of a token row.
+//   partial [tile][split][CTA of a pair][tokens of a tile][128]
+template <int BT>
+__global__ void __launch_bounds__(256)
+add_partials_kernel(const float* __restrict__ partial, const TcParams p, int ctas, int64_t token_tiles, int64_t ftiles) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");               // the partial tiles come from the grid before
+  const int lane = threadIdx.x & 31;
+  const int64_t rows = p.M * p.segments, units = rows * ftiles * ctas;
+  for (int64_t u = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; u < units; u += static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5)) {
+    const int64_t row = u / (ftiles * ctas), rest = u - row * (ftiles * ctas), ft = rest / ctas;
+    const int rank = static_cast<int>(rest - ft * ctas);
+    const int64_t seg = row / p.M, in_seg = row - seg * p.M, tt = in_seg / BT, tile = (seg * token_tiles + tt) * ftiles + ft;
+    const float* at = partial + ((tile * p.split * ctas + rank) * BT + (in_seg - tt * BT)) * kBF + lane * 4;
+    float4 sum = __ldcg(reinterpret_cast<const float4*>(at));
+#pragma unroll 4
+    for (int v = 1; v < p.split; ++v) {
+      const float4 f = __ldcg(reinterpret_cast<const float4*>(at + static_cast<int64_t>(v) * ctas * BT * kBF));
+      sum.x += f.x; sum.y += f.y; sum.z += f.z; sum.w += f.w;
+    }
+    const int64_t feat = (ft * ctas + rank) * kBF + lane * 4, o = row * p.N + feat;
+    const float out[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (feat + i < p.N) {
+        if (p.y_dtype == QMM_BF16) reinterpret_cast<__nv_bfloat16*>(p.y)[o + i] = __float2bfloat16_rn(out[i]);
+        else if (p.y_dtype == QMM_F16) reinterpret_cast<__half*>(p.y)[o + i] = __float2half_rn(out[i]);
+        else reinterpret_cast<float*>(p.y)[o + i] = out[i];
+      }
+    }
+  }
 }
 
 // ---- host side ---------------------------------------------------------------------------
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(sym);
-  }
-  return fn;
+// A value for TcParams::epoch: no two launches of a process share one, and scratch that held anything else
+// (float32 sums, zeros, other launches' values) does not hold it.
+unsigned long long next_epoch() {
+  static std::atomic<unsigned long long> count{0};
+  return (count.fetch_add(1, std::memory_order_relaxed) + 1) * 0x9E3779B97F4A7C15ull;
 }
 
-int make_map(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t inner, uint64_t outer,
-             uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swz) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return fail(QMM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {row_bytes};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(QMM_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-  return QMM_OK;
-}
+// Shares below this many weight boxes cost more in filling their pipeline than the idle workers.
+constexpr int kLeastBoxes = 2;
+// (More of them of wide tiles write and read more partial sums than they save.)
+constexpr int most_shares(int bt) { return bt >= 256 ? 8 : 16; }
+// What handing partial tiles from worker to worker takes, in K blocks (512 rows mxfp4 5760 x 2880, 46 tiles of 45 blocks on 74 pairs: 30 us shared
+// out, 26 a tile each).
+constexpr int exchange_blocks(int bt) { return bt >= 256 ? 32 : 12; }
 
-int* status_word() {
-  return device_status_word();
-}
-
-int sm_count() { return device_sm_count(); }
-
-// Launches with programmatic stream serialization (QMM_TC_PDL=0: plain stream order): the
-// kernels of this file wait for the grid before them themselves, as late as they can.
-bool tc_pdl() {
-  static const bool on = [] {
-    const char* e = getenv("QMM_TC_PDL");
-    return !(e && e[0] == '0');
-  }();
-  return on;
-}
-
-template <typename... Params, typename... Args>
-void launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream,
-                      Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = tc_pdl() ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);      // a failure stays as the last error: check_launch reports it
-}
-
-// Sums the float32 partial tiles of a split product in split order and casts to y's type.
-__global__ void splitk_reduce_kernel(const float* __restrict__ partial, void* __restrict__ y, int y_dtype,
-                                     int64_t total, int splits) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");               // the partial tiles come from the grid before
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x * 4;
-  for (int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4; i < total; i += stride) {
-    float4 acc = *reinterpret_cast<const float4*>(partial + i);
-    for (int s = 1; s < splits; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(partial + static_cast<int64_t>(s) * total + i);
-      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+// Clusters of `ctas` that fit the device at once. Asked once per kernel and size (with the first call's shared memory: all but all of it
+// either way, one CTA per SM).
+template <typename Kernel>
+int64_t max_clusters(Kernel kernel, int ctas, size_t smem) {
+  static std::atomic<int> known[kMaxDevices][9];
+  const int dev = current_device();
+  std::atomic<int>& n = known[dev][ctas];
+  int have = n.load(std::memory_order_relaxed);
+  if (!have) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(ctas);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&have, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      have = 0;
     }
-    if (y_dtype == QMM_BF16) {
-      __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
-      *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(y) + i) =
-          make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-    } else if (y_dtype == QMM_F16) {
-      __half2 lo = __floats2half2_rn(acc.x, acc.y), hi = __floats2half2_rn(acc.z, acc.w);
-      *reinterpret_cast<uint2*>(static_cast<__half*>(y) + i) =
-          make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-    } else {
-      *reinterpret_cast<float4*>(static_cast<float*>(y) + i) = acc;
-    }
+    if (have < 1) have = -1;
+    n.store(have, std::memory_order_relaxed);
   }
-}
-
-// The same for a split last wave: partial[split][tile][BT][128] -> the tiles' places in y
-// (one dense segment; tile t of the walk is token tile t / ftiles, feature tile t % ftiles).
-__global__ void splitk_tail_reduce_kernel(const float* __restrict__ partial, void* __restrict__ y, int y_dtype,
-                                          int64_t M, int64_t N, int64_t ftiles, int64_t tile0, int64_t tiles,
-                                          int bt, int splits) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int64_t per_tile = static_cast<int64_t>(bt) * kBF, total = tiles * per_tile;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const int64_t tl = i / per_tile, in = i - tl * per_tile;
-    const int64_t r = in / kBF, c = in - r * kBF;
-    const int64_t t = tile0 + tl;
-    const int64_t row = (t / ftiles) * bt + r, col = (t % ftiles) * kBF + c;
-    if (row >= M || col >= N) continue;
-    float acc = partial[i];
-    for (int s = 1; s < splits; ++s) acc += partial[static_cast<int64_t>(s) * total + i];
-    const int64_t o = row * N + col;
-    if (y_dtype == QMM_BF16) static_cast<__nv_bfloat16*>(y)[o] = __float2bfloat16_rn(acc);
-    else if (y_dtype == QMM_F16) static_cast<__half*>(y)[o] = __float2half_rn(acc);
-    else static_cast<float*>(y)[o] = acc;
-  }
-}
-
-// How many CTAs share one tile's K blocks. A short row run against a narrow weight leaves most
-// SMs without a tile while each busy CTA walks all of K alone; dividing K among CTAs fills the
-// machine. Only for one dense segment, N a multiple of 4 (the reduce kernel's vectors), and
-// never fewer than 8 K blocks per share.
-bool tail_split_enabled() {
-  static const bool on = [] { const char* e = getenv("QMM_TC_TAIL_SPLIT"); return !(e && *e == '0'); }();
-  return on;
-}
-
-int choose_splits(const qmm_problem& p, int64_t tiles, int num_kb) {
-  if (p.group_sizes || p.batch != 1 || (p.N & 3)) return 1;
-  int64_t s = sm_count() / (tiles < 1 ? 1 : tiles);
-  if (s > num_kb / 8) s = num_kb / 8;
-  if (s > 8) s = 8;
-  return s < 2 ? 1 : static_cast<int>(s);
+  return have;
 }
 
 template <int QK, typename XT, int BT>
@@ -902,150 +1025,147 @@ int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
   const int64_t w_rows = (p.w_batch_stride ? p.batch : 1) * p.N;
   CUtensorMap xm, wm;
   int rc;
-  const CUtensorMapDataType xdt =
-      std::is_same<XT, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  if ((rc = make_map(&xm, xdt, p.x, static_cast<uint64_t>(p.K), static_cast<uint64_t>(x_rows),
-                     static_cast<uint64_t>(p.K) * 2, kBK, BT, CU_TENSOR_MAP_SWIZZLE_128B)))
+  if ((rc = tensor_map_2d(&xm, p.x_dtype, p.x, static_cast<uint64_t>(p.K), static_cast<uint64_t>(x_rows), static_cast<uint64_t>(p.K) * 2, kBK, BT / P::kCtas, 1)))
     return rc;
   const uint64_t wrow_bytes = static_cast<uint64_t>(p.K) * P::kBits / 8;
-  if ((rc = make_map(&wm, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.w, wrow_bytes, static_cast<uint64_t>(w_rows),
-                     wrow_bytes, P::kWRowBytes, kBF, QK == kFloat ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE)))
-    return rc;
-  TcParams tp;
+  if (QK == kFloat)
+    rc = tensor_map_2d(&wm, p.x_dtype, p.w, static_cast<uint64_t>(p.K), static_cast<uint64_t>(w_rows), wrow_bytes, kBK, kBF, 1);
+  else
+    rc = tensor_map_2d(&wm, QMM_U8, p.w, wrow_bytes, static_cast<uint64_t>(w_rows), wrow_bytes, kBoxBytes, kBF, 1);
+  if (rc) return rc;
+  const ScratchBlock* block = scratch_override();
+  TcParams tp = {};
   tp.scales = p.scales; tp.biases = p.biases; tp.y = p.y; tp.group_sizes = p.group_sizes;
-  tp.status = scratch_override() ? scratch_override()->status : status_word();
-#if QMM_TC_TRACING
-  static long long* trace_buf = nullptr;
-  static const bool trace_on = getenv("QMM_TC_TRACE") != nullptr;
-  if (trace_on && !trace_buf) {
-    cudaMalloc(&trace_buf, sizeof(long long) * 16 * 1024);
-  }
-  if (trace_on) cudaMemsetAsync(trace_buf, 0, sizeof(long long) * 16 * 1024, stream);
-  tp.trace = trace_on ? trace_buf : nullptr;
-#else
-  tp.trace = nullptr;
-#endif
+  tp.status = block ? block->status : device_status_word();
   if (!tp.status) return fail(QMM_ERR_CUDA, "could not allocate the device status word");
-  tp.M = p.M; tp.K = p.K; tp.N = p.N;
-  tp.segments = p.batch;
+  tp.M = p.M; tp.K = static_cast<int>(p.K); tp.N = p.N;
+  tp.segments = static_cast<int>(p.batch);
   tp.w_seg_rows = p.w_batch_stride ? p.N : 0;
-  tp.group_size = p.group_size; tp.table_dtype = p.table_dtype; tp.y_dtype = p.y_dtype;
-  tp.splits = 1;
-  tp.partial = nullptr;
-  tp.item0 = 0;
-  tp.item_end = INT64_MAX;
-  tp.tail_tile0 = -1;
-  tp.tail_tiles = 0;
+  const int group = QK == kMx4 ? 32 : p.group_size;
+  tp.group_shift = group == 128 ? 7 : group == 64 ? 6 : 5;
+  tp.table_dtype = p.table_dtype; tp.y_dtype = p.y_dtype;
 
+  // The rings: as many weight boxes as fit next to the table chunks that go with them. A chunk is at least 8 bytes of a row (a
+  // box of 8-bit codes in groups of 128 has 2): the copies are per row, and their number is what they cost.
+  int box_bytes = 0, row_table = 0;
+  if (QK != kFloat) {
+    tp.table_entry = QK == kMx4 ? 1 : (p.table_dtype == QMM_F32 ? 4 : 2);
+    box_bytes = (P::kPer * kBK >> tp.group_shift) * tp.table_entry;
+    row_table = static_cast<int>(p.K >> tp.group_shift) * tp.table_entry;
+    tp.table_unit = row_table % 8 == 0 ? 8 : row_table % 4 == 0 ? 4 : 1;
+    while (box_bytes << tp.chunk_shift < 8) ++tp.chunk_shift;
+    const int chunk_bytes = box_bytes << tp.chunk_shift;
+    tp.table_pitch = tp.table_unit >= 4 ? chunk_bytes : chunk_bytes + 4;
+    tp.table_bytes = w_rows * row_table;
+  }
+  // (as many chunks as boxes: a chunk has a box at least, so that the chunk before in its place has been used up when the box before in its
+  // first box's place has)
+  const int chunk_slot = QK == kFloat ? 0 : (QK == kMx4 ? 1 : 2) * kBF * tp.table_pitch;
+  tp.w_stages = (P::kBudget - P::kFixed) / (P::kWBytes + chunk_slot);
+  if (tp.w_stages > P::kMostBoxes) tp.w_stages = P::kMostBoxes;
+  if (tp.w_stages < P::kLeastPlaces) return fail(QMM_ERR_UNSUPPORTED, "qmm_gemm_tc_kernel: the weight ring does not fit shared memory");
+  const size_t smem = P::kFixed + static_cast<size_t>(tp.w_stages) * (P::kWBytes + chunk_slot);
+  tp.w_inverse = 0xFFFFFFFFu / tp.w_stages + 1;
+
+  auto kernel = qmm_gemm_tc_kernel<QK, XT, BT>;
   static bool configured[kMaxDevices] = {};     // the attribute is per device
   const int dev = current_device();
   if (dev < 0) return QMM_ERR_DEVICE;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(qmm_gemm_tc_kernel<QK, XT, BT, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, P::kSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(qmm_gemm_tc_kernel<QK, XT, BT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               P::kSmem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::kBudget);
     if (e != cudaSuccess) return fail(QMM_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     configured[dev] = true;
   }
-  const int64_t ftiles = (p.N + kBF - 1) / kBF;
-  int64_t max_tiles = ragged ? ((p.M + BT - 1) / BT + p.batch) * ftiles
-                             : p.batch * ((p.M + BT - 1) / BT) * ftiles;
-  // Split products need float32 scratch for the partial tiles: the caller's static block
-  // (qmm_quantized_matmul_static) or a stream-ordered allocation that lives until the reduce
-  // kernel has run. No scratch, no split.
-  const int num_kb = static_cast<int>((p.K + kBK - 1) / kBK);
-  int splits = choose_splits(p, max_tiles, num_kb);
-  bool scratch_async = false;
-  if (splits > 1) {
-    const size_t need = static_cast<size_t>(splits) * p.M * p.N * sizeof(float);
-    const ScratchBlock* block = scratch_override();
+  const int sms = device_sm_count();
+  const int num_kb = static_cast<int>((p.K + kBK - 1) / kBK), boxes = (num_kb + P::kPer - 1) / P::kPer;
+  const int64_t ftiles = (p.N + kBF * P::kCtas - 1) / (kBF * P::kCtas), ttiles = (p.M + BT - 1) / BT;
+  const int64_t tiles = ragged ? (ttiles + p.batch) * ftiles : p.batch * ttiles * ftiles;      // (ragged: at most)
+  int64_t workers = sms / P::kCtas;
+  int64_t shared = 0, split = 1;
+  if (ragged) {
+    if (tiles < workers) workers = tiles;
+  } else if (tiles * 2 <= workers) {
+    // Few tiles: several workers share a tile's K, at least kLeastBoxes each. Where clusters of them (8 CTAs at most) fill half of the
+    // machine they add up over distributed shared memory: no scratch, one kernel, the sum spread over the cluster (64 rows of
+    // 4096 x 14336: 31.4 us with a second kernel, 21.9). Where they do not, more workers to a tile and a second kernel.
+    split = workers / tiles;
+    if (split > boxes / kLeastBoxes) split = boxes / kLeastBoxes;
+    if (split > most_shares(BT)) split = most_shares(BT);
+    if (split < 1) split = 1;
+    int64_t in_cluster = split < 8 / P::kCtas ? split : 8 / P::kCtas;
+    while (in_cluster > 1 && max_clusters(kernel, static_cast<int>(in_cluster) * P::kCtas, smem) < tiles) --in_cluster;
+    if (P::kMaySplit && in_cluster > 1 && tiles * in_cluster * 2 >= workers) {
+      split = in_cluster;
+      tp.cluster_adds = 1;
+    }
+    workers = tiles * split;
+  } else {
+    // Otherwise a tile each, in rounds; the last whole round and what is left over are shared out evenly by boxes, if that
+    // shortens it by more than the exchange of partial tiles takes.
+    const int64_t rest = tiles % workers, rounds = tiles / workers;
+    const int64_t region = rounds ? workers + rest : tiles;
+    if (rest && (rounds ? 2 : 1) * boxes - region * boxes / workers > exchange_blocks(BT) / P::kPer) shared = region;
+    if (!shared && tiles < workers) workers = tiles;
+  }
+  // Partial tiles: the caller's static block (qmm_quantized_matmul_static) or a stream-ordered allocation. No scratch,
+  // no sharing.
+  void* scratch = nullptr;
+  if (shared || (split > 1 && !tp.cluster_adds)) {
+    const size_t per_worker = P::kCtas * (static_cast<size_t>(BT) * kBF * sizeof(float) + (shared ? kDequantWarps * sizeof(unsigned long long) : 0));
     if (block) {
+      // (a call is refused when the partial results of its K shares as whole float32 matrices exceed the block)
+      const int64_t old_tiles = ttiles * ((p.N + kBF - 1) / kBF);
+      int64_t s = p.batch != 1 || (p.N & 3) ? 1 : sms / old_tiles;
+      if (s > num_kb / 8) s = num_kb / 8;
+      if (s > 8) s = 8;
+      const size_t need = static_cast<size_t>(s < 2 ? 0 : s) * p.M * p.N * sizeof(float);
       if (need > block->bytes)
-        return fail(QMM_ERR_TOO_LARGE, "split product needs %zu bytes of scratch, the static block has %zu", need,
-                    block->bytes);
-      tp.partial = static_cast<float*>(block->ptr);
+        return fail(QMM_ERR_TOO_LARGE, "split product needs %zu bytes of scratch, the static block has %zu", need, block->bytes);
+      if (split > 1)
+        while (split > 1 && per_worker * tiles * split > block->bytes) --split;
+      if (split > 1) workers = tiles * split;
+      if (per_worker * workers <= block->bytes) tp.partial = static_cast<float*>(block->ptr);
     } else {
-      tp.partial = static_cast<float*>(scratch_alloc(need, stream));
-      scratch_async = tp.partial != nullptr;
-      if (!scratch_async) splits = 1;
+      tp.partial = static_cast<float*>(scratch = scratch_alloc(per_worker * workers, stream));
+    }
+    if (!tp.partial || (!shared && split == 1)) {
+      shared = 0;
+      split = 1;
+      if (tiles < workers) workers = tiles;
     }
   }
-  tp.splits = splits;
-  int64_t items = max_tiles * splits;
-  int grid = sm_count();
-  if (items < grid) grid = static_cast<int>(items < 1 ? 1 : items);
-  // More tiles than SMs and a last wave that does not fill them: the full waves run unsplit, and
-  // the leftover tiles' K blocks are divided among the SMs (compact float32 partial tiles, a small
-  // reduce) instead of some CTAs walking all of K while the rest idle.
-  if (splits == 1 && !ragged && p.batch == 1 && max_tiles > grid && tail_split_enabled()) {
-    const int64_t rem = max_tiles % grid;
-    // (only a last wave that fills under half of the SMs: dividing a fuller one was measured and
-    // lost more to the short K shares' pipeline fill than the idle SMs cost)
-    int64_t s = rem ? grid / rem : 0;
-    if (s > num_kb / 8) s = num_kb / 8;
-    if (s > 8) s = 8;
-    if (rem > 0 && s >= 2) {
-      const size_t need = static_cast<size_t>(s) * rem * BT * kBF * sizeof(float);
-      const ScratchBlock* block = scratch_override();
-      float* part = nullptr;
-      bool part_async = false;
-      if (block) {
-        if (need <= block->bytes) part = static_cast<float*>(block->ptr);
-      } else {
-        part = static_cast<float*>(scratch_alloc(need, stream));
-        part_async = part != nullptr;
-      }
-      if (part) {
-        TcParams head = tp, tail = tp;
-        head.item_end = max_tiles - rem;
-        launch_dependent(qmm_gemm_tc_kernel<QK, XT, BT, false>, grid, P::kThreads, P::kSmem, stream, xm, wm, head);
-        tail.splits = static_cast<int>(s);
-        tail.partial = part;
-        tail.tail_tile0 = max_tiles - rem;
-        tail.tail_tiles = rem;
-        tail.item0 = (max_tiles - rem) * s;
-        tail.item_end = max_tiles * s;
-        const int64_t tail_grid = rem * s < grid ? rem * s : grid;
-        launch_dependent(qmm_gemm_tc_kernel<QK, XT, BT, true>, static_cast<unsigned>(tail_grid), P::kThreads, P::kSmem, stream, xm, wm, tail);
-        const int64_t total = rem * BT * kBF;
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
-        launch_dependent(splitk_tail_reduce_kernel, static_cast<unsigned>(blocks), 256, 0, stream, part, p.y, p.y_dtype, p.M, p.N,
-                         ftiles, max_tiles - rem, rem, BT, static_cast<int>(s));
-        count_launch(3);
-        if (part_async) scratch_free(part, stream);
-        return check_launch("qmm_gemm_tc_kernel");
-      }
-    }
+  tp.split = static_cast<int>(split);
+  if (shared) {
+    tp.ready = reinterpret_cast<unsigned long long*>(tp.partial + static_cast<int64_t>(P::kCtas) * workers * BT * kBF);
+    tp.epoch = next_epoch();
+    tp.shared_tiles = static_cast<int>(shared);
+    tp.share = static_cast<unsigned>(shared * boxes / workers);
+    tp.share_more = static_cast<unsigned>(shared * boxes % workers);
   }
-  if (splits > 1) launch_dependent(qmm_gemm_tc_kernel<QK, XT, BT, true>, grid, P::kThreads, P::kSmem, stream, xm, wm, tp);
-  else launch_dependent(qmm_gemm_tc_kernel<QK, XT, BT, false>, grid, P::kThreads, P::kSmem, stream, xm, wm, tp);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(workers * P::kCtas));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  const int cluster = P::kCtas * (tp.cluster_adds ? tp.split : 1);
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, kernel, xm, wm, tp);      // a failure stays as the last error: check_launch reports it
   count_launch();
-  if (splits > 1) {
-    const int64_t total = p.M * p.N;
-    int64_t blocks = (total / 4 + 255) / 256;
-    if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
-    launch_dependent(splitk_reduce_kernel, static_cast<unsigned>(blocks), 256, 0, stream, tp.partial, p.y, p.y_dtype, total, splits);
+  if (split > 1 && !tp.cluster_adds) {
+    const int64_t rows = p.M * p.batch, warps = rows * ftiles * P::kCtas;
+    const int64_t most = static_cast<int64_t>(sms) * 8;
+    launch_early(add_partials_kernel<BT>, static_cast<unsigned>((warps + 7) / 8 < most ? (warps + 7) / 8 : most), 256, 0, stream,
+                 tp.partial, tp, P::kCtas, ttiles, ftiles);
     count_launch();
-    if (scratch_async) scratch_free(tp.partial, stream);
   }
-#if QMM_TC_TRACING
-  if (trace_on) {   // development aid: average cycles per wait site over the CTAs
-    cudaStreamSynchronize(stream);
-    static long long host[16 * 1024];
-    cudaMemcpy(host, trace_buf, sizeof(long long) * 16 * grid, cudaMemcpyDeviceToHost);
-    double avg[16] = {0};
-    for (int c = 0; c < grid; ++c)
-      for (int i = 0; i < 16; ++i) avg[i] += static_cast<double>(host[c * 16 + i]) / grid;
-    fprintf(stderr, "qmm_gemm_tc CTA lifetime %.0f cycles, %.1f us -> %.0f MHz\n", avg[14], avg[15] / 1e3,
-            avg[14] / (avg[15] / 1e3));
-    fprintf(stderr, "qmm_gemm_tc cycles/CTA: producer.empty %.0f | mma.issue %.0f mma.d_empty %.0f mma.fence %.0f mma.a_full %.0f |"
-            " dequant.st %.0f dequant.full %.0f dequant.a_empty %.0f dequant.d_full %.0f\n",
-            avg[1], avg[8], avg[8 + 2], avg[8 + 3], avg[8 + 4], avg[0], avg[5], avg[6], avg[7]);
-  }
-#endif
+  if (scratch) scratch_free(scratch, stream);
   return check_launch("qmm_gemm_tc_kernel");
 }
 
@@ -1071,10 +1191,12 @@ bool gemm_tc_supports(const qmm_problem& p) {
   if (p.x_dtype != QMM_BF16 && p.x_dtype != QMM_F16) return false;
   if (p.lhs_idx || p.rhs_idx) return false;                   // unsorted gathers go elsewhere
   if (p.batch > kMaxSegments) return false;
-  if (p.K < kBK || p.K % (p.mode == QMM_MODE_FLOAT ? 8 : 32)) return false;
+  if (p.K < kBK || p.K % (p.mode == QMM_MODE_FLOAT ? 8 : 32) || p.K >= (1LL << 30)) return false;
   if ((p.K * 2) % 16) return false;
   if (!p.group_sizes && p.batch > 1 && p.x_batch_stride != p.M * p.K) return false;
   if (!p.group_sizes && p.batch > 1 && p.y_batch_stride != p.M * p.N) return false;
+  // (tiles are counted in 32 bits)
+  if (((p.M + 63) / 64 + p.batch) * (p.group_sizes ? 1 : p.batch) * ((p.N + 127) / 128) * ((p.K + 63) / 64) >= (1LL << 31)) return false;
   if (p.M * (p.group_sizes ? 1 : p.batch) >= (1LL << 31) || p.N * p.batch >= (1LL << 31)) return false;
   return true;
 }
