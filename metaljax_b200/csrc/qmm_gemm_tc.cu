@@ -34,10 +34,12 @@
 // the first that it makes, and waits only on lower-numbered workers, which were scheduled before it.
 //
 // Measured (device time, before: one CTA per tile at every width, 32-byte boxes, tables from global memory, an issuer behind a branch, split
-// products added up by a second kernel), int4 group 64: 2048 rows 14336 x 4096 248 -> 202 us, 4096 x 14336 219 -> 178; 512 rows 28672 x 4096
-// 130 -> 102; 64 rows 28672 x 4096 59.7 -> 41.6, 4096 x 4096 16.4 -> 11.6, 4096 x 14336 31.2 -> 21.7; 128 rows 4096 x 14336 47 -> 24.6; 8-bit
-// group 128, 45 rows 14336 x 4096 33 -> 24. What bounds it: at 64 rows the dequantizing warps (about 300 clocks a K block and SM), at 256 the tensor
-// cores' 514 clocks a block plus what the dequantization does not keep up with, under the power cap.
+// products added up by a second kernel), int4 group 64: 2048 rows 14336 x 4096 248 -> 189 us, 4096 x 14336 219 -> 174; 512 rows 28672 x 4096
+// 130 -> 100; 64 rows 28672 x 4096 59.7 -> 37.8, 4096 x 4096 16.4 -> 10.8, 4096 x 14336 31.2 -> 20.9; 128 rows 4096 x 14336 47 -> 22; 8-bit
+// group 128, 45 rows 14336 x 4096 33 -> 25. What bounds it: at 64 rows the dequantizing warps (400 clocks a K block and SM: some 300 instructions a
+// warp and block at four warps a scheduler), at 256 the tensor cores (500 clocks a block between a tile's ends, under the power cap) and the ends,
+// where the accumulator is drained by the warps that would dequantize for the next tile. (Draining it after the first steps of the next
+// tile was built: the state that lives across the epilogue then spills, and every size lost.)
 //
 // Every wait is bounded: when a barrier does not flip within ~2 s of SM clock the kernel
 // records the place in a status word, stops issuing work and drains.
@@ -272,24 +274,33 @@ struct Half2Ops<__half> {
   }
 };
 
+// (a & mask) | bits in one LOP3: with both constants known the compiler makes two of it, an immediate each.
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(mask), "r"(bits));
+  return d;
+}
+__device__ __forceinline__ uint32_t in_register(uint32_t v) {
+  asm volatile("" : "+r"(v));
+  return v;
+}
+
 // 4-bit affine, NW packed words -> NW*4 pairs. A byte holds elements (2i, 2i+1): PRMT takes
 // it from the word (even element in its low nibble) into byte 0 and from the word shifted
 // right by four (odd element) into byte 2, one LOP3 keeps the two nibbles under the magic
 // exponent (128 + q, or 1024 + q for f16, both exact), an exact subtraction removes the
 // magic, and one FMA with (s, s), (b, b) rounds once.
 template <typename XT, int NW>
-__device__ __forceinline__ void dequant_aff4(const uint32_t (&w)[NW], float s, float b, uint32_t* out) {
+__device__ __forceinline__ void dequant_aff4(const uint32_t (&w)[NW], uint32_t s2, uint32_t b2, uint32_t mask, uint32_t magic, uint32_t* out) {
   using H = Half2Ops<XT>;
-  const uint32_t s2 = H::pack(s, s);
-  const uint32_t b2 = H::pack(b, b);
 #pragma unroll
   for (int j = 0; j < NW; ++j) {
     const uint32_t hi = w[j] >> 4;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint32_t t = __byte_perm(w[j], hi, i | ((4 + i) << 8));
-      const uint32_t v = (t & 0x000F000Fu) | H::kMagic;
-      out[j * 4 + i] = H::fma(H::sub(v, H::kMagic), s2, b2);
+      const uint32_t v = and_or(t, mask, magic);
+      out[j * 4 + i] = H::fma(H::sub(v, magic), s2, b2);
     }
   }
 }
@@ -484,7 +495,8 @@ struct Walk {
   }
 };
 
-template <int QK, typename XT, int BT>
+// SAME: the tables are of the activation type (the pairs for the arithmetic are the entries themselves).
+template <int QK, typename XT, int BT, bool SAME>
 __global__ void __launch_bounds__(kThreads, 1)
 qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const TcParams p) {
   using P = Plan<QK, BT>;
@@ -683,7 +695,10 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
     const int frow = quarter * 32 + lane;        // feature row within the CTA's tile
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const int groups = QK == kFloat ? 1 : p.K >> p.group_shift;
-    const bool twide = p.table_dtype == QMM_F32;
+    const bool twide = !SAME && p.table_dtype == QMM_F32;
+    const int entry = QK == kMx4 ? 1 : SAME ? 2 : p.table_entry;
+    [[maybe_unused]] const uint32_t mask = in_register(0x000F000Fu), magic = in_register(Half2Ops<XT>::kMagic);
+    const uint32_t bias_off = kBF * p.table_pitch, swizzle = (frow & 7) << 4;
     const uint32_t a_bar = kPair ? in_cta(a_full, leader) : a_full, d_bar = kPair ? in_cta(d_empty, leader) : d_empty;
     const uint32_t wthread = w_at + frow * kBoxBytes;
     uint32_t wbase = 0, sbase = 0, cbase = 0, piece = 0;    // boxes, steps and table chunks before this piece
@@ -695,64 +710,76 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
       const uint32_t trow = static_cast<uint32_t>(pc.seg * p.w_seg_rows + feat) * static_cast<uint32_t>(groups);   // row of the tables (its low bits count)
       const int nkb = pc.kb_hi - pc.kb_lo, steps = (nkb + kStep - 1) / kStep;
       constexpr int kHalfBytes = P::kRowBytes / 2;                 // packed bytes of a half block
+      // where the team's next step is in the rings: slot, box (and how often round)
+      uint32_t s = (sbase + team) % kStages, ph = (sbase + team) / kStages & 1u;
+      uint32_t wi = wbase + team * kStep / kPer, wph = __umulhi(wi, p.w_inverse), ws = wi - wph * p.w_stages;
       for (int i = team; i < steps; i += kTeams) {
         const int j = i * kStep;                   // first K block of the step
-        const int halves = j + kStep <= nkb ? 2 * kStep : 2 * (nkb - j);
-        const uint32_t si = sbase + i, s = si % kStages, ph = (si / kStages) & 1u;
         if (!(ok = wait(empty + 8 * s, ph ^ 1u, 7))) break;
-        uint32_t wi = wbase + j / kPer, wround = __umulhi(wi, p.w_inverse), ws = wi - wround * p.w_stages;
-        if (!(ok = wait(wfull + 8 * ws, wround & 1u, 6))) break;
+        if (!(ok = wait(wfull + 8 * ws, wph & 1u, 6))) break;
         __syncwarp();
         tc_fence_after();
         // This row's entries of the chunk: where the first is, and which is the last of the whole row
-        const int box = (pc.kb_lo + j) / kPer, chunk = box >> p.chunk_shift;
-        const int g0 = ((chunk << p.chunk_shift) * (kPer * kBK)) >> p.group_shift, glast = groups - 1 - g0;
-        const int k0 = (pc.kb_lo + j) * kBK - (chunk << p.chunk_shift) * (kPer * kBK);      // the step's first element in the chunk
+        const int chunk = (pc.kb_lo + j) / kPer >> p.chunk_shift, chunk_k = (chunk << p.chunk_shift) * (kPer * kBK);
+        const int g0 = chunk_k >> p.group_shift, glast = groups - 1 - g0;
+        const int k0 = (pc.kb_lo + j) * kBK - chunk_k;                 // the step's first element in the chunk
         const uint32_t ci = cbase + chunk - (pc.kb_lo / kPer >> p.chunk_shift), ts = ci - __umulhi(ci, p.w_inverse) * p.w_stages;
-        const uint32_t tbox = t_at + ts * (kTables * kBF * p.table_pitch) + frow * p.table_pitch + (p.table_unit < 4 ? ((trow + g0) * p.table_entry & 3u) : 0u);
-        auto half = [&](int q) {
-          // 16-byte chunk c of row r sits at chunk c ^ (r & 7) (the TMA unit's 128-byte swizzle): eight lanes read distinct banks
-          const uint32_t wrow = wthread + ws * P::kWBytes;
-          const int in_box = ((j % kPer) * 2 + q) % (2 * kPer);    // which 32 elements of the box
-          uint32_t packed[kHalfBytes / 4], out[16];
-#pragma unroll
-          for (int c = 0; c < kHalfBytes / 16; ++c) {
-            const uint4 v = lds128<0>(wrow + (((in_box * (kHalfBytes / 16) + c) ^ (frow & 7)) << 4));
-            packed[c * 4] = v.x; packed[c * 4 + 1] = v.y; packed[c * 4 + 2] = v.z; packed[c * 4 + 3] = v.w;
-          }
-          if constexpr (QK == kFloat) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) out[e] = packed[e];
-          } else {
-            const int g = min((k0 + q * 32) >> p.group_shift, glast);
-            const uint32_t at = tbox + g * p.table_entry, bias_at = at + kBF * p.table_pitch;
-            if constexpr (QK == kMx4) {
-              dequant_mx4<XT>(packed, lds8(at), out);
-            } else {
-              const float fs = twide ? __uint_as_float(lds32<0>(at)) : table_value(lds16(at), p.table_dtype);
-              const float fb = twide ? __uint_as_float(lds32<0>(bias_at)) : table_value(lds16(bias_at), p.table_dtype);
-              if constexpr (QK == kAff8) dequant_aff8<XT>(packed, fs, fb, out);
-              else if (twide) dequant_aff4_wide<XT>(packed, fs, fb, out);
-              else dequant_aff4<XT>(packed, fs, fb, out);
-            }
-          }
-          tmem_st16(tmem_base + lane_addr + P::kACol0 + s * (32 * kStep) + q * 16, out);
-        };
+        const uint32_t tbox = t_at + ts * (kTables * kBF * p.table_pitch) + frow * p.table_pitch + (p.table_unit < 4 ? ((trow + g0) * entry & 3u) : 0u);
         // (a block at a time, not the whole step unrolled: the sixteen warps are at sixteen places of this code, and much more of it
         // no longer stays in the instruction caches)
+        const int blocks = nkb - j < kStep ? nkb - j : kStep;
 #pragma unroll 1
-        for (int q = 0; q < halves; q += 2) {
-          if (kPer == 1 && q == 2) {               // (float weights: a box is one block)
+        for (int b = 0; b < blocks; ++b) {
+          if (kPer == 1 && b == 1) {               // (float weights: a box is one block)
             __syncwarp();
             if (lane == 0) arrive_n(wempty + 8 * ws, 1);
-            ++wi;
-            wround = __umulhi(wi, p.w_inverse);
-            ws = wi - wround * p.w_stages;
-            if (!(ok = wait(wfull + 8 * ws, wround & 1u, 6))) break;
+            if (++ws == static_cast<uint32_t>(p.w_stages)) { ws = 0; ++wph; }
+            if (!(ok = wait(wfull + 8 * ws, wph & 1u, 6))) break;
             __syncwarp();
           }
-          half(q);
-          half(q + 1);
+          // 16-byte chunk c of row r sits at chunk c ^ (r & 7) (the TMA unit's 128-byte swizzle): eight lanes read distinct banks
+          const uint32_t first = wthread + ws * P::kWBytes + (static_cast<uint32_t>((j + b) % kPer * P::kRowBytes) ^ swizzle);
+          uint32_t sc = 0u, bi = 0u;               // the half block's table entries
+          auto entries = [&](int k) {
+            const uint32_t at = tbox + min(k >> p.group_shift, glast) * entry;
+            if constexpr (QK == kMx4) {
+              sc = lds8(at);
+            } else if (twide) {
+              sc = lds32<0>(at);
+              bi = lds32<0>(at + bias_off);
+            } else {
+              sc = lds16(at);
+              bi = lds16(at + bias_off);
+            }
+          };
+          if constexpr (QK != kFloat) entries(k0 + b * kBK);
+#pragma unroll(QK == kAff8 ? 1 : 2)
+          for (int h = 0; h < 2; ++h) {
+            uint32_t packed[kHalfBytes / 4], out[16];
+#pragma unroll
+            for (int c = 0; c < kHalfBytes / 16; ++c) {
+              const uint4 v = lds128<0>(first ^ ((h * (kHalfBytes / 16) + c) << 4));
+              packed[c * 4] = v.x; packed[c * 4 + 1] = v.y; packed[c * 4 + 2] = v.z; packed[c * 4 + 3] = v.w;
+            }
+            if constexpr (QK != kFloat)
+              if (h == 1 && p.group_shift == 5) entries(k0 + b * kBK + 32);
+            if constexpr (QK == kFloat) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) out[e] = packed[e];
+            } else if constexpr (QK == kMx4) {
+              dequant_mx4<XT>(packed, sc, out);
+            } else if constexpr (QK == kAff4 && SAME) {
+              dequant_aff4<XT>(packed, __byte_perm(sc, sc, 0x1010), __byte_perm(bi, bi, 0x1010), mask, magic, out);
+            } else {
+              const int td = SAME ? (std::is_same<XT, __nv_bfloat16>::value ? QMM_BF16 : QMM_F16) : p.table_dtype;
+              const float fs = twide ? __uint_as_float(sc) : table_value(sc, td);
+              const float fb = twide ? __uint_as_float(bi) : table_value(bi, td);
+              if constexpr (QK == kAff8) dequant_aff8<XT>(packed, fs, fb, out);
+              else if (twide) dequant_aff4_wide<XT>(packed, fs, fb, out);
+              else dequant_aff4<XT>(packed, Half2Ops<XT>::pack(fs, fs), Half2Ops<XT>::pack(fb, fb), mask, magic, out);
+            }
+            tmem_st16(tmem_base + lane_addr + P::kACol0 + s * (32 * kStep) + b * 32 + h * 16, out);
+          }
         }
         if (!ok) break;
         __syncwarp();
@@ -768,6 +795,10 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
           if constexpr (kPair) remote_arrive_n(a_bar + 8 * s, 1);
           else arrive_n(a_bar + 8 * s, 1);
         }
+        s += kTeams;
+        if (s >= static_cast<uint32_t>(kStages)) { s -= kStages; ph ^= 1u; }
+        ws += kPer == 1 ? kTeams * kStep - (kStep - 1) : kTeams * kStep / kPer;
+        while (ws >= static_cast<uint32_t>(p.w_stages)) { ws -= p.w_stages; ++wph; }
       }
       wbase += static_cast<uint32_t>(nkb + kPer - 1) / kPer;
       sbase += static_cast<uint32_t>(nkb + kStep - 1) / kStep;
@@ -1017,8 +1048,8 @@ int64_t max_clusters(Kernel kernel, int ctas, size_t smem) {
   return have;
 }
 
-template <int QK, typename XT, int BT>
-int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
+template <int QK, typename XT, int BT, bool SAME>
+int launch_tables(const qmm_problem& p, cudaStream_t stream) {
   using P = Plan<QK, BT>;
   const bool ragged = p.group_sizes != nullptr;
   const int64_t x_rows = ragged ? p.M : p.batch * p.M;
@@ -1067,7 +1098,7 @@ int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
   const size_t smem = P::kFixed + static_cast<size_t>(tp.w_stages) * (P::kWBytes + chunk_slot);
   tp.w_inverse = 0xFFFFFFFFu / tp.w_stages + 1;
 
-  auto kernel = qmm_gemm_tc_kernel<QK, XT, BT>;
+  auto kernel = qmm_gemm_tc_kernel<QK, XT, BT, SAME>;
   static bool configured[kMaxDevices] = {};     // the attribute is per device
   const int dev = current_device();
   if (dev < 0) return QMM_ERR_DEVICE;
@@ -1167,6 +1198,13 @@ int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
   }
   if (scratch) scratch_free(scratch, stream);
   return check_launch("qmm_gemm_tc_kernel");
+}
+
+template <int QK, typename XT, int BT>
+int launch_cfg(const qmm_problem& p, cudaStream_t stream) {
+  if constexpr (QK == kAff4 || QK == kAff8)
+    if (p.table_dtype != (std::is_same<XT, __nv_bfloat16>::value ? QMM_BF16 : QMM_F16)) return launch_tables<QK, XT, BT, false>(p, stream);
+  return launch_tables<QK, XT, BT, true>(p, stream);
 }
 
 template <int QK, typename XT>
