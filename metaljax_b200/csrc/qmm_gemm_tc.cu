@@ -426,6 +426,7 @@ struct Plan {
   static_assert(kStages >= kTeams, "");
   static_assert(kACol0 + kStages * kStep * 32 <= 512, "the A ring fits tensor memory");
   static_assert(kFixed + kLeastPlaces * kWBytes <= kBudget, "");
+  static_assert(kTeams * kStep % kPer == 0, "a team's next step lies whole boxes ahead");
   static_assert((2 * kMostBoxes + 3 * kStages + 2) * 8 + 16 <= kBarBytes, "");
 };
 

@@ -430,7 +430,7 @@ class State:
     """Per-program recognizer state: matches, the skip set, root dispatch and the flat
     list of packed arrays `emit` reads by slot."""
 
-    __slots__ = ("matches", "skip", "roots", "values", "active", "moe", "fn", "floats")
+    __slots__ = ("matches", "skip", "roots", "values", "active", "moe", "fn", "floats", "plan")
 
     def __init__(self):
         self.matches = []
@@ -441,6 +441,7 @@ class State:
         self.roots = {}
         self.values = []
         self.active = False
+        self.plan = None
 
     def rebuild(self):
         live = [m for m in self.matches if not m.disabled]
@@ -455,6 +456,7 @@ class State:
             skip.update(g.skip_keys)
         self.skip = frozenset(skip)
         self.active = bool(self.roots)
+        self.plan = None             # (the interpreter's list of what is left to run)
 
 
 def build_pack(m: Match, codes, scale_map, zero_map=None, leaves=()) -> _Pack:
@@ -857,7 +859,8 @@ def emit(interp, m, env):
     x = env[m.lhs]
     if m.lperm is not None and list(m.lperm) != list(range(x.dim())):
         x = x.permute(*m.lperm)
-    x = x.reshape([m.B, m.M, m.K] if m.bshape else [m.M, m.K])
+    if m.bshape or x.dim() != 2:     # (a reshape or a list costs the host a microsecond: none where the shape is right already)
+        x = x.reshape([m.B, m.M, m.K] if m.bshape else [m.M, m.K])
     if x.dtype not in _FLOATS:
         x = x.to(m.out_dtype)
     if m.has_perm:
@@ -867,6 +870,6 @@ def emit(interp, m, env):
                          bits=m.bits, mode=m.mode, out_dtype=m.out_dtype)
     if m.swapped:
         y = y.transpose(-1, -2).reshape(list(m.bshape) + list(m.nshape) + list(m.mshape))
-    else:
+    elif m.bshape or len(m.mshape) != 1 or len(m.nshape) != 1:
         y = y.reshape(list(m.bshape) + list(m.mshape) + list(m.nshape))
     return [y]
