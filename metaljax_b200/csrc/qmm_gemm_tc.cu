@@ -820,6 +820,14 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
         }
         break;
       }
+      auto drained = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (kPair) remote_arrive_n(d_bar, 1);
+          else arrive_n(d_bar, 1);
+        }
+      };
       const bool mine = team * 32 < pc.rows;
       const bool whole = pc.begins && pc.ends, part_only = !pc.ends || p.split > 1;
       if (mine && !part_only && !whole) {          // the tile's earlier pieces, made by the workers before this one
@@ -866,6 +874,7 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
         uint32_t r[32];
         tmem_ld32(tmem_base + lane_addr + c0, r);
         tmem_wait_ld();
+        if (c0 + 32 * kTeams >= pc.rows) drained();      // this warp's last columns: the next tile's MMAs need not wait for the stores
         if (part_only) {
           float* part = p.partial + static_cast<int64_t>(blockIdx.x) * (BT * kBF) + in_partial;
 #pragma unroll
@@ -890,12 +899,7 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if constexpr (kPair) remote_arrive_n(d_bar, 1);
-        else arrive_n(d_bar, 1);
-      }
+      if (!mine) drained();
       if (p.split > 1) break;
       if (mine && part_only) {                     // this warp's part of the partial tile is there
         if (lane == 0) {

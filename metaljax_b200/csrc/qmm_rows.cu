@@ -124,7 +124,7 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
   const int slices = (rp.K + kSliceK - 1) / kSliceK;
   // Rows of a chunk: what the registers take. Nine to sixteen rows are two chunks: the CTAs that work on either half pass over
   // the weight side by side, so that the second reads it from L2 (16 rows of 4096 x 4096: 9.2 us; as one chunk of 16, half of whose activations
-  // live in shared memory, 14.2; 14336 x 4096 25.0 against 30.5 on the tensor cores, 8-bit 14336 x 4096 31 against 51).
+  // live in shared memory, 14.2).
   const int chunk = p.x_dtype == QMM_F32 ? 4 : 8;
   const int64_t per_seg = p.group_sizes ? (p.M + p.batch - 1) / p.batch : p.M;      // grouped: of an average expert
   const int64_t live = p.group_sizes ? (p.batch < p.M ? p.batch : p.M) : p.batch;
