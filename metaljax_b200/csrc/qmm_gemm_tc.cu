@@ -280,27 +280,51 @@ __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t b
   asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(mask), "r"(bits));
   return d;
 }
+// Bytes of {a, b}; a selector of 8 + i is byte i's sign, eight times (which __byte_perm does not pass on).
+__device__ __forceinline__ uint32_t permute(uint32_t a, uint32_t b, uint32_t selector) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(selector));
+  return d;
+}
 __device__ __forceinline__ uint32_t in_register(uint32_t v) {
   asm volatile("" : "+r"(v));
   return v;
 }
 
-// 4-bit affine, NW packed words -> NW*4 pairs. A byte holds elements (2i, 2i+1): PRMT takes
-// it from the word (even element in its low nibble) into byte 0 and from the word shifted
-// right by four (odd element) into byte 2, one LOP3 keeps the two nibbles under the magic
-// exponent (128 + q, or 1024 + q for f16, both exact), an exact subtraction removes the
-// magic, and one FMA with (s, s), (b, b) rounds once.
+// 4-bit affine, NW packed words -> NW*4 pairs; s2, b2 are scale and bias as pairs of the type.
+//
+// bf16: the even and the odd nibbles of a word under a byte mask each; PRMT takes byte i of either into bytes 0 and 2 of a
+// pair and zeros (their signs) into 1 and 3. A code in the low bits is the subnormal q 2^-133: a product with 2^127 makes it the
+// exact q / 64, and one FMA with (64 s, 64 s), (b, b) rounds once. (Scales below 2^121.) 15 instructions a word, 7 of them on the
+// half-rate logic pipe; with a magic exponent per pair they were 17 and 9.
+//
+// f16 has no factor for that: there PRMT takes a byte from the word (even element in its low nibble) into byte 0 and from
+// the word shifted right by four into byte 2, one LOP3 keeps the two nibbles under the magic exponent (1024 + q, exact),
+// an exact subtraction removes the magic, and the FMA rounds once.
 template <typename XT, int NW>
 __device__ __forceinline__ void dequant_aff4(const uint32_t (&w)[NW], uint32_t s2, uint32_t b2, uint32_t mask, uint32_t magic, uint32_t* out) {
   using H = Half2Ops<XT>;
+  if constexpr (std::is_same<XT, __nv_bfloat16>::value) {
+    const uint32_t s64 = H::mul(s2, 0x42804280u);
 #pragma unroll
-  for (int j = 0; j < NW; ++j) {
-    const uint32_t hi = w[j] >> 4;
+    for (int j = 0; j < NW; ++j) {
+      const uint32_t even = w[j] & 0x0F0F0F0Fu, odd = (w[j] >> 4) & 0x0F0F0F0Fu;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t t = __byte_perm(w[j], hi, i | ((4 + i) << 8));
-      const uint32_t v = and_or(t, mask, magic);
-      out[j * 4 + i] = H::fma(H::sub(v, magic), s2, b2);
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t q = permute(even, odd, i | ((8 + i) << 4) | ((4 + i) << 8) | ((12 + i) << 12));
+        out[j * 4 + i] = H::fma(H::mul(q, 0x7F007F00u), s64, b2);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NW; ++j) {
+      const uint32_t hi = w[j] >> 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t t = __byte_perm(w[j], hi, i | ((4 + i) << 8));
+        const uint32_t v = and_or(t, mask, magic);
+        out[j * 4 + i] = H::fma(H::sub(v, magic), s2, b2);
+      }
     }
   }
 }
@@ -1020,9 +1044,10 @@ unsigned long long next_epoch() {
 constexpr int kLeastBoxes = 2;
 // (More of them of wide tiles write and read more partial sums than they save.)
 constexpr int most_shares(int bt) { return bt >= 256 ? 8 : 16; }
-// What handing partial tiles from worker to worker takes, in K blocks (512 rows mxfp4 5760 x 2880, 46 tiles of 45 blocks on 74 pairs: 30 us shared
-// out, 26 a tile each).
-constexpr int exchange_blocks(int bt) { return bt >= 256 ? 32 : 12; }
+// What handing partial tiles from worker to worker takes, in K blocks (us, shared out / a tile each: 64 rows 14336 x 4096, 112 tiles of 64
+// blocks on 148 workers, 23.4 / 20.3; 64 rows 28672 x 4096 37.5 / 35.6; 512 rows mxfp4 5760 x 2880, 46 of 45 on 74 pairs, 30 / 24; 512 rows 28672 x 4096,
+// which it shortens by a third of a round more than that, 99.7 / 105.8).
+constexpr int kExchangeBlocks = 32;
 
 // Clusters of `ctas` that fit the device at once. Asked once per kernel and size (with the first call's shared memory: all but all of it
 // either way, one CTA per SM).
@@ -1140,7 +1165,7 @@ int launch_tables(const qmm_problem& p, cudaStream_t stream) {
     // shortens it by more than the exchange of partial tiles takes.
     const int64_t rest = tiles % workers, rounds = tiles / workers;
     const int64_t region = rounds ? workers + rest : tiles;
-    if (rest && (rounds ? 2 : 1) * boxes - region * boxes / workers > exchange_blocks(BT) / P::kPer) shared = region;
+    if (rest && (rounds ? 2 : 1) * boxes - region * boxes / workers > kExchangeBlocks / P::kPer) shared = region;
     if (!shared && tiles < workers) workers = tiles;
   }
   // Partial tiles: the caller's static block (qmm_quantized_matmul_static) or a stream-ordered allocation. No scratch,
