@@ -898,14 +898,19 @@ class Interpreter:
         return [env[v] for v in fn.returns]
 
     def _plan(self, st):
+        taken = st.skip | set(st.roots)
+        gates = {id(op): found for op in self.func.ops if id(op) not in taken and (found := _gate(op, taken)) is not None}
+        inside = {id(op) for _, ops in gates.values() for op in ops}
         plan = []
         for op in self.func.ops:
             key = id(op)
             root = st.roots.get(key)
             if root is not None:
                 plan.append((self._fused(root), op, (), op.results))
-            elif key in st.skip:
+            elif key in st.skip or key in inside:
                 continue
+            elif key in gates:
+                plan.append((_run_gate, op, gates[key][0], op.results))
             elif op.name in hlo.EVAL and not op.opaque:
                 fn = hlo.EVAL[op.name]
                 plan.append((lambda op, env, *ins, fn=fn: (fn(op, *ins),), op, op.operands, op.results))
@@ -934,6 +939,32 @@ class Interpreter:
             return id(op) in st.skip
 
         return hook
+
+
+def _gate(op, taken):
+    """`(g * logistic(g)) * u` with both inner values used nowhere else, at the last product: ((g, u), the two inner ops).
+    The multiplications may have either order. None where it is something else."""
+    if op.name != "stablehlo.multiply" or op.results[0].type.dtype not in (torch.bfloat16, torch.float16):
+        return None
+    for a, u in (op.operands, op.operands[::-1]):
+        silu = a.op
+        if silu is None or silu.name != "stablehlo.multiply" or id(silu) in taken or len(a.uses) != 1:
+            continue
+        for g, s in (silu.operands, silu.operands[::-1]):
+            sig = s.op
+            if sig is not None and sig.name == "stablehlo.logistic" and id(sig) not in taken and len(s.uses) == 1 and sig.operands[0] is g:
+                return (g, u), (sig, silu)
+    return None
+
+
+def _run_gate(op, env, g, u):
+    # One pass and two roundings instead of three of each. Feed-forward of 4096 x 11264: 64 rows 94.6 -> 79.2 us, 512 rows
+    # 186.8 -> 174.8; 4 rows of 2048 x 5632 44.0 -> 42.3, within that case's noise (the host's launches bound it). The
+    # kernel reads 16 bytes at a time: element counts and addresses that are not multiples of that run as the program says.
+    if g.is_cuda and g.is_contiguous() and u.is_contiguous() and not g.numel() % 8 and not (g.data_ptr() | u.data_ptr()) % 16:
+        from . import moe
+        return (moe.silu_mul(g, u),)
+    return (g * torch.sigmoid(g) * u,)
 
 
 class _Single:
