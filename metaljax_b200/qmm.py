@@ -881,7 +881,9 @@ def emit(interp, m, env):
     x = env[m.lhs]
     if m.lperm is not None and list(m.lperm) != list(range(x.dim())):
         x = x.permute(*m.lperm)
-    if m.bshape or x.dim() != 2:     # (a reshape or a list costs the host a microsecond: none where the shape is right already)
+    # (A reshape or a list costs the host a microsecond: none where the shape is right already. Two dimensions alone are
+    # not [M, K]: both may be contracted, [heads, head_dim] against [N, heads, head_dim].)
+    if m.bshape or x.dim() != 2 or x.shape[1] != m.K:
         x = x.reshape([m.B, m.M, m.K] if m.bshape else [m.M, m.K])
     if x.dtype not in _FLOATS:
         x = x.to(m.out_dtype)

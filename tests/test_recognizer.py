@@ -328,3 +328,37 @@ def test_composite_decomposition_is_inlined():
     it = recognizer.Interpreter(text)
     assert not any(o.name == "stablehlo.composite" for o in it.func.walk())
     assert len(recognizer.analyze(it).matches) == 1
+
+
+def test_both_dimensions_of_the_activation_contracted(monkeypatch):
+    """One token's heads against a projection `[N, heads, head_dim]`: the activation has two dimensions and M is 1. The fused op
+    gets `[M, K]`, and the program's result is the literal one's."""
+    full, wide = "tensor<16x4x64xbf16>", "tensor<16x4x2x32xbf16>"
+    text = f"""module @jit_output_projection {{
+  func.func public @main(%arg0: tensor<4x64xbf16>, %arg1: tensor<16x4x64xi8>, %arg2: tensor<16x4x2xbf16>) -> (tensor<16xbf16>) {{
+    %0 = stablehlo.convert %arg1 : (tensor<16x4x64xi8>) -> {full}
+    %1 = stablehlo.broadcast_in_dim %arg2, dims = [0, 1, 2] : (tensor<16x4x2xbf16>) -> {wide}
+    %2 = stablehlo.reshape %1 : ({wide}) -> {full}
+    %3 = stablehlo.multiply %0, %2 : {full}
+    %4 = stablehlo.dot_general %arg0, %3, contracting_dims = [0, 1] x [1, 2] : (tensor<4x64xbf16>, {full}) -> tensor<16xbf16>
+    return %4 : tensor<16xbf16>
+  }}
+}}
+"""
+    g = torch.Generator().manual_seed(11)
+    x = torch.randn((4, 64), generator=g).to(torch.bfloat16)
+    codes = torch.randint(-8, 8, (16, 4, 64), generator=g, dtype=torch.int8)
+    scales = (torch.rand((16, 4, 2), generator=g) * 0.02 + 0.01).to(torch.bfloat16)
+
+    def product(x, w, s, b, transpose=True, group_size=64, bits=4, mode="affine", out_dtype=None):
+        assert tuple(x.shape) == (1, 256)
+        words, tables = w.view(torch.int32).numpy().view(np.uint32), [t.float().numpy() for t in (s, b)]
+        y = O.qmm_exact(x.float().numpy(), words, *tables, group_size, bits)
+        return torch.from_numpy(np.asarray(y)).to(out_dtype)
+
+    monkeypatch.setattr(qmm, "quantized_matmul", product)
+    it = recognizer.Interpreter(text)
+    got = it.execute([x, codes, scales])[0]
+    assert it.fused_calls == 1
+    want = torch.einsum("hd,nhd->n", x.float(), codes.float() * scales.float().repeat_interleave(32, -1))
+    assert tuple(got.shape) == (16,) and torch.allclose(got.float(), want, rtol=2e-2, atol=2e-2)
