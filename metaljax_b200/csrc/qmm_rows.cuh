@@ -25,6 +25,14 @@
 // three columns (8 + 8 + 8 bits of bf16, or 11 + 11 + 11 of f16) that are added at the end; for f16 fragments of bf16 or float32 activations
 // each row of each slice is scaled to [2^14, 2^15) by its largest magnitude, and back in its partial sums. The K order inside a group is
 // free as long as codes and activations agree: lane t takes 16 consecutive codes (8 in groups of 32), in the pair order one LOP3 extracts.
+//
+// Float32 activations are for float32 results, and the magic number, though it cancels, costs those the bits in which 128 or 1024 is
+// larger than a code. There one exact subtraction a pair makes it q - 8 or q - 128, the accumulators start at nought, and the bias that goes with
+// the sum of x is b + 8 s or b + 128 s (nought for most weights). What is left is the tensor core's truncation of a float32 sum. (Codes as f16
+// subnormals need neither the magic nor the subtraction, but are aligned as if they had all their bits.)
+// Relative error against float64 (2-norm, the largest over K 512 to 14336 and all group sizes) of the SIMT kernel / with the magic number / so, for N(0, 1),
+// one sign, outliers of 300: 4-bit 3.8e-7 / 4.9e-6 / 1.1e-7, 6.0e-7 / 1.3e-5 / 0.7e-7, 4.5e-7 / 1.1e-5 / 1.1e-7; 8-bit 2.6e-7 / 3.5e-6 / 1.4e-7,
+// 6.8e-7 / 2.2e-4 / 1.3e-7, 3.7e-7 / 5.4e-6 / 3.0e-7. 33 rows of 4096 x 4096: 34.8 us with the magic number, 35.6 so.
 // (8-bit float MMAs would take the codes with a third of the instructions, but `mma.sync` on e4m3 is emulated here with
 // conversions to f16: 88 against 67 us for 8 rows of 128256 x 4096.)
 //
@@ -172,6 +180,18 @@ __device__ __forceinline__ float2 unpack2(uint32_t u) {
   else return __half22float2(*reinterpret_cast<const __half2*>(&u));
 }
 
+// The codes under the magic exponent minus (magic + centre): exact.
+template <typename AT>
+__device__ __forceinline__ uint32_t centred(uint32_t pair, float offset) {
+  if constexpr (std::is_same<AT, __nv_bfloat16>::value) {
+    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&pair), __float2bfloat162_rn(offset));
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&pair), __float2half2_rn(offset));
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -251,6 +271,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   using AT = typename std::conditional<QK == kAff4, typename std::conditional<std::is_same<XT, float>::value, __nv_bfloat16, XT>::type, __half>::type;
   constexpr bool kScaled = std::is_same<AT, __half>::value && !std::is_same<XT, __half>::value;
+  constexpr bool kCentred = std::is_same<XT, float>::value && QK != kMx4;      // the magic number is taken off the codes, not off the sums
+  constexpr float kCentre = QK == kAff8 ? 128.0f : 8.0f;
+  constexpr float kSumIs = kCentred ? 1.0f : -Mma<AT>::kMagicValue;   // the groups' sums of x are kept times this
   // Columns: piece i of the tokens of octet q is column group q * kPieces + i, its column c token 8 q + c. With 4 tokens two pieces share
   // a group: column c is token c & 3 of piece 2 h + (c >> 2).
   constexpr int kPieces = std::is_same<XT, float>::value ? 3 : 1;
@@ -268,7 +291,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   constexpr int kMmas = kBlk / 16;
   constexpr int kGroups = kSliceK / (32 * SPG);                       // groups of a slice
   constexpr int kBlocksPerGroup = kBlocks / kGroups;
-  constexpr bool kBiasMma = TT == kTabBf16;                           // the bias term is an MMA of its own (see load_x)
+  constexpr bool kBiasMma = TT == kTabBf16 && !kCentred;              // the bias term is an MMA of its own (see load_x)
   constexpr int kBiasMmas = kGroups == 16 ? 3 : kGroups == 8 ? 2 : 1;
   constexpr int kEntry = entry_bytes(TT);
   constexpr int kRowBytes = table_row_bytes(kGroups, TT);             // a weight row's table entries in a slice
@@ -617,8 +640,8 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
           if (c % kPer == kPer - 1) {
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            // (kept as -C sum x: where the group's accumulators start)
-            if (t == 0) sts32(sums_at + ((q * kGroups + c / kPer) * 8 + g) * 4, -Mma<AT>::kMagicValue * sum);
+            // (kept as -C sum x where the group's accumulators start there)
+            if (t == 0) sts32(sums_at + ((q * kGroups + c / kPer) * 8 + g) * 4, kSumIs * sum);
             if constexpr (kBiasMma) group_sum[c / kPer] = kHalf && g >= 4 ? 0.0f : sum;
             sum = 0.0f;
           }
@@ -689,9 +712,6 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     }
     __syncwarp();
   };
-
-  // (4 tokens: only the columns of the first piece start at -C sum x, which is of the whole value)
-  [[maybe_unused]] auto half_start = [&](float c) -> float { return t < 2 ? c : 0.0f; };
 
   // ---- the tiles ----
   // A lane's bytes of block 0 of row rho in a slot; block j is at this address XOR its chunk term.
@@ -853,7 +873,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     static_for<kGroups>([&](auto gc) {
       constexpr int gi = decltype(gc)::value;
       float acc[R][NT][4];
-      float start[Q][2];                           // -C sum x of the group
+      float start[Q][2];                           // kSumIs * sum x of the group
 #pragma unroll
       for (int q = 0; q < Q; ++q) start[q][0] = start[q][1] = 0.0f;
       if constexpr (QK != kMx4)
@@ -906,14 +926,15 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
                 a[0] = place_bits(v0, n0); a[1] = place_bits(v1, n0); a[2] = place_bits(v0, n0 + 1); a[3] = place_bits(v1, n0 + 1);
               }
             }
+            if constexpr (kCentred) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) a[i] = centred<AT>(a[i], Mma<AT>::kMagicValue + kCentre);
+            }
 #pragma unroll
             for (int h = 0; h < NT; ++h) {
-              // (all pieces but the first start from zero: -C sum x is of the whole value)
-              const bool of_first = kHalf ? h == 0 : h % kPieces == 0;
-              const int q = kHalf ? 0 : h / kPieces;
-              if constexpr (jj == 0 && mi == 0)
-                Mma<AT>::first(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1], of_first ? (kHalf ? half_start(start[q][0]) : start[q][0]) : 0.0f,
-                               of_first ? (kHalf ? half_start(start[q][1]) : start[q][1]) : 0.0f);
+              if constexpr (jj == 0 && mi == 0)     // (16-bit activations alone, one piece, keep the magic number)
+                Mma<AT>::first(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1], kCentred ? 0.0f : start[0][0],
+                               kCentred ? 0.0f : start[0][1]);
               else
                 Mma<AT>::run(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1]);
             }
@@ -939,8 +960,12 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
           fma2(y[r][h][2], y[r][h][3], s1, acc[r][h][2], acc[r][h][3]);
         }
         if constexpr (QK != kMx4 && !kBiasMma) {
-          constexpr float kPer = -1.0f / Mma<AT>::kMagicValue;
-          const float b0 = kPer * value(lds32<kTable + kAt>(trow)), b1 = kPer * value(lds32<kTable + kAt8>(trow));
+          float b0 = value(lds32<kTable + kAt>(trow)), b1 = value(lds32<kTable + kAt8>(trow));
+          if constexpr (kCentred) {
+            b0 = fmaf(kCentre, s0, b0); b1 = fmaf(kCentre, s1, b1);
+          } else {
+            b0 *= 1.0f / kSumIs; b1 *= 1.0f / kSumIs;
+          }
 #pragma unroll
           for (int q = 0; q < Q; ++q) {
             fma2(yb[r][q][0], yb[r][q][1], b0, start[q][0], start[q][1]);

@@ -70,3 +70,40 @@ def test_few_rows_per_expert(kind, x, sizes):
     assert not got[sum(sizes):].any()
     if sum(sizes):
         assert O.rel_err(got, O.ragged_qmm_exact(xs, w, s, b, gsz, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))) <= 1e-2
+
+
+def _styled(rng, shape, style):
+    """Activations N(0, 1), of one sign, or with outliers of 300."""
+    v = rng.standard_normal(shape)
+    if style == "one sign":
+        v = np.abs(v)
+    elif style == "outliers":
+        v[..., ::97] *= 300.0
+    return v.astype(np.float32)
+
+
+def _weight64(w, s, b, kw):
+    """The weight in float64 (the oracle's is rounded to float32 element by element)."""
+    if b is None:
+        return O.dequantize(w, s, None, 32, 4, "mxfp4").astype(np.float64)
+    gs = kw["group_size"]
+    codes = O.dequantize(w, np.ones(s.shape, np.float32), np.zeros(s.shape, np.float32), gs, kw["bits"], "affine").astype(np.float64)
+    return codes * np.repeat(s.astype(np.float64), gs, -1) + np.repeat(b.astype(np.float64), gs, -1)
+
+
+@pytest.mark.parametrize("style", ["normal", "one sign", "outliers"])
+@pytest.mark.parametrize("kind,gs,tdt", [("int4", 32, "f32"), ("int4", 128, "bf16"), ("int8", 32, "bf16"), ("int8", 128, "f32"), ("mxfp4", 32, None)])
+@pytest.mark.parametrize("m,k,n", [(3, 512, 130), (33, 5632, 96)])
+def test_float32_is_as_exact_as_plain_float32(kind, gs, tdt, style, m, k, n):
+    """Against the SIMT kernel, which sums float32 products one by one: the few-rows kernel is no further from the exact product.
+    Both errors are sums of roundings of 2^-24 that scatter by a few percent; a quarter is allowed for that."""
+    rng = np.random.default_rng(m + k)
+    (w, s, b), kw = _case(rng, kind, n, k, gs, tdt)
+    xs = _styled(rng, (m, k), style)
+    args = [to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV)]
+    exact = xs.astype(np.float64) @ _weight64(w, s, b, kw).T
+    error = lambda y: np.linalg.norm(to_numpy(y).astype(np.float64) - exact) / np.linalg.norm(exact)
+    got = error(qmm.quantized_matmul(*args, **kw))
+    with _lib.force_route("simt"):
+        plain = error(qmm.quantized_matmul(*args, **kw))
+    assert got <= 1.25 * plain
