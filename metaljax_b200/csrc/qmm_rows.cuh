@@ -23,7 +23,7 @@
 // magic number out again). The bias term is an MMA of its own per 16 rows and slice: the bf16 bias entries against the groups' sums of x
 // in three bf16 pieces. Activations that the element type cannot hold as they are become several columns or carry a power of two: float32 is
 // three columns (8 + 8 + 8 bits of bf16, or 11 + 11 + 11 of f16) that are added at the end; for f16 fragments of bf16 or float32 activations
-// each row of each slice is scaled to [2^14, 2^15) by its largest magnitude, and back in its partial sums. The K order inside a group is
+// each row of each slice is scaled to [2^14, 2^15) by its largest finite magnitude, and back in its partial sums. The K order inside a group is
 // free as long as codes and activations agree: lane t takes 16 consecutive codes (8 in groups of 32), in the pair order one LOP3 extracts.
 //
 // Float32 activations are for float32 results, and the magic number, though it cancels, costs those the bits in which 128 or 1024 is
@@ -33,6 +33,9 @@
 // Relative error against float64 (2-norm, the largest over K 512 to 14336 and all group sizes) of the SIMT kernel / with the magic number / so, for N(0, 1),
 // one sign, outliers of 300: 4-bit 3.8e-7 / 4.9e-6 / 1.1e-7, 6.0e-7 / 1.3e-5 / 0.7e-7, 4.5e-7 / 1.1e-5 / 1.1e-7; 8-bit 2.6e-7 / 3.5e-6 / 1.4e-7,
 // 6.8e-7 / 2.2e-4 / 1.3e-7, 3.7e-7 / 5.4e-6 / 3.0e-7. 33 rows of 4096 x 4096: 34.8 us with the magic number, 35.6 so.
+// Range: an infinite activation makes its row's results infinite or NaN, as a sum of products does (affine codes: NaN where s (q - C) x and
+// the bias term have opposite signs); finite ones up to 2^120 give finite results where those fit. 4-bit codes take float32
+// activations below 2^-110 with fewer than 24 bits.
 // (8-bit float MMAs would take the codes with a third of the instructions, but `mma.sync` on e4m3 is emulated here with
 // conversions to f16: 88 against 67 us for 8 rows of 128256 x 4096.)
 //
@@ -179,6 +182,9 @@ __device__ __forceinline__ float2 unpack2(uint32_t u) {
   if constexpr (std::is_same<AT, __nv_bfloat16>::value) return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
   else return __half22float2(*reinterpret_cast<const __half2*>(&u));
 }
+
+// What `got`, a value rounded to fewer bits, leaves of it (exact; nothing of an infinity).
+__device__ __forceinline__ float left_of(float value, float got) { return fabsf(got) > 3.402823466e38f ? 0.0f : value - got; }
 
 // The codes under the magic exponent minus (magic + centre): exact.
 template <typename AT>
@@ -601,26 +607,21 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
       };
       float up = 1.0f;
       if constexpr (kScaled) {
-        float big = 0.0f;
-        bool bad = false;                                              // a NaN or an infinity: the row's results are NaN
+        float big = 0.0f;                                              // (infinities and NaN need no room: they are what they are in any unit)
 #pragma unroll
         for (int c = 0; c < kSliceK / 32; ++c) {
           float f[8];
           load8(c, f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            big = fmaxf(big, fabsf(f[i]));
-            bad |= !(fabsf(f[i]) <= 3.402823466e38f);
-          }
+          for (int i = 0; i < 8; ++i) big = fmaxf(big, fabsf(f[i]) <= 3.402823466e38f ? fabsf(f[i]) : 0.0f);
         }
         big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
         big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
-        bad = __ballot_sync(0xffffffffu, bad) & (0xfu << (lane & ~3));
         // largest magnitude to [2^14, 2^15); a warp's later slices no finer than its earlier ones, whose sums are brought to their units
-        const uint32_t e = min(max(__float_as_uint(big) >> 23, sub > 0 ? least_e[q] : 15u), 253u);
+        const uint32_t e = max(__float_as_uint(big) >> 23, sub > 0 ? least_e[q] : 15u);
         least_e[q] = e;
         up = __uint_as_float((268u - e) << 23);
-        const float down = bad ? __uint_as_float(0x7fc00000u) : __uint_as_float((e - 14u) << 23);
+        const float down = __uint_as_float((e - 14u) << 23);
         back[q][0] = __shfl_sync(0xffffffffu, down, 8 * t);
         back[q][1] = __shfl_sync(0xffffffffu, down, 8 * t + 4);
       }
@@ -657,7 +658,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float2 got = unpack2<AT>(u[j]);
-              f[2 * j] -= got.x; f[2 * j + 1] -= got.y;
+              f[2 * j] = left_of(f[2 * j], got.x); f[2 * j + 1] = left_of(f[2 * j + 1], got.y);
             }
           }
           if constexpr (QK != kAff8) {                                 // 4-bit codes: (0,4) (1,5) (2,6) (3,7); 8-bit ones in order, (0,1) (2,3)
@@ -691,9 +692,10 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
         auto split = [&](float a, float b, uint32_t (&piece)[3]) {
           piece[0] = pack2<B16>(a, b);
           const float2 f0 = unpack2<B16>(piece[0]);
-          piece[1] = pack2<B16>(a - f0.x, b - f0.y);
+          const float a1 = left_of(a, f0.x), b1 = left_of(b, f0.y);
+          piece[1] = pack2<B16>(a1, b1);
           const float2 f1 = unpack2<B16>(piece[1]);
-          piece[2] = pack2<B16>((a - f0.x) - f1.x, (b - f0.y) - f1.y);
+          piece[2] = pack2<B16>(a1 - f1.x, b1 - f1.y);
         };
         uint32_t lower[3];
         split(pick(0), pick(1), lower);

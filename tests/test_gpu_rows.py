@@ -107,3 +107,31 @@ def test_float32_is_as_exact_as_plain_float32(kind, gs, tdt, style, m, k, n):
     with _lib.force_route("simt"):
         plain = error(qmm.quantized_matmul(*args, **kw))
     assert got <= 1.25 * plain
+
+
+@pytest.mark.parametrize("x", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("value", [np.inf, -np.inf])
+def test_infinite_activations_are_summed_as_they_are(x, value):
+    """MXFP4 has no bias: an infinity times a positive, a negative or a zero weight, and the rows beside it as ever."""
+    rng = np.random.default_rng(5)
+    (w, s, _), kw = _case(rng, "mxfp4", 70, 1120, 32, None)
+    xs = activations(rng, (3, 1120), x)
+    xs[1, 17] = value
+    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None, out_dtype=torch.float32, **kw))
+    column = O.qmm_exact(np.eye(1120, dtype=np.float32)[17:18], w, s, None, 32, 4, mode="mxfp4")[0]      # the weights that the infinity meets
+    with np.errstate(invalid="ignore"):
+        np.testing.assert_array_equal(y[1], np.float32(value) * column.astype(np.float32))
+    rest = O.qmm_exact(xs[[0, 2]], w, s, None, 32, 4, mode="mxfp4")
+    assert O.rel_err(y[[0, 2]], rest) <= 1e-5
+
+
+@pytest.mark.parametrize("kind,gs", [("int4", 64), ("int8", 64), ("mxfp4", 32)])
+@pytest.mark.parametrize("size", [2.0 ** 120, 2.0 ** -100])
+def test_large_and_small_float32_activations(kind, gs, size):
+    """Finite results of finite activations, whatever their size: as exact as those near one (the gate for float32)."""
+    rng = np.random.default_rng(6)
+    (w, s, b), kw = _case(rng, kind, 70, 1152, gs, "f32")
+    xs = activations(rng, (5, 1152), "f32") * np.float32(size / 8)
+    y = qmm.quantized_matmul(to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV), **kw)
+    exact = O.qmm_exact(xs.astype(np.float64) / size, w, s, b, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
+    assert O.rel_err(to_numpy(y).astype(np.float64) / size, exact) <= 1e-5
