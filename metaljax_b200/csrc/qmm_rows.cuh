@@ -17,16 +17,17 @@
 // a cluster the CTAs' sums travel to the tile's leader (in turn) by st.async and are added in rank order.
 // No global scratch, no atomics, fixed order of summation.
 //
-// Arithmetic. The codes are never dequantized: a nibble pair under a magic exponent is an exact bf16 (128 + q) or f16 (1024 + q) A
-// fragment of `mma.sync.m16n8k16`, an 8-bit pair an f16 one (a byte permute), an E2M1 pair an exact f16 times 2^-14; scale and bias
+// Arithmetic. The codes are never dequantized: a nibble pair under a magic exponent is an exact bf16 (128 + q) or f16 (16 + q) A
+// fragment of `mma.sync.m16n8k16`, an 8-bit pair an f16 one (1024 + q, a byte permute), an E2M1 pair an exact f16 times 2^-14; scale and bias
 // meet the float32 accumulators once per group (the 16 K slots of an MMA lie in one group; the accumulators start at -C sum x, which takes the
-// magic number out again). The bias term is an MMA of its own per 16 rows and slice: the bf16 bias entries against the groups' sums of x
+// magic number out again; 16 + q, with the code at the top of the mantissa, is a shift more per two words than 1024 + q and leaves that much less to cancel:
+// 8 rows of f16, one sign, 4.6e-4 -> 1.2e-6 of the result's norm in float32, grouped products 1.4e-4 -> 5e-7). The bias term is an MMA of its own per 16 rows and slice: the bf16 bias entries against the groups' sums of x
 // in three bf16 pieces. Activations that the element type cannot hold as they are become several columns or carry a power of two: float32 is
 // three columns (8 + 8 + 8 bits of bf16, or 11 + 11 + 11 of f16) that are added at the end; for f16 fragments of bf16 or float32 activations
 // each row of each slice is scaled to [2^14, 2^15) by its largest finite magnitude, and back in its partial sums. The K order inside a group is
 // free as long as codes and activations agree: lane t takes 16 consecutive codes (8 in groups of 32), in the pair order one LOP3 extracts.
 //
-// Float32 activations are for float32 results, and the magic number, though it cancels, costs those the bits in which 128 or 1024 is
+// Float32 activations are for float32 results, and the magic number, though it cancels, costs those the bits in which it is
 // larger than a code. There one exact subtraction a pair makes it q - 8 or q - 128, the accumulators start at nought, and the bias that goes with
 // the sum of x is b + 8 s or b + 128 s (nought for most weights). What is left is the tensor core's truncation of a float32 sum. (Codes as f16
 // subnormals need neither the magic nor the subtraction, but are aligned as if they had all their bits.)
@@ -109,8 +110,6 @@ template <typename AT>
 struct Mma;
 template <>
 struct Mma<__nv_bfloat16> {
-  static constexpr uint32_t kMagic = 0x43004300u;
-  static constexpr float kMagicValue = 128.0f;
   static __device__ __forceinline__ void run(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -125,8 +124,6 @@ struct Mma<__nv_bfloat16> {
 };
 template <>
 struct Mma<__half> {
-  static constexpr uint32_t kMagic = 0x64006400u;
-  static constexpr float kMagicValue = 1024.0f;
   static __device__ __forceinline__ void run(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -277,9 +274,12 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   using AT = typename std::conditional<QK == kAff4, typename std::conditional<std::is_same<XT, float>::value, __nv_bfloat16, XT>::type, __half>::type;
   constexpr bool kScaled = std::is_same<AT, __half>::value && !std::is_same<XT, __half>::value;
+  // A pair of codes under this exponent is kMagicValue + code.
+  constexpr uint32_t kMagic = QK == kAff8 ? 0x64006400u : std::is_same<AT, __half>::value ? 0x4C004C00u : 0x43004300u;
+  constexpr float kMagicValue = QK == kAff8 ? 1024.0f : std::is_same<AT, __half>::value ? 16.0f : 128.0f;
   constexpr bool kCentred = std::is_same<XT, float>::value && QK != kMx4;      // the magic number is taken off the codes, not off the sums
   constexpr float kCentre = QK == kAff8 ? 128.0f : 8.0f;
-  constexpr float kSumIs = kCentred ? 1.0f : -Mma<AT>::kMagicValue;   // the groups' sums of x are kept times this
+  constexpr float kSumIs = kCentred ? 1.0f : -kMagicValue;   // the groups' sums of x are kept times this
   // Columns: piece i of the tokens of octet q is column group q * kPieces + i, its column c token 8 q + c. With 4 tokens two pieces share
   // a group: column c is token c & 3 of piece 2 h + (c >> 2).
   constexpr int kPieces = std::is_same<XT, float>::value ? 3 : 1;
@@ -720,7 +720,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   const uint32_t wthread = ring_at + rho * kBoxBytes +
                            (QK == kAff8 ? (SPG == 1 ? ((((t >> 1) ^ rho) << 4) + (t & 1) * 8) : ((t ^ rho) << 4))
                                         : (SPG == 1 ? ((rho << 4) + t * 4) : ((((t >> 1) ^ rho) << 4) + (t & 1) * 8)));
-  uint32_t nib_mask = 0x000F000Fu, magic = Mma<AT>::kMagic;
+  uint32_t nib_mask = std::is_same<AT, __half>::value ? 0x03C003C0u : 0x000F000Fu, magic = kMagic;
   asm volatile("" : "+r"(nib_mask), "+r"(magic));                      // constants in registers: one LOP3 per use
   const uint32_t tthread = tables_at + rho * kPitch, scol = sums_at + 8 * t;
   int turn = 0, which = 0, tile = tile0, sub = 0, count = 0;
@@ -914,9 +914,13 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
             } else {                                                      // half a word: nibbles (0,4) (1,5), or (2,6) (3,7)
               const uint32_t v0 = u[0][mi / 2], v1 = u[1][mi / 2];
               if constexpr (QK == kAff4) {
-                constexpr int sh = (mi & 1) * 8;
-                a[0] = and_or(v0 >> sh, nib_mask, magic);       a[1] = and_or(v1 >> sh, nib_mask, magic);
-                a[2] = and_or(v0 >> (sh + 4), nib_mask, magic); a[3] = and_or(v1 >> (sh + 4), nib_mask, magic);
+                auto codes = [&](uint32_t v, int nib) -> uint32_t {
+                  const int right = 4 * nib - (std::is_same<AT, __half>::value ? 6 : 0);
+                  return and_or(right < 0 ? v << -right : v >> right, nib_mask, magic);
+                };
+                constexpr int n0 = (mi & 1) * 2;
+                a[0] = codes(v0, n0);     a[1] = codes(v1, n0);
+                a[2] = codes(v0, n0 + 1); a[3] = codes(v1, n0 + 1);
               } else {
                 // magnitude bits of an E2M1 code at f16's exponent / mantissa boundary (the value times 2^-14,
                 // the subnormal 0.5 included), its sign at the sign
@@ -930,7 +934,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
             }
             if constexpr (kCentred) {
 #pragma unroll
-              for (int i = 0; i < 4; ++i) a[i] = centred<AT>(a[i], Mma<AT>::kMagicValue + kCentre);
+              for (int i = 0; i < 4; ++i) a[i] = centred<AT>(a[i], kMagicValue + kCentre);
             }
 #pragma unroll
             for (int h = 0; h < NT; ++h) {

@@ -135,3 +135,19 @@ def test_large_and_small_float32_activations(kind, gs, size):
     y = qmm.quantized_matmul(to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV), **kw)
     exact = O.qmm_exact(xs.astype(np.float64) / size, w, s, b, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
     assert O.rel_err(to_numpy(y).astype(np.float64) / size, exact) <= 1e-5
+
+
+@pytest.mark.parametrize("sizes", [[3, 0, 9, 1, 20, 2], [5, 1, 0, 8, 1, 1]])
+def test_half_nibbles_of_one_sign(sizes):
+    """4-bit codes against f16 of one sign, where the sums are far larger than the results: no further from the exact product than the
+    tensor-core kernel, whose weights are rounded to f16."""
+    rng = np.random.default_rng(sum(sizes))
+    (w, s, b), kw = _case(rng, "int4", 96, 2048, 64, "f16", lead=(len(sizes),))
+    xs = np.abs(activations(rng, (sum(sizes), 2048), "f16"))
+    gsz = np.array(sizes, np.int32)
+    args = [to_torch(a, DEV) for a in (xs, w, s, b)] + [torch.from_numpy(gsz).to(DEV)]
+    exact = O.ragged_qmm_exact(xs, w, s, b, gsz, kw["group_size"], kw["bits"]).astype(np.float64)
+    error = lambda y: np.linalg.norm(to_numpy(y).astype(np.float64) - exact) / np.linalg.norm(exact)
+    got = error(moe.ragged_dot(*args, out_dtype=torch.float32, **kw))
+    with _lib.force_route("gemm_tc"):
+        assert got <= error(moe.ragged_dot(*args, out_dtype=torch.float32, **kw))
