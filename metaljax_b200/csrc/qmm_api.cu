@@ -216,7 +216,9 @@ int launch_problem(const qmm_problem& p, cudaStream_t stream) {
     case QMM_ROUTE_GEMM_TC: return launch_gemm_tc(p, stream);
     // Float32 activations and what the others decline (unsorted gathers of more than 16 rows, K below 64): the
     // few-rows kernel takes them as columns of its MMAs; the plain SIMT kernel is what a forced route cross-checks with.
-    default: return route_override() != QMM_ROUTE_SIMT && rows_supports(p) ? launch_rows(p, stream) : launch_simt(p, stream);
+    // Its codes go in without a magic number here, since the SIMT kernel's float32 sums are what such calls had: with it a float32 result
+    // of activations of one sign was 60 (4-bit) to 140 times (8-bit) further from the exact one than the SIMT kernel's.
+    default: return route_override() != QMM_ROUTE_SIMT && rows_supports(p) ? launch_rows(p, stream, nullptr, true) : launch_simt(p, stream);
   }
 }
 

@@ -53,7 +53,8 @@ struct RowsGather {            // grouped products whose rows of x are picked by
   const int32_t* x_rows;       // [M] row of x behind each row of the product
   int64_t total_x_rows;
 };
-int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr);
+// `exact`: 16-bit activations whose sums are to be as exact as plain float32 ones (float32 activations' always are).
+int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr, bool exact = false);
 bool rows_supports(const qmm_problem& p);
 bool rows_grouped_pays(const qmm_problem& p);
 // A checked problem on the kernel its route names; and whether that is the few-rows kernel for a grouped one.

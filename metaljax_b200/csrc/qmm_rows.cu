@@ -38,7 +38,7 @@ RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh
   const int sms = device_sm_count();
   RowsPlan best = {};
   double best_load = 0.0;
-  for (int blocks = kMaxBlocks; blocks >= 1; --blocks) {
+  for (int blocks = kMaxBlocks; blocks >= (sh.exact ? kMaxBlocks : 1); --blocks) {
     const int64_t items = chunks * ((rows + kBlockRows * blocks - 1) / (kBlockRows * blocks));
     for (int c = 1; c <= kMaxCluster; c *= 2) {
       if (c > slices && c > 1) break;
@@ -101,7 +101,7 @@ bool gemv_supports(const qmm_problem& p) {
   return (p.x_dtype == QMM_BF16 || p.x_dtype == QMM_F16) && !p.group_sizes && p.M <= 16 && p.batch <= 65535 && rows_supports(p);
 }
 
-int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather) {
+int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather, bool exact) {
   RowsParams rp = {};
   rp.x = p.x; rp.scales = p.scales; rp.biases = p.biases; rp.y = p.y;
   rp.lhs_idx = p.lhs_idx; rp.rhs_idx = p.rhs_idx; rp.group_sizes = p.group_sizes;
@@ -130,7 +130,7 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
   const int64_t live = p.group_sizes ? (p.batch < p.M ? p.batch : p.M) : p.batch;
   const int entry = mx ? 1 : (p.table_dtype == QMM_F32 ? 4 : 2);
   const RowsShape sh = {chunk, kSliceK / group, mx ? kTabE8 : (p.table_dtype == QMM_BF16 ? kTabBf16 : (p.table_dtype == QMM_F16 ? kTabF16 : kTabF32)),
-                        kBlockRows * kSliceK * bits / 8};
+                        kBlockRows * kSliceK * bits / 8, exact && !mx && p.x_dtype != QMM_F32};
   const int64_t nweights = p.num_weights > 0 ? p.num_weights : (p.w_batch_stride ? p.batch : 1);
   rp.table_bytes = nweights * p.N * rp.groups * entry;
   // (a slice's entries start on the units that its own row of entries and a row of the table are multiples of)

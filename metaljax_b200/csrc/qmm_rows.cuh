@@ -27,8 +27,8 @@
 // each row of each slice is scaled to [2^14, 2^15) by its largest finite magnitude, and back in its partial sums. The K order inside a group is
 // free as long as codes and activations agree: lane t takes 16 consecutive codes (8 in groups of 32), in the pair order one LOP3 extracts.
 //
-// Float32 activations are for float32 results, and the magic number, though it cancels, costs those the bits in which it is
-// larger than a code. There one exact subtraction a pair makes it q - 8 or q - 128, the accumulators start at nought, and the bias that goes with
+// Where the results are meant to be float32 -- float32 activations, and the 16-bit ones of unsorted gathers of more than 16 rows (EXACT) -- the
+// magic number, though it cancels, would cost them the bits in which it is larger than a code. There one exact subtraction a pair makes it q - 8 or q - 128, the accumulators start at nought, and the bias that goes with
 // the sum of x is b + 8 s or b + 128 s (nought for most weights). What is left is the tensor core's truncation of a float32 sum. (Codes as f16
 // subnormals need neither the magic nor the subtraction, but are aligned as if they had all their bits.)
 // Relative error against float64 (2-norm, the largest over K 512 to 14336 and all group sizes) of the SIMT kernel / with the magic number / so, for N(0, 1),
@@ -268,8 +268,9 @@ constexpr int sums_bytes(int groups) { return groups * 32; }
 constexpr int more_x_bytes(int tokens) { return tokens == 8 ? 0 : kSliceK * 16; }
 
 // QK: quantization kind. XT: activation type in memory. T: activation rows (tokens) of a chunk, 8 (16-bit) or 4 (float32). SPG: 32-code
-// steps per quantization group (1, 2, 4). TT: what the table entries are. R: 16-row blocks of a tile.
-template <int QK, typename XT, int T, int SPG, int TT, int R>
+// steps per quantization group (1, 2, 4). TT: what the table entries are. R: 16-row blocks of a tile. EXACT: the magic number is taken off the codes, not
+// off the sums (affine codes).
+template <int QK, typename XT, int T, int SPG, int TT, int R, bool EXACT>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   using AT = typename std::conditional<QK == kAff4, typename std::conditional<std::is_same<XT, float>::value, __nv_bfloat16, XT>::type, __half>::type;
@@ -277,7 +278,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   // A pair of codes under this exponent is kMagicValue + code.
   constexpr uint32_t kMagic = QK == kAff8 ? 0x64006400u : std::is_same<AT, __half>::value ? 0x4C004C00u : 0x43004300u;
   constexpr float kMagicValue = QK == kAff8 ? 1024.0f : std::is_same<AT, __half>::value ? 16.0f : 128.0f;
-  constexpr bool kCentred = std::is_same<XT, float>::value && QK != kMx4;      // the magic number is taken off the codes, not off the sums
+  constexpr bool kCentred = EXACT && QK != kMx4;
   constexpr float kCentre = QK == kAff8 ? 128.0f : 8.0f;
   constexpr float kSumIs = kCentred ? 1.0f : -kMagicValue;   // the groups' sums of x are kept times this
   // Columns: piece i of the tokens of octet q is column group q * kPieces + i, its column c token 8 q + c. With 4 tokens two pieces share
@@ -938,7 +939,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
             }
 #pragma unroll
             for (int h = 0; h < NT; ++h) {
-              if constexpr (jj == 0 && mi == 0)     // (16-bit activations alone, one piece, keep the magic number)
+              if constexpr (jj == 0 && mi == 0)     // (what keeps the magic number has one piece)
                 Mma<AT>::first(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1], kCentred ? 0.0f : start[0][0],
                                kCentred ? 0.0f : start[0][1]);
               else
@@ -1068,6 +1069,7 @@ struct RowsPlan {
 
 struct RowsShape {
   int tokens, groups, tt, stage;         // rows of a chunk; groups per slice; bytes of codes of a 16-row block and slice
+  bool exact;                            // 16-bit activations, results in plain float32 (tiles of kMaxBlocks only)
 };
 
 // Clusters of this shape that fit the device at once (a GPC's SMs do not always divide by the cluster
@@ -1087,9 +1089,9 @@ inline int max_clusters(Kernel kernel, const cudaLaunchConfig_t& cfg, int cluste
   return n;
 }
 
-template <int QK, typename XT, int T, int SPG, int TT, int R>
+template <int QK, typename XT, int T, int SPG, int TT, int R, bool EXACT>
 int launch_kernel_of(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool early, cudaStream_t stream) {
-  auto kernel = qmm_rows_kernel<QK, XT, T, SPG, TT, R>;
+  auto kernel = qmm_rows_kernel<QK, XT, T, SPG, TT, R, EXACT>;
   static bool configured[kMaxDevices] = {};     // the attribute is per device
   const int dev = current_device();
   if (dev < 0) return QMM_ERR_DEVICE;
@@ -1130,40 +1132,43 @@ int launch_kernel_of(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool e
 }
 
 template <int QK, typename XT, int T, int SPG, int TT>
-int launch_kernel(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool early, cudaStream_t stream) {
-  if (pl.blocks == 1) return launch_kernel_of<QK, XT, T, SPG, TT, 1>(wm, rp, pl, early, stream);
-  return launch_kernel_of<QK, XT, T, SPG, TT, kMaxBlocks>(wm, rp, pl, early, stream);
+int launch_kernel(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
+  constexpr bool kFloat = std::is_same<XT, float>::value;
+  if constexpr (QK != kMx4 && !kFloat)
+    if (sh.exact) return launch_kernel_of<QK, XT, T, SPG, TT, kMaxBlocks, true>(wm, rp, pl, early, stream);
+  if (pl.blocks == 1) return launch_kernel_of<QK, XT, T, SPG, TT, 1, kFloat>(wm, rp, pl, early, stream);
+  return launch_kernel_of<QK, XT, T, SPG, TT, kMaxBlocks, kFloat>(wm, rp, pl, early, stream);
 }
 
 // (QK, XT) by T, group size and table type.
 template <int QK, typename XT, int T, int SPG>
-int launch_tt(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, int tt, bool early, cudaStream_t stream) {
+int launch_tt(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
   if constexpr (QK == kMx4) {
-    return launch_kernel<QK, XT, T, SPG, kTabE8>(wm, rp, pl, early, stream);
+    return launch_kernel<QK, XT, T, SPG, kTabE8>(wm, rp, pl, sh, early, stream);
   } else {
-    if (tt == kTabBf16) return launch_kernel<QK, XT, T, SPG, kTabBf16>(wm, rp, pl, early, stream);
-    if (tt == kTabF16) return launch_kernel<QK, XT, T, SPG, kTabF16>(wm, rp, pl, early, stream);
-    return launch_kernel<QK, XT, T, SPG, kTabF32>(wm, rp, pl, early, stream);
+    if (sh.tt == kTabBf16) return launch_kernel<QK, XT, T, SPG, kTabBf16>(wm, rp, pl, sh, early, stream);
+    if (sh.tt == kTabF16) return launch_kernel<QK, XT, T, SPG, kTabF16>(wm, rp, pl, sh, early, stream);
+    return launch_kernel<QK, XT, T, SPG, kTabF32>(wm, rp, pl, sh, early, stream);
   }
 }
 
 template <int QK, typename XT, int T>
-int launch_spg(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, int groups, int tt, bool early, cudaStream_t stream) {
+int launch_spg(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
   if constexpr (QK == kMx4) {
-    return launch_tt<QK, XT, T, 1>(wm, rp, pl, tt, early, stream);
+    return launch_tt<QK, XT, T, 1>(wm, rp, pl, sh, early, stream);
   } else {
-    if (groups == kSliceK / 32) return launch_tt<QK, XT, T, 1>(wm, rp, pl, tt, early, stream);
-    if (groups == kSliceK / 64) return launch_tt<QK, XT, T, 2>(wm, rp, pl, tt, early, stream);
-    return launch_tt<QK, XT, T, 4>(wm, rp, pl, tt, early, stream);
+    if (sh.groups == kSliceK / 32) return launch_tt<QK, XT, T, 1>(wm, rp, pl, sh, early, stream);
+    if (sh.groups == kSliceK / 64) return launch_tt<QK, XT, T, 2>(wm, rp, pl, sh, early, stream);
+    return launch_tt<QK, XT, T, 4>(wm, rp, pl, sh, early, stream);
   }
 }
 
 template <int QK, typename XT>
 int launch_rows_kernel(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
   if constexpr (sizeof(XT) == 4) {
-    return launch_spg<QK, XT, 4>(wm, rp, pl, sh.groups, sh.tt, early, stream);
+    return launch_spg<QK, XT, 4>(wm, rp, pl, sh, early, stream);
   } else {
-    return launch_spg<QK, XT, 8>(wm, rp, pl, sh.groups, sh.tt, early, stream);
+    return launch_spg<QK, XT, 8>(wm, rp, pl, sh, early, stream);
   }
 }
 

@@ -151,3 +151,20 @@ def test_half_nibbles_of_one_sign(sizes):
     got = error(moe.ragged_dot(*args, out_dtype=torch.float32, **kw))
     with _lib.force_route("gemm_tc"):
         assert got <= error(moe.ragged_dot(*args, out_dtype=torch.float32, **kw))
+
+
+@pytest.mark.parametrize("kind,x", [("int4", "bf16"), ("int4", "f16"), ("int8", "bf16"), ("int8", "f16")])
+@pytest.mark.parametrize("m,k", [(17, 2048), (32, 32)])
+def test_gathers_of_many_rows_sum_in_plain_float32(kind, x, m, k):
+    """Unsorted gathers of more than 16 rows, activations of one sign, a float32 result: no further from the exact product than the SIMT kernel
+    (a quarter for the scatter of the roundings, as above)."""
+    rng = np.random.default_rng(m + k)
+    (w, s, b), kw = _case(rng, kind, 96, k, 32, x, lead=(4,))
+    xs = np.abs(activations(rng, (5, m, k), x))
+    li, ri = rng.integers(0, 5, 9), rng.integers(0, 4, 9)
+    args = [to_torch(a, DEV) for a in (xs, w, s, b)] + [torch.from_numpy(i).to(DEV) for i in (li, ri)]
+    exact = np.stack([xs[i].astype(np.float64) @ _weight64(w[j], s[j], b[j], kw).T for i, j in zip(li, ri)])
+    error = lambda y: np.linalg.norm(to_numpy(y).astype(np.float64) - exact) / np.linalg.norm(exact)
+    got = error(moe.gather_qmm(*args, out_dtype=torch.float32, **kw))
+    with _lib.force_route("simt"):
+        assert got <= 1.25 * error(moe.gather_qmm(*args, out_dtype=torch.float32, **kw))
