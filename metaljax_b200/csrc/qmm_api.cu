@@ -186,10 +186,11 @@ int route_of(const qmm_problem& p) {
   if (forced == QMM_ROUTE_GEMV || forced == QMM_ROUTE_GEMV_FMMA) return gemv_supports(p) ? QMM_ROUTE_GEMV : -QMM_ERR_UNSUPPORTED;
   if (forced == QMM_ROUTE_GEMM_TC) return gemm_tc_supports(p) ? forced : -QMM_ERR_UNSUPPORTED;
   if (forced == QMM_ROUTE_SIMT) return forced;
-  // Nine to sixteen rows are two passes of the few-rows kernel. Where K is longer than one of its CTAs takes (8 warps x 512), so that
-  // they also meet in clusters, the tensor-core kernel's one pass is the faster (16 rows, us: 5632 x 2048 10.6 against 8.7, 14336 x 4096 25.0 / 19.7,
-  // 8-bit 31 / 23; at 4096 x 4096 9.3 / 9.8, at 4096 x 28672 34.5 / 35.7).
-  const bool long_k = p.M > 8 && p.K > 4096 && p.batch == 1 && !p.lhs_idx && gemm_tc_supports(p);
+  // Nine to sixteen rows are two passes of the few-rows kernel; against a long K, where its CTAs also meet in clusters, the
+  // tensor-core kernel's one pass is the faster (16 rows, us: 4096 x 14336 22.1 against 17.4; at 4096 x 4096 9.3 / 9.8). It would be from K 4096 on
+  // (5632 x 2048 10.6 / 8.7), but it rounds each weight to 16 bits, the few-rows kernel none: 1.4e-3 of a float32 result's norm against 1e-6,
+  // and 2.2e-3 against 1.7e-3 once the result is bf16. Below 8192, where these products were never rounded so, they are not.
+  const bool long_k = p.M > 8 && p.K >= 8192 && p.batch == 1 && !p.lhs_idx && gemm_tc_supports(p);
   if (gemv_supports(p) && !long_k) return QMM_ROUTE_GEMV;
   if (p.group_sizes && p.x_dtype != QMM_F32 && rows_grouped_pays(p)) return QMM_ROUTE_GEMV;
   if (gemm_tc_supports(p)) return QMM_ROUTE_GEMM_TC;

@@ -98,3 +98,13 @@ def test_routes():
     assert qmm.route(0, 4096, 4096) == "none"
     with pytest.raises(_lib.QmmError):
         qmm.route(1, 4096 + 16, 4096)
+
+
+def test_rows_that_were_never_rounded_to_16_bits_are_not():
+    """Nine to sixteen rows leave the kernel that keeps scale and bias in float32 only where they always did, from K 8192 on."""
+    for m in (9, 16):
+        for bits, group in ((4, 64), (8, 128)):
+            assert qmm.route(m, 4096 + 128, 2048, bits=bits, group_size=group) == "gemv"
+            assert qmm.route(m, 8192 - 128, 2048, bits=bits, group_size=group) == "gemv"
+            assert qmm.route(m, 8192, 2048, bits=bits, group_size=group) == "gemm_tc"
+        assert qmm.route(m, 5760, 2880, group_size=32, mode="mxfp4") == "gemv"

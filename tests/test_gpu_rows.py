@@ -168,3 +168,17 @@ def test_gathers_of_many_rows_sum_in_plain_float32(kind, x, m, k):
     got = error(moe.gather_qmm(*args, out_dtype=torch.float32, **kw))
     with _lib.force_route("simt"):
         assert got <= 1.25 * error(moe.gather_qmm(*args, out_dtype=torch.float32, **kw))
+
+
+@pytest.mark.parametrize("kind", ["int4", "int8", "mxfp4"])
+@pytest.mark.parametrize("m,k", [(9, 4224), (16, 5760)])
+def test_nine_to_sixteen_rows_keep_float32_weights(kind, m, k):
+    """A float32 result of bf16 activations. 4-bit codes are summed as 128 + q, of which 128 of some 10 cancel: 2^-24 * 16 of a term, of which K
+    random ones add up as their root does and so do the results; 2^-18 leaves four times that. (Weights rounded to bf16 are 2^-10 off.)"""
+    rng = np.random.default_rng(m + k)
+    (w, s, b), kw = _case(rng, kind, 96, k, 64, "bf16")
+    xs = activations(rng, (m, k), "bf16")
+    args = [to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV)]
+    y = to_numpy(qmm.quantized_matmul(*args, out_dtype=torch.float32, **kw)).astype(np.float64)
+    exact = xs.astype(np.float64) @ _weight64(w, s, b, kw).T
+    assert np.linalg.norm(y - exact) <= 2.0 ** -18 * np.linalg.norm(exact)
