@@ -91,10 +91,17 @@ bool rows_supports(const qmm_problem& p) {
   return nw * p.N < (1LL << 31);                    // TMA row coordinates are 32-bit
 }
 
-// A grouped product of at most this many rows per expert on average streams its experts' weights here; above it
-// the tensor-core kernel's wide token tiles win. (Experts' shares are only known on the device: an expert
-// of more than 8 rows passes its weight once per 8.)
-bool rows_grouped_pays(const qmm_problem& p) { return rows_supports(p) && p.M <= 16 * p.batch; }
+// A grouped product of at most 8 rows per expert on average streams its experts' weights here: an even share is one pass of a weight, and what
+// routing makes uneven still costs less than the tensor-core kernel's 64-row tiles. Above it those win, even shares or not. Experts' shares are
+// only known on the device, and a share of n rows passes its weight ceil(n / 8) times: the worst, all rows on one expert, is dearer here from 3 rows an
+// expert on. us here / tensor cores (weights from HBM), even, random and all on one:
+//   rows an expert            4                                    8                                     12
+//   4-bit  8 x 14336 x 4096   75/120   76/120   44/29              77/121   102/121  72/30               129/121  129/121   99/44
+//   4-bit  8 x 4096 x 14336   92/121   84/121   52/62              93/121   127/121  88/64               159/122  158/121  122/64
+//   4-bit 32 x 2048 x 2048    34/46    33/47    21/21              35/46     41/47   30/21                49/47    50/47    38/21
+//   mxfp4 32 x 2880 x 2880    75/95    76/94    42/28              75/95     98/94   73/30               133/95   129/94   101/30
+//   8-bit  8 x 4096 x 4096    42/55    43/55    25/32              43/55     47/55   35/32                56/56    56/55    43/32
+bool rows_grouped_pays(const qmm_problem& p) { return rows_supports(p) && p.M <= 8 * p.batch; }
 
 // The decode family as callers may force it: dense or gathered products of up to 16 rows of 16-bit activations.
 bool gemv_supports(const qmm_problem& p) {

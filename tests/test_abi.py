@@ -108,3 +108,10 @@ def test_rows_that_were_never_rounded_to_16_bits_are_not():
             assert qmm.route(m, 8192 - 128, 2048, bits=bits, group_size=group) == "gemv"
             assert qmm.route(m, 8192, 2048, bits=bits, group_size=group) == "gemm_tc"
         assert qmm.route(m, 5760, 2880, group_size=32, mode="mxfp4") == "gemv"
+
+
+def test_grouped_products_of_few_rows_per_expert():
+    """At most 8 rows per expert on average stream the weights; above, the tensor-core kernel's tiles win even where the shares are even."""
+    for experts in (1, 8, 32):
+        assert qmm.route(8 * experts, 4096, 2048, batch=experts, ragged=True) == "gemv"
+        assert qmm.route(8 * experts + 1, 4096, 2048, batch=experts, ragged=True) == "gemm_tc"

@@ -182,3 +182,16 @@ def test_nine_to_sixteen_rows_keep_float32_weights(kind, m, k):
     y = to_numpy(qmm.quantized_matmul(*args, out_dtype=torch.float32, **kw)).astype(np.float64)
     exact = xs.astype(np.float64) @ _weight64(w, s, b, kw).T
     assert np.linalg.norm(y - exact) <= 2.0 ** -18 * np.linalg.norm(exact)
+
+
+@pytest.mark.parametrize("sizes", [[0, 64, 0, 0, 0, 0, 0, 0], [32, 0, 0, 0, 0, 0, 0, 32], [57, 1, 1, 1, 1, 1, 1, 1], [0, 0, 0, 65, 0, 0, 0, 0], [0, 0, 128, 0, 0, 0, 0, 0]])
+@pytest.mark.parametrize("kind,x", [("int4", "bf16"), ("mxfp4", "f16")])
+def test_skewed_routing(kind, x, sizes):
+    """All or nearly all rows on one or two experts, on either side of the rule that picks the kernel by the average."""
+    rng = np.random.default_rng(sum(sizes) + sizes[0])
+    (w, s, b), kw = _case(rng, kind, 90, 704, 64, x, lead=(8,))
+    xs = activations(rng, (sum(sizes), 704), x)
+    gsz = np.array(sizes, np.int32)
+    y = moe.ragged_dot(to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV), torch.from_numpy(gsz).to(DEV), **kw)
+    exact = O.ragged_qmm_exact(xs, w, s, b, gsz, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
+    assert O.rel_err(to_numpy(y).astype(np.float32), exact) <= TOL[x]
