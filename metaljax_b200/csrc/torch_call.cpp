@@ -31,6 +31,8 @@ QuantizedMatmul g_quantized_matmul = nullptr;
 MoeWorkspace g_moe_workspace = nullptr;
 MoeExperts g_moe_experts = nullptr;
 
+constexpr int kDeclined = -1;         // (the library's codes are not negative)
+
 bool dtype_of(at::ScalarType t, qmm_dtype* d) {
   d->lanes = 1;
   switch (t) {
@@ -64,6 +66,22 @@ bool view_of(const at::Tensor& t, qmm_tensor* v) {
   return true;
 }
 
+// Runs f without the interpreter's lock, as ctypes and torch's own bindings do: a full launch queue makes an enqueue wait for the
+// device, which may be waiting for another thread of Python (a host callback in the stream), and a copy or an allocation may wait too.
+// What f throws is thrown again with the lock held.
+template <typename F>
+auto unlocked(F&& f) -> decltype(f()) {
+  PyThreadState* state = PyEval_SaveThread();
+  try {
+    auto result = f();
+    PyEval_RestoreThread(state);
+    return result;
+  } catch (const std::exception&) {
+    PyEval_RestoreThread(state);
+    throw;
+  }
+}
+
 // The packed words: uint32, or int32 of the same bits.
 bool words_of(const at::Tensor& t, qmm_tensor* v) {
   if (!view_of(t, v)) return false;
@@ -85,42 +103,45 @@ PyObject* quantized_matmul(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
   }
   const int64_t lead = x->dim() - 2, m = x->size(-2), k = x->size(-1), cols = w->size(-2);
-  at::Tensor y, xc;
+  at::Tensor y;
+  at::ScalarType dt = x->scalar_type();
   if (a[8] != Py_None) {
     const at::Tensor* out = plain_tensor(a[8]);
     if (!out || !out->is_contiguous() || out->dim() != x->dim() || out->size(-1) != cols || out->size(-2) != m) Py_RETURN_NONE;
     for (int64_t d = 0; d < lead; ++d)
       if (out->size(d) != x->size(d)) Py_RETURN_NONE;
     y = *out;
-  } else {
-    at::ScalarType dt = x->scalar_type();
-    if (a[9] != Py_None) {
-      if (!THPDtype_Check(a[9])) Py_RETURN_NONE;
-      dt = reinterpret_cast<THPDtype*>(a[9])->scalar_type;
+  } else if (a[9] != Py_None) {
+    if (!THPDtype_Check(a[9])) Py_RETURN_NONE;
+    dt = reinterpret_cast<THPDtype*>(a[9])->scalar_type;
+  }
+  const int rc = unlocked([&]() -> int {
+    if (!y.defined()) {
+      c10::SmallVector<int64_t, 5> shape(x->sizes().begin(), x->sizes().end());
+      shape[lead + 1] = cols;
+      y = at::detail::empty_cuda(shape, dt, x->device(), std::nullopt);
     }
-    c10::SmallVector<int64_t, 5> shape(x->sizes().begin(), x->sizes().end());
-    shape[lead + 1] = cols;
-    y = at::detail::empty_cuda(shape, dt, x->device(), std::nullopt);
-  }
-  xc = x->is_contiguous() ? *x : x->contiguous();
-  qmm_tensor vx, vw, vs, vb, vy;
-  if (!view_of(xc, &vx) || !words_of(*w, &vw) || !view_of(*s, &vs) || (b && !view_of(*b, &vb)) || !view_of(y, &vy)) Py_RETURN_NONE;
-  int64_t xs[3], ys[3];
-  if (lead > 0) {                          // one weight per batch of x, or a shared one: then the batches are more rows
-    const int64_t batches = x->numel() / (m * k);
-    const bool shared = w->dim() != 3;
-    vx.ndim = vy.ndim = shared ? 2 : 3;
-    xs[0] = ys[0] = shared ? batches * m : batches;
-    xs[1] = shared ? k : m;
-    ys[1] = shared ? cols : m;
-    xs[2] = k;
-    ys[2] = cols;
-    vx.shape = xs;
-    vy.shape = ys;
-    vx.strides = vy.strides = nullptr;
-  }
-  const int rc = g_quantized_matmul(&vx, &vw, &vs, b ? &vb : nullptr, &vy, transpose, static_cast<int>(gs), static_cast<int>(bits),
-                                    static_cast<int>(mode), c10::cuda::getCurrentCUDAStream(x->get_device()).stream());
+    const at::Tensor xc = x->is_contiguous() ? *x : x->contiguous();
+    qmm_tensor vx, vw, vs, vb, vy;
+    if (!view_of(xc, &vx) || !words_of(*w, &vw) || !view_of(*s, &vs) || (b && !view_of(*b, &vb)) || !view_of(y, &vy)) return kDeclined;
+    int64_t xs[3], ys[3];
+    if (lead > 0) {                        // one weight per batch of x, or a shared one: then the batches are more rows
+      const int64_t batches = x->numel() / (m * k);
+      const bool shared = w->dim() != 3;
+      vx.ndim = vy.ndim = shared ? 2 : 3;
+      xs[0] = ys[0] = shared ? batches * m : batches;
+      xs[1] = shared ? k : m;
+      ys[1] = shared ? cols : m;
+      xs[2] = k;
+      ys[2] = cols;
+      vx.shape = xs;
+      vy.shape = ys;
+      vx.strides = vy.strides = nullptr;
+    }
+    return g_quantized_matmul(&vx, &vw, &vs, b ? &vb : nullptr, &vy, transpose, static_cast<int>(gs), static_cast<int>(bits),
+                              static_cast<int>(mode), c10::cuda::getCurrentCUDAStream(x->get_device()).stream());
+  });
+  if (rc == kDeclined) Py_RETURN_NONE;
   if (rc) return PyLong_FromLong(rc);
   if (a[8] != Py_None) {
     Py_INCREF(a[8]);
@@ -180,13 +201,15 @@ PyObject* moe_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (idx->device() != x->device() || wts->device() != x->device()) Py_RETURN_NONE;
   const int64_t need = g_moe_workspace(&b);
   if (need < 0) Py_RETURN_NONE;
-  at::Tensor y, work, w32;
-  w32 = wts->scalar_type() == at::kFloat && wts->is_contiguous() ? *wts : wts->to(at::kFloat).contiguous();
-  y = at::detail::empty_cuda({b.tokens, b.d}, x->scalar_type(), x->device(), std::nullopt);
-  work = at::detail::empty_cuda({need}, at::kByte, x->device(), std::nullopt);
-  b.x = x->const_data_ptr(); b.indices = idx->const_data_ptr(); b.weights = w32.const_data_ptr<float>();
-  b.out = y.data_ptr(); b.workspace = work.data_ptr(); b.workspace_bytes = need;
-  const int rc = g_moe_experts(&b, c10::cuda::getCurrentCUDAStream(x->get_device()).stream());
+  at::Tensor y;
+  const int rc = unlocked([&]() -> int {
+    const at::Tensor w32 = wts->scalar_type() == at::kFloat && wts->is_contiguous() ? *wts : wts->to(at::kFloat).contiguous();
+    y = at::detail::empty_cuda({b.tokens, b.d}, x->scalar_type(), x->device(), std::nullopt);
+    const at::Tensor work = at::detail::empty_cuda({need}, at::kByte, x->device(), std::nullopt);
+    b.x = x->const_data_ptr(); b.indices = idx->const_data_ptr(); b.weights = w32.const_data_ptr<float>();
+    b.out = y.data_ptr(); b.workspace = work.data_ptr(); b.workspace_bytes = need;
+    return g_moe_experts(&b, c10::cuda::getCurrentCUDAStream(x->get_device()).stream());
+  });
   if (rc) return PyLong_FromLong(rc);
   return THPVariable_Wrap(std::move(y));
 }
