@@ -166,6 +166,7 @@ PyObject* moe_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 15 || !g_moe_experts) Py_RETURN_NONE;
   const at::Tensor *x = plain_tensor(a[0]), *idx = plain_tensor(a[1]), *wts = plain_tensor(a[2]);
   if (!x || !idx || !wts || x->dim() != 2 || idx->dim() != 2 || !x->is_contiguous() || !idx->is_contiguous()) Py_RETURN_NONE;
+  if (reinterpret_cast<uintptr_t>(x->const_data_ptr()) % 16) Py_RETURN_NONE;      // (the steps gather its rows into memory of their own)
   const long gs = PyLong_AsLong(a[12]), bits = PyLong_AsLong(a[13]), mode = PyLong_AsLong(a[14]);
   if (PyErr_Occurred()) {
     PyErr_Clear();

@@ -44,3 +44,20 @@ def test_expert_block_in_one_call(kind, x, index, tokens, experts, k):
     moe.moe_experts(xs, idx, wts, *packs, **kw)
     with pytest.raises(_lib.QmmError):
         _lib.poll_status()
+
+
+def test_activations_at_any_address():
+    """A contiguous view that starts on no 16-byte boundary: the same result as a copy of it."""
+    rng = np.random.default_rng(3)
+    d, f, t = 192, 320, 5
+    packs = []
+    for n, kk in ((f, d), (f, d), (d, f)):
+        arrays, kw = _case(rng, "int4", n, kk, "bf16", lead=(4,))
+        packs.append(tuple(to_torch(a, DEV) for a in arrays))
+    flat = to_torch(activations(rng, (4 + t * d,)), DEV)
+    x = flat[4:].view(t, d)
+    assert x.data_ptr() % 16
+    idx = torch.from_numpy(rng.integers(0, 4, (t, 2))).to(DEV)
+    wts = torch.rand((t, 2), device=DEV)
+    got, want = moe.moe_experts(x, idx, wts, *packs, **kw), moe.moe_experts(x.clone(), idx, wts, *packs, **kw)
+    assert O.rel_err(to_numpy(got).astype(np.float32), to_numpy(want).astype(np.float64)) <= 1e-2
