@@ -224,6 +224,9 @@ typedef struct {
 } qmm_moe_block;
 int64_t qmm_moe_workspace_bytes(const qmm_moe_block* block);
 int qmm_moe_experts(const qmm_moe_block* block, void* stream);
+/* The same, and an expert index outside [0, experts) is refused by this call itself (QMM_ERR_SHAPE; `out` is then undefined): it returns
+ * once the device has looked at every index, which is the first thing it does. On a stream that is being captured it is qmm_moe_experts. */
+int qmm_moe_experts_checked(const qmm_moe_block* block, void* stream);
 
 /* Replaces `mx.dequantize(w, scales, biases, group_size, bits[, mode])`, which the
  * reference uses to pin the packed layout (tests/test_qmm.py:121,

@@ -119,6 +119,7 @@ _SIGNATURES = {
                                           ctypes.c_void_p]),
     "qmm_moe_workspace_bytes": (ctypes.c_int64, [_T]),
     "qmm_moe_experts": (ctypes.c_int, [_T, ctypes.c_void_p]),
+    "qmm_moe_experts_checked": (ctypes.c_int, [_T, ctypes.c_void_p]),
     "qmm_launch": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.c_void_p]),
     # include/qmm_decode.h
     "qmm_decode_add_rmsnorm": (ctypes.c_int, [ctypes.c_void_p] * 5 + [ctypes.c_int64, ctypes.c_int64,
@@ -187,7 +188,7 @@ def native():
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
         loader.exec_module(module)
         module.bind(*(ctypes.cast(getattr(lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul", "qmm_moe_workspace_bytes",
-                                                                                             "qmm_moe_experts")))
+                                                                                             "qmm_moe_experts_checked")))
         _native = module
     return _native
 

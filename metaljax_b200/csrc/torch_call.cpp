@@ -226,7 +226,7 @@ PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   }
 }
 
-// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts)
+// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts_checked)
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 3) {
     PyErr_SetString(PyExc_TypeError, "bind takes the entry points' addresses");

@@ -114,6 +114,7 @@ def moe_experts(x, indices, weights, w1, w3, w2, group_size=64, bits=4, mode="af
     Pairs are sorted by expert and every projection is one `ragged_dot`; the routing
     weights are applied and the K terms summed in `sum_dtype` as the reference does
     after its gathered dots (src/metaljax/moe.py:1446-1453).
+    An index outside `[0, E)` raises (on a stream that is being captured it is reported by `qmm_poll_status`).
     """
     if sum_dtype == torch.float32:           # the whole block in one native call
         done = _lib.native().moe_experts(x, indices, weights, *w1, *w3, *w2, group_size, bits, _mode_id(mode))

@@ -40,10 +40,12 @@ def test_expert_block_in_one_call(kind, x, index, tokens, experts, k):
     act = moe.silu_mul(moe.ragged_dot(rows, *packs[0], sizes, **kw), moe.ragged_dot(rows, *packs[1], sizes, **kw))
     want = moe.routed_sum(moe.ragged_dot(act, *packs[2], sizes, **kw), order, wts, tokens, k)
     assert O.rel_err(to_numpy(got).astype(np.float32), to_numpy(want).astype(np.float64)) <= 1e-2
-    idx[0, 0] = experts                                       # an index outside the experts: reported, never followed
-    moe.moe_experts(xs, idx, wts, *packs, **kw)
-    with pytest.raises(_lib.QmmError):
-        _lib.poll_status()
+    for outside in (experts, -1, 1 << 20):                    # an index outside the experts: refused, never followed
+        bad = idx.clone()
+        bad[-1, -1] = outside
+        with pytest.raises(RuntimeError):
+            moe.moe_experts(xs, bad, wts, *packs, **kw)
+    assert torch.equal(moe.moe_experts(xs, idx, wts, *packs, **kw), got) and _lib.poll_status() == 0
 
 
 def test_activations_at_any_address():

@@ -59,7 +59,7 @@ def test_other_threads_run_while_a_call_waits(call, tmp_path):
     loader = importlib.machinery.ExtensionFileLoader("_native", _lib.NATIVE_PATH)
     native = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
     loader.exec_module(native)
-    ours = [ctypes.cast(getattr(_lib.lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul", "qmm_moe_workspace_bytes", "qmm_moe_experts")]
+    ours = [ctypes.cast(getattr(_lib.lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul", "qmm_moe_workspace_bytes", "qmm_moe_experts_checked")]
     x, w, s, b = _operands(m=4, n=128, k=128)
     idx = torch.zeros((4, 1), dtype=torch.int64, device=DEV)
     weights = torch.ones((4, 1), device=DEV)
