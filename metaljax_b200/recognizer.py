@@ -883,10 +883,12 @@ class Interpreter:
         device = args[0].device if args else None
         # What is left of the function once the matched chains are out, with every op's way of running looked up: walking all
         # ops through a hook cost more than launching the few that run (a four-row feed-forward: 22 ops, 6 of them live).
-        if st.plan is None:
-            st.plan = self._plan(st)
+        # (The list is this call's own from here on: another thread's prologue may drop it for a new one at any time.)
+        plan = st.plan
+        if plan is None:
+            plan = st.plan = self._plan(st)
         hook = None
-        for how, op, operands, results in st.plan:
+        for how, op, operands, results in plan:
             if how is not None:
                 outs = how(op, env, *[env[o] for o in operands])
                 for r, t in zip(results, outs):

@@ -362,3 +362,25 @@ def test_both_dimensions_of_the_activation_contracted(monkeypatch):
     assert it.fused_calls == 1
     want = torch.einsum("hd,nhd->n", x.float(), codes.float() * scales.float().repeat_interleave(32, -1))
     assert tuple(got.shape) == (16,) and torch.allclose(got.float(), want, rtol=2e-2, atol=2e-2)
+
+
+def test_a_plan_dropped_while_a_program_runs(monkeypatch):
+    """Another thread's prologue (a weight buffer that changed) drops the list of live ops: a call that is under way keeps its own."""
+    it = recognizer.Interpreter(SHARED_WEIGHT)
+    args = sub_channel_inputs(seed=4)
+    want = it.execute(args)
+    st = it._qmm
+    st.plan = None
+    make = it._plan
+
+    class Dropped(qmm.State):
+        plan = property(lambda self: None, lambda self, value: None)
+
+    dropped = Dropped.__new__(Dropped)
+    for name in qmm.State.__slots__:
+        if name != "plan":
+            setattr(dropped, name, getattr(st, name))
+    monkeypatch.setattr(it, "_qmm", dropped, raising=False)
+    monkeypatch.setattr(it, "_plan", lambda state: make(st), raising=False)
+    for got, w in zip(it.execute(args), want):
+        assert torch.equal(got, w)
