@@ -1049,33 +1049,20 @@ constexpr int most_shares(int bt) { return bt >= 256 ? 8 : 16; }
 // which it shortens by a third of a round more than that, 99.7 / 105.8).
 constexpr int kExchangeBlocks = 32;
 
-// Clusters of `ctas` that fit the device at once. Asked once per kernel and size (with the first call's shared memory: all but all of it
-// either way, one CTA per SM).
+// Clusters of `ctas` that fit the device at once.
 template <typename Kernel>
 int64_t max_clusters(Kernel kernel, int ctas, size_t smem) {
-  static std::atomic<int> known[kMaxDevices][9];
-  const int dev = current_device();
-  std::atomic<int>& n = known[dev][ctas];
-  int have = n.load(std::memory_order_relaxed);
-  if (!have) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = static_cast<unsigned>(ctas);
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&have, kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      have = 0;
-    }
-    if (have < 1) have = -1;
-    n.store(have, std::memory_order_relaxed);
-  }
-  return have;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return max_active_clusters(reinterpret_cast<const void*>(kernel), cfg, ctas);
 }
 
 template <int QK, typename XT, int BT, bool SAME>

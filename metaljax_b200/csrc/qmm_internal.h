@@ -136,6 +136,10 @@ int launch_pack_codes(const uint8_t* codes, uint32_t* out, int64_t rows, int64_t
                       cudaStream_t stream);
 
 #ifdef __CUDACC__
+// Clusters of `ctas` of this launch (kernel, block, dynamic shared memory) that fit the current device at once; 0: none, or not known. Asked of
+// the runtime once per kernel, size and shared memory -- all that the answer depends on --, then looked up.
+int max_active_clusters(const void* kernel, const cudaLaunchConfig_t& cfg, int ctas);
+
 // Launches with programmatic stream serialization: a kernel that begins with griddepcontrol.wait is scheduled while the one
 // before it drains. A failure stays as the last error (check_launch reports it).
 template <typename... Params, typename... Args>

@@ -57,7 +57,6 @@
 
 
 
-#include <mutex>
 #include <type_traits>
 
 #include "qmm_internal.h"
@@ -1072,23 +1071,6 @@ struct RowsShape {
   bool exact;                            // 16-bit activations, results in plain float32 (tiles of kMaxBlocks only)
 };
 
-// Clusters of this shape that fit the device at once (a GPC's SMs do not always divide by the cluster
-// size): more of them than that would be a second wave of persistent CTAs. Asked once per shape.
-template <typename Kernel>
-inline int max_clusters(Kernel kernel, const cudaLaunchConfig_t& cfg, int cluster, int warps, int ring) {
-  static std::mutex mutex;
-  static int known[kMaxDevices][4][kMaxWarps + 1][kMaxRing + 1] = {};
-  const int dev = current_device();
-  const int ci = cluster == 8 ? 3 : cluster == 4 ? 2 : cluster == 2 ? 1 : 0;
-  std::lock_guard<std::mutex> lock(mutex);
-  int& n = known[dev][ci][warps][ring];
-  if (!n && (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1)) {
-    cudaGetLastError();
-    n = 1;
-  }
-  return n;
-}
-
 template <int QK, typename XT, int T, int SPG, int TT, int R, bool EXACT>
 int launch_kernel_of(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool early, cudaStream_t stream) {
   auto kernel = qmm_rows_kernel<QK, XT, T, SPG, TT, R, EXACT>;
@@ -1113,8 +1095,9 @@ int launch_kernel_of(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool e
     attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
     ++cfg.numAttrs;
     cfg.gridDim = dim3(pl.grid);
-    const int most = max_clusters(kernel, cfg, pl.cluster, pl.warps, pl.ring);
-    if (pl.grid > most * pl.cluster) pl.grid = most * pl.cluster;
+    // (a GPC's SMs do not always divide by the cluster size: more clusters than fit at once would be a second wave of persistent CTAs)
+    const int most = max_active_clusters(reinterpret_cast<const void*>(kernel), cfg, pl.cluster);
+    if (pl.grid > most * pl.cluster) pl.grid = most > 0 ? most * pl.cluster : pl.cluster;
   }
   cfg.gridDim = dim3(pl.grid);
   const unsigned clusters = static_cast<unsigned>(pl.grid / pl.cluster);

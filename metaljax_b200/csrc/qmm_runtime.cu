@@ -3,7 +3,9 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <map>
 #include <mutex>
+#include <tuple>
 
 #include "qmm_internal.h"
 
@@ -154,6 +156,24 @@ int device_sm_count() {
     if (n <= 0) n = 148;
     g_sm_count[dev].store(n, std::memory_order_relaxed);
   }
+  return n;
+}
+
+int max_active_clusters(const void* kernel, const cudaLaunchConfig_t& cfg, int ctas) {
+  static std::mutex mutex;
+  static std::map<std::tuple<int, const void*, int, unsigned, size_t>, int> known;
+  const int dev = current_device();
+  if (dev < 0) return 0;
+  const auto key = std::make_tuple(dev, kernel, ctas, cfg.blockDim.x, cfg.dynamicSmemBytes);
+  std::lock_guard<std::mutex> lock(mutex);
+  const auto found = known.find(key);
+  if (found != known.end()) return found->second;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  known[key] = n;
   return n;
 }
 
