@@ -748,6 +748,8 @@ def _pack_dense(packed, scale, zero, k, n, out_dtype):
     g = scale.shape[0]
     if packed.dtype != torch.int8 or packed.shape[1] != -(-n // 2) or any(tuple(t.shape) != (g, n) for t in tables) or n == 0:
         return None
+    if k >= 1 << 24 or n >= 1 << 30:                                        # (the kernels' grids and 32-bit counts)
+        return None
     if k % g or (k // g) % 32 or scale.dtype not in _FLOATS or (zero is not None and zero.dtype not in (*_FLOATS, torch.int8, torch.uint8)):
         return None
     if _SCALE_WIDTH not in ("auto", "source", "f32"):

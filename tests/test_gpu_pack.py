@@ -41,3 +41,13 @@ def test_device_pack_rejects_what_the_host_pack_rejects():
     zero = torch.full((4, 6), 0.5, device=DEV)                # no integer
     with pytest.raises(qmm._Reject):
         qmm.from_keras_int4(packed, scale, zero, columns=6)
+
+
+def test_a_longer_layer_than_the_device_kernels_take():
+    k, n = 1 << 24, 2
+    packed = torch.arange(k, dtype=torch.int64).to(torch.int8)[:, None].contiguous()
+    scale = torch.full((k // 128, n), 0.5)
+    want = qmm.from_keras_int4(packed, scale, columns=n)
+    got = qmm.from_keras_int4(packed.to(DEV), scale.to(DEV), columns=n)
+    assert (got.gs, got.bits) == (want.gs, want.bits)
+    assert torch.equal(got.w.cpu().view(torch.int32), want.w.view(torch.int32)) and torch.equal(got.biases.cpu(), want.biases)
