@@ -630,6 +630,8 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
           if (++s == static_cast<uint32_t>(kStages)) { s = 0; ph ^= 1u; }
         }
       }
+      if (!ok)                                     // gave up: what is on the way lands first (of each place, its last load)
+        for (uint32_t i = 0; i < static_cast<uint32_t>(kStages); ++i) mbar_drain(xfull + 8 * i, i < s ? ph : ph ^ 1u);
     }
   } else if (warp == kWarps - 1) {
     // ---------------- weights and tables (nothing the grid before writes: they need not wait for it) ----------------
@@ -687,11 +689,16 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
         if (++s == p.w_stages) { s = 0; ph ^= 1u; }
       }
     }
+    if (!ok) {
+      cp_async_drain();
+      for (int i = 0; i < p.w_stages; ++i) mbar_drain(wfull + 8 * i, i < s ? ph : ph ^ 1u);
+    }
   } else if (warp == 1) {
     // ---------------- MMA issuer (of a pair: the leader's) ----------------
     if (!kPair || rank == 0) {
       constexpr uint32_t idesc0 = instr_desc(std::is_same<XT, __nv_bfloat16>::value ? 1 : 0, kBF * kCtas);
       uint32_t s = 0, ph = 0, piece = 0;
+      bool issued = false;
       for (; walk.take(&pc, seg_tile0, seg_row0, nseg, ftiles, kBF * kCtas); ++piece) {
         const uint32_t idesc = __shfl_sync(0xffffffffu, idesc0 | (static_cast<uint32_t>(columns() >> 3) << 17), 0);
         const int nkb = __shfl_sync(0xffffffffu, pc.kb_hi - pc.kb_lo, 0);
@@ -707,11 +714,14 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
           tc_mma_block<kPair>(tmem_base, acol, blo, kDescHigh, idesc, j ? 1u : 0u);
           if (kStep == 2 && j + 1 < nkb) tc_mma_block<kPair>(tmem_base, acol + 32, blo + P::kXBlock / 16, kDescHigh, idesc, 1u);
           tc_commit<kPair>(empty + 8 * s, pair_mask);
+          issued = true;
           if (++s == static_cast<uint32_t>(kStages)) { s = 0; ph ^= 1u; }
         }
         if (!__all_sync(0xffffffffu, ok)) break;
         tc_commit<kPair>(d_full, pair_mask);
       }
+      // gave up, or done: the MMAs issued last complete before tensor memory is given back (they complete in order)
+      if (issued) mbar_drain(empty + 8 * (s ? s - 1 : kStages - 1), s ? ph : ph ^ 1u);
     }
   } else {
     // ---------------- dequant + epilogue warps ----------------
@@ -938,6 +948,7 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
         }
       }
     }
+    tmem_wait_st();                                // (of a step that was given up)
     // ragged: rows past the last group are zero
     if (p.group_sizes) {
       const int64_t used = seg_row0[nseg];

@@ -143,6 +143,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   return true;
 }
 
+// For a warp that has given up: waits a little longer (~10 ms) for a phase of a barrier that copies of its own are to complete, so that none of
+// them lands in the shared memory of a CTA that has left.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  uint32_t done = 0;
+  while (!done && clock64() - t0 < 20000000LL)
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+}
+__device__ __forceinline__ void cp_async_drain() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Asynchronous copies of 8 or 4 bytes (of the latter `bytes` are read, the rest is zero) into shared memory, and
 // this thread's arrival on `bar` once all its earlier ones have landed (the barrier's count includes it).
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {

@@ -1074,7 +1074,13 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     for (int64_t i = used + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < all; i += static_cast<int64_t>(gridDim.x) * blockDim.x)
       store_y(p.y, p.y_dtype, i, 0.0f);
   }
-  if (!ok && lane == 0) atomicCAS(p.status, 0, *abort_flag);
+  if (!ok) {                                       // gave up: the boxes on the way land first
+    cp_async_drain();
+    if (lane == 0) {
+      atomicCAS(p.status, 0, *abort_flag);
+      for (uint32_t i = 0; i < static_cast<uint32_t>(p.ring); ++i) mbar_drain(my_full + i * 8, i < slot ? slot_phase ^ 1u : slot_phase);
+    }
+  }
   if (csize > 1) {                                 // nobody leaves while a peer may still write to its shared memory
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
