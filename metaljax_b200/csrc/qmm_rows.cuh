@@ -281,12 +281,11 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   constexpr bool kCentred = EXACT && QK != kMx4;
   constexpr float kCentre = QK == kAff8 ? 128.0f : 8.0f;
   constexpr float kSumIs = kCentred ? 1.0f : -kMagicValue;   // the groups' sums of x are kept times this
-  // Columns: piece i of the tokens of octet q is column group q * kPieces + i, its column c token 8 q + c. With 4 tokens two pieces share
+  // Columns: piece i of the tokens is column group i, its column c token c. With 4 tokens two pieces share
   // a group: column c is token c & 3 of piece 2 h + (c >> 2).
   constexpr int kPieces = std::is_same<XT, float>::value ? 3 : 1;
   constexpr bool kHalf = T == 4;
-  constexpr int Q = 1;                                                // groups of 8 output columns
-  constexpr int NT = kHalf ? (kPieces + 1) / 2 : Q * kPieces;
+  constexpr int NT = kHalf ? (kPieces + 1) / 2 : kPieces;
   constexpr int kBits = QK == kAff8 ? 8 : 4;
   constexpr int kTileRows = kBlockRows * R;
   constexpr int kBoxSmem = kTileRows * kBoxBytes;
@@ -319,9 +318,9 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   // (every access below goes through 32-bit shared addresses)
   const uint32_t ring_at = smem + kHeadBytes + warp * p.ring * kStage;
   const uint32_t tables_at = smem + kHeadBytes + warps * p.ring * kStage + warp * p.ring * (kSlot - kStage);
-  const uint32_t red_at = smem + kHeadBytes + warps * p.ring * kSlot;                           // [bufs][warps][R Q][32] float4
-  const uint32_t xbuf_at = red_at + p.red_bufs * warps * R * Q * 512;                          // [slots][cluster][R Q][32] float4
-  const uint32_t own_at = xbuf_at + (csize > 1 ? kExchangeSlots * csize * R * Q * 512 : 0);
+  const uint32_t red_at = smem + kHeadBytes + warps * p.ring * kSlot;                           // [bufs][warps][R][32] float4
+  const uint32_t xbuf_at = red_at + p.red_bufs * warps * R * 512;                          // [slots][cluster][R][32] float4
+  const uint32_t own_at = xbuf_at + (csize > 1 ? kExchangeSlots * csize * R * 512 : 0);
   const uint32_t sums_at = own_at + warp * sums_bytes(kGroups);                              // [warps] sums of x
   const uint32_t more_x_at = own_at + warps * sums_bytes(kGroups) + warp * more_x_bytes(T) + lane * 16;      // [warps][MMA pairs][32] 16 bytes
   const uint32_t segs_at = own_at + warps * (sums_bytes(kGroups) + more_x_bytes(T));         // grouped: [segs] chunks, [segs + 1] first rows
@@ -531,11 +530,10 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   uint32_t xf[kSliceK / 8];                        // column group 0: two registers per MMA of the slice
   // The bias term sum_g bias[n, g] sum x_g of a slice is an MMA of 16 K slots: bias entries as they are in the table
   // (bf16) against the groups' sums of x, each split into three bf16 pieces (24 bits) that take a slot of their own.
-  [[maybe_unused]] uint32_t bf[Q][kBiasMmas][2];
-  float back[Q][2];                                // what a unit of the scaled activations of output columns 2t, 2t + 1 is worth
-#pragma unroll
-  for (int q = 0; q < Q; ++q) back[q][0] = back[q][1] = 1.0f;
-  [[maybe_unused]] uint32_t least_e[Q];
+  [[maybe_unused]] uint32_t bf[kBiasMmas][2];
+  float back[2];                                   // what a unit of the scaled activations of output columns 2t, 2t + 1 is worth
+  back[0] = back[1] = 1.0f;
+  [[maybe_unused]] uint32_t least_e = 15u;
   auto load_x = [&](const Place& pl, int slice, int sub) {
     int64_t base = 0;
     if (!grouped) {
@@ -550,190 +548,186 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
       base = b * p.x_batch_stride;
     }
     __syncwarp();                                  // (the sums below may still be read)
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const int m = kHalf ? g & 3 : q * 8 + g;
-      const bool live = m < pl.rows_left;
-      int64_t xr = pl.chunk * T + m;
-      if (grouped && live) {
-        xr += seg_row[pl.seg];
-        if (p.x_rows) {
-          xr = p.x_rows[xr];
-          if (xr < 0 || xr >= p.total_x_rows) {
-            if (t == 0) atomicCAS(p.status, 0, QMM_DEVICE_BAD_INDEX);
-            xr = 0;
-          }
+    const int m = kHalf ? g & 3 : g;
+    const bool live = m < pl.rows_left;
+    int64_t xr = pl.chunk * T + m;
+    if (grouped && live) {
+      xr += seg_row[pl.seg];
+      if (p.x_rows) {
+        xr = p.x_rows[xr];
+        if (xr < 0 || xr >= p.total_x_rows) {
+          if (t == 0) atomicCAS(p.status, 0, QMM_DEVICE_BAD_INDEX);
+          xr = 0;
         }
       }
-      const XT* src = reinterpret_cast<const XT*>(p.x) + base + (live ? xr : 0) * p.K;
-      const int k0 = slice * kSliceK + t * kLane;
-      // The lane's c-th eight elements. Where they are looked at twice (scaled) and are the ones that end up in xf,
-      // they wait there as they are: one trip to memory instead of two (8 rows, mxfp4 5760 x 2880: see below).
-      constexpr bool kMayStay = kScaled && sizeof(XT) == 2;
-      const bool stays = kMayStay && q == 0;
-      auto element_of = [&](int c) -> int { return k0 + (c / (kLane / 8)) * kBlk + (c % (kLane / 8)) * 8; };
-      if (stays) {
+    }
+    const XT* src = reinterpret_cast<const XT*>(p.x) + base + (live ? xr : 0) * p.K;
+    const int k0 = slice * kSliceK + t * kLane;
+    // The lane's c-th eight elements. Where they are looked at twice (scaled) and are the ones that end up in xf,
+    // they wait there as they are: one trip to memory instead of two (8 rows, mxfp4 5760 x 2880: see below).
+    constexpr bool kStays = kScaled && sizeof(XT) == 2;
+    auto element_of = [&](int c) -> int { return k0 + (c / (kLane / 8)) * kBlk + (c % (kLane / 8)) * 8; };
+    if constexpr (kStays) {
 #pragma unroll
-        for (int c = 0; c < kSliceK / 32; ++c) {
-          const int k = element_of(c);
-          const uint4 v = live && k < p.K ? __ldg(reinterpret_cast<const uint4*>(src + k)) : make_uint4(0u, 0u, 0u, 0u);
-          xf[c * 4] = v.x; xf[c * 4 + 1] = v.y; xf[c * 4 + 2] = v.z; xf[c * 4 + 3] = v.w;
-        }
-      }
-      auto load8 = [&](int c, float (&f)[8]) {
+      for (int c = 0; c < kSliceK / 32; ++c) {
         const int k = element_of(c);
-        if (stays) {
+        const uint4 v = live && k < p.K ? __ldg(reinterpret_cast<const uint4*>(src + k)) : make_uint4(0u, 0u, 0u, 0u);
+        xf[c * 4] = v.x; xf[c * 4 + 1] = v.y; xf[c * 4 + 2] = v.z; xf[c * 4 + 3] = v.w;
+      }
+    }
+    auto load8 = [&](int c, float (&f)[8]) {
+      const int k = element_of(c);
+      if (kStays) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 w = unpack2<XT>(xf[c * 4 + i]);
+          f[2 * i] = w.x; f[2 * i + 1] = w.y;
+        }
+      } else if (live && k < p.K) {
+        if constexpr (sizeof(XT) == 4) {
+          const float4 a = __ldg(reinterpret_cast<const float4*>(src + k)), b = __ldg(reinterpret_cast<const float4*>(src + k) + 1);
+          f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+        } else {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + k));
+          const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const float2 w = unpack2<XT>(xf[c * 4 + i]);
+            const float2 w = unpack2<XT>(u[i]);
             f[2 * i] = w.x; f[2 * i + 1] = w.y;
           }
-        } else if (live && k < p.K) {
-          if constexpr (sizeof(XT) == 4) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(src + k)), b = __ldg(reinterpret_cast<const float4*>(src + k) + 1);
-            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-          } else {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + k));
-            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float2 w = unpack2<XT>(u[i]);
-              f[2 * i] = w.x; f[2 * i + 1] = w.y;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) f[i] = 0.0f;
         }
-      };
-      float up = 1.0f;
-      [[maybe_unused]] bool infinite = false;      // some row's slice has an infinity in it
-      if constexpr (kScaled) {
-        auto largest = [&](auto finite) -> float {
-          float big = 0.0f;                                            // (a NaN is no larger than anything, and one in any unit)
+      } else {
 #pragma unroll
-          for (int c = 0; c < kSliceK / 32; ++c) {
-            float f[8];
-            load8(c, f);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) big = fmaxf(big, !decltype(finite)::value || fabsf(f[i]) <= kMaxFloat ? fabsf(f[i]) : 0.0f);
-          }
-          big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
-          return fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
-        };
-        float big = largest(std::false_type());
-        if (__any_sync(0xffffffffu, big > kMaxFloat)) {
-          infinite = true;
-          big = largest(std::true_type());
-        }
-        // largest magnitude to [2^14, 2^15); a warp's later slices no finer than its earlier ones, whose sums are brought to their units
-        const uint32_t e = max(__float_as_uint(big) >> 23, sub > 0 ? least_e[q] : 15u);
-        least_e[q] = e;
-        up = __uint_as_float((268u - e) << 23);
-        const float down = __uint_as_float((e - 14u) << 23);
-        back[q][0] = __shfl_sync(0xffffffffu, down, 8 * t);
-        back[q][1] = __shfl_sync(0xffffffffu, down, 8 * t + 4);
+        for (int i = 0; i < 8; ++i) f[i] = 0.0f;
       }
-      [[maybe_unused]] float group_sum[kGroups];
-      // CAREFUL: the second piece of an infinity is nought (it would be a NaN), for its results to be what a sum of products makes of them. (A
-      // comparison for every element costs a scaled row more than what its largest magnitude already tells: 33 rows of float32 against MXFP4,
-      // 4096 x 4096, 98 us with it everywhere, 74 so; 69 without.)
-      auto fragments = [&](auto careful) {
-        float sum = 0.0f;
+    };
+    float up = 1.0f;
+    [[maybe_unused]] bool infinite = false;      // some row's slice has an infinity in it
+    if constexpr (kScaled) {
+      auto largest = [&](auto finite) -> float {
+        float big = 0.0f;                                            // (a NaN is no larger than anything, and one in any unit)
 #pragma unroll
         for (int c = 0; c < kSliceK / 32; ++c) {
           float f[8];
           load8(c, f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            if constexpr (kScaled) f[i] *= up;
-            sum += f[i];
+          for (int i = 0; i < 8; ++i) big = fmaxf(big, !decltype(finite)::value || fabsf(f[i]) <= kMaxFloat ? fabsf(f[i]) : 0.0f);
+        }
+        big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
+        return fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
+      };
+      float big = largest(std::false_type());
+      if (__any_sync(0xffffffffu, big > kMaxFloat)) {
+        infinite = true;
+        big = largest(std::true_type());
+      }
+      // largest magnitude to [2^14, 2^15); a warp's later slices no finer than its earlier ones, whose sums are brought to their units
+      const uint32_t e = max(__float_as_uint(big) >> 23, sub > 0 ? least_e : 15u);
+      least_e = e;
+      up = __uint_as_float((268u - e) << 23);
+      const float down = __uint_as_float((e - 14u) << 23);
+      back[0] = __shfl_sync(0xffffffffu, down, 8 * t);
+      back[1] = __shfl_sync(0xffffffffu, down, 8 * t + 4);
+    }
+    [[maybe_unused]] float group_sum[kGroups];
+    // CAREFUL: the second piece of an infinity is nought (it would be a NaN), for its results to be what a sum of products makes of them. (A
+    // comparison for every element costs a scaled row more than what its largest magnitude already tells: 33 rows of float32 against MXFP4,
+    // 4096 x 4096, 98 us with it everywhere, 74 so; 69 without.)
+    auto fragments = [&](auto careful) {
+      float sum = 0.0f;
+#pragma unroll
+      for (int c = 0; c < kSliceK / 32; ++c) {
+        float f[8];
+        load8(c, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if constexpr (kScaled) f[i] *= up;
+          sum += f[i];
+        }
+        if constexpr (QK != kMx4) {
+          constexpr int kPer = kSliceK / 32 / kGroups;                 // eights per group
+          if (c % kPer == kPer - 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            // (kept as -C sum x where the group's accumulators start there)
+            if (t == 0) sts32(sums_at + ((c / kPer) * 8 + g) * 4, kSumIs * sum);
+            if constexpr (kBiasMma) group_sum[c / kPer] = kHalf && g >= 4 ? 0.0f : sum;
+            sum = 0.0f;
           }
-          if constexpr (QK != kMx4) {
-            constexpr int kPer = kSliceK / 32 / kGroups;                 // eights per group
-            if (c % kPer == kPer - 1) {
-              sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-              sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-              // (kept as -C sum x where the group's accumulators start there)
-              if (t == 0) sts32(sums_at + ((q * kGroups + c / kPer) * 8 + g) * 4, kSumIs * sum);
-              if constexpr (kBiasMma) group_sum[c / kPer] = kHalf && g >= 4 ? 0.0f : sum;
-              sum = 0.0f;
-            }
-          }
+        }
 #pragma unroll
-          for (int i = 0; i < kPieces; ++i) {
-            const int h = kHalf ? i / 2 : q * kPieces + i;
-            const bool here = !kHalf || (g >> 2) == (i & 1);             // (4 tokens: which of the two pieces this lane's column is)
-            uint32_t u[4];
+        for (int i = 0; i < kPieces; ++i) {
+          const int h = kHalf ? i / 2 : i;
+          const bool here = !kHalf || (g >> 2) == (i & 1);             // (4 tokens: which of the two pieces this lane's column is)
+          uint32_t u[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) u[j] = pack2<AT>(f[2 * j], f[2 * j + 1]);
-            if (i + 1 < kPieces) {                                       // what this piece leaves over (exact)
+          for (int j = 0; j < 4; ++j) u[j] = pack2<AT>(f[2 * j], f[2 * j + 1]);
+          if (i + 1 < kPieces) {                                       // what this piece leaves over (exact)
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 got = unpack2<AT>(u[j]);
-                if (decltype(careful)::value && i == 0) {
-                  f[2 * j] = left_of(f[2 * j], got.x); f[2 * j + 1] = left_of(f[2 * j + 1], got.y);
-                } else {
-                  f[2 * j] -= got.x; f[2 * j + 1] -= got.y;
-                }
+            for (int j = 0; j < 4; ++j) {
+              const float2 got = unpack2<AT>(u[j]);
+              if (decltype(careful)::value && i == 0) {
+                f[2 * j] = left_of(f[2 * j], got.x); f[2 * j + 1] = left_of(f[2 * j + 1], got.y);
+              } else {
+                f[2 * j] -= got.x; f[2 * j + 1] -= got.y;
               }
             }
-            if constexpr (QK != kAff8) {                                 // 4-bit codes: (0,4) (1,5) (2,6) (3,7); 8-bit ones in order, (0,1) (2,3)
-              const uint32_t v[4] = {u[0], u[1], u[2], u[3]};
-              u[0] = __byte_perm(v[0], v[2], 0x5410); u[1] = __byte_perm(v[0], v[2], 0x7632);
-              u[2] = __byte_perm(v[1], v[3], 0x5410); u[3] = __byte_perm(v[1], v[3], 0x7632);
-            }
-            if (h == 0) {
+          }
+          if constexpr (QK != kAff8) {                                 // 4-bit codes: (0,4) (1,5) (2,6) (3,7); 8-bit ones in order, (0,1) (2,3)
+            const uint32_t v[4] = {u[0], u[1], u[2], u[3]};
+            u[0] = __byte_perm(v[0], v[2], 0x5410); u[1] = __byte_perm(v[0], v[2], 0x7632);
+            u[2] = __byte_perm(v[1], v[3], 0x5410); u[3] = __byte_perm(v[1], v[3], 0x7632);
+          }
+          if (h == 0) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (!kHalf || i % 2 == 0 || here) xf[c * 4 + j] = u[j];
-            } else {
-              const bool empty = kHalf && !here;                         // (the half of the last group that no piece is left for)
-              sts128(more_x_at + c * 512, __uint_as_float(empty ? 0u : u[0]), __uint_as_float(empty ? 0u : u[1]), __uint_as_float(empty ? 0u : u[2]),
-                     __uint_as_float(empty ? 0u : u[3]));
-            }
+            for (int j = 0; j < 4; ++j)
+              if (!kHalf || i % 2 == 0 || here) xf[c * 4 + j] = u[j];
+          } else {
+            const bool empty = kHalf && !here;                         // (the half of the last group that no piece is left for)
+            sts128(more_x_at + c * 512, __uint_as_float(empty ? 0u : u[0]), __uint_as_float(empty ? 0u : u[1]), __uint_as_float(empty ? 0u : u[2]),
+                   __uint_as_float(empty ? 0u : u[3]));
           }
         }
-      };
-      if constexpr (kPieces == 1 || !kScaled) {
-        fragments(std::bool_constant<(kPieces > 1)>());
-      } else {
-        if (infinite) fragments(std::true_type());
-        else fragments(std::false_type());
       }
-      if constexpr (kBiasMma) {
-        // K slots of the bias MMAs: 16 groups -- one MMA per piece of the sums (lane t: groups 2t, 2t + 1, 2t + 8, 2t + 9);
-        // 8 groups -- (hi | mid) and (lo | 0) with lane t's groups 2t, 2t + 1; 4 groups -- lanes t < 2 (hi | mid), t >= 2 (lo | 0)
-        // with groups 2 (t & 1), 2 (t & 1) + 1
-        auto pick = [&](int first) -> float {        // group_sum[first + 2 t], without indexing registers
-          float v = group_sum[first];
+    };
+    if constexpr (kPieces == 1 || !kScaled) {
+      fragments(std::bool_constant<(kPieces > 1)>());
+    } else {
+      if (infinite) fragments(std::true_type());
+      else fragments(std::false_type());
+    }
+    if constexpr (kBiasMma) {
+      // K slots of the bias MMAs: 16 groups -- one MMA per piece of the sums (lane t: groups 2t, 2t + 1, 2t + 8, 2t + 9);
+      // 8 groups -- (hi | mid) and (lo | 0) with lane t's groups 2t, 2t + 1; 4 groups -- lanes t < 2 (hi | mid), t >= 2 (lo | 0)
+      // with groups 2 (t & 1), 2 (t & 1) + 1
+      auto pick = [&](int first) -> float {        // group_sum[first + 2 t], without indexing registers
+        float v = group_sum[first];
 #pragma unroll
-          for (int i = 1; i < (kGroups == 4 ? 2 : 4); ++i)
-            if ((kGroups == 4 ? t & 1 : t) == i) v = group_sum[first + 2 * i];
-          return v;
-        };
-        using B16 = __nv_bfloat16;
-        auto split = [&](float a, float b, uint32_t (&piece)[3]) {
-          piece[0] = pack2<B16>(a, b);
-          const float2 f0 = unpack2<B16>(piece[0]);
-          const float a1 = left_of(a, f0.x), b1 = left_of(b, f0.y);
-          piece[1] = pack2<B16>(a1, b1);
-          const float2 f1 = unpack2<B16>(piece[1]);
-          piece[2] = pack2<B16>(a1 - f1.x, b1 - f1.y);
-        };
-        uint32_t lower[3];
-        split(pick(0), pick(1), lower);
-        if constexpr (kGroups == 16) {
-          uint32_t upper[3];
-          split(pick(8), pick(9), upper);
+        for (int i = 1; i < (kGroups == 4 ? 2 : 4); ++i)
+          if ((kGroups == 4 ? t & 1 : t) == i) v = group_sum[first + 2 * i];
+        return v;
+      };
+      using B16 = __nv_bfloat16;
+      auto split = [&](float a, float b, uint32_t (&piece)[3]) {
+        piece[0] = pack2<B16>(a, b);
+        const float2 f0 = unpack2<B16>(piece[0]);
+        const float a1 = left_of(a, f0.x), b1 = left_of(b, f0.y);
+        piece[1] = pack2<B16>(a1, b1);
+        const float2 f1 = unpack2<B16>(piece[1]);
+        piece[2] = pack2<B16>(a1 - f1.x, b1 - f1.y);
+      };
+      uint32_t lower[3];
+      split(pick(0), pick(1), lower);
+      if constexpr (kGroups == 16) {
+        uint32_t upper[3];
+        split(pick(8), pick(9), upper);
 #pragma unroll
-          for (int i = 0; i < 3; ++i) { bf[q][i][0] = lower[i]; bf[q][i][1] = upper[i]; }
-        } else if constexpr (kGroups == 8) {
-          bf[q][0][0] = lower[0]; bf[q][0][1] = lower[1];
-          bf[q][kBiasMmas - 1][0] = lower[2]; bf[q][kBiasMmas - 1][1] = 0u;
-        } else {
-          bf[q][0][0] = t < 2 ? lower[0] : lower[2]; bf[q][0][1] = t < 2 ? lower[1] : 0u;
-        }
+        for (int i = 0; i < 3; ++i) { bf[i][0] = lower[i]; bf[i][1] = upper[i]; }
+      } else if constexpr (kGroups == 8) {
+        bf[0][0] = lower[0]; bf[0][1] = lower[1];
+        bf[kBiasMmas - 1][0] = lower[2]; bf[kBiasMmas - 1][1] = 0u;
+      } else {
+        bf[0][0] = t < 2 ? lower[0] : lower[2]; bf[0][1] = t < 2 ? lower[1] : 0u;
       }
     }
     __syncwarp();
@@ -754,17 +748,17 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   uint32_t done_buf = 0, done_phase = 0;
   auto add_up = [&]() -> bool {
     // ---- the warps' shares, in warp order ----
-    const uint32_t shares = red_at + done_buf * warps * (R * Q * 512) + lane * 16;
+    const uint32_t shares = red_at + done_buf * warps * (R * 512) + lane * 16;
     if (!mbar_wait(smem + kRedFullAt + done_buf * 8, done_phase, abort_at, 13)) return false;
     __syncwarp();
-    float v[R * Q][4];
+    float v[R][4];
 #pragma unroll
-    for (int h = 0; h < R * Q; ++h) v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0.0f;
+    for (int h = 0; h < R; ++h) v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0.0f;
 #pragma unroll 4
     for (int i = 0; i < warps; ++i)
 #pragma unroll
-      for (int h = 0; h < R * Q; ++h) {
-        const float4 f = ldsf128<0>(shares + (i * R * Q + h) * 512);
+      for (int h = 0; h < R; ++h) {
+        const float4 f = ldsf128<0>(shares + (i * R + h) * 512);
         v[h][0] += f.x; v[h][1] += f.y; v[h][2] += f.z; v[h][3] += f.w;
       }
     __syncwarp();
@@ -774,27 +768,27 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
       // ---- the CTAs' sums meet at the tile's leader (in turn; `lap` counts its tiles), in rank order ----
       const int xs = lap % kExchangeSlots;
       const uint32_t xphase = static_cast<uint32_t>(lap / kExchangeSlots) & 1u;
-      const uint32_t xslot = xbuf_at + xs * csize * (R * Q * 512) + lane * 16;
+      const uint32_t xslot = xbuf_at + xs * csize * (R * 512) + lane * 16;
       mine = leader == rank;
       if (!mine) {
         if (!mbar_wait_cluster(smem + kXFreeAt + (leader * kExchangeSlots + xs) * 8, xphase ^ 1u, abort_at, 14)) return false;
         __syncwarp();
-        const uint32_t bar = remote(smem + kXFullAt + xs * 8, leader), to = remote(xslot + rank * (R * Q * 512), leader);
+        const uint32_t bar = remote(smem + kXFullAt + xs * 8, leader), to = remote(xslot + rank * (R * 512), leader);
 #pragma unroll
-        for (int h = 0; h < R * Q; ++h) st_async4(to + h * 512, bar, v[h]);
+        for (int h = 0; h < R; ++h) st_async4(to + h * 512, bar, v[h]);
       } else {
-        if (lane == 0) mbar_expect_tx(smem + kXFullAt + xs * 8, (csize - 1) * R * Q * 512);
+        if (lane == 0) mbar_expect_tx(smem + kXFullAt + xs * 8, (csize - 1) * R * 512);
         if (!mbar_wait_cluster(smem + kXFullAt + xs * 8, xphase, abort_at, 15)) return false;
         __syncwarp();
 #pragma unroll
-        for (int h = 0; h < R * Q; ++h) {
-          sts128(xslot + rank * (R * Q * 512) + h * 512, v[h][0], v[h][1], v[h][2], v[h][3]);
+        for (int h = 0; h < R; ++h) {
+          sts128(xslot + rank * (R * 512) + h * 512, v[h][0], v[h][1], v[h][2], v[h][3]);
           v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0.0f;
         }
         for (int r = 0; r < csize; ++r)
 #pragma unroll
-          for (int h = 0; h < R * Q; ++h) {
-            const float4 f = ldsf128<0>(xslot + (r * R * Q + h) * 512);
+          for (int h = 0; h < R; ++h) {
+            const float4 f = ldsf128<0>(xslot + (r * R + h) * 512);
             v[h][0] += f.x; v[h][1] += f.y; v[h][2] += f.z; v[h][3] += f.w;
           }
         __syncwarp();
@@ -807,23 +801,19 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
 #pragma unroll
       for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int col = q * 8 + 2 * t + (i & 1), n = done_tile * kTileRows + r * kBlockRows + rho + (i >> 1) * 8;
-            if (col < rows_left && col < T && n < p.N) store_y(p.y, p.y_dtype, y0 + static_cast<int64_t>(col) * p.N + n, v[r * Q + q][i]);
-          }
+        for (int i = 0; i < 4; ++i) {
+          const int col = 2 * t + (i & 1), n = done_tile * kTileRows + r * kBlockRows + rho + (i >> 1) * 8;
+          if (col < rows_left && col < T && n < p.N) store_y(p.y, p.y_dtype, y0 + static_cast<int64_t>(col) * p.N + n, v[r][i]);
+        }
     }
     return true;
   };
   bool ok = true, stale = true;
   float y[R][NT][4];                               // per column group: sums of scale * codes * digits
-  [[maybe_unused]] float yb[R][Q][4];              // ... and, where it is no MMA, the bias term per output column
+  [[maybe_unused]] float yb[R][4];                 // ... and, where it is no MMA, the bias term per output column
   while (left > 0) {
     if (stale) {
-      float unit[Q][2];
-#pragma unroll
-      for (int q = 0; q < Q; ++q) { unit[q][0] = back[q][0]; unit[q][1] = back[q][1]; }
+      const float unit[2] = {back[0], back[1]};
       load_x(place[which], first_slice + sub, sub);
       if (kScaled && sub > 0) {                    // the sums so far in the new slice's units (a power of two)
 #pragma unroll
@@ -833,13 +823,11 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
 #pragma unroll
             for (int h = 0; h < NT; ++h) {
               // (with 4 tokens the upper lanes' columns are the lower lanes' tokens)
-              float u0 = unit[kHalf ? 0 : h / kPieces][i & 1] / back[kHalf ? 0 : h / kPieces][i & 1];
+              float u0 = unit[i & 1] / back[i & 1];
               if (kHalf) u0 = __shfl_sync(0xffffffffu, u0, lane & ~2);
               y[r][h][i] *= u0;
             }
-            if constexpr (QK != kMx4)
-#pragma unroll
-              for (int q = 0; q < Q; ++q) yb[r][q][i] *= unit[q][i & 1] / back[q][i & 1];
+            if constexpr (QK != kMx4) yb[r][i] *= unit[i & 1] / back[i & 1];
           }
       }
       stale = p.slices_per_warp > 1;
@@ -849,8 +837,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
       for (int r = 0; r < R; ++r) {
 #pragma unroll
         for (int h = 0; h < NT; ++h) y[r][h][0] = y[r][h][1] = y[r][h][2] = y[r][h][3] = 0.0f;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) yb[r][q][0] = yb[r][q][1] = yb[r][q][2] = yb[r][q][3] = 0.0f;
+        yb[r][0] = yb[r][1] = yb[r][2] = yb[r][3] = 0.0f;
       }
     }
     // where this warp goes next
@@ -891,23 +878,17 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
         uint32_t a[4] = {b0, b1, b0, b1};
         if constexpr (kGroups == 16) { a[2] = lds32<kAt + 16>(at); a[3] = lds32<kAt + 8 * kPitch + 16>(at); }
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-#pragma unroll
-          for (int i = 0; i < kBiasMmas; ++i) Mma<__nv_bfloat16>::run(yb[r][q], a, bf[q][i][0], bf[q][i][1]);
+        for (int i = 0; i < kBiasMmas; ++i) Mma<__nv_bfloat16>::run(yb[r], a, bf[i][0], bf[i][1]);
       });
     }
     static_for<kGroups>([&](auto gc) {
       constexpr int gi = decltype(gc)::value;
       float acc[R][NT][4];
-      float start[Q][2];                           // kSumIs * sum x of the group
-#pragma unroll
-      for (int q = 0; q < Q; ++q) start[q][0] = start[q][1] = 0.0f;
-      if constexpr (QK != kMx4)
-        static_for<Q>([&](auto qc) {
-          constexpr int q = decltype(qc)::value;
-          const uint2 sr = lds64<(q * kGroups + gi) * 32>(scol);
-          start[q][0] = __uint_as_float(sr.x); start[q][1] = __uint_as_float(sr.y);
-        });
+      float start[2] = {0.0f, 0.0f};               // kSumIs * sum x of the group
+      if constexpr (QK != kMx4) {
+        const uint2 sr = lds64<gi * 32>(scol);
+        start[0] = __uint_as_float(sr.x); start[1] = __uint_as_float(sr.y);
+      }
       static_for<kBlocksPerGroup>([&](auto bc) {
         constexpr int jj = decltype(bc)::value, j = gi * kBlocksPerGroup + jj;      // block of the slice
         constexpr int kLaneWords = kLane * kBits / 32;
@@ -963,8 +944,8 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
 #pragma unroll
             for (int h = 0; h < NT; ++h) {
               if constexpr (jj == 0 && mi == 0)     // (what keeps the magic number has one piece)
-                Mma<AT>::first(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1], kCentred ? 0.0f : start[0][0],
-                               kCentred ? 0.0f : start[0][1]);
+                Mma<AT>::first(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1], kCentred ? 0.0f : start[0],
+                               kCentred ? 0.0f : start[1]);
               else
                 Mma<AT>::run(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1]);
             }
@@ -996,11 +977,8 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
           } else {
             b0 *= 1.0f / kSumIs; b1 *= 1.0f / kSumIs;
           }
-#pragma unroll
-          for (int q = 0; q < Q; ++q) {
-            fma2(yb[r][q][0], yb[r][q][1], b0, start[q][0], start[q][1]);
-            fma2(yb[r][q][2], yb[r][q][3], b1, start[q][0], start[q][1]);
-          }
+          fma2(yb[r][0], yb[r][1], b0, start[0], start[1]);
+          fma2(yb[r][2], yb[r][3], b1, start[0], start[1]);
         }
       });
     });
@@ -1017,30 +995,20 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     // ---- this warp's share of the tile ----
     if (!(ok = mbar_wait(smem + kRedEmptyAt + buf * 8, buf_phase ^ 1u, abort_at, 12))) break;
     // the pieces of a column together, the bias term, the scale
-    const uint32_t rbuf = red_at + (buf * warps + warp) * (R * Q * 512) + lane * 16;
+    const uint32_t rbuf = red_at + (buf * warps + warp) * (R * 512) + lane * 16;
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+    for (int r = 0; r < R; ++r) {
+      float v[4];
 #pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        float v[4];
+      for (int i = 0; i < 4; ++i) {
+        float s = y[r][NT - 1][i];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if constexpr (kHalf) {
-            float s = y[r][NT - 1][i];
-#pragma unroll
-            for (int h = NT - 2; h >= 0; --h) s += y[r][h][i];
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            v[i] = s;
-          } else {
-            float s = y[r][q * kPieces + kPieces - 1][i];
-#pragma unroll
-            for (int h = kPieces - 2; h >= 0; --h) s += y[r][q * kPieces + h][i];
-            v[i] = s;
-          }
-          v[i] = fmaf(v[i], kUnit, yb[r][q][i]) * back[q][i & 1];
-        }
-        sts128(rbuf + (r * Q + q) * 512, v[0], v[1], v[2], v[3]);
+        for (int h = NT - 2; h >= 0; --h) s += y[r][h][i];
+        if constexpr (kHalf) s += __shfl_xor_sync(0xffffffffu, s, 2);
+        v[i] = fmaf(s, kUnit, yb[r][i]) * back[i & 1];
       }
+      sts128(rbuf + r * 512, v[0], v[1], v[2], v[3]);
+    }
     __syncwarp();
     if (lane == 0) mbar_arrive(smem + kRedFullAt + buf * 8);
     // the tile before this one: its shares have all been written by now, or nearly (adding up this very tile would make each adder wait
