@@ -1,5 +1,6 @@
-"""The expert block in one native call against its steps one by one, at the edges of the pair sort (one pair, experts
-without a pair, more pairs than a warp, more than a block's warps) and on either product kernel. Needs a B200."""
+"""The expert block in one native call against its steps one by one and against the oracle's product pair by pair, at the edges of
+the pair sort (one pair, experts without a pair, more pairs than a warp, more than a block's warps) and on either product
+kernel. Needs a B200."""
 
 import numpy as np
 import pytest
@@ -20,21 +21,38 @@ def _case(rng, kind, n, k, tdt, lead):
     return affine_case(rng, n, k, 64, 4, tdt, lead=lead)[1:], dict(group_size=64, bits=4)
 
 
+def _exact_block(xs, idx, wts, packs, gs, mode):
+    """The block in float64 on the dequantized weights, nothing rounded in between."""
+    w1, w3, w2 = (O.dequantize(w, s, b, gs, 4, mode).astype(np.float64) for w, s, b in packs)
+    out = np.zeros((len(xs), w2.shape[1]))
+    for t, x in enumerate(xs.astype(np.float64)):
+        for e, weight in zip(idx[t], wts[t].astype(np.float64)):
+            gate = w1[e] @ x
+            out[t] += weight * (w2[e] @ (gate / (1.0 + np.exp(-gate)) * (w3[e] @ x)))
+    return out
+
+
 @pytest.mark.parametrize("tokens,experts,k", [(1, 4, 1), (3, 8, 2), (33, 40, 4), (150, 4, 2)])
 @pytest.mark.parametrize("kind,x,index", [("int4", "bf16", torch.int64), ("mxfp4", "f16", torch.int32)])
 def test_expert_block_in_one_call(kind, x, index, tokens, experts, k):
     """Against the block's steps one by one: the same kernels on either side of the same 16-bit hand-offs, so
-    what differs is the order of float32 sums (a chunk of rows may be another width) and what 8 bits make of that: the parity gate."""
+    what differs is the order of float32 sums (a chunk of rows may be another width) and what 8 bits make of that: the parity gate. And against
+    float64: gate, up, SwiGLU (twice) and down are rounded to 16 bits, five independent errors of 2^-9 a value of which
+    the down projection averages four over 320 terms: the parity gate again."""
     rng = np.random.default_rng(tokens + experts)
     d, f = 192, 320
-    packs, kw = [], None
+    packs, host, kw = [], [], None
     for n, kk in ((f, d), (f, d), (d, f)):
         arrays, kw = _case(rng, kind, n, kk, x, lead=(experts,))
+        host.append(arrays)
         packs.append(tuple(None if a is None else to_torch(a, DEV) for a in arrays))
-    xs = to_torch(activations(rng, (tokens, d), x, 0.5), DEV)
+    xs_host = activations(rng, (tokens, d), x, 0.5)
+    xs = to_torch(xs_host, DEV)
     idx = torch.from_numpy(np.stack([rng.permutation(experts)[:k] for _ in range(tokens)])).to(index).to(DEV)
     wts = torch.from_numpy(rng.random((tokens, k)).astype(np.float32)).to(DEV)
     got = moe.moe_experts(xs, idx, wts, *packs, **kw)
+    exact = _exact_block(xs_host, idx.cpu().numpy(), wts.cpu().numpy(), host, kw["group_size"], kw.get("mode", "affine"))
+    assert O.rel_err(to_numpy(got).astype(np.float32), exact) <= 1e-2
     order, tok, sizes = moe.sort_pairs(idx.to(torch.int64), experts)
     rows = xs.index_select(0, tok)
     act = moe.silu_mul(moe.ragged_dot(rows, *packs[0], sizes, **kw), moe.ragged_dot(rows, *packs[1], sizes, **kw))
