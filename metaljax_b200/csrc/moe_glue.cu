@@ -50,7 +50,6 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // the product to T.
 template <typename T>
 __global__ void silu_mul_kernel(const uint4* gate, const uint4* up, uint4* out,   // (out may be gate)
-                               
                                 int64_t pieces) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -34,9 +34,9 @@
 // the first that it makes, and waits only on lower-numbered workers, which were scheduled before it.
 //
 // Measured (device time, before: one CTA per tile at every width, 32-byte boxes, tables from global memory, an issuer behind a branch, split
-// products added up by a second kernel), int4 group 64: 2048 rows 14336 x 4096 248 -> 189 us, 4096 x 14336 219 -> 174; 512 rows 28672 x 4096
-// 130 -> 100; 64 rows 28672 x 4096 59.7 -> 37.8, 4096 x 4096 16.4 -> 10.8, 4096 x 14336 31.2 -> 20.9; 128 rows 4096 x 14336 47 -> 22; 8-bit
-// group 128, 45 rows 14336 x 4096 33 -> 25. What bounds it: at 64 rows the dequantizing warps (400 clocks a K block and SM: some 300 instructions a
+// products added up by a second kernel), int4 group 64: 2048 rows 14336 x 4096 248 -> 181..189 us (the clock under load decides), 4096 x 14336
+// 219 -> 167..174; 512 rows 28672 x 4096 130 -> 97; 64 rows 28672 x 4096 59.7 -> 33.1, 4096 x 4096 16.4 -> 10.5, 4096 x 14336 31.2 -> 19.4; 128 rows
+// 4096 x 14336 47 -> 21; 8-bit group 128, 45 rows 14336 x 4096 33 -> 20.6. What bounds it: at 64 rows the dequantizing warps (400 clocks a K block and SM: some 300 instructions a
 // warp and block at four warps a scheduler), at 256 the tensor cores (500 clocks a block between a tile's ends, under the power cap) and the ends,
 // where the accumulator is drained by the warps that would dequantize for the next tile. (Draining it after the first steps of the next
 // tile was built: the state that lives across the epilogue then spills, and every size lost.)

@@ -28,12 +28,19 @@ size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
          (pl.cluster > 1 ? kExchangeSlots * pl.cluster * shares : 0) + (segs ? (2 * static_cast<size_t>(segs) + 1) * 4 : 0);
 }
 
-// How K and the tiles are shared out. An SM's time is the slices it works through, so the plan with the fewest
-// slices on the busiest SM wins: tiles per cluster x warps per CTA x CTAs per SM (a tile's fixed costs count
-// as half a slice of 32 rows per warp, meeting in a cluster as two slices). More CTAs per tile (a larger cluster) is
-// what fills the machine when a weight has few tiles, and what keeps K within 8 warps x 512 codes of registers when K is
-// long. Tiles of one block cost more per row, but an SM that has one tile or two waits less for them (8 rows, mxfp4
-// 5760 x 2880: 2.4 tiles of 16 rows per SM instead of 1.2 -> 2 of 32).
+// How K and the tiles are shared out: the plan of the least load. The load stands for the time of the busiest SM, in slices of 32
+// rows that one warp works through: tiles per cluster x warps resident on the SM (at least 6: fewer leave it waiting for memory) x
+// what a tile costs a warp -- its slices (half as much where a tile is one block of 16 rows), plus what it costs besides its codes,
+// half a slice for 32 rows and 0.35 for 16 (barriers and addresses are per tile, not per row), 0.05 more in a cluster -- and 4 for the
+// cluster's meeting at the start and the end. More CTAs per tile (a larger cluster) is what keeps K within 8 warps x 512 codes of
+// registers when K is long, and what fills the machine when a weight has few tiles; more than one slice per warp reloads the
+// activations with every tile and is left for where nothing else fits. Tiles of one block cost more per row, but an SM that has one tile
+// or two waits less for them (8 rows, mxfp4 5760 x 2880: 2.4 tiles of 16 rows per SM instead of 1.2 -> 2 of 32).
+//
+// The constants were fitted to measured times; what they pick against the best of all plans, us: 8 rows 28672 x 4096 20.1 / 20.1 (the
+// next best 22.0, a cluster of two), 128256 x 4096 65.6 / 65.6 (73.0), 4096 x 14336 16.0 / 16.0 (17.0), 4096 x 4096 7.1 / 7.1 (7.6), 1024 x 1024 5.9 / 5.9,
+// 16 rows 4096 x 4096 8.6 / 8.6 (9.3), 4 rows 5632 x 2048 6.1 / 6.1 (6.6), 2048 x 5632 7.8 / 7.8, 8-bit 8 rows 14336 x 4096 14.6 / 14.6 (15.2),
+// mxfp4 8 rows 5760 x 2880 8.9 / 8.7, float32 33 rows 4096 x 4096 34.8 / 33.2.
 RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh, int segs) {
   const int sms = device_sm_count();
   RowsPlan best = {};

@@ -33,17 +33,17 @@
 // subnormals need neither the magic nor the subtraction, but are aligned as if they had all their bits.)
 // Relative error against float64 (2-norm, the largest over K 512 to 14336 and all group sizes) of the SIMT kernel / with the magic number / so, for N(0, 1),
 // one sign, outliers of 300: 4-bit 3.8e-7 / 4.9e-6 / 1.1e-7, 6.0e-7 / 1.3e-5 / 0.7e-7, 4.5e-7 / 1.1e-5 / 1.1e-7; 8-bit 2.6e-7 / 3.5e-6 / 1.4e-7,
-// 6.8e-7 / 2.2e-4 / 1.3e-7, 3.7e-7 / 5.4e-6 / 3.0e-7. 33 rows of 4096 x 4096: 34.8 us with the magic number, 35.6 so.
+// 6.8e-7 / 2.2e-4 / 1.3e-7, 3.7e-7 / 5.4e-6 / 3.0e-7. 33 rows of 4096 x 4096: 34.8 us with the magic number, 34.5 so; 8-bit 43 and 47.
 // Range: an infinite activation makes its row's results infinite or NaN, as a sum of products does (affine codes: NaN where s (q - C) x and
 // the bias term have opposite signs); finite ones up to 2^120 give finite results where those fit. 4-bit codes take float32
 // activations below 2^-110 with fewer than 24 bits.
 // (8-bit float MMAs would take the codes with a third of the instructions, but `mma.sync` on e4m3 is emulated here with
 // conversions to f16: 88 against 67 us for 8 rows of 128256 x 4096.)
 //
-// Measured (device time, weights from HBM; before: the kernel that dequantized in registers and staged its
-// activations in shared memory; float32: the SIMT kernel), int4 group 64: 8 rows 28672 x 4096 27.1 -> 21.4 us (3.1 TB/s), 128256 x 4096
-// 99.5 -> 66.6 (4.4 TB/s), 4096 x 14336 26.8 -> 16.8, 16 rows 128256 x 4096 170 -> 128, 16 rows 4096 x 4096 12.2 -> 9.2; 8-bit 14336 x 4096 22.6
-// -> 15.5 (3.9 TB/s); float32 33 rows 4096 x 4096 323 -> 36. At the small end (2 rows 4096 x 4096 6.3 -> 7.1 us) it is the chain launch, activations,
+// Measured (device time, weights from HBM; before: a kernel with the same fragments under the same kind of magic
+// number that read its activations from shared memory for every tile and staged each tile's tables there behind barriers of the CTA; float32: the SIMT kernel), int4 group 64: 8 rows 28672 x 4096 27.1 -> 20.2 us (3.3 TB/s), 128256 x 4096
+// 99.5 -> 65.6 (4.5 TB/s), 4096 x 14336 26.8 -> 16.8, 16 rows 128256 x 4096 170 -> 128, 16 rows 4096 x 4096 12.2 -> 9.2; 8-bit 14336 x 4096 22.6
+// -> 15.5 (3.9 TB/s); float32 33 rows 4096 x 4096 323 -> 34.5. At the small end (2 rows 4096 x 4096 6.3 -> 7.1 us) it is the chain launch, activations,
 // one tile, sum that counts, not a stream.
 //
 // Every wait on an mbarrier is bounded. The kernel is launched with programmatic stream
@@ -54,8 +54,6 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
-
-
 
 #include <type_traits>
 
