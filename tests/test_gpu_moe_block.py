@@ -2,6 +2,8 @@
 the pair sort (one pair, experts without a pair, more pairs than a warp, more than a block's warps) and on either product
 kernel. Needs a B200."""
 
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -81,3 +83,61 @@ def test_activations_at_any_address():
     wts = torch.rand((t, 2), device=DEV)
     got, want = moe.moe_experts(x, idx, wts, *packs, **kw), moe.moe_experts(x.clone(), idx, wts, *packs, **kw)
     assert O.rel_err(to_numpy(got).astype(np.float32), to_numpy(want).astype(np.float64)) <= 1e-2
+
+
+def _small_block(t=6, experts=4, d=192, f=320):
+    rng = np.random.default_rng(9)
+    packs = []
+    for n, kk in ((f, d), (f, d), (d, f)):
+        arrays, kw = _case(rng, "int4", n, kk, "bf16", lead=(experts,))
+        packs.append(tuple(to_torch(a, DEV) for a in arrays))
+    x = to_torch(activations(rng, (t, d), "bf16", 0.5), DEV)
+    idx = torch.from_numpy(rng.integers(0, experts, (t, 2))).to(DEV)
+    return x, idx, torch.rand((t, 2), device=DEV), packs, kw
+
+
+def test_captured_block():
+    """In a graph nothing can be looked at by the host: a replay computes, and an index out of range is reported by the status."""
+    x, idx, wts, packs, kw = _small_block()
+    want = moe.moe_experts(x, idx, wts, *packs, **kw)
+    index, stream = idx.clone(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = moe.moe_experts(x, index, wts, *packs, **kw)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and _lib.poll_status() == 0
+    index[0, 0] = 4
+    graph.replay()
+    with pytest.raises(_lib.QmmError):
+        _lib.poll_status()
+
+
+def test_blocks_of_several_threads():
+    """Every call waits for the report of its own sort: one thread's indices are out of range, and it alone is refused."""
+    x, idx, wts, packs, kw = _small_block()
+    want = moe.moe_experts(x, idx, wts, *packs, **kw)
+    bad = idx.clone()
+    bad[3, 1] = -7
+    torch.cuda.synchronize()
+    outcome = {}
+
+    def calls(number):
+        refused, right = 0, 0
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(25):
+                try:
+                    y = moe.moe_experts(x, bad if number == 2 else idx, wts, *packs, **kw)
+                    torch.cuda.current_stream().synchronize()
+                    right += bool(torch.equal(y, want))
+                except _lib.QmmError:
+                    refused += 1
+        outcome[number] = (refused, right)
+
+    threads = [threading.Thread(target=calls, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert outcome == {0: (0, 25), 1: (0, 25), 2: (25, 0), 3: (0, 25)} and _lib.poll_status() == 0
