@@ -15,8 +15,8 @@
 // dequantizes its own 128 features and holds half of the tokens' activations, so an SM reads 16 KB of activations per 64 K
 // instead of 32: a lone CTA's 36 KB per 64 K were what L2 could not deliver (42 bytes a clock and SM at 974 TFLOP/s).
 //
-// Scales and biases of a box travel with it (cp.async by the weights' producer, a few bytes a row): read by the dequantizing
-// threads from global memory, 2 bytes per row and 64 K, they thrashed what is left of L1 next to 200 KB of shared memory, and their
+// Scales and biases travel with the boxes, 32 bytes of a table row at a time (cp.async by the weights' producer, two lanes to a row): read by the
+// dequantizing threads from global memory they thrashed what is left of L1 next to 200 KB of shared memory, and their
 // latency was the dequantization's. Packed weights come in boxes of 128 rows x 128 bytes (256 4-bit K-elements, 128 8-bit ones, 64 float ones) through a
 // ring of their own: a box of 32 bytes a row for 64 4-bit elements costs the TMA unit and L2 a request per 32 bytes.
 //
@@ -36,7 +36,9 @@
 // Measured (device time, before: one CTA per tile at every width, 32-byte boxes, tables from global memory, an issuer behind a branch, split
 // products added up by a second kernel), int4 group 64: 2048 rows 14336 x 4096 248 -> 181..189 us (the clock under load decides), 4096 x 14336
 // 219 -> 167..174; 512 rows 28672 x 4096 130 -> 97; 64 rows 28672 x 4096 59.7 -> 33.1, 4096 x 4096 16.4 -> 10.5, 4096 x 14336 31.2 -> 19.4; 128 rows
-// 4096 x 14336 47 -> 21; 8-bit group 128, 45 rows 14336 x 4096 33 -> 20.6. What bounds it: at 64 rows the dequantizing warps (400 clocks a K block and SM: some 300 instructions a
+// 4096 x 14336 47 -> 21; 8-bit group 128, 45 rows 14336 x 4096 33 -> 20.6. Table entries a sector of a row at a time instead of the 8 bytes of
+// every box (a row a lane: 32 lines an instruction; without the dequantization 64 rows then took 345 clocks a K block and SM, 204 without those copies):
+// 64 rows 28672 x 4096 33.3 -> 30.6, 65760 x 2880 (rows of 90 table bytes) 79.3 -> 48.7, float32 tables in groups of 32 14336 x 4096 42 -> 33. What bounds it: at 64 rows the dequantizing warps (400 clocks a K block and SM: some 300 instructions a
 // warp and block at four warps a scheduler), at 256 the tensor cores (500 clocks a block between a tile's ends, under the power cap) and the ends,
 // where the accumulator is drained by the warps that would dequantize for the next tile. (Draining it after the first steps of the next
 // tile was built: the state that lives across the epilogue then spills, and every size lost.)
@@ -66,6 +68,8 @@ constexpr int kWarps = 3 + kDequantWarps;
 constexpr int kThreads = kWarps * 32;
 constexpr int kMaxSegments = 256;
 constexpr int kBoxBytes = 128;  // bytes of a weight row in a box
+constexpr int kChunkBytes = 32; // bytes of a table row in a chunk: a sector of memory ...
+constexpr int kTablePitch = 48; // ... and in shared memory, where they keep their distance from a 16-byte boundary
 
 enum { kAff4 = 0, kAff8 = 1, kMx4 = 2, kFloat = 3 };    // kFloat: the weight holds values of the activation type (nothing to dequantize)
 
@@ -79,9 +83,9 @@ struct TcParams {
   int64_t N;
   int64_t w_seg_rows;          // rows of the packed weight between segments (N, or 0 = shared)
   int K, segments, group_shift, table_dtype, y_dtype;
-  int w_stages;                // places of the weight ring, and of the ring of table chunks
-  unsigned w_inverse;          // 2^32 / w_stages rounded up: counts are divided by a multiplication
-  int table_entry, table_pitch, table_unit;   // bytes of a table entry; of a row's entries in shared memory; on which every chunk's entries start (8, 4 or less)
+  int w_stages, t_stages;      // places of the weight ring, and of the ring of table chunks
+  unsigned w_inverse, t_inverse;              // 2^32 / w_stages and t_stages, rounded up: counts are divided by a multiplication
+  int table_entry, skewed;     // bytes of a table entry; whether some chunk's entries start off a 16-byte boundary
   int chunk_shift;             // weight boxes per table chunk (log2)
   int64_t table_bytes;         // of a whole table
   int split;                   // > 1: `split` consecutive workers share the K of each tile (and the walk is one tile long): a cluster that
@@ -637,15 +641,13 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
     // ---------------- weights and tables (nothing the grid before writes: they need not wait for it) ----------------
     const int groups = QK == kFloat ? 1 : p.K >> p.group_shift;
     int s = 0;
-    [[maybe_unused]] int ts = 0;
+    [[maybe_unused]] int ts = -1;                  // place of the chunk that is being read
+    [[maybe_unused]] uint32_t issued = 0, chunks = 0, last_box = 0;    // boxes and chunks so far; (lane i) the last box of the chunk in place i
     uint32_t ph = 0;
     bool ok = true;
     while (ok && walk.take(&pc, seg_tile0, seg_row0, nseg, ftiles, kBF * kCtas)) {
       const int row = static_cast<int>(pc.seg * p.w_seg_rows + pc.f0) + rank * kBF;
       const int last = static_cast<int>(p.N - pc.f0) - rank * kBF - 1;                  // the tile's last row of this weight (or before its first)
-      int64_t row_at[kBF / 32];                    // where the lane's rows start in a table
-#pragma unroll
-      for (int i = 0; i < kBF / 32; ++i) row_at[i] = static_cast<int64_t>(row + min(i * 32 + lane, last)) * groups * p.table_entry;
       for (int kb = pc.kb_lo; kb < pc.kb_hi; kb += kPer) {
         if (!(ok = wait(wempty + 8 * s, ph ^ 1u, 3))) break;
         const uint32_t bar = wfull + 8 * s;
@@ -658,32 +660,43 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
           // when all of a lane's earlier copies have landed, so any box of a chunk answers for its entries.
           const int box = kb / kPer, chunk = box >> p.chunk_shift;
           if (kb == pc.kb_lo || (box & ((1 << p.chunk_shift) - 1)) == 0) {
+            if (++ts == p.t_stages) ts = 0;
+            if (chunks >= static_cast<uint32_t>(p.t_stages)) {        // the last box of the chunk that was here has been read
+              const uint32_t was = __shfl_sync(0xffffffffu, last_box, ts), lap = __umulhi(was, p.w_inverse);
+              if (issued - was < static_cast<uint32_t>(p.w_stages) && !(ok = wait(wempty + 8 * (was - lap * p.w_stages), lap & 1u, 3))) {
+                ++s;                               // (its codes are on the way: see below)
+                break;
+              }
+            }
+            ++chunks;
             const int g0 = ((chunk << p.chunk_shift) * (kPer * kBK)) >> p.group_shift, most = (kPer * kBK << p.chunk_shift) >> p.group_shift;
             const int bytes = (groups - g0 < most ? groups - g0 : most) * p.table_entry;
-            const uint32_t slot = t_at + ts * (kTables * kBF * p.table_pitch) + lane * p.table_pitch;
-            if (++ts == p.w_stages) ts = 0;
+            const uint32_t slot = t_at + ts * (kTables * kBF * kTablePitch);
+            const int64_t row_bytes = static_cast<int64_t>(groups) * p.table_entry, at0 = row * row_bytes + g0 * p.table_entry;
+            // 16 bytes a lane, neighbouring lanes to a row: an instruction meets as few lines of memory as it can. Entries that start off a
+            // 16-byte boundary come with what lies before them; nothing past the table's end is read.
+            auto copy = [&](const void* table, uint32_t to) {
+              const uint8_t* src = static_cast<const uint8_t*>(table) + at0;
+              if (!p.skewed) {
+                const int o = (lane & 1) * 16;
+                if (o < bytes)
 #pragma unroll
-            for (int i = 0; i < kBF / 32; ++i) {
-              const int64_t at = row_at[i] + g0 * p.table_entry;
-              const uint32_t dst = slot + i * 32 * p.table_pitch;
-              auto copy = [&](const void* table, uint32_t to) {
-                const uint8_t* src = static_cast<const uint8_t*>(table) + at;
-                if (p.table_unit == 8) {
-#pragma unroll 1
-                  for (int o = 0; o < bytes; o += 8) cp_async8(to + o, src + o);
-                } else {                           // from the word the first entry lies in; nothing past the table's end is read
-                  const int skew = static_cast<int>(at & 3);
-#pragma unroll 1
-                  for (int o = -skew; o < bytes; o += 4) {
-                    const int64_t room = p.table_bytes - (at + o);
-                    cp_async4(to + skew + o, src + o, room >= 4 ? 4 : static_cast<int>(room));
-                  }
+                  for (int i = lane >> 1; i < kBF; i += 16) cp_async16(to + i * kTablePitch + o, src + min(i, last) * row_bytes + o, 16);
+              } else {
+                const int o = (lane & 3) * 16;
+                const uint64_t end = reinterpret_cast<uint64_t>(table) + p.table_bytes;
+#pragma unroll 4
+                for (int i = lane >> 2; i < kBF; i += 8) {
+                  const uint64_t at = reinterpret_cast<uint64_t>(src) + min(i, last) * row_bytes, from = (at & ~15ull) + o;
+                  if (from < at + bytes) cp_async16(to + i * kTablePitch + o, reinterpret_cast<const void*>(from), end - from < 16 ? static_cast<int>(end - from) : 16);
                 }
-              };
-              copy(p.scales, dst);
-              if constexpr (QK != kMx4) copy(p.biases, dst + kBF * p.table_pitch);
-            }
+              }
+            };
+            copy(p.scales, slot);
+            if constexpr (QK != kMx4) copy(p.biases, slot + kBF * kTablePitch);
           }
+          if (lane == ts) last_box = issued;
+          ++issued;
           cp_async_arrive(bar);
         }
         if (++s == p.w_stages) { s = 0; ph ^= 1u; }
@@ -733,7 +746,7 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
     const bool twide = !SAME && p.table_dtype == QMM_F32;
     const int entry = QK == kMx4 ? 1 : SAME ? 2 : p.table_entry;
     [[maybe_unused]] const uint32_t mask = in_register(0x000F000Fu), magic = in_register(Half2Ops<XT>::kMagic);
-    const uint32_t bias_off = kBF * p.table_pitch, swizzle = (frow & 7) << 4;
+    const uint32_t swizzle = (frow & 7) << 4;
     const uint32_t a_bar = kPair ? in_cta(a_full, leader) : a_full, d_bar = kPair ? in_cta(d_empty, leader) : d_empty;
     const uint32_t wthread = w_at + frow * kBoxBytes;
     uint32_t wbase = 0, sbase = 0, cbase = 0, piece = 0;    // boxes, steps and table chunks before this piece
@@ -758,8 +771,13 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
         const int chunk = (pc.kb_lo + j) / kPer >> p.chunk_shift, chunk_k = (chunk << p.chunk_shift) * (kPer * kBK);
         const int g0 = chunk_k >> p.group_shift, glast = groups - 1 - g0;
         const int k0 = (pc.kb_lo + j) * kBK - chunk_k;                 // the step's first element in the chunk
-        const uint32_t ci = cbase + chunk - (pc.kb_lo / kPer >> p.chunk_shift), ts = ci - __umulhi(ci, p.w_inverse) * p.w_stages;
-        const uint32_t tbox = t_at + ts * (kTables * kBF * p.table_pitch) + frow * p.table_pitch + (p.table_unit < 4 ? ((trow + g0) * entry & 3u) : 0u);
+        const uint32_t ci = cbase + chunk - (pc.kb_lo / kPer >> p.chunk_shift), ts = ci - __umulhi(ci, p.t_inverse) * p.t_stages;
+        uint32_t tbox = t_at + ts * (kTables * kBF * kTablePitch) + frow * kTablePitch, bias_off = kBF * kTablePitch;
+        if (p.skewed) {
+          const uint32_t at = (trow + g0) * entry, skew = (at + static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.scales))) & 15u;
+          tbox += skew;
+          if constexpr (QK != kMx4) bias_off += ((at + static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.biases))) & 15u) - skew;
+        }
         // (a block at a time, not the whole step unrolled: the sixteen warps are at sixteen places of this code, and much more of it
         // no longer stays in the instruction caches)
         const int blocks = nkb - j < kStep ? nkb - j : kStep;
@@ -1104,27 +1122,37 @@ int launch_tables(const qmm_problem& p, cudaStream_t stream) {
   tp.group_shift = group == 128 ? 7 : group == 64 ? 6 : 5;
   tp.table_dtype = p.table_dtype; tp.y_dtype = p.y_dtype;
 
-  // The rings: as many weight boxes as fit next to the table chunks that go with them. A chunk is at least 8 bytes of a row (a
-  // box of 8-bit codes in groups of 128 has 2): the copies are per row, and their number is what they cost.
-  int box_bytes = 0, row_table = 0;
+  // The rings: as many weight boxes as fit next to the table chunks that go with them. Entries travel a sector of a row at a time: the copies are
+  // per row, and what they cost the producer is the lines that they touch (8 bytes of 32 rows an instruction, with every box, was what bound
+  // 64 rows: see the head of the file).
+  int chunk_boxes = 0, chunk_slot = 0;
   if (QK != kFloat) {
     tp.table_entry = QK == kMx4 ? 1 : (p.table_dtype == QMM_F32 ? 4 : 2);
-    box_bytes = (P::kPer * kBK >> tp.group_shift) * tp.table_entry;
-    row_table = static_cast<int>(p.K >> tp.group_shift) * tp.table_entry;
-    tp.table_unit = row_table % 8 == 0 ? 8 : row_table % 4 == 0 ? 4 : 1;
-    while (box_bytes << tp.chunk_shift < 8) ++tp.chunk_shift;
-    const int chunk_bytes = box_bytes << tp.chunk_shift;
-    tp.table_pitch = tp.table_unit >= 4 ? chunk_bytes : chunk_bytes + 4;
+    const int box_bytes = (P::kPer * kBK >> tp.group_shift) * tp.table_entry, row_table = static_cast<int>(p.K >> tp.group_shift) * tp.table_entry;
+    const uintptr_t start = reinterpret_cast<uintptr_t>(p.scales) | (QK == kMx4 ? 0 : reinterpret_cast<uintptr_t>(p.biases));
+    tp.skewed = row_table % 16 != 0 || start % 16 != 0;
+    while (box_bytes << tp.chunk_shift < kChunkBytes) ++tp.chunk_shift;
+    chunk_boxes = 1 << tp.chunk_shift;
     tp.table_bytes = w_rows * row_table;
+    chunk_slot = (QK == kMx4 ? 1 : 2) * kBF * kTablePitch;
   }
-  // (as many chunks as boxes: a chunk has a box at least, so that the chunk before in its place has been used up when the box before in its
-  // first box's place has)
-  const int chunk_slot = QK == kFloat ? 0 : (QK == kMx4 ? 1 : 2) * kBF * tp.table_pitch;
-  tp.w_stages = (P::kBudget - P::kFixed) / (P::kWBytes + chunk_slot);
-  if (tp.w_stages > P::kMostBoxes) tp.w_stages = P::kMostBoxes;
+  // Chunks for every box of the ring that lies ahead of the one that is read, if they fit (with fewer the producer waits a little earlier).
+  const int room = P::kBudget - P::kFixed;
+  for (tp.w_stages = P::kMostBoxes; tp.w_stages >= P::kLeastPlaces; --tp.w_stages) {
+    if (QK == kFloat) {
+      if (tp.w_stages * P::kWBytes <= room) break;
+      continue;
+    }
+    tp.t_stages = 1 + (tp.w_stages - 1 + chunk_boxes - 1) / chunk_boxes;
+    if (tp.t_stages < 2) tp.t_stages = 2;
+    if (tp.w_stages == P::kLeastPlaces)
+      while (tp.t_stages > 2 && tp.w_stages * P::kWBytes + tp.t_stages * chunk_slot > room) --tp.t_stages;
+    if (tp.w_stages * P::kWBytes + tp.t_stages * chunk_slot <= room) break;
+  }
   if (tp.w_stages < P::kLeastPlaces) return fail(QMM_ERR_UNSUPPORTED, "qmm_gemm_tc_kernel: the weight ring does not fit shared memory");
-  const size_t smem = P::kFixed + static_cast<size_t>(tp.w_stages) * (P::kWBytes + chunk_slot);
+  const size_t smem = P::kFixed + static_cast<size_t>(tp.w_stages) * P::kWBytes + static_cast<size_t>(tp.t_stages) * chunk_slot;
   tp.w_inverse = 0xFFFFFFFFu / tp.w_stages + 1;
+  tp.t_inverse = tp.t_stages ? 0xFFFFFFFFu / tp.t_stages + 1 : 0;
 
   auto kernel = qmm_gemm_tc_kernel<QK, XT, BT, SAME>;
   static bool configured[kMaxDevices] = {};     // the attribute is per device

@@ -151,10 +151,13 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
 }
 __device__ __forceinline__ void cp_async_drain() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Asynchronous copies of 8 or 4 bytes (of the latter `bytes` are read, the rest is zero) into shared memory, and
+// Asynchronous copies of 16, 8 or 4 bytes (where it is given, `bytes` are read and the rest is zero) into shared memory, and
 // this thread's arrival on `bar` once all its earlier ones have landed (the barrier's count includes it).
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes = 4) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
