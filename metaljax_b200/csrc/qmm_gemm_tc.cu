@@ -38,8 +38,11 @@
 // 219 -> 167..174; 512 rows 28672 x 4096 130 -> 97; 64 rows 28672 x 4096 59.7 -> 33.1, 4096 x 4096 16.4 -> 10.5, 4096 x 14336 31.2 -> 19.4; 128 rows
 // 4096 x 14336 47 -> 21; 8-bit group 128, 45 rows 14336 x 4096 33 -> 20.6. Table entries a sector of a row at a time instead of the 8 bytes of
 // every box (a row a lane: 32 lines an instruction; without the dequantization 64 rows then took 345 clocks a K block and SM, 204 without those copies):
-// 64 rows 28672 x 4096 33.3 -> 30.6, 65760 x 2880 (rows of 90 table bytes) 79.3 -> 48.7, float32 tables in groups of 32 14336 x 4096 42 -> 33. What bounds it: at 64 rows the dequantizing warps (400 clocks a K block and SM: some 300 instructions a
-// warp and block at four warps a scheduler), at 256 the tensor cores (500 clocks a block between a tile's ends, under the power cap) and the ends,
+// 64 rows 28672 x 4096 33.3 -> 30.6, 65760 x 2880 (rows of 90 table bytes) 79.3 -> 48.7, float32 tables in groups of 32 14336 x 4096 42 -> 33. What an epilogue
+// costs: 4.6 us a tile of 256 x 256 with 2-byte stores behind a check each (2.1 at 64 tokens); drained into registers and rounded first, stored in pairs of features: 64 rows 28672 x
+// 4096 30.6 -> 27.0, 512 rows mxfp4 5760 x 2880 22.8 -> 20.6, 2048 rows 14336 x 4096 183 -> 172.
+// What bounds it: at 64 rows memory and the dequantizing warps together (335 clocks a K block and SM; 260 without the dequantization, 210 of them the weights' bytes) and some
+// 6 us of a launch's ends, at 256 the tensor cores (500 clocks a block between a tile's ends, under the power cap) and the ends,
 // where the accumulator is drained by the warps that would dequantize for the next tile. (Draining it after the first steps of the next
 // tile was built: the state that lives across the epilogue then spills, and every size lost.)
 //
@@ -216,7 +219,13 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
                : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : QMM_ASM_W(0), QMM_ASM_W(8)
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -441,6 +450,8 @@ struct Plan {
   static constexpr int kXBytes = kStep * kXBlock;
   static constexpr int kWBytes = kBF * kBoxBytes;
   static constexpr int kACol0 = BT;                           // the A ring starts behind D's columns [0, BT)
+  static constexpr int kTeamCols = BT / kTeams;               // columns of D that a team drains ...
+  static constexpr int kCols = BT == 128 ? 32 : 16;            // ... so many at a time
   static constexpr int kStages = kStep == 1 || (BT <= 64 && QK != kFloat) ? 6 : 4;
   static constexpr int kBarBytes = 1024;
   static constexpr int kBudget = 227 * 1024 - 4608;           // dynamic shared memory (the tile tables are static)
@@ -861,14 +872,16 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
       if (!(ok = wait(d_full, piece & 1, 8))) break;
       __syncwarp();      // lanes leave the wait loop one by one; tcgen05.ld needs the whole warp
       tc_fence_after();
+      constexpr int kCols = P::kCols;
+      const int first_col = team * P::kTeamCols, end_col = min(first_col + P::kTeamCols, pc.rows);
       if (P::kMaySplit && p.cluster_adds) {        // this worker's share of the sums, over its activation ring (which is done with)
 #pragma unroll 1
-        for (int c0 = team * 32; c0 < pc.rows; c0 += 32 * kTeams) {
-          uint32_t r[32];
-          tmem_ld32(tmem_base + lane_addr + c0, r);
+        for (int c0 = first_col; c0 < end_col; c0 += kCols) {
+          uint32_t r[kCols];
+          tmem_ld(tmem_base + lane_addr + c0, r);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) sts32(x_at + ((c0 + j) * kBF + frow) * 4, __uint_as_float(r[j]));
+          for (int j = 0; j < kCols; ++j) sts32(x_at + ((c0 + j) * kBF + frow) * 4, __uint_as_float(r[j]));
         }
         break;
       }
@@ -880,7 +893,7 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
           else arrive_n(d_bar, 1);
         }
       };
-      const bool mine = team * 32 < pc.rows;
+      const bool mine = first_col < pc.rows;
       const bool whole = pc.begins && pc.ends, part_only = !pc.ends || p.split > 1;
       if (mine && !part_only && !whole) {          // the tile's earlier pieces, made by the workers before this one
         const int tile_box0 = pc.tile * walk.boxes;
@@ -902,53 +915,101 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }
+      // COLS rounded columns of the tile, two to a word, stored. Even N: neighbouring lanes (features) swap halves, so that
+      // the even one stores both features of one token and the odd one those of the next.
+      auto store_halves = [&](const auto& h, int c0) {
+        constexpr int kPairs = sizeof(h) / 4;
+        const int rows_left = feat_ok ? pc.rows - c0 : 0, n = static_cast<int>(p.N);
+        uint16_t* y = reinterpret_cast<uint16_t*>(p.y) + ((pc.row0 + c0) * p.N + feat);
+        if ((n & 1) == 0) {
+          const int odd = lane & 1;
+          const uint32_t swap = odd ? 0x3276u : 0x5410u;
+          if (odd) y += n - 1;
+#pragma unroll
+          for (int j = 0; j < kPairs; ++j) {
+            const uint32_t v = __byte_perm(h[j], __shfl_xor_sync(0xffffffffu, h[j], 1), swap);
+            if (2 * j + odd < rows_left) *reinterpret_cast<uint32_t*>(y) = v;
+            y += 2 * static_cast<int64_t>(n);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < kPairs; ++j) {
+            if (2 * j < rows_left) y[0] = static_cast<uint16_t>(h[j]);
+            if (2 * j + 1 < rows_left) y[n] = static_cast<uint16_t>(h[j] >> 16);
+            y += 2 * static_cast<int64_t>(n);
+          }
+        }
+      };
+      auto round = [&](const uint32_t (&r)[kCols], uint32_t* h) {
+        if (p.y_dtype == QMM_BF16) {
+#pragma unroll
+          for (int j = 0; j < kCols; j += 2) h[j / 2] = Half2Ops<__nv_bfloat16>::pack(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+        } else {
+#pragma unroll
+          for (int j = 0; j < kCols; j += 2) h[j / 2] = Half2Ops<__half>::pack(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+        }
+      };
+      if (whole && !part_only && p.y_dtype != QMM_F32) {      // all of it into registers first: the next tile's MMAs need not wait for the stores
+        uint32_t h[P::kTeamCols / 2];
+#pragma unroll
+        for (int i = 0; i < P::kTeamCols / kCols; ++i) {
+          if (first_col + i * kCols < pc.rows) {
+            uint32_t r[kCols];
+            tmem_ld(tmem_base + lane_addr + first_col + i * kCols, r);
+            tmem_wait_ld();
+            round(r, h + i * (kCols / 2));
+          }
+        }
+        drained();
+        if (mine) store_halves(h, first_col);
+        continue;
+      }
 #pragma unroll 1
-      for (int c0 = team * 32; c0 < BT; c0 += 32 * kTeams) {
-        if (c0 >= pc.rows) break;                  // warp-uniform: no valid token rows left
+      for (int c0 = first_col; c0 < end_col; c0 += kCols) {
         const int64_t in_partial = static_cast<int64_t>(c0) * kBF + frow;
-        float sum[32];
+        float sum[kCols];
         if (!part_only && !whole) {                // in K order: the workers' pieces, then this one
           const int tile_box0 = pc.tile * walk.boxes;
           int v = worker - 1;
           while (Walk<BT, kPer>::first_box(p, v) > tile_box0) --v;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) sum[j] = 0.0f;
+          for (int j = 0; j < kCols; ++j) sum[j] = 0.0f;
           for (; v < worker; ++v) {
             const float* part = p.partial + (static_cast<int64_t>(v) * kCtas + rank) * (BT * kBF) + in_partial;
-            float f[32];
-            // (volatile: all 32 requests go out before the first is waited for)
+            float f[kCols];
+            // (volatile: all requests go out before the first is waited for)
 #pragma unroll
-            for (int j = 0; j < 32; ++j) asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(f[j]) : "l"(part + j * kBF));
+            for (int j = 0; j < kCols; ++j) asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(f[j]) : "l"(part + j * kBF));
 #pragma unroll
-            for (int j = 0; j < 32; ++j) sum[j] += f[j];
+            for (int j = 0; j < kCols; ++j) sum[j] += f[j];
           }
         }
-        uint32_t r[32];
-        tmem_ld32(tmem_base + lane_addr + c0, r);
+        uint32_t r[kCols];
+        tmem_ld(tmem_base + lane_addr + c0, r);
         tmem_wait_ld();
-        if (c0 + 32 * kTeams >= pc.rows) drained();      // this warp's last columns: the next tile's MMAs need not wait for the stores
+        if (c0 + kCols >= end_col) drained();      // this warp's last columns
         if (part_only) {
           float* part = p.partial + static_cast<int64_t>(blockIdx.x) * (BT * kBF) + in_partial;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) __stcg(part + j * kBF, __uint_as_float(r[j]));
+          for (int j = 0; j < kCols; ++j) __stcg(part + j * kBF, __uint_as_float(r[j]));
           continue;
         }
         if (!whole) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[j] + __uint_as_float(r[j]));
+          for (int j = 0; j < kCols; ++j) r[j] = __float_as_uint(sum[j] + __uint_as_float(r[j]));
         }
-        if (feat_ok) {
-          const int64_t o0 = (pc.row0 + c0) * p.N + feat;
+        if (p.y_dtype == QMM_F32) {
+          float* y = reinterpret_cast<float*>(p.y) + ((pc.row0 + c0) * p.N + feat);
+          const int rows_left = feat_ok ? pc.rows - c0 : 0;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (c0 + j < pc.rows) {
-              const int64_t o = o0 + j * p.N;
-              const float v = __uint_as_float(r[j]);
-              if (p.y_dtype == QMM_BF16) reinterpret_cast<__nv_bfloat16*>(p.y)[o] = __float2bfloat16_rn(v);
-              else if (p.y_dtype == QMM_F16) reinterpret_cast<__half*>(p.y)[o] = __float2half_rn(v);
-              else reinterpret_cast<float*>(p.y)[o] = v;
-            }
+          for (int j = 0; j < kCols; ++j) {
+            if (j < rows_left) *y = __uint_as_float(r[j]);
+            y += p.N;
           }
+        } else {
+          uint32_t h[kCols / 2];
+          round(r, h);
+          store_halves(h, c0);
         }
       }
       if (!mine) drained();
