@@ -40,7 +40,8 @@
 // every box (a row a lane: 32 lines an instruction; without the dequantization 64 rows then took 345 clocks a K block and SM, 204 without those copies):
 // 64 rows 28672 x 4096 33.3 -> 30.6, 65760 x 2880 (rows of 90 table bytes) 79.3 -> 48.7, float32 tables in groups of 32 14336 x 4096 42 -> 33. What an epilogue
 // costs: 4.6 us a tile of 256 x 256 with 2-byte stores behind a check each (2.1 at 64 tokens); drained into registers and rounded first, stored in pairs of features: 64 rows 28672 x
-// 4096 30.6 -> 27.0, 512 rows mxfp4 5760 x 2880 22.8 -> 20.6, 2048 rows 14336 x 4096 183 -> 172.
+// 4096 30.6 -> 27.0, 512 rows mxfp4 5760 x 2880 22.8 -> 20.6, 2048 rows 14336 x 4096 183 -> 172. The weights' producer on its way before the rest is set up: 64 rows 28672 x 4096 27.0 ->
+// 26.3, 4096 x 14336 17.6 -> 17.2.
 // What bounds it: at 64 rows memory and the dequantizing warps together (335 clocks a K block and SM; 260 without the dequantization, 210 of them the weights' bytes) and some
 // 6 us of a launch's ends, at 256 the tensor cores (500 clocks a block between a tile's ends, under the power cap) and the ends,
 // where the accumulator is drained by the warps that would dequantize for the next tile. (Draining it after the first steps of the next
@@ -572,55 +573,67 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
   // product -- is read only after a griddepcontrol.wait, and everything this grid writes is
   // downstream of those reads.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (p.group_sizes) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int s = threadIdx.x; s < nseg; s += kThreads) seg_row0[s + 1] = p.group_sizes[s] > 0 ? p.group_sizes[s] : 0;
-    __syncthreads();
+  auto init = [](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n)); };
+  uint32_t tmem_base = 0;
+  if (warp == kWarps - 1) {
+    // The weights' producer lays out the walk and its own barriers and does not wait for the rest: its first boxes are on their way (a trip to
+    // memory, 2 us when every CTA asks at once) while the others set up tensor memory and their barriers (0.7 us).
+    if (p.group_sizes) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      for (int s = lane; s < nseg; s += 32) seg_row0[s + 1] = p.group_sizes[s] > 0 ? p.group_sizes[s] : 0;
+      __syncwarp();
+    }
+    if (lane == 0) {
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(abort_at), "r"(0) : "memory");
+      int64_t rows = 0;
+      int tiles = 0;
+      seg_row0[0] = 0;
+      seg_tile0[0] = 0;
+      for (int s = 0; s < nseg; ++s) {
+        int64_t r = p.group_sizes ? seg_row0[s + 1] : p.M;
+        if (p.group_sizes && rows + r > p.M) r = p.M - rows;
+        rows += r;
+        tiles += static_cast<int>((r + BT - 1) / BT) * ftiles;
+        seg_tile0[s + 1] = tiles;
+        seg_row0[s + 1] = rows;
+      }
+      for (int i = 0; i < p.w_stages; ++i) {
+        init(wfull + 8 * i, QK == kFloat ? 1 : 1 + 32);
+        init(wempty + 8 * i, 4 * P::kStepsPerBox);
+      }
+      mbar_init_fence();
+    }
+    __syncwarp();
+    asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
+    if constexpr (kPair) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  } else {
+    if (threadIdx.x == 0) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&x_map)) : "memory");
+      for (int i = 0; i < kStages; ++i) {
+        init(xfull + 8 * i, 1);
+        init(empty + 8 * i, 1);
+        init(a_full + 8 * i, 4 * kCtas);
+      }
+      init(d_full, 1);
+      init(d_empty, kDequantWarps * kCtas);
+      mbar_init_fence();
+    }
+    if (warp == 1) {
+      if constexpr (kPair) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+      } else {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+      }
+    }
+    tc_fence_before();
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+    if constexpr (kPair) cluster_barrier();        // the partner's barriers and tensor memory are there
+    tc_fence_after();
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot) : "memory");
+    tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
   }
-  if (threadIdx.x == 0) {
-    int64_t rows = 0;
-    int tiles = 0;
-    seg_row0[0] = 0;
-    seg_tile0[0] = 0;
-    for (int s = 0; s < nseg; ++s) {
-      int64_t r = p.group_sizes ? seg_row0[s + 1] : p.M;
-      if (p.group_sizes && rows + r > p.M) r = p.M - rows;
-      rows += r;
-      tiles += static_cast<int>((r + BT - 1) / BT) * ftiles;
-      seg_tile0[s + 1] = tiles;
-      seg_row0[s + 1] = rows;
-    }
-    auto init = [](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n)); };
-    for (int i = 0; i < p.w_stages; ++i) {
-      init(wfull + 8 * i, QK == kFloat ? 1 : 1 + 32);
-      init(wempty + 8 * i, 4 * P::kStepsPerBox);
-    }
-    for (int i = 0; i < kStages; ++i) {
-      init(xfull + 8 * i, 1);
-      init(empty + 8 * i, 1);
-      init(a_full + 8 * i, 4 * kCtas);
-    }
-    init(d_full, 1);
-    init(d_empty, kDequantWarps * kCtas);
-    asm volatile("st.shared.u32 [%0], %1;" ::"r"(abort_at), "r"(0) : "memory");
-    mbar_init_fence();
-  }
-  if (warp == 1) {
-    if constexpr (kPair) {
-      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512) : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    } else {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512) : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if constexpr (kPair) cluster_barrier();          // the partner's barriers and tensor memory are there
-  tc_fence_after();
-  uint32_t tmem_base;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot) : "memory");
-  tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
   const int tiles = seg_tile0[nseg];
   Walk<BT, kPer> walk(p, worker, workers, num_kb, tiles);
   Piece pc = {};
@@ -716,6 +729,10 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
     if (!ok) {
       cp_async_drain();
       for (int i = 0; i < p.w_stages; ++i) mbar_drain(wfull + 8 * i, i < s ? ph : ph ^ 1u);
+    }
+    if constexpr (kPair) {
+      __syncwarp();
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // (of the arrival above)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (of a pair: the leader's) ----------------
