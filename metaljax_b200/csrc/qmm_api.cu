@@ -219,7 +219,10 @@ int launch_problem(const qmm_problem& p, cudaStream_t stream) {
     // few-rows kernel takes them as columns of its MMAs; the plain SIMT kernel is what a forced route cross-checks with.
     // Its codes go in without a magic number here, since the SIMT kernel's float32 sums are what such calls had: with it a float32 result
     // of activations of one sign was 60 (4-bit) to 140 times (8-bit) further from the exact one than the SIMT kernel's.
-    default: return route_override() != QMM_ROUTE_SIMT && rows_supports(p) ? launch_rows(p, stream, nullptr, true) : launch_simt(p, stream);
+    default:
+      if (route_override() == QMM_ROUTE_SIMT) return launch_simt(p, stream);
+      if (f32_tc_pays(p)) return launch_f32_tc(p, stream);
+      return rows_supports(p) ? launch_rows(p, stream, nullptr, true) : launch_simt(p, stream);
   }
 }
 

@@ -1,0 +1,737 @@
+// Float32 activations of more than a few rows on the 5th-generation tensor cores (`y = x . deq(w)^T`, src/metaljax/qmm.py:2491,
+// in the precision that keras keeps by default).
+//
+// Arithmetic, that of the few-rows kernel (qmm_rows.cuh) in another place: the codes are never dequantized. A code minus its centre (q - 8,
+// q - 128, an E2M1 value) is an exact bf16, the MMA's A operand in tensor memory; a float32 activation is three bf16 pieces (8 + 8 + 8 bits),
+// the B operand. Every 64 codes (32 in groups of 32) have accumulators of their own, two columns of tensor memory per row, one for the first piece and one for the
+// others: a tensor core truncates each sum that it makes, and the small pieces' sums are small. They are read back, scaled and added up in
+// float32 registers: y += s * sum (q - C) x, and once a tile, where that is not nought for every row of a warp, sum (b + C s) sum x.
+//
+// Split. K is shared out to the CTAs of a cluster (up to 8). A CTA converts its stretch of K of a chunk of 16, 32 or 48 activation rows once, into
+// swizzled tiles that stay in shared memory; tiles of 128 weight rows pass by. The CTAs' partial tiles are pushed with st.async to the CTA that owns 128 / c of the
+// tile's rows, which adds them up in rank order a tile late. No scratch, no atomics, fixed order of summation.
+//
+// What bounds it: the few-rows kernel takes four rows a pass over the weight, and takes the codes apart for each of them (33 rows: nine times). Here a pass
+// takes up to 48. 33 rows of 4096 x 4096: 34.6 -> 24.0 us (13 K clocks a tile and cluster of eight: 8 K of them the codes, the MMAs' issue and the adding up, which
+// are latency at 18 warps, the rest the exchange; 14 such clusters fit the machine); 64 rows of 14336 x 4096 178 -> 83, 4096 x 14336 234 -> 114.
+// Relative error against float64 (2-norm; N(0, 1) / one sign / outliers of 300), few-rows kernel -> here: 4-bit 33 rows K 4096 8.6e-8 / 5.2e-8 / 9.4e-8 ->
+// 8.2e-8 / 5.1e-8 / 9.1e-8, K 14336 9.3e-8 / 4.4e-8 / 1.0e-7 -> 9.2e-8 / 4.9e-8 / 1.0e-7, 8-bit K 4096 1.3e-7 / 7.4e-8 / 2.1e-7 -> 8.5e-8 / 7.9e-8 / 1.3e-7, MXFP4 K 2880
+// 8.8e-8 / 7.6e-8 / 1.1e-7 -> 8.9e-8 / 8.7e-8 / 9.2e-8. (All pieces in one accumulator: 9.4e-8 / 6.4e-8 / 9.7e-8, and 2.4e-7 in groups of 128.)
+//
+// Warps: 0 = weights' producer, 1 = MMA issuer (+ tensor memory), 2..9 = two teams that turn codes into A, 10..17 = adding up, half of the rows
+// to each four. All of them convert the activations. A step is two K blocks: a wait costs a warp about as much as a third of a block's codes, and
+// a warp by itself issues an instruction in some four clocks, so that there are many of either kind.
+// Every wait on an mbarrier is bounded. Launched with programmatic stream serialization: before griddepcontrol.wait only the weights are touched.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+#include "qmm_internal.h"
+#include "qmm_ptx.cuh"
+#include "qmm_tcgen05.cuh"
+
+namespace qmm {
+namespace {
+
+using namespace ptx;
+using namespace tc;
+
+constexpr int kTileRows = 128;         // weight rows of a tile: lanes of tensor memory
+constexpr int kBK = 64;                // K of a block: 32 columns of A
+constexpr int kStepK = 2 * kBK;        // K of a step: a weight box, a slot of A
+constexpr int kTeams = 2;
+constexpr int kAddWarps = 8;
+constexpr int kWarps = 2 + 4 * kTeams + kAddWarps;
+constexpr int kThreads = kWarps * 32;
+constexpr int kAddWarp = 2 + 4 * kTeams;
+constexpr int box_bytes(int bits) { return kTileRows * kStepK * bits / 8; }
+constexpr int kMaxBoxes = 8;
+constexpr int kASlots = 4;             // steps of A in tensor memory
+constexpr int kASlotsAt = 0, kDAt = kASlots * 64;
+constexpr int d_slots(int t) { return t == 48 ? 2 : 4; }     // accumulators in tensor memory
+constexpr int kMaxDSlots = 4;
+constexpr int kMaxCluster = 8;
+constexpr int kSmemLimit = 227 * 1024;
+static_assert(kTeams <= kASlots, "a parity cannot tell a slot's use from the one two rounds before");
+
+enum { kAff4 = 0, kAff8 = 1, kMx4 = 2 };
+
+struct F32Params {
+  const float* x;
+  const void* scales;
+  const void* biases;
+  void* y;
+  int* status;
+  int64_t M, N;
+  int K, groups, group_shift, table_dtype, y_dtype;
+  int tiles, steps, most_steps;        // tiles of the weight; steps of K, and the most of them that a CTA has
+  int cluster, slots, boxes;           // CTAs that share K; partial tiles on their way to an owner; places of the weights' ring
+  unsigned most_inverse, less_inverse; // 2^32 / (16 steps) rounded up, of a CTA with most_steps and of one with a step less
+  unsigned share, share_more;          // (chunk, tile) items of every cluster, and how many clusters have one more
+};
+
+// Shared memory from the 1024-byte aligned start: barriers, the activations [block][piece][T rows x 128 bytes], the weights' ring, the activations' sums over 32 codes
+// [4 steps][T], the partial tiles [slot][128 rows][T + 4].
+constexpr int kWFull = 0, kWEmpty = kWFull + 8 * kMaxBoxes, kAFull = kWEmpty + 8 * kMaxBoxes, kAEmpty = kAFull + 8 * kASlots, kDFull = kAEmpty + 8 * kASlots,
+              kDEmpty = kDFull + 8 * kMaxDSlots, kXFull = kDEmpty + 8 * kMaxDSlots, kXFree = kXFull + 16, kTmemSlot = kXFree + 16, kAbort = kTmemSlot + 4, kHead = 1024;
+static_assert(kAbort + 4 <= kHead, "");
+constexpr int partial_row(int t) { return (t + 4) * 4; }
+constexpr int partial_bytes(int t) { return kTileRows * partial_row(t); }
+constexpr int x_block(int t) { return 3 * t * 128; }
+constexpr size_t smem_of(int t, int steps, int slots, int boxes, int bits) {
+  return 1024 + kHead + boxes * box_bytes(bits) + static_cast<size_t>(steps) * (2 * x_block(t) + 4 * t * 4) + static_cast<size_t>(slots) * partial_bytes(t);
+}
+
+// NW packed words -> pairs of bf16 codes minus their centre (exact).
+template <int QK>
+__device__ __forceinline__ void codes16(const uint32_t (&w)[4], uint32_t* out) {
+  if constexpr (QK == kAff4) {         // 32 codes, as (q - 8) / 64: a code in the low bits is the subnormal q 2^-133, one FMA with 2^127 and -1 / 8 takes it there (exactly)
+    using H = Half2Ops<__nv_bfloat16>;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t even = w[j] & 0x0F0F0F0Fu, odd = (w[j] >> 4) & 0x0F0F0F0Fu;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[j * 4 + i] = H::fma(permute(even, odd, i | ((8 + i) << 4) | ((4 + i) << 8) | ((12 + i) << 12)), 0x7F007F00u, 0xBE00BE00u);
+    }
+  } else if constexpr (QK == kAff8) {  // 16 codes, through float32: 2^23 + q - (2^23 + 128)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float q[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) q[e] = __uint_as_float(__byte_perm(w[j], 0x4B000000u, 0x7540u + e)) - 8388736.0f;
+      out[j * 2] = Half2Ops<__nv_bfloat16>::pack(q[0], q[1]);
+      out[j * 2 + 1] = Half2Ops<__nv_bfloat16>::pack(q[2], q[3]);
+    }
+  } else {                             // 32 E2M1 codes: magnitude at the exponent's boundary is the value times 2^-126
+    using H = Half2Ops<__nv_bfloat16>;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t hi = w[j] >> 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t t = __byte_perm(w[j], hi, i | ((4 + i) << 8)) & 0x000F000Fu;
+        out[j * 4 + i] = H::mul(((t & 0x00070007u) << 6) | ((t & 0x00080008u) << 12), 0x7E807E80u);      // 2^126
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void fma2(float& y0, float& y1, float s, float a0, float a1) {
+  asm("{ .reg .b64 y, s, a; mov.b64 y, {%0, %1}; mov.b64 s, {%2, %2}; mov.b64 a, {%3, %4}; fma.rn.f32x2 y, s, a, y; mov.b64 {%0, %1}, y; }"
+      : "+f"(y0), "+f"(y1) : "f"(s), "f"(a0), "f"(a1));
+}
+// y0, y1 += s * (a + b), two at a time.
+__device__ __forceinline__ void add_fma2(float& y0, float& y1, float s, const uint32_t* a, const uint32_t* b) {
+  asm("{ .reg .b64 y, s, a, b; mov.b64 y, {%0, %1}; mov.b64 s, {%2, %2}; mov.b64 a, {%3, %4}; mov.b64 b, {%5, %6}; add.rn.f32x2 a, a, b; fma.rn.f32x2 y, s, a, y; mov.b64 {%0, %1}, y; }"
+      : "+f"(y0), "+f"(y1) : "f"(s), "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ void st_async4(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar) : "memory");
+}
+
+// QK: quantization kind. T: activation rows of a chunk. WIDE: float32 tables.
+template <int QK, int T, bool WIDE>
+__global__ void __launch_bounds__(kThreads, 1)
+qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) {
+  constexpr int kBits = QK == kAff8 ? 8 : 4;
+  constexpr int kRowBytes = kBK * kBits / 8, kBoxBytes = 2 * kRowBytes, kBox = box_bytes(kBits);      // of a weight row in a block, in a box
+  constexpr float kCentre = QK == kAff8 ? 128.0f : 8.0f, kUnit = QK == kAff4 ? 64.0f : 1.0f;     // (4-bit codes go in divided by 64)
+  constexpr int kXBlock = x_block(T), kPiece = T * 128, kRow = partial_row(T), kDSlots = d_slots(T);
+  static_assert(kDAt + kDSlots * 2 * T <= 512 && T % 16 == 0, "");
+
+  extern __shared__ uint8_t f32_smem_raw[];
+  const uint32_t smem = (smem_u32(f32_smem_raw) + 1023) & ~1023u;
+  const uint32_t x_at = smem + kHead, w_at = x_at + p.most_steps * 2 * kXBlock, sums_at = w_at + p.boxes * kBox, part_at = sums_at + p.most_steps * 4 * T * 4;
+  const uint32_t abort_at = smem + kAbort;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  // (what the issuer's operands come from is the same in all lanes, and is made known as such: see tc_mma_block)
+  auto same = [](int v) -> int { return __shfl_sync(0xffffffffu, v, 0); };
+  const int csize = p.cluster, rank = same(csize > 1 ? static_cast<int>(cluster_rank()) : 0);
+  const int step0 = same(p.steps * rank / csize), nsteps = same(p.steps * (rank + 1) / csize - step0);
+  const bool halves = p.group_shift == 5;                // two accumulators a block
+  const unsigned cluster = blockIdx.x / csize;
+  const unsigned first = cluster * p.share + min(cluster, p.share_more);
+  const int items = same(p.share + (cluster < p.share_more ? 1u : 0u));
+
+  auto wait = [&](uint32_t bar, uint32_t parity, int where) -> bool { return wait_phase(smem + bar, parity, abort_at, where); };
+  auto init = [&](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem + bar), "r"(n)); };
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  // What an adding-up lane reads of a tile's tables: four entries of its row at a time, and which of them lie in its CTA's K.
+  const int trow_lane = (warp & 3) * 32 + lane;
+  constexpr int kEntry = QK == kMx4 ? 1 : WIDE ? 4 : 2;
+  const int g_first = step0 * kStepK >> p.group_shift, g_end = min((step0 + nsteps) * kStepK >> p.group_shift, p.groups);
+  auto table_row = [&](int tile) -> int64_t {
+    const int64_t n = static_cast<int64_t>(tile) * kTileRows + trow_lane;
+    return (n < p.N ? n : p.N - 1) * p.groups;
+  };
+  auto ahead = [&](int tile) {                           // into L2
+    if (tile >= p.tiles) return;
+    const int64_t at = table_row(tile);
+    auto lines = [&](const void* table) {
+      const uint8_t* q = static_cast<const uint8_t*>(table) + at * kEntry;
+      for (int o = g_first * kEntry; o < g_end * kEntry; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(q + (g_end - 1) * kEntry));
+    };
+    lines(p.scales);
+    if constexpr (QK != kMx4) lines(p.biases);
+  };
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < p.boxes; ++i) { init(kWFull + 8 * i, 1); init(kWEmpty + 8 * i, 4); }
+    for (int i = 0; i < kASlots; ++i) { init(kAFull + 8 * i, 4); init(kAEmpty + 8 * i, 1); }
+    for (int i = 0; i < kDSlots; ++i) { init(kDFull + 8 * i, 1); init(kDEmpty + 8 * i, kAddWarps); }
+    for (int i = 0; i < 2; ++i) { init(kXFull + 8 * i, 1); init(kXFree + 8 * i, kAddWarps * csize); }
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(abort_at), "r"(0) : "memory");
+    mbar_init_fence();
+    const int tile0 = static_cast<int>(first % p.tiles);
+    for (int b = 0; b < p.boxes && b < nsteps && items; ++b) {        // the first boxes travel while the rest is set up
+      mbar_expect_tx(smem + kWFull + 8 * b, kBox);
+      tma_load_2d(&w_map, w_at + b * kBox, smem + kWFull + 8 * b, (step0 + b) * kBoxBytes, tile0 * kTileRows);
+    }
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem + kTmemSlot), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp >= kAddWarp && items) ahead(static_cast<int>(first % p.tiles));
+  tc_fence_before();
+  __syncthreads();
+  if (csize > 1) cluster_barrier();
+  tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(smem + kTmemSlot) : "memory");
+  tmem = __shfl_sync(0xffffffffu, tmem, 0);
+
+  bool ok = true;
+  // where each role is in its rings, over all chunks
+  uint32_t slot = 0, phase = 0;                          // producer: box; issuer: slot of A
+  uint32_t dslot = 0, dphase = 0;                        // issuer and adding up: accumulator
+  uint32_t steps_before = 0;                             // the teams: steps of earlier tiles
+  int added = 0;                                         // adding up: tiles pushed
+  int late_tile = -1;                                    // ... and the one that is to be added up (a tile late)
+  int64_t late_row = 0;
+  bool issued = false;
+
+  // The owner's part of a tile: 128 / csize of its rows, the CTAs' partial sums in rank order.
+  const int own_shift = 7 - (31 - __clz(csize)), own = 1 << own_shift;
+  auto add_up = [&](int item, int tile, int64_t row0) -> bool {
+    const uint32_t s = p.slots == 1 ? 0u : item & 1u, ph = (p.slots == 1 ? item : item >> 1) & 1u;
+    const int thread = (warp - kAddWarp) * 32 + lane;
+    if (thread == 0) mbar_expect_tx(smem + kXFull + 8 * s, kTileRows * T * 4);
+    if (!wait_phase<true>(smem + kXFull + 8 * s, ph, abort_at, 35)) return false;
+    __syncwarp();
+    const uint32_t from = part_at + s * partial_bytes(T);
+    constexpr int kAdders = 32 * kAddWarps, kMost = kTileRows * (T / 4) / kAdders;       // (all of a tile's rows are this CTA's where there is no cluster)
+#pragma unroll 2
+    for (int j = 0; j < kMost; ++j) {
+      const int i = thread + j * kAdders;
+      if (i >= own * (T / 4)) break;
+      const int r = i & (own - 1), t4 = i >> own_shift;
+      const uint32_t at = from + r * kRow + t4 * 16;
+      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      auto sum = [&](auto count) {
+#pragma unroll
+        for (int c = 0; c < decltype(count)::value; ++c) {
+          const float4 f = ldsf128<0>(at + (c << own_shift) * kRow);
+          v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
+        }
+      };
+      if (csize == 8) sum(std::integral_constant<int, 8>());
+      else if (csize == 4) sum(std::integral_constant<int, 4>());
+      else if (csize == 2) sum(std::integral_constant<int, 2>());
+      else sum(std::integral_constant<int, 1>());
+      const int64_t n = static_cast<int64_t>(tile) * kTileRows + rank * own + r, m = row0 + t4 * 4;
+      int64_t o = m * p.N + n;
+      const int left = n < p.N ? static_cast<int>(p.M - m < 4 ? p.M - m : 4) : 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (e < left) {
+          if (p.y_dtype == QMM_F32) reinterpret_cast<float*>(p.y)[o] = v[e];
+          else if (p.y_dtype == QMM_BF16) reinterpret_cast<__nv_bfloat16*>(p.y)[o] = __float2bfloat16_rn(v[e]);
+          else reinterpret_cast<__half*>(p.y)[o] = __float2half_rn(v[e]);
+        }
+        o += p.N;
+      }
+    }
+    __syncwarp();                                        // this warp has read its part of the slot: tell those who fill it
+    if (lane < csize) remote_arrive_release(in_cta(smem + kXFree + 8 * s, lane));
+    return true;
+  };
+
+  for (int done = 0; done < items && ok;) {
+    const unsigned chunk = (first + done) / p.tiles;
+    const int tile0 = same(static_cast<int>(first + done - chunk * p.tiles)), tiles = same(items - done < p.tiles - tile0 ? items - done : p.tiles - tile0);
+    const int64_t row0 = static_cast<int64_t>(chunk) * T;
+
+    if (done == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // ---- this CTA's stretch of K of the chunk's rows, as three pieces ----
+    {
+      const int pieces = nsteps * 16, units = T * pieces;
+      const unsigned inverse = nsteps == p.most_steps ? p.most_inverse : p.less_inverse;
+      auto row_of = [&](int u) -> int { return static_cast<int>(__umulhi(static_cast<unsigned>(u), inverse)); };
+      constexpr int kAtOnce = 4;                         // requests in flight
+      for (int u0 = threadIdx.x; u0 < units; u0 += kThreads * kAtOnce) {
+        float4 a[kAtOnce], b[kAtOnce];
+#pragma unroll
+        for (int j = 0; j < kAtOnce; ++j) {
+          const int u = u0 + j * kThreads, t = row_of(u), k = step0 * kStepK + (u - t * pieces) * 8;
+          const int64_t m = row0 + t;
+          a[j] = b[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (u < units && m < p.M && k < p.K) {
+            const float4* src = reinterpret_cast<const float4*>(p.x + m * p.K + k);
+            a[j] = __ldg(src);
+            b[j] = __ldg(src + 1);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < kAtOnce; ++j) {
+          const int u = u0 + j * kThreads, t = row_of(u), c = u - t * pieces;
+          if (u >= units) continue;                      // (whole warps: a row has eight pieces a block, and T is a multiple of 16)
+          float f[8] = {a[j].x, a[j].y, a[j].z, a[j].w, b[j].x, b[j].y, b[j].z, b[j].w};
+          float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+          const bool odd = !(fabsf(sum) <= 3.402823466e38f);       // an infinity or a NaN among them, perhaps
+          if constexpr (QK != kMx4) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            if ((lane & 3) == 0) sts32(sums_at + ((c >> 2) * T + t) * 4, sum);
+          }
+          // A piece is the eight bits of a mantissa that come next, cut off: what it leaves over is exact. An infinity leaves nothing (not a NaN), and a
+          // NaN stays one.
+          const uint32_t to = x_at + (c >> 3) * kXBlock + t * 128 + (((c ^ t) & 7) << 4);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            uint32_t h[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) h[e] = __byte_perm(__float_as_uint(f[2 * e]), __float_as_uint(f[2 * e + 1]), 0x7632);
+            sts128(to + i * kPiece, __uint_as_float(h[0]), __uint_as_float(h[1]), __uint_as_float(h[2]), __uint_as_float(h[3]));
+            if (i < 2) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) f[e] -= __uint_as_float(__float_as_uint(f[e]) & 0xffff0000u);
+              if (i == 0 && odd) {
+                const float was[8] = {a[j].x, a[j].y, a[j].z, a[j].w, b[j].x, b[j].y, b[j].z, b[j].w};
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                  if (fabsf(was[e]) > 3.402823466e38f && was[e] == was[e]) f[e] = 0.0f;
+              }
+            }
+          }
+        }
+      }
+    }
+    fence_proxy_async();
+    __syncthreads();
+
+    if (warp == 0) {
+      // ---------------- weights ----------------
+      if (lane == 0) {
+        for (int i = 0; ok && i < tiles; ++i) {
+          for (int b = 0; b < nsteps; ++b) {
+            if (done || i || b >= p.boxes) {             // (the first ones went out at the start)
+              if (!(ok = wait(kWEmpty + 8 * slot, phase ^ 1u, 31))) break;
+              mbar_expect_tx(smem + kWFull + 8 * slot, kBox);
+              tma_load_2d(&w_map, w_at + slot * kBox, smem + kWFull + 8 * slot, (step0 + b) * kBoxBytes, (tile0 + i) * kTileRows);
+            }
+            if (++slot == static_cast<uint32_t>(p.boxes)) { slot = 0; phase ^= 1u; }
+          }
+        }
+      }
+    } else if (warp == 1) {
+      // ---------------- MMA issuer ----------------
+      // first piece and second side by side, 2 T columns; the third on top of the second
+      constexpr uint32_t idesc1 = instr_desc(1, kTileRows) | (static_cast<uint32_t>(T >> 3) << 17), idesc2 = instr_desc(1, kTileRows) | (static_cast<uint32_t>(T >> 2) << 17);
+      // (variables of this branch alone, known to be the same in all lanes, and one loop that is left where all lanes have seen a wait run out)
+      uint32_t as = same(slot), aph = same(phase), ds = same(dslot), dph = same(dphase);
+      const int total = same(tiles * nsteps);
+      int b = 0;
+      for (int i = 0; i < total; ++i) {
+        if (!__all_sync(0xffffffffu, wait(kAFull + 8 * as, aph, 32))) break;
+        bool there = true;
+#pragma unroll 1
+        for (int u = 0; u < (halves ? 4 : 2); ++u) {     // the step's accumulators
+          there = wait(kDEmpty + 8 * ds, dph ^ 1u, 33);
+          if (!__all_sync(0xffffffffu, there)) break;
+          tc_fence_after();
+          const uint32_t d = tmem + kDAt + ds * (2 * T);
+          if (!halves) {
+            const uint32_t acol = tmem + kASlotsAt + as * 64 + u * 32, desc = desc_low(x_at + (2 * b + u) * kXBlock);
+            tc_mma_block<false>(d, acol, desc, kDescHigh, idesc2, 0u);
+            tc_mma_block<false>(d + T, acol, desc + 2 * (kPiece / 16), kDescHigh, idesc1, 1u);
+          } else {
+            const uint32_t acol = tmem + kASlotsAt + as * 64 + u * 16, desc = desc_low(x_at + (2 * b + (u >> 1)) * kXBlock) + (u & 1) * 4;
+            tc_mma_half(d, acol, desc, kDescHigh, idesc2, 0u);
+            tc_mma_half(d + T, acol, desc + 2 * (kPiece / 16), kDescHigh, idesc1, 1u);
+          }
+          tc_commit<false>(smem + kDFull + 8 * ds, 0);
+          if (++ds == kDSlots) { ds = 0; dph ^= 1u; }
+        }
+        if (!__all_sync(0xffffffffu, there)) break;
+        tc_commit<false>(smem + kAEmpty + 8 * as, 0);
+        issued = true;
+        if (++as == kASlots) { as = 0; aph ^= 1u; }
+        if (++b == nsteps) b = 0;
+      }
+      slot = as; phase = aph; dslot = ds; dphase = dph;
+      // (done with the chunk, or gave up: what was issued completes before the activations are overwritten or tensor memory is given back)
+      if (issued) mbar_drain(smem + kAEmpty + 8 * (slot ? slot - 1 : kASlots - 1), slot ? phase : phase ^ 1u);
+    } else if (warp < kAddWarp) {
+      // ---------------- codes -> A ----------------
+      const int team = (warp - 2) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+      // 16-byte chunk c of a row lies at chunk c XOR row & 7 (rows of 128 bytes) or row / 2 & 3 (of 64): the TMA unit's swizzle of that width
+      const uint32_t wrow = w_at + row * kBoxBytes, chunk0 = (kBoxBytes == 128 ? row & 7 : (row >> 1) & 3) << 4, to = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kASlotsAt;
+      const uint32_t n_end = steps_before + tiles * nsteps;
+      for (uint32_t n = steps_before + ((team - steps_before) & (kTeams - 1)); n < n_end; n += kTeams) {
+        // (the slot first: it says that the step kASlots before is done with, and so that the box before in this step's place, of kASlots or more, is too)
+        const uint32_t lap = n / p.boxes, bs = n - lap * p.boxes;
+        if (!(ok = wait(kAEmpty + 8 * (n % kASlots), (n / kASlots & 1u) ^ 1u, 34) && wait(kWFull + 8 * bs, lap & 1u, 36))) break;
+        __syncwarp();
+        tc_fence_after();
+        const uint32_t from = wrow + bs * kBox;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {                    // 32 codes -> 16 columns
+          uint32_t out[16];
+#pragma unroll
+          for (int c = 0; c < kRowBytes / 32; ++c) {
+            const uint4 v = lds128<0>(from + (((q * (kRowBytes / 32) + c) << 4) ^ chunk0));
+            const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+            codes16<QK>(words, out + c * 8);
+          }
+          tmem_st16(to + (n % kASlots) * 64 + q * 16, out);
+        }
+        __syncwarp();
+        if (lane == 0) arrive_n(smem + kWEmpty + 8 * bs, 1);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_n(smem + kAFull + 8 * (n % kASlots), 1);
+      }
+      steps_before = n_end;
+    } else {
+      // ---------------- adding up ----------------
+      constexpr int kOwn = T / 2;                        // activation rows of four warps
+      const int t_own = (warp - kAddWarp) / 4 * kOwn;
+      const uint32_t from = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kDAt + t_own;
+      struct Entries { uint32_t v[WIDE ? 4 : QK == kMx4 ? 1 : 2]; };
+      const bool aligned = p.groups % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.scales) | (QK == kMx4 ? 0 : reinterpret_cast<uintptr_t>(p.biases))) & 15) == 0;
+      auto entries = [&](const void* table, int64_t trow, int g) -> Entries {      // of groups g .. g + 3
+        Entries e;
+        if (aligned) {
+          const uint8_t* q = static_cast<const uint8_t*>(table) + (trow + g) * kEntry;
+          if constexpr (WIDE) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(q));
+            e.v[0] = u.x; e.v[1] = u.y; e.v[2] = u.z; e.v[3] = u.w;
+          } else if constexpr (QK == kMx4) {
+            e.v[0] = __ldg(reinterpret_cast<const uint32_t*>(q));
+          } else {
+            const uint2 u = __ldg(reinterpret_cast<const uint2*>(q));
+            e.v[0] = u.x; e.v[1] = u.y;
+          }
+        } else {
+          uint32_t one[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int64_t at = trow + min(g + i, p.groups - 1);
+            if constexpr (WIDE) one[i] = __ldg(static_cast<const uint32_t*>(table) + at);
+            else if constexpr (QK == kMx4) one[i] = __ldg(static_cast<const uint8_t*>(table) + at);
+            else one[i] = __ldg(static_cast<const uint16_t*>(table) + at);
+          }
+          if constexpr (WIDE) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) e.v[i] = one[i];
+          } else if constexpr (QK == kMx4) {
+            e.v[0] = one[0] | one[1] << 8 | one[2] << 16 | one[3] << 24;
+          } else {
+            e.v[0] = one[0] | one[1] << 16; e.v[1] = one[2] | one[3] << 16;
+          }
+        }
+        return e;
+      };
+      auto value = [&](const Entries& e, int i) -> float {
+        if constexpr (WIDE) return __uint_as_float(e.v[i]);
+        else if constexpr (QK == kMx4) return __uint_as_float(max((e.v[0] >> (8 * i) & 0xffu) << 23, 0x00400000u));      // 2^(e8 - 127)
+        else return table_value(e.v[i >> 1] >> (16 * (i & 1)) & 0xffffu, p.table_dtype);
+      };
+      const int g_batch = g_first & ~3;
+      Entries sc = {}, bi = {};                          // of the tile's first groups
+      auto first_entries = [&](int tile) {
+        sc = entries(p.scales, table_row(tile), g_batch);
+        if constexpr (QK != kMx4) bi = entries(p.biases, table_row(tile), g_batch);
+      };
+      first_entries(tile0);
+      for (int i = 0; ok && i < tiles; ++i) {
+        const int tile = tile0 + i;
+        const int64_t trow = table_row(tile);
+        Entries sc_next = sc, bi_next = bi;
+        ahead(i + 1 < tiles ? tile + 1 : p.tiles);
+        float y[kOwn];
+#pragma unroll
+        for (int t = 0; t < kOwn; ++t) y[t] = 0.0f;
+        // (sums of 512 codes at a time, as in the few-rows kernel: a rounding is relative to the sum so far. 48 rows have no more.)
+        constexpr bool kTwoLevels = T < 48;
+        const int kLong = halves ? 16 : 8;
+        float total[kTwoLevels ? kOwn : 1];
+#pragma unroll
+        for (int t = 0; t < (kTwoLevels ? kOwn : 1); ++t) total[t] = 0.0f;
+        bool biased = false;
+        int unit = step0 * (halves ? 4 : 2);             // the accumulator that comes next, in 32 or 64 codes
+        const int units_end = (step0 + nsteps) * (halves ? 4 : 2), per_group = p.group_shift == 7 ? 1 : 0;
+        int sum_end = unit + kLong;                      // where the sums of this stretch join those before
+#pragma unroll 1
+        for (int g0 = g_batch; ok && unit < units_end; g0 += 4) {
+          if (kTwoLevels && unit >= sum_end) {
+#pragma unroll
+            for (int t = 0; t < (kTwoLevels ? kOwn : 0); ++t) {
+              total[t] += y[t];
+              y[t] = 0.0f;
+            }
+            sum_end += kLong;
+          }
+          if (g0 + 4 < g_end) {                          // (the next four are on their way while these are used)
+            sc_next = entries(p.scales, trow, g0 + 4);
+            if constexpr (QK != kMx4) bi_next = entries(p.biases, trow, g0 + 4);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int g = g0 + e;
+            // (the second half of a last block that ends with its first lies past the last group: its sums are nought)
+            const float s = g < p.groups ? value(sc, e) : 0.0f;
+            if constexpr (QK != kMx4) biased |= g < p.groups && g >= g_first && fmaf(kCentre, s, value(bi, e)) != 0.0f;
+#pragma unroll 1
+            while (unit < units_end && unit >> per_group == g) {
+              ok = wait(kDFull + 8 * dslot, dphase, 37);
+              if (!(ok = __all_sync(0xffffffffu, ok))) break;
+              tc_fence_after();
+              const uint32_t d = from + dslot * (2 * T);
+#pragma unroll
+              for (int t = 0; t < kOwn; t += 8) {
+                uint32_t hi[8], lo[8];
+                tmem_ld(d + t, hi);
+                tmem_ld(d + T + t, lo);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) add_fma2(y[t + j], y[t + j + 1], s, hi + j, lo + j);
+              }
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) arrive_n(smem + kDEmpty + 8 * dslot, 1);
+              if (++dslot == kDSlots) { dslot = 0; dphase ^= 1u; }
+              ++unit;
+            }
+            if (!ok) break;
+          }
+          sc = sc_next;
+          bi = bi_next;
+        }
+        if (!ok) break;
+        if (kTwoLevels) {
+#pragma unroll
+          for (int t = 0; t < (kTwoLevels ? kOwn : 0); ++t) y[t] += total[t];
+        }
+        if constexpr (kUnit != 1.0f) {
+#pragma unroll
+          for (int t = 0; t < kOwn; ++t) y[t] *= kUnit;
+        }
+        if constexpr (QK != kMx4) {
+          if (__any_sync(0xffffffffu, biased)) {         // (b + C s) sum x, in sums of its own
+#pragma unroll
+            for (int t0 = 0; t0 < kOwn; t0 += 8) {
+              float yb[8];
+#pragma unroll
+              for (int t = 0; t < 8; ++t) yb[t] = 0.0f;
+#pragma unroll 1
+              for (int g = g_first; g < g_end; ++g) {
+                const Entries s1 = entries(p.scales, trow, g & ~3), b1 = entries(p.biases, trow, g & ~3);
+                float bc = 0.0f;
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                  if ((g & 3) == e) bc = fmaf(kCentre, value(s1, e), value(b1, e));
+                const int lo = ((g << p.group_shift) - step0 * kStepK) >> 5, hi = lo + (1 << p.group_shift >> 5);
+#pragma unroll
+                for (int t = 0; t < 8; t += 4) {
+                  float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                  for (int u = lo; u < hi; ++u) {
+                    const float4 v = ldsf128<0>(sums_at + (u * T + t_own + t0 + t) * 4);
+                    f.x += v.x; f.y += v.y; f.z += v.z; f.w += v.w;
+                  }
+                  fma2(yb[t], yb[t + 1], bc, f.x, f.y);
+                  fma2(yb[t + 2], yb[t + 3], bc, f.z, f.w);
+                }
+              }
+#pragma unroll
+              for (int t = 0; t < 8; ++t) y[t0 + t] += yb[t];
+            }
+          }
+        }
+        if (i + 1 < tiles) first_entries(tile + 1);      // (on their way while this tile is passed on)
+        // to the CTA that owns this row
+        const uint32_t s = p.slots == 1 ? 0u : added & 1u, ph = (p.slots == 1 ? added : added >> 1) & 1u;
+        ok = wait_phase<true>(smem + kXFree + 8 * s, ph ^ 1u, abort_at, 38);
+        if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        const int owner = trow_lane >> own_shift;
+        const uint32_t bar = in_cta(smem + kXFull + 8 * s, owner);
+        const uint32_t to = in_cta(part_at + s * partial_bytes(T) + ((rank << own_shift) + (trow_lane & (own - 1))) * kRow + t_own * 4, owner);
+#pragma unroll
+        for (int t = 0; t < kOwn; t += 4) st_async4(to + t * 4, bar, y[t], y[t + 1], y[t + 2], y[t + 3]);
+        if (p.slots == 1) {
+          if (!(ok = add_up(added, tile, row0))) break;
+        } else {
+          if (late_tile >= 0 && !(ok = add_up(added - 1, late_tile, late_row))) break;
+          late_tile = tile;
+          late_row = row0;
+        }
+        ++added;
+      }
+    }
+    done += tiles;
+    __syncthreads();                                     // every role is done with the chunk's activations
+    uint32_t gave_up;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(gave_up) : "r"(abort_at) : "memory");
+    ok = ok && gave_up == 0;
+    if (!ok && warp == 0 && lane == 0)                   // somebody gave up: the boxes on the way land first
+      for (uint32_t i = 0; i < static_cast<uint32_t>(p.boxes); ++i) mbar_drain(smem + kWFull + 8 * i, i < slot ? phase : phase ^ 1u);
+  }
+  if (warp >= kAddWarp && ok && late_tile >= 0) add_up(added - 1, late_tile, late_row);
+
+  tc_fence_before();
+  __syncthreads();
+  if (csize > 1) {
+    __syncwarp();
+    cluster_barrier();                                   // nobody leaves while a peer may still write to its shared memory
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+  if (threadIdx.x == 0) {
+    int gave_up;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(gave_up) : "r"(abort_at) : "memory");
+    if (gave_up) atomicCAS(p.status, 0, gave_up);
+  }
+}
+
+struct F32Plan {
+  int t, cluster, most_steps, slots, boxes;      // t == 0: the activations do not fit
+};
+
+// The plan of the least load, in clocks of the busiest cluster: rounds of tiles x (its K blocks, plus what a tile costs besides: the push, the sum), and the
+// conversion of the activations. What it picks against the best of all plans, us (float32 tables, the few-rows kernel last): 33 rows 4096 x 4096 24.0 / 24.0 / 34.8,
+// 64 rows 14336 x 4096 82.8 / 82.8 / 178, 4096 x 14336 114 / 114 / 234, 8-bit 64 rows 16384 x 1536 41 / 41 / 102, mxfp4 33 rows 5760 x 2880 26.2 / 26.2 / 47.3,
+// 12 rows 65536 x 512 21.0 / 20.9 / 35.4, 1024 x 14336 18.1 / 18.0 / 20.4, 10 rows 4096 x 4096 13.9 / 13.9 / 17.0, 20 rows 2048 x 1024 in groups of 32 8.0 / 8.0 / 8.2.
+F32Plan plan_of(const qmm_problem& p) {
+  const int64_t steps_all = (p.K + kStepK - 1) / kStepK, tiles = (p.N + kTileRows - 1) / kTileRows;
+  const int sms = device_sm_count(), bits = p.mode != QMM_MODE_MXFP4 && p.bits == 8 ? 8 : 4;
+  F32Plan best = {};
+  double least = 0.0;
+  for (int c = kMaxCluster; c >= 1; c /= 2) {
+    if (c > steps_all) continue;
+    const int steps = static_cast<int>((steps_all + c - 1) / c);
+    for (int t = 48; t >= 16; t -= 16) {
+      // (48 rows' sums are of 512 codes: see kTwoLevels)
+      if ((t == 48 && steps > 4) || smem_of(t, steps, 1, kASlots, bits) > kSmemLimit) continue;
+      const int64_t chunks = (p.M + t - 1) / t, items = chunks * tiles, clusters = sms / c < items ? sms / c : items, rounds = (items + clusters - 1) / clusters;
+      const double passes = static_cast<double>(chunks < rounds ? chunks : rounds);
+      const double load = rounds * (steps * 2 * (180.0 + 2.0 * t) + (c > 1 ? 250.0 + 200.0 * c : 400.0) + 10.0 * t) + passes * steps * t * 10.0;
+      if (!best.t || load < least) {
+        least = load;
+        const int slots = smem_of(t, steps, 2, kASlots, bits) <= kSmemLimit ? 2 : 1, boxes = static_cast<int>((kSmemLimit - smem_of(t, steps, slots, 0, bits)) / box_bytes(bits));
+        best = {t, c, steps, slots, boxes < kMaxBoxes ? boxes : kMaxBoxes};
+      }
+    }
+  }
+  return best;
+}
+
+template <int QK, int T, bool WIDE>
+int launch_w(const qmm_problem& p, const F32Plan& pl, const CUtensorMap& wm, F32Params& fp, cudaStream_t stream) {
+  auto kernel = qmm_f32_tc_kernel<QK, T, WIDE>;
+  static bool configured[kMaxDevices] = {};     // the attribute is per device
+  const int dev = current_device();
+  if (dev < 0) return QMM_ERR_DEVICE;
+  if (!configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e != cudaSuccess) return fail(QMM_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    configured[dev] = true;
+  }
+  const int64_t items = (p.M + T - 1) / T * fp.tiles;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem_of(T, pl.most_steps, pl.slots, pl.boxes, QK == kAff8 ? 8 : 4);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = pl.cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int64_t clusters = device_sm_count() / pl.cluster;
+  if (pl.cluster > 1) {
+    cfg.gridDim = dim3(static_cast<unsigned>(clusters * pl.cluster));
+    const int most = max_active_clusters(reinterpret_cast<const void*>(kernel), cfg, pl.cluster);
+    if (most > 0 && clusters > most) clusters = most;
+  }
+  if (clusters > items) clusters = items;
+  if (clusters < 1) clusters = 1;
+  cfg.gridDim = dim3(static_cast<unsigned>(clusters * pl.cluster));
+  fp.share = static_cast<unsigned>(items / clusters);
+  fp.share_more = static_cast<unsigned>(items % clusters);
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, wm, fp);
+  if (e != cudaSuccess) return fail(QMM_ERR_CUDA, "qmm_f32_tc_kernel launch: %s", cudaGetErrorString(e));
+  count_launch();
+  return check_launch("qmm_f32_tc_kernel");
+}
+
+template <int QK, int T>
+int launch_t(const qmm_problem& p, const F32Plan& pl, const CUtensorMap& wm, F32Params& fp, cudaStream_t stream) {
+  if constexpr (QK != kMx4)
+    if (p.table_dtype == QMM_F32) return launch_w<QK, T, true>(p, pl, wm, fp, stream);
+  return launch_w<QK, T, false>(p, pl, wm, fp, stream);
+}
+
+template <int QK>
+int launch_kind(const qmm_problem& p, const F32Plan& pl, const CUtensorMap& wm, F32Params& fp, cudaStream_t stream) {
+  if (pl.t == 48) return launch_t<QK, 48>(p, pl, wm, fp, stream);
+  if (pl.t == 32) return launch_t<QK, 32>(p, pl, wm, fp, stream);
+  return launch_t<QK, 16>(p, pl, wm, fp, stream);
+}
+
+}  // namespace
+
+bool f32_tc_pays(const qmm_problem& p) {
+  if (p.x_dtype != QMM_F32 || p.batch != 1 || p.lhs_idx || p.rhs_idx || p.group_sizes || p.mode == QMM_MODE_FLOAT) return false;
+  if (p.M <= 8 || p.K < kBK || p.K % 32 || p.K >= (1LL << 24) || p.N < 1 || p.N >= (1LL << 31) - 256) return false;
+  if ((p.M + 15) / 16 * ((p.N + kTileRows - 1) / kTileRows) >= (1LL << 31)) return false;
+  return plan_of(p).t != 0;
+}
+
+int launch_f32_tc(const qmm_problem& p, cudaStream_t stream) {
+  const F32Plan pl = plan_of(p);
+  const bool mx = p.mode == QMM_MODE_MXFP4;
+  const int bits = !mx && p.bits == 8 ? 8 : 4, group = mx ? 32 : p.group_size;
+  F32Params fp = {};
+  fp.x = static_cast<const float*>(p.x); fp.scales = p.scales; fp.biases = p.biases; fp.y = p.y;
+  fp.status = device_status_word();
+  if (!fp.status) return fail(QMM_ERR_CUDA, "could not allocate the device status word");
+  fp.M = p.M; fp.N = p.N; fp.K = static_cast<int>(p.K);
+  fp.groups = fp.K / group;
+  fp.group_shift = group == 128 ? 7 : group == 64 ? 6 : 5;
+  fp.table_dtype = p.table_dtype; fp.y_dtype = p.y_dtype;
+  fp.tiles = static_cast<int>((p.N + kTileRows - 1) / kTileRows);
+  fp.steps = (fp.K + kStepK - 1) / kStepK;
+  fp.most_steps = pl.most_steps; fp.cluster = pl.cluster; fp.slots = pl.slots; fp.boxes = pl.boxes;
+  fp.most_inverse = 0xFFFFFFFFu / (16 * pl.most_steps) + 1;
+  fp.less_inverse = 0xFFFFFFFFu / (16 * (pl.most_steps > 1 ? pl.most_steps - 1 : 1)) + 1;
+  const uint64_t row_bytes = static_cast<uint64_t>(p.K) * bits / 8;
+  CUtensorMap wm;
+  const int rc = tensor_map_2d(&wm, QMM_U8, p.w, row_bytes, static_cast<uint64_t>(p.N), row_bytes, kStepK * bits / 8, kTileRows, bits == 8 ? 1 : 2);
+  if (rc) return rc;
+  if (mx) return launch_kind<kMx4>(p, pl, wm, fp, stream);
+  if (bits == 8) return launch_kind<kAff8>(p, pl, wm, fp, stream);
+  return launch_kind<kAff4>(p, pl, wm, fp, stream);
+}
+
+}  // namespace qmm

@@ -56,6 +56,9 @@ struct RowsGather {            // grouped products whose rows of x are picked by
 // `exact`: 16-bit activations whose sums are to be as exact as plain float32 ones (float32 activations' always are).
 int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr, bool exact = false);
 bool rows_supports(const qmm_problem& p);
+// Float32 activations of more than a few rows on the tensor cores (f32_tc_pays: it takes them, and wins).
+int launch_f32_tc(const qmm_problem& p, cudaStream_t stream);
+bool f32_tc_pays(const qmm_problem& p);
 bool rows_grouped_pays(const qmm_problem& p);
 // A checked problem on the kernel its route names; and whether that is the few-rows kernel for a grouped one.
 int run_problem(const qmm_problem& p, cudaStream_t stream);
@@ -115,9 +118,9 @@ int read_status_word(int* out);
 
 // Encodes a 2-D TMA descriptor (a CUtensorMap, 128 bytes at `map_out`): `inner` x `outer`
 // elements of kind `elem_kind` (a qmm_elem; QMM_U8 for raw bytes), rows `row_bytes` apart,
-// copied in boxes of box_inner x box_outer, optionally in the 128-byte swizzle.
+// copied in boxes of box_inner x box_outer, in the 128-byte (swizzle 1) or the 64-byte one (2), or in none (0).
 int tensor_map_2d(void* map_out, int elem_kind, const void* base, uint64_t inner, uint64_t outer,
-                  uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle128);
+                  uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle);
 
 // The current device's word in which kernels record a bounded wait that ran out (one word per
 // device, allocated on first use and kept), or NULL.

@@ -31,7 +31,7 @@ EncodeTiledFn encode_fn() {
 }  // namespace
 
 int tensor_map_2d(void* map_out, int elem_kind, const void* base, uint64_t inner, uint64_t outer,
-                  uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle128) {
+                  uint64_t row_bytes, uint32_t box_inner, uint32_t box_outer, int swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(QMM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_UINT8;
@@ -44,7 +44,7 @@ int tensor_map_2d(void* map_out, int elem_kind, const void* base, uint64_t inner
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(static_cast<CUtensorMap*>(map_out), dt, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  swizzle == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(QMM_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return QMM_OK;

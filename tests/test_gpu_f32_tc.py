@@ -1,0 +1,103 @@
+"""Float32 activations on the tensor cores at the sizes where the split can go wrong -- one row more than the few-rows kernel
+keeps, chunks of 16, 32 and 48 rows and one more, a last step of K that is half or a quarter full, one tile and a ragged last one, one to eight
+CTAs to a tile, tables whose rows start on no word, biases that are not the centre's -- against the exact product of the oracle. Needs a B200.
+
+Tolerance: 4e-7 of the result's norm (2^-24 = 6e-8 for each of: an activation's three pieces, which are exact; a tensor core's truncated sum
+of 16 products, four in a row; the scaled sums of up to 8 groups and of up to 8 CTAs, square roots of that many)."""
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import activations, affine_case, mxfp4_case, to_numpy, to_torch
+from metaljax_b200 import _lib, qmm
+from oracle import qmm_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def _case(m, k, n, kind, gs, tdt, seed=0):
+    rng = np.random.default_rng(m * k + n + seed)
+    if kind == "mxfp4":
+        w, s, b, kw = *mxfp4_case(rng, n, k)[-2:], None, dict(group_size=32, bits=4, mode="mxfp4")
+    else:
+        (w, s, b), kw = affine_case(rng, n, k, gs, int(kind[3:]), tdt)[1:], dict(group_size=gs, bits=int(kind[3:]))
+    xs = activations(rng, (m, k), "f32")
+    exact = O.qmm_exact(xs, w, s, b, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
+    return xs, [to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV)], kw, exact
+
+
+def _far(y, exact):
+    return np.linalg.norm(to_numpy(y).astype(np.float64) - exact) / np.linalg.norm(exact)
+
+
+@pytest.mark.parametrize("m,k,n,kind,gs,tdt", [
+    (9, 64, 1, "int4", 64, "f32"),              # half a step
+    (16, 96, 127, "mxfp4", 32, None),           # three quarters of one
+    (17, 160, 129, "int4", 32, "bf16"),         # two steps, the last a quarter full; two tiles
+    (33, 4096, 640, "int4", 64, "f32"),         # 48 rows, eight CTAs
+    (49, 4096, 2500, "int4", 128, "f16"),       # two chunks, more tiles than clusters
+    (64, 2112, 385, "int8", 64, "f32"),         # 17 steps over eight CTAs
+    (100, 1088, 257, "int8", 32, "bf16"),
+    (12, 14720, 256, "int4", 128, "f32"),       # the longest stretch of K that 16 rows leave room for
+    (20, 14976, 130, "mxfp4", 32, None),        # ... and one that does not fit: the few-rows kernel
+    (48, 2880, 700, "mxfp4", 32, None),         # 90 table bytes a row
+    (31, 320, 200, "int8", 64, "f16"),
+    (200, 576, 19300, "int4", 64, "f32"),       # many tiles, no cluster
+])
+def test_float32_rows(m, k, n, kind, gs, tdt):
+    xs, args, kw, exact = _case(m, k, n, kind, gs, tdt)
+    y = qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw)
+    assert _far(y, exact) <= 4e-7
+    assert _lib.poll_status() == 0
+
+
+def test_float32_rows_with_biases_of_their_own():
+    """(b + C s) sum x is left out where it is nought for a warp's rows: here one row of a tile has one."""
+    xs, (w, s, b), kw, _ = _case(40, 512, 300, "int4", 64, "f32")
+    b = -8 * s
+    b[200, 3] = 0.7
+    exact = O.qmm_exact(xs, to_numpy(w), to_numpy(s), to_numpy(b), 64, 4)
+    assert _far(qmm.quantized_matmul(to_torch(xs, DEV), w, s, b, **kw), exact) <= 4e-7
+
+
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float16])
+def test_float32_rows_to_16_bits(out):
+    xs, args, kw, exact = _case(37, 1024, 260, "int4", 64, "f32")
+    y = qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw, out_dtype=out)
+    assert torch.equal(y, qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw).to(out))
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_float32_rows_that_are_not_finite(value):
+    """An infinity times a positive, a negative or a zero weight, as a sum of products has it; the rows beside it as ever."""
+    xs, args, kw, exact = _case(20, 1120, 300, "mxfp4", 32, None)
+    column = O.qmm_exact(np.eye(1120, dtype=np.float32)[17:18], to_numpy(args[0]), to_numpy(args[1]), None, 32, 4, mode="mxfp4")[0]
+    xs[3, 17] = value
+    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw))
+    with np.errstate(invalid="ignore"):
+        want = (np.float32(value) * column.astype(np.float32))
+    assert np.array_equal(np.isnan(y[3]), np.isnan(want)) and np.array_equal(y[3][~np.isnan(want)], want[~np.isnan(want)])
+    rest = np.arange(20) != 3
+    assert _far(to_torch(y[rest], "cpu"), exact[rest]) <= 4e-7
+
+
+def test_float32_rows_replay():
+    xs, args, kw, exact = _case(64, 2048, 1024, "int4", 64, "f32")
+    x, y = to_torch(xs, DEV), torch.zeros((64, 1024), device=DEV)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        qmm.quantized_matmul(x, *args, out=y, **kw)
+        stream.synchronize()
+        first = y.clone()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(3):
+                qmm.quantized_matmul(x, *args, out=y, **kw)
+        y.zero_()
+        graph.replay()
+        stream.synchronize()
+    assert torch.equal(y, first) and _far(first, exact) <= 4e-7
+    assert _lib.poll_status() == 0
