@@ -79,6 +79,7 @@ class Program:
         self.out_dims = [tuple(v.type.shape) for v in fn.returns]
         self.donated_params = sorted(fn.donated)
         self.param_types = [a.type for a in fn.args]
+        self.param_shapes = [tuple(t.shape) for t in self.param_types]
         self.executions = 0
 
 
@@ -158,17 +159,13 @@ def execute(program: Program, buffers) -> list:
     if len(buffers) != program.num_params:
         raise ValueError(f"{program.name} takes {program.num_params} arguments, got {len(buffers)}")
     args = []
-    for b, t in zip(buffers, program.param_types):
-        if tuple(b.dims) != tuple(t.shape):
-            raise ValueError(f"argument of shape {tuple(b.dims)} for a parameter of type {t}")
+    for b, shape in zip(buffers, program.param_shapes):
+        if b.dims != shape and tuple(b.dims) != shape:
+            raise ValueError(f"argument of shape {tuple(b.dims)} for a parameter of type {program.param_types[len(args)]}")
         args.append(b.data)
     outs = program.interp.execute(args)
     program.executions += 1
-    fn = program.interp.func
-    res = []
-    for v, t in zip(fn.returns, outs):
-        res.append(DeviceBuffer(t.contiguous(), _EL_TO_ENUM[v.type.el]))
-    return res
+    return [DeviceBuffer(t if t.is_contiguous() else t.contiguous(), enum) for enum, t in zip(program.out_types, outs)]
 
 
 def stats(program: Program) -> dict:

@@ -35,7 +35,7 @@ import weakref
 
 import torch
 
-from . import hlo, qmm
+from . import _lib, hlo, qmm
 from .qmm import Match, State, _Reject
 
 SHAPE_OPS = ("stablehlo.reshape", "stablehlo.transpose", "stablehlo.broadcast_in_dim")
@@ -887,6 +887,10 @@ class Interpreter:
         plan = st.plan
         if plan is None:
             plan = st.plan = self._plan(st)
+        if plan.steps is not None and device is not None and device.type == "cuda":
+            outs = self._run_steps(plan, st.values, args)
+            if outs is not None:
+                return outs
         hook = None
         for how, op, operands, results in plan:
             if how is not None:
@@ -903,7 +907,7 @@ class Interpreter:
         taken = st.skip | set(st.roots)
         gates = {id(op): found for op in self.func.ops if id(op) not in taken and (found := _gate(op, taken)) is not None}
         inside = {id(op) for _, ops in gates.values() for op in ops}
-        plan = []
+        plan = _Plan()
         for op in self.func.ops:
             key = id(op)
             root = st.roots.get(key)
@@ -918,7 +922,28 @@ class Interpreter:
                 plan.append((lambda op, env, *ins, fn=fn: (fn(op, *ins),), op, op.operands, op.results))
             else:                                              # loops, constants: the general walk
                 plan.append((None, _Single(op), (), ()))
+        plan.number(self.func, st)
         return plan
+
+    def _run_steps(self, plan, values, args):
+        """The plan in one native call (`_native.run_steps`), or None: run it op by op."""
+        steps = []
+        for step in plan.steps:
+            m = step[2]
+            if m.__class__ is qmm.Match:
+                if m.has_perm:
+                    return None
+                at = m.slot
+                steps.append((step[0], step[1], values[at], values[at + 1], values[at + 2] if m.mode == "affine" else None, m.gs, m.bits, qmm._mode_id(m.mode),
+                              m.out_dtype))
+            else:
+                steps.append(step)
+        outs = _lib.native().run_steps(list(args), steps, plan.returns, plan.count)
+        if outs.__class__ is int:
+            _lib.check(outs)
+        if outs is not None:
+            self.fused_calls += plan.products
+        return outs
 
     def _fused(self, root):
         from . import moe_recognizer
@@ -941,6 +966,35 @@ class Interpreter:
             return id(op) in st.skip
 
         return hook
+
+
+class _Plan(list):
+    """(how, op, operands, results) of every op that is left to run; and, where all of them are plain products and gates, `steps`: the
+    same with the function's values numbered, arguments first -- (x, result, match) or (gate, result, up)."""
+
+    steps = None
+
+    def number(self, func, st):
+        numbers = {v: i for i, v in enumerate(func.args)}
+        steps, products = [], 0
+        for how, op, operands, results in self:
+            m = st.roots.get(id(op))
+            if how is _run_gate:
+                step = (operands[0], operands[1])
+            elif m.__class__ is qmm.Match:
+                # (what `emit` has to permute, reshape or convert first, or turn round afterwards, goes its way)
+                if (m.swapped or m.bshape or len(m.mshape) != 1 or len(m.nshape) != 1 or m.lperm is not None and list(m.lperm) != [0, 1]
+                        or tuple(m.lhs.type.shape) != (m.M, m.K) or m.lhs.type.dtype not in qmm._FLOATS):
+                    return
+                step, products = (m.lhs, m), products + 1
+            else:
+                return
+            if any(v.__class__ is not qmm.Match and v not in numbers for v in step) or len(results) != 1:
+                return
+            numbers[results[0]] = len(numbers)
+            steps.append((numbers[step[0]], numbers[results[0]], step[1] if step[1].__class__ is qmm.Match else numbers[step[1]]))
+        if steps and all(v in numbers for v in func.returns):
+            self.steps, self.returns, self.count, self.products = steps, [numbers[v] for v in func.returns], len(numbers), products
 
 
 def _gate(op, taken):

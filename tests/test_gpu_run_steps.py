@@ -1,0 +1,101 @@
+"""A program of products and gates in one native call, against the same program op by op: equal bit for bit where it is taken, and declined --
+not wrong -- where an argument is laid out another way or carries a gradient. Needs a B200."""
+
+import pytest
+import torch
+
+from metaljax_b200 import _lib, recognizer
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+EL = {torch.bfloat16: "bf16", torch.float16: "f16", torch.float32: "f32"}
+
+
+def program(m, d, f, dtype, gate=True, returns_x=False):
+    """silu(x Wg) * (x Wu) Wd, or x Wg Wd; the weights as int8 codes with a scale per group of 32."""
+    el, lines, args, count = EL[dtype], [], [f"%arg0: tensor<{m}x{d}x{EL[dtype]}>"], [0]
+
+    def op(text):
+        lines.append(f"    %{count[0]} = stablehlo.{text}")
+        count[0] += 1
+        return f"%{count[0] - 1}"
+
+    def dense(x, k, n):
+        i = len(args)
+        full, small, wide = f"tensor<{n}x{k}x{el}>", f"tensor<{n}x{k // 32}x{el}>", f"tensor<{n}x{k // 32}x32x{el}>"
+        args.extend([f"%arg{i}: tensor<{n}x{k}xi8>", f"%arg{i + 1}: {small}"])
+        c = op(f"convert %arg{i} : (tensor<{n}x{k}xi8>) -> {full}")
+        b = op(f"broadcast_in_dim %arg{i + 1}, dims = [0, 1] : ({small}) -> {wide}")
+        c = op(f"multiply {c}, {op(f'reshape {b} : ({wide}) -> {full}')} : {full}")
+        return op(f"dot_general {x}, {c}, contracting_dims = [1] x [1] : (tensor<{m}x{k}x{el}>, {full}) -> tensor<{m}x{n}x{el}>")
+
+    mid = f"tensor<{m}x{f}x{el}>"
+    h = dense("%arg0", d, f)
+    if gate:
+        up = dense("%arg0", d, f)
+        act = op(f"multiply {h}, {op(f'logistic {h} : {mid}')} : {mid}")
+        h = op(f"multiply {act}, {up} : {mid}")
+    y = dense(h, f, d)
+    out = f"tensor<{m}x{d}x{el}>"
+    results = (f"({out}, {out})", f"return %arg0, {y} : {out}, {out}") if returns_x else (f"({out})", f"return {y} : {out}")
+    return "module @jit_f {\n  func.func public @main(" + ", ".join(args) + f") -> {results[0]} {{\n" + "\n".join(lines) + f"\n    {results[1]}\n  }}\n}}\n"
+
+
+def arguments(m, d, f, dtype, gate=True):
+    g = torch.Generator(device=DEV).manual_seed(m + d + f)
+    out = [torch.randn((m, d), generator=g, device=DEV).to(dtype)]
+    for n, k in ((f, d), (f, d), (d, f)) if gate else ((f, d), (d, f)):
+        out.append(torch.randint(-8, 8, (n, k), generator=g, device=DEV, dtype=torch.int8))
+        out.append((torch.rand((n, k // 32), generator=g, device=DEV) * 0.018 + 0.002).to(dtype))
+    return out
+
+
+def both(text, args):
+    """(in one call or not, the results, the results op by op)"""
+    it = recognizer.Interpreter(text)
+    it.execute(args)
+    plan = it._qmm.plan
+    if plan.steps is None:
+        return None, None, None
+    one = it._run_steps(plan, it._qmm.values, args)
+    before = it.fused_calls
+    got = it.execute(args)
+    assert it.fused_calls == before + plan.products
+    steps, plan.steps = plan.steps, None
+    want = it.execute(args)
+    plan.steps = steps
+    assert _lib.poll_status() == 0
+    return one is not None, got, want
+
+
+@pytest.mark.parametrize("m,d,f,dtype,gate,returns_x", [
+    (4, 128, 256, torch.bfloat16, True, False), (1, 64, 96, torch.float16, True, True), (33, 160, 288, torch.bfloat16, True, False),
+    (200, 256, 512, torch.float16, True, False), (3, 96, 64, torch.float32, False, True), (12, 128, 64, torch.float32, False, False),
+])
+def test_one_call_equals_op_by_op(m, d, f, dtype, gate, returns_x):
+    args = arguments(m, d, f, dtype, gate)
+    taken, got, want = both(program(m, d, f, dtype, gate, returns_x), args)
+    assert taken
+    assert all(torch.equal(a, b) and a.dtype == b.dtype for a, b in zip(got, want))
+    if returns_x:
+        assert got[0] is args[0]
+
+
+def test_what_is_not_plain_is_declined():
+    text = program(6, 128, 256, torch.bfloat16)
+    args = arguments(6, 128, 256, torch.bfloat16)
+    wide = torch.randn((6, 256), device=DEV).to(torch.bfloat16)
+    for x in (wide[:, ::2], wide[:, 64:192]):
+        taken, got, want = both(text, [x, *args[1:]])
+        assert taken is False
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    it = recognizer.Interpreter(text)
+    it.execute(args)
+    with pytest.raises(BufferError):                      # refused, as a call by itself is
+        it.execute([args[0].detach().clone().requires_grad_(), *args[1:]])
+
+
+def test_a_float32_gate_runs_op_by_op():
+    args = arguments(4, 64, 96, torch.float32)
+    assert both(program(4, 64, 96, torch.float32), args)[0] is None
