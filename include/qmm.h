@@ -269,18 +269,23 @@ int qmm_quantized_matmul_static(const qmm_tensor* x, const qmm_tensor* w, const 
 int qmm_pack_codes(const qmm_tensor* codes, qmm_tensor* out, int bits, void* stream);
 
 /* A quantized Dense layer as keras stores it (tests/test_qmm.py:179-199) made into the fused op's operands, raw
- * device pointers. The three steps of `qmm.from_keras_int4`:
+ * device pointers. The steps of `qmm.from_keras_int4`:
  *   codes   packed int8 [K, ceil(N/2)], byte j of row k = columns 2j (low nibble) and 2j + 1, two's complement
  *           -> words [N, K/8] of code + 8; *digest (zeroed by the caller) accumulates their content digest
  *   facts   scale, zero (or NULL) [G, N], K / G a multiple of 32: *facts (zeroed) gets bit 0 / 1 if they are not constant
  *           within 128 / 64 codes, bit 2 if -scale (zero + 8) does not narrow to the scales' type exactly, bit 3 if they hold
  *           a NaN or a zero point that is no integer of at most 32768
- *   tables  scales and biases = -scale (zero + 8), [N, K/group_size], float32 or (narrow) the scales' type */
+ *   tables  scales and biases = -scale (zero + 8), [N, K/group_size], float32 or (narrow) the scales' type
+ *   layer   all three in one launch, for a group_size that divides K / G, and the wait for it: *digest and *facts are host
+ *           memory and complete on return (not in a stream that is being captured: QMM_ERR_UNSUPPORTED) */
 int qmm_pack_dense_codes(const void* packed, uint32_t* words, int64_t K, int64_t N, uint64_t* digest, void* stream);
 int qmm_pack_dense_facts(const void* scale, const void* zero, int scale_dtype, int zero_dtype, int64_t G, int64_t N, int64_t K,
                          uint32_t* facts, void* stream);
 int qmm_pack_dense_tables(const void* scale, const void* zero, int scale_dtype, int zero_dtype, void* scales, void* biases,
                           int narrow, int64_t G, int64_t N, int64_t K, int group_size, void* stream);
+int qmm_pack_dense_layer(const void* packed, uint32_t* words, const void* scale, const void* zero, int scale_dtype, int zero_dtype,
+                         void* scales, void* biases, int narrow, int64_t G, int64_t N, int64_t K, int group_size,
+                         uint64_t* digest, uint32_t* facts, void* stream);
 
 /* ---- raw-pointer form (C/C++ callers such as the PJRT entry) ------------------ */
 

@@ -112,6 +112,8 @@ _SIGNATURES = {
     "qmm_pack_dense_facts": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_int] * 2 + [ctypes.c_int64] * 3 + [ctypes.c_void_p] * 2),
     "qmm_pack_dense_tables": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2 + [ctypes.c_int]
                               + [ctypes.c_int64] * 3 + [ctypes.c_int, ctypes.c_void_p]),
+    "qmm_pack_dense_layer": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2 + [ctypes.c_int]
+                             + [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.c_void_p] * 3),
     "qmm_moe_silu_mul": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
                                         ctypes.c_int, ctypes.c_void_p]),
     "qmm_moe_routed_sum": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,

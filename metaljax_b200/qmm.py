@@ -22,9 +22,9 @@ fused ops raise when libqmm or a CUDA device is missing.
 
 from __future__ import annotations
 
+import ctypes
 import math
 import os
-import threading
 import weakref
 
 import numpy as np
@@ -725,22 +725,9 @@ def unpack_keras_int4(packed: torch.Tensor, columns: int) -> torch.Tensor:
     return ((both ^ 8) - 8).to(torch.int8)
 
 
-_PINNED = threading.local()       # a few bytes of page-locked memory per thread: where a packer's facts arrive
-
-
-def _facts_arrive(index):
-    """This thread's page-locked words and event for a device's facts."""
-    kept = getattr(_PINNED, "facts", None)
-    if kept is None:
-        kept = _PINNED.facts = {}
-    if index not in kept:
-        kept[index] = (torch.empty(2, dtype=torch.int64).pin_memory(), torch.cuda.Event())
-    return kept[index]
-
-
 def _pack_dense(packed, scale, zero, k, n, out_dtype):
     """`from_keras_int4` on the GPU for consecutive groups of a multiple of 32 rows: codes and tables in one
-    kernel each and one wait for the device (which group size the tables allow, and whether the biases narrow, is in the data).
+    kernel and one wait for the device (which group size the tables allow, and whether the biases narrow, is in the data).
     None where the general way has to look (host arrays, other layouts, zero points it may reject)."""
     tables = (scale,) if zero is None else (scale, zero)
     if not all(t.is_cuda and t.is_contiguous() and t.dim() == 2 and t.device == packed.device for t in (packed, *tables)):
@@ -756,37 +743,30 @@ def _pack_dense(packed, scale, zero, k, n, out_dtype):
         return None
     lib, stream, dev = _lib.lib(), _lib.stream_ptr(packed), packed.device
     with torch.cuda.device(dev):
-        facts = torch.zeros(2, dtype=torch.int64, device=dev)               # [digest, flags]
-        at = facts.data_ptr()
         words = torch.empty((n, k // 8), dtype=torch.uint32, device=dev)
         args = (scale.data_ptr(), None if zero is None else zero.data_ptr(), _lib.ELEM[scale.dtype], 0 if zero is None else _lib.ELEM[zero.dtype])
-        _lib.check(lib.qmm_pack_dense_facts(*args, g, n, k, at + 8, stream))
-        _lib.check(lib.qmm_pack_dense_codes(packed.data_ptr(), words.data_ptr(), k, n, at, stream))
-        host, arrived = _facts_arrive(dev.index)
-        host.copy_(facts, non_blocking=True)
-        arrived.record()
-        # The tables are made while the facts travel, as nearly every layer's are: one entry per stored group (the widest
+        # The tables are made before the facts are known, as nearly every layer's are: one entry per stored group (the widest
         # group size that divides it), biases in float32 where there are zero points (a product of a scale and
-        # an integer seldom fits the scale's type; 8 times the scale does). The facts can only ask for others:
-        # [4096, 14336] 83 us, 96 with the launch after the wait.
+        # an integer seldom fits the scale's type; 8 times the scale does). The facts can only ask for others.
         may_narrow = scale.dtype != torch.float32 and _SCALE_WIDTH != "f32"
         plan = (next(s for s in _GROUP_SIZES if k // g % s == 0), may_narrow and (zero is None or _SCALE_WIDTH == "source"))
 
         def tables(group, narrow):
             scales = torch.empty((n, k // group), dtype=scale.dtype if narrow else torch.float32, device=dev)
-            biases = torch.empty_like(scales)
-            _lib.check(lib.qmm_pack_dense_tables(*args, scales.data_ptr(), biases.data_ptr(), int(narrow), g, n, k, group, stream))
-            return scales, biases
+            return scales, torch.empty_like(scales)
 
         scales, biases = tables(*plan)
-        arrived.synchronize()
-        digest, flags = host.tolist()
+        digest, flags = ctypes.c_uint64(), ctypes.c_uint32()
+        _lib.check(lib.qmm_pack_dense_layer(packed.data_ptr(), words.data_ptr(), *args, scales.data_ptr(), biases.data_ptr(), int(plan[1]), g, n, k, plan[0],
+                                            ctypes.byref(digest), ctypes.byref(flags), stream))
+        digest, flags = digest.value, flags.value
         if flags & 8:
             return None
         group = next(s for s in _GROUP_SIZES if k % s == 0 and not (flags & {128: 1, 64: 2, 32: 0}[s]))
         narrow = may_narrow and (_SCALE_WIDTH == "source" or not flags & 4)
         if (group, narrow) != plan:
             scales, biases = tables(group, narrow)
+            _lib.check(lib.qmm_pack_dense_tables(*args, scales.data_ptr(), biases.data_ptr(), int(narrow), g, n, k, group, stream))
     m = Match()
     m.mode, m.N, m.K = "affine", n, k
     m.out_dtype = out_dtype or scale.dtype

@@ -51,3 +51,35 @@ def test_a_longer_layer_than_the_device_kernels_take():
     got = qmm.from_keras_int4(packed.to(DEV), scale.to(DEV), columns=n)
     assert (got.gs, got.bits) == (want.gs, want.bits)
     assert torch.equal(got.w.cpu().view(torch.int32), want.w.view(torch.int32)) and torch.equal(got.biases.cpu(), want.biases)
+
+
+def test_layers_packed_one_after_another_and_by_several_threads():
+    """What a layer's blocks add up is nought again when the next one starts, and each call has sums of its own."""
+    import threading
+
+    layers, want = [], []
+    for i in range(6):
+        g = torch.Generator().manual_seed(i)
+        packed = torch.randint(-128, 128, (256 + 128 * i, 40), generator=g, dtype=torch.int8)
+        scale = (torch.rand((packed.shape[0] // 64, 80), generator=g) * 0.02 + 0.01).to(torch.bfloat16)
+        layers.append((packed.to(DEV), scale.to(DEV)))
+        want.append(qmm.from_keras_int4(packed, scale))
+    wrong = []
+
+    def pack(turn):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(len(layers)):
+                at = (i + turn) % len(layers)
+                got = qmm.from_keras_int4(*layers[at])
+                torch.cuda.current_stream().synchronize()
+                if not (torch.equal(got.w.cpu().view(torch.int32), want[at].w.view(torch.int32)) and torch.equal(got.scales.cpu(), want[at].scales)
+                        and torch.equal(got.biases.cpu(), want[at].biases)):
+                    wrong.append(at)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=pack, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
