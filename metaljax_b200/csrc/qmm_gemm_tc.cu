@@ -41,7 +41,7 @@
 // 64 rows 28672 x 4096 33.3 -> 30.6, 65760 x 2880 (rows of 90 table bytes) 79.3 -> 48.7, float32 tables in groups of 32 14336 x 4096 42 -> 33. What an epilogue
 // costs: 4.6 us a tile of 256 x 256 with 2-byte stores behind a check each (2.1 at 64 tokens); drained into registers and rounded first, stored in pairs of features: 64 rows 28672 x
 // 4096 30.6 -> 27.0, 512 rows mxfp4 5760 x 2880 22.8 -> 20.6, 2048 rows 14336 x 4096 183 -> 172. The weights' producer on its way before the rest is set up: 64 rows 28672 x 4096 27.0 ->
-// 26.3, 4096 x 14336 17.6 -> 17.2.
+// 26.3, 4096 x 14336 17.6 -> 17.2. MXFP4 codes looked up: 64 rows 65760 x 2880 48.1 -> 43.0; and shorter tiles where there are few: 512 rows 5760 x 2880 20.5 -> 18.8.
 // What bounds it: at 64 rows memory and the dequantizing warps together (335 clocks a K block and SM; 260 without the dequantization, 210 of them the weights' bytes) and some
 // 6 us of a launch's ends, at 256 the tensor cores (500 clocks a block between a tile's ends, under the power cap) and the ends,
 // where the accumulator is drained by the warps that would dequantize for the next tile. (Draining it after the first steps of the next
@@ -94,6 +94,7 @@ struct TcParams {
   int table_entry, skewed;     // bytes of a table entry; whether some chunk's entries start off a 16-byte boundary
   int chunk_shift;             // weight boxes per table chunk (log2)
   int64_t table_bytes;         // of a whole table
+  int tile_rows;               // token rows of a tile: the template's, or fewer where that fills the machine in one round
   int split;                   // > 1: `split` consecutive workers share the K of each tile (and the walk is one tile long): a cluster that
   int cluster_adds;            // adds up over distributed shared memory, or partial tiles for the kernel that follows
   int shared_tiles;            // the first tiles of the walk are shared out by weight boxes ...
@@ -206,28 +207,30 @@ __device__ __forceinline__ void dequant_aff8(const uint32_t (&w)[NW], float s, f
   }
 }
 
-// MXFP4, NW packed words of one 32-element group -> NW*4 pairs. The three magnitude bits of a
-// code, placed at the 16-bit type's exponent/mantissa boundary, are the E2M1 value scaled by
-// 2^-126 (bf16) or 2^-14 (f16), including the subnormal code 1 = 0.5; two exact power-of-two
-// multiplies undo that and apply the group's E8M0 scale.
+// MXFP4, NW packed words of one 32-element group -> NW*4 pairs. The group's eight magnitudes, each times the group's E8M0 scale (a product of exact values, rounded
+// once where the type cannot hold it), are made once and split into their low and their high bytes: a byte permute then looks four codes up at a time,
+// and their signs go in on top. 15 instructions a word and 8 a group; with the bits of each pair moved to the exponent's place and multiplied twice they were 29 a word.
 template <typename XT, int NW>
 __device__ __forceinline__ void dequant_mx4(const uint32_t (&w)[NW], uint32_t e8, uint32_t* out) {
   using H = Half2Ops<XT>;
   constexpr bool kBf = std::is_same<XT, __nv_bfloat16>::value;
-  constexpr int kShift = kBf ? 6 : 9;  // magnitude bit 0 -> top mantissa bit
-  const float unbias = kBf ? 8.507059173023462e37f /* 2^126 */ : 16384.0f /* 2^14 */;
-  const uint32_t u2 = H::pack(unbias, unbias);
+  // 0, 1/2 | 1, 3/2 | 2, 3 | 4, 6
+  constexpr uint32_t kMagnitudes[4] = {kBf ? 0x3F000000u : 0x38000000u, kBf ? 0x3FC03F80u : 0x3E003C00u, kBf ? 0x40404000u : 0x42004000u, kBf ? 0x40C04080u : 0x46004400u};
   const float sc = __uint_as_float(e8 ? (e8 << 23) : 0x00400000u);
   const uint32_t s2 = H::pack(sc, sc);
+  uint32_t m[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) m[i] = H::mul(kMagnitudes[i], s2);
+  const uint32_t low[2] = {permute(m[0], m[1], 0x6420), permute(m[2], m[3], 0x6420)}, high[2] = {permute(m[0], m[1], 0x7531), permute(m[2], m[3], 0x7531)};
 #pragma unroll
   for (int j = 0; j < NW; ++j) {
-    const uint32_t hi = w[j] >> 4;
+    const uint32_t codes = w[j] & 0x77777777u, even = w[j] << 4;       // (a byte of `even` has the sign of its even code on top, one of the word that of its odd one)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      // byte 0 <- byte i of w (even element in its low nibble), byte 2 <- byte i of w>>4
-      const uint32_t t = __byte_perm(w[j], hi, i | ((4 + i) << 8)) & 0x000F000Fu;
-      const uint32_t bits = ((t & 0x00070007u) << kShift) | ((t & 0x00080008u) << 12);
-      out[j * 4 + i] = H::mul(H::mul(bits, u2), s2);
+    for (int h = 0; h < 2; ++h) {                  // four codes
+      const uint32_t at = h ? codes >> 16 : codes;
+      const uint32_t lo = permute(low[0], low[1], at), hi = and_or(permute(even, w[j], h ? 0x7362 : 0x5140), 0x80808080u, permute(high[0], high[1], at));
+      out[j * 4 + 2 * h] = permute(lo, hi, 0x5140);
+      out[j * 4 + 2 * h + 1] = permute(lo, hi, 0x7362);
     }
   }
 }
@@ -280,9 +283,10 @@ struct Piece {
 // The walk of worker `w` of `workers`: its stretch of the shared tiles from the end, then every workers-th tile.
 template <int BT, int kPer>
 struct Walk {
-  int lo, hi, next, w, workers, boxes, num_kb, tiles;
+  int lo, hi, next, w, workers, boxes, num_kb, tiles, tile_rows;
   __device__ __forceinline__ Walk(const TcParams& p, int w_, int workers_, int num_kb_, int tiles_) : w(w_), workers(workers_), num_kb(num_kb_), tiles(tiles_) {
     boxes = (num_kb + kPer - 1) / kPer;
+    tile_rows = p.tile_rows;
     lo = hi = 0;
     if (p.split > 1) {                             // one piece, its stretch of K of the cluster's tile
       const int tile = w / p.split, part = w - tile * p.split;
@@ -327,9 +331,9 @@ struct Walk {
     // tile and stream disjoint weight rows
     const unsigned tt = local / static_cast<unsigned>(ftiles), ft = local - tt * static_cast<unsigned>(ftiles);
     out->seg = s;
-    out->row0 = seg_row0[s] + static_cast<int64_t>(tt) * BT;
+    out->row0 = seg_row0[s] + static_cast<int64_t>(tt) * static_cast<unsigned>(tile_rows);
     const int64_t left = seg_row0[s + 1] - out->row0;
-    out->rows = static_cast<int>(left < BT ? left : BT);
+    out->rows = static_cast<int>(left < tile_rows ? left : tile_rows);
     out->f0 = static_cast<int64_t>(ft) * features;
     return true;
   }
@@ -392,7 +396,7 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
         int64_t r = p.group_sizes ? seg_row0[s + 1] : p.M;
         if (p.group_sizes && rows + r > p.M) r = p.M - rows;
         rows += r;
-        tiles += static_cast<int>((r + BT - 1) / BT) * ftiles;
+        tiles += static_cast<int>((r + p.tile_rows - 1) / p.tile_rows) * ftiles;
         seg_tile0[s + 1] = tiles;
         seg_row0[s + 1] = rows;
       }
@@ -916,8 +920,8 @@ add_partials_kernel(const float* __restrict__ partial, const TcParams p, int cta
   for (int64_t u = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; u < units; u += static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5)) {
     const int64_t row = u / (ftiles * ctas), rest = u - row * (ftiles * ctas), ft = rest / ctas;
     const int rank = static_cast<int>(rest - ft * ctas);
-    const int64_t seg = row / p.M, in_seg = row - seg * p.M, tt = in_seg / BT, tile = (seg * token_tiles + tt) * ftiles + ft;
-    const float* at = partial + ((tile * p.split * ctas + rank) * BT + (in_seg - tt * BT)) * kBF + lane * 4;
+    const int64_t seg = row / p.M, in_seg = row - seg * p.M, tt = in_seg / p.tile_rows, tile = (seg * token_tiles + tt) * ftiles + ft;
+    const float* at = partial + ((tile * p.split * ctas + rank) * BT + (in_seg - tt * p.tile_rows)) * kBF + lane * 4;
     float4 sum = __ldcg(reinterpret_cast<const float4*>(at));
 #pragma unroll 4
     for (int v = 1; v < p.split; ++v) {
@@ -1043,7 +1047,8 @@ int launch_tables(const qmm_problem& p, cudaStream_t stream) {
   const int sms = device_sm_count();
   const int num_kb = static_cast<int>((p.K + kBK - 1) / kBK), boxes = (num_kb + P::kPer - 1) / P::kPer;
   const int64_t ftiles = (p.N + kBF * P::kCtas - 1) / (kBF * P::kCtas), ttiles = (p.M + BT - 1) / BT;
-  const int64_t tiles = ragged ? (ttiles + p.batch) * ftiles : p.batch * ttiles * ftiles;      // (ragged: at most)
+  int64_t tiles = ragged ? (ttiles + p.batch) * ftiles : p.batch * ttiles * ftiles;      // (ragged: at most)
+  tp.tile_rows = BT;
   int64_t workers = sms / P::kCtas;
   int64_t shared = 0, split = 1;
   if (ragged) {
@@ -1069,6 +1074,18 @@ int launch_tables(const qmm_problem& p, cudaStream_t stream) {
     const int64_t rest = tiles % workers, rounds = tiles / workers;
     const int64_t region = rounds ? workers + rest : tiles;
     if (rest && (rounds ? 2 : 1) * boxes - region * boxes / workers > kExchangeBlocks / P::kPer) shared = region;
+    // Less than a round that is not shared out leaves workers idle: shorter tiles take less time each, as long as there are no more of them than workers (and
+    // down to 160 tokens, below which the dequantization is what a K block costs). 512 rows mxfp4 5760 x 2880: 46 tiles of 256 tokens on 74 pairs, 69 of 192.
+    if (!shared && !rounds && P::kPair)
+      for (int h = 160; h < BT; h += 32) {
+        const int64_t shorter = p.batch * ((p.M + h - 1) / h) * ftiles;
+        if (shorter > workers) continue;
+        if (shorter > tiles) {
+          tp.tile_rows = h;
+          tiles = shorter;
+        }
+        break;
+      }
     if (!shared && tiles < workers) workers = tiles;
   }
   // Partial tiles: the caller's static block (qmm_quantized_matmul_static) or a stream-ordered allocation. No scratch,
