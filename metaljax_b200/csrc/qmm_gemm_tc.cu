@@ -1074,16 +1074,15 @@ int launch_tables(const qmm_problem& p, cudaStream_t stream) {
     const int64_t rest = tiles % workers, rounds = tiles / workers;
     const int64_t region = rounds ? workers + rest : tiles;
     if (rest && (rounds ? 2 : 1) * boxes - region * boxes / workers > kExchangeBlocks / P::kPer) shared = region;
-    // Less than a round that is not shared out leaves workers idle: shorter tiles take less time each, as long as there are no more of them than workers (and
-    // down to 160 tokens, below which the dequantization is what a K block costs). 512 rows mxfp4 5760 x 2880: 46 tiles of 256 tokens on 74 pairs, 69 of 192.
+    // Less than a round that is not shared out is as long as its longest tile: the shortest tiles that are one round still take its place (down to
+    // 160 tokens, below which the dequantization is what a K block costs). 512 rows mxfp4 5760 x 2880: 46 tiles of 256 tokens on 74 pairs, 69 of 192, 20.5 -> 18.8 us;
+    // 300 rows 6144 x 4096: 48, 48 of 160 and 140 instead of 256 and 44, 23.0 -> 19.5; 280 rows mxfp4 5760 x 2880 17.5 -> 16.0; 384 rows 8192 x 2048 8-bit 16.2 -> 15.7.
     if (!shared && !rounds && P::kPair)
       for (int h = 160; h < BT; h += 32) {
         const int64_t shorter = p.batch * ((p.M + h - 1) / h) * ftiles;
         if (shorter > workers) continue;
-        if (shorter > tiles) {
-          tp.tile_rows = h;
-          tiles = shorter;
-        }
+        tp.tile_rows = h;
+        tiles = shorter;
         break;
       }
     if (!shared && tiles < workers) workers = tiles;
