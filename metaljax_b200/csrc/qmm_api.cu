@@ -216,7 +216,7 @@ int launch_problem(const qmm_problem& p, cudaStream_t stream) {
     case QMM_ROUTE_GEMV: return p.group_sizes ? launch_rows(p, stream) : launch_gemv(p, stream);
     case QMM_ROUTE_GEMM_TC: return launch_gemm_tc(p, stream);
     // Float32 activations and what the others decline (unsorted gathers of more than 16 rows, K below 64): the
-    // few-rows kernel takes them as columns of its MMAs; the plain SIMT kernel is what a forced route cross-checks with.
+    // few-rows kernel takes them as columns of its MMAs, or, float32 activations of more than 8 rows, the tensor-core kernel of their own; the plain SIMT kernel is what a forced route cross-checks with.
     // Its codes go in without a magic number here, since the SIMT kernel's float32 sums are what such calls had: with it a float32 result
     // of activations of one sign was 60 (4-bit) to 140 times (8-bit) further from the exact one than the SIMT kernel's.
     default:

@@ -1,7 +1,7 @@
 // The few-rows kernel of the fused dequantize-and-matmul (`y = x . deq(w)^T`,
 // src/metaljax/qmm.py:2491): 2..16 rows of 16-bit activations against a streamed weight (and one row
 // where the single-row integer kernel declines), unsorted expert gathers, grouped products of a few rows
-// per expert, and every product of float32 activations.
+// per expert, and products of float32 activations: up to 8 rows, and what qmm_f32_tc.cu does not take.
 //
 // What bounds it. An SM's share of HBM is 23 bytes a clock, 46 4-bit codes: at four instructions a
 // clock that leaves 22 warp instructions per 256 codes, two thirds of what a dequantization element by

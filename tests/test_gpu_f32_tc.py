@@ -41,8 +41,8 @@ def _far(y, exact):
     (49, 4096, 2500, "int4", 128, "f16"),       # two chunks, more tiles than clusters
     (64, 2112, 385, "int8", 64, "f32"),         # 17 steps over eight CTAs
     (100, 1088, 257, "int8", 32, "bf16"),
-    (12, 14720, 256, "int4", 128, "f32"),       # the longest stretch of K that 16 rows leave room for
-    (20, 14976, 130, "mxfp4", 32, None),        # ... and one that does not fit: the few-rows kernel
+    (12, 14336, 256, "int4", 128, "f32"),       # the longest stretch of K that 16 rows leave room for
+    (20, 14368, 130, "mxfp4", 32, None),        # ... and 32 codes more, which do not fit: the few-rows kernel
     (48, 2880, 700, "mxfp4", 32, None),         # 90 table bytes a row
     (31, 320, 200, "int8", 64, "f16"),
     (200, 576, 19300, "int4", 64, "f32"),       # many tiles, no cluster
