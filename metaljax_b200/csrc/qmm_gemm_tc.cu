@@ -954,9 +954,9 @@ unsigned long long next_epoch() {
 constexpr int kLeastBoxes = 2;
 // (More of them of wide tiles write and read more partial sums than they save.)
 constexpr int most_shares(int bt) { return bt >= 256 ? 8 : 16; }
-// What handing partial tiles from worker to worker takes, in K blocks (us, shared out / a tile each: 64 rows 14336 x 4096, 112 tiles of 64
-// blocks on 148 workers, 23.4 / 20.3; 64 rows 28672 x 4096 37.5 / 35.6; 512 rows mxfp4 5760 x 2880, 46 of 45 on 74 pairs, 30 / 24; 512 rows 28672 x 4096,
-// which it shortens by a third of a round more than that, 99.7 / 105.8).
+// What handing partial tiles from worker to worker takes, in K blocks (us, shared out / a tile each: 64 rows 28672 x 4096, 224 tiles of 64
+// blocks on 148 workers, 29.9 / 27.0; 14336 x 4096, 112 tiles, 20.3 / 15.3; 11008 x 4096 18.4 / 14.7; 128 rows 28672 x 4096 35.7 / 33.0; 300 rows 14336 x 4096, 112 tiles on
+// 74 pairs, 51 / 43; mxfp4 64 rows 28800 x 2880 27..29 / 25.6).
 constexpr int kExchangeBlocks = 32;
 
 // Clusters of `ctas` that fit the device at once.
