@@ -2,10 +2,13 @@
 // in the precision that keras keeps by default).
 //
 // Arithmetic, that of the few-rows kernel (qmm_rows.cuh) in another place: the codes are never dequantized. A code minus its centre (q - 8,
-// q - 128, an E2M1 value) is an exact bf16, the MMA's A operand in tensor memory; a float32 activation is three bf16 pieces (8 + 8 + 8 bits),
-// the B operand. Every 64 codes (32 in groups of 32) have accumulators of their own, two columns of tensor memory per row, one for the first piece and one for the
+// q - 128, an E2M1 value) is exact in 16 bits, the MMA's A operand in tensor memory; a float32 activation is three pieces, the B operand: against 4-bit codes
+// bf16 ones (8 + 8 + 8 bits), against 8-bit and MXFP4 ones f16 (11 + 11 + 11), for which each 512 codes of a row are brought to [2^14, 2^15) by
+// their largest finite magnitude, and their sums back. Every 64 codes (32 in groups of 32) have accumulators of their own, two columns of tensor memory per row, one for the first piece and one for the
 // others: a tensor core truncates each sum that it makes, and the small pieces' sums are small. They are read back, scaled and added up in
 // float32 registers: y += s * sum (q - C) x, and once a tile, where that is not nought for every row of a warp, sum (b + C s) sum x.
+// Range: activations up to 2^120 give finite results where those fit (against 8-bit codes as bf16 pieces, unscaled, a group's sum was infinite from 2^118 on, and below
+// 2^-110 the pieces ran out of exponents: 4.5e-3 of the result's norm at 2^-126). 4-bit codes take those below 2^-110 with fewer than 24 bits.
 //
 // Split. K is shared out to the CTAs of a cluster (up to 8). A CTA converts its stretch of K of a chunk of 16, 32 or 48 activation rows once, into
 // swizzled tiles that stay in shared memory; tiles of 128 weight rows pass by. The CTAs' partial tiles are pushed with st.async to the CTA that owns 128 / c of the
@@ -73,18 +76,20 @@ struct F32Params {
 };
 
 // Shared memory from the 1024-byte aligned start: barriers, the activations [block][piece][T rows x 128 bytes], the weights' ring, the activations' sums over 32 codes
-// [4 steps][T], the partial tiles [slot][128 rows][T + 4].
+// [4 steps][T], what the slices' sums are multiplied by [slice][T], the partial tiles [slot][128 rows][T + 4].
 constexpr int kWFull = 0, kWEmpty = kWFull + 8 * kMaxBoxes, kAFull = kWEmpty + 8 * kMaxBoxes, kAEmpty = kAFull + 8 * kASlots, kDFull = kAEmpty + 8 * kASlots,
               kDEmpty = kDFull + 8 * kMaxDSlots, kXFull = kDEmpty + 8 * kMaxDSlots, kXFree = kXFull + 16, kTmemSlot = kXFree + 16, kAbort = kTmemSlot + 4, kHead = 1024;
 static_assert(kAbort + 4 <= kHead, "");
 constexpr int partial_row(int t) { return (t + 4) * 4; }
 constexpr int partial_bytes(int t) { return kTileRows * partial_row(t); }
 constexpr int x_block(int t) { return 3 * t * 128; }
+constexpr int kSliceSteps = 4;         // 512 codes of a row are scaled together (48 rows: all of a CTA's, which are no more)
+constexpr int most_slices(int t, int steps) { return t == 48 ? 1 : (steps + kSliceSteps - 2) / kSliceSteps + 1; }      // slices start at multiples of 512 codes
 constexpr size_t smem_of(int t, int steps, int slots, int boxes, int bits) {
-  return 1024 + kHead + boxes * box_bytes(bits) + static_cast<size_t>(steps) * (2 * x_block(t) + 4 * t * 4) + static_cast<size_t>(slots) * partial_bytes(t);
+  return 1024 + kHead + boxes * box_bytes(bits) + static_cast<size_t>(steps) * (2 * x_block(t) + 4 * t * 4) + most_slices(t, steps) * t * 4 + static_cast<size_t>(slots) * partial_bytes(t);
 }
 
-// NW packed words -> pairs of bf16 codes minus their centre (exact).
+// Packed words -> pairs of codes minus their centre (exact): bf16 (4-bit) or f16.
 template <int QK>
 __device__ __forceinline__ void codes16(const uint32_t (&w)[4], uint32_t* out) {
   if constexpr (QK == kAff4) {         // 32 codes, as (q - 8) / 64: a code in the low bits is the subnormal q 2^-133, one FMA with 2^127 and -1 / 8 takes it there (exactly)
@@ -95,24 +100,22 @@ __device__ __forceinline__ void codes16(const uint32_t (&w)[4], uint32_t* out) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) out[j * 4 + i] = H::fma(permute(even, odd, i | ((8 + i) << 4) | ((4 + i) << 8) | ((12 + i) << 12)), 0x7F007F00u, 0xBE00BE00u);
     }
-  } else if constexpr (QK == kAff8) {  // 16 codes, through float32: 2^23 + q - (2^23 + 128)
+  } else if constexpr (QK == kAff8) {  // 16 codes: 1024 + q - 1152
+    using H = Half2Ops<__half>;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float q[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) q[e] = __uint_as_float(__byte_perm(w[j], 0x4B000000u, 0x7540u + e)) - 8388736.0f;
-      out[j * 2] = Half2Ops<__nv_bfloat16>::pack(q[0], q[1]);
-      out[j * 2 + 1] = Half2Ops<__nv_bfloat16>::pack(q[2], q[3]);
+      out[j * 2] = H::sub(__byte_perm(w[j], 0x64646464u, 0x4140u), 0x64806480u);
+      out[j * 2 + 1] = H::sub(__byte_perm(w[j], 0x64646464u, 0x4342u), 0x64806480u);
     }
-  } else {                             // 32 E2M1 codes: magnitude at the exponent's boundary is the value times 2^-126
-    using H = Half2Ops<__nv_bfloat16>;
+  } else {                             // 32 E2M1 codes: magnitude at the exponent's boundary is the value times 2^-14
+    using H = Half2Ops<__half>;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t hi = w[j] >> 4;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const uint32_t t = __byte_perm(w[j], hi, i | ((4 + i) << 8)) & 0x000F000Fu;
-        out[j * 4 + i] = H::mul(((t & 0x00070007u) << 6) | ((t & 0x00080008u) << 12), 0x7E807E80u);      // 2^126
+        out[j * 4 + i] = H::mul(((t & 0x00070007u) << 9) | ((t & 0x00080008u) << 12), 0x74007400u);      // 2^14
       }
     }
   }
@@ -139,11 +142,13 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
   constexpr int kRowBytes = kBK * kBits / 8, kBoxBytes = 2 * kRowBytes, kBox = box_bytes(kBits);      // of a weight row in a block, in a box
   constexpr float kCentre = QK == kAff8 ? 128.0f : 8.0f, kUnit = QK == kAff4 ? 64.0f : 1.0f;     // (4-bit codes go in divided by 64)
   constexpr int kXBlock = x_block(T), kPiece = T * 128, kRow = partial_row(T), kDSlots = d_slots(T);
+  constexpr bool kScaled = QK != kAff4;                // f16 pieces of scaled slices
   static_assert(kDAt + kDSlots * 2 * T <= 512 && T % 16 == 0, "");
 
   extern __shared__ uint8_t f32_smem_raw[];
   const uint32_t smem = (smem_u32(f32_smem_raw) + 1023) & ~1023u;
-  const uint32_t x_at = smem + kHead, w_at = x_at + p.most_steps * 2 * kXBlock, sums_at = w_at + p.boxes * kBox, part_at = sums_at + p.most_steps * 4 * T * 4;
+  const uint32_t x_at = smem + kHead, w_at = x_at + p.most_steps * 2 * kXBlock, sums_at = w_at + p.boxes * kBox, back_at = sums_at + p.most_steps * 4 * T * 4,
+                 part_at = back_at + most_slices(T, p.most_steps) * T * 4;
   const uint32_t abort_at = smem + kAbort;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // (what the issuer's operands come from is the same in all lanes, and is made known as such: see tc_mma_block)
@@ -268,7 +273,77 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
 
     if (done == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     // ---- this CTA's stretch of K of the chunk's rows, as three pieces ----
-    {
+    if constexpr (kScaled) {                             // a warp has a row's slice, sixteen elements a lane
+      const int eights = nsteps * 16, slice0 = T == 48 ? 0 : step0 / kSliceSteps, slices = T == 48 ? 1 : (step0 + nsteps - 1) / kSliceSteps - slice0 + 1;
+      constexpr int kAtOnce = 2;
+      for (int u0 = warp; u0 < T * slices; u0 += kWarps * kAtOnce) {
+        float f[kAtOnce][2][8];
+        auto place = [&](int u, int h) -> int { return (T == 48 ? 0 : (slice0 + u / T) * (kSliceSteps * 16) - step0 * 16) + h * 32 + lane; };      // which eight elements
+#pragma unroll
+        for (int j = 0; j < kAtOnce; ++j) {
+          const int u = u0 + j * kWarps;
+          const int64_t m = row0 + u % T;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c = place(u, h), k = step0 * kStepK + c * 8;
+            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+            if (u < T * slices && m < p.M && c >= 0 && c < eights && k < p.K) {
+              const float4* src = reinterpret_cast<const float4*>(p.x + m * p.K + k);
+              a = __ldg(src);
+              b = __ldg(src + 1);
+            }
+            f[j][h][0] = a.x; f[j][h][1] = a.y; f[j][h][2] = a.z; f[j][h][3] = a.w;
+            f[j][h][4] = b.x; f[j][h][5] = b.y; f[j][h][6] = b.z; f[j][h][7] = b.w;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < kAtOnce; ++j) {
+          const int u = u0 + j * kWarps, t = u % T;
+          if (u >= T * slices) continue;
+          uint32_t most = 0;
+          bool odd = false;                              // an infinity or a NaN among them
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const uint32_t bits = __float_as_uint(f[j][i >> 3][i & 7]) & 0x7FFFFFFFu;
+            odd |= bits >= 0x7F800000u;
+            most = max(most, bits >= 0x7F800000u ? 0u : bits);
+          }
+          const uint32_t e = max(__reduce_max_sync(0xffffffffu, most) >> 23, 15u);
+          const float up = __uint_as_float((268u - e) << 23);
+          if (lane == 0) sts32(back_at + (u / T * T + t) * 4, __uint_as_float((e - 14u) << 23));
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c = place(u, h);
+            const bool here = c >= 0 && c < eights;
+            auto& g = f[j][h];
+            if constexpr (QK != kMx4) {
+              float sum = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7]));
+              sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+              sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+              if ((lane & 3) == 0 && here) sts32(sums_at + ((c >> 2) * T + t) * 4, sum);
+            }
+            const uint32_t to = x_at + (c >> 3) * kXBlock + t * 128 + (((c ^ t) & 7) << 4);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) g[i] *= up;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              uint32_t v[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                v[q] = Half2Ops<__half>::pack(g[2 * q], g[2 * q + 1]);
+                if (i < 2) {                             // what the piece leaves over (exact); an infinity leaves nothing, a NaN stays one
+                  const float2 got = __half22float2(*reinterpret_cast<const __half2*>(&v[q]));
+                  const bool whole0 = odd && i == 0 && fabsf(g[2 * q]) > 3.402823466e38f, whole1 = odd && i == 0 && fabsf(g[2 * q + 1]) > 3.402823466e38f;
+                  g[2 * q] = whole0 ? 0.0f : g[2 * q] - got.x;
+                  g[2 * q + 1] = whole1 ? 0.0f : g[2 * q + 1] - got.y;
+                }
+              }
+              if (here) sts128(to + i * kPiece, __uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
+            }
+          }
+        }
+      }
+    } else {
       const int pieces = nsteps * 16, units = T * pieces;
       const unsigned inverse = nsteps == p.most_steps ? p.most_inverse : p.less_inverse;
       auto row_of = [&](int u) -> int { return static_cast<int>(__umulhi(static_cast<unsigned>(u), inverse)); };
@@ -293,11 +368,9 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
           float f[8] = {a[j].x, a[j].y, a[j].z, a[j].w, b[j].x, b[j].y, b[j].z, b[j].w};
           float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
           const bool odd = !(fabsf(sum) <= 3.402823466e38f);       // an infinity or a NaN among them, perhaps
-          if constexpr (QK != kMx4) {
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            if ((lane & 3) == 0) sts32(sums_at + ((c >> 2) * T + t) * 4, sum);
-          }
+          sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+          if ((lane & 3) == 0) sts32(sums_at + ((c >> 2) * T + t) * 4, sum);
           // A piece is the eight bits of a mantissa that come next, cut off: what it leaves over is exact. An infinity leaves nothing (not a NaN), and a
           // NaN stays one.
           const uint32_t to = x_at + (c >> 3) * kXBlock + t * 128 + (((c ^ t) & 7) << 4);
@@ -341,7 +414,8 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
     } else if (warp == 1) {
       // ---------------- MMA issuer ----------------
       // first piece and second side by side, 2 T columns; the third on top of the second
-      constexpr uint32_t idesc1 = instr_desc(1, kTileRows) | (static_cast<uint32_t>(T >> 3) << 17), idesc2 = instr_desc(1, kTileRows) | (static_cast<uint32_t>(T >> 2) << 17);
+      constexpr int kFormat = kScaled ? 0 : 1;
+      constexpr uint32_t idesc1 = instr_desc(kFormat, kTileRows) | (static_cast<uint32_t>(T >> 3) << 17), idesc2 = instr_desc(kFormat, kTileRows) | (static_cast<uint32_t>(T >> 2) << 17);
       // (variables of this branch alone, known to be the same in all lanes, and one loop that is left where all lanes have seen a wait run out)
       uint32_t as = same(slot), aph = same(phase), ds = same(dslot), dph = same(dphase);
       const int total = same(tiles * nsteps);
@@ -468,26 +542,16 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
         float y[kOwn];
 #pragma unroll
         for (int t = 0; t < kOwn; ++t) y[t] = 0.0f;
-        // (sums of 512 codes at a time, as in the few-rows kernel: a rounding is relative to the sum so far. 48 rows have no more.)
+        // (the sums of four groups at a time, in their slice's units: a rounding is relative to the sum so far. 48 rows' are of 512 codes at most.)
         constexpr bool kTwoLevels = T < 48;
-        const int kLong = halves ? 16 : 8;
         float total[kTwoLevels ? kOwn : 1];
 #pragma unroll
         for (int t = 0; t < (kTwoLevels ? kOwn : 1); ++t) total[t] = 0.0f;
         bool biased = false;
         int unit = step0 * (halves ? 4 : 2);             // the accumulator that comes next, in 32 or 64 codes
         const int units_end = (step0 + nsteps) * (halves ? 4 : 2), per_group = p.group_shift == 7 ? 1 : 0;
-        int sum_end = unit + kLong;                      // where the sums of this stretch join those before
 #pragma unroll 1
         for (int g0 = g_batch; ok && unit < units_end; g0 += 4) {
-          if (kTwoLevels && unit >= sum_end) {
-#pragma unroll
-            for (int t = 0; t < (kTwoLevels ? kOwn : 0); ++t) {
-              total[t] += y[t];
-              y[t] = 0.0f;
-            }
-            sum_end += kLong;
-          }
           if (g0 + 4 < g_end) {                          // (the next four are on their way while these are used)
             sc_next = entries(p.scales, trow, g0 + 4);
             if constexpr (QK != kMx4) bi_next = entries(p.biases, trow, g0 + 4);
@@ -523,11 +587,28 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
           }
           sc = sc_next;
           bi = bi_next;
+          if constexpr (kTwoLevels) {
+            const uint32_t back = back_at + (((g0 << p.group_shift) / (kSliceSteps * kStepK) - step0 / kSliceSteps) * T + t_own) * 4;
+#pragma unroll
+            for (int t = 0; t < kOwn; t += 4) {
+              float4 f = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+              if constexpr (kScaled) f = ldsf128<0>(back + t * 4);
+              total[t] = fmaf(y[t], f.x, total[t]); total[t + 1] = fmaf(y[t + 1], f.y, total[t + 1]);
+              total[t + 2] = fmaf(y[t + 2], f.z, total[t + 2]); total[t + 3] = fmaf(y[t + 3], f.w, total[t + 3]);
+              y[t] = y[t + 1] = y[t + 2] = y[t + 3] = 0.0f;
+            }
+          }
         }
         if (!ok) break;
-        if (kTwoLevels) {
+        if constexpr (kTwoLevels) {
 #pragma unroll
-          for (int t = 0; t < (kTwoLevels ? kOwn : 0); ++t) y[t] += total[t];
+          for (int t = 0; t < kOwn; ++t) y[t] = total[t];
+        } else if constexpr (kScaled) {
+#pragma unroll
+          for (int t = 0; t < kOwn; t += 4) {
+            const float4 f = ldsf128<0>(back_at + (t_own + t) * 4);
+            y[t] *= f.x; y[t + 1] *= f.y; y[t + 2] *= f.z; y[t + 3] *= f.w;
+          }
         }
         if constexpr (kUnit != 1.0f) {
 #pragma unroll
@@ -628,7 +709,7 @@ F32Plan plan_of(const qmm_problem& p) {
     if (c > steps_all) continue;
     const int steps = static_cast<int>((steps_all + c - 1) / c);
     for (int t = 48; t >= 16; t -= 16) {
-      // (48 rows' sums are of 512 codes: see kTwoLevels)
+      // (48 rows' sums and slices are of 512 codes at most: see kTwoLevels)
       if ((t == 48 && steps > 4) || smem_of(t, steps, 1, kASlots, bits) > kSmemLimit) continue;
       const int64_t chunks = (p.M + t - 1) / t, items = chunks * tiles, clusters = sms / c < items ? sms / c : items, rounds = (items + clusters - 1) / clusters;
       const double passes = static_cast<double>(chunks < rounds ? chunks : rounds);

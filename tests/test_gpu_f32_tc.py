@@ -70,6 +70,23 @@ def test_float32_rows_to_16_bits(out):
     assert torch.equal(y, qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw).to(out))
 
 
+@pytest.mark.parametrize("m", [12, 40])            # with slices of 512 codes, and with one for all of a stretch
+@pytest.mark.parametrize("kind,k,power", [("int8", 1088, 120), ("int8", 1088, 118), ("int8", 1088, -118), ("int8", 640, -128),
+                                          ("mxfp4", 1120, 118), ("mxfp4", 1120, -116), ("mxfp4", 640, -128), ("int4", 1088, 120), ("int4", 1088, -108)])
+def test_float32_rows_at_the_ends_of_their_range(m, kind, k, power):
+    """Activations of up to some 2^122 whose results fit, and such that have no 24 bits above bf16's smallest number, keep the precision of the middle
+    of the range; slices that lie 2^60 apart do not share a scale."""
+    xs, args, kw, _ = _case(m, k, 200, kind, 32 if kind == "mxfp4" else 64, "f32")
+    xs = np.ldexp(xs, power)
+    if power < 0 and kind != "int4":
+        xs[1, 512:] = np.ldexp(xs[1, 512:], 60)
+    exact = O.qmm_exact(xs, to_numpy(args[0]), to_numpy(args[1]), None if args[2] is None else to_numpy(args[2]), kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
+    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw)).astype(np.float64)
+    assert np.isfinite(y).all()
+    far = np.linalg.norm(y - exact, axis=1) / np.linalg.norm(exact, axis=1)      # of each row: they are as far apart as their slices
+    assert far.max() <= 4e-7
+
+
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
 def test_float32_rows_that_are_not_finite(value):
     """An infinity times a positive, a negative or a zero weight, as a sum of products has it; the rows beside it as ever."""
