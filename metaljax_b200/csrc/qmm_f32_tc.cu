@@ -371,14 +371,15 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
           sum += __shfl_xor_sync(0xffffffffu, sum, 1);
           sum += __shfl_xor_sync(0xffffffffu, sum, 2);
           if ((lane & 3) == 0) sts32(sums_at + ((c >> 2) * T + t) * 4, sum);
-          // A piece is the eight bits of a mantissa that come next, cut off: what it leaves over is exact. An infinity leaves nothing (not a NaN), and a
-          // NaN stays one.
+          // A piece is the eight bits of a mantissa that come next, cut off: what it leaves over is exact (the last eight are; below 2^-110, where it is more than
+          // bf16's exponents reach, it is rounded). An infinity leaves nothing (not a NaN), and a NaN stays one.
           const uint32_t to = x_at + (c >> 3) * kXBlock + t * 128 + (((c ^ t) & 7) << 4);
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             uint32_t h[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) h[e] = __byte_perm(__float_as_uint(f[2 * e]), __float_as_uint(f[2 * e + 1]), 0x7632);
+            for (int e = 0; e < 4; ++e)
+              h[e] = i < 2 ? __byte_perm(__float_as_uint(f[2 * e]), __float_as_uint(f[2 * e + 1]), 0x7632) : Half2Ops<__nv_bfloat16>::pack(f[2 * e], f[2 * e + 1]);
             sts128(to + i * kPiece, __uint_as_float(h[0]), __uint_as_float(h[1]), __uint_as_float(h[2]), __uint_as_float(h[3]));
             if (i < 2) {
 #pragma unroll

@@ -87,6 +87,16 @@ def test_float32_rows_at_the_ends_of_their_range(m, kind, k, power):
     assert far.max() <= 4e-7
 
 
+def test_float32_rows_below_the_range_of_4_bit_codes():
+    """Below 2^-110 an activation is rounded to a multiple of 2^-133, the smallest bf16: an error of 2^-133 / sqrt(12) each, and a quarter more."""
+    xs, args, kw, _ = _case(40, 1024, 200, "int4", 64, "f32")
+    xs = np.ldexp(xs, -122)
+    w, s, b = (to_numpy(a) for a in args)
+    dense = O.qmm_exact(np.eye(1024, dtype=np.float32), w, s, b, 64, 4)
+    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw)).astype(np.float64)
+    assert np.linalg.norm(y - O.qmm_exact(xs, w, s, b, 64, 4)) <= 1.25 * 2.0 ** -133 / np.sqrt(12) * np.sqrt(len(xs)) * np.linalg.norm(dense)
+
+
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
 def test_float32_rows_that_are_not_finite(value):
     """An infinity times a positive, a negative or a zero weight, as a sum of products has it; the rows beside it as ever."""
