@@ -4,7 +4,7 @@
 // Arithmetic, that of the few-rows kernel (qmm_rows.cuh) in another place: the codes are never dequantized. A code minus its centre (q - 8,
 // q - 128, an E2M1 value) is exact in 16 bits, the MMA's A operand in tensor memory; a float32 activation is three pieces, the B operand: against 4-bit codes
 // bf16 ones (8 + 8 + 8 bits), against 8-bit and MXFP4 ones f16 (11 + 11 + 11), for which each 512 codes of a row are brought to [2^14, 2^15) by
-// their largest finite magnitude, and their sums back. Every 64 codes (32 in groups of 32) have accumulators of their own, two columns of tensor memory per row, one for the first piece and one for the
+// their largest finite magnitude, and their sums back. Every group (of 8-bit codes, every 64) has accumulators of its own, two columns of tensor memory per row, one for the first piece and one for the
 // others: a tensor core truncates each sum that it makes, and the small pieces' sums are small. They are read back, scaled and added up in
 // float32 registers: y += s * sum (q - C) x, and once a tile, where that is not nought for every row of a warp, sum (b + C s) sum x.
 // Range: activations up to 2^120 give finite results where those fit (against 8-bit codes as bf16 pieces, unscaled, a group's sum was infinite from 2^118 on, and below
@@ -17,9 +17,10 @@
 // What bounds it: the few-rows kernel takes four rows a pass over the weight, and takes the codes apart for each of them (33 rows: nine times). Here a pass
 // takes up to 48. 33 rows of 4096 x 4096: 34.6 -> 24.0 us (13 K clocks a tile and cluster of eight: 8 K of them the codes, the MMAs' issue and the adding up, which
 // are latency at 18 warps, the rest the exchange; 14 such clusters fit the machine); 64 rows of 14336 x 4096 178 -> 83, 4096 x 14336 234 -> 114.
-// Relative error against float64 (2-norm; N(0, 1) / one sign / outliers of 300), few-rows kernel -> here: 4-bit 33 rows K 4096 8.6e-8 / 5.2e-8 / 9.4e-8 ->
-// 8.2e-8 / 5.1e-8 / 9.1e-8, K 14336 9.3e-8 / 4.4e-8 / 1.0e-7 -> 9.2e-8 / 4.9e-8 / 1.0e-7, 8-bit K 4096 1.3e-7 / 7.4e-8 / 2.1e-7 -> 8.5e-8 / 7.9e-8 / 1.3e-7, MXFP4 K 2880
-// 8.8e-8 / 7.6e-8 / 1.1e-7 -> 8.9e-8 / 8.7e-8 / 9.2e-8. (All pieces in one accumulator: 9.4e-8 / 6.4e-8 / 9.7e-8, and 2.4e-7 in groups of 128.)
+// Relative error against float64 (1e-8, 2-norm; N(0, 1) / one sign / outliers of 300; 33 rows), few-rows kernel -> here: 4-bit groups of 64 K 4096 8.5 / 5.4 / 9.5 -> 7.3 /
+// 4.2 / 8.3, K 14336 9.4 / 4.6 / 10.1 -> 8.6 / 4.3 / 9.4, of 128 K 4096 7.8 / 5.2 / 10.2 -> 6.8 / 4.2 / 9.4; 8-bit of 128 K 12288 13.4 / 12.5 / 20.4 -> 10.2 / 9.4 / 13.4; MXFP4
+// K 4096 9.3 / 9.3 / 11.1 -> 7.8 / 7.8 / 9.3, K 14336 10.1 / 10.1 / 11.5 -> 9.8 / 9.9 / 10.9. (Ranks added up one after another and two sums to a group of 128: K 14336 9.1 / 5.0
+// / 9.8, of 128 9.1 / 5.0 / 9.9, MXFP4 K 4096 9.7 / 9.7 / 10.0. All pieces in one accumulator: 9.4 / 6.4 / 9.7 at K 4096, and 24 in groups of 128.)
 //
 // Warps: 0 = weights' producer, 1 = MMA issuer (+ tensor memory), 2..9 = two teams that turn codes into A, 10..17 = adding up, half of the rows
 // to each four. All of them convert the activations. A step is two K blocks: a wait costs a warp about as much as a third of a block's codes, and
@@ -155,7 +156,8 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
   auto same = [](int v) -> int { return __shfl_sync(0xffffffffu, v, 0); };
   const int csize = p.cluster, rank = same(csize > 1 ? static_cast<int>(cluster_rank()) : 0);
   const int step0 = same(p.steps * rank / csize), nsteps = same(p.steps * (rank + 1) / csize - step0);
-  const bool halves = p.group_shift == 5;                // two accumulators a block
+  // Accumulators of a step: one a group, or of 8-bit codes one every 64 (11 + 8 + 7 bits are more than a float32 sum holds: 1.25e-7 of the result's norm, 1.0e-7 so).
+  const int group_units = QK == kAff8 && p.group_shift == 7 ? 2 : 1, step_units = (kStepK >> p.group_shift) * group_units;
   const unsigned cluster = blockIdx.x / csize;
   const unsigned first = cluster * p.share + min(cluster, p.share_more);
   const int items = same(p.share + (cluster < p.share_more ? 1u : 0u));
@@ -236,13 +238,19 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
       if (i >= own * (T / 4)) break;
       const int r = i & (own - 1), t4 = i >> own_shift;
       const uint32_t at = from + r * kRow + t4 * 16;
-      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      float v[4];
+      // Neighbours first, then their sums: a rounding is relative to the sum so far, and one after another the last ones were all of a whole result (K 14336, one
+      // sign: 5.0e-8, the few-rows kernel 4.6e-8).
       auto sum = [&](auto count) {
+        constexpr int kCount = decltype(count)::value;
+        float4 f[kCount];
 #pragma unroll
-        for (int c = 0; c < decltype(count)::value; ++c) {
-          const float4 f = ldsf128<0>(at + (c << own_shift) * kRow);
-          v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
-        }
+        for (int c = 0; c < kCount; ++c) f[c] = ldsf128<0>(at + (c << own_shift) * kRow);
+#pragma unroll
+        for (int d = 1; d < kCount; d *= 2)
+#pragma unroll
+          for (int c = 0; c < kCount; c += 2 * d) f[c] = make_float4(f[c].x + f[c + d].x, f[c].y + f[c + d].y, f[c].z + f[c + d].z, f[c].w + f[c + d].w);
+        v[0] = f[0].x; v[1] = f[0].y; v[2] = f[0].z; v[3] = f[0].w;
       };
       if (csize == 8) sum(std::integral_constant<int, 8>());
       else if (csize == 4) sum(std::integral_constant<int, 4>());
@@ -425,19 +433,21 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
         if (!__all_sync(0xffffffffu, wait(kAFull + 8 * as, aph, 32))) break;
         bool there = true;
 #pragma unroll 1
-        for (int u = 0; u < (halves ? 4 : 2); ++u) {     // the step's accumulators
+        for (int u = 0; u < step_units; ++u) {
           there = wait(kDEmpty + 8 * ds, dph ^ 1u, 33);
           if (!__all_sync(0xffffffffu, there)) break;
           tc_fence_after();
           const uint32_t d = tmem + kDAt + ds * (2 * T);
-          if (!halves) {
-            const uint32_t acol = tmem + kASlotsAt + as * 64 + u * 32, desc = desc_low(x_at + (2 * b + u) * kXBlock);
-            tc_mma_block<false>(d, acol, desc, kDescHigh, idesc2, 0u);
-            tc_mma_block<false>(d + T, acol, desc + 2 * (kPiece / 16), kDescHigh, idesc1, 1u);
-          } else {
+          if (step_units == 4) {
             const uint32_t acol = tmem + kASlotsAt + as * 64 + u * 16, desc = desc_low(x_at + (2 * b + (u >> 1)) * kXBlock) + (u & 1) * 4;
             tc_mma_half(d, acol, desc, kDescHigh, idesc2, 0u);
             tc_mma_half(d + T, acol, desc + 2 * (kPiece / 16), kDescHigh, idesc1, 1u);
+          } else {
+            for (int h = 0; h < 3 - step_units; ++h) {   // K blocks of the accumulator
+              const uint32_t acol = tmem + kASlotsAt + as * 64 + (u + h) * 32, desc = desc_low(x_at + (2 * b + u + h) * kXBlock);
+              tc_mma_block<false>(d, acol, desc, kDescHigh, idesc2, h);
+              tc_mma_block<false>(d + T, acol, desc + 2 * (kPiece / 16), kDescHigh, idesc1, 1u);
+            }
           }
           tc_commit<false>(smem + kDFull + 8 * ds, 0);
           if (++ds == kDSlots) { ds = 0; dph ^= 1u; }
@@ -549,10 +559,9 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
 #pragma unroll
         for (int t = 0; t < (kTwoLevels ? kOwn : 1); ++t) total[t] = 0.0f;
         bool biased = false;
-        int unit = step0 * (halves ? 4 : 2);             // the accumulator that comes next, in 32 or 64 codes
-        const int units_end = (step0 + nsteps) * (halves ? 4 : 2), per_group = p.group_shift == 7 ? 1 : 0;
+        const int last = (step0 + nsteps) * kStepK >> p.group_shift;       // (past the last group, perhaps: the end of the last step)
 #pragma unroll 1
-        for (int g0 = g_batch; ok && unit < units_end; g0 += 4) {
+        for (int g0 = g_batch; ok && g0 < last; g0 += 4) {
           if (g0 + 4 < g_end) {                          // (the next four are on their way while these are used)
             sc_next = entries(p.scales, trow, g0 + 4);
             if constexpr (QK != kMx4) bi_next = entries(p.biases, trow, g0 + 4);
@@ -560,11 +569,11 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int g = g0 + e;
-            // (the second half of a last block that ends with its first lies past the last group: its sums are nought)
+            // (what lies past the last group has sums of nought)
             const float s = g < p.groups ? value(sc, e) : 0.0f;
             if constexpr (QK != kMx4) biased |= g < p.groups && g >= g_first && fmaf(kCentre, s, value(bi, e)) != 0.0f;
 #pragma unroll 1
-            while (unit < units_end && unit >> per_group == g) {
+            for (int u = g >= g_first && g < last ? group_units : 0; u > 0; --u) {
               ok = wait(kDFull + 8 * dslot, dphase, 37);
               if (!(ok = __all_sync(0xffffffffu, ok))) break;
               tc_fence_after();
@@ -582,7 +591,6 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
               __syncwarp();
               if (lane == 0) arrive_n(smem + kDEmpty + 8 * dslot, 1);
               if (++dslot == kDSlots) { dslot = 0; dphase ^= 1u; }
-              ++unit;
             }
             if (!ok) break;
           }

@@ -87,6 +87,20 @@ def test_float32_rows_at_the_ends_of_their_range(m, kind, k, power):
     assert far.max() <= 4e-7
 
 
+@pytest.mark.parametrize("kind,gs,k,one_sign", [("int4", 64, 14336, True), ("int4", 32, 8192, True), ("int4", 128, 4096, False), ("int8", 128, 4096, False),
+                                                ("int8", 64, 12288, True), ("mxfp4", 32, 4096, False), ("mxfp4", 32, 14336, True)])
+def test_float32_rows_are_as_exact_as_eight_at_a_time(kind, gs, k, one_sign):
+    """Against the few-rows kernel, which calls of eight rows take: no further from the exact product (the errors of 49152 results have a root
+    mean square that varies by 0.4 %: 2 % is five times that)."""
+    xs, args, kw, _ = _case(48, k, 1024, kind, gs, "f32" if kind != "mxfp4" else None, 3)
+    if one_sign:
+        xs = np.abs(xs)
+    exact = O.qmm_exact(xs, to_numpy(args[0]), to_numpy(args[1]), None if args[2] is None else to_numpy(args[2]), gs, kw["bits"], mode=kw.get("mode", "affine"))
+    x = to_torch(xs, DEV)
+    by_eight = torch.cat([qmm.quantized_matmul(x[i:i + 8], *args, **kw) for i in range(0, 48, 8)])
+    assert _far(qmm.quantized_matmul(x, *args, **kw), exact) <= 1.02 * _far(by_eight, exact)
+
+
 def test_float32_rows_below_the_range_of_4_bit_codes():
     """Below 2^-110 an activation is rounded to a multiple of 2^-133, the smallest bf16: an error of 2^-133 / sqrt(12) each, and a quarter more."""
     xs, args, kw, _ = _case(40, 1024, 200, "int4", 64, "f32")
