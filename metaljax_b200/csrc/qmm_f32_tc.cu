@@ -6,7 +6,7 @@
 // bf16 ones (8 + 8 + 8 bits), against 8-bit and MXFP4 ones f16 (11 + 11 + 11), for which each 512 codes of a row are brought to [2^14, 2^15) by
 // their largest finite magnitude, and their sums back. Every group (of 8-bit codes, every 64) has accumulators of its own, two columns of tensor memory per row, one for the first piece and one for the
 // others: a tensor core truncates each sum that it makes, and the small pieces' sums are small. They are read back, scaled and added up in
-// float32 registers: y += s * sum (q - C) x, and once a tile, where that is not nought for every row of a warp, sum (b + C s) sum x.
+// float32 registers: y += s * sum (q - C) x, and, for a row whose four groups have biases of their own (b + C s is not nought), (b + C s) sum x.
 // Range: activations up to 2^120 give finite results where those fit (against 8-bit codes as bf16 pieces, unscaled, a group's sum was infinite from 2^118 on, and below
 // 2^-110 the pieces ran out of exponents: 4.5e-3 of the result's norm at 2^-126). 4-bit codes take those below 2^-110 with fewer than 24 bits.
 //
@@ -76,7 +76,7 @@ struct F32Params {
   unsigned share, share_more;          // (chunk, tile) items of every cluster, and how many clusters have one more
 };
 
-// Shared memory from the 1024-byte aligned start: barriers, the activations [block][piece][T rows x 128 bytes], the weights' ring, the activations' sums over 32 codes
+// Shared memory from the 1024-byte aligned start: barriers, the activations [block][piece][T rows x 128 bytes], the weights' ring, the activations' sums over a group
 // [4 steps][T], what the slices' sums are multiplied by [slice][T], the partial tiles [slot][128 rows][T + 4].
 constexpr int kWFull = 0, kWEmpty = kWFull + 8 * kMaxBoxes, kAFull = kWEmpty + 8 * kMaxBoxes, kAEmpty = kAFull + 8 * kASlots, kDFull = kAEmpty + 8 * kASlots,
               kDEmpty = kDFull + 8 * kMaxDSlots, kXFull = kDEmpty + 8 * kMaxDSlots, kXFree = kXFull + 16, kTmemSlot = kXFree + 16, kAbort = kTmemSlot + 4, kHead = 1024;
@@ -232,7 +232,7 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
     __syncwarp();
     const uint32_t from = part_at + s * partial_bytes(T);
     constexpr int kAdders = 32 * kAddWarps, kMost = kTileRows * (T / 4) / kAdders;       // (all of a tile's rows are this CTA's where there is no cluster)
-#pragma unroll 2
+#pragma unroll 1                                         // (two at a time spill: 9 rows 4096 x 14336 in groups of 32 65.0 us, 57.2 so)
     for (int j = 0; j < kMost; ++j) {
       const int i = thread + j * kAdders;
       if (i >= own * (T / 4)) break;
@@ -281,6 +281,15 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
 
     if (done == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     // ---- this CTA's stretch of K of the chunk's rows, as three pieces ----
+    // (a lane has eight elements of a row, its neighbours those beside them)
+    [[maybe_unused]] auto group_sum = [&](float sum, int c, int t, bool here) {
+      const int eights = 1 << (p.group_shift - 3);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      if (eights > 4) sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+      if (eights > 8) sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+      if ((lane & (eights - 1)) == 0 && here) sts32(sums_at + ((c >> (p.group_shift - 3)) * T + t) * 4, sum);
+    };
     if constexpr (kScaled) {                             // a warp has a row's slice, sixteen elements a lane
       const int eights = nsteps * 16, slice0 = T == 48 ? 0 : step0 / kSliceSteps, slices = T == 48 ? 1 : (step0 + nsteps - 1) / kSliceSteps - slice0 + 1;
       constexpr int kAtOnce = 2;
@@ -324,15 +333,10 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
             const int c = place(u, h);
             const bool here = c >= 0 && c < eights;
             auto& g = f[j][h];
-            if constexpr (QK != kMx4) {
-              float sum = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7]));
-              sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-              sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-              if ((lane & 3) == 0 && here) sts32(sums_at + ((c >> 2) * T + t) * 4, sum);
-            }
             const uint32_t to = x_at + (c >> 3) * kXBlock + t * 128 + (((c ^ t) & 7) << 4);
 #pragma unroll
             for (int i = 0; i < 8; ++i) g[i] *= up;
+            if constexpr (QK != kMx4) group_sum(((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7])), c, t, here);
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
               uint32_t v[4];
@@ -376,9 +380,7 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
           float f[8] = {a[j].x, a[j].y, a[j].z, a[j].w, b[j].x, b[j].y, b[j].z, b[j].w};
           float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
           const bool odd = !(fabsf(sum) <= 3.402823466e38f);       // an infinity or a NaN among them, perhaps
-          sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-          if ((lane & 3) == 0) sts32(sums_at + ((c >> 2) * T + t) * 4, sum);
+          group_sum(sum, c, t, true);
           // A piece is the eight bits of a mantissa that come next, cut off: what it leaves over is exact (the last eight are; below 2^-110, where it is more than
           // bf16's exponents reach, it is rounded). An infinity leaves nothing (not a NaN), and a NaN stays one.
           const uint32_t to = x_at + (c >> 3) * kXBlock + t * 128 + (((c ^ t) & 7) << 4);
@@ -558,7 +560,6 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
         float total[kTwoLevels ? kOwn : 1];
 #pragma unroll
         for (int t = 0; t < (kTwoLevels ? kOwn : 1); ++t) total[t] = 0.0f;
-        bool biased = false;
         const int last = (step0 + nsteps) * kStepK >> p.group_shift;       // (past the last group, perhaps: the end of the last step)
 #pragma unroll 1
         for (int g0 = g_batch; ok && g0 < last; g0 += 4) {
@@ -566,12 +567,35 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
             sc_next = entries(p.scales, trow, g0 + 4);
             if constexpr (QK != kMx4) bi_next = entries(p.biases, trow, g0 + 4);
           }
+          // (b + C s) sum x, while the accumulators are made: 25.5 -> 28.3 us at 33 rows of 4096 x 4096 (83 with the entries read again for each group in a pass of its own)
+          if constexpr (QK != kMx4) {
+            float bc[4];
+            bool own = false;                            // a row has biases that are not the centre's
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              bc[e] = g0 + e >= g_first && g0 + e < g_end ? fmaf(kCentre, value(sc, e), value(bi, e)) * (1.0f / kUnit) : 0.0f;
+              own |= bc[e] != 0.0f;
+            }
+            if (own) {
+              const uint32_t at = sums_at + ((g0 - g_first) * T + t_own) * 4;
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                if (g0 + e < g_first || g0 + e >= g_end) continue;
+#pragma unroll
+                for (int t = 0; t < kOwn; t += 4) {
+                  const float4 f = ldsf128<0>(at + (e * T + t) * 4);
+                  fma2(y[t], y[t + 1], bc[e], f.x, f.y);
+                  fma2(y[t + 2], y[t + 3], bc[e], f.z, f.w);
+                }
+              }
+            }
+            __syncwarp();
+          }
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int g = g0 + e;
             // (what lies past the last group has sums of nought)
             const float s = g < p.groups ? value(sc, e) : 0.0f;
-            if constexpr (QK != kMx4) biased |= g < p.groups && g >= g_first && fmaf(kCentre, s, value(bi, e)) != 0.0f;
 #pragma unroll 1
             for (int u = g >= g_first && g < last ? group_units : 0; u > 0; --u) {
               ok = wait(kDFull + 8 * dslot, dphase, 37);
@@ -622,37 +646,6 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
         if constexpr (kUnit != 1.0f) {
 #pragma unroll
           for (int t = 0; t < kOwn; ++t) y[t] *= kUnit;
-        }
-        if constexpr (QK != kMx4) {
-          if (__any_sync(0xffffffffu, biased)) {         // (b + C s) sum x, in sums of its own
-#pragma unroll
-            for (int t0 = 0; t0 < kOwn; t0 += 8) {
-              float yb[8];
-#pragma unroll
-              for (int t = 0; t < 8; ++t) yb[t] = 0.0f;
-#pragma unroll 1
-              for (int g = g_first; g < g_end; ++g) {
-                const Entries s1 = entries(p.scales, trow, g & ~3), b1 = entries(p.biases, trow, g & ~3);
-                float bc = 0.0f;
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                  if ((g & 3) == e) bc = fmaf(kCentre, value(s1, e), value(b1, e));
-                const int lo = ((g << p.group_shift) - step0 * kStepK) >> 5, hi = lo + (1 << p.group_shift >> 5);
-#pragma unroll
-                for (int t = 0; t < 8; t += 4) {
-                  float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                  for (int u = lo; u < hi; ++u) {
-                    const float4 v = ldsf128<0>(sums_at + (u * T + t_own + t0 + t) * 4);
-                    f.x += v.x; f.y += v.y; f.z += v.z; f.w += v.w;
-                  }
-                  fma2(yb[t], yb[t + 1], bc, f.x, f.y);
-                  fma2(yb[t + 2], yb[t + 3], bc, f.z, f.w);
-                }
-              }
-#pragma unroll
-              for (int t = 0; t < 8; ++t) y[t0 + t] += yb[t];
-            }
-          }
         }
         if (i + 1 < tiles) first_entries(tile + 1);      // (on their way while this tile is passed on)
         // to the CTA that owns this row

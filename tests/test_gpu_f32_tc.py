@@ -63,6 +63,35 @@ def test_float32_rows_with_biases_of_their_own():
     assert _far(qmm.quantized_matmul(to_torch(xs, DEV), w, s, b, **kw), exact) <= 4e-7
 
 
+@pytest.mark.parametrize("m,kind,gs,k,tdt", [(48, "int4", 64, 4096, "f32"), (33, "int4", 32, 1056, "f32"), (20, "int4", 128, 2688, "f16"), (48, "int8", 128, 3200, "f32"),
+                                             (17, "int8", 32, 2080, "bf16"), (64, "int8", 64, 8256, "f32"), (12, "int4", 32, 14336, "f32")])
+def test_float32_rows_with_zero_points(m, kind, gs, k, tdt):
+    """Every group has a bias of its own: exact, and no further off than eight rows at a time (see below)."""
+    xs, (w, s, b), kw, _ = _case(m, k, 900, kind, gs, tdt, 5)
+    b = b + s * torch.randint(-5, 6, s.shape, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)).to(s.dtype)
+    exact = O.qmm_exact(xs, to_numpy(w), to_numpy(s), to_numpy(b), gs, kw["bits"])
+    x = to_torch(xs, DEV)
+    by_eight = torch.cat([qmm.quantized_matmul(x[i:i + 8], w, s, b, **kw) for i in range(0, m, 8)])
+    far = _far(qmm.quantized_matmul(x, w, s, b, **kw), exact)
+    assert far <= 4e-7 and far <= 1.05 * _far(by_eight, exact)      # (10800 results at least: their root mean square varies by 1 %)
+
+
+def test_float32_rows_infinite_beside_biases_of_their_own():
+    """A weight row with centred biases makes of an infinity what its weight does, whatever the biases of the rows beside it."""
+    xs, (w, s, b), kw, _ = _case(20, 256, 140, "int4", 64, "f32")
+    b = -8 * s
+    b[7] += s[7]
+    column = O.qmm_exact(np.eye(256, dtype=np.float32)[77:78], to_numpy(w), to_numpy(s), to_numpy(b), 64, 4)[0]
+    xs[2, 77] = np.inf
+    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), w, s, b, **kw))
+    with np.errstate(invalid="ignore"):
+        want = np.float32(np.inf) * column.astype(np.float32)
+    rest = np.arange(140) != 7
+    assert np.array_equal(np.isnan(y[2][rest]), np.isnan(want[rest]))
+    finite = rest & ~np.isnan(want)
+    assert np.array_equal(y[2][finite], want[finite])
+
+
 @pytest.mark.parametrize("out", [torch.bfloat16, torch.float16])
 def test_float32_rows_to_16_bits(out):
     xs, args, kw, exact = _case(37, 1024, 260, "int4", 64, "f32")
