@@ -103,8 +103,10 @@ typedef enum {
   QMM_ROUTE_GEMV = 1,       /* decode: M <= 16, weight streaming */
   QMM_ROUTE_GEMM_TC = 2,    /* prefill: tcgen05 tensor-core kernel */
   QMM_ROUTE_SIMT = 3,       /* float32 activations / shapes the others decline */
-  QMM_ROUTE_GEMV_FMMA = 4   /* only as an override: the decode family's floating-point mma.sync
+  QMM_ROUTE_GEMV_FMMA = 4,  /* only as an override: the decode family's floating-point mma.sync
                              * kernel also where the single-row integer kernel would be chosen */
+  QMM_ROUTE_F32_TC = 5      /* only as an override: the tensor-core kernel of float32 activations
+                             * also where the few-rows kernel would be chosen (see qmm_float32_plan) */
 } qmm_route_id;
 
 /* ---- library ---------------------------------------------------------------- */
@@ -327,6 +329,11 @@ int qmm_launch(const qmm_problem* problem, void* stream);
 /* The kernel family `qmm_launch` would choose for this problem (a qmm_route_id),
  * after the same validation, without touching the device. Negative = -qmm_status. */
 int qmm_route(const qmm_problem* problem);
+
+/* Of float32 activations (whose family is QMM_ROUTE_SIMT whichever kernel takes them): the plan of
+ * the tensor-core kernel -- rows of a chunk, CTAs that share K, partial tiles on their way to an
+ * owner -- or zeros where another kernel would run. Does not touch the device. */
+int qmm_float32_plan(const qmm_problem* problem, int32_t plan[3]);
 
 /* Validates exactly like qmm_quantized_matmul but launches nothing and accepts
  * host tensors: returns the status the real call would give for these shapes and

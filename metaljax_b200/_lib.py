@@ -19,7 +19,7 @@ NATIVE_PATH = os.path.join(_HERE, "_native.so")
 LIB_PATH = os.environ.get("QMM_LIBRARY") or os.path.join(_HERE, "libqmm.so")     # (a development build can be named)
 
 MODE = {"affine": 0, "mxfp4": 1}
-ROUTES = {0: "none", 1: "gemv", 2: "gemm_tc", 3: "simt", 4: "gemv_fmma"}
+ROUTES = {0: "none", 1: "gemv", 2: "gemm_tc", 3: "simt", 4: "gemv_fmma", 5: "f32_tc"}
 ELEM = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2, torch.uint8: 3,
         torch.uint32: 4, torch.int32: 5, torch.int8: 6}
 
@@ -148,6 +148,7 @@ _SIGNATURES = {
                                                                    ctypes.c_int, ctypes.c_int, ctypes.POINTER(Exchange),
                                                                    ctypes.c_void_p]),
     "qmm_route": (ctypes.c_int, [ctypes.POINTER(Problem)]),
+    "qmm_float32_plan": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.POINTER(ctypes.c_int32)]),
     # include/qmm_ep.h
     "qmm_ep_dispatch": (ctypes.c_int, [ctypes.POINTER(EpExchange), ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                        ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p]),
@@ -227,7 +228,7 @@ def stream_ptr(t) -> int:
 class force_route:
     """Context manager for tests: every launch inside goes to one kernel family
     ("gemv", "gemm_tc", "simt"; "gemv_fmma" = the decode family's floating-point mma.sync kernel
-    even for a single row) or fails with status 7 if that family declines it."""
+    even for a single row, "f32_tc" = the tensor-core kernel of float32 activations however few) or fails with status 7 if that family declines it."""
 
     def __init__(self, name: str):
         self.route = {v: k for k, v in ROUTES.items()}[name]

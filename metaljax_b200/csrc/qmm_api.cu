@@ -185,6 +185,7 @@ int route_of(const qmm_problem& p) {
   const int forced = g_route_override.load(std::memory_order_relaxed);
   if (forced == QMM_ROUTE_GEMV || forced == QMM_ROUTE_GEMV_FMMA) return gemv_supports(p) ? QMM_ROUTE_GEMV : -QMM_ERR_UNSUPPORTED;
   if (forced == QMM_ROUTE_GEMM_TC) return gemm_tc_supports(p) ? forced : -QMM_ERR_UNSUPPORTED;
+  if (forced == QMM_ROUTE_F32_TC) return f32_tc_supports(p) ? forced : -QMM_ERR_UNSUPPORTED;
   if (forced == QMM_ROUTE_SIMT) return forced;
   // Nine to sixteen rows are two passes of the few-rows kernel; against a long K, where its CTAs also meet in clusters, the
   // tensor-core kernel's one pass is the faster (16 rows, us: 4096 x 14336 22.1 against 17.4; at 4096 x 4096 9.3 / 9.8). It would be from K 4096 on
@@ -215,6 +216,7 @@ int launch_problem(const qmm_problem& p, cudaStream_t stream) {
     case QMM_ROUTE_NONE: return QMM_OK;
     case QMM_ROUTE_GEMV: return p.group_sizes ? launch_rows(p, stream) : launch_gemv(p, stream);
     case QMM_ROUTE_GEMM_TC: return launch_gemm_tc(p, stream);
+    case QMM_ROUTE_F32_TC: return launch_f32_tc(p, stream);
     // Float32 activations and what the others decline (unsorted gathers of more than 16 rows, K below 64): the
     // few-rows kernel takes them as columns of its MMAs, or, float32 activations of more than 8 rows, the tensor-core kernel of their own; the plain SIMT kernel is what a forced route cross-checks with.
     // Its codes go in without a magic number here, since the SIMT kernel's float32 sums are what such calls had: with it a float32 result
@@ -365,7 +367,7 @@ int qmm_version(void) { return QMM_VERSION; }
 const char* qmm_last_error(void) { return g_error; }
 
 int qmm_set_route_override(int route) {
-  if (route < QMM_ROUTE_NONE || route > QMM_ROUTE_GEMV_FMMA) return fail(QMM_ERR_UNSUPPORTED, "unknown route %d", route);
+  if (route < QMM_ROUTE_NONE || route > QMM_ROUTE_F32_TC) return fail(QMM_ERR_UNSUPPORTED, "unknown route %d", route);
   g_route_override.store(route, std::memory_order_relaxed);
   return QMM_OK;
 }
@@ -421,6 +423,17 @@ int qmm_route(const qmm_problem* problem) {
   const int route = route_of(*problem);
   if (route < 0) fail(-route, "the forced kernel family does not support this problem");
   return route;
+}
+
+int qmm_float32_plan(const qmm_problem* problem, int32_t plan[3]) {
+  if (!problem || !plan) return fail(QMM_ERR_NULL, "problem or plan is NULL");
+  int rc = validate_problem(*problem, false);
+  if (rc) return rc;
+  plan[0] = plan[1] = plan[2] = 0;
+  const int route = route_of(*problem);
+  if (route < 0) return fail(-route, "the forced kernel family does not support this problem");
+  if (route == QMM_ROUTE_F32_TC || (route == QMM_ROUTE_SIMT && route_override() != QMM_ROUTE_SIMT && f32_tc_pays(*problem))) f32_tc_plan(*problem, plan);
+  return QMM_OK;
 }
 
 int qmm_check_quantized_matmul(const qmm_tensor* x, const qmm_tensor* w, const qmm_tensor* scales,

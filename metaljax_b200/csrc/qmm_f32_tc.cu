@@ -787,11 +787,18 @@ int launch_kind(const qmm_problem& p, const F32Plan& pl, const CUtensorMap& wm, 
 // From nine rows on a pass here is cheaper than the few-rows kernel's (four rows each): 9 rows of 4096 x 4096 13.9 us against 16.8, of 256 x 512 4.8 against 6.2; up to
 // eight are two of its passes (5 rows 12.6). One weight, no gather; K as far as 16 rows' pieces fit shared memory (14336 with
 // 4-bit codes, 12288 with 8-bit ones).
-bool f32_tc_pays(const qmm_problem& p) {
+bool f32_tc_supports(const qmm_problem& p) {
   if (p.x_dtype != QMM_F32 || p.batch != 1 || p.lhs_idx || p.rhs_idx || p.group_sizes || p.mode == QMM_MODE_FLOAT) return false;
-  if (p.M <= 8 || p.K < kBK || p.K % 32 || p.K >= (1LL << 24) || p.N < 1 || p.N >= (1LL << 31) - 256) return false;
+  if (p.M < 1 || p.K < kBK || p.K % 32 || p.K >= (1LL << 24) || p.N < 1 || p.N >= (1LL << 31) - 256) return false;
   if ((p.M + 15) / 16 * ((p.N + kTileRows - 1) / kTileRows) >= (1LL << 31)) return false;
   return plan_of(p).t != 0;
+}
+
+bool f32_tc_pays(const qmm_problem& p) { return p.M > 8 && f32_tc_supports(p); }
+
+void f32_tc_plan(const qmm_problem& p, int plan[3]) {
+  const F32Plan pl = plan_of(p);
+  plan[0] = pl.t; plan[1] = pl.cluster; plan[2] = pl.slots;
 }
 
 int launch_f32_tc(const qmm_problem& p, cudaStream_t stream) {

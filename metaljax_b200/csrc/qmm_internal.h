@@ -58,6 +58,8 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
 bool rows_supports(const qmm_problem& p);
 // Float32 activations of more than a few rows on the tensor cores (f32_tc_pays: it takes them, and wins).
 int launch_f32_tc(const qmm_problem& p, cudaStream_t stream);
+bool f32_tc_supports(const qmm_problem& p);
+void f32_tc_plan(const qmm_problem& p, int plan[3]);     // of a problem that it supports: rows of a chunk, CTAs that share K, partial tiles on their way
 bool f32_tc_pays(const qmm_problem& p);
 bool rows_grouped_pays(const qmm_problem& p);
 // A checked problem on the kernel its route names; and whether that is the few-rows kernel for a grouped one.

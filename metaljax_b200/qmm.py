@@ -333,10 +333,8 @@ def dequantize(w, scales, biases=None, group_size=64, bits=4, mode="affine",
     return out
 
 
-def route(M, K, N, group_size=64, bits=4, mode="affine", x_dtype=torch.bfloat16,
-          table_dtype=None, y_dtype=None, batch=1, gather=False, ragged=False) -> str:
-    """Name of the kernel family libqmm picks for a problem of this shape (no device
-    work): "gemv", "gemm_tc", "simt" or "none"."""
+def _problem(M, K, N, group_size=64, bits=4, mode="affine", x_dtype=torch.bfloat16,
+             table_dtype=None, y_dtype=None, batch=1, gather=False, ragged=False):
     p = _lib.Problem()
     p.struct_size = _lib.ctypes.sizeof(_lib.Problem)
     p.mode, p.bits, p.group_size = _mode_id(mode), bits, group_size
@@ -349,10 +347,27 @@ def route(M, K, N, group_size=64, bits=4, mode="affine", x_dtype=torch.bfloat16,
         p.lhs_idx = p.rhs_idx = 16
     if ragged:
         p.group_sizes = 16
+    return p
+
+
+def route(M, K, N, group_size=64, bits=4, mode="affine", x_dtype=torch.bfloat16,
+          table_dtype=None, y_dtype=None, batch=1, gather=False, ragged=False) -> str:
+    """Name of the kernel family libqmm picks for a problem of this shape (no device
+    work): "gemv", "gemm_tc", "simt" or "none"."""
+    p = _problem(M, K, N, group_size, bits, mode, x_dtype, table_dtype, y_dtype, batch, gather, ragged)
     r = _lib.lib().qmm_route(_lib.ctypes.byref(p))
     if r < 0:
         _lib.check(-r)
     return _lib.ROUTES[r]
+
+
+def float32_plan(M, K, N, group_size=64, bits=4, mode="affine", table_dtype=None):
+    """Of a product of float32 activations: (rows of a chunk, CTAs that share K, partial tiles on their way) on the
+    tensor-core kernel, or None where another kernel takes it (no device work)."""
+    p = _problem(M, K, N, group_size, bits, mode, torch.float32, table_dtype)
+    plan = (ctypes.c_int32 * 3)()
+    _lib.check(_lib.lib().qmm_float32_plan(_lib.ctypes.byref(p), plan))
+    return tuple(plan) if plan[0] else None
 
 
 # --------------------------------------------------------------------------------------

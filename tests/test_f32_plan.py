@@ -1,0 +1,42 @@
+"""Which products of float32 activations the tensor-core kernel takes, and in what plan: asked without a device."""
+
+import pytest
+import torch
+
+from metaljax_b200 import _lib, qmm
+
+
+def test_rows_that_are_few_enough_for_the_few_rows_kernel():
+    assert qmm.float32_plan(8, 4096, 4096) is None
+    assert qmm.float32_plan(9, 4096, 4096) is not None
+    with _lib.force_route("f32_tc"):
+        assert qmm.float32_plan(8, 4096, 4096) is not None
+    with _lib.force_route("simt"):
+        assert qmm.float32_plan(9, 4096, 4096) is None
+
+
+@pytest.mark.parametrize("kind,gs,longest", [("affine", 64, 14336), ("affine8", 64, 12288), ("mxfp4", 32, 14336)])
+def test_the_longest_contraction(kind, gs, longest):
+    kw = dict(group_size=gs, bits=8 if kind == "affine8" else 4, mode="mxfp4" if kind == "mxfp4" else "affine")
+    with _lib.force_route("f32_tc"):
+        assert qmm.float32_plan(64, longest, 4096, **kw)[1] == 8
+        with pytest.raises(_lib.QmmError):
+            qmm.float32_plan(64, longest + gs, 4096, **kw)
+    assert qmm.float32_plan(64, longest + gs, 4096, **kw) is None
+
+
+def test_48_rows_have_no_more_than_512_codes_to_a_cta():
+    """Their sums have one level (and one scale)."""
+    with _lib.force_route("f32_tc"):
+        for k in range(128, 14337, 128):
+            rows, cluster, slots = qmm.float32_plan(48, k, 14336)
+            assert rows in (16, 32, 48) and cluster in (1, 2, 4, 8) and slots in (1, 2)
+            assert rows < 48 or -(-k // 128) <= 4 * cluster
+
+
+def test_what_it_does_not_take():
+    p = qmm._problem(64, 4096, 4096, x_dtype=torch.float32, batch=2)
+    plan = (_lib.ctypes.c_int32 * 3)(7, 7, 7)
+    _lib.check(_lib.lib().qmm_float32_plan(_lib.ctypes.byref(p), plan))
+    assert list(plan) == [0, 0, 0]
+    assert _lib.lib().qmm_float32_plan(None, plan) == 1

@@ -29,29 +29,46 @@ def _case(m, k, n, kind, gs, tdt, seed=0):
     return xs, [to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV)], kw, exact
 
 
+def _product(x, *args, **kw):
+    """On the tensor-core kernel, or not at all."""
+    with _lib.force_route("f32_tc"):
+        return qmm.quantized_matmul(x, *args, **kw)
+
+
 def _far(y, exact):
     return np.linalg.norm(to_numpy(y).astype(np.float64) - exact) / np.linalg.norm(exact)
 
 
-@pytest.mark.parametrize("m,k,n,kind,gs,tdt", [
-    (9, 64, 1, "int4", 64, "f32"),              # half a step
-    (16, 96, 127, "mxfp4", 32, None),           # three quarters of one
-    (17, 160, 129, "int4", 32, "bf16"),         # two steps, the last a quarter full; two tiles
-    (33, 4096, 640, "int4", 64, "f32"),         # 48 rows, eight CTAs
-    (49, 4096, 2500, "int4", 128, "f16"),       # two chunks, more tiles than clusters
-    (64, 2112, 385, "int8", 64, "f32"),         # 17 steps over eight CTAs
-    (100, 1088, 257, "int8", 32, "bf16"),
-    (12, 14336, 256, "int4", 128, "f32"),       # the longest stretch of K that 16 rows leave room for
-    (20, 14368, 130, "mxfp4", 32, None),        # ... and 32 codes more, which do not fit: the few-rows kernel
-    (48, 2880, 700, "mxfp4", 32, None),         # 90 table bytes a row
-    (31, 320, 200, "int8", 64, "f16"),
-    (200, 576, 19300, "int4", 64, "f32"),       # many tiles, no cluster
+@pytest.mark.parametrize("m,k,n,kind,gs,tdt,plan", [
+    (9, 64, 1, "int4", 64, "f32", (16, 1, 2)),              # half a step
+    (16, 96, 127, "mxfp4", 32, None, (16, 1, 2)),           # three quarters of one
+    (17, 160, 129, "int4", 32, "bf16", (16, 2, 2)),         # two steps, the last a quarter full; two tiles
+    (33, 4096, 1790, "int4", 64, "f32", (48, 8, 1)),        # 48 rows, eight CTAs, one partial tile on its way
+    (33, 4096, 640, "int4", 64, "f32", (16, 8, 2)),         # three chunks of 16
+    (49, 4096, 2500, "int4", 128, "f16", (32, 8, 2)),       # two chunks, more tiles than clusters
+    (64, 2112, 385, "int8", 64, "f32", (16, 8, 2)),         # 17 steps over eight CTAs
+    (100, 1088, 257, "int8", 32, "bf16", (16, 4, 2)),
+    (12, 14336, 256, "int4", 128, "f32", (16, 8, 2)),       # the longest stretch of K that 16 rows leave room for
+    (12, 12288, 300, "int8", 64, "f32", (16, 8, 1)),        # ... of 8-bit codes: one partial tile on its way
+    (48, 2880, 700, "mxfp4", 32, None, (16, 8, 2)),         # 90 table bytes a row
+    (31, 320, 200, "int8", 64, "f16", (16, 2, 2)),
+    (200, 576, 19300, "int4", 64, "f32", (32, 1, 2)),       # many tiles, no cluster
 ])
-def test_float32_rows(m, k, n, kind, gs, tdt):
+def test_float32_rows(m, k, n, kind, gs, tdt, plan):
     xs, args, kw, exact = _case(m, k, n, kind, gs, tdt)
-    y = qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw)
+    with _lib.force_route("f32_tc"):
+        assert qmm.float32_plan(m, k, n, table_dtype=args[1].dtype, **kw) == plan
+    y = _product(to_torch(xs, DEV), *args, **kw)
     assert _far(y, exact) <= 4e-7
     assert _lib.poll_status() == 0
+
+
+def test_float32_rows_that_do_not_fit():
+    """32 codes more than 16 rows' stretches leave room for: the few-rows kernel's."""
+    xs, args, kw, exact = _case(20, 14368, 130, "mxfp4", 32, None)
+    with pytest.raises(_lib.QmmError):
+        _product(to_torch(xs, DEV), *args, **kw)
+    assert _far(qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw), exact) <= 4e-7
 
 
 def test_float32_rows_with_biases_of_their_own():
@@ -60,7 +77,7 @@ def test_float32_rows_with_biases_of_their_own():
     b = -8 * s
     b[200, 3] = 0.7
     exact = O.qmm_exact(xs, to_numpy(w), to_numpy(s), to_numpy(b), 64, 4)
-    assert _far(qmm.quantized_matmul(to_torch(xs, DEV), w, s, b, **kw), exact) <= 4e-7
+    assert _far(_product(to_torch(xs, DEV), w, s, b, **kw), exact) <= 4e-7
 
 
 @pytest.mark.parametrize("m,kind,gs,k,tdt", [(48, "int4", 64, 4096, "f32"), (33, "int4", 32, 1056, "f32"), (20, "int4", 128, 2688, "f16"), (48, "int8", 128, 3200, "f32"),
@@ -72,7 +89,7 @@ def test_float32_rows_with_zero_points(m, kind, gs, k, tdt):
     exact = O.qmm_exact(xs, to_numpy(w), to_numpy(s), to_numpy(b), gs, kw["bits"])
     x = to_torch(xs, DEV)
     by_eight = torch.cat([qmm.quantized_matmul(x[i:i + 8], w, s, b, **kw) for i in range(0, m, 8)])
-    far = _far(qmm.quantized_matmul(x, w, s, b, **kw), exact)
+    far = _far(_product(x, w, s, b, **kw), exact)
     assert far <= 4e-7 and far <= 1.05 * _far(by_eight, exact)      # (10800 results at least: their root mean square varies by 1 %)
 
 
@@ -83,7 +100,7 @@ def test_float32_rows_infinite_beside_biases_of_their_own():
     b[7] += s[7]
     column = O.qmm_exact(np.eye(256, dtype=np.float32)[77:78], to_numpy(w), to_numpy(s), to_numpy(b), 64, 4)[0]
     xs[2, 77] = np.inf
-    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), w, s, b, **kw))
+    y = to_numpy(_product(to_torch(xs, DEV), w, s, b, **kw))
     with np.errstate(invalid="ignore"):
         want = np.float32(np.inf) * column.astype(np.float32)
     rest = np.arange(140) != 7
@@ -95,8 +112,8 @@ def test_float32_rows_infinite_beside_biases_of_their_own():
 @pytest.mark.parametrize("out", [torch.bfloat16, torch.float16])
 def test_float32_rows_to_16_bits(out):
     xs, args, kw, exact = _case(37, 1024, 260, "int4", 64, "f32")
-    y = qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw, out_dtype=out)
-    assert torch.equal(y, qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw).to(out))
+    y = _product(to_torch(xs, DEV), *args, **kw, out_dtype=out)
+    assert torch.equal(y, _product(to_torch(xs, DEV), *args, **kw).to(out))
 
 
 @pytest.mark.parametrize("m", [12, 40])            # with slices of 512 codes, and with one for all of a stretch
@@ -110,7 +127,7 @@ def test_float32_rows_at_the_ends_of_their_range(m, kind, k, power):
     if power < 0 and kind != "int4":
         xs[1, 512:] = np.ldexp(xs[1, 512:], 60)
     exact = O.qmm_exact(xs, to_numpy(args[0]), to_numpy(args[1]), None if args[2] is None else to_numpy(args[2]), kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
-    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw)).astype(np.float64)
+    y = to_numpy(_product(to_torch(xs, DEV), *args, **kw)).astype(np.float64)
     assert np.isfinite(y).all()
     far = np.linalg.norm(y - exact, axis=1) / np.linalg.norm(exact, axis=1)      # of each row: they are as far apart as their slices
     assert far.max() <= 4e-7
@@ -127,7 +144,7 @@ def test_float32_rows_are_as_exact_as_eight_at_a_time(kind, gs, k, one_sign):
     exact = O.qmm_exact(xs, to_numpy(args[0]), to_numpy(args[1]), None if args[2] is None else to_numpy(args[2]), gs, kw["bits"], mode=kw.get("mode", "affine"))
     x = to_torch(xs, DEV)
     by_eight = torch.cat([qmm.quantized_matmul(x[i:i + 8], *args, **kw) for i in range(0, 48, 8)])
-    assert _far(qmm.quantized_matmul(x, *args, **kw), exact) <= 1.02 * _far(by_eight, exact)
+    assert _far(_product(x, *args, **kw), exact) <= 1.02 * _far(by_eight, exact)
 
 
 def test_float32_rows_below_the_range_of_4_bit_codes():
@@ -136,17 +153,19 @@ def test_float32_rows_below_the_range_of_4_bit_codes():
     xs = np.ldexp(xs, -122)
     w, s, b = (to_numpy(a) for a in args)
     dense = O.qmm_exact(np.eye(1024, dtype=np.float32), w, s, b, 64, 4)
-    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw)).astype(np.float64)
+    y = to_numpy(_product(to_torch(xs, DEV), *args, **kw)).astype(np.float64)
     assert np.linalg.norm(y - O.qmm_exact(xs, w, s, b, 64, 4)) <= 1.25 * 2.0 ** -133 / np.sqrt(12) * np.sqrt(len(xs)) * np.linalg.norm(dense)
 
 
+@pytest.mark.parametrize("kind", ["mxfp4", "int4", "int8"])
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
-def test_float32_rows_that_are_not_finite(value):
+def test_float32_rows_that_are_not_finite(value, kind):
     """An infinity times a positive, a negative or a zero weight, as a sum of products has it; the rows beside it as ever."""
-    xs, args, kw, exact = _case(20, 1120, 300, "mxfp4", 32, None)
-    column = O.qmm_exact(np.eye(1120, dtype=np.float32)[17:18], to_numpy(args[0]), to_numpy(args[1]), None, 32, 4, mode="mxfp4")[0]
+    xs, args, kw, exact = _case(20, 1120, 300, kind, 32, None if kind == "mxfp4" else "f32")
+    w, s, b = (None if a is None else to_numpy(a) for a in args)
+    column = O.qmm_exact(np.eye(1120, dtype=np.float32)[17:18], w, s, b, 32, kw["bits"], mode=kw.get("mode", "affine"))[0]
     xs[3, 17] = value
-    y = to_numpy(qmm.quantized_matmul(to_torch(xs, DEV), *args, **kw))
+    y = to_numpy(_product(to_torch(xs, DEV), *args, **kw))
     with np.errstate(invalid="ignore"):
         want = (np.float32(value) * column.astype(np.float32))
     assert np.array_equal(np.isnan(y[3]), np.isnan(want)) and np.array_equal(y[3][~np.isnan(want)], want[~np.isnan(want)])
@@ -159,13 +178,13 @@ def test_float32_rows_replay():
     x, y = to_torch(xs, DEV), torch.zeros((64, 1024), device=DEV)
     stream = torch.cuda.Stream()
     with torch.cuda.stream(stream):
-        qmm.quantized_matmul(x, *args, out=y, **kw)
+        _product(x, *args, out=y, **kw)
         stream.synchronize()
         first = y.clone()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, stream=stream):
             for _ in range(3):
-                qmm.quantized_matmul(x, *args, out=y, **kw)
+                _product(x, *args, out=y, **kw)
         y.zero_()
         graph.replay()
         stream.synchronize()
