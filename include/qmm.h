@@ -366,7 +366,8 @@ int qmm_poll_status_static(int* status_out);
 int qmm_set_wait_limit(long long clocks);
 
 /* The split products' scratch comes from a memory pool of the library, one per device, which keeps
- * up to 64 MiB between calls. Returns what the current device's pool holds unused to the driver.
+ * up to 64 MiB between calls. Returns what the current device's pool holds unused to the driver, and
+ * the few bytes that qmm_pack_dense_layer keeps for every call that was under way at the same time.
  * No counterpart in the reference. */
 int qmm_release_scratch(void);
 

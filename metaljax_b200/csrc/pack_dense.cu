@@ -256,7 +256,7 @@ int with_types(int scale_dtype, int zero_dtype, F&& f) {
   return fail(QMM_ERR_DTYPE, "pack_dense: scales are bf16, f16 or f32");
 }
 
-// Sums and host words, one pair per call that is under way; they stay for later calls of the device.
+// Sums and host words, one pair per call that is under way; they stay for later calls of the device (qmm_release_scratch gives them back).
 struct Slot {
   Sums* sums;
   volatile Told* told;
@@ -282,6 +282,7 @@ bool take_slot(int dev, cudaStream_t stream, Slot* out) {
     if (d) cudaFree(d);
     return false;
   }
+  count_alloc();
   out->sums = static_cast<Sums*>(d);
   out->told = static_cast<volatile Told*>(h);
   out->told->ticket = 0;
@@ -290,6 +291,21 @@ bool take_slot(int dev, cudaStream_t stream, Slot* out) {
 }
 
 }  // namespace
+
+void release_pack_slots() {
+  const int dev = current_device();
+  if (dev < 0) return;
+  std::vector<Slot> slots;
+  {
+    std::lock_guard<std::mutex> lock(g_slots_mutex);
+    slots.swap(g_slots[dev]);
+  }
+  for (const Slot& s : slots) {
+    cudaFree(s.sums);
+    cudaFreeHost(const_cast<Told*>(s.told));
+  }
+}
+
 }  // namespace qmm
 
 using namespace qmm;
@@ -301,6 +317,8 @@ extern "C" int qmm_pack_dense_layer(const void* packed, uint32_t* words, const v
   if (group_size < 32 || (K / G) % group_size) return fail(QMM_ERR_SHAPE, "pack_dense_layer: the group size divides the stored groups");
   const int64_t table_tiles = (N + 31) / 32 * ((K / group_size + 31) / 32), code_tiles = (N + kTileN - 1) / kTileN * ((K + kTileK - 1) / kTileK);
   if (table_tiles + code_tiles >= (1LL << 31)) return fail(QMM_ERR_SHAPE, "pack_dense_layer: the layer is too large");
+  const int rt = with_types(scale_dtype, zero ? zero_dtype : QMM_U8, [](auto, auto) -> int { return QMM_OK; });
+  if (rt) return rt;                               // (before a slot is taken: one that does not come back is lost)
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)

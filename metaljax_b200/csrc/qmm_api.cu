@@ -403,7 +403,10 @@ int qmm_set_wait_limit(long long clocks) {
   return QMM_OK;
 }
 
-int qmm_release_scratch(void) { return release_scratch(); }
+int qmm_release_scratch(void) {
+  release_pack_slots();
+  return release_scratch();
+}
 
 uint64_t qmm_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 

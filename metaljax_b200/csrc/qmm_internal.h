@@ -45,6 +45,7 @@ void set_scratch_override(const ScratchBlock* block);
 void* scratch_alloc(size_t bytes, cudaStream_t stream);
 void scratch_free(void* ptr, cudaStream_t stream);
 int release_scratch();
+void release_pack_slots();               // ... what qmm_pack_dense_layer keeps on the current device
 
 int launch_gemv(const qmm_problem& p, cudaStream_t stream);
 bool gemv_supports(const qmm_problem& p);

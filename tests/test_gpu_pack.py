@@ -2,10 +2,12 @@
 every word and table entry the same, at the edges of the 64 x 256 tile, odd column counts, group sizes that
 allow 128, 64 and 32 codes per table entry, and tables that have to stay float32. Needs a B200."""
 
+import ctypes
+
 import pytest
 import torch
 
-from metaljax_b200 import qmm
+from metaljax_b200 import _lib, qmm
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +85,33 @@ def test_layers_packed_one_after_another_and_by_several_threads():
     for t in threads:
         t.join()
     assert not wrong
+
+
+def _layer(packed, scale, zero, group, narrow=False, scale_dtype=None):
+    """qmm_pack_dense_layer itself: (status, words, scales, biases, digest, facts)."""
+    k, n = packed.shape[0], scale.shape[1]
+    words = torch.empty((n, k // 8), dtype=torch.uint32, device=DEV)
+    tables = [torch.empty((n, k // group), dtype=scale.dtype if narrow else torch.float32, device=DEV) for _ in range(2)]
+    digest, facts = ctypes.c_uint64(), ctypes.c_uint32()
+    rc = _lib.lib().qmm_pack_dense_layer(packed.data_ptr(), words.data_ptr(), scale.data_ptr(), None if zero is None else zero.data_ptr(),
+                                         _lib.ELEM[scale.dtype] if scale_dtype is None else scale_dtype, 0 if zero is None else _lib.ELEM[zero.dtype],
+                                         tables[0].data_ptr(), tables[1].data_ptr(), int(narrow), scale.shape[0], n, k, group, ctypes.byref(digest), ctypes.byref(facts),
+                                         _lib.stream_ptr(packed))
+    return rc, words, *tables, digest.value, facts.value
+
+
+def test_what_a_layer_keeps_is_counted_and_given_back():
+    """A call's sums and host words stay for the next one; a call that is refused takes none."""
+    packed, scale = torch.zeros((64, 4), dtype=torch.int8, device=DEV), torch.ones((1, 8), device=DEV)
+    lib = _lib.lib()
+    _lib.release_scratch()
+    before = _lib.alloc_count()
+    for _ in range(3):
+        assert _layer(packed, scale, None, 64, scale_dtype=_lib.ELEM[torch.uint8])[0] == 2
+    assert _lib.alloc_count() == before and b"scales" in lib.qmm_last_error()
+    for _ in range(3):
+        assert _layer(packed, scale, None, 64)[0] == 0
+    assert _lib.alloc_count() == before + 1
+    _lib.release_scratch()
+    assert _layer(packed, scale, None, 64)[0] == 0
+    assert _lib.alloc_count() == before + 2
