@@ -696,6 +696,7 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
 
 struct F32Plan {
   int t, cluster, most_steps, slots, boxes;      // t == 0: the activations do not fit
+  int64_t items, chunks;                         // (chunk, tile) items, chunks of t rows
 };
 
 // The plan of the least load, in clocks of the busiest cluster: rounds of tiles x (its K blocks, plus what a tile costs besides: the push, the sum), and the
@@ -719,11 +720,25 @@ F32Plan plan_of(const qmm_problem& p) {
       if (!best.t || load < least) {
         least = load;
         const int slots = smem_of(t, steps, 2, kASlots, bits) <= kSmemLimit ? 2 : 1, boxes = static_cast<int>((kSmemLimit - smem_of(t, steps, slots, 0, bits)) / box_bytes(bits));
-        best = {t, c, steps, slots, boxes < kMaxBoxes ? boxes : kMaxBoxes};
+        best = {t, c, steps, slots, boxes < kMaxBoxes ? boxes : kMaxBoxes, items, chunks};
       }
     }
   }
   return best;
+}
+
+// What a plan is expected to take, in us: rounds of tiles -- a step's codes, its accumulators (one a group; reading, scaling and adding T columns of each),
+// the rows passed on -- and the conversion of the activations for every chunk that a cluster meets. GPCs differ in their SMs, so that fewer clusters fit than
+// their CTAs would: of eight 14 or 15 of 18, of four 33 of 37. Fitted to 2650 timed plans of 1400 random products (9..100 rows, K 128..14336, N 128..32000, all
+// kinds); root mean square error 10 %.
+double estimate(const qmm_problem& p, const F32Plan& pl) {
+  const bool mx = p.mode == QMM_MODE_MXFP4, bytes = !mx && p.bits == 8;
+  const int sms = device_sm_count(), step_units = mx ? 4 : bytes && p.group_size == 128 ? 2 : kStepK / p.group_size;
+  const int64_t fit = pl.cluster == 8 ? sms * 14 / 148 : pl.cluster == 4 ? sms * 33 / 148 : sms / pl.cluster, clusters = fit < pl.items ? fit > 0 ? fit : 1 : pl.items;
+  const int64_t rounds = (pl.items + clusters - 1) / clusters, tiles = pl.items / pl.chunks, meets = rounds > 1 ? (rounds + tiles - 2) / tiles + 1 : 1;
+  const int64_t passes = pl.chunks < meets ? pl.chunks : meets, steps = pl.most_steps;
+  return 3.6 + rounds * (0.75 + steps * (bytes ? 0.46 : 0.31) + steps * step_units * (0.14 + 0.0013 * pl.t) + 0.048 * pl.t) +
+         passes * steps * pl.t * (mx || bytes ? 0.026 : 0.014);
 }
 
 template <int QK, int T, bool WIDE>
@@ -782,19 +797,25 @@ int launch_kind(const qmm_problem& p, const F32Plan& pl, const CUtensorMap& wm, 
   return launch_t<QK, 16>(p, pl, wm, fp, stream);
 }
 
-}  // namespace
-
-// From nine rows on a pass here is cheaper than the few-rows kernel's (four rows each): 9 rows of 4096 x 4096 13.9 us against 16.8, of 256 x 512 4.8 against 6.2; up to
-// eight are two of its passes (5 rows 12.6). One weight, no gather; K as far as 16 rows' pieces fit shared memory (14336 with
-// 4-bit codes, 12288 with 8-bit ones).
-bool f32_tc_supports(const qmm_problem& p) {
+// One weight, no gather; and K as far as 16 rows' pieces fit shared memory (14336 with 4-bit codes, 12288 with 8-bit ones), which the plan says.
+bool may_take(const qmm_problem& p) {
   if (p.x_dtype != QMM_F32 || p.batch != 1 || p.lhs_idx || p.rhs_idx || p.group_sizes || p.mode == QMM_MODE_FLOAT) return false;
   if (p.M < 1 || p.K < kBK || p.K % 32 || p.K >= (1LL << 24) || p.N < 1 || p.N >= (1LL << 31) - 256) return false;
-  if ((p.M + 15) / 16 * ((p.N + kTileRows - 1) / kTileRows) >= (1LL << 31)) return false;
-  return plan_of(p).t != 0;
+  return (p.M + 15) / 16 * ((p.N + kTileRows - 1) / kTileRows) < (1LL << 31);
 }
 
-bool f32_tc_pays(const qmm_problem& p) { return p.M > 8 && f32_tc_supports(p); }
+}  // namespace
+
+bool f32_tc_supports(const qmm_problem& p) { return may_take(p) && plan_of(p).t != 0; }
+
+// Up to eight rows are two passes of the few-rows kernel, which a pass here does not beat (5 rows of 4096 x 4096 12.6 us). From nine on the two estimates decide. Of
+// 1214 random products (as above) 224 were more than 3 % slower here than there, up to 2.4 times (few tiles of little K, groups of 32, whose accumulators are
+// many: 9 rows mxfp4 160 x 8576 16.5 / 9.0 us); as decided 28 are, and all take 1 % more than the better kernel of each would.
+bool f32_tc_pays(const qmm_problem& p) {
+  if (p.M <= 8 || !may_take(p)) return false;
+  const F32Plan pl = plan_of(p);
+  return pl.t != 0 && (!rows_supports(p) || estimate(p, pl) <= 0.97 * rows_estimate(p));
+}
 
 void f32_tc_plan(const qmm_problem& p, int plan[3]) {
   const F32Plan pl = plan_of(p);

@@ -57,6 +57,7 @@ struct RowsGather {            // grouped products whose rows of x are picked by
 // `exact`: 16-bit activations whose sums are to be as exact as plain float32 ones (float32 activations' always are).
 int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr, bool exact = false);
 bool rows_supports(const qmm_problem& p);
+double rows_estimate(const qmm_problem& p);      // what a dense product of float32 activations is expected to take here, us
 // Float32 activations of more than a few rows on the tensor cores (f32_tc_pays: it takes them, and wins).
 int launch_f32_tc(const qmm_problem& p, cudaStream_t stream);
 bool f32_tc_supports(const qmm_problem& p);

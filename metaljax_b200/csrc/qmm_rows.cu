@@ -44,7 +44,6 @@ size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
 RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh, int segs) {
   const int sms = device_sm_count();
   RowsPlan best = {};
-  double best_load = 0.0;
   for (int blocks = kMaxBlocks; blocks >= (sh.exact ? kMaxBlocks : 1); --blocks) {
     const int64_t items = chunks * ((rows + kBlockRows * blocks - 1) / (kBlockRows * blocks));
     for (int c = 1; c <= kMaxCluster; c *= 2) {
@@ -78,16 +77,30 @@ RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh
       const double tile = blocks == 2 ? pl.slices_per_warp + (c > 1 ? 0.55 : 0.5) : 0.5 * pl.slices_per_warp + (c > 1 ? 0.4 : 0.35);
       double load = static_cast<double>(tiles) * busy * tile + (c > 1 ? 4.0 : 0.0);
       if (pl.ring == 1) load *= 100.0;               // (nothing is loaded while a box is worked on: where nothing else fits)
-      if (!best.warps || load < best_load) {
-        best = pl;
-        best_load = load;
-      }
+      pl.load = load;
+      if (!best.warps || load < best.load) best = pl;
     }
   }
   return best;
 }
 
+// Rows of a chunk are what the registers take. Nine to sixteen rows are two chunks: the CTAs that work on either half pass over
+// the weight side by side, so that the second reads it from L2 (16 rows of 4096 x 4096: 9.2 us; as one chunk of 16, half of whose activations
+// live in shared memory, 14.2).
+RowsShape shape_of(const qmm_problem& p, bool exact) {
+  const bool mx = p.mode == QMM_MODE_MXFP4;
+  const int bits = (!mx && p.bits == 8) ? 8 : 4, group = mx ? 32 : p.group_size;
+  return {p.x_dtype == QMM_F32 ? 4 : 8, kSliceK / group, mx ? kTabE8 : (p.table_dtype == QMM_BF16 ? kTabBf16 : (p.table_dtype == QMM_F16 ? kTabF16 : kTabF32)),
+          kBlockRows * kSliceK * bits / 8, exact && !mx && p.x_dtype != QMM_F32};
+}
+
 }  // namespace
+
+double rows_estimate(const qmm_problem& p) {
+  const RowsShape sh = shape_of(p, true);
+  const double load = plan_rows((p.M + sh.tokens - 1) / sh.tokens, p.N, static_cast<int>((p.K + kSliceK - 1) / kSliceK), sh, 0).load;
+  return 5.3 + load * (sh.groups == 16 ? 0.41 : sh.groups == 8 ? 0.38 : 0.34);
+}
 
 bool rows_supports(const qmm_problem& p) {
   if (p.mode == QMM_MODE_FLOAT || p.K < 32 || p.K % 32 || p.K >= (1LL << 30) || p.N < 1 || p.M < 1 || p.batch < 1) return false;
@@ -136,15 +149,11 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
   rp.weight_rows = (p.rhs_idx || p.group_sizes || p.w_batch_stride) ? rp.N : 0;
   rp.table_dtype = p.table_dtype; rp.y_dtype = p.y_dtype;
   const int slices = (rp.K + kSliceK - 1) / kSliceK;
-  // Rows of a chunk: what the registers take. Nine to sixteen rows are two chunks: the CTAs that work on either half pass over
-  // the weight side by side, so that the second reads it from L2 (16 rows of 4096 x 4096: 9.2 us; as one chunk of 16, half of whose activations
-  // live in shared memory, 14.2).
-  const int chunk = p.x_dtype == QMM_F32 ? 4 : 8;
+  const RowsShape sh = shape_of(p, exact);
+  const int chunk = sh.tokens;
   const int64_t per_seg = p.group_sizes ? (p.M + p.batch - 1) / p.batch : p.M;      // grouped: of an average expert
   const int64_t live = p.group_sizes ? (p.batch < p.M ? p.batch : p.M) : p.batch;
   const int entry = mx ? 1 : (p.table_dtype == QMM_F32 ? 4 : 2);
-  const RowsShape sh = {chunk, kSliceK / group, mx ? kTabE8 : (p.table_dtype == QMM_BF16 ? kTabBf16 : (p.table_dtype == QMM_F16 ? kTabF16 : kTabF32)),
-                        kBlockRows * kSliceK * bits / 8, exact && !mx && p.x_dtype != QMM_F32};
   const int64_t nweights = p.num_weights > 0 ? p.num_weights : (p.w_batch_stride ? p.batch : 1);
   rp.table_bytes = nweights * p.N * rp.groups * entry;
   // (a slice's entries start on the units that its own row of entries and a row of the table are multiples of)

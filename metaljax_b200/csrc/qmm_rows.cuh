@@ -1060,6 +1060,7 @@ struct RowsPlan {
   int blocks, cluster, warps, slices_per_cta, slices_per_warp, ring, red_bufs, grid;
   int64_t items;                 // (chunk, tile) items of a dense product
   size_t smem;
+  double load;                   // what it is expected to take (see plan_rows)
 };
 
 struct RowsShape {

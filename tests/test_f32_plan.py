@@ -40,3 +40,18 @@ def test_what_it_does_not_take():
     _lib.check(_lib.lib().qmm_float32_plan(_lib.ctypes.byref(p), plan))
     assert list(plan) == [0, 0, 0]
     assert _lib.lib().qmm_float32_plan(None, plan) == 1
+
+
+@pytest.mark.parametrize("m,k,n,kw,taken", [
+    (9, 8576, 160, dict(group_size=32, mode="mxfp4"), False),       # us on a B200, few-rows / tensor cores: 9.0 / 16.5
+    (14, 8192, 160, dict(group_size=32), False),                    # 9.7 / 15.0
+    (44, 2304, 128, dict(group_size=32, bits=8), False),            # 7.5 / 10.5
+    (9, 4096, 4096, dict(), True),                                  # 18.2 / 14.0
+    (33, 4096, 4096, dict(), True),                                 # 35.5 / 25.0
+    (64, 14336, 4096, dict(group_size=32), True),                   # 272 / 185
+    (16, 4096, 14336, dict(group_size=32, mode="mxfp4"), True),     # 88 / 47
+    (64, 1024, 1024, dict(group_size=128, bits=8), True),           # 14.5 / 8.6
+])
+def test_the_kernel_that_is_expected_to_be_the_faster(m, k, n, kw, taken):
+    plan = qmm.float32_plan(m, k, n, **kw)
+    assert (plan is not None) == taken
