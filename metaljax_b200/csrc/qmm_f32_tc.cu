@@ -164,7 +164,6 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
 
   auto wait = [&](uint32_t bar, uint32_t parity, int where) -> bool { return wait_phase(smem + bar, parity, abort_at, where); };
   auto init = [&](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem + bar), "r"(n)); };
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   // What an adding-up lane reads of a tile's tables: four entries of its row at a time, and which of them lie in its CTA's K.
   const int trow_lane = (warp & 3) * 32 + lane;
@@ -208,6 +207,9 @@ qmm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const F32Params p) 
   __syncthreads();
   if (csize > 1) cluster_barrier();
   tc_fence_after();
+  // Not before tensor memory is this CTA's: a CTA of the next launch that came first (two fit an SM's shared memory where K is short; today registers forbid it) would
+  // hold some while it waits for this grid, and the allocation above has no limit.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   uint32_t tmem;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(smem + kTmemSlot) : "memory");
   tmem = __shfl_sync(0xffffffffu, tmem, 0);

@@ -268,6 +268,8 @@ struct Plan {
   static_assert(kStages >= kTeams, "");
   static_assert(kACol0 + kStages * kStep * 32 <= 512, "the A ring fits tensor memory");
   static_assert(kFixed + kLeastPlaces * kWBytes <= kBudget, "");
+  // (the next launch may start before this one's tensor memory is allocated: none of its CTAs may get onto the SM with some of it)
+  static_assert(kFixed + kLeastPlaces * kWBytes > 128 * 1024, "one CTA an SM, and none of qmm_f32_tc.cu's (100 KB and more) beside it");
   static_assert(kTeams * kStep % kPer == 0, "a team's next step lies whole boxes ahead");
   static_assert((2 * kMostBoxes + 3 * kStages + 2) * 8 + 16 <= kBarBytes, "");
 };
