@@ -254,7 +254,11 @@ struct Plan {
   static constexpr int kWBytes = kBF * kBoxBytes;
   static constexpr int kACol0 = BT;                           // the A ring starts behind D's columns [0, BT)
   static constexpr int kTeamCols = BT / kTeams;               // columns of D that a team drains ...
-  static constexpr int kCols = BT == 128 ? 32 : 16;            // ... so many at a time
+  // ... so many at a time. At 128 tokens 32 spill some 200 bytes and are the faster for 4-bit codes all the same (us, 32 / 16: 96 rows 28672 x 4096 31.8 / 33.8, mxfp4 35.3 /
+  // 37.7, 4096 x 14336 19.5 / 20.6), but not for 8-bit ones (44.2 / 42.8, 128 rows 4096 x 4096 13.7 / 13.5) and float weights (8 x 100 rows 2880 x 2880 45.5 / 43.5).
+  static constexpr int kCols = BT == 128 && kBits == 4 ? 32 : 16;
+  // A tile goes into registers rounded, whole, before it is stored. (Not float weights' 256 tokens: they spilled 156 bytes; 8 x 2048 rows 4096 x 4096 409 us, 388 so.)
+  static constexpr bool kHeld = !(QK == kFloat && BT == 256);
   static constexpr int kStages = kStep == 1 || (BT <= 64 && QK != kFloat) ? 6 : 4;
   static constexpr int kBarBytes = 1024;
   static constexpr int kBudget = 227 * 1024 - 4608;           // dynamic shared memory (the tile tables are static)
@@ -771,7 +775,7 @@ qmm_gemm_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
           for (int j = 0; j < kCols; j += 2) h[j / 2] = Half2Ops<__half>::pack(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
         }
       };
-      if (whole && !part_only && p.y_dtype != QMM_F32) {      // all of it into registers first: the next tile's MMAs need not wait for the stores
+      if (P::kHeld && whole && !part_only && p.y_dtype != QMM_F32) {      // all of it into registers first: the next tile's MMAs need not wait for the stores
         uint32_t h[P::kTeamCols / 2];
 #pragma unroll
         for (int i = 0; i < P::kTeamCols / kCols; ++i) {
@@ -957,7 +961,7 @@ constexpr int kLeastBoxes = 2;
 // (More of them of wide tiles write and read more partial sums than they save.)
 constexpr int most_shares(int bt) { return bt >= 256 ? 8 : 16; }
 // What handing partial tiles from worker to worker takes, in K blocks (us, shared out / a tile each: 64 rows 28672 x 4096, 224 tiles of 64
-// blocks on 148 workers, 29.9 / 27.0; 14336 x 4096, 112 tiles, 20.3 / 15.3; 11008 x 4096 18.4 / 14.7; 128 rows 28672 x 4096 35.7 / 33.0; 300 rows 14336 x 4096, 112 tiles on
+// blocks on 148 workers, 29.9 / 27.0 (before the producer's early start; 26.3 with it); 14336 x 4096, 112 tiles, 20.3 / 15.3; 11008 x 4096 18.4 / 14.7; 128 rows 28672 x 4096 35.7 / 33.0; 300 rows 14336 x 4096, 112 tiles on
 // 74 pairs, 51 / 43; mxfp4 64 rows 28800 x 2880 27..29 / 25.6).
 constexpr int kExchangeBlocks = 32;
 
