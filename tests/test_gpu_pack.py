@@ -1,5 +1,5 @@
 """A stored int4 Dense layer packed on the device against the same call on host arrays (the general way):
-every word and table entry the same, at the edges of the 64 x 256 tile, odd column counts, group sizes that
+every word and table entry the same, at the edges of the 128 x 256 tile, odd column counts, group sizes that
 allow 128, 64 and 32 codes per table entry, and tables that have to stay float32. Needs a B200."""
 
 import ctypes
@@ -19,6 +19,9 @@ DEV = "cuda:0"
     (288, 65, 3, torch.float16, torch.float16, False), (320, 63, 5, torch.float32, torch.float32, False),
     (1024, 130, 32, torch.bfloat16, None, False), (1024, 130, 32, torch.bfloat16, torch.uint8, True),
     (512, 7, 8, torch.float16, None, False), (4096, 200, 32, torch.bfloat16, torch.bfloat16, False),
+    (224, 127, 7, torch.bfloat16, torch.int8, False), (256, 128, 4, torch.bfloat16, None, False),        # a column less, a whole tile,
+    (288, 129, 9, torch.float32, torch.uint8, False), (512, 256, 4, torch.float16, torch.int8, False),   # one more (bytes of a row in fours and not), two tiles
+    (544, 257, 17, torch.bfloat16, None, False),
 ])
 def test_device_pack_is_the_host_pack(k, n, groups, sdt, zdt, constant):
     g = torch.Generator().manual_seed(k + n)
@@ -115,3 +118,63 @@ def test_what_a_layer_keeps_is_counted_and_given_back():
     _lib.release_scratch()
     assert _layer(packed, scale, None, 64)[0] == 0
     assert _lib.alloc_count() == before + 2
+
+
+def _dense(k, n, groups, sdt, zdt, seed=0):
+    g = torch.Generator().manual_seed(seed + k + n)
+    packed = torch.randint(-128, 128, (k, -(-n // 2)), generator=g, dtype=torch.int8)
+    if n % 2:
+        packed[:, -1] &= 15
+    scale = (torch.rand((groups, n), generator=g) * 0.02 + 0.01).to(sdt)
+    zero = None if zdt is None else torch.randint(0, 5, (groups, n), generator=g).to(zdt)
+    return packed.to(DEV), scale.to(DEV), None if zero is None else zero.to(DEV)
+
+
+@pytest.mark.parametrize("k,n", [(256, 128), (288, 129), (224, 127)])
+def test_the_digest_tells_layers_apart(k, n):
+    """Equal codes have an equal digest, however their bytes lie; one code more or less, or two that change places, another."""
+    packed, scale, _ = _dense(k, n, k // 32, torch.float32, None)
+    first = _layer(packed, scale, None, 32)
+    assert first[0] == 0 and _layer(packed.clone(), scale, None, 32)[4] == first[4]
+    shifted = torch.empty(packed.numel() + 1, dtype=torch.int8, device=DEV)[1:].view(packed.shape)      # starts on no word
+    shifted.copy_(packed)
+    assert _layer(shifted, scale, None, 32)[4] == first[4]
+    seen = {first[4]}
+    for row, col in ((0, 0), (k - 1, packed.shape[1] - 1), (k // 2, 1)):
+        other = packed.clone()
+        other[row, col] ^= 1
+        seen.add(_layer(other, scale, None, 32)[4])
+    other = packed.clone()
+    other[[3, 4]] = packed[[4, 3]]
+    seen.add(_layer(other, scale, None, 32)[4])
+    assert len(seen) == 5
+
+
+@pytest.mark.parametrize("k,n,groups,sdt,zdt", [(288, 129, 9, torch.bfloat16, torch.int8), (512, 256, 4, torch.float16, None), (1024, 63, 8, torch.float32, torch.float32)])
+def test_the_steps_in_a_captured_stream_are_the_layer(k, n, groups, sdt, zdt):
+    """Codes, facts and tables by their own entries, which a stream that is being captured takes, against all of it in one, which it does not."""
+    packed, scale, zero = _dense(k, n, groups, sdt, zdt)
+    group = next(s for s in (128, 64, 32) if k // groups % s == 0)
+    _, words, scales, biases, digest, facts = _layer(packed, scale, zero, group)
+    lib, types = _lib.lib(), (_lib.ELEM[sdt], 0 if zdt is None else _lib.ELEM[zdt])
+    tables = (scale.data_ptr(), None if zero is None else zero.data_ptr(), *types)
+    got = [torch.zeros_like(words), torch.zeros_like(scales), torch.zeros_like(biases)]
+    sums = torch.zeros(2, dtype=torch.int64, device=DEV)
+    stream, refused = torch.cuda.Stream(), []
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        st = stream.cuda_stream
+        sums.zero_()
+        _lib.check(lib.qmm_pack_dense_codes(packed.data_ptr(), got[0].data_ptr(), k, n, sums.data_ptr(), st))
+        _lib.check(lib.qmm_pack_dense_facts(*tables, groups, n, k, sums.data_ptr() + 8, st))
+        _lib.check(lib.qmm_pack_dense_tables(*tables, got[1].data_ptr(), got[2].data_ptr(), 0, groups, n, k, group, st))
+        d, f = ctypes.c_uint64(), ctypes.c_uint32()
+        refused.append(lib.qmm_pack_dense_layer(packed.data_ptr(), words.data_ptr(), *tables, scales.data_ptr(), biases.data_ptr(), 0, groups, n, k, group,
+                                                ctypes.byref(d), ctypes.byref(f), st))
+    assert refused == [7]
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got[0].view(torch.int32), words.view(torch.int32)) and torch.equal(got[1], scales) and torch.equal(got[2], biases)
+    assert sums[0].item() % (1 << 64) == digest and sums[1].item() == facts
