@@ -1,6 +1,8 @@
 """A program of products and gates in one native call, against the same program op by op: equal bit for bit where it is taken, and declined --
 not wrong -- where an argument is laid out another way or carries a gradient. Needs a B200."""
 
+import threading
+
 import pytest
 import torch
 
@@ -99,3 +101,56 @@ def test_what_is_not_plain_is_declined():
 def test_a_float32_gate_runs_op_by_op():
     args = arguments(4, 64, 96, torch.float32)
     assert both(program(4, 64, 96, torch.float32), args)[0] is None
+
+
+def test_on_a_stream_of_the_callers():
+    """The call enqueues on the current stream: it sees what that stream wrote before, and is replayed from a graph of it."""
+    text, args = program(6, 128, 256, torch.bfloat16), arguments(6, 128, 256, torch.bfloat16)
+    it = recognizer.Interpreter(text)
+    want = it.execute(args)[0].clone()
+    other = it.execute([args[0] * 2, *args[1:]])[0].clone()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    x = torch.zeros_like(args[0])
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(2_000_000)
+        x.copy_(args[0], non_blocking=True)
+        got = it.execute([x, *args[1:]])[0]
+        stream.synchronize()
+        assert torch.equal(got, want)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            y = it.execute([x, *args[1:]])[0]
+        x.copy_(args[0] * 2)
+        graph.replay()
+        stream.synchronize()
+    assert torch.equal(y, other)
+
+
+def test_two_threads_at_once():
+    """Each on a stream and with arguments of its own, through one interpreter."""
+    text = program(5, 128, 256, torch.float16)
+    it = recognizer.Interpreter(text)
+    sets = [arguments(5, 128, 256, torch.float16) for _ in range(2)]
+    sets[1][0] = sets[1][0].flip(0).contiguous()
+    want = []
+    for args in sets:                                     # (weights of the same values: one plan)
+        want.append(it.execute([args[0], *sets[0][1:]])[0].clone())
+    torch.cuda.synchronize()
+    wrong, start = [], threading.Barrier(2)
+
+    def run(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            start.wait()
+            for _ in range(200):
+                got = it.execute([sets[i][0], *sets[0][1:]])[0]
+                torch.cuda.current_stream().synchronize()
+                if not torch.equal(got, want[i]):
+                    wrong.append(i)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong and _lib.poll_status() == 0
