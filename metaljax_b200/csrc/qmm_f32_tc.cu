@@ -15,8 +15,8 @@
 // tile's rows, which adds them up in rank order a tile late. No scratch, no atomics, fixed order of summation.
 //
 // What bounds it: the few-rows kernel takes four rows a pass over the weight, and takes the codes apart for each of them (33 rows: nine times). Here a pass
-// takes up to 48. 33 rows of 4096 x 4096: 34.6 -> 24.0 us (13 K clocks a tile and cluster of eight: 8 K of them the codes, the MMAs' issue and the adding up, which
-// are latency at 18 warps, the rest the exchange; 14 such clusters fit the machine); 64 rows of 14336 x 4096 178 -> 83, 4096 x 14336 234 -> 114.
+// takes up to 48. 33 rows of 4096 x 4096: 34.6 -> 24.5 us (13 K clocks a tile and cluster of eight: 8 K of them the codes, the MMAs' issue and the adding up, which
+// are latency at 18 warps, the rest the exchange; 14 or 15 such clusters fit the machine); 64 rows of 14336 x 4096 178 -> 85, 4096 x 14336 234 -> 108.
 // Relative error against float64 (1e-8, 2-norm; N(0, 1) / one sign / outliers of 300; 33 rows), few-rows kernel -> here: 4-bit groups of 64 K 4096 8.5 / 5.4 / 9.5 -> 7.3 /
 // 4.2 / 8.3, K 14336 9.4 / 4.6 / 10.1 -> 8.6 / 4.3 / 9.4, of 128 K 4096 7.8 / 5.2 / 10.2 -> 6.8 / 4.2 / 9.4; 8-bit of 128 K 12288 13.4 / 12.5 / 20.4 -> 10.2 / 9.4 / 13.4; MXFP4
 // K 4096 9.3 / 9.3 / 11.1 -> 7.8 / 7.8 / 9.3, K 14336 10.1 / 10.1 / 11.5 -> 9.8 / 9.9 / 10.9. (Ranks added up one after another and two sums to a group of 128: K 14336 9.1 / 5.0
@@ -699,7 +699,8 @@ struct F32Plan {
 };
 
 // The plan of the least load, in clocks of the busiest cluster: rounds of tiles x (its K blocks, plus what a tile costs besides: the push, the sum), and the
-// conversion of the activations. What it picks against the best of all plans, us (float32 tables, the few-rows kernel last): 33 rows 4096 x 4096 24.0 / 24.0 / 34.8,
+// conversion of the activations. What it picked against the best of all plans when it was fitted, us (float32 tables, the few-rows kernel last; since then scaled pieces and the tree have
+// changed these by up to 6 %): 33 rows 4096 x 4096 24.0 / 24.0 / 34.8,
 // 64 rows 14336 x 4096 82.8 / 82.8 / 178, 4096 x 14336 114 / 114 / 234, 8-bit 64 rows 16384 x 1536 41 / 41 / 102, mxfp4 33 rows 5760 x 2880 26.2 / 26.2 / 47.3,
 // 12 rows 65536 x 512 21.0 / 20.9 / 35.4, 1024 x 14336 18.1 / 18.0 / 20.4, 10 rows 4096 x 4096 13.9 / 13.9 / 17.0, 20 rows 2048 x 1024 in groups of 32 8.0 / 8.0 / 8.2.
 F32Plan plan_of(const qmm_problem& p) {
