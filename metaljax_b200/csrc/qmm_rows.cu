@@ -158,7 +158,7 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
   rp.table_bytes = nweights * p.N * rp.groups * entry;
   // (a slice's entries start on the units that its own row of entries and a row of the table are multiples of)
   const int slice_bytes = sh.groups * entry, row_bytes_t = rp.groups * entry;
-  rp.table_unit = (row_bytes_t | slice_bytes) % 8 == 0 && row_bytes_t % slice_bytes == 0 ? 8 : (row_bytes_t | slice_bytes) % 4 == 0 ? 4 : 1;
+  rp.table_unit = (row_bytes_t | slice_bytes) % 8 == 0 && row_bytes_t % slice_bytes == 0 ? (slice_bytes % 16 == 0 ? 16 : 8) : (row_bytes_t | slice_bytes) % 4 == 0 ? 4 : 1;
   RowsPlan pl = plan_rows(live * ((per_seg + chunk - 1) / chunk), rp.N, slices, sh, p.group_sizes ? rp.segs : 0);
   if (!pl.warps) return fail(QMM_ERR_UNSUPPORTED, "few-rows kernel: no plan fits shared memory");
   const int tile_rows = kBlockRows * pl.blocks;

@@ -14,7 +14,8 @@
 // of 16 rows pass by: 16 x 128-byte boxes by TMA (128-byte swizzle) through a ring of its own per warp,
 // a few boxes ahead across tiles, so the HBM stream never waits for a barrier of the CTA. The warps'
 // partial sums of a tile meet in shared memory, one warp (in turn) adds them up in warp order; in
-// a cluster the CTAs' sums travel to the tile's leader (in turn) by st.async and are added in rank order.
+// a cluster the CTAs' sums travel to the tile's leader (in turn) by st.async and are added in rank order, when the leader's next tile comes: waiting for
+// them there and then held up a warp for each tile (8 rows of 4096 x 14336 15.9 -> 13.9 us).
 // No global scratch, no atomics, fixed order of summation.
 //
 // Arithmetic. The codes are never dequantized: a nibble pair under a magic exponent is an exact bf16 (128 + q) or f16 (16 + q) A
@@ -26,6 +27,13 @@
 // three columns (8 + 8 + 8 bits of bf16, or 11 + 11 + 11 of f16) that are added at the end; for f16 fragments of bf16 or float32 activations
 // each row of each slice is scaled to [2^14, 2^15) by its largest finite magnitude, and back in its partial sums. The K order inside a group is
 // free as long as codes and activations agree: lane t takes 16 consecutive codes (8 in groups of 32), in the pair order one LOP3 extracts.
+// Masks and shifts run at half the rate of the issue (16 lanes a clock), so that seven of them in eight codes of a lane are 14 clocks against the
+// MMAs' 8: as bf16 the upper nibble of a byte comes out of its place by a mask and an FMA (below), 10 clocks and 4 of another pipe
+// (8 rows of 128256 x 4096 64.6 -> 58.0 us, with the sums below and accumulators that start from a register quad).
+// The fragments of 16-bit activations are the loaded words, and the groups' sums MMAs of them against ones (element by element in float32 they
+// took 800 instructions a warp, some 2 us of every launch); the sums of bf16 numbers within 2^16 of one another are exact either way.
+// A launch releases its successor in its first instruction: the way from there to the next launch's CTAs bounds the rate of small products (2 rows of 4096 x 4096
+// 6.3 -> 5.5 us, 4 rows of 5632 x 2048 5.7 -> 4.8, 8 rows of 1024 x 1024 4.1 -> 3.3).
 //
 // Where the results are meant to be float32 -- float32 activations, and the 16-bit ones of unsorted gathers of more than 16 rows (EXACT) -- the
 // magic number, though it cancels, would cost them the bits in which it is larger than a code. There one exact subtraction a pair makes it q - 8 or q - 128, the accumulators start at nought, and the bias that goes with
@@ -40,7 +48,11 @@
 // (8-bit float MMAs would take the codes with a third of the instructions, but `mma.sync` on e4m3 is emulated here with
 // conversions to f16: 88 against 67 us for 8 rows of 128256 x 4096.)
 //
-// Measured (device time, weights from HBM; before: a kernel with the same fragments under the same kind of magic
+// Measured (device time, weights from HBM): int4 group 64 8 rows 28672 x 4096 18.1 us (3.7 TB/s), 128256 x 4096 58.0 (5.1 TB/s), 4096 x 14336 13.9, 16 rows 128256 x 4096 114,
+// 4096 x 4096 7.7; 8-bit 14336 x 4096 13.9. Tried: fragments in tensor memory (tcgen05.st / ld), rolled loops and two CTAs of 8 warps on an SM: 20.1 us at 28672 x 4096 when the above
+// was not there yet, 19.1 with it (16 rows a tile cost more instructions a code; the allocation delays the next launch's release); a last tile of 16 rows where a CTA's
+// share is not whole tiles: 4096 x 14336 14.8 instead of 13.9 (its code is fetched for it alone).
+// Where this kernel came from (before: a kernel with the same fragments under the same kind of magic
 // number that read its activations from shared memory for every tile and staged each tile's tables there behind barriers of the CTA; float32: the SIMT kernel), int4 group 64: 8 rows 28672 x 4096 27.1 -> 20.2 us (3.3 TB/s), 128256 x 4096
 // 99.5 -> 65.6 (4.5 TB/s), 4096 x 14336 26.8 -> 16.8, 16 rows 128256 x 4096 170 -> 128, 16 rows 4096 x 4096 12.2 -> 9.2; 8-bit 14336 x 4096 22.6
 // -> 15.5 (3.9 TB/s); float32 33 rows 4096 x 4096 323 -> 34.5. At the small end (2 rows 4096 x 4096 6.3 -> 7.1 us) it is the chain launch, activations,
@@ -112,11 +124,11 @@ struct Mma<__nv_bfloat16> {
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
-  // ... starting from c0, c1 (its two columns) in both rows
-  static __device__ __forceinline__ void first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0, float c1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
+  // ... starting from c (its two columns in both rows: the same two floats twice)
+  static __device__ __forceinline__ void first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
   }
 };
 template <>
@@ -126,10 +138,10 @@ struct Mma<__half> {
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
-  static __device__ __forceinline__ void first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0, float c1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%10,%11};"
+  static __device__ __forceinline__ void first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
   }
 };
 
@@ -180,6 +192,14 @@ __device__ __forceinline__ float2 unpack2(uint32_t u) {
 // What `got`, a value rounded to fewer bits, leaves of it (exact; nothing of an infinity).
 constexpr float kMaxFloat = 3.402823466e38f;
 __device__ __forceinline__ float left_of(float value, float got) { return fabsf(got) > kMaxFloat ? 0.0f : value - got; }
+
+// A pair of bf16: a * b + c. (Bits 0 to 7 of a bf16 whose others are nought are a whole number times 2^-133, subnormal or not: a nibble comes out
+// of either place by one mask and one of these, exactly and on the pipe that the masks leave idle.)
+__device__ __forceinline__ uint32_t fma_bf16(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
 
 // The codes under the magic exponent minus (magic + centre): exact.
 template <typename AT>
@@ -242,7 +262,8 @@ constexpr int kAbortAt = kXFreeAt + kMaxCluster * kExchangeSlots * 8;  // the ab
 constexpr int kStateAt = kAbortAt + 16;                                // [16 warps][2] where a warp's consumer is
 constexpr int kStateBytes = 32;
 constexpr int kAheadAt = kStateAt + kMaxWarps * 2 * kStateBytes;       // [16 warps] where its requests are: segment, chunk
-constexpr int kHeadBytes = (kAheadAt + kMaxWarps * 8 + 1023) / 1024 * 1024;
+constexpr int kLedAt = kAheadAt + kMaxWarps * 8;                                   // [kExchangeSlots] where a tile that this CTA leads goes: element of y, rows, tile
+constexpr int kHeadBytes = (kLedAt + kExchangeSlots * 16 + 1023) / 1024 * 1024;
 
 struct Place {            // one chunk of the walk: 8 NT columns against every row of one weight
   int64_t y0;             // element of y that its first column's first weight row goes to
@@ -259,9 +280,11 @@ constexpr int kMaxBlocks = 2;
 // that 8-byte copies and conflict-free 4-byte reads allow, with a word to spare for entries that do not start
 // on a word.
 constexpr int table_row_bytes(int groups, int tt) { return groups * entry_bytes(tt); }
-constexpr int table_pitch(int groups, int tt) { return table_row_bytes(groups, tt) == 4 ? 8 : table_row_bytes(groups, tt) == 8 ? 16 : table_row_bytes(groups, tt) + 8; }
-constexpr int table_stage_bytes(int blocks, int groups, int tt) { return kBlockRows * blocks * table_pitch(groups, tt) * (tt == kTabE8 ? 1 : 2); }
-constexpr int sums_bytes(int groups) { return groups * 32; }
+constexpr int table_pitch(int groups, int tt) { return table_row_bytes(groups, tt) == 4 ? 8 : table_row_bytes(groups, tt) == 8 ? 16 : table_row_bytes(groups, tt) + 16; }
+// (16 bytes at a pitch of 32: every four rows another 16 further on, for their reads to meet all banks)
+constexpr int table_at(int row, int groups, int tt) { return row * table_pitch(groups, tt) + (table_row_bytes(groups, tt) == 16 ? (row >> 2) * 16 : 0); }
+constexpr int table_stage_bytes(int blocks, int groups, int tt) { return table_at(kBlockRows * blocks, groups, tt) * (tt == kTabE8 ? 1 : 2); }
+constexpr int sums_bytes(int groups) { return groups * 64; }      // a pair of columns twice: what an accumulator of two rows starts at
 // Fragments of a second column group (the third piece of float32): they would not fit the registers.
 constexpr int more_x_bytes(int tokens) { return tokens == 8 ? 0 : kSliceK * 16; }
 
@@ -277,6 +300,8 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   constexpr uint32_t kMagic = QK == kAff8 ? 0x64006400u : std::is_same<AT, __half>::value ? 0x4C004C00u : 0x43004300u;
   constexpr float kMagicValue = QK == kAff8 ? 1024.0f : std::is_same<AT, __half>::value ? 16.0f : 128.0f;
   constexpr bool kCentred = EXACT && QK != kMx4;
+  // 4-bit codes as bf16: of each pair of nibbles the upper one by an FMA, as (128 + q) / 4 against four times the activation, or both as (q - 8) / 64.
+  constexpr bool kNibbles = QK == kAff4 && std::is_same<AT, __nv_bfloat16>::value, kQuarters = kNibbles && !kCentred;
   constexpr float kCentre = QK == kAff8 ? 128.0f : 8.0f;
   constexpr float kSumIs = kCentred ? 1.0f : -kMagicValue;   // the groups' sums of x are kept times this
   // Columns: piece i of the tokens is column group i, its column c token c. With 4 tokens two pieces share
@@ -294,16 +319,22 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   constexpr int kLane = kBlk / 4;                                     // consecutive codes of a lane in a block
   constexpr int kMmas = kBlk / 16;
   constexpr int kGroups = kSliceK / (32 * SPG);                       // groups of a slice
-  constexpr int kBlocksPerGroup = kBlocks / kGroups;
+  // The codes are worked through in chunks of 64 (eight fragment registers of a column group), four to a half of the slice.
+  constexpr int kChunkBlocks = 64 / kBlk;
+  constexpr int kHalfGroups = kGroups / 2;
+  constexpr int kChunkWords = 64 * kBits / 128;                       // words of a lane and row in a chunk
   constexpr bool kBiasMma = TT == kTabBf16 && !kCentred;              // the bias term is an MMA of its own (see load_x)
   constexpr int kBiasMmas = kGroups == 16 ? 3 : kGroups == 8 ? 2 : 1;
   constexpr int kEntry = entry_bytes(TT);
   constexpr int kRowBytes = table_row_bytes(kGroups, TT);             // a weight row's table entries in a slice
-  constexpr int kPitch = table_pitch(kGroups, TT);
-  constexpr int kTable = kTileRows * kPitch;                          // one table of a tile
+  constexpr int kTable = table_at(kTileRows, kGroups, TT);            // one table of a tile
+  constexpr int kEight = table_at(8, kGroups, TT);                    // its next eight rows
   constexpr int kSlot = kStage + table_stage_bytes(R, kGroups, TT);   // codes, scales, biases: a place of the ring
-  constexpr float kUnit = QK == kMx4 ? 16384.0f : 1.0f;               // (the E2M1 fragments are the values times 2^-14)
+  constexpr float kUnit = QK == kMx4 ? 16384.0f : kNibbles && kCentred ? 64.0f : 1.0f;               // (the E2M1 fragments are the values times 2^-14)
 
+  // The next launch may be made ready from here on: it touches nothing of this one's before its own wait, and the way from here to its CTAs' start is what
+  // bounds the rate of small products (see the head of the file).
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ uint8_t rows_smem_raw[];
   const uint32_t smem = (smem_u32(rows_smem_raw) + 1023) & ~1023u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -331,17 +362,15 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   int* ahead_at = reinterpret_cast<int*>(head + kAheadAt) + warp * 2;
 
   if (lane == 0) {
-    auto init = [](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n)); };
     if (warp == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&w_map)) : "memory");
-    for (int i = 0; i < p.ring; ++i) init(my_full + i * 8, 1 + 32);    // the boxes, and every lane's table entries
-    if (warp == 0) {
-      for (int i = 0; i < 4; ++i) {
-        init(smem + kRedFullAt + i * 8, warps);
-        init(smem + kRedEmptyAt + i * 8, 1);
-      }
-      for (int i = 0; i < kExchangeSlots; ++i) init(smem + kXFullAt + i * 8, 1);
-      for (int i = 0; i < kMaxCluster * kExchangeSlots; ++i) init(smem + kXFreeAt + i * 8, 1);
-      *abort_flag = 0;
+    *abort_flag = 0;
+  }
+  {
+    auto init = [](uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n)); };
+    if (lane < p.ring) init(my_full + lane * 8, 1 + 32);               // the boxes, and every lane's table entries
+    if (warp == 0) {                                                   // (a lane a barrier, of those that follow one another)
+      static_assert(kRedEmptyAt == kRedFullAt + 32 && kXFullAt == kRedEmptyAt + 32 && kXFreeAt == kXFullAt + kExchangeSlots * 8 && kExchangeSlots * (kMaxCluster + 1) <= 24, "");
+      if (lane < 8 + kExchangeSlots * (kMaxCluster + 1)) init(smem + kRedFullAt + lane * 8, lane < 4 ? warps : 1);
     }
     mbar_init_fence();
   }
@@ -404,7 +433,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     }
     const unsigned lo = cluster * share + min(cluster, more);
     left = static_cast<int>(share + (cluster < more ? 1u : 0u));
-    unsigned c = lo / p.tiles;
+    unsigned c = lo < static_cast<unsigned>(p.tiles) ? 0u : lo / p.tiles;
     tile0 = static_cast<int>(lo - c * p.tiles);
     if (grouped) {
       while (seg0 + 1 < p.segs && c >= static_cast<unsigned>(seg_chunks[seg0])) c -= seg_chunks[seg0++];
@@ -434,6 +463,10 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   }
   // (a slice past the end of K is given the row's first entries: what they multiply is zero)
   auto first_entry = [&](int slice) -> int { return slice * kGroups < p.groups ? slice * kGroups : 0; };
+  constexpr bool kBothTables = R == 2 || TT == kTabE8;
+  const int table_row = kTileRows == 32 ? lane : lane & 15, table_row_size = p.groups * kEntry;
+  const uint8_t* my_table = static_cast<const uint8_t*>(kBothTables || lane < 16 ? p.scales : p.biases);
+  const uint32_t my_tables = tables_at + table_at(table_row, kGroups, TT) + (kBothTables || lane < 16 ? 0 : kTable);
   auto request = [&]() {               // the whole warp; ahead_left > 0
     const uint32_t bar = my_full + ahead_slot * 8;
     const int slice = first_slice + ahead_sub;
@@ -446,18 +479,19 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     {
       // a lane's share of the tables: a weight row of one table, or (two blocks) of both. Entries past the end of a row are
       // some other entry of it: what they multiply is zero.
-      constexpr bool kBoth = R == 2 || TT == kTabE8;
-      const int row = kTileRows == 32 ? lane : lane & 15;
-      const int64_t at = (static_cast<int64_t>(min(ahead_row + row, ahead_last)) * p.groups + first_entry(slice)) * kEntry;
-      const uint32_t dst = tables_at + ahead_slot * (kSlot - kStage) + row * kPitch;
-      auto copy = [&](const void* table, uint32_t to) {
-        const uint8_t* src = static_cast<const uint8_t*>(table) + at;
-        if (p.table_unit == 8 && kRowBytes >= 8) {
+      const int64_t at = static_cast<int64_t>(min(ahead_row + table_row, ahead_last)) * table_row_size + first_entry(slice) * kEntry;
+      const uint32_t dst = my_tables + ahead_slot * (kSlot - kStage);
+      auto copy = [&](const uint8_t* table, uint32_t to) {
+        const uint8_t* src = table + at;
+        if (p.table_unit == 16 && kRowBytes >= 16) {
+#pragma unroll
+          for (int i = 0; i < kRowBytes; i += 16) cp_async16(to + i, src + i);
+        } else if (p.table_unit >= 8 && kRowBytes >= 8) {
 #pragma unroll
           for (int i = 0; i < kRowBytes; i += 8) cp_async8(to + i, src + i);
         } else if (p.table_unit >= 4) {
 #pragma unroll
-          for (int i = 0; i < kRowBytes; i += 4) cp_async4(to + i, slice * kGroups * kEntry + i < p.groups * kEntry ? src + i : src);
+          for (int i = 0; i < kRowBytes; i += 4) cp_async4(to + i, slice * kGroups * kEntry + i < table_row_size ? src + i : src);
         } else {                         // from the word the first entry lies in; nothing past the table's end is read
           const int skew = static_cast<int>(at & 3);
 #pragma unroll
@@ -467,11 +501,11 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
           }
         }
       };
-      if (kBoth) {
-        if (kTileRows == 32 || lane < 16) copy(p.scales, dst);
-        if (TT != kTabE8) copy(p.biases, dst + kTable);
+      if (kBothTables) {
+        if (kTileRows == 32 || lane < 16) copy(static_cast<const uint8_t*>(p.scales), dst);
+        if (TT != kTabE8) copy(static_cast<const uint8_t*>(p.biases), dst + kTable);
       } else {
-        copy(lane < 16 ? p.scales : p.biases, dst + (lane < 16 ? 0 : kTable));
+        copy(my_table, dst);
       }
       cp_async_arrive(bar);
     }
@@ -515,13 +549,12 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     __syncwarp();
   };
   if (left > 0) set_place(0, seg0, chunk0);
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (!grouped && !p.lhs_idx) asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();                                 // the shared barriers are initialised
   if (csize > 1) {                                 // ... in every CTA of the cluster
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
+  if (!grouped && !p.lhs_idx) asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // ---- activations: this warp's slice as MMA fragments ----
   static_assert(NT <= 2, "one column group in registers, one in shared memory");
@@ -561,149 +594,200 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     }
     const XT* src = reinterpret_cast<const XT*>(p.x) + base + (live ? xr : 0) * p.K;
     const int k0 = slice * kSliceK + t * kLane;
-    // The lane's c-th eight elements. Where they are looked at twice (scaled) and are the ones that end up in xf,
-    // they wait there as they are: one trip to memory instead of two (8 rows, mxfp4 5760 x 2880: see below).
-    constexpr bool kStays = kScaled && sizeof(XT) == 2;
-    auto element_of = [&](int c) -> int { return k0 + (c / (kLane / 8)) * kBlk + (c % (kLane / 8)) * 8; };
-    if constexpr (kStays) {
-#pragma unroll
-      for (int c = 0; c < kSliceK / 32; ++c) {
-        const int k = element_of(c);
-        const uint4 v = live && k < p.K ? __ldg(reinterpret_cast<const uint4*>(src + k)) : make_uint4(0u, 0u, 0u, 0u);
-        xf[c * 4] = v.x; xf[c * 4 + 1] = v.y; xf[c * 4 + 2] = v.z; xf[c * 4 + 3] = v.w;
+    auto element_of = [&](int c) -> int { return k0 + (c / (kLane / 8)) * kBlk + (c % (kLane / 8)) * 8; };      // the lane's c-th eight elements
+    auto arranged = [](uint32_t (&u)[4]) {         // in the order in which codes come apart: (0,4) (1,5) (2,6) (3,7) of 4 bits, (0,1) (2,3) of 8
+      if constexpr (QK != kAff8) {
+        const uint32_t v[4] = {u[0], u[1], u[2], u[3]};
+        u[0] = __byte_perm(v[0], v[2], 0x5410); u[1] = __byte_perm(v[0], v[2], 0x7632);
+        u[2] = __byte_perm(v[1], v[3], 0x5410); u[3] = __byte_perm(v[1], v[3], 0x7632);
       }
-    }
-    auto load8 = [&](int c, float (&f)[8]) {
-      const int k = element_of(c);
-      if (kStays) {
+    };
+    constexpr int kPer = kSliceK / 32 / kGroups;   // eights per group
+    if constexpr (kPieces == 1) {
+      // 16-bit activations: fragments as they are (or scaled), and the groups' sums by MMAs of theirs against ones, which leave them where
+      // the tiles' accumulators want them. (Element by element in float32 this took 800 instructions a warp, 2 us of every launch.)
+      // (all of the lane's elements are asked for at once: a trip to L2 is a third of what this takes)
+      constexpr int kPart = kSliceK / 32;
+      uint4 v[kPart];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 w = unpack2<XT>(xf[c * 4 + i]);
-          f[2 * i] = w.x; f[2 * i + 1] = w.y;
+      for (int c = 0; c < kPart; ++c) {
+        const int k = element_of(c);
+        v[c] = live && k < p.K ? __ldg(reinterpret_cast<const uint4*>(src + k)) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      float up = 1.0f;
+      if constexpr (kScaled) {
+        // largest finite magnitude of the row's slice (of a pair of bf16 patterns, as whole numbers)
+        auto over_row = [&](uint32_t big) -> uint32_t {
+          big = max(big & 0xffffu, big >> 16);
+          big = max(big, __shfl_xor_sync(0xffffffffu, big, 1));
+          return max(big, __shfl_xor_sync(0xffffffffu, big, 2));
+        };
+        auto largest = [&](auto finite) -> uint32_t {
+          uint32_t pair = 0u;
+#pragma unroll
+          for (int c = 0; c < kPart; ++c) {
+            const uint32_t u[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint32_t m = u[j] & 0x7fff7fffu;
+              if (decltype(finite)::value) m = ((m & 0xffffu) >= 0x7f80u ? 0u : m & 0xffffu) | (m >= 0x7f800000u ? 0u : m & 0xffff0000u);
+              pair = __vmaxu2(pair, m);
+            }
+          }
+          return over_row(pair);
+        };
+        uint32_t big = largest(std::false_type());
+        if (__any_sync(0xffffffffu, big >= 0x7f80u)) big = largest(std::true_type());      // an infinity or a NaN somewhere
+        // largest magnitude to [2^14, 2^15); a warp's later slices no finer than its earlier ones, whose sums are brought to their units
+        const uint32_t e = max(big >> 7, sub > 0 ? least_e : 15u);
+        least_e = e;
+        up = __uint_as_float((268u - e) << 23);
+        const float down = __uint_as_float((e - 14u) << 23);
+        back[0] = __shfl_sync(0xffffffffu, down, 8 * t);
+        back[1] = __shfl_sync(0xffffffffu, down, 8 * t + 4);
+      }
+      float total[2];
+#pragma unroll
+      for (int c = 0; c < kPart; ++c) {
+        uint32_t u[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+        if constexpr (kScaled) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = unpack2<XT>(u[j]);
+            u[j] = pack2<AT>(f.x * up, f.y * up);
+          }
         }
-      } else if (live && k < p.K) {
-        if constexpr (sizeof(XT) == 4) {
+        arranged(u);
+        if constexpr (kQuarters) {               // (what goes with the codes that are (128 + q) / 4)
+          u[1] = fma_bf16(u[1], 0x40804080u, 0x80008000u);
+          u[3] = fma_bf16(u[3], 0x40804080u, 0x80008000u);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xf[c * 4 + j] = u[j];
+        if constexpr (QK != kMx4) {
+          constexpr uint32_t kOnes = std::is_same<AT, __half>::value ? 0x3C003C00u : 0x3F803F80u, kUpper = kQuarters ? 0x3E803E80u : kOnes;
+          const uint32_t ones[4] = {kOnes, kOnes, kUpper, kUpper};
+          const float nought[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          float lower[4], upper[4];                // (added up in registers, rounded: the tensor core cuts off)
+          Mma<AT>::first(lower, ones, u[0], u[1], nought);
+          Mma<AT>::first(upper, ones, u[2], u[3], nought);
+          total[0] = (c % kPer == 0 ? 0.0f : total[0]) + (lower[0] + upper[0]);
+          total[1] = (c % kPer == 0 ? 0.0f : total[1]) + (lower[1] + upper[1]);
+          if (c % kPer == kPer - 1) {            // (kept as -C sum x where the group's accumulators start there)
+            const int group = c / kPer;
+            const float a = kSumIs * total[0], b = kSumIs * total[1];
+            if (g == (group & 7)) sts128(sums_at + group * 64 + t * 16, a, b, a, b);
+          }
+        }
+      }
+    } else {
+      auto load8 = [&](int c, float (&f)[8]) {
+        const int k = element_of(c);
+        if (live && k < p.K) {
           const float4 a = __ldg(reinterpret_cast<const float4*>(src + k)), b = __ldg(reinterpret_cast<const float4*>(src + k) + 1);
           f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
         } else {
-          const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + k));
-          const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 w = unpack2<XT>(u[i]);
-            f[2 * i] = w.x; f[2 * i + 1] = w.y;
-          }
+          for (int i = 0; i < 8; ++i) f[i] = 0.0f;
         }
-      } else {
+      };
+      float up = 1.0f;
+      [[maybe_unused]] bool infinite = false;      // some row's slice has an infinity in it
+      if constexpr (kScaled) {
+        auto largest = [&](auto finite) -> float {
+          float big = 0.0f;                                            // (a NaN is no larger than anything, and one in any unit)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = 0.0f;
+          for (int c = 0; c < kSliceK / 32; ++c) {
+            float f[8];
+            load8(c, f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) big = fmaxf(big, !decltype(finite)::value || fabsf(f[i]) <= kMaxFloat ? fabsf(f[i]) : 0.0f);
+          }
+          big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
+          return fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
+        };
+        float big = largest(std::false_type());
+        if (__any_sync(0xffffffffu, big > kMaxFloat)) {
+          infinite = true;
+          big = largest(std::true_type());
+        }
+        // largest magnitude to [2^14, 2^15); a warp's later slices no finer than its earlier ones, whose sums are brought to their units
+        const uint32_t e = max(__float_as_uint(big) >> 23, sub > 0 ? least_e : 15u);
+        least_e = e;
+        up = __uint_as_float((268u - e) << 23);
+        const float down = __uint_as_float((e - 14u) << 23);
+        back[0] = __shfl_sync(0xffffffffu, down, 8 * t);
+        back[1] = __shfl_sync(0xffffffffu, down, 8 * t + 4);
       }
-    };
-    float up = 1.0f;
-    [[maybe_unused]] bool infinite = false;      // some row's slice has an infinity in it
-    if constexpr (kScaled) {
-      auto largest = [&](auto finite) -> float {
-        float big = 0.0f;                                            // (a NaN is no larger than anything, and one in any unit)
+      // CAREFUL: the second piece of an infinity is nought (it would be a NaN), for its results to be what a sum of products makes of them. (A
+      // comparison for every element costs a scaled row more than what its largest magnitude already tells: 33 rows of float32 against MXFP4,
+      // 4096 x 4096, 98 us with it everywhere, 74 so; 69 without.)
+      auto fragments = [&](auto careful) {
+        float sum = 0.0f;
 #pragma unroll
         for (int c = 0; c < kSliceK / 32; ++c) {
           float f[8];
           load8(c, f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) big = fmaxf(big, !decltype(finite)::value || fabsf(f[i]) <= kMaxFloat ? fabsf(f[i]) : 0.0f);
-        }
-        big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 1));
-        return fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 2));
-      };
-      float big = largest(std::false_type());
-      if (__any_sync(0xffffffffu, big > kMaxFloat)) {
-        infinite = true;
-        big = largest(std::true_type());
-      }
-      // largest magnitude to [2^14, 2^15); a warp's later slices no finer than its earlier ones, whose sums are brought to their units
-      const uint32_t e = max(__float_as_uint(big) >> 23, sub > 0 ? least_e : 15u);
-      least_e = e;
-      up = __uint_as_float((268u - e) << 23);
-      const float down = __uint_as_float((e - 14u) << 23);
-      back[0] = __shfl_sync(0xffffffffu, down, 8 * t);
-      back[1] = __shfl_sync(0xffffffffu, down, 8 * t + 4);
-    }
-    [[maybe_unused]] float group_sum[kGroups];
-    // CAREFUL: the second piece of an infinity is nought (it would be a NaN), for its results to be what a sum of products makes of them. (A
-    // comparison for every element costs a scaled row more than what its largest magnitude already tells: 33 rows of float32 against MXFP4,
-    // 4096 x 4096, 98 us with it everywhere, 74 so; 69 without.)
-    auto fragments = [&](auto careful) {
-      float sum = 0.0f;
-#pragma unroll
-      for (int c = 0; c < kSliceK / 32; ++c) {
-        float f[8];
-        load8(c, f);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          if constexpr (kScaled) f[i] *= up;
-          sum += f[i];
-        }
-        if constexpr (QK != kMx4) {
-          constexpr int kPer = kSliceK / 32 / kGroups;                 // eights per group
-          if (c % kPer == kPer - 1) {
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            // (kept as -C sum x where the group's accumulators start there)
-            if (t == 0) sts32(sums_at + ((c / kPer) * 8 + g) * 4, kSumIs * sum);
-            if constexpr (kBiasMma) group_sum[c / kPer] = kHalf && g >= 4 ? 0.0f : sum;
-            sum = 0.0f;
+          for (int i = 0; i < 8; ++i) {
+            if constexpr (kScaled) f[i] *= up;
+            sum += f[i];
           }
-        }
+          if constexpr (QK != kMx4) {
+            if (c % kPer == kPer - 1) {
+              sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+              sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+              // (kept as -C sum x where the group's accumulators start there)
+              if (t < 2) sts32(sums_at + (c / kPer) * 64 + (g >> 1) * 16 + (g & 1) * 4 + t * 8, kSumIs * sum);
+              sum = 0.0f;
+            }
+          }
+          [[maybe_unused]] uint32_t frag[4];
 #pragma unroll
-        for (int i = 0; i < kPieces; ++i) {
-          const int h = kHalf ? i / 2 : i;
-          const bool here = !kHalf || (g >> 2) == (i & 1);             // (4 tokens: which of the two pieces this lane's column is)
-          uint32_t u[4];
+          for (int i = 0; i < kPieces; ++i) {
+            const bool here = !kHalf || (g >> 2) == (i & 1);             // (4 tokens: which of the two pieces this lane's column is)
+            uint32_t u[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) u[j] = pack2<AT>(f[2 * j], f[2 * j + 1]);
-          if (i + 1 < kPieces) {                                       // what this piece leaves over (exact)
+            for (int j = 0; j < 4; ++j) u[j] = pack2<AT>(f[2 * j], f[2 * j + 1]);
+            if (i + 1 < kPieces) {                                       // what this piece leaves over (exact)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 got = unpack2<AT>(u[j]);
-              if (decltype(careful)::value && i == 0) {
-                f[2 * j] = left_of(f[2 * j], got.x); f[2 * j + 1] = left_of(f[2 * j + 1], got.y);
-              } else {
-                f[2 * j] -= got.x; f[2 * j + 1] -= got.y;
+              for (int j = 0; j < 4; ++j) {
+                const float2 got = unpack2<AT>(u[j]);
+                if (decltype(careful)::value && i == 0) {
+                  f[2 * j] = left_of(f[2 * j], got.x); f[2 * j + 1] = left_of(f[2 * j + 1], got.y);
+                } else {
+                  f[2 * j] -= got.x; f[2 * j + 1] -= got.y;
+                }
+              }
+            }
+            arranged(u);
+            if (kHalf) {                                                 // (the half of the last group that no piece is left for: nought)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) frag[j] = here ? u[j] : i % 2 ? frag[j] : 0u;
+              if (i == 1) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) xf[c * 4 + j] = frag[j];
+              } else if (i + 1 == kPieces) {
+                sts128(more_x_at + c * 512, __uint_as_float(frag[0]), __uint_as_float(frag[1]), __uint_as_float(frag[2]), __uint_as_float(frag[3]));
               }
             }
           }
-          if constexpr (QK != kAff8) {                                 // 4-bit codes: (0,4) (1,5) (2,6) (3,7); 8-bit ones in order, (0,1) (2,3)
-            const uint32_t v[4] = {u[0], u[1], u[2], u[3]};
-            u[0] = __byte_perm(v[0], v[2], 0x5410); u[1] = __byte_perm(v[0], v[2], 0x7632);
-            u[2] = __byte_perm(v[1], v[3], 0x5410); u[3] = __byte_perm(v[1], v[3], 0x7632);
-          }
-          if (h == 0) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (!kHalf || i % 2 == 0 || here) xf[c * 4 + j] = u[j];
-          } else {
-            const bool empty = kHalf && !here;                         // (the half of the last group that no piece is left for)
-            sts128(more_x_at + c * 512, __uint_as_float(empty ? 0u : u[0]), __uint_as_float(empty ? 0u : u[1]), __uint_as_float(empty ? 0u : u[2]),
-                   __uint_as_float(empty ? 0u : u[3]));
-          }
         }
+      };
+      if constexpr (!kScaled) {
+        fragments(std::true_type());
+      } else {
+        if (infinite) fragments(std::true_type());
+        else fragments(std::false_type());
       }
-    };
-    if constexpr (kPieces == 1 || !kScaled) {
-      fragments(std::bool_constant<(kPieces > 1)>());
-    } else {
-      if (infinite) fragments(std::true_type());
-      else fragments(std::false_type());
     }
+    __syncwarp();                                  // the sums are there
     if constexpr (kBiasMma) {
       // K slots of the bias MMAs: 16 groups -- one MMA per piece of the sums (lane t: groups 2t, 2t + 1, 2t + 8, 2t + 9);
       // 8 groups -- (hi | mid) and (lo | 0) with lane t's groups 2t, 2t + 1; 4 groups -- lanes t < 2 (hi | mid), t >= 2 (lo | 0)
       // with groups 2 (t & 1), 2 (t & 1) + 1
-      auto pick = [&](int first) -> float {        // group_sum[first + 2 t], without indexing registers
-        float v = group_sum[first];
-#pragma unroll
-        for (int i = 1; i < (kGroups == 4 ? 2 : 4); ++i)
-          if ((kGroups == 4 ? t & 1 : t) == i) v = group_sum[first + 2 * i];
-        return v;
+      auto pick = [&](int first) -> float {        // sum of x of column g in group first + 2 t
+        return __uint_as_float(lds32<0>(sums_at + (first + 2 * (kGroups == 4 ? t & 1 : t)) * 64 + (g >> 1) * 16 + (g & 1) * 4)) * (1.0f / kSumIs);
       };
       using B16 = __nv_bfloat16;
       auto split = [&](float a, float b, uint32_t (&piece)[3]) {
@@ -737,13 +821,44 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
                            (QK == kAff8 ? (SPG == 1 ? ((((t >> 1) ^ rho) << 4) + (t & 1) * 8) : ((t ^ rho) << 4))
                                         : (SPG == 1 ? ((rho << 4) + t * 4) : ((((t >> 1) ^ rho) << 4) + (t & 1) * 8)));
   uint32_t nib_mask = std::is_same<AT, __half>::value ? 0x03C003C0u : 0x000F000Fu, magic = kMagic;
+  [[maybe_unused]] uint32_t upper_mask = 0x00F000F0u, times = 0x7F007F00u;       // (2^127)
   asm volatile("" : "+r"(nib_mask), "+r"(magic));                      // constants in registers: one LOP3 per use
-  const uint32_t tthread = tables_at + rho * kPitch, scol = sums_at + 8 * t;
+  const uint32_t tthread = tables_at + table_at(rho, kGroups, TT), scol = sums_at + 16 * t;
   int turn = 0, which = 0, tile = tile0, sub = 0, count = 0;
   uint32_t slot = 0, slot_phase = 0, buf = 0, buf_phase = 0;
   // the tile that is to be added up next
   int done_tile = 0, done_which = 0, lap = 0, leader = 0;
   uint32_t done_buf = 0, done_phase = 0;
+  auto store_tile = [&](const float (&v)[R][4], int64_t y0, int rows_left, int at_tile) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int col = 2 * t + (i & 1), n = at_tile * kTileRows + r * kBlockRows + rho + (i >> 1) * 8;
+        if (col < rows_left && col < T && n < p.N) store_y(p.y, p.y_dtype, y0 + static_cast<int64_t>(col) * p.N + n, v[r][i]);
+      }
+  };
+  // A tile that this CTA leads: the CTAs' sums in rank order.
+  auto finish = [&](int led) -> bool {
+    const int xs = led % kExchangeSlots;
+    if (!mbar_wait_cluster(smem + kXFullAt + xs * 8, static_cast<uint32_t>(led / kExchangeSlots) & 1u, abort_at, 15)) return false;
+    __syncwarp();
+    const uint32_t xslot = xbuf_at + xs * csize * (R * 512) + lane * 16;
+    float v[R][4];
+#pragma unroll
+    for (int h = 0; h < R; ++h) v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0.0f;
+    for (int r = 0; r < csize; ++r)
+#pragma unroll
+      for (int h = 0; h < R; ++h) {
+        const float4 f = ldsf128<0>(xslot + (r * R + h) * 512);
+        v[h][0] += f.x; v[h][1] += f.y; v[h][2] += f.z; v[h][3] += f.w;
+      }
+    const uint4 to = lds128<kLedAt>(smem + xs * 16);
+    __syncwarp();
+    if (lane < csize && lane != rank) remote_arrive(remote(smem + kXFreeAt + (rank * kExchangeSlots + xs) * 8, lane));
+    store_tile(v, static_cast<int64_t>(static_cast<uint64_t>(to.y) << 32 | to.x), static_cast<int>(to.z), static_cast<int>(to.w));
+    return true;
+  };
   auto add_up = [&]() -> bool {
     // ---- the warps' shares, in warp order ----
     const uint32_t shares = red_at + done_buf * warps * (R * 512) + lane * 16;
@@ -761,49 +876,30 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
       }
     __syncwarp();
     if (lane == 0) mbar_arrive(smem + kRedEmptyAt + done_buf * 8);
-    bool mine = true;
-    if (csize > 1) {
-      // ---- the CTAs' sums meet at the tile's leader (in turn; `lap` counts its tiles), in rank order ----
-      const int xs = lap % kExchangeSlots;
-      const uint32_t xphase = static_cast<uint32_t>(lap / kExchangeSlots) & 1u;
-      const uint32_t xslot = xbuf_at + xs * csize * (R * 512) + lane * 16;
-      mine = leader == rank;
-      if (!mine) {
-        if (!mbar_wait_cluster(smem + kXFreeAt + (leader * kExchangeSlots + xs) * 8, xphase ^ 1u, abort_at, 14)) return false;
-        __syncwarp();
-        const uint32_t bar = remote(smem + kXFullAt + xs * 8, leader), to = remote(xslot + rank * (R * 512), leader);
-#pragma unroll
-        for (int h = 0; h < R; ++h) st_async4(to + h * 512, bar, v[h]);
-      } else {
-        if (lane == 0) mbar_expect_tx(smem + kXFullAt + xs * 8, (csize - 1) * R * 512);
-        if (!mbar_wait_cluster(smem + kXFullAt + xs * 8, xphase, abort_at, 15)) return false;
-        __syncwarp();
-#pragma unroll
-        for (int h = 0; h < R; ++h) {
-          sts128(xslot + rank * (R * 512) + h * 512, v[h][0], v[h][1], v[h][2], v[h][3]);
-          v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0.0f;
-        }
-        for (int r = 0; r < csize; ++r)
-#pragma unroll
-          for (int h = 0; h < R; ++h) {
-            const float4 f = ldsf128<0>(xslot + (r * R + h) * 512);
-            v[h][0] += f.x; v[h][1] += f.y; v[h][2] += f.z; v[h][3] += f.w;
-          }
-        __syncwarp();
-        if (lane < csize && lane != rank) remote_arrive(remote(smem + kXFreeAt + (rank * kExchangeSlots + xs) * 8, lane));
-      }
+    const int rows_left = place[done_which].rows_left;
+    const int64_t y0 = place[done_which].y0;
+    if (csize == 1) {
+      store_tile(v, y0, rows_left, done_tile);
+      return true;
     }
-    if (mine) {
-      const int rows_left = place[done_which].rows_left;
-      const int64_t y0 = place[done_which].y0;
+    // ---- the CTAs' sums meet at the tile's leader (in turn; `lap` counts its tiles), who adds them up when its next tile comes: by then they are there ----
+    const int xs = lap % kExchangeSlots;
+    const uint32_t xslot = xbuf_at + xs * csize * (R * 512) + lane * 16;
+    if (leader != rank) {
+      if (!mbar_wait_cluster(smem + kXFreeAt + (leader * kExchangeSlots + xs) * 8, (static_cast<uint32_t>(lap / kExchangeSlots) & 1u) ^ 1u, abort_at, 14)) return false;
+      __syncwarp();
+      const uint32_t bar = remote(smem + kXFullAt + xs * 8, leader), to = remote(xslot + rank * (R * 512), leader);
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int col = 2 * t + (i & 1), n = done_tile * kTileRows + r * kBlockRows + rho + (i >> 1) * 8;
-          if (col < rows_left && col < T && n < p.N) store_y(p.y, p.y_dtype, y0 + static_cast<int64_t>(col) * p.N + n, v[r][i]);
-        }
+      for (int h = 0; h < R; ++h) st_async4(to + h * 512, bar, v[h]);
+      return true;
     }
+    if (lap > 0 && !finish(lap - 1)) return false;
+#pragma unroll
+    for (int h = 0; h < R; ++h) sts128(xslot + rank * (R * 512) + h * 512, v[h][0], v[h][1], v[h][2], v[h][3]);
+    if (lane == 0)
+      sts128(smem + kLedAt + xs * 16, __uint_as_float(static_cast<uint32_t>(y0)), __uint_as_float(static_cast<uint32_t>(y0 >> 32)), __int_as_float(rows_left), __int_as_float(done_tile));
+    __syncwarp();
+    if (lane == 0) mbar_expect_tx(smem + kXFullAt + xs * 8, (csize - 1) * R * 512);      // (what finishes the tile sees the above as well)
     return true;
   };
   bool ok = true, stale = true;
@@ -859,7 +955,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
           word = next;
         }
       };
-      const uint32_t at = tables_at + slot * (kSlot - kStage) + row * kPitch;
+      const uint32_t at = tables_at + slot * (kSlot - kStage) + table_at(row, kGroups, TT);
       if (R == 2 || TT == kTabE8) {
         if (kTileRows == 32 || lane < 16) straighten(at);
         if (TT != kTabE8) straighten(at + kTable);
@@ -870,114 +966,168 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     }
     if constexpr (kBiasMma) {
       static_for<R>([&](auto rc) {
-        constexpr int r = decltype(rc)::value, kAt = kTable + r * kBlockRows * kPitch;
+        constexpr int r = decltype(rc)::value, kAt = kTable + r * 2 * kEight;
         const uint32_t at = trow + (kGroups == 4 ? t & 1 : t) * 4;
-        const uint32_t b0 = lds32<kAt>(at), b1 = lds32<kAt + 8 * kPitch>(at);
+        const uint32_t b0 = lds32<kAt>(at), b1 = lds32<kAt + kEight>(at);
         uint32_t a[4] = {b0, b1, b0, b1};
-        if constexpr (kGroups == 16) { a[2] = lds32<kAt + 16>(at); a[3] = lds32<kAt + 8 * kPitch + 16>(at); }
+        if constexpr (kGroups == 16) { a[2] = lds32<kAt + 16>(at); a[3] = lds32<kAt + kEight + 16>(at); }
 #pragma unroll
         for (int i = 0; i < kBiasMmas; ++i) Mma<__nv_bfloat16>::run(yb[r], a, bf[i][0], bf[i][1]);
       });
     }
-    static_for<kGroups>([&](auto gc) {
-      constexpr int gi = decltype(gc)::value;
-      float acc[R][NT][4];
-      float start[2] = {0.0f, 0.0f};               // kSumIs * sum x of the group
-      if constexpr (QK != kMx4) {
-        const uint2 sr = lds64<gi * 32>(scol);
-        start[0] = __uint_as_float(sr.x); start[1] = __uint_as_float(sr.y);
-      }
-      static_for<kBlocksPerGroup>([&](auto bc) {
-        constexpr int jj = decltype(bc)::value, j = gi * kBlocksPerGroup + jj;      // block of the slice
+    // Chunks of 64 codes; a chunk's codes are requested while the one before it is worked on.
+    constexpr int kChunks = kSliceK / 64;
+    uint32_t cw[2][R][2][kChunkWords];
+    auto fetch = [&](auto qc, auto& c) {
+      static_for<kChunkBlocks>([&](auto bc) {
+        constexpr int jj = decltype(bc)::value, j = decltype(qc)::value * kChunkBlocks + jj;  // block of the slice
         constexpr int kLaneWords = kLane * kBits / 32;
-        constexpr int kPerBox = kBoxBytes * 8 / kBits / kBlk, kChunk = kBlk * kBits / 8;      // blocks of a box, bytes of a row in a block
-        const uint32_t a0 = (wrow ^ ((j % kPerBox) * kChunk)) + (j / kPerBox) * kBoxSmem;
-        static_for<R>([&](auto rc) {
-          constexpr int r = decltype(rc)::value, kRow = r * kBlockRows * kBoxBytes;
-          uint32_t u[2][kLaneWords];               // words of this lane, rows rho and rho + 8 of block r
-          [[maybe_unused]] uint4 more = make_uint4(0u, 0u, 0u, 0u);
+        constexpr int kPerBox = kBoxBytes * 8 / kBits / kBlk, kBlkBytes = kBlk * kBits / 8;   // blocks of a box, bytes of a row in a block
+        constexpr int kBoxAt = (j / kPerBox) * kBoxSmem;
+        const uint32_t a0 = wrow ^ ((j % kPerBox) * kBlkBytes);
+        static_for<2 * R>([&](auto rc) {
+          constexpr int r = decltype(rc)::value / 2, i = decltype(rc)::value % 2, kRow = kBoxAt + (r * kBlockRows + i * 8) * kBoxBytes;      // rows rho and rho + 8 of block r
+          uint32_t* u = &c[r][i][jj * kLaneWords];
           if constexpr (kLaneWords == 1) {
-            u[0][0] = lds32<kRow>(a0);
-            u[1][0] = lds32<kRow + 8 * kBoxBytes>(a0);
+            u[0] = lds32<kRow>(a0);
           } else if constexpr (kLaneWords == 2) {
-            const uint2 v0 = lds64<kRow>(a0), v1 = lds64<kRow + 8 * kBoxBytes>(a0);
-            u[0][0] = v0.x; u[0][1] = v0.y; u[1][0] = v1.x; u[1][1] = v1.y;
+            const uint2 v = lds64<kRow>(a0);
+            u[0] = v.x; u[1] = v.y;
           } else {
-            const uint4 v0 = lds128<kRow>(a0), v1 = lds128<kRow + 8 * kBoxBytes>(a0);
-            u[0][0] = v0.x; u[0][1] = v0.y; u[0][2] = v0.z; u[0][3] = v0.w;
-            u[1][0] = v1.x; u[1][1] = v1.y; u[1][2] = v1.z; u[1][3] = v1.w;
+            const uint4 v = lds128<kRow>(a0);
+            u[0] = v.x; u[1] = v.y; u[2] = v.z; u[3] = v.w;
           }
-          static_for<kMmas>([&](auto mc) {
-            constexpr int mi = decltype(mc)::value, x0 = (j * kMmas + mi) * 2;
-            if constexpr (NT > 1 && mi % 2 == 0) more = lds128<(x0 / 4) * 512>(more_x_at);
+        });
+      });
+    };
+    fetch(std::integral_constant<int, 0>(), cw[0]);
+    static_for<2>([&](auto hc) {
+      constexpr int half = decltype(hc)::value;
+      const uint32_t thalf = trow + half * (kHalfGroups * kEntry), shalf = scol + half * (kHalfGroups * 64);
+      float acc[R][NT][4], start[4];
+      constexpr bool kStarts = QK != kMx4 && !kCentred;
+      const float nought[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      // (16-bit and 8-bit entries of the half's groups, rows rho and rho + 8)
+      constexpr int kHalfWords = kEntry < 4 ? kHalfGroups * kEntry / 4 : 0;
+      [[maybe_unused]] uint32_t sw[R][2][kHalfWords ? kHalfWords : 1];
+      static_for<kHalfWords ? 2 * R : 0>([&](auto ic) {
+        constexpr int r = decltype(ic)::value / 2, i = decltype(ic)::value % 2, kAt = r * 2 * kEight + i * kEight;
+        if constexpr (kHalfWords == 1) {
+          sw[r][i][0] = lds32<kAt>(thalf);
+        } else {
+          static_for<kHalfWords / 2>([&](auto jc) {
+            constexpr int j = decltype(jc)::value;
+            const uint2 v = lds64<kAt + j * 8>(thalf);
+            sw[r][i][2 * j] = v.x; sw[r][i][2 * j + 1] = v.y;
+          });
+        }
+      });
+      static_for<4>([&](auto qc) {
+        constexpr int q = decltype(qc)::value, qq = half * 4 + q;
+        auto& c = cw[q % 2];
+        if constexpr (qq + 1 < kChunks) fetch(std::integral_constant<int, qq + 1>(), cw[(q + 1) % 2]);
+        [[maybe_unused]] uint4 more = make_uint4(0u, 0u, 0u, 0u);
+        static_for<4>([&](auto mc) {
+          constexpr int m = decltype(mc)::value;                       // MMA of the chunk
+          constexpr int kPerGroup = 2 * SPG, at = q * 4 + m, gi = at / kPerGroup;      // MMAs of a group; MMA and group of the half
+          constexpr bool kFirst = at % kPerGroup == 0, kLast = at % kPerGroup == kPerGroup - 1;
+          if constexpr (kFirst && QK != kMx4) {    // kSumIs * sum x of the group
+            const float4 sr = ldsf128<gi * 64>(shalf);
+            start[0] = sr.x; start[1] = sr.y; start[2] = sr.z; start[3] = sr.w;
+          }
+          if constexpr (NT > 1 && m % 2 == 0) more = lds128<((qq * 4 + m) / 2) * 512>(more_x_at);
+          static_for<R>([&](auto rc) {
+            constexpr int r = decltype(rc)::value;
             uint32_t a[4];
             if constexpr (QK == kAff8) {                                  // one word: codes (0,1) and (2,3)
-              a[0] = __byte_perm(u[0][mi], 0x64646464u, 0x4140); a[1] = __byte_perm(u[1][mi], 0x64646464u, 0x4140);
-              a[2] = __byte_perm(u[0][mi], 0x64646464u, 0x4342); a[3] = __byte_perm(u[1][mi], 0x64646464u, 0x4342);
+              const uint32_t v0 = c[r][0][m], v1 = c[r][1][m];
+              a[0] = __byte_perm(v0, 0x64646464u, 0x4140); a[1] = __byte_perm(v1, 0x64646464u, 0x4140);
+              a[2] = __byte_perm(v0, 0x64646464u, 0x4342); a[3] = __byte_perm(v1, 0x64646464u, 0x4342);
             } else {                                                      // half a word: nibbles (0,4) (1,5), or (2,6) (3,7)
-              const uint32_t v0 = u[0][mi / 2], v1 = u[1][mi / 2];
-              if constexpr (QK == kAff4) {
+              const uint32_t v0 = c[r][0][m / 2], v1 = c[r][1][m / 2];
+              constexpr int n0 = (m & 1) * 2;
+              if constexpr (kNibbles) {            // bytes 0 and 2 of the word, then 1 and 3
+                const uint32_t b0 = m & 1 ? v0 >> 8 : v0, b1 = m & 1 ? v1 >> 8 : v1;
+                if constexpr (kCentred) {
+                  a[0] = fma_bf16(b0 & nib_mask, times, 0xBE00BE00u);
+                  a[1] = fma_bf16(b1 & nib_mask, times, 0xBE00BE00u);
+                  a[2] = fma_bf16(b0 & upper_mask, 0x7D007D00u, 0xBE00BE00u);      // 2^123
+                  a[3] = fma_bf16(b1 & upper_mask, 0x7D007D00u, 0xBE00BE00u);
+                } else {
+                  a[0] = and_or(b0, nib_mask, magic);
+                  a[1] = and_or(b1, nib_mask, magic);
+                  a[2] = fma_bf16(b0 & upper_mask, times, 0x42004200u);            // 32
+                  a[3] = fma_bf16(b1 & upper_mask, times, 0x42004200u);
+                }
+              } else if constexpr (QK == kAff4) {
                 auto codes = [&](uint32_t v, int nib) -> uint32_t {
                   const int right = 4 * nib - (std::is_same<AT, __half>::value ? 6 : 0);
                   return and_or(right < 0 ? v << -right : v >> right, nib_mask, magic);
                 };
-                constexpr int n0 = (mi & 1) * 2;
                 a[0] = codes(v0, n0);     a[1] = codes(v1, n0);
                 a[2] = codes(v0, n0 + 1); a[3] = codes(v1, n0 + 1);
               } else {
                 // magnitude bits of an E2M1 code at f16's exponent / mantissa boundary (the value times 2^-14,
                 // the subnormal 0.5 included), its sign at the sign
                 auto place_bits = [](uint32_t v, int nib) -> uint32_t {
-                  const uint32_t m = nib == 3 ? v >> 3 : v << (9 - 4 * nib);
-                  return (m & 0x0E000E00u) | ((v << (12 - 4 * nib)) & 0x80008000u);
+                  const uint32_t mag = nib == 3 ? v >> 3 : v << (9 - 4 * nib);
+                  return (mag & 0x0E000E00u) | ((v << (12 - 4 * nib)) & 0x80008000u);
                 };
-                constexpr int n0 = (mi & 1) * 2;
                 a[0] = place_bits(v0, n0); a[1] = place_bits(v1, n0); a[2] = place_bits(v0, n0 + 1); a[3] = place_bits(v1, n0 + 1);
               }
             }
-            if constexpr (kCentred) {
+            if constexpr (kCentred && !kNibbles) {
 #pragma unroll
               for (int i = 0; i < 4; ++i) a[i] = centred<AT>(a[i], kMagicValue + kCentre);
             }
 #pragma unroll
             for (int h = 0; h < NT; ++h) {
-              if constexpr (jj == 0 && mi == 0)     // (what keeps the magic number has one piece)
-                Mma<AT>::first(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1], kCentred ? 0.0f : start[0],
-                               kCentred ? 0.0f : start[1]);
+              const uint32_t x0 = h ? (m & 1 ? more.z : more.x) : xf[(qq * 4 + m) * 2], x1 = h ? (m & 1 ? more.w : more.y) : xf[(qq * 4 + m) * 2 + 1];
+              if constexpr (kFirst && kStarts)      // (what keeps the magic number has one piece)
+                Mma<AT>::first(acc[r][h], a, x0, x1, start);
+              else if constexpr (kFirst)
+                Mma<AT>::first(acc[r][h], a, x0, x1, nought);
               else
-                Mma<AT>::run(acc[r][h], a, h ? (mi & 1 ? more.z : more.x) : xf[x0], h ? (mi & 1 ? more.w : more.y) : xf[x0 + 1]);
+                Mma<AT>::run(acc[r][h], a, x0, x1);
             }
           });
-        });
-      });
-      // fold the group: rows rho (acc 0, 1) and rho + 8 (acc 2, 3), columns 2t and 2t + 1
-      static_for<R>([&](auto rc) {
-        constexpr int r = decltype(rc)::value;
-        constexpr int kWord = gi * kEntry / 4;
-        [[maybe_unused]] constexpr int kIn = gi * kEntry % 4;
-        constexpr int kAt = r * kBlockRows * kPitch + kWord * 4, kAt8 = kAt + 8 * kPitch;      // rows rho and rho + 8
-        auto value = [](uint32_t w) -> float {
-          if constexpr (TT == kTabE8) return __uint_as_float(max(((w >> (8 * kIn)) & 0xffu) << 23, 0x00400000u));      // 2^(e8 - 127)
-          else if constexpr (TT == kTabF32) return __uint_as_float(w);
-          else if constexpr (TT == kTabBf16) return __uint_as_float(kIn ? (w & 0xffff0000u) : (w << 16));
-          else return table_value(kIn ? w >> 16 : w & 0xffffu, QMM_F16);
-        };
-        const float s0 = value(lds32<kAt>(trow)), s1 = value(lds32<kAt8>(trow));
+          if constexpr (kLast) {
+            // fold the group: rows rho (acc 0, 1) and rho + 8 (acc 2, 3), columns 2t and 2t + 1
+            static_for<R>([&](auto rc) {
+              constexpr int r = decltype(rc)::value;
+              constexpr int kWord = gi * kEntry / 4;
+              [[maybe_unused]] constexpr int kIn = gi * kEntry % 4;
+              constexpr int kAt = r * 2 * kEight + kWord * 4, kAt8 = kAt + kEight;      // rows rho and rho + 8
+              auto value = [](uint32_t w) -> float {
+                if constexpr (TT == kTabE8) return __uint_as_float(max(((w >> (8 * kIn)) & 0xffu) << 23, 0x00400000u));      // 2^(e8 - 127)
+                else if constexpr (TT == kTabF32) return __uint_as_float(w);
+                else if constexpr (TT == kTabBf16) return __uint_as_float(kIn ? (w & 0xffff0000u) : (w << 16));
+                else return table_value(kIn ? w >> 16 : w & 0xffffu, QMM_F16);
+              };
+              float s0, s1;
+              if constexpr (kHalfWords > 0) {
+                s0 = value(sw[r][0][kWord]); s1 = value(sw[r][1][kWord]);
+              } else {
+                s0 = value(lds32<kAt>(thalf)); s1 = value(lds32<kAt8>(thalf));
+              }
 #pragma unroll
-        for (int h = 0; h < NT; ++h) {
-          fma2(y[r][h][0], y[r][h][1], s0, acc[r][h][0], acc[r][h][1]);
-          fma2(y[r][h][2], y[r][h][3], s1, acc[r][h][2], acc[r][h][3]);
-        }
-        if constexpr (QK != kMx4 && !kBiasMma) {
-          float b0 = value(lds32<kTable + kAt>(trow)), b1 = value(lds32<kTable + kAt8>(trow));
-          if constexpr (kCentred) {
-            b0 = fmaf(kCentre, s0, b0); b1 = fmaf(kCentre, s1, b1);
-          } else {
-            b0 *= 1.0f / kSumIs; b1 *= 1.0f / kSumIs;
+              for (int h = 0; h < NT; ++h) {
+                fma2(y[r][h][0], y[r][h][1], s0, acc[r][h][0], acc[r][h][1]);
+                fma2(y[r][h][2], y[r][h][3], s1, acc[r][h][2], acc[r][h][3]);
+              }
+              if constexpr (QK != kMx4 && !kBiasMma) {
+                float b0 = value(lds32<kTable + kAt>(thalf)), b1 = value(lds32<kTable + kAt8>(thalf));
+                if constexpr (kCentred) {
+                  b0 = fmaf(kCentre, s0, b0); b1 = fmaf(kCentre, s1, b1);
+                } else {
+                  b0 *= 1.0f / kSumIs; b1 *= 1.0f / kSumIs;
+                }
+                fma2(yb[r][0], yb[r][1], b0, start[0], start[1]);
+                fma2(yb[r][2], yb[r][3], b1, start[0], start[1]);
+              }
+            });
           }
-          fma2(yb[r][0], yb[r][1], b0, start[0], start[1]);
-          fma2(yb[r][2], yb[r][3], b1, start[0], start[1]);
-        }
+        });
       });
     });
     // every read of the slot has been consumed above: the warp's next box may land in it
@@ -1032,7 +1182,12 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     }
   }
 
-  if (ok && count > 0 && warp == turn) ok = add_up();      // the last tile
+  if (ok && count > 0 && warp == turn) {
+    ok = add_up();                                 // the last tile
+    // ... and the last one that this CTA leads (the tile `leader` is at stands for the cluster's last)
+    const int last_led = leader >= rank ? lap : lap - 1;
+    if (ok && csize > 1 && last_led >= 0) ok = finish(last_led);
+  }
 
   // ---- rows past the last expert's are zero ----
   if (grouped) {

@@ -195,3 +195,20 @@ def test_skewed_routing(kind, x, sizes):
     y = moe.ragged_dot(to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV), torch.from_numpy(gsz).to(DEV), **kw)
     exact = O.ragged_qmm_exact(xs, w, s, b, gsz, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
     assert O.rel_err(to_numpy(y).astype(np.float32), exact) <= TOL[x]
+
+
+@pytest.mark.parametrize("kind,gs,x,tdt", [("int4", 64, "bf16", "bf16"), ("int4", 128, "f16", "f16"), ("int4", 32, "bf16", "f32"), ("mxfp4", 32, "bf16", None)])
+@pytest.mark.parametrize("k", [1024, 5632, 14336])
+@pytest.mark.parametrize("n", [16, 33, 528, 6000])
+def test_tiles_of_a_cluster_are_finished_a_lap_late(kind, gs, x, tdt, k, n):
+    """K of one CTA, of clusters of two and of four; from one tile to a dozen of a cluster, so that the last lap of leaders is whole, partial or the only one.
+    The result is float32: every term is a product of 16-bit numbers, and what the sums round off is below 2^-24 of the largest of them, 128 sum |x| s
+    against a result of some 8 sum |x| s sqrt(1 / K): 1e-4 of the largest result."""
+    rng = np.random.default_rng(n + k)
+    (w, s, b), kw = _case(rng, kind, n, k, gs, tdt)
+    xs = activations(rng, (5, k), x)
+    args = [to_torch(xs, DEV), to_torch(w, DEV), to_torch(s, DEV), None if b is None else to_torch(b, DEV)]
+    with _lib.force_route("gemv_fmma"):
+        y = qmm.quantized_matmul(*args, out_dtype=torch.float32, **kw)
+    exact = O.qmm_exact(xs, w, s, b, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
+    assert O.rel_err(to_numpy(y).astype(np.float32), exact) <= 1e-4
