@@ -5,8 +5,8 @@
 // Through generic tensor passes (unpack to int16, transpose, widen to int64, minimum and maximum, repack, expanded
 // scale and zero maps, ...) a [4096, 14336] layer took 2.8 ms and a dozen waits for the device; the bytes that have to move
 // are 69 MB, 11 us of HBM. As a memset, three kernels, a copy of the facts and an event it took 84 us, 30 of them the kernels'; now one kernel does all
-// of it -- a CTA has a tile of codes or of tables -- and its last CTA writes the facts to host memory that the call watches: 70 us a call, 39 of
-// them the launch, the kernel and the look (the codes alone, 59 MB, take 21).
+// of it -- a CTA has a tile of codes or of tables -- and its last CTA writes the facts to host memory that the call watches: 42 us a call from Python
+// (the codes alone, 59 MB, take 17).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -26,18 +26,23 @@ constexpr int kTileN = 128, kTileK = 256;          // output rows and codes of a
 constexpr uint32_t kMix = 2246822519u;
 
 // packed int8 [K, bytes] (byte j of row k: columns 2j, 2j + 1, two's complement nibbles) -> out words [N, K / 8], codes + 8.
-// A thread owns 4 bytes (8 columns) x 8 rows, twice: eight 4-byte reads, a byte transpose, a nibble squeeze, eight words.
-// `digest` accumulates the content digest of the words (the sharing table's key).
+// A thread owns 4 bytes (8 columns) x 8 rows, twice: eight 4-byte reads, then the even rows' bytes and the odd rows' as columns, of which
+// a select each makes an even and an odd column's word. `digest` accumulates the content digest of the words (the sharing table's key).
+// (Five instructions a nibble pair to squeeze each column's nibbles together and a word at a time out of a tile with four-way bank conflicts
+// kept it at 22.2 us for the codes of [4096, 14336], 16.9 so; rows that start on no word took four loads for one: [4096, 14337] a whole call 68.6 -> 57.0.)
 struct CodeTile {
-  uint32_t tile[kTileN][kTileK / 8 + 1];
+  alignas(16) uint32_t tile[kTileN * kTileK / 8];  // [column][word], a row of words turned by 4 for every eight columns (see word_at)
   unsigned long long warp_sum[8];
 };
+constexpr int kTileWords = kTileK / 8;
+__device__ __forceinline__ int word_at(int column, int word) { return column * kTileWords + ((word + (column >> 3) * 4) & (kTileWords - 1)); }
 __device__ __forceinline__ void transpose_pack(CodeTile& shared, int n0, int k0, const uint8_t* __restrict__ packed, uint32_t* __restrict__ out, int K, int N, int bytes,
                                                bool words4, unsigned long long* digest) {
   auto& tile = shared.tile;
   auto& warp_sum = shared.warp_sum;
   const int q = threadIdx.x & 15, byte0 = n0 / 2 + q * 4;            // which 4 bytes of a row
   const bool whole = words4 && byte0 + 4 <= bytes;
+  const uintptr_t first = reinterpret_cast<uintptr_t>(packed), end = first + static_cast<int64_t>(K) * bytes;
   constexpr int kParts = kTileK / 128;                                 // 128 rows at a time, all requests first
   uint32_t r[kParts][8];
 #pragma unroll
@@ -48,8 +53,11 @@ __device__ __forceinline__ void transpose_pack(CodeTile& shared, int n0, int k0,
       r[h][i] = 0u;
       if (row0 + i < K) {
         const uint8_t* src = packed + static_cast<int64_t>(row0 + i) * bytes + byte0;
+        const uintptr_t at = reinterpret_cast<uintptr_t>(src), word = at & ~uintptr_t(3);
         if (whole) {
           r[h][i] = __ldcs(reinterpret_cast<const uint32_t*>(src));
+        } else if (byte0 + 4 <= bytes && word >= first && word + 8 <= end) {       // rows that start on no word: out of the two that it lies in
+          r[h][i] = __funnelshift_r(__ldg(reinterpret_cast<const uint32_t*>(word)), __ldg(reinterpret_cast<const uint32_t*>(word) + 1), static_cast<unsigned>(at & 3) * 8);
         } else {
           for (int b = 0; b < 4; ++b)
             if (byte0 + b < bytes) r[h][i] |= static_cast<uint32_t>(src[b]) << (8 * b);
@@ -63,35 +71,41 @@ __device__ __forceinline__ void transpose_pack(CodeTile& shared, int n0, int k0,
     t[0] = __byte_perm(x0, y0, 0x5410); t[1] = __byte_perm(x0, y0, 0x7632);
     t[2] = __byte_perm(x1, y1, 0x5410); t[3] = __byte_perm(x1, y1, 0x7632);
   };
-  auto squeeze = [](uint32_t v) -> uint32_t {      // the low nibbles of four bytes as 16 bits
-    v &= 0x0F0F0F0Fu;
-    v = (v | (v >> 4)) & 0x00FF00FFu;
-    return (v | (v >> 8)) & 0xFFFFu;
-  };
 #pragma unroll
   for (int h = 0; h < kParts; ++h) {
     const int o = h * 16 + (threadIdx.x >> 4);
-    uint32_t lo[4], hi[4];
-    transpose(r[h][0], r[h][1], r[h][2], r[h][3], lo);
-    transpose(r[h][4], r[h][5], r[h][6], r[h][7], hi);
+    uint32_t even[4], odd[4];                      // of rows 0, 2, 4, 6 and 1, 3, 5, 7; two's complement + 8 is an exclusive or with 8
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {                  // two's complement + 8 is an exclusive or with 8
-      tile[q * 8 + 2 * c][o] = (squeeze(lo[c]) | (squeeze(hi[c]) << 16)) ^ 0x88888888u;
-      tile[q * 8 + 2 * c + 1][o] = (squeeze(lo[c] >> 4) | (squeeze(hi[c] >> 4) << 16)) ^ 0x88888888u;
+    for (int i = 0; i < 8; ++i) r[h][i] ^= 0x88888888u;
+    transpose(r[h][0], r[h][2], r[h][4], r[h][6], even);
+    transpose(r[h][1], r[h][3], r[h][5], r[h][7], odd);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      tile[word_at(q * 8 + 2 * c, o)] = (even[c] & 0x0F0F0F0Fu) | ((odd[c] << 4) & 0xF0F0F0F0u);
+      tile[word_at(q * 8 + 2 * c + 1, o)] = ((even[c] >> 4) & 0x0F0F0F0Fu) | (odd[c] & 0xF0F0F0F0u);
     }
   }
   __syncthreads();
-  const int words = K / 8, w = threadIdx.x & 31, wk = k0 / 8 + w;
+  // four words of a column at a time
+  const int words = K / 8, w = (threadIdx.x & 7) * 4, wk = k0 / 8 + w;
+  const bool quads = (reinterpret_cast<uintptr_t>(out) & 15) == 0;     // (K is a multiple of 32: its rows of words then start there too)
   unsigned long long sum = 0;
-  for (int i = threadIdx.x >> 5; i < kTileN; i += 8) {
+#pragma unroll 4
+  for (int i = threadIdx.x >> 3; i < kTileN; i += 32) {
     const int n = n0 + i;
     if (n < N && wk < words) {
-      const uint32_t v = tile[i][w];
+      const uint4 v = *reinterpret_cast<const uint4*>(&tile[word_at(i, w)]);
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
       const int64_t at = static_cast<int64_t>(n) * words + wk;
-      __stcs(out + at, v);
-      uint32_t m = (v ^ (static_cast<uint32_t>(at) * 2654435761u)) * kMix;
-      m ^= m >> 15;
-      sum += m;
+      if (quads) __stcs(reinterpret_cast<uint4*>(out + at), v);
+      const uint32_t mixed = static_cast<uint32_t>(at) * 2654435761u;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (!quads) __stcs(out + at + j, u[j]);
+        uint32_t m = (u[j] ^ (mixed + static_cast<uint32_t>(j) * 2654435761u)) * kMix;
+        m ^= m >> 15;
+        sum += m;
+      }
     }
   }
   for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
@@ -102,7 +116,7 @@ __device__ __forceinline__ void transpose_pack(CodeTile& shared, int n0, int k0,
     atomicAdd(digest, sum);
   }
 }
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 8)
 transpose_pack_kernel(const uint8_t* __restrict__ packed, uint32_t* __restrict__ out, int K, int N, int bytes, bool words4, unsigned long long* digest) {
   __shared__ CodeTile shared;
   transpose_pack(shared, blockIdx.x * kTileN, blockIdx.y * kTileK, packed, out, K, N, bytes, words4, digest);
@@ -206,7 +220,7 @@ struct Told {                        // host memory
   unsigned long long digest, flags, ticket;
 };
 template <typename S, typename Z, typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 8)
 pack_layer_kernel(const uint8_t* __restrict__ packed, uint32_t* __restrict__ out, const S* __restrict__ scale, const Z* __restrict__ zero, T* __restrict__ scales, T* __restrict__ biases,
                   int K, int N, int G, int g, int bytes, bool words4, int table_tiles, Sums* sums, volatile Told* told, unsigned long long ticket) {
   __shared__ union { CodeTile codes; TableTile tables; } shared;
