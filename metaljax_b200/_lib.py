@@ -191,7 +191,7 @@ def native():
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
         loader.exec_module(module)
         module.bind(*(ctypes.cast(getattr(lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul", "qmm_moe_workspace_bytes",
-                                                                                             "qmm_moe_experts_checked", "qmm_moe_silu_mul")))
+                                                                                             "qmm_moe_experts_checked", "qmm_moe_silu_mul", "qmm_pack_dense_layer")))
         _native = module
     return _native
 

@@ -11,6 +11,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -26,6 +27,7 @@ typedef int (*QuantizedMatmul)(const qmm_tensor*, const qmm_tensor*, const qmm_t
                                int, int, int, void*);
 
 typedef int (*SiluMul)(const void*, const void*, void*, int64_t, int, void*);
+typedef int (*PackLayer)(const void*, uint32_t*, const void*, const void*, int, int, void*, void*, int, int64_t, int64_t, int64_t, int, uint64_t*, uint32_t*, void*);
 typedef int64_t (*MoeWorkspace)(const qmm_moe_block*);
 typedef int (*MoeExperts)(const qmm_moe_block*, void*);
 
@@ -33,6 +35,7 @@ typedef int (*MoeExperts)(const qmm_moe_block*, void*);
 // process, whichever file it was loaded from).
 QuantizedMatmul g_quantized_matmul = nullptr;
 SiluMul g_silu_mul = nullptr;
+PackLayer g_pack_layer = nullptr;
 MoeWorkspace g_moe_workspace = nullptr;
 MoeExperts g_moe_experts = nullptr;
 
@@ -220,6 +223,51 @@ PyObject* moe_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(y));
 }
 
+// A stored int4 Dense layer with consecutive groups (qmm._pack_dense): pack_layer(packed, scale, zero | None, K, N, wide, source)
+// -> (words, scales, biases, digest, flags, group size, whether the tables are the scales' type), a status code, or None (declined). The tables are made
+// before what they hold is known, as nearly every layer's are: one entry per stored group (the widest group size that divides it), biases in float32
+// where there are zero points (a product of a scale and an integer seldom fits the scale's type; 8 times the scale does). `wide`, `source`: the tables' type is
+// float32, or the scales', whatever they hold.
+PyObject* pack_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 7 || !g_pack_layer) Py_RETURN_NONE;
+  const at::Tensor *packed = plain_tensor(a[0]), *scale = plain_tensor(a[1]);
+  const at::Tensor* zero = a[2] == Py_None ? nullptr : plain_tensor(a[2]);
+  const int64_t k = PyLong_AsLongLong(a[3]), cols = PyLong_AsLongLong(a[4]);
+  const int wide = PyObject_IsTrue(a[5]), source = PyObject_IsTrue(a[6]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
+  if (!packed || !scale || (!zero && a[2] != Py_None)) Py_RETURN_NONE;
+  for (const at::Tensor* t : {packed, scale, zero ? zero : scale})
+    if (t->dim() != 2 || !t->is_contiguous() || t->device() != packed->device()) Py_RETURN_NONE;
+  const int64_t g = scale->size(0);
+  if (packed->scalar_type() != at::kChar || packed->size(0) != k || packed->size(1) != (cols + 1) / 2 || scale->size(1) != cols || (zero && zero->sizes() != scale->sizes())) Py_RETURN_NONE;
+  if (k >= (1LL << 24) || cols >= (1LL << 30) || k % g || k / g % 32) Py_RETURN_NONE;
+  const at::ScalarType st = scale->scalar_type(), zt = zero ? zero->scalar_type() : at::kByte;
+  const int scale_type = elem_of(st), zero_type = zt == at::kChar ? QMM_I8 : elem_of(zt);
+  if (scale_type < 0 || st == at::kByte || zero_type < 0) Py_RETURN_NONE;
+  const int64_t stored = k / g;
+  const int group = stored % 128 == 0 ? 128 : stored % 64 == 0 ? 64 : 32;
+  const int narrow = st != at::kFloat && !wide && (!zero || source);
+  at::Tensor words, scales, biases;
+  uint64_t digest = 0;
+  uint32_t flags = 0;
+  const int rc = unlocked([&]() -> int {
+    const c10::cuda::CUDAGuard on(packed->device());
+    const at::ScalarType table = narrow ? st : at::kFloat;
+    words = at::detail::empty_cuda({cols, k / 8}, at::kUInt32, packed->device(), std::nullopt);
+    scales = at::detail::empty_cuda({cols, k / group}, table, packed->device(), std::nullopt);
+    biases = at::detail::empty_cuda({cols, k / group}, table, packed->device(), std::nullopt);
+    return g_pack_layer(packed->const_data_ptr(), static_cast<uint32_t*>(words.data_ptr()), scale->const_data_ptr(), zero ? zero->const_data_ptr() : nullptr, scale_type,
+                        zero ? zero_type : 0, scales.data_ptr(), biases.data_ptr(), narrow, g, cols, k, group, &digest, &flags,
+                        c10::cuda::getCurrentCUDAStream(packed->get_device()).stream());
+  });
+  if (rc) return PyLong_FromLong(rc);
+  return Py_BuildValue("(NNNKIiO)", THPVariable_Wrap(std::move(words)), THPVariable_Wrap(std::move(scales)), THPVariable_Wrap(std::move(biases)),
+                       static_cast<unsigned long long>(digest), static_cast<unsigned int>(flags), group, narrow ? Py_True : Py_False);
+}
+
 // What is left of a program when all of it is products of two-dimensional activations and gates between them:
 // run_steps(arguments, steps, returns, values): the program's values are numbered, its arguments first; `returns` are numbers; a step is
 //   (x, result, w, scales, biases | None, group_size, bits, mode, dtype)    result = x . deq(w)^T as dtype
@@ -360,16 +408,17 @@ PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   }
 }
 
-// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts_checked[, qmm_moe_silu_mul])
+// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts_checked[, qmm_moe_silu_mul[, qmm_pack_dense_layer]])
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 3 && n != 4) {
+  if (n < 3 || n > 5) {
     PyErr_SetString(PyExc_TypeError, "bind takes the entry points' addresses");
     return nullptr;
   }
   g_quantized_matmul = reinterpret_cast<QuantizedMatmul>(PyLong_AsVoidPtr(a[0]));
   g_moe_workspace = reinterpret_cast<MoeWorkspace>(PyLong_AsVoidPtr(a[1]));
   g_moe_experts = reinterpret_cast<MoeExperts>(PyLong_AsVoidPtr(a[2]));
-  if (n == 4) g_silu_mul = reinterpret_cast<SiluMul>(PyLong_AsVoidPtr(a[3]));
+  if (n > 3) g_silu_mul = reinterpret_cast<SiluMul>(PyLong_AsVoidPtr(a[3]));
+  if (n > 4) g_pack_layer = reinterpret_cast<PackLayer>(PyLong_AsVoidPtr(a[4]));
   if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }
@@ -378,6 +427,7 @@ PyMethodDef kMethods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(bind)), METH_FASTCALL, nullptr},
     {"quantized_matmul", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<quantized_matmul>)), METH_FASTCALL, nullptr},
     {"moe_experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<moe_experts>)), METH_FASTCALL, nullptr},
+    {"pack_layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<pack_layer>)), METH_FASTCALL, nullptr},
     {"run_steps", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(guarded<run_steps>)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 

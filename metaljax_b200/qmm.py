@@ -740,10 +740,46 @@ def unpack_keras_int4(packed: torch.Tensor, columns: int) -> torch.Tensor:
     return ((both ^ 8) - 8).to(torch.int8)
 
 
+_FACT_OF = {128: 1, 64: 2, 32: 0}        # the fact that rules a group size out
+
+
 def _pack_dense(packed, scale, zero, k, n, out_dtype):
     """`from_keras_int4` on the GPU for consecutive groups of a multiple of 32 rows: codes and tables in one
-    kernel and one wait for the device (which group size the tables allow, and whether the biases narrow, is in the data).
+    kernel and one wait for the device (which group size the tables allow, and whether the biases narrow, is in the data),
+    made natively (csrc/torch_call.cpp: 512 x 256 49 -> 24 us a call, nearly all of it the host's).
     None where the general way has to look (host arrays, other layouts, zero points it may reject)."""
+    if not packed.is_cuda or _SCALE_WIDTH not in ("auto", "source", "f32"):
+        return None
+    made = _lib.native().pack_layer(packed, scale, zero, k, n, _SCALE_WIDTH == "f32", _SCALE_WIDTH == "source")
+    if made is None:
+        made = _pack_layer(packed, scale, zero, k, n)
+        if made is None:
+            return None
+    elif type(made) is int:
+        _lib.check(made)
+    words, scales, biases, digest, flags, group, narrow = made
+    if flags & 8:
+        return None
+    plan = (group, narrow)
+    for group in _GROUP_SIZES:
+        if k % group == 0 and not flags & _FACT_OF[group]:
+            break
+    narrow = scale.dtype != torch.float32 and (_SCALE_WIDTH == "source" or _SCALE_WIDTH != "f32" and not flags & 4)
+    if (group, narrow) != plan:                                             # the facts ask for other tables
+        with torch.cuda.device(packed.device):
+            scales = torch.empty((n, k // group), dtype=scale.dtype if narrow else torch.float32, device=packed.device)
+            biases = torch.empty_like(scales)
+            _lib.check(_lib.lib().qmm_pack_dense_tables(scale.data_ptr(), None if zero is None else zero.data_ptr(), _lib.ELEM[scale.dtype],
+                                                        0 if zero is None else _lib.ELEM[zero.dtype], scales.data_ptr(), biases.data_ptr(), int(narrow),
+                                                        scale.shape[0], n, k, group, _lib.stream_ptr(packed)))
+    m = Match()
+    m.mode, m.N, m.K = "affine", n, k
+    m.out_dtype = out_dtype or scale.dtype
+    return _record_pack(m, _Pack((packed, scale), words, scales, biases, None, group, 4, "affine"), digest & 0xFFFFFFFFFFFF)
+
+
+def _pack_layer(packed, scale, zero, k, n):
+    """The native `pack_layer` for tensors that it declines (subclasses, tensors that require a gradient)."""
     tables = (scale,) if zero is None else (scale, zero)
     if not all(t.is_cuda and t.is_contiguous() and t.dim() == 2 and t.device == packed.device for t in (packed, *tables)):
         return None
@@ -754,38 +790,18 @@ def _pack_dense(packed, scale, zero, k, n, out_dtype):
         return None
     if k % g or (k // g) % 32 or scale.dtype not in _FLOATS or (zero is not None and zero.dtype not in (*_FLOATS, torch.int8, torch.uint8)):
         return None
-    if _SCALE_WIDTH not in ("auto", "source", "f32"):
-        return None
-    lib, stream, dev = _lib.lib(), _lib.stream_ptr(packed), packed.device
+    dev = packed.device
     with torch.cuda.device(dev):
+        group = next(s for s in _GROUP_SIZES if k // g % s == 0)
+        narrow = scale.dtype != torch.float32 and _SCALE_WIDTH != "f32" and (zero is None or _SCALE_WIDTH == "source")
         words = torch.empty((n, k // 8), dtype=torch.uint32, device=dev)
-        args = (scale.data_ptr(), None if zero is None else zero.data_ptr(), _lib.ELEM[scale.dtype], 0 if zero is None else _lib.ELEM[zero.dtype])
-        # The tables are made before the facts are known, as nearly every layer's are: one entry per stored group (the widest
-        # group size that divides it), biases in float32 where there are zero points (a product of a scale and
-        # an integer seldom fits the scale's type; 8 times the scale does). The facts can only ask for others.
-        may_narrow = scale.dtype != torch.float32 and _SCALE_WIDTH != "f32"
-        plan = (next(s for s in _GROUP_SIZES if k // g % s == 0), may_narrow and (zero is None or _SCALE_WIDTH == "source"))
-
-        def tables(group, narrow):
-            scales = torch.empty((n, k // group), dtype=scale.dtype if narrow else torch.float32, device=dev)
-            return scales, torch.empty_like(scales)
-
-        scales, biases = tables(*plan)
+        scales = torch.empty((n, k // group), dtype=scale.dtype if narrow else torch.float32, device=dev)
+        biases = torch.empty_like(scales)
         digest, flags = ctypes.c_uint64(), ctypes.c_uint32()
-        _lib.check(lib.qmm_pack_dense_layer(packed.data_ptr(), words.data_ptr(), *args, scales.data_ptr(), biases.data_ptr(), int(plan[1]), g, n, k, plan[0],
-                                            ctypes.byref(digest), ctypes.byref(flags), stream))
-        digest, flags = digest.value, flags.value
-        if flags & 8:
-            return None
-        group = next(s for s in _GROUP_SIZES if k % s == 0 and not (flags & {128: 1, 64: 2, 32: 0}[s]))
-        narrow = may_narrow and (_SCALE_WIDTH == "source" or not flags & 4)
-        if (group, narrow) != plan:
-            scales, biases = tables(group, narrow)
-            _lib.check(lib.qmm_pack_dense_tables(*args, scales.data_ptr(), biases.data_ptr(), int(narrow), g, n, k, group, stream))
-    m = Match()
-    m.mode, m.N, m.K = "affine", n, k
-    m.out_dtype = out_dtype or scale.dtype
-    return _record_pack(m, _Pack((packed, scale), words, scales, biases, None, group, 4, "affine"), digest & 0xFFFFFFFFFFFF)
+        _lib.check(_lib.lib().qmm_pack_dense_layer(packed.data_ptr(), words.data_ptr(), scale.data_ptr(), None if zero is None else zero.data_ptr(), _lib.ELEM[scale.dtype],
+                                                   0 if zero is None else _lib.ELEM[zero.dtype], scales.data_ptr(), biases.data_ptr(), int(narrow), g, n, k, group,
+                                                   ctypes.byref(digest), ctypes.byref(flags), _lib.stream_ptr(packed)))
+    return words, scales, biases, digest.value, flags.value, group, narrow
 
 
 def from_keras_int4(packed, scale, zero=None, g_idx=None, columns=None, out_dtype=None):

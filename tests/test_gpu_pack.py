@@ -178,3 +178,31 @@ def test_the_steps_in_a_captured_stream_are_the_layer(k, n, groups, sdt, zdt):
     torch.cuda.synchronize()
     assert torch.equal(got[0].view(torch.int32), words.view(torch.int32)) and torch.equal(got[1], scales) and torch.equal(got[2], biases)
     assert sums[0].item() % (1 << 64) == digest and sums[1].item() == facts
+
+
+@pytest.mark.parametrize("skew", [1, 2, 3])
+@pytest.mark.parametrize("k,n", [(32, 1), (288, 9), (256, 262), (544, 515)])
+def test_codes_that_start_on_no_word(k, n, skew):
+    """Rows of 1, 5, 131 and 258 bytes, the first of which starts on no word, with nothing allocated before or behind it that is this layer's; the words written on no 16 bytes."""
+    g = torch.Generator().manual_seed(k + n + skew)
+    rows = torch.randint(-128, 128, (k, -(-n // 2)), generator=g, dtype=torch.int8)
+    scale = torch.full((k // 32, n), 0.5)
+    want = qmm.from_keras_int4(rows, scale, columns=n)
+    flat = torch.empty(skew + rows.numel(), dtype=torch.int8, device=DEV)
+    packed = flat[skew:].view(rows.shape)
+    packed.copy_(rows)
+    got = qmm.from_keras_int4(packed, scale.to(DEV), columns=n)
+    assert torch.equal(got.w.cpu().view(torch.int32), want.w.view(torch.int32))
+    words = torch.zeros(n * (k // 8) + 2, dtype=torch.int32, device=DEV)
+    digest = torch.zeros(1, dtype=torch.int64, device=DEV)
+    _lib.check(_lib.lib().qmm_pack_dense_codes(packed.data_ptr(), words.data_ptr() + 4, k, n, digest.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(words[1:-1].cpu(), want.w.view(torch.int32).reshape(-1)) and words[0] == 0 and words[-1] == 0
+
+
+def test_a_tensor_that_requires_a_gradient_is_packed_all_the_same():
+    """What the native call declines takes the way through ctypes: the same words."""
+    g = torch.Generator().manual_seed(5)
+    packed = torch.randint(-128, 128, (256, 33), generator=g, dtype=torch.int8).to(DEV)
+    scale = (torch.rand((4, 66), generator=g) * 0.02 + 0.01).to(DEV)
+    got, want = qmm.from_keras_int4(packed, scale.clone().requires_grad_()), qmm.from_keras_int4(packed, scale)
+    assert torch.equal(got.w.view(torch.int32), want.w.view(torch.int32)) and torch.equal(got.biases, want.biases)
