@@ -312,6 +312,9 @@ qmm_gemv_imma_kernel(const __grid_constant__ CUtensorMap w_map, const ImmaParams
   (void)trace;
 #endif
   QMM_TRACE(trace, 0);               // CTA resident
+  // The way from here to the next launch's start is part of every small call (4096 x 4096 5.48 -> 5.31 us); a decode step's launches, whose
+  // successors are other kernels, are better off with their own boxes requested first (1997 against 1970 us).
+  if constexpr (!FUSED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // ---- barriers, then this warp's first boxes: before anything else ----
   uint64_t* full = full_all + warp * kMaxRing;
   uint8_t* wring = smem + warp * ring * kBoxSmem;
@@ -335,7 +338,7 @@ qmm_gemv_imma_kernel(const __grid_constant__ CUtensorMap w_map, const ImmaParams
       for (int i = 0; i < ring && itile < ntiles; ++i) issue_box();
   }
   if (threadIdx.x < 16) zeros[threadIdx.x] = 0u;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if constexpr (FUSED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __syncwarp();
 
   // ---- lane constants ----
