@@ -182,6 +182,13 @@ int qmm_ragged_dot(const qmm_tensor* x, const qmm_tensor* w, const qmm_tensor* s
 int qmm_ragged_mm(const qmm_tensor* x, const qmm_tensor* w, const qmm_tensor* group_sizes,
                   qmm_tensor* y, void* stream);
 
+/* y = silu(x . deq(gate)^T) * (x . deq(up)^T) as one launch, each step rounded to y's type as qmm_quantized_matmul and
+ * qmm_moe_silu_mul round it: x, y 2-D (or more leading dimensions of one weight) of 2 to 16 rows, bf16 or f16 alike, two
+ * weights of one shape and table type. QMM_ERR_UNSUPPORTED, with nothing launched, for what the few-rows kernel does not take. */
+int qmm_gated_matmul(const qmm_tensor* x, const qmm_tensor* gate_w, const qmm_tensor* gate_scales, const qmm_tensor* gate_biases,
+                     const qmm_tensor* up_w, const qmm_tensor* up_scales, const qmm_tensor* up_biases, qmm_tensor* y, int group_size,
+                     int bits, int mode, void* stream);
+
 /* The two element-wise steps of a gathered expert block, raw pointers (dtype: QMM_BF16 |
  * QMM_F16; 16-byte aligned). The reference runs them as generic pair-space ops after its
  * gathered dots (src/metaljax/moe.py:1425-1461).

@@ -114,6 +114,7 @@ _SIGNATURES = {
                               + [ctypes.c_int64] * 3 + [ctypes.c_int, ctypes.c_void_p]),
     "qmm_pack_dense_layer": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2 + [ctypes.c_int]
                              + [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.c_void_p] * 3),
+    "qmm_gated_matmul": (ctypes.c_int, [_T] * 8 + [ctypes.c_int] * 3 + [ctypes.c_void_p]),
     "qmm_moe_silu_mul": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
                                         ctypes.c_int, ctypes.c_void_p]),
     "qmm_moe_routed_sum": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
@@ -191,7 +192,8 @@ def native():
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
         loader.exec_module(module)
         module.bind(*(ctypes.cast(getattr(lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul", "qmm_moe_workspace_bytes",
-                                                                                             "qmm_moe_experts_checked", "qmm_moe_silu_mul", "qmm_pack_dense_layer")))
+                                                                                             "qmm_moe_experts_checked", "qmm_moe_silu_mul", "qmm_pack_dense_layer",
+                                                                                             "qmm_gated_matmul")))
         _native = module
     return _native
 

@@ -446,6 +446,19 @@ int qmm_check_quantized_matmul(const qmm_tensor* x, const qmm_tensor* w, const q
   return build_dense(x, w, scales, biases, y, transpose, group_size, bits, mode, false, &p);
 }
 
+int qmm_gated_matmul(const qmm_tensor* x, const qmm_tensor* gate_w, const qmm_tensor* gate_scales, const qmm_tensor* gate_biases, const qmm_tensor* up_w, const qmm_tensor* up_scales,
+                     const qmm_tensor* up_biases, qmm_tensor* y, int group_size, int bits, int mode, void* stream) {
+  qmm_problem gate, up;
+  int rc;
+  if ((rc = build_dense(x, gate_w, gate_scales, gate_biases, y, 1, group_size, bits, mode, true, &gate)) || (rc = validate_problem(gate, true))) return rc;
+  if ((rc = build_dense(x, up_w, up_scales, up_biases, y, 1, group_size, bits, mode, true, &up)) || (rc = validate_problem(up, true))) return rc;
+  const bool alike = gate.batch == 1 && up.batch == 1 && gate.table_dtype == up.table_dtype;
+  if (!alike || gate.M < 2 || gate.K == 0 || route_of(gate) != QMM_ROUTE_GEMV || route_of(up) != QMM_ROUTE_GEMV || !rows_pair_supports(gate))
+    return fail(QMM_ERR_UNSUPPORTED, "gated_matmul: two products and a gate, of 2 to 16 rows of 16-bit activations, that the few-rows kernel takes");
+  const RowsPair second = {up.w, up.scales, up.biases};
+  return launch_rows(gate, static_cast<cudaStream_t>(stream), nullptr, false, &second);
+}
+
 int qmm_quantized_matmul(const qmm_tensor* x, const qmm_tensor* w, const qmm_tensor* scales,
                          const qmm_tensor* biases, qmm_tensor* y, int transpose, int group_size,
                          int bits, int mode, void* stream) {

@@ -55,7 +55,15 @@ struct RowsGather {            // grouped products whose rows of x are picked by
   int64_t total_x_rows;
 };
 // `exact`: 16-bit activations whose sums are to be as exact as plain float32 ones (float32 activations' always are).
-int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr, bool exact = false);
+// `pair`: a second weight of the same shape, types and strides; y = silu(x . deq(w)^T) * (x . deq(pair)^T), each step rounded to y's type, which is x's
+// (rows_pair_supports).
+struct RowsPair {
+  const void* w;
+  const void* scales;
+  const void* biases;
+};
+int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr, bool exact = false, const RowsPair* pair = nullptr);
+bool rows_pair_supports(const qmm_problem& p);
 bool rows_supports(const qmm_problem& p);
 double rows_estimate(const qmm_problem& p);      // what a dense product of float32 activations is expected to take here, us
 // Float32 activations of more than a few rows on the tensor cores (f32_tc_pays: it takes them, and wins).

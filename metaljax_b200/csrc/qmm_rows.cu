@@ -7,7 +7,7 @@ using namespace rows;
 
 namespace rows {
 #define QMM_ROWS_EXTERN(QK, XT) \
-  extern template int launch_rows_kernel<QK, XT>(const CUtensorMap&, RowsParams&, RowsPlan&, const RowsShape&, bool, cudaStream_t);
+  extern template int launch_rows_kernel<QK, XT>(const CUtensorMap&, const CUtensorMap&, RowsParams&, RowsPlan&, const RowsShape&, bool, cudaStream_t);
 QMM_ROWS_EXTERN(kAff4, __nv_bfloat16)
 QMM_ROWS_EXTERN(kAff4, __half)
 QMM_ROWS_EXTERN(kAff4, float)
@@ -41,11 +41,12 @@ size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
 // next best 22.0, a cluster of two), 128256 x 4096 65.6 / 65.6 (73.0), 4096 x 14336 16.0 / 16.0 (17.0), 4096 x 4096 7.1 / 7.1 (7.6), 1024 x 1024 5.9 / 5.9,
 // 16 rows 4096 x 4096 8.6 / 8.6 (9.3), 4 rows 5632 x 2048 6.1 / 6.1 (6.6), 2048 x 5632 7.8 / 7.8, 8-bit 8 rows 14336 x 4096 14.6 / 14.6 (15.2),
 // mxfp4 8 rows 5760 x 2880 8.9 / 8.7, float32 33 rows 4096 x 4096 34.8 / 33.2.
-RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh, int segs) {
+RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh, int segs, bool pair = false) {
   const int sms = device_sm_count();
   RowsPlan best = {};
-  for (int blocks = kMaxBlocks; blocks >= (sh.exact ? kMaxBlocks : 1); --blocks) {
-    const int64_t items = chunks * ((rows + kBlockRows * blocks - 1) / (kBlockRows * blocks));
+  for (int blocks = kMaxBlocks; blocks >= (sh.exact || pair ? kMaxBlocks : 1); --blocks) {
+    const int tile_rows = pair ? kBlockRows : kBlockRows * blocks;
+    const int64_t items = chunks * ((rows + tile_rows - 1) / tile_rows);
     for (int c = 1; c <= kMaxCluster; c *= 2) {
       if (c > slices && c > 1) break;
       RowsPlan pl = {};
@@ -128,10 +129,14 @@ bool gemv_supports(const qmm_problem& p) {
   return (p.x_dtype == QMM_BF16 || p.x_dtype == QMM_F16) && !p.group_sizes && p.M <= 16 && p.batch <= 65535 && rows_supports(p);
 }
 
-int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather, bool exact) {
+int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather, bool exact, const RowsPair* pair) {
   RowsParams rp = {};
   rp.x = p.x; rp.scales = p.scales; rp.biases = p.biases; rp.y = p.y;
   rp.lhs_idx = p.lhs_idx; rp.rhs_idx = p.rhs_idx; rp.group_sizes = p.group_sizes;
+  if (pair) {
+    rp.scales2 = pair->scales;
+    rp.biases2 = pair->biases;
+  }
   if (gather) {
     rp.x_rows = gather->x_rows;
     rp.total_x_rows = gather->total_x_rows;
@@ -159,9 +164,9 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
   // (a slice's entries start on the units that its own row of entries and a row of the table are multiples of)
   const int slice_bytes = sh.groups * entry, row_bytes_t = rp.groups * entry;
   rp.table_unit = (row_bytes_t | slice_bytes) % 8 == 0 && row_bytes_t % slice_bytes == 0 ? (slice_bytes % 16 == 0 ? 16 : 8) : (row_bytes_t | slice_bytes) % 4 == 0 ? 4 : 1;
-  RowsPlan pl = plan_rows(live * ((per_seg + chunk - 1) / chunk), rp.N, slices, sh, p.group_sizes ? rp.segs : 0);
+  RowsPlan pl = plan_rows(live * ((per_seg + chunk - 1) / chunk), rp.N, slices, sh, p.group_sizes ? rp.segs : 0, pair != nullptr);
   if (!pl.warps) return fail(QMM_ERR_UNSUPPORTED, "few-rows kernel: no plan fits shared memory");
-  const int tile_rows = kBlockRows * pl.blocks;
+  const int tile_rows = pair ? kBlockRows : kBlockRows * pl.blocks;
   rp.tiles = (rp.N + tile_rows - 1) / tile_rows;
   pl.items = p.batch * ((p.M + chunk - 1) / chunk) * rp.tiles;
   rp.cluster = pl.cluster; rp.slices_per_cta = pl.slices_per_cta; rp.slices_per_warp = pl.slices_per_warp;
@@ -173,17 +178,26 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
   CUtensorMap wm;
   const int rc = tensor_map_2d(&wm, QMM_U8, p.w, row_bytes, static_cast<uint64_t>(p.N) * nweights, row_bytes, kBoxBytes, tile_rows, 1);
   if (rc) return rc;
+  CUtensorMap wm2 = wm;
+  if (pair) {
+    const int rc2 = tensor_map_2d(&wm2, QMM_U8, pair->w, row_bytes, static_cast<uint64_t>(p.N) * nweights, row_bytes, kBoxBytes, tile_rows, 1);
+    if (rc2) return rc2;
+  }
   // A gather's indices decide which weight the first boxes come from: it is serialized in the ordinary way.
   const bool early = !p.lhs_idx;
   auto launch = [&](auto kind) {
     constexpr int QK = decltype(kind)::value;
-    if (p.x_dtype == QMM_BF16) return launch_rows_kernel<QK, __nv_bfloat16>(wm, rp, pl, sh, early, stream);
-    if (p.x_dtype == QMM_F16) return launch_rows_kernel<QK, __half>(wm, rp, pl, sh, early, stream);
-    return launch_rows_kernel<QK, float>(wm, rp, pl, sh, early, stream);
+    if (p.x_dtype == QMM_BF16) return launch_rows_kernel<QK, __nv_bfloat16>(wm, wm2, rp, pl, sh, early, stream);
+    if (p.x_dtype == QMM_F16) return launch_rows_kernel<QK, __half>(wm, wm2, rp, pl, sh, early, stream);
+    return launch_rows_kernel<QK, float>(wm, wm2, rp, pl, sh, early, stream);
   };
   if (mx) return launch(std::integral_constant<int, kMx4>());
   if (bits == 8) return launch(std::integral_constant<int, kAff8>());
   return launch(std::integral_constant<int, kAff4>());
+}
+
+bool rows_pair_supports(const qmm_problem& p) {
+  return (p.x_dtype == QMM_BF16 || p.x_dtype == QMM_F16) && p.y_dtype == p.x_dtype && !p.lhs_idx && rows_supports(p);
 }
 
 int launch_gemv(const qmm_problem& p, cudaStream_t stream) {

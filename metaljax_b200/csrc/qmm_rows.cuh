@@ -112,6 +112,8 @@ struct RowsParams {
   int table_unit;                // bytes on which every row's table entries of every slice start: 8, 4, or less
   int64_t table_bytes;           // of a whole table
   int64_t total_x_rows;          // grouped: rows of x that x_rows may name
+  const void* scales2;           // a pair of weights of one shape (two blocks): block 0 of a tile is 16 rows of the first, block 1 the same
+  const void* biases2;           //   rows of the second, and y is silu(first) * second; NULL: one weight
 };
 
 // d (+)= A (16 rows of weights) * B (8 columns of activations), K 16.
@@ -291,15 +293,19 @@ constexpr int more_x_bytes(int tokens) { return tokens == 8 ? 0 : kSliceK * 16; 
 // QK: quantization kind. XT: activation type in memory. T: activation rows (tokens) of a chunk, 8 (16-bit) or 4 (float32). SPG: 32-code
 // steps per quantization group (1, 2, 4). TT: what the table entries are. R: 16-row blocks of a tile. EXACT: the magic number is taken off the codes, not
 // off the sums (affine codes).
+// With a second weight (scales2; two blocks, 16-bit activations) the two blocks of a tile are the same rows of both, and y is silu(first) * second: three launches
+// as one. 4 rows of a feed-forward block of 2048 x 5632 23.1 -> 17.0 us. It is no kernel of its own, though that would cost plain products nothing (18.0 against 18.3 us, 8 rows of
+// 28672 x 4096): where this one and another of its size take turns, each launch is slower (16.6 -> 22.3 us a launch of two kernels in turn; the feed-forward
+// block 20.3, 8 tokens through 8 experts 198 against 178).
 template <int QK, typename XT, int T, int SPG, int TT, int R, bool EXACT>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
-qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
+qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap w2_map, const RowsParams p) {
   using AT = typename std::conditional<QK == kAff4, typename std::conditional<std::is_same<XT, float>::value, __nv_bfloat16, XT>::type, __half>::type;
   constexpr bool kScaled = std::is_same<AT, __half>::value && !std::is_same<XT, __half>::value;
   // A pair of codes under this exponent is kMagicValue + code.
   constexpr uint32_t kMagic = QK == kAff8 ? 0x64006400u : std::is_same<AT, __half>::value ? 0x4C004C00u : 0x43004300u;
   constexpr float kMagicValue = QK == kAff8 ? 1024.0f : std::is_same<AT, __half>::value ? 16.0f : 128.0f;
-  constexpr bool kCentred = EXACT && QK != kMx4;
+  constexpr bool kCentred = EXACT && QK != kMx4, kMayPair = !EXACT && R == 2 && sizeof(XT) == 2;
   // 4-bit codes as bf16: of each pair of nibbles the upper one by an FMA, as (128 + q) / 4 against four times the activation, or both as (q - 8) / 64.
   constexpr bool kNibbles = QK == kAff4 && std::is_same<AT, __nv_bfloat16>::value, kQuarters = kNibbles && !kCentred;
   constexpr float kCentre = QK == kAff8 ? 128.0f : 8.0f;
@@ -450,6 +456,9 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     do { ++seg; } while (seg + 1 < p.segs && chunks_of(seg) == 0);
   };
 
+  const bool pair = kMayPair && p.scales2 != nullptr;
+  const int step_rows = pair ? kBlockRows : kTileRows;             // weight rows from a tile to the next
+
   // ---- the ring: boxes in the order they are consumed, a few ahead ----
   const int first_slice = rank * p.slices_per_cta + warp * p.slices_per_warp;
   int ahead_left = left * p.slices_per_warp, ahead_row = 0, ahead_last = 0, ahead_tiles = p.tiles - tile0, ahead_sub = 0;
@@ -457,7 +466,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   if (left > 0) {
     ahead_row = weight_row_of(seg0);
     ahead_last = ahead_row + p.N - 1;
-    ahead_row += tile0 * kTileRows;
+    ahead_row += tile0 * step_rows;
     if (lane == 0) { ahead_at[0] = seg0; ahead_at[1] = chunk0; }
     __syncwarp();
   }
@@ -474,12 +483,16 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
       const uint32_t dst = ring_at + ahead_slot * kStage;
       mbar_expect_tx(bar, kStage);
 #pragma unroll
-      for (int b = 0; b < kBoxes; ++b) tma_load_2d(&w_map, dst + b * kBoxSmem, bar, (slice * kBoxes + b) * kBoxBytes, ahead_row);
+      for (int b = 0; b < kBoxes; ++b) {
+        tma_load_2d(&w_map, dst + b * kBoxSmem, bar, (slice * kBoxes + b) * kBoxBytes, ahead_row);
+        if (pair) tma_load_2d(&w2_map, dst + b * kBoxSmem + kBlockRows * kBoxBytes, bar, (slice * kBoxes + b) * kBoxBytes, ahead_row);
+      }
     }
     {
       // a lane's share of the tables: a weight row of one table, or (two blocks) of both. Entries past the end of a row are
       // some other entry of it: what they multiply is zero.
-      const int64_t at = static_cast<int64_t>(min(ahead_row + table_row, ahead_last)) * table_row_size + first_entry(slice) * kEntry;
+      const int64_t at = static_cast<int64_t>(min(ahead_row + (pair ? table_row & 15 : table_row), ahead_last)) * table_row_size + first_entry(slice) * kEntry;
+      const bool second = pair && lane >= 16;
       const uint32_t dst = my_tables + ahead_slot * (kSlot - kStage);
       auto copy = [&](const uint8_t* table, uint32_t to) {
         const uint8_t* src = table + at;
@@ -502,8 +515,8 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
         }
       };
       if (kBothTables) {
-        if (kTileRows == 32 || lane < 16) copy(static_cast<const uint8_t*>(p.scales), dst);
-        if (TT != kTabE8) copy(static_cast<const uint8_t*>(p.biases), dst + kTable);
+        if (kTileRows == 32 || lane < 16) copy(static_cast<const uint8_t*>(second ? p.scales2 : p.scales), dst);
+        if (TT != kTabE8) copy(static_cast<const uint8_t*>(second ? p.biases2 : p.biases), dst + kTable);
       } else {
         copy(my_table, dst);
       }
@@ -515,7 +528,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
       if (++ahead_sub < p.slices_per_warp) return;
       ahead_sub = 0;
     }
-    ahead_row += kTileRows;
+    ahead_row += step_rows;
     if (--ahead_tiles == 0) {
       ahead_tiles = p.tiles;
       if (ahead_left > 0) {
@@ -830,6 +843,20 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
   int done_tile = 0, done_which = 0, lap = 0, leader = 0;
   uint32_t done_buf = 0, done_phase = 0;
   auto store_tile = [&](const float (&v)[R][4], int64_t y0, int rows_left, int at_tile) {
+    if (pair) {                                    // rounded as products, gate and their product are when each is a launch of its own
+      auto gated = [&](auto type, int i) {
+        using YT = decltype(type);
+        const float gate = static_cast<float>(static_cast<YT>(v[0][i])), up = static_cast<float>(static_cast<YT>(v[1][i]));
+        return static_cast<float>(static_cast<YT>(gate / (1.0f + __expf(-gate)))) * up;
+      };
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int col = 2 * t + (i & 1), n = at_tile * kBlockRows + rho + (i >> 1) * 8;
+        if (col < rows_left && n < p.N)
+          store_y(p.y, p.y_dtype, y0 + static_cast<int64_t>(col) * p.N + n, p.y_dtype == QMM_BF16 ? gated(__nv_bfloat16(), i) : gated(__half(), i));
+      }
+      return;
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -945,7 +972,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const RowsParams p) {
     if (kEntry < 4 && p.table_unit < 4) {          // entries that do not start on words: shifted to where they would, once per tile
       const int row = kTileRows == 32 ? lane : lane & 15;
       auto straighten = [&](uint32_t at) {
-        const int wr = place[which].weight_row + min(tile * kTileRows + row, p.N - 1);
+        const int wr = place[which].weight_row + min(tile * step_rows + (pair ? row & 15 : row), p.N - 1);
         const uint32_t skew = ((static_cast<uint32_t>(wr) * static_cast<uint32_t>(p.groups) + first_entry(first_slice + sub)) * kEntry & 3u) * 8;
         uint32_t word = lds32<0>(at);
 #pragma unroll
@@ -1224,7 +1251,7 @@ struct RowsShape {
 };
 
 template <int QK, typename XT, int T, int SPG, int TT, int R, bool EXACT>
-int launch_kernel_of(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool early, cudaStream_t stream) {
+int launch_kernel_of(const CUtensorMap& wm, const CUtensorMap& wm2, RowsParams& rp, RowsPlan& pl, bool early, cudaStream_t stream) {
   auto kernel = qmm_rows_kernel<QK, XT, T, SPG, TT, R, EXACT>;
   static bool configured[kMaxDevices] = {};     // the attribute is per device
   const int dev = current_device();
@@ -1260,50 +1287,50 @@ int launch_kernel_of(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, bool e
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++cfg.numAttrs;
   }
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, wm, rp);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, wm, wm2, rp);
   if (e != cudaSuccess) return fail(QMM_ERR_CUDA, "qmm_rows_kernel launch: %s", cudaGetErrorString(e));
   count_launch();
   return check_launch("qmm_rows_kernel");
 }
 
 template <int QK, typename XT, int T, int SPG, int TT>
-int launch_kernel(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
+int launch_kernel(const CUtensorMap& wm, const CUtensorMap& wm2, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
   constexpr bool kFloat = std::is_same<XT, float>::value;
   if constexpr (QK != kMx4 && !kFloat)
-    if (sh.exact) return launch_kernel_of<QK, XT, T, SPG, TT, kMaxBlocks, true>(wm, rp, pl, early, stream);
-  if (pl.blocks == 1) return launch_kernel_of<QK, XT, T, SPG, TT, 1, kFloat>(wm, rp, pl, early, stream);
-  return launch_kernel_of<QK, XT, T, SPG, TT, kMaxBlocks, kFloat>(wm, rp, pl, early, stream);
+    if (sh.exact) return launch_kernel_of<QK, XT, T, SPG, TT, kMaxBlocks, true>(wm, wm2, rp, pl, early, stream);
+  if (pl.blocks == 1) return launch_kernel_of<QK, XT, T, SPG, TT, 1, kFloat>(wm, wm2, rp, pl, early, stream);
+  return launch_kernel_of<QK, XT, T, SPG, TT, kMaxBlocks, kFloat>(wm, wm2, rp, pl, early, stream);
 }
 
 // (QK, XT) by T, group size and table type.
 template <int QK, typename XT, int T, int SPG>
-int launch_tt(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
+int launch_tt(const CUtensorMap& wm, const CUtensorMap& wm2, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
   if constexpr (QK == kMx4) {
-    return launch_kernel<QK, XT, T, SPG, kTabE8>(wm, rp, pl, sh, early, stream);
+    return launch_kernel<QK, XT, T, SPG, kTabE8>(wm, wm2, rp, pl, sh, early, stream);
   } else {
-    if (sh.tt == kTabBf16) return launch_kernel<QK, XT, T, SPG, kTabBf16>(wm, rp, pl, sh, early, stream);
-    if (sh.tt == kTabF16) return launch_kernel<QK, XT, T, SPG, kTabF16>(wm, rp, pl, sh, early, stream);
-    return launch_kernel<QK, XT, T, SPG, kTabF32>(wm, rp, pl, sh, early, stream);
+    if (sh.tt == kTabBf16) return launch_kernel<QK, XT, T, SPG, kTabBf16>(wm, wm2, rp, pl, sh, early, stream);
+    if (sh.tt == kTabF16) return launch_kernel<QK, XT, T, SPG, kTabF16>(wm, wm2, rp, pl, sh, early, stream);
+    return launch_kernel<QK, XT, T, SPG, kTabF32>(wm, wm2, rp, pl, sh, early, stream);
   }
 }
 
 template <int QK, typename XT, int T>
-int launch_spg(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
+int launch_spg(const CUtensorMap& wm, const CUtensorMap& wm2, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
   if constexpr (QK == kMx4) {
-    return launch_tt<QK, XT, T, 1>(wm, rp, pl, sh, early, stream);
+    return launch_tt<QK, XT, T, 1>(wm, wm2, rp, pl, sh, early, stream);
   } else {
-    if (sh.groups == kSliceK / 32) return launch_tt<QK, XT, T, 1>(wm, rp, pl, sh, early, stream);
-    if (sh.groups == kSliceK / 64) return launch_tt<QK, XT, T, 2>(wm, rp, pl, sh, early, stream);
-    return launch_tt<QK, XT, T, 4>(wm, rp, pl, sh, early, stream);
+    if (sh.groups == kSliceK / 32) return launch_tt<QK, XT, T, 1>(wm, wm2, rp, pl, sh, early, stream);
+    if (sh.groups == kSliceK / 64) return launch_tt<QK, XT, T, 2>(wm, wm2, rp, pl, sh, early, stream);
+    return launch_tt<QK, XT, T, 4>(wm, wm2, rp, pl, sh, early, stream);
   }
 }
 
 template <int QK, typename XT>
-int launch_rows_kernel(const CUtensorMap& wm, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
+int launch_rows_kernel(const CUtensorMap& wm, const CUtensorMap& wm2, RowsParams& rp, RowsPlan& pl, const RowsShape& sh, bool early, cudaStream_t stream) {
   if constexpr (sizeof(XT) == 4) {
-    return launch_spg<QK, XT, 4>(wm, rp, pl, sh, early, stream);
+    return launch_spg<QK, XT, 4>(wm, wm2, rp, pl, sh, early, stream);
   } else {
-    return launch_spg<QK, XT, 8>(wm, rp, pl, sh, early, stream);
+    return launch_spg<QK, XT, 8>(wm, wm2, rp, pl, sh, early, stream);
   }
 }
 

@@ -1,5 +1,5 @@
 // One kind of the few-rows kernel: int4 weights, f16 activations (a file of its own so that they compile side by side).
 #include "qmm_rows.cuh"
 
-template int qmm::rows::launch_rows_kernel<qmm::rows::kAff4, __half>(const CUtensorMap&, qmm::rows::RowsParams&, qmm::rows::RowsPlan&,
+template int qmm::rows::launch_rows_kernel<qmm::rows::kAff4, __half>(const CUtensorMap&, const CUtensorMap&, qmm::rows::RowsParams&, qmm::rows::RowsPlan&,
                                                                     const qmm::rows::RowsShape&, bool, cudaStream_t);

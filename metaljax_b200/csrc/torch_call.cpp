@@ -27,6 +27,8 @@ typedef int (*QuantizedMatmul)(const qmm_tensor*, const qmm_tensor*, const qmm_t
                                int, int, int, void*);
 
 typedef int (*SiluMul)(const void*, const void*, void*, int64_t, int, void*);
+typedef int (*GatedMatmul)(const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, qmm_tensor*, int, int, int,
+                           void*);
 typedef int (*PackLayer)(const void*, uint32_t*, const void*, const void*, int, int, void*, void*, int, int64_t, int64_t, int64_t, int, uint64_t*, uint32_t*, void*);
 typedef int64_t (*MoeWorkspace)(const qmm_moe_block*);
 typedef int (*MoeExperts)(const qmm_moe_block*, void*);
@@ -35,6 +37,7 @@ typedef int (*MoeExperts)(const qmm_moe_block*, void*);
 // process, whichever file it was loaded from).
 QuantizedMatmul g_quantized_matmul = nullptr;
 SiluMul g_silu_mul = nullptr;
+GatedMatmul g_gated_matmul = nullptr;
 PackLayer g_pack_layer = nullptr;
 MoeWorkspace g_moe_workspace = nullptr;
 MoeExperts g_moe_experts = nullptr;
@@ -280,6 +283,8 @@ struct Step {
   const at::Tensor *w, *scales, *biases;
   int group_size, bits, mode;
   at::ScalarType dtype;
+  int gate_from, up_from;              // a gate whose two products nothing else reads: their steps, left for it to make (else < 0)
+  bool left;                           // a product that is left for its gate
 };
 
 PyObject* run_steps(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -318,7 +323,8 @@ PyObject* run_steps(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Step& s = steps[i];
     s.x = static_cast<int>(number(0));
     s.result = static_cast<int>(number(1));
-    s.up = -1;
+    s.up = s.gate_from = s.up_from = -1;
+    s.left = false;
     bool fine = argument(s.x) && s.result >= nargs && s.result < count && !known[s.result];
     if (fine && size == 3) {
       s.up = static_cast<int>(number(2));
@@ -359,24 +365,65 @@ PyObject* run_steps(PyObject*, PyObject* const* a, Py_ssize_t n) {
     returns[i] = static_cast<int>(v);
   }
   if (device < 0) Py_RETURN_NONE;
+  // A gate of two products of one x that nothing else reads, of as few rows as the library's one launch for the three takes.
+  std::vector<int> readers(count, 0), maker(count, -1);
+  for (Py_ssize_t i = 0; i < nsteps; ++i) {
+    ++readers[steps[i].x];
+    if (steps[i].up >= 0) ++readers[steps[i].up];
+    maker[steps[i].result] = static_cast<int>(i);
+  }
+  for (int v : returns) ++readers[v];
+  for (Step& s : steps) {
+    if (s.up < 0 || s.x == s.up || !g_gated_matmul || maker[s.x] < 0 || maker[s.up] < 0 || readers[s.x] != 1 || readers[s.up] != 1) continue;
+    Step &g = steps[maker[s.x]], &u = steps[maker[s.up]];
+    const int64_t rows = shapes[s.x][0];
+    if (g.up >= 0 || u.up >= 0 || g.x != u.x || rows < 2 || rows > 16 || g.group_size != u.group_size || g.bits != u.bits || g.mode != u.mode || g.dtype != u.dtype || g.dtype != types[g.x])
+      continue;
+    s.gate_from = maker[s.x];
+    s.up_from = maker[s.up];
+    g.left = u.left = true;
+  }
   std::vector<at::Tensor> made(count);
   const int rc = unlocked([&]() -> int {
     void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
     const at::Device on(at::kCUDA, static_cast<c10::DeviceIndex>(device));
     auto value = [&](int i) -> const at::Tensor& { return given[i] ? *given[i] : made[i]; };
-    for (const Step& s : steps) {
+    auto result = [&](const Step& s) -> at::Tensor& {
       at::Tensor& y = made[s.result];
       y = at::detail::empty_cuda({shapes[s.result][0], shapes[s.result][1]}, types[s.result], on, std::nullopt);
-      const at::Tensor& x = value(s.x);
+      return y;
+    };
+    struct Weight {
+      qmm_tensor w, scales, biases;
+      bool of(const Step& s) { return words_of(*s.w, &w) && view_of(*s.scales, &scales) && (!s.biases || view_of(*s.biases, &biases)); }
+      const qmm_tensor* b(const Step& s) const { return s.biases ? &biases : nullptr; }
+    };
+    auto product = [&](const Step& s) -> int {
+      qmm_tensor vx, vy;
+      Weight weight;
+      if (!view_of(value(s.x), &vx) || !weight.of(s) || !view_of(result(s), &vy)) return kDeclined;
+      return g_quantized_matmul(&vx, &weight.w, &weight.scales, weight.b(s), &vy, 1, s.group_size, s.bits, s.mode, stream);
+    };
+    for (const Step& s : steps) {
+      if (s.left) continue;
       int rc;
-      if (s.up >= 0) {
-        rc = g_silu_mul(x.const_data_ptr(), value(s.up).const_data_ptr(), y.data_ptr(), x.numel(), elem_of(types[s.x]), stream);
-      } else {
-        qmm_tensor vx, vw, vs, vb, vy;
-        if (!view_of(x, &vx) || !words_of(*s.w, &vw) || !view_of(*s.scales, &vs) || (s.biases && !view_of(*s.biases, &vb)) || !view_of(y, &vy)) return kDeclined;
-        rc = g_quantized_matmul(&vx, &vw, &vs, s.biases ? &vb : nullptr, &vy, 1, s.group_size, s.bits, s.mode, stream);
+      if (s.up < 0) {
+        if ((rc = product(s))) return rc;
+        continue;
       }
-      if (rc) return rc;
+      at::Tensor& y = result(s);
+      if (s.gate_from >= 0) {
+        const Step &g = steps[s.gate_from], &u = steps[s.up_from];
+        qmm_tensor vx, vy;
+        Weight gate, up;
+        if (!view_of(value(g.x), &vx) || !gate.of(g) || !up.of(u) || !view_of(y, &vy)) return kDeclined;
+        rc = g_gated_matmul(&vx, &gate.w, &gate.scales, gate.b(g), &up.w, &up.scales, up.b(u), &vy, g.group_size, g.bits, g.mode, stream);
+        if (rc == 0) continue;
+        if (rc != QMM_ERR_UNSUPPORTED) return rc;
+        if ((rc = product(g)) || (rc = product(u))) return rc;
+      }
+      const at::Tensor& x = value(s.x);
+      if ((rc = g_silu_mul(x.const_data_ptr(), value(s.up).const_data_ptr(), y.data_ptr(), x.numel(), elem_of(types[s.x]), stream))) return rc;
     }
     return 0;
   });
@@ -408,9 +455,9 @@ PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   }
 }
 
-// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts_checked[, qmm_moe_silu_mul[, qmm_pack_dense_layer]])
+// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts_checked[, qmm_moe_silu_mul[, qmm_pack_dense_layer[, qmm_gated_matmul]]])
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n < 3 || n > 5) {
+  if (n < 3 || n > 6) {
     PyErr_SetString(PyExc_TypeError, "bind takes the entry points' addresses");
     return nullptr;
   }
@@ -419,6 +466,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   g_moe_experts = reinterpret_cast<MoeExperts>(PyLong_AsVoidPtr(a[2]));
   if (n > 3) g_silu_mul = reinterpret_cast<SiluMul>(PyLong_AsVoidPtr(a[3]));
   if (n > 4) g_pack_layer = reinterpret_cast<PackLayer>(PyLong_AsVoidPtr(a[4]));
+  if (n > 5) g_gated_matmul = reinterpret_cast<GatedMatmul>(PyLong_AsVoidPtr(a[5]));
   if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }

@@ -212,3 +212,38 @@ def test_tiles_of_a_cluster_are_finished_a_lap_late(kind, gs, x, tdt, k, n):
         y = qmm.quantized_matmul(*args, out_dtype=torch.float32, **kw)
     exact = O.qmm_exact(xs, w, s, b, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine"))
     assert O.rel_err(to_numpy(y).astype(np.float32), exact) <= 1e-4
+
+
+@pytest.mark.parametrize("kind,gs,x,tdt", [("int4", 64, "bf16", "bf16"), ("int4", 32, "f16", "f32"), ("int8", 128, "f16", "f16"), ("mxfp4", 32, "bf16", None)])
+@pytest.mark.parametrize("m,k,n", [(2, 128, 1), (8, 512, 16), (5, 1152, 17), (9, 4224, 300), (16, 5632, 40), (3, 640, 2500)])
+def test_two_products_and_their_gate_in_one_launch(kind, gs, x, tdt, m, k, n):
+    """silu(x . Wg) * (x . Wu) with the weights' rows side by side in a tile, against the exact products, gate and all in float64: the results are rounded to 16 bits
+    four times (both products, the gate, their product: 2^-9 each for bf16), and the three launches that it stands for are as far off."""
+    rng = np.random.default_rng(m * k + n)
+    (w, s, b), kw = _case(rng, kind, n, k, gs, tdt)
+    (w2, s2, b2), _ = _case(rng, kind, n, k, gs, tdt)
+    xs = activations(rng, (m, k), x) * np.float32(0.05)
+    xt = to_torch(xs, DEV).to(DT[x])
+    xs = to_numpy(xt).astype(np.float32)
+    y = torch.full((m, n), float("nan"), dtype=DT[x], device=DEV)
+    one, two = ([to_torch(a, DEV) if a is not None else None for a in weight] for weight in ((w, s, b), (w2, s2, b2)))
+    v = _lib.Views()
+    _lib.check(_lib.lib().qmm_gated_matmul(v(xt), *(v(a) for a in one), *(v(a) for a in two), v(y), kw["group_size"], kw["bits"], int(kind == "mxfp4"), torch.cuda.current_stream().cuda_stream))
+    gate = O.qmm_exact(xs, w, s, b, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine")).astype(np.float64)
+    up = O.qmm_exact(xs, w2, s2, b2, kw["group_size"], kw["bits"], mode=kw.get("mode", "affine")).astype(np.float64)
+    assert O.rel_err(to_numpy(y).astype(np.float32), (gate / (1.0 + np.exp(-gate)) * up).astype(np.float32)) <= 1e-2
+    apart = moe.silu_mul(qmm.quantized_matmul(xt, *one, **kw), qmm.quantized_matmul(xt, *two, **kw)) if m <= 8 and m * n % 8 == 0 else None
+    if apart is not None:
+        assert O.rel_err(to_numpy(y).astype(np.float32), to_numpy(apart).astype(np.float32)) <= 1e-2
+
+
+def test_what_one_launch_does_not_take_is_refused():
+    rng = np.random.default_rng(0)
+    (w, s, b), kw = _case(rng, "int4", 64, 256, 64, "bf16")
+    weight = [to_torch(a, DEV) for a in (w, s, b)]
+    for m, x, out in ((1, "bf16", "bf16"), (17, "bf16", "bf16"), (4, "f32", "f32"), (4, "bf16", "f32")):
+        xt, y = torch.zeros((m, 256), dtype=DT[x], device=DEV), torch.zeros((m, 64), dtype=DT[out], device=DEV)
+        v = _lib.Views()
+        before = _lib.lib().qmm_launch_count()
+        assert _lib.lib().qmm_gated_matmul(v(xt), *(v(a) for a in weight), *(v(a) for a in weight), v(y), 64, 4, 0, torch.cuda.current_stream().cuda_stream) == 7
+        assert _lib.lib().qmm_launch_count() == before
