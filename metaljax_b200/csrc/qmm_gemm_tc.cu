@@ -120,9 +120,10 @@ __device__ __forceinline__ uint32_t in_register(uint32_t v) {
 // 4-bit affine, NW packed words -> NW*4 pairs; s2, b2 are scale and bias as pairs of the type.
 //
 // bf16: the even and the odd nibbles of a word under a byte mask each; PRMT takes byte i of either into bytes 0 and 2 of a
-// pair and zeros (their signs) into 1 and 3. A code in the low bits is the subnormal q 2^-133: a product with 2^127 makes it the
-// exact q / 64, and one FMA with (64 s, 64 s), (b, b) rounds once. (Scales below 2^121.) 15 instructions a word, 7 of them on the
-// half-rate logic pipe; with a magic exponent per pair they were 17 and 9.
+// pair and zeros (the sign of the even one's byte) into 1 and 3. A code in bits 0 to 3 is the subnormal q 2^-133, one in bits 4 to 7 q 2^-129 (bit 7 is the first
+// exponent's, where numbers go on as the subnormals do): a product with 2^127 or 2^123 makes it the
+// exact q / 64, and one FMA with (64 s, 64 s), (b, b) rounds once. (Scales below 2^121.) 14 instructions a word, 6 of them on the
+// half-rate logic pipe; with the odd nibbles shifted down 15 and 7, with a magic exponent per pair 17 and 9.
 //
 // f16 has no factor for that: there PRMT takes a byte from the word (even element in its low nibble) into byte 0 and from
 // the word shifted right by four into byte 2, one LOP3 keeps the two nibbles under the magic exponent (1024 + q, exact),
@@ -134,11 +135,11 @@ __device__ __forceinline__ void dequant_aff4(const uint32_t (&w)[NW], uint32_t s
     const uint32_t s64 = H::mul(s2, 0x42804280u);
 #pragma unroll
     for (int j = 0; j < NW; ++j) {
-      const uint32_t even = w[j] & 0x0F0F0F0Fu, odd = (w[j] >> 4) & 0x0F0F0F0Fu;
+      const uint32_t even = w[j] & 0x0F0F0F0Fu, odd = w[j] & 0xF0F0F0F0u;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const uint32_t q = permute(even, odd, i | ((8 + i) << 4) | ((4 + i) << 8) | ((12 + i) << 12));
-        out[j * 4 + i] = H::fma(H::mul(q, 0x7F007F00u), s64, b2);
+        const uint32_t q = permute(even, odd, i | ((8 + i) << 4) | ((4 + i) << 8) | ((8 + i) << 12));
+        out[j * 4 + i] = H::fma(H::mul(q, 0x7D007F00u), s64, b2);
       }
     }
   } else {
