@@ -148,20 +148,30 @@ decode_attention_kernel(const AttnParams p) {
     request_v(lo);
     request_k(lo);
   }
+  // The rotation's angles are known beforehand too (a thread has one pair of every kRotate).
+  constexpr int kHalf = HD / 2, kRotate = ((REP + 1) * kHalf + kAttnThreads - 1) / kAttnThreads;
+  const float inv_sqrt = rsqrtf(static_cast<float>(HD));
+  float sine[kRotate], cosine[kRotate];
+#pragma unroll
+  for (int u = 0; u < kRotate; ++u) {
+    const int j = (tid + u * kAttnThreads) % kHalf;
+    const float freq = exp2f(-2.0f * static_cast<float>(j) / static_cast<float>(HD) * log2f(p.theta));
+    sincosf(static_cast<float>(p.pos) * freq, &sine[u], &cosine[u]);
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   QMM_TRACE(trace, 1);
 
   // ---- rotary embedding of this head group's queries and key (rotate-half pairing), the value ----
-  constexpr int kHalf = HD / 2;
-  const float inv_sqrt = rsqrtf(static_cast<float>(HD));
-  for (int i = tid; i < (REP + 1) * kHalf; i += kAttnThreads) {
+#pragma unroll
+  for (int u = 0; u < kRotate; ++u) {
+    const int i = tid + u * kAttnThreads;
+    if (i >= (REP + 1) * kHalf) break;
     const int h = i / kHalf, j = i - h * kHalf;
     const __nv_bfloat16* src = h < REP ? row + (kvh * REP + h) * HD : row + (p.heads + kvh) * HD;
     const float a = __bfloat162float(src[j]), c = __bfloat162float(src[j + kHalf]);
-    float sn, cs;
-    const float freq = exp2f(-2.0f * static_cast<float>(j) / static_cast<float>(HD) * log2f(p.theta));
-    sincosf(static_cast<float>(p.pos) * freq, &sn, &cs);
-    const float rlo = bf16_round(a * cs - c * sn), rhi = bf16_round(c * cs + a * sn);
+    const float sn = sine[u], cs = cosine[u];
+    // (contracted as the rotary kernel of its own is: the two append the same bits)
+    const float rlo = bf16_round(__fmaf_rn(a, cs, -__fmul_rn(c, sn))), rhi = bf16_round(__fmaf_rn(c, cs, __fmul_rn(a, sn)));
     if (h < REP) {
       q_s[h][j] = rlo * inv_sqrt;
       q_s[h][j + kHalf] = rhi * inv_sqrt;
@@ -305,21 +315,32 @@ decode_attention_kernel(const AttnParams p) {
     mine[tid * kStat + HD] = m_run[tid];
     mine[tid * kStat + HD + 1] = l_run[tid];
   }
-  __threadfence();
   __syncthreads();
   uint32_t* counter = p.counters + b * p.kv_heads + kvh;
   if (tid == 0) {
-    const bool last = atomicAdd(counter, 1u) == static_cast<uint32_t>(p.splits - 1);
+    // (the barrier puts the CTA's stores before this thread's release, and its acquire before the CTA's reads)
+    uint32_t before;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+    const bool last = before == static_cast<uint32_t>(p.splits - 1);
     if (last) *counter = 0;
     is_last = last;
   }
   __syncthreads();
   QMM_TRACE(trace, 4);               // partials published
   if (!is_last) return;
-  __threadfence();
 
   // ---- the last slice of this (row, head) to finish combines them all ----
   const float* all = p.part + (static_cast<int64_t>(b) * p.kv_heads + kvh) * p.splits * REP * kStat;
+  // (the first slices' values are on their way beside what says what they weigh; thread <-> 4 consecutive dimensions)
+  constexpr int kFours = REP * HD / 4, kAhead = 16;
+  static_assert(kFours <= kAttnThreads, "");
+  const int ch = tid / (HD / 4), cd = (tid - ch * (HD / 4)) * 4;
+  float4 ahead[kAhead];
+  if (tid < kFours) {
+#pragma unroll
+    for (int sp = 0; sp < kAhead; ++sp)
+      if (sp < p.splits) ahead[sp] = __ldcg(reinterpret_cast<const float4*>(all + (sp * REP + ch) * kStat + cd));
+  }
   {
     // per head: one warp takes the slices' maxima and sums (lane <-> slice), leaves every slice's
     // weight exp(max_s - max) and the common denominator in shared memory
@@ -350,11 +371,19 @@ decode_attention_kernel(const AttnParams p) {
   __syncthreads();
   const uint32_t stamp = p.push_world > 0
       ? (*reinterpret_cast<const volatile uint32_t*>(p.epoch) << 10) | static_cast<uint32_t>(p.push_site + 1) : 0u;
-  for (int i = tid; i < REP * HD / 4; i += kAttnThreads) {        // thread <-> 4 consecutive dimensions
-    const int h = i / (HD / 4), d0 = (i - h * (HD / 4)) * 4;
+  if (tid < kFours) {
+    const int h = ch, d0 = cd;
     float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int sp = 0; sp < kAhead; ++sp) {
+      if (sp >= p.splits) break;
+      const float4 v = ahead[sp];
+      const float w = wsplit[h][sp];
+      num.x = fmaf(w, v.x, num.x); num.y = fmaf(w, v.y, num.y);
+      num.z = fmaf(w, v.z, num.z); num.w = fmaf(w, v.w, num.w);
+    }
 #pragma unroll 8
-    for (int sp = 0; sp < p.splits; ++sp) {
+    for (int sp = kAhead; sp < p.splits; ++sp) {
       const float4 v = __ldcg(reinterpret_cast<const float4*>(all + (sp * REP + h) * kStat + d0));
       const float w = wsplit[h][sp];
       num.x = fmaf(w, v.x, num.x); num.y = fmaf(w, v.y, num.y);
