@@ -15,6 +15,10 @@
 // (row, head) to finish combines the slices and writes the row. The slice that contains the
 // decode position appends the rotated key and the value to the cache; that position is always
 // taken from shared memory, never read back.
+//
+// What bounds it (one sequence, 2048 positions: 8 MB, 1.3 us of HBM): trips one after another. The angles' sines are taken before the wait for the
+// query row, the publishing of a slice is one release by one thread instead of a fence of every thread, and the last CTA asks for the slices' values beside what they weigh:
+// a step of 32 layers 1998 -> 1927 us.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
