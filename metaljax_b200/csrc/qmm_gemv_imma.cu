@@ -905,10 +905,14 @@ ImmaPlan make_plan(const qmm_problem& p, int nchunks, int plane_bytes, int group
   const size_t kOnePerSm = 226 * 1024;
   const bool small = (p.N + 31) / 32 <= sms;
   for (int pass = 0; pass < 2; ++pass) {
-    // the decode step's linears: sixteen warps, except a weight of at least `big` rows (many
-    // tiles per SM), which streams better from two eight-warp CTAs per SM
+    // the decode step's linears: sixteen warps, except a weight of at least `big` rows that is more than a tile of 32 rows
+    // per SM, or whose rows have no box for each of sixteen warps: it streams better from two eight-warp CTAs per SM.
+    // (One tile per SM of 4096 codes and more is latency, and a kernel that the down projection runs too: a step of 32 layers of 4096 x 4096 attention outputs
+    // 1927 -> 1882 us. Three layers of that width with 6144 and 14336 features 177.5 -> 167.7 and 209.9 -> 202.8; four of width 2048, whose qkv is as many rows of
+    // eight boxes, 136.5 -> 139.5 with sixteen warps. qkv of 6144 rows by sixteen: 1918.)
     static const int big = env_int("QMM_IMMA_FUSED_BIG", 4096);
-    const int nw = fused ? ((p.N >= big && pass == 0) ? 8 : 16)
+    const bool streams = p.N >= big && (p.N > 32 * sms || nchunks < 16);
+    const int nw = fused ? ((streams && pass == 0) ? 8 : 16)
                          : (force_nw ? force_nw : ((pass == 0) == small ? 16 : 8));
     for (int r = 4; r >= 1; r >>= 1) {
       if (force_r && r != force_r) continue;
