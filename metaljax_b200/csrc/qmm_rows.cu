@@ -37,10 +37,10 @@ size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
 // activations with every tile and is left for where nothing else fits. Tiles of one block cost more per row, but an SM that has one tile
 // or two waits less for them (8 rows, mxfp4 5760 x 2880: 2.4 tiles of 16 rows per SM instead of 1.2 -> 2 of 32).
 //
-// The constants were fitted to measured times; what they pick against the best of all plans, us: 8 rows 28672 x 4096 20.1 / 20.1 (the
-// next best 22.0, a cluster of two), 128256 x 4096 65.6 / 65.6 (73.0), 4096 x 14336 16.0 / 16.0 (17.0), 4096 x 4096 7.1 / 7.1 (7.6), 1024 x 1024 5.9 / 5.9,
-// 16 rows 4096 x 4096 8.6 / 8.6 (9.3), 4 rows 5632 x 2048 6.1 / 6.1 (6.6), 2048 x 5632 7.8 / 7.8, 8-bit 8 rows 14336 x 4096 14.6 / 14.6 (15.2),
-// mxfp4 8 rows 5760 x 2880 8.9 / 8.7, float32 33 rows 4096 x 4096 34.8 / 33.2.
+// The constants were fitted to measured times; what they pick against the best of all plans, us (today's kernel): 8 rows 28672 x 4096 18.0 / 18.0 (the
+// next best 20.5), 128256 x 4096 58.0 / 58.0 (72.5), 4096 x 14336 13.9 / 13.9 (17.3), 4096 x 4096 6.0 / 6.0, 1024 x 1024 3.3 / 3.3,
+// 16 rows 4096 x 4096 7.7 / 7.7 (8.5), 4 rows 5632 x 2048 4.8 / 4.8 (5.3), 2048 x 5632 7.1 / 6.8, 8-bit 8 rows 14336 x 4096 13.8 / 13.3,
+// mxfp4 8 rows 5760 x 2880 8.8 / 8.8, float32 4 rows 4096 x 4096 9.1 / 9.1.
 RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh, int segs, bool pair = false) {
   const int sms = device_sm_count();
   RowsPlan best = {};
@@ -115,7 +115,7 @@ bool rows_supports(const qmm_problem& p) {
 // A grouped product of at most 8 rows per expert on average streams its experts' weights here: an even share is one pass of a weight, and what
 // routing makes uneven still costs less than the tensor-core kernel's 64-row tiles. Above it those win, even shares or not. Experts' shares are
 // only known on the device, and a share of n rows passes its weight ceil(n / 8) times: the worst, all rows on one expert, is dearer here from 3 rows an
-// expert on. us here / tensor cores (weights from HBM), even, random and all on one:
+// expert on. us here / tensor cores (weights from HBM; since then this side has become some 10 % faster), even, random and all on one:
 //   rows an expert            4                                    8                                     12
 //   4-bit  8 x 14336 x 4096   75/120   76/120   44/29              77/121   102/121  72/30               129/121  129/121   99/44
 //   4-bit  8 x 4096 x 14336   92/121   84/121   52/62              93/121   127/121  88/64               159/122  158/121  122/64
@@ -197,7 +197,9 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
 }
 
 bool rows_pair_supports(const qmm_problem& p) {
-  return (p.x_dtype == QMM_BF16 || p.x_dtype == QMM_F16) && p.y_dtype == p.x_dtype && !p.lhs_idx && rows_supports(p);
+  if ((p.x_dtype != QMM_BF16 && p.x_dtype != QMM_F16) || p.y_dtype != p.x_dtype || p.lhs_idx || !rows_supports(p)) return false;
+  // (tiles of two blocks alone: 8-bit codes with the widest tables, the longest K and a thousand experts leave no room for them)
+  return plan_rows(1, p.N, static_cast<int>((p.K + kSliceK - 1) / kSliceK), shape_of(p, false), p.group_sizes ? static_cast<int>(p.batch) : 0, true).warps != 0;
 }
 
 int launch_gemv(const qmm_problem& p, cudaStream_t stream) {

@@ -154,3 +154,23 @@ def test_two_threads_at_once():
     for t in threads:
         t.join()
     assert not wrong and _lib.poll_status() == 0
+
+
+@pytest.mark.parametrize("m", [2, 5, 16])
+def test_a_product_that_is_read_twice_keeps_its_launch(m):
+    """The gate's products are one launch with it (m rows of 2 to 16), but not where the program returns one of them as well."""
+    text, args = program(m, 128, 256, torch.bfloat16), arguments(m, 128, 256, torch.bfloat16)
+    first = next(line.split("=")[0].strip() for line in text.splitlines() if "dot_general" in line)
+    mid, out = f"tensor<{m}x256xbf16>", f"tensor<{m}x128xbf16>"
+    last = text.rsplit("return ", 1)[1].split(" ")[0]
+    more = text.replace(f"-> ({out}) {{", f"-> ({mid}, {out}) {{").replace(f"return {last} : {out}", f"return {first}, {last} : {mid}, {out}")
+    counts = []
+    for t in (text, more):
+        taken, got, want = both(t, args)
+        assert taken and all(torch.equal(a, b) for a, b in zip(got, want))
+        it = recognizer.Interpreter(t)
+        it.execute(args)
+        before = _lib.lib().qmm_launch_count()
+        it.execute(args)
+        counts.append(_lib.lib().qmm_launch_count() - before)
+    assert counts == [2, 4]
