@@ -30,8 +30,8 @@
 // Masks and shifts run at half the rate of the issue (16 lanes a clock), so that seven of them in eight codes of a lane are 14 clocks against the
 // MMAs' 8: as bf16 the upper nibble of a byte comes out of its place by a mask and an FMA (below), 10 clocks and 4 of another pipe
 // (8 rows of 128256 x 4096 64.6 -> 58.0 us, with the sums below and accumulators that start from a register quad).
-// The fragments of 16-bit activations are the loaded words, and the groups' sums MMAs of them against ones (element by element in float32 they
-// took 800 instructions a warp, some 2 us of every launch); the sums of bf16 numbers within 2^16 of one another are exact either way.
+// The fragments of 16-bit activations are the loaded words, and the groups' sums float32 additions of them that take a 16-bit operand (with a conversion
+// each they took 800 instructions a warp, some 2 us of every launch).
 // A launch releases its successor in its first instruction: the way from there to the next launch's CTAs bounds the rate of small products (2 rows of 4096 x 4096
 // 6.3 -> 5.5 us, 4 rows of 5632 x 2048 5.7 -> 4.8, 8 rows of 1024 x 1024 4.1 -> 3.3).
 //
@@ -201,6 +201,20 @@ __device__ __forceinline__ uint32_t fma_bf16(uint32_t a, uint32_t b, uint32_t c)
   uint32_t d;
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
   return d;
+}
+
+// a + the lower, + the upper of a pair, rounded after each.
+template <typename AT>
+__device__ __forceinline__ float add_pair(float a, uint32_t pair) {
+  const uint16_t lower = static_cast<uint16_t>(pair), upper = static_cast<uint16_t>(pair >> 16);
+  if constexpr (std::is_same<AT, __half>::value) {
+    asm("add.rn.f32.f16 %0, %1, %0;" : "+f"(a) : "h"(lower));
+    asm("add.rn.f32.f16 %0, %1, %0;" : "+f"(a) : "h"(upper));
+  } else {
+    asm("add.rn.f32.bf16 %0, %1, %0;" : "+f"(a) : "h"(lower));
+    asm("add.rn.f32.bf16 %0, %1, %0;" : "+f"(a) : "h"(upper));
+  }
+  return a;
 }
 
 // The codes under the magic exponent minus (magic + centre): exact.
@@ -617,8 +631,10 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     };
     constexpr int kPer = kSliceK / 32 / kGroups;   // eights per group
     if constexpr (kPieces == 1) {
-      // 16-bit activations: fragments as they are (or scaled), and the groups' sums by MMAs of theirs against ones, which leave them where
-      // the tiles' accumulators want them. (Element by element in float32 this took 800 instructions a warp, 2 us of every launch.)
+      // 16-bit activations: fragments as they are (or scaled), and the groups' sums of them in float32, by additions that take a 16-bit operand and
+      // round. (Conversions and additions of float32 took 800 instructions a warp, 2 us of every launch. MMAs of the fragments against ones are 0.1 us faster in
+      // small launches, but each cuts off: activations of 22 binades and both signs were 14 % further from the exact sums, and 8-bit codes against bf16 spilled
+      // up to 232 bytes, 8 rows of 14336 x 4096 in groups of 64 with f16 tables 16.8 us instead of 13.7.)
       // (all of the lane's elements are asked for at once: a trip to L2 is a third of what this takes)
       constexpr int kPart = kSliceK / 32;
       uint4 v[kPart];
@@ -659,7 +675,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         back[0] = __shfl_sync(0xffffffffu, down, 8 * t);
         back[1] = __shfl_sync(0xffffffffu, down, 8 * t + 4);
       }
-      float total[2];
+      float sum = 0.0f;
 #pragma unroll
       for (int c = 0; c < kPart; ++c) {
         uint32_t u[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
@@ -670,6 +686,17 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
             u[j] = pack2<AT>(f.x * up, f.y * up);
           }
         }
+        if constexpr (QK != kMx4) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) sum = add_pair<AT>(sum, u[j]);
+          if (c % kPer == kPer - 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            // (kept as -C sum x where the group's accumulators start there)
+            if (t < 2) sts32(sums_at + (c / kPer) * 64 + (g >> 1) * 16 + (g & 1) * 4 + t * 8, kSumIs * sum);
+            sum = 0.0f;
+          }
+        }
         arranged(u);
         if constexpr (kQuarters) {               // (what goes with the codes that are (128 + q) / 4)
           u[1] = fma_bf16(u[1], 0x40804080u, 0x80008000u);
@@ -677,21 +704,6 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) xf[c * 4 + j] = u[j];
-        if constexpr (QK != kMx4) {
-          constexpr uint32_t kOnes = std::is_same<AT, __half>::value ? 0x3C003C00u : 0x3F803F80u, kUpper = kQuarters ? 0x3E803E80u : kOnes;
-          const uint32_t ones[4] = {kOnes, kOnes, kUpper, kUpper};
-          const float nought[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-          float lower[4], upper[4];                // (added up in registers, rounded: the tensor core cuts off)
-          Mma<AT>::first(lower, ones, u[0], u[1], nought);
-          Mma<AT>::first(upper, ones, u[2], u[3], nought);
-          total[0] = (c % kPer == 0 ? 0.0f : total[0]) + (lower[0] + upper[0]);
-          total[1] = (c % kPer == 0 ? 0.0f : total[1]) + (lower[1] + upper[1]);
-          if (c % kPer == kPer - 1) {            // (kept as -C sum x where the group's accumulators start there)
-            const int group = c / kPer;
-            const float a = kSumIs * total[0], b = kSumIs * total[1];
-            if (g == (group & 7)) sts128(sums_at + group * 64 + t * 16, a, b, a, b);
-          }
-        }
       }
     } else {
       auto load8 = [&](int c, float (&f)[8]) {

@@ -247,3 +247,36 @@ def test_what_one_launch_does_not_take_is_refused():
         before = _lib.lib().qmm_launch_count()
         assert _lib.lib().qmm_gated_matmul(v(xt), *(v(a) for a in weight), *(v(a) for a in weight), v(y), 64, 4, 0, torch.cuda.current_stream().cuda_stream) == 7
         assert _lib.lib().qmm_launch_count() == before
+
+
+@pytest.mark.parametrize("kind,gs,tdt", [("int4", 32, "f32"), ("int4", 64, "bf16"), ("int8", 64, "f32"), ("int8", 128, "bf16")])
+@pytest.mark.parametrize("x", ["bf16", "f16"])
+@pytest.mark.parametrize("m", [5, 24])
+@pytest.mark.parametrize("style", ["one sign", "outliers", "binades"])
+def test_float32_results_of_uneven_activations(kind, gs, tdt, x, m, style):
+    """Activations of one sign, with one in 97 300 times as large, and of 22 binades. Everything is a product of 16-bit numbers and a float32 sum: what is rounded or cut off is below 2^-24 of what has been
+    added up, (2^bits sum |x| s) at most, over 16 additions one after another in an MMA and K / 512 of them; 24 rows are a gather, which takes the codes without the magic number: sum |x (q - centre)| s."""
+    k, n, bits = 2176, 200, int(kind[3:])
+    rng = np.random.default_rng(gs + m + len(style))
+    (w, s, b), kw = _case(rng, kind, n, k, gs, tdt)
+    xs = activations(rng, (m, k), x).astype(np.float32)
+    if style == "one sign":
+        xs = np.abs(xs)
+    elif style == "outliers":
+        xs[:, ::97] *= 300
+    else:
+        xs = np.sign(xs) * np.exp2(rng.uniform(-12, 10, xs.shape)).astype(np.float32)
+    xt = torch.from_numpy(xs).to(DEV).to(DT[x])
+    wt, st, bt = (to_torch(a, DEV) for a in (w, s, b))
+    if m == 5:
+        with _lib.force_route("gemv_fmma"):
+            y = qmm.quantized_matmul(xt, wt, st, bt, out_dtype=torch.float32, **kw)
+    else:
+        idx = torch.zeros(1, dtype=torch.int32, device=DEV)
+        y = moe.gather_qmm(xt[None], wt[None], st[None], bt[None], idx, idx, out_dtype=torch.float32, **kw)[0]
+    codes = wt.view(torch.uint8).reshape(n, -1)
+    codes = codes if bits == 8 else torch.stack((codes & 15, codes >> 4), -1).reshape(n, k)
+    wide = lambda t: t.double().repeat_interleave(gs, -1)
+    exact = xt.double() @ (codes.double() * wide(st) + wide(bt)).T
+    largest = 2.0 ** (bits if m == 24 else bits + 4 if bits == 4 else bits + 3)               # (a code under the magic number is below 256 or 2048)
+    assert bool(((y.double() - exact).abs() <= (16 + k / 512) * 2.0 ** -24 * largest * (xt.double().abs() @ wide(st).abs().T)).all())
