@@ -342,6 +342,10 @@ int qmm_route(const qmm_problem* problem);
  * owner -- or zeros where another kernel would run. Does not touch the device. */
 int qmm_float32_plan(const qmm_problem* problem, int32_t plan[3]);
 
+/* How the few-rows kernel would share out a problem, and (gated) qmm_gated_matmul one of its two products: 16-row blocks of a tile, CTAs that
+ * share K, warps of a CTA, its ring's slots, CTAs -- or zeros where another kernel would run. Does not touch the device. */
+int qmm_few_rows_plan(const qmm_problem* problem, int gated, int32_t plan[5]);
+
 /* Validates exactly like qmm_quantized_matmul but launches nothing and accepts
  * host tensors: returns the status the real call would give for these shapes and
  * types (device checks excepted). */

@@ -149,6 +149,7 @@ _SIGNATURES = {
                                                                    ctypes.c_int, ctypes.c_int, ctypes.POINTER(Exchange),
                                                                    ctypes.c_void_p]),
     "qmm_route": (ctypes.c_int, [ctypes.POINTER(Problem)]),
+    "qmm_few_rows_plan": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.c_int, ctypes.POINTER(ctypes.c_int32)]),
     "qmm_float32_plan": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.POINTER(ctypes.c_int32)]),
     # include/qmm_ep.h
     "qmm_ep_dispatch": (ctypes.c_int, [ctypes.POINTER(EpExchange), ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,

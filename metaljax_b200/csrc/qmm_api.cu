@@ -439,6 +439,19 @@ int qmm_float32_plan(const qmm_problem* problem, int32_t plan[3]) {
   return QMM_OK;
 }
 
+int qmm_few_rows_plan(const qmm_problem* problem, int gated, int32_t plan[5]) {
+  if (!problem || !plan) return fail(QMM_ERR_NULL, "problem or plan is NULL");
+  int rc = validate_problem(*problem, false);
+  if (rc) return rc;
+  for (int i = 0; i < 5; ++i) plan[i] = 0;
+  const int route = route_of(*problem);
+  if (route < 0) return fail(-route, "the forced kernel family does not support this problem");
+  const bool one_row = !problem->group_sizes && route_override() != QMM_ROUTE_GEMV_FMMA && gemv_imma_supports(*problem);
+  const bool plain = route == QMM_ROUTE_GEMV && !one_row, exact = route == QMM_ROUTE_SIMT && route_override() != QMM_ROUTE_SIMT && !f32_tc_pays(*problem) && rows_supports(*problem);
+  if (gated ? !(plain && rows_pair_supports(*problem)) : !plain && !exact) return QMM_OK;
+  return rows_plan(*problem, exact, gated != 0, plan) ? QMM_OK : fail(QMM_ERR_UNSUPPORTED, "few-rows kernel: no plan fits shared memory");
+}
+
 int qmm_check_quantized_matmul(const qmm_tensor* x, const qmm_tensor* w, const qmm_tensor* scales,
                                const qmm_tensor* biases, const qmm_tensor* y, int transpose,
                                int group_size, int bits, int mode) {

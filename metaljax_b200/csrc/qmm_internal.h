@@ -65,6 +65,7 @@ struct RowsPair {
 int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr, bool exact = false, const RowsPair* pair = nullptr);
 bool rows_pair_supports(const qmm_problem& p);
 bool rows_supports(const qmm_problem& p);
+bool rows_plan(const qmm_problem& p, bool exact, bool pair, int32_t plan[5]);
 double rows_estimate(const qmm_problem& p);      // what a dense product of float32 activations is expected to take here, us
 // Float32 activations of more than a few rows on the tensor cores (f32_tc_pays: it takes them, and wins).
 int launch_f32_tc(const qmm_problem& p, cudaStream_t stream);

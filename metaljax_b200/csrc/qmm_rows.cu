@@ -1,6 +1,8 @@
 // The few-rows kernel's plan and entry points (the kernel itself: qmm_rows.cuh; its instantiations: qmm_rows_*.cu).
 #include "qmm_rows.cuh"
 
+#include <algorithm>
+
 namespace qmm {
 
 using namespace rows;
@@ -22,9 +24,12 @@ QMM_ROWS_EXTERN(kMx4, float)
 namespace {
 
 size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
-  const size_t shares = static_cast<size_t>(pl.blocks) * 512;
-  return 1024 + kHeadBytes +
-         static_cast<size_t>(pl.warps) * (pl.ring * (pl.blocks * sh.stage + table_stage_bytes(pl.blocks, sh.groups, sh.tt)) + pl.red_bufs * shares + sums_bytes(sh.groups) + more_x_bytes(sh.tokens)) +
+  const int qk = sh.tt == kTabE8 ? kMx4 : sh.stage == kBlockRows * kSliceK ? kAff8 : kAff4;
+  const bool quads = table_quads(sh.groups, sh.tt, sh.tokens), twice = sums_twice(qk, sh.groups, sh.tt, sh.exact || sh.tokens == 4);
+  auto own = [&](bool q, bool t) { return pl.ring * (pl.blocks * sh.stage + table_stage_bytes(pl.blocks, sh.groups, sh.tt, q)) + sums_bytes(sh.groups, t); };
+  // (at least what the plainest layout takes: a few hundred bytes decide between plans whose costs are close, and the costs were fitted with these)
+  const size_t shares = static_cast<size_t>(pl.blocks) * 512, warp = std::max(own(quads, twice), own(false, false));
+  return 1024 + kHeadBytes + static_cast<size_t>(pl.warps) * (warp + pl.red_bufs * shares + more_x_bytes(sh.tokens)) +
          (pl.cluster > 1 ? kExchangeSlots * pl.cluster * shares : 0) + (segs ? (2 * static_cast<size_t>(segs) + 1) * 4 : 0);
 }
 
@@ -129,6 +134,23 @@ bool gemv_supports(const qmm_problem& p) {
   return (p.x_dtype == QMM_BF16 || p.x_dtype == QMM_F16) && !p.group_sizes && p.M <= 16 && p.batch <= 65535 && rows_supports(p);
 }
 
+namespace {
+
+// The plan of a problem (grouped: of an even share of its rows for every expert).
+RowsPlan plan_of(const qmm_problem& p, const RowsShape& sh, bool pair) {
+  const int64_t per_seg = p.group_sizes ? (p.M + p.batch - 1) / p.batch : p.M, live = p.group_sizes ? (p.batch < p.M ? p.batch : p.M) : p.batch;
+  return plan_rows(live * ((per_seg + sh.tokens - 1) / sh.tokens), p.N, static_cast<int>((p.K + kSliceK - 1) / kSliceK), sh, p.group_sizes ? static_cast<int>(p.batch) : 0, pair);
+}
+
+}  // namespace
+
+bool rows_plan(const qmm_problem& p, bool exact, bool pair, int32_t plan[5]) {
+  const RowsPlan pl = plan_of(p, shape_of(p, exact), pair);
+  const int32_t of[5] = {pl.blocks, pl.cluster, pl.warps, pl.ring, pl.grid};
+  for (int i = 0; i < 5; ++i) plan[i] = of[i];
+  return pl.warps != 0;
+}
+
 int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather, bool exact, const RowsPair* pair) {
   RowsParams rp = {};
   rp.x = p.x; rp.scales = p.scales; rp.biases = p.biases; rp.y = p.y;
@@ -153,18 +175,15 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
   rp.groups = rp.K / group;
   rp.weight_rows = (p.rhs_idx || p.group_sizes || p.w_batch_stride) ? rp.N : 0;
   rp.table_dtype = p.table_dtype; rp.y_dtype = p.y_dtype;
-  const int slices = (rp.K + kSliceK - 1) / kSliceK;
   const RowsShape sh = shape_of(p, exact);
   const int chunk = sh.tokens;
-  const int64_t per_seg = p.group_sizes ? (p.M + p.batch - 1) / p.batch : p.M;      // grouped: of an average expert
-  const int64_t live = p.group_sizes ? (p.batch < p.M ? p.batch : p.M) : p.batch;
   const int entry = mx ? 1 : (p.table_dtype == QMM_F32 ? 4 : 2);
   const int64_t nweights = p.num_weights > 0 ? p.num_weights : (p.w_batch_stride ? p.batch : 1);
   rp.table_bytes = nweights * p.N * rp.groups * entry;
   // (a slice's entries start on the units that its own row of entries and a row of the table are multiples of)
   const int slice_bytes = sh.groups * entry, row_bytes_t = rp.groups * entry;
   rp.table_unit = (row_bytes_t | slice_bytes) % 8 == 0 && row_bytes_t % slice_bytes == 0 ? (slice_bytes % 16 == 0 ? 16 : 8) : (row_bytes_t | slice_bytes) % 4 == 0 ? 4 : 1;
-  RowsPlan pl = plan_rows(live * ((per_seg + chunk - 1) / chunk), rp.N, slices, sh, p.group_sizes ? rp.segs : 0, pair != nullptr);
+  RowsPlan pl = plan_of(p, sh, pair != nullptr);
   if (!pl.warps) return fail(QMM_ERR_UNSUPPORTED, "few-rows kernel: no plan fits shared memory");
   const int tile_rows = pair ? kBlockRows : kBlockRows * pl.blocks;
   rp.tiles = (rp.N + tile_rows - 1) / tile_rows;
@@ -199,7 +218,7 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
 bool rows_pair_supports(const qmm_problem& p) {
   if ((p.x_dtype != QMM_BF16 && p.x_dtype != QMM_F16) || p.y_dtype != p.x_dtype || p.lhs_idx || !rows_supports(p)) return false;
   // (tiles of two blocks alone: 8-bit codes with the widest tables, the longest K and a thousand experts leave no room for them)
-  return plan_rows(1, p.N, static_cast<int>((p.K + kSliceK - 1) / kSliceK), shape_of(p, false), p.group_sizes ? static_cast<int>(p.batch) : 0, true).warps != 0;
+  return plan_of(p, shape_of(p, false), true).warps != 0;
 }
 
 int launch_gemv(const qmm_problem& p, cudaStream_t stream) {

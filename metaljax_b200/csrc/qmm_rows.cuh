@@ -109,7 +109,7 @@ struct RowsParams {
   int cluster, slices_per_cta, slices_per_warp;
   unsigned share, share_more;    // dense: (chunk, tile) items of every cluster, and how many clusters have one more
   int ring, red_bufs;
-  int table_unit;                // bytes on which every row's table entries of every slice start: 8, 4, or less
+  int table_unit;                // bytes on which every row's table entries of every slice start: 16, 8, 4, or less
   int64_t table_bytes;           // of a whole table
   int64_t total_x_rows;          // grouped: rows of x that x_rows may name
   const void* scales2;           // a pair of weights of one shape (two blocks): block 0 of a tile is 16 rows of the first, block 1 the same
@@ -292,15 +292,23 @@ static_assert(sizeof(Place) <= kStateBytes, "");
 // 16-row blocks of a tile: two halve what a tile costs apart from its codes, one halves the wait for a lone tile (plan_rows).
 constexpr int kMaxBlocks = 2;
 
-// A tile's table entries travel with its codes: per weight row the slice's entries as they are in memory, at a pitch
-// that 8-byte copies and conflict-free 4-byte reads allow, with a word to spare for entries that do not start
-// on a word.
+// A tile's table entries travel with its codes: per weight row the slice's entries as they are in memory, so far apart that reads of a word of eight rows meet
+// all banks, with a word to spare for entries that do not start on a word. QUADS (affine tables of 16-bit activations): rows of 16 bytes and more lie on
+// multiples of 16, for one copy to take that many, every few rows another 16 bytes further on, and the spare words behind the rows. The others are copied by
+// eights at most: a fourth way to copy cost float32 and MXFP4 kernels registers. (A pitch of the row and 16 bytes for all of them took memory that rings and
+// plans were made of: steps of 2 sequences 251 -> 271 us, float32 against 8-bit codes 28480 x 2048 17.3 -> 25.7, 8 rows of 4096 x 28672 16.8 as now; with eights alone 17.4.)
 constexpr int table_row_bytes(int groups, int tt) { return groups * entry_bytes(tt); }
-constexpr int table_pitch(int groups, int tt) { return table_row_bytes(groups, tt) == 4 ? 8 : table_row_bytes(groups, tt) == 8 ? 16 : table_row_bytes(groups, tt) + 16; }
-// (16 bytes at a pitch of 32: every four rows another 16 further on, for their reads to meet all banks)
-constexpr int table_at(int row, int groups, int tt) { return row * table_pitch(groups, tt) + (table_row_bytes(groups, tt) == 16 ? (row >> 2) * 16 : 0); }
-constexpr int table_stage_bytes(int blocks, int groups, int tt) { return table_at(kBlockRows * blocks, groups, tt) * (tt == kTabE8 ? 1 : 2); }
-constexpr int sums_bytes(int groups) { return groups * 64; }      // a pair of columns twice: what an accumulator of two rows starts at
+constexpr bool table_quads(int groups, int tt, int tokens) { return tokens == 8 && tt != kTabE8 && table_row_bytes(groups, tt) >= 16; }
+constexpr int table_at(int row, int groups, int tt, bool quads) {
+  const int bytes = table_row_bytes(groups, tt);
+  return quads ? row * bytes + (bytes == 32 ? (row >> 2) * 16 : bytes == 64 ? (row >> 1) * 16 : 0) : row * (bytes == 8 ? 16 : bytes + 8);
+}
+constexpr int table_bytes(int rows, int groups, int tt, bool quads) { return table_at(rows, groups, tt, quads) + (quads && entry_bytes(tt) < 4 ? rows * 4 : 0); }
+constexpr int table_stage_bytes(int blocks, int groups, int tt, bool quads) { return table_bytes(kBlockRows * blocks, groups, tt, quads) * (tt == kTabE8 ? 1 : 2); }
+// The groups' sums of a slice's columns; a pair of columns twice where accumulators of two rows start there (one read, no moves, and no spills: 16-bit tables in groups of
+// 32 11 % slower without), but not where no plan has the memory for it.
+constexpr bool sums_twice(int qk, int groups, int tt, bool centred) { return qk != kMx4 && !centred && !(groups == 16 && tt == kTabF32) && !(qk == kAff8 && groups == 4 && tt != kTabF32); }
+constexpr int sums_bytes(int groups, bool twice) { return groups * (twice ? 64 : 32); }
 // Fragments of a second column group (the third piece of float32): they would not fit the registers.
 constexpr int more_x_bytes(int tokens) { return tokens == 8 ? 0 : kSliceK * 16; }
 
@@ -347,9 +355,11 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   constexpr int kBiasMmas = kGroups == 16 ? 3 : kGroups == 8 ? 2 : 1;
   constexpr int kEntry = entry_bytes(TT);
   constexpr int kRowBytes = table_row_bytes(kGroups, TT);             // a weight row's table entries in a slice
-  constexpr int kTable = table_at(kTileRows, kGroups, TT);            // one table of a tile
-  constexpr int kEight = table_at(8, kGroups, TT);                    // its next eight rows
-  constexpr int kSlot = kStage + table_stage_bytes(R, kGroups, TT);   // codes, scales, biases: a place of the ring
+  constexpr bool kQuads = table_quads(kGroups, TT, T), kTwice = sums_twice(QK, kGroups, TT, kCentred);
+  constexpr int kSums = sums_bytes(1, kTwice);                        // the columns' sums of a group
+  constexpr int kTable = table_bytes(kTileRows, kGroups, TT, kQuads); // one table of a tile
+  constexpr int kEight = table_at(8, kGroups, TT, kQuads);            // its next eight rows
+  constexpr int kSlot = kStage + table_stage_bytes(R, kGroups, TT, kQuads);   // codes, scales, biases: a place of the ring
   constexpr float kUnit = QK == kMx4 ? 16384.0f : kNibbles && kCentred ? 64.0f : 1.0f;               // (the E2M1 fragments are the values times 2^-14)
 
   // The next launch may be made ready from here on: it touches nothing of this one's before its own wait, and the way from here to its CTAs' start is what
@@ -370,9 +380,9 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   const uint32_t red_at = smem + kHeadBytes + warps * p.ring * kSlot;                           // [bufs][warps][R][32] float4
   const uint32_t xbuf_at = red_at + p.red_bufs * warps * R * 512;                          // [slots][cluster][R][32] float4
   const uint32_t own_at = xbuf_at + (csize > 1 ? kExchangeSlots * csize * R * 512 : 0);
-  const uint32_t sums_at = own_at + warp * sums_bytes(kGroups);                              // [warps] sums of x
-  const uint32_t more_x_at = own_at + warps * sums_bytes(kGroups) + warp * more_x_bytes(T) + lane * 16;      // [warps][MMA pairs][32] 16 bytes
-  const uint32_t segs_at = own_at + warps * (sums_bytes(kGroups) + more_x_bytes(T));         // grouped: [segs] chunks, [segs + 1] first rows
+  const uint32_t sums_at = own_at + warp * sums_bytes(kGroups, kTwice);                              // [warps] sums of x
+  const uint32_t more_x_at = own_at + warps * sums_bytes(kGroups, kTwice) + warp * more_x_bytes(T) + lane * 16;      // [warps][MMA pairs][32] 16 bytes
+  const uint32_t segs_at = own_at + warps * (sums_bytes(kGroups, kTwice) + more_x_bytes(T));         // grouped: [segs] chunks, [segs + 1] first rows
   int* seg_chunks = reinterpret_cast<int*>(rows_smem_raw + (segs_at - smem_u32(rows_smem_raw)));
   int* seg_row = seg_chunks + p.segs;
   uint8_t* head = rows_smem_raw + (smem - smem_u32(rows_smem_raw));
@@ -489,7 +499,9 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   constexpr bool kBothTables = R == 2 || TT == kTabE8;
   const int table_row = kTileRows == 32 ? lane : lane & 15, table_row_size = p.groups * kEntry;
   const uint8_t* my_table = static_cast<const uint8_t*>(kBothTables || lane < 16 ? p.scales : p.biases);
-  const uint32_t my_tables = tables_at + table_at(table_row, kGroups, TT) + (kBothTables || lane < 16 ? 0 : kTable);
+  // (where the word behind a row's entries goes)
+  const int spare = kQuads && kEntry < 4 ? table_at(kTileRows, kGroups, TT, kQuads) + table_row * 4 - table_at(table_row, kGroups, TT, kQuads) : kRowBytes;
+  const uint32_t my_tables = tables_at + table_at(table_row, kGroups, TT, kQuads) + (kBothTables || lane < 16 ? 0 : kTable);
   auto request = [&]() {               // the whole warp; ahead_left > 0
     const uint32_t bar = my_full + ahead_slot * 8;
     const int slice = first_slice + ahead_sub;
@@ -510,12 +522,13 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
       const uint32_t dst = my_tables + ahead_slot * (kSlot - kStage);
       auto copy = [&](const uint8_t* table, uint32_t to) {
         const uint8_t* src = table + at;
-        if (p.table_unit == 16 && kRowBytes >= 16) {
+        constexpr int kWhole = kQuads ? 16 : 8;
+        if (p.table_unit >= kWhole && kRowBytes >= kWhole) {
 #pragma unroll
-          for (int i = 0; i < kRowBytes; i += 16) cp_async16(to + i, src + i);
-        } else if (p.table_unit >= 8 && kRowBytes >= 8) {
-#pragma unroll
-          for (int i = 0; i < kRowBytes; i += 8) cp_async8(to + i, src + i);
+          for (int i = 0; i < kRowBytes; i += kWhole) {
+            if constexpr (kQuads) cp_async16(to + i, src + i);
+            else cp_async8(to + i, src + i);
+          }
         } else if (p.table_unit >= 4) {
 #pragma unroll
           for (int i = 0; i < kRowBytes; i += 4) cp_async4(to + i, slice * kGroups * kEntry + i < table_row_size ? src + i : src);
@@ -524,7 +537,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
 #pragma unroll
           for (int i = 0; i <= kRowBytes; i += 4) {
             const int64_t room = p.table_bytes - (at - skew + i);
-            cp_async4(to + i, room > 0 ? src - skew + i : src - skew, room >= 4 ? 4 : room > 0 ? static_cast<int>(room) : 0);
+            cp_async4(to + (i < kRowBytes ? i : spare), room > 0 ? src - skew + i : src - skew, room >= 4 ? 4 : room > 0 ? static_cast<int>(room) : 0);
           }
         }
       };
@@ -630,6 +643,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
       }
     };
     constexpr int kPer = kSliceK / 32 / kGroups;   // eights per group
+    auto sum_at = [](int column) -> int { return kTwice ? (column >> 1) * 16 + (column & 1) * 4 : column * 4; };
     if constexpr (kPieces == 1) {
       // 16-bit activations: fragments as they are (or scaled), and the groups' sums of them in float32, by additions that take a 16-bit operand and
       // round. (Conversions and additions of float32 took 800 instructions a warp, 2 us of every launch. MMAs of the fragments against ones are 0.1 us faster in
@@ -693,7 +707,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
             // (kept as -C sum x where the group's accumulators start there)
-            if (t < 2) sts32(sums_at + (c / kPer) * 64 + (g >> 1) * 16 + (g & 1) * 4 + t * 8, kSumIs * sum);
+            if (t < (kTwice ? 2 : 1)) sts32(sums_at + (c / kPer) * kSums + sum_at(g) + t * 8, kSumIs * sum);
             sum = 0.0f;
           }
         }
@@ -763,7 +777,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
               sum += __shfl_xor_sync(0xffffffffu, sum, 1);
               sum += __shfl_xor_sync(0xffffffffu, sum, 2);
               // (kept as -C sum x where the group's accumulators start there)
-              if (t < 2) sts32(sums_at + (c / kPer) * 64 + (g >> 1) * 16 + (g & 1) * 4 + t * 8, kSumIs * sum);
+              if (t < (kTwice ? 2 : 1)) sts32(sums_at + (c / kPer) * kSums + sum_at(g) + t * 8, kSumIs * sum);
               sum = 0.0f;
             }
           }
@@ -812,7 +826,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
       // 8 groups -- (hi | mid) and (lo | 0) with lane t's groups 2t, 2t + 1; 4 groups -- lanes t < 2 (hi | mid), t >= 2 (lo | 0)
       // with groups 2 (t & 1), 2 (t & 1) + 1
       auto pick = [&](int first) -> float {        // sum of x of column g in group first + 2 t
-        return __uint_as_float(lds32<0>(sums_at + (first + 2 * (kGroups == 4 ? t & 1 : t)) * 64 + (g >> 1) * 16 + (g & 1) * 4)) * (1.0f / kSumIs);
+        return __uint_as_float(lds32<0>(sums_at + (first + 2 * (kGroups == 4 ? t & 1 : t)) * kSums + sum_at(g))) * (1.0f / kSumIs);
       };
       using B16 = __nv_bfloat16;
       auto split = [&](float a, float b, uint32_t (&piece)[3]) {
@@ -848,7 +862,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   uint32_t nib_mask = std::is_same<AT, __half>::value ? 0x03C003C0u : 0x000F000Fu, magic = kMagic;
   [[maybe_unused]] uint32_t upper_mask = 0x00F000F0u, times = 0x7F007F00u;       // (2^127)
   asm volatile("" : "+r"(nib_mask), "+r"(magic));                      // constants in registers: one LOP3 per use
-  const uint32_t tthread = tables_at + table_at(rho, kGroups, TT), scol = sums_at + 16 * t;
+  const uint32_t tthread = tables_at + table_at(rho, kGroups, TT, kQuads), scol = sums_at + (kTwice ? 16 : 8) * t;
   int turn = 0, which = 0, tile = tile0, sub = 0, count = 0;
   uint32_t slot = 0, slot_phase = 0, buf = 0, buf_phase = 0;
   // the tile that is to be added up next
@@ -989,12 +1003,12 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         uint32_t word = lds32<0>(at);
 #pragma unroll
         for (int i = 0; i < kRowBytes; i += 4) {
-          const uint32_t next = lds32<0>(at + i + 4);
+          const uint32_t next = lds32<0>(at + (i + 4 < kRowBytes ? i + 4 : spare));
           sts32(at + i, __uint_as_float(__funnelshift_r(word, next, skew)));
           word = next;
         }
       };
-      const uint32_t at = tables_at + slot * (kSlot - kStage) + table_at(row, kGroups, TT);
+      const uint32_t at = tables_at + slot * (kSlot - kStage) + table_at(row, kGroups, TT, kQuads);
       if (R == 2 || TT == kTabE8) {
         if (kTileRows == 32 || lane < 16) straighten(at);
         if (TT != kTabE8) straighten(at + kTable);
@@ -1042,7 +1056,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     fetch(std::integral_constant<int, 0>(), cw[0]);
     static_for<2>([&](auto hc) {
       constexpr int half = decltype(hc)::value;
-      const uint32_t thalf = trow + half * (kHalfGroups * kEntry), shalf = scol + half * (kHalfGroups * 64);
+      const uint32_t thalf = trow + half * (kHalfGroups * kEntry), shalf = scol + half * (kHalfGroups * kSums);
       float acc[R][NT][4], start[4];
       constexpr bool kStarts = QK != kMx4 && !kCentred;
       const float nought[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -1071,8 +1085,13 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
           constexpr int kPerGroup = 2 * SPG, at = q * 4 + m, gi = at / kPerGroup;      // MMAs of a group; MMA and group of the half
           constexpr bool kFirst = at % kPerGroup == 0, kLast = at % kPerGroup == kPerGroup - 1;
           if constexpr (kFirst && QK != kMx4) {    // kSumIs * sum x of the group
-            const float4 sr = ldsf128<gi * 64>(shalf);
-            start[0] = sr.x; start[1] = sr.y; start[2] = sr.z; start[3] = sr.w;
+            if constexpr (kTwice) {
+              const float4 sr = ldsf128<gi * kSums>(shalf);
+              start[0] = sr.x; start[1] = sr.y; start[2] = sr.z; start[3] = sr.w;
+            } else {
+              const uint2 sr = lds64<gi * kSums>(shalf);
+              start[0] = start[2] = __uint_as_float(sr.x); start[1] = start[3] = __uint_as_float(sr.y);
+            }
           }
           if constexpr (NT > 1 && m % 2 == 0) more = lds128<((qq * 4 + m) / 2) * 512>(more_x_at);
           static_for<R>([&](auto rc) {

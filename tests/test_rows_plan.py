@@ -1,0 +1,33 @@
+"""How the few-rows kernel shares a product out, asked without a device (on a machine of 148 SMs)."""
+
+import pytest
+import torch
+
+from metaljax_b200 import _lib, qmm
+
+BF16, F16, F32 = torch.bfloat16, torch.float16, torch.float32
+
+
+def plan(*args, gated=0, **kw):
+    out = (_lib.ctypes.c_int32 * 5)(7, 7, 7, 7, 7)
+    _lib.check(_lib.lib().qmm_few_rows_plan(_lib.ctypes.byref(qmm._problem(*args, **kw)), gated, out))
+    return tuple(out)
+
+
+@pytest.mark.parametrize("m,k,n,kw,want", [
+    (2, 4096, 24576, dict(), (2, 1, 8, 2, 148)),                                                       # two sequences' gate and up, four CTAs of two warps a tile instead: 8 % of a step
+    (1, 2048, 28480, dict(bits=8, x_dtype=F32, table_dtype=BF16), (1, 1, 4, 2, 296)),                    # 17.3 us, with clusters of two 25.7
+    (1, 4096, 14336, dict(bits=8, x_dtype=F32, table_dtype=BF16), (1, 1, 8, 2, 148)),                    # 18.2 / 25.8
+    (2, 14208, 3164, dict(group_size=128, x_dtype=F32), (2, 4, 7, 2, 148)),                              # 17.2 / 18.3 with tiles of 16 rows
+    (48, 2816, 8576, dict(group_size=128, bits=8, batch=8, ragged=True), (2, 1, 6, 2, 148)),             # 48 rows of 8 experts: the block 169 / 196 us
+])
+def test_the_memory_of_tables_and_sums_leaves_the_plan(m, k, n, kw, want):
+    """Plans that a few hundred bytes more per warp had changed for slower ones."""
+    assert plan(m, k, n, **kw) == want
+
+
+def test_what_has_no_plan():
+    assert plan(1, 4096, 4096) == (0, 0, 0, 0, 0)                          # one row: another kernel's
+    assert plan(17, 4096, 4096) == (0, 0, 0, 0, 0)                         # the tensor cores'
+    assert plan(8, 4096, 4096, gated=1) != (0, 0, 0, 0, 0) == plan(8, 4096, 4096, gated=1, x_dtype=F32)
+    assert _lib.lib().qmm_few_rows_plan(None, 0, (_lib.ctypes.c_int32 * 5)()) == 1
