@@ -42,6 +42,10 @@ size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
 // activations with every tile and is left for where nothing else fits. Tiles of one block cost more per row, but an SM that has one tile
 // or two waits less for them (8 rows, mxfp4 5760 x 2880: 2.4 tiles of 16 rows per SM instead of 1.2 -> 2 of 32).
 //
+// Clusters of CTAs of one or two warps, three or four CTAs on an SM, cost more than the load says, and whether one of them came out ahead hung on the tables' bytes: 8 rows,
+// float32 against MXFP4 28480 x 2048 49.9 us as 222 clusters of two, 31.4 as tiles of whole K; 2 rows 24512 x 4096 in groups of 32 26.0 / 17.2; 22464 x 7680 mxfp4 53.4 / 35.4.
+// Of 56 shapes where such a plan had the least load none was the faster for it.
+//
 // The constants were fitted to measured times; what they pick against the best of all plans, us (today's kernel): 8 rows 28672 x 4096 18.0 / 18.0 (the
 // next best 20.5), 128256 x 4096 58.0 / 58.0 (72.5), 4096 x 14336 13.9 / 13.9 (17.3), 4096 x 4096 6.0 / 6.0, 1024 x 1024 3.3 / 3.3,
 // 16 rows 4096 x 4096 7.7 / 7.7 (8.5), 4 rows 5632 x 2048 4.8 / 4.8 (5.3), 2048 x 5632 7.1 / 6.8, 8-bit 8 rows 14336 x 4096 13.8 / 13.3,
@@ -62,6 +66,7 @@ RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh
       if (pl.slices_per_warp > 1 && c < kMaxCluster) continue;        // (reloading activations per tile: only where nothing else is left)
       pl.warps = (pl.slices_per_cta + pl.slices_per_warp - 1) / pl.slices_per_warp;
       pl.slices_per_cta = pl.warps * pl.slices_per_warp;
+      if (c > 1 && pl.warps < 3) continue;                            // (see above)
       int per_sm = kMaxWarps / pl.warps;
       if (per_sm > 4) per_sm = 4;
       pl.ring = kMaxRing;
