@@ -342,6 +342,10 @@ int qmm_route(const qmm_problem* problem);
  * owner -- or zeros where another kernel would run. Does not touch the device. */
 int qmm_float32_plan(const qmm_problem* problem, int32_t plan[3]);
 
+/* 1 if qmm_gated_matmul takes two products like this one and their gate and is expected to be no slower than the three launches, else 0.
+ * Sizes and types alone are looked at. */
+int qmm_gated_matmul_pays(const qmm_problem* product);
+
 /* How the few-rows kernel would share out a problem, and (gated) qmm_gated_matmul one of its two products: 16-row blocks of a tile, CTAs that
  * share K, warps of a CTA, its ring's slots, CTAs -- or zeros where another kernel would run. Does not touch the device. */
 int qmm_few_rows_plan(const qmm_problem* problem, int gated, int32_t plan[5]);

@@ -149,6 +149,7 @@ _SIGNATURES = {
                                                                    ctypes.c_int, ctypes.c_int, ctypes.POINTER(Exchange),
                                                                    ctypes.c_void_p]),
     "qmm_route": (ctypes.c_int, [ctypes.POINTER(Problem)]),
+    "qmm_gated_matmul_pays": (ctypes.c_int, [ctypes.POINTER(Problem)]),
     "qmm_few_rows_plan": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.c_int, ctypes.POINTER(ctypes.c_int32)]),
     "qmm_float32_plan": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.POINTER(ctypes.c_int32)]),
     # include/qmm_ep.h
@@ -194,7 +195,7 @@ def native():
         loader.exec_module(module)
         module.bind(*(ctypes.cast(getattr(lib(), name), ctypes.c_void_p).value for name in ("qmm_quantized_matmul", "qmm_moe_workspace_bytes",
                                                                                              "qmm_moe_experts_checked", "qmm_moe_silu_mul", "qmm_pack_dense_layer",
-                                                                                             "qmm_gated_matmul")))
+                                                                                             "qmm_gated_matmul", "qmm_gated_matmul_pays")))
         _native = module
     return _native
 

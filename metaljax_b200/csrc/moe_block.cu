@@ -260,7 +260,8 @@ static int enqueue_block(const qmm_moe_block* block, void* stream, const Report&
     count_launch();
   }
   if ((rc = check_launch("moe_sort_kernel"))) return rc;
-  if (gathered && rows_pair_supports(gate)) {      // both products and the gate as one launch
+  const bool paired = gathered && rows_pair_pays(gate);
+  if (paired) {                                    // both products and the gate as one launch
     const RowsPair second = {up.w, up.scales, up.biases};
     if ((rc = launch_rows(gate, st, &pick, false, &second))) return rc;
   } else if (gathered) {
@@ -268,7 +269,7 @@ static int enqueue_block(const qmm_moe_block* block, void* stream, const Report&
   } else {
     if ((rc = run_problem(gate, st)) || (rc = run_problem(up, st))) return rc;
   }
-  if (!(gathered && rows_pair_supports(gate)) && (rc = qmm_moe_silu_mul(base + ws.gate, base + ws.up, base + ws.gate, pairs * b.ffn, b.x_dtype, stream))) return rc;
+  if (!paired && (rc = qmm_moe_silu_mul(base + ws.gate, base + ws.up, base + ws.gate, pairs * b.ffn, b.x_dtype, stream))) return rc;
   if ((rc = run_problem(down, st))) return rc;
   return qmm_moe_routed_sum(base + ws.down, rows, b.weights, b.out, b.tokens, b.k, b.d, pairs, b.x_dtype, stream);
 }

@@ -472,6 +472,10 @@ int qmm_gated_matmul(const qmm_tensor* x, const qmm_tensor* gate_w, const qmm_te
   return launch_rows(gate, static_cast<cudaStream_t>(stream), nullptr, false, &second);
 }
 
+int qmm_gated_matmul_pays(const qmm_problem* p) {
+  return p && !validate_problem(*p, false) && p->batch == 1 && p->M >= 2 && p->K > 0 && !p->group_sizes && route_of(*p) == QMM_ROUTE_GEMV && rows_pair_pays(*p);
+}
+
 int qmm_quantized_matmul(const qmm_tensor* x, const qmm_tensor* w, const qmm_tensor* scales,
                          const qmm_tensor* biases, qmm_tensor* y, int transpose, int group_size,
                          int bits, int mode, void* stream) {

@@ -64,6 +64,7 @@ struct RowsPair {
 };
 int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gather = nullptr, bool exact = false, const RowsPair* pair = nullptr);
 bool rows_pair_supports(const qmm_problem& p);
+bool rows_pair_pays(const qmm_problem& p);       // ... and is no slower than the two products and the gate
 bool rows_supports(const qmm_problem& p);
 bool rows_plan(const qmm_problem& p, bool exact, bool pair, int32_t plan[5]);
 double rows_estimate(const qmm_problem& p);      // what a dense product of float32 activations is expected to take here, us

@@ -220,10 +220,27 @@ int launch_rows(const qmm_problem& p, cudaStream_t stream, const RowsGather* gat
   return launch(std::integral_constant<int, kAff4>());
 }
 
-bool rows_pair_supports(const qmm_problem& p) {
-  if ((p.x_dtype != QMM_BF16 && p.x_dtype != QMM_F16) || p.y_dtype != p.x_dtype || p.lhs_idx || !rows_supports(p)) return false;
-  // (tiles of two blocks alone: 8-bit codes with the widest tables, the longest K and a thousand experts leave no room for them)
-  return plan_of(p, shape_of(p, false), true).warps != 0;
+namespace {
+
+bool pair_takes(const qmm_problem& p) { return (p.x_dtype == QMM_BF16 || p.x_dtype == QMM_F16) && p.y_dtype == p.x_dtype && !p.lhs_idx && rows_supports(p); }
+
+}  // namespace
+
+// (tiles of two blocks alone: 8-bit codes with the widest tables, the longest K and a thousand experts leave no room for them)
+bool rows_pair_supports(const qmm_problem& p) { return pair_takes(p) && plan_of(p, shape_of(p, false), true).warps != 0; }
+
+// 4-bit codes have the same tiles either way: one launch took 0.64 of the time of two products and the gate on average of 39 shapes (MXFP4 0.70 of 44, but 14016 x 7296 101 us against
+// 92); dense ones always have a plan, and are not asked for it. Of 8-bit codes tiles of two blocks, 16 rows of each weight, leave two slots of a ring or half the warps, and then two products
+// in plans of their own are the faster. By the plans' loads (one is some 0.35 us): expert blocks, us as one launch / two, by what one has more than twice the other: 16 of 8 experts 2816 -> 8576
+// 1.00 93 / 101, 14 of 32 3328 -> 4736 1.57 189 / 153, 2 of 16 2688 -> 6528 1.89 78 / 58, 6 of 8 896 -> 5888 1.32 59 / 48. Dense ones save two launches, 18 of these units or less: 2 rows
+// 1280 -> 11080 +14 11.8 / 14.3, 9 rows 3200 -> 3944 +22 30.3 / 25.4, 16 rows 2048 -> 13192 +26 26.4 / 28.8, 4 rows 3968 -> 14720 +30 37.4 / 32.7.
+bool rows_pair_pays(const qmm_problem& p) {
+  if (!pair_takes(p)) return false;
+  const bool eight = p.mode != QMM_MODE_MXFP4 && p.bits == 8;
+  if (!eight && !p.group_sizes) return true;
+  const RowsShape sh = shape_of(p, false);
+  const RowsPlan one = plan_of(p, sh, true);
+  return one.warps && (!eight || one.load <= 2.0 * plan_of(p, sh, false).load + (p.group_sizes ? 0.0 : 18.0));
 }
 
 int launch_gemv(const qmm_problem& p, cudaStream_t stream) {

@@ -29,6 +29,7 @@ typedef int (*QuantizedMatmul)(const qmm_tensor*, const qmm_tensor*, const qmm_t
 typedef int (*SiluMul)(const void*, const void*, void*, int64_t, int, void*);
 typedef int (*GatedMatmul)(const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, const qmm_tensor*, qmm_tensor*, int, int, int,
                            void*);
+typedef int (*GatedPays)(const qmm_problem*);
 typedef int (*PackLayer)(const void*, uint32_t*, const void*, const void*, int, int, void*, void*, int, int64_t, int64_t, int64_t, int, uint64_t*, uint32_t*, void*);
 typedef int64_t (*MoeWorkspace)(const qmm_moe_block*);
 typedef int (*MoeExperts)(const qmm_moe_block*, void*);
@@ -38,6 +39,7 @@ typedef int (*MoeExperts)(const qmm_moe_block*, void*);
 QuantizedMatmul g_quantized_matmul = nullptr;
 SiluMul g_silu_mul = nullptr;
 GatedMatmul g_gated_matmul = nullptr;
+GatedPays g_gated_pays = nullptr;
 PackLayer g_pack_layer = nullptr;
 MoeWorkspace g_moe_workspace = nullptr;
 MoeExperts g_moe_experts = nullptr;
@@ -365,7 +367,7 @@ PyObject* run_steps(PyObject*, PyObject* const* a, Py_ssize_t n) {
     returns[i] = static_cast<int>(v);
   }
   if (device < 0) Py_RETURN_NONE;
-  // A gate of two products of one x that nothing else reads, of as few rows as the library's one launch for the three takes.
+  // A gate of two products of one x that nothing else reads, where the library's one launch for the three is the faster.
   std::vector<int> readers(count, 0), maker(count, -1);
   for (Py_ssize_t i = 0; i < nsteps; ++i) {
     ++readers[steps[i].x];
@@ -374,11 +376,22 @@ PyObject* run_steps(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   for (int v : returns) ++readers[v];
   for (Step& s : steps) {
-    if (s.up < 0 || s.x == s.up || !g_gated_matmul || maker[s.x] < 0 || maker[s.up] < 0 || readers[s.x] != 1 || readers[s.up] != 1) continue;
+    if (s.up < 0 || s.x == s.up || !g_gated_matmul || !g_gated_pays || maker[s.x] < 0 || maker[s.up] < 0 || readers[s.x] != 1 || readers[s.up] != 1) continue;
     Step &g = steps[maker[s.x]], &u = steps[maker[s.up]];
-    const int64_t rows = shapes[s.x][0];
-    if (g.up >= 0 || u.up >= 0 || g.x != u.x || rows < 2 || rows > 16 || g.group_size != u.group_size || g.bits != u.bits || g.mode != u.mode || g.dtype != u.dtype || g.dtype != types[g.x])
+    if (g.up >= 0 || u.up >= 0 || g.x != u.x || g.scales->scalar_type() != u.scales->scalar_type() || g.group_size != u.group_size || g.bits != u.bits || g.mode != u.mode || g.dtype != u.dtype || g.dtype != types[g.x])
       continue;
+    qmm_problem p = {};
+    p.struct_size = sizeof(p);
+    p.mode = g.mode;
+    p.bits = g.bits;
+    p.group_size = g.group_size;
+    p.x_dtype = p.y_dtype = elem_of(g.dtype);
+    p.table_dtype = elem_of(g.scales->scalar_type());
+    p.batch = 1;
+    p.M = shapes[g.x][0];
+    p.K = shapes[g.x][1];
+    p.N = shapes[s.x][1];
+    if (p.M < 2 || p.M > 16 || p.x_dtype < 0 || p.table_dtype < 0 || g_gated_pays(&p) != 1) continue;
     s.gate_from = maker[s.x];
     s.up_from = maker[s.up];
     g.left = u.left = true;
@@ -455,9 +468,9 @@ PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   }
 }
 
-// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts_checked[, qmm_moe_silu_mul[, qmm_pack_dense_layer[, qmm_gated_matmul]]])
+// bind(addresses of qmm_quantized_matmul, qmm_moe_workspace_bytes, qmm_moe_experts_checked[, qmm_moe_silu_mul[, qmm_pack_dense_layer[, qmm_gated_matmul, qmm_gated_matmul_pays]]])
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n < 3 || n > 6) {
+  if (n < 3 || n > 7) {
     PyErr_SetString(PyExc_TypeError, "bind takes the entry points' addresses");
     return nullptr;
   }
@@ -467,6 +480,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n > 3) g_silu_mul = reinterpret_cast<SiluMul>(PyLong_AsVoidPtr(a[3]));
   if (n > 4) g_pack_layer = reinterpret_cast<PackLayer>(PyLong_AsVoidPtr(a[4]));
   if (n > 5) g_gated_matmul = reinterpret_cast<GatedMatmul>(PyLong_AsVoidPtr(a[5]));
+  if (n > 6) g_gated_pays = reinterpret_cast<GatedPays>(PyLong_AsVoidPtr(a[6]));
   if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }

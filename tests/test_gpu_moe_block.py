@@ -141,3 +141,28 @@ def test_blocks_of_several_threads():
     for t in threads:
         t.join()
     assert outcome == {0: (0, 25), 1: (0, 25), 2: (25, 0), 3: (0, 25)} and _lib.poll_status() == 0
+
+
+@pytest.mark.parametrize("kind,d,f,launches", [("int8", 896, 2944, 6), ("int8", 2304, 320, 4), ("int4", 896, 2944, 4)])
+def test_both_products_in_one_launch_where_that_is_faster(kind, d, f, launches):
+    """8-bit codes of many tiles have both products of the block by themselves and a gate behind them, the others one launch: the sort, that, the down projection and the weighted sum."""
+    rng = np.random.default_rng(d + f)
+    experts, tokens, k, bits = 8, 6, 2, int(kind[3:])
+    host = [affine_case(rng, n, kk, 64, bits, "bf16", lead=(experts,))[1:] for n, kk in ((f, d), (f, d), (d, f))]
+    packs = [tuple(to_torch(a, DEV) for a in arrays) for arrays in host]
+    xs_host = activations(rng, (tokens, d), "bf16", 0.25)
+    xs = to_torch(xs_host, DEV)
+    idx = torch.from_numpy(np.stack([rng.permutation(experts)[:k] for _ in range(tokens)])).to(DEV)
+    wts = torch.from_numpy(rng.random((tokens, k)).astype(np.float32)).to(DEV)
+    kw = dict(group_size=64, bits=bits)
+    got = moe.moe_experts(xs, idx, wts, *packs, **kw)
+    before = _lib.lib().qmm_launch_count()
+    assert torch.equal(moe.moe_experts(xs, idx, wts, *packs, **kw), got)
+    assert _lib.lib().qmm_launch_count() - before == launches
+    w1, w3, w2 = (O.dequantize(w, s, b, 64, bits, "affine").astype(np.float32) for w, s, b in host)
+    exact = np.zeros((tokens, d))
+    for t, x in enumerate(xs_host.astype(np.float64)):
+        for e, weight in zip(idx[t].tolist(), wts[t].tolist()):
+            gate = w1[e] @ x
+            exact[t] += weight * (w2[e] @ (gate / (1.0 + np.exp(-gate)) * (w3[e] @ x)))
+    assert O.rel_err(to_numpy(got).astype(np.float32), exact) <= 1e-2

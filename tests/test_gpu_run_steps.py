@@ -174,3 +174,16 @@ def test_a_product_that_is_read_twice_keeps_its_launch(m):
         it.execute(args)
         counts.append(_lib.lib().qmm_launch_count() - before)
     assert counts == [2, 4]
+
+
+@pytest.mark.parametrize("m,d,f,dtype,launches", [(12, 8192, 64, torch.bfloat16, 6), (12, 8160, 64, torch.float16, 2), (1, 128, 256, torch.bfloat16, 4), (17, 128, 256, torch.bfloat16, 4)])
+def test_gates_that_keep_their_launches(m, d, f, dtype, launches):
+    """One row, 17, and 12 of the longest K are other kernels' than the one that takes both products (the tensor cores' from K = 8192 on, in two launches each): two products, a gate and the product behind it."""
+    text, args = program(m, d, f, dtype), arguments(m, d, f, dtype)
+    taken, got, want = both(text, args)
+    assert taken and all(torch.equal(a, b) for a, b in zip(got, want))
+    it = recognizer.Interpreter(text)
+    it.execute(args)
+    before = _lib.lib().qmm_launch_count()
+    it.execute(args)
+    assert _lib.lib().qmm_launch_count() - before == launches

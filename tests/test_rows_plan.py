@@ -42,3 +42,16 @@ def test_clusters_are_of_three_warps_and_more(kind, x):
             for m in (2, 8) if x == BF16 else (1, 4, 8):
                 blocks, cluster, warps, ring, ctas = plan(m, k, n, x_dtype=x, **kind)
                 assert warps and (cluster == 1 or warps >= 3) and ctas % cluster == 0
+
+
+@pytest.mark.parametrize("m,k,n,kw,pays", [
+    (4, 2048, 5632, dict(), True), (16, 4096, 14336, dict(group_size=128, x_dtype=F16), True),             # us on a B200, one launch / three: 9 / 13.5
+    (2, 1280, 11080, dict(bits=8, group_size=128, x_dtype=F16), True),                                     # 11.8 / 14.3
+    (4, 3968, 14720, dict(bits=8, group_size=128), False), (16, 3968, 18968, dict(bits=8, group_size=128), False),      # 37.4 / 32.7, 83.0 / 61.7
+    (1, 4096, 14336, dict(), False), (17, 4096, 14336, dict(), False), (12, 8192, 1024, dict(), False),    # other kernels'
+    (4, 2048, 5632, dict(x_dtype=F32), False), (4, 2048, 5632, dict(y_dtype=F32), False), (4, 0, 64, dict(), False), (4, 64, 0, dict(), False),
+    (4, 2048, 5632, dict(group_size=48), False), (4, 2048, 5632, dict(batch=2), False), (4, 2048, 5632, dict(batch=4, ragged=True), False),
+])
+def test_two_products_and_their_gate_in_one_launch_where_that_is_faster(m, k, n, kw, pays):
+    assert _lib.lib().qmm_gated_matmul_pays(_lib.ctypes.byref(qmm._problem(m, k, n, **kw))) == pays
+    assert _lib.lib().qmm_gated_matmul_pays(None) == 0
