@@ -26,6 +26,7 @@
 
 #include "../../include/qmm_decode.h"
 #include "qmm_internal.h"
+#include "rotary.cuh"
 
 namespace qmm {
 namespace {
@@ -174,8 +175,8 @@ decode_attention_kernel(const AttnParams p) {
     const __nv_bfloat16* src = h < REP ? row + (kvh * REP + h) * HD : row + (p.heads + kvh) * HD;
     const float a = __bfloat162float(src[j]), c = __bfloat162float(src[j + kHalf]);
     const float sn = sine[u], cs = cosine[u];
-    // (contracted as the rotary kernel of its own is: the two append the same bits)
-    const float rlo = bf16_round(__fmaf_rn(a, cs, -__fmul_rn(c, sn))), rhi = bf16_round(__fmaf_rn(c, cs, __fmul_rn(a, sn)));
+    const float2 turned = rotate_half(a, c, sn, cs);
+    const float rlo = bf16_round(turned.x), rhi = bf16_round(turned.y);
     if (h < REP) {
       q_s[h][j] = rlo * inv_sqrt;
       q_s[h][j + kHalf] = rhi * inv_sqrt;
@@ -545,7 +546,8 @@ decode_attention_mma_kernel(const AttnParams p) {
     float sn, cs;
     const float freq = exp2f(-2.0f * static_cast<float>(j) / static_cast<float>(HD) * log2f(p.theta));
     sincosf(static_cast<float>(p.pos) * freq, &sn, &cs);
-    const __nv_bfloat16 rlo = __float2bfloat16_rn(a * cs - c * sn), rhi = __float2bfloat16_rn(c * cs + a * sn);
+    const float2 turned = rotate_half(a, c, sn, cs);
+    const __nv_bfloat16 rlo = __float2bfloat16_rn(turned.x), rhi = __float2bfloat16_rn(turned.y);
     if (h < REP) {
       q_s[h * HD + j] = rlo;
       q_s[h * HD + j + kHalf] = rhi;

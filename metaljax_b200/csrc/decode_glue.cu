@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "qmm_internal.h"
+#include "rotary.cuh"
 #include "../../include/qmm_decode.h"
 
 namespace qmm {
@@ -110,7 +111,8 @@ __global__ void rope_kv_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloa
       // by positions of up to 10^5
       const float freq = exp2f(-2.0f * static_cast<float>(j) / static_cast<float>(head_dim) * log2f(theta));
       sincosf(static_cast<float>(pos) * freq, &s, &c);
-      const float rlo = lo * c - hi * s, rhi = hi * c + lo * s;
+      const float2 turned = rotate_half(lo, hi, s, c);
+      const float rlo = turned.x, rhi = turned.y;
       if (head < heads) {
         __nv_bfloat16* dst = q_out + (static_cast<int64_t>(b) * heads + head) * head_dim;
         dst[j] = __float2bfloat16_rn(rlo);
