@@ -321,3 +321,24 @@ def test_decode_argmax_kernel(rows, n, stride):
         assert torch.equal(val, want_val)
         first = (ref == want_val[:, None]).float().argmax(dim=-1)
         assert torch.equal(idx, first + 1000)
+
+
+@pytest.mark.parametrize("n,k", [(4096, 4096), (4100, 4096), (4736, 8192), (4768, 4096), (4096, 3840), (4096, 14336)])
+def test_decode_linear_of_a_tile_per_sm(n, k):
+    """The fused form where one tile of 32 rows per SM has sixteen warps (4096 to 4736 rows of sixteen boxes and more) and to either side of that, against float64: the codes meet in integer sums, what is rounded is
+    the row (22 bits and more of it are kept) and the result, 2^-9 of each."""
+    import ctypes
+    from metaljax_b200 import _lib, llama
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    weight = llama._Linear(n, k, DEV, g, 64, "normal")
+    x = torch.randn((1, k), generator=g, device=DEV).to(torch.bfloat16)
+    y = torch.full((1, n), float("nan"), device=DEV, dtype=torch.bfloat16)
+    fz = _lib.DecodeFusion()
+    fz.wait_slot = fz.push_slot = -1
+    p = weight.problem(x, y)
+    _lib.check(_lib.lib().qmm_decode_linear(ctypes.byref(p), ctypes.byref(fz), None, _lib.stream_ptr(x)))
+    codes = weight.w.view(torch.uint8).reshape(n, -1)
+    w = torch.stack((codes & 15, codes >> 4), -1).reshape(n, k).double() * weight.s.double().repeat_interleave(64, -1) + weight.b.double().repeat_interleave(64, -1)
+    exact = x.double() @ w.T
+    assert ((y.double() - exact).norm() / exact.norm()).item() <= 2.0 ** -9
+    assert _lib.poll_status() == 0

@@ -280,3 +280,77 @@ def test_float32_results_of_uneven_activations(kind, gs, tdt, x, m, style):
     exact = xt.double() @ (codes.double() * wide(st) + wide(bt)).T
     largest = 2.0 ** (bits if m == 24 else bits + 4 if bits == 4 else bits + 3)               # (a code under the magic number is below 256 or 2048)
     assert bool(((y.double() - exact).abs() <= (16 + k / 512) * 2.0 ** -24 * largest * (xt.double().abs() @ wide(st).abs().T)).all())
+
+
+def _dequantized(w, s, b, kind, gs):
+    """The weight in float64, on the device."""
+    codes = w.view(torch.uint8)
+    codes = codes if kind == "int8" else torch.stack((codes & 15, codes >> 4), -1)
+    codes = codes.reshape(*w.shape[:-1], -1)
+    if kind == "mxfp4":
+        values = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, 0, -0.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64, device=w.device)
+        return values[codes.long()] * torch.exp2(s.double() - 127).repeat_interleave(32, -1)
+    return codes.double() * s.double().repeat_interleave(gs, -1) + b.double().repeat_interleave(gs, -1)
+
+
+def _gated(xt, one, two, y, kw, kind):
+    v = _lib.Views()
+    _lib.check(_lib.lib().qmm_gated_matmul(v(xt), *(v(a) for a in one), *(v(a) for a in two), v(y), kw["group_size"], kw["bits"], int(kind == "mxfp4"), torch.cuda.current_stream().cuda_stream))
+    return y
+
+
+@pytest.mark.parametrize("kind,gs,x,tdt", [("int4", 64, "bf16", "bf16"), ("int4", 32, "f16", "f32"), ("int8", 128, "bf16", "bf16"), ("mxfp4", 32, "bf16", None)])
+@pytest.mark.parametrize("m,k,n", [(5, 4096, 6000), (12, 5632, 6000), (8, 14336, 3000), (16, 4224, 4500), (9, 1088, 9001)])
+def test_gated_tiles_that_follow_one_another(kind, gs, x, tdt, m, k, n):
+    """Several tiles a worker -- slots of the ring used again, chunks of 8 rows one after the other in one CTA, laps of a cluster's leaders -- with table rows of whole 16 bytes, of words
+    and of neither. Against float64: four roundings to 16 bits, 2^-9 each for bf16, as when each step is a launch."""
+    if k % gs:
+        pytest.skip("not whole groups")
+    rng = np.random.default_rng(m + k + n)
+    (w, s, b), kw = _case(rng, kind, n, k, gs, tdt)
+    (w2, s2, b2), _ = _case(rng, kind, n, k, gs, tdt)
+    xt = to_torch(activations(rng, (m, k), x) * np.float32(0.05), DEV).to(DT[x])
+    one, two = ([to_torch(a, DEV) if a is not None else None for a in weight] for weight in ((w, s, b), (w2, s2, b2)))
+    y = _gated(xt, one, two, torch.full((m, n), float("nan"), dtype=DT[x], device=DEV), kw, kind)
+    gate, up = (xt.double() @ _dequantized(*weight, kind, gs).T for weight in (one, two))
+    exact = gate / (1.0 + torch.exp(-gate)) * up
+    assert ((y.double() - exact).abs().max() / exact.abs().max()).item() <= 1e-2
+    assert ((y.double() - exact).norm() / exact.norm()).item() <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("x", ["bf16", "f16"])
+def test_gates_that_are_not_finite(x):
+    """Infinities and NaN of either product, and gates so negative that their exponential overflows, come out as from the three launches."""
+    k, n, gs = 256, 64, 64
+    rng = np.random.default_rng(3)
+    (w, s, b), kw = _case(rng, "int4", n, k, gs, x)
+    (w2, s2, b2), _ = _case(rng, "int4", n, k, gs, x)
+    xt = to_torch(activations(rng, (8, k), x), DEV).to(DT[x])
+    xt[1, 7], xt[2, 100], xt[3, 200] = float("inf"), float("-inf"), float("nan")
+    xt[4] = 200.0 * xt[4].sign()
+    xt[5] = 0.0
+    one, two = ([to_torch(a, DEV) for a in weight] for weight in ((w, s, b), (w2, s2, b2)))
+    y = _gated(xt, one, two, torch.zeros((8, n), dtype=DT[x], device=DEV), kw, "int4")
+    apart = moe.silu_mul(qmm.quantized_matmul(xt, *one, **kw), qmm.quantized_matmul(xt, *two, **kw))
+    assert torch.equal(y.isnan(), apart.isnan()) and torch.equal(y.isinf(), apart.isinf()) and bool(y.isnan().any())
+    fine = apart.isfinite()
+    assert torch.equal(y.sign()[fine], apart.sign()[fine]) and (y - apart)[fine].abs().max() <= 1e-2 * apart[fine].abs().max()
+
+
+@pytest.mark.parametrize("kind,gs,x,tdt", [("int8", 64, "bf16", "bf16"), ("int8", 128, "f16", "f32")])
+@pytest.mark.parametrize("sizes,k,n", [([5], 5632, 6000), ([5], 14336, 3000), ([3, 0, 9, 1], 5632, 2500), ([8, 2], 14336, 1500)])
+def test_laps_of_leaders_with_8_bit_codes_and_with_experts(kind, gs, x, tdt, sizes, k, n):
+    """What the leaders of a cluster add up a lap late, of 8-bit codes, dense (one size) and grouped: a dozen tiles a cluster, whose last lap is partial. Against float64, the result rounded to 16 bits."""
+    rng = np.random.default_rng(k + n + len(sizes))
+    dense = len(sizes) == 1
+    (w, s, b), kw = _case(rng, kind, n, k, gs, tdt, lead=() if dense else (len(sizes),))
+    xt = to_torch(activations(rng, (sum(sizes), k), x), DEV).to(DT[x])
+    args = [to_torch(a, DEV) for a in (w, s, b)]
+    weights = _dequantized(*args, kind, gs)
+    if dense:
+        y, exact = qmm.quantized_matmul(xt, *args, **kw), xt.double() @ weights.T
+    else:
+        y = moe.ragged_dot(xt, *args, torch.tensor(sizes, device=DEV), **kw)
+        exact = torch.cat([rows @ e.T for rows, e in zip(xt.double().split(sizes), weights)])
+    assert ((y.double() - exact).abs().max() / exact.abs().max()).item() <= 1e-2
+    assert ((y.double() - exact).norm() / exact.norm()).item() <= 2.0 ** -8
