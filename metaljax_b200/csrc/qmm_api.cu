@@ -188,8 +188,8 @@ int route_of(const qmm_problem& p) {
   if (forced == QMM_ROUTE_F32_TC) return f32_tc_supports(p) ? forced : -QMM_ERR_UNSUPPORTED;
   if (forced == QMM_ROUTE_SIMT) return forced;
   // Nine to sixteen rows are two passes of the few-rows kernel; against a long K, where its CTAs also meet in clusters, the
-  // tensor-core kernel's one pass is the faster (16 rows, us: 4096 x 14336 22.1 against 17.4; at 4096 x 4096 9.3 / 9.8). It would be from K 4096 on
-  // (5632 x 2048 10.6 / 8.7), but it rounds each weight to 16 bits, the few-rows kernel none: 1.4e-3 of a float32 result's norm against 1e-6,
+  // tensor-core kernel's one pass is the faster (16 rows, us: 4096 x 14336 21.6 against 16.0, 9 rows of 4096 x 8192 13.8 / 12.0; at 4096 x 4096 7.6 / 9.4, 5632 x 2048 6.5 / 8.8). It would be from
+  // K 4096 on for wide weights (14336 x 4096 17.2 / 14.4), but it rounds each weight to 16 bits, the few-rows kernel none: 1.4e-3 of a float32 result's norm against 1e-6,
   // and 2.2e-3 against 1.7e-3 once the result is bf16. Below 8192, where these products were never rounded so, they are not.
   const bool long_k = p.M > 8 && p.K >= 8192 && p.batch == 1 && !p.lhs_idx && gemm_tc_supports(p);
   if (gemv_supports(p) && !long_k) return QMM_ROUTE_GEMV;

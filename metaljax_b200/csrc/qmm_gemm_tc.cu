@@ -192,7 +192,7 @@ __device__ __forceinline__ void take_magic_and_scale(float& x0, float& x1, float
 }
 
 // 8-bit affine, NW packed words -> NW*2 pairs, f16; s2, b2 are scale and bias as pairs. Two bytes of the word under a magic exponent are the f16 1024 + q; an exact subtraction and one
-// FMA, which rounds once. Six instructions a word; in float32 (below) ten, four of them byte permutes at half rate, and two roundings: 45 rows of 4096 x 14336 19.4 -> 17.8 us, 2048 rows of
+// FMA, which rounds once. Six instructions a word; in float32 (below) ten, four of them byte permutes at half rate, and two roundings: 45 rows of 4096 x 14336 20.6 -> 19.2 us, 2048 rows of
 // 14336 x 4096 192.8 -> 186.2. bf16 has no such exponent: its bytes are q 2^-133 as they stand, which takes 64 times the scale, and a way of its own for scales from 2^121 on: with
 // both in a kernel 2048 rows took 181.8 instead of 185.0 us, but 24 rows of 4096 x 4096 12.6 instead of 11.4, and it stays in float32.
 template <int NW>

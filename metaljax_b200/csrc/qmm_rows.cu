@@ -46,10 +46,10 @@ size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
 // float32 against MXFP4 28480 x 2048 49.9 us as 222 clusters of two, 31.4 as tiles of whole K; 2 rows 24512 x 4096 in groups of 32 26.0 / 17.2; 22464 x 7680 mxfp4 53.4 / 35.4.
 // Of 56 shapes where such a plan had the least load none was the faster for it.
 //
-// The constants were fitted to measured times; what they pick against the best of all plans, us (today's kernel): 8 rows 28672 x 4096 18.0 / 18.0 (the
-// next best 20.5), 128256 x 4096 58.0 / 58.0 (72.5), 4096 x 14336 13.9 / 13.9 (17.3), 4096 x 4096 6.0 / 6.0, 1024 x 1024 3.3 / 3.3,
-// 16 rows 4096 x 4096 7.7 / 7.7 (8.5), 4 rows 5632 x 2048 4.8 / 4.8 (5.3), 2048 x 5632 7.1 / 6.8, 8-bit 8 rows 14336 x 4096 13.8 / 13.3,
-// mxfp4 8 rows 5760 x 2880 8.8 / 8.8, float32 4 rows 4096 x 4096 9.1 / 9.1.
+// The constants were fitted to measured times of an earlier form of the kernel; what they pick against the best of all plans, us back to back in a graph: 8 rows 28672 x 4096 17.2 / 17.2 (the
+// next best 21.2), 128256 x 4096 58.2 / 58.2 (68.8), 4096 x 14336 14.1 / 14.1 (17.2), 4096 x 4096 5.9 / 5.8, 1024 x 1024 3.3 / 3.3,
+// 16 rows 4096 x 4096 7.7 / 7.7 (8.5), 128256 x 4096 109 / 109 (138), 4 rows 5632 x 2048 4.7 / 4.7 (4.9), 2048 x 5632 7.0 / 7.0, 8-bit 8 rows 14336 x 4096 in groups of 64 13.5 / 13.5, of 128 13.5 / 13.1,
+// 4096 x 14336 17.8 / 15.8, mxfp4 8 rows 5760 x 2880 8.4 / 8.4, float32 4 rows 4096 x 4096 9.2 / 9.2.
 RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh, int segs, bool pair = false) {
   const int sms = device_sm_count();
   RowsPlan best = {};
@@ -96,8 +96,8 @@ RowsPlan plan_rows(int64_t chunks, int64_t rows, int slices, const RowsShape& sh
 }
 
 // Rows of a chunk are what the registers take. Nine to sixteen rows are two chunks: the CTAs that work on either half pass over
-// the weight side by side, so that the second reads it from L2 (16 rows of 4096 x 4096: 9.2 us; as one chunk of 16, half of whose activations
-// live in shared memory, 14.2).
+// the weight side by side, so that the second reads it from L2 (16 rows of 4096 x 4096: 7.7 us; as one chunk of 16, half of whose activations
+// live in shared memory, 14.2 when this was 9.2).
 RowsShape shape_of(const qmm_problem& p, bool exact) {
   const bool mx = p.mode == QMM_MODE_MXFP4;
   const int bits = (!mx && p.bits == 8) ? 8 : 4, group = mx ? 32 : p.group_size;
@@ -125,13 +125,14 @@ bool rows_supports(const qmm_problem& p) {
 // A grouped product of at most 8 rows per expert on average streams its experts' weights here: an even share is one pass of a weight, and what
 // routing makes uneven still costs less than the tensor-core kernel's 64-row tiles. Above it those win, even shares or not. Experts' shares are
 // only known on the device, and a share of n rows passes its weight ceil(n / 8) times: the worst, all rows on one expert, is dearer here from 3 rows an
-// expert on. us here / tensor cores (weights from HBM; since then this side has become some 10 % faster), even, random and all on one:
+// expert on. us here / tensor cores (back to back in a graph, weights from HBM), even, random and all on one:
 //   rows an expert            4                                    8                                     12
-//   4-bit  8 x 14336 x 4096   75/120   76/120   44/29              77/121   102/121  72/30               129/121  129/121   99/44
-//   4-bit  8 x 4096 x 14336   92/121   84/121   52/62              93/121   127/121  88/64               159/122  158/121  122/64
-//   4-bit 32 x 2048 x 2048    34/46    33/47    21/21              35/46     41/47   30/21                49/47    50/47    38/21
-//   mxfp4 32 x 2880 x 2880    75/95    76/94    42/28              75/95     98/94   73/30               133/95   129/94   101/30
-//   8-bit  8 x 4096 x 4096    42/55    43/55    25/32              43/55     47/55   35/32                56/56    56/55    43/32
+//   4-bit  8 x 14336 x 4096   56/88    56/88    30/17              56/88     68/88   54/17               103/89   103/89    78/30
+//   4-bit  8 x 4096 x 14336   71/82    71/82    39/42              72/81     87/82   69/42               133/82   132/82   101/42
+//   4-bit 32 x 2048 x 2048    22/37    22/37    13/14              22/37     27/37   20/14                36/37    34/37    28/15
+//   mxfp4 32 x 2880 x 2880    69/64    74/64    35/18              69/64     90/64   67/19               127/64   121/64    95/19
+//   8-bit  8 x 4096 x 4096    29/37    29/37    17/19              30/37     32/37   26/19                45/37    46/37    34/19
+// (MXFP4 would be as fast or faster there from few rows on, since that kernel looks its values up; it rounds each weight to 16 bits, this one none.)
 bool rows_grouped_pays(const qmm_problem& p) { return rows_supports(p) && p.M <= 8 * p.batch; }
 
 // The decode family as callers may force it: dense or gathered products of up to 16 rows of 16-bit activations.

@@ -48,15 +48,17 @@
 // (8-bit float MMAs would take the codes with a third of the instructions, but `mma.sync` on e4m3 is emulated here with
 // conversions to f16: 88 against 67 us for 8 rows of 128256 x 4096.)
 //
-// Measured (device time, weights from HBM): int4 group 64 8 rows 28672 x 4096 18.1 us (3.7 TB/s), 128256 x 4096 58.0 (5.1 TB/s), 4096 x 14336 13.9, 16 rows 128256 x 4096 114,
-// 4096 x 4096 7.7; 8-bit 14336 x 4096 13.9. Tried: fragments in tensor memory (tcgen05.st / ld), rolled loops and two CTAs of 8 warps on an SM: 20.1 us at 28672 x 4096 when the above
+// Measured (device time, weights from HBM): int4 group 64 8 rows 28672 x 4096 17.2 us (3.8 TB/s; 18.6 a call by itself), 128256 x 4096 58.2 (5.1 TB/s), 4096 x 14336 14.1, 16 rows 128256 x 4096 109,
+// 4096 x 4096 7.7; 8-bit 14336 x 4096 13.5 in groups of 64 or 128, bf16 activations and tables. Tried: fragments in tensor memory (tcgen05.st / ld), rolled loops and two CTAs of 8 warps on an SM: 20.1 us at 28672 x 4096 when the above
 // was not there yet, 19.1 with it (16 rows a tile cost more instructions a code; the allocation delays the next launch's release); a last tile of 16 rows where a CTA's
 // share is not whole tiles: 4096 x 14336 14.8 instead of 13.9 (its code is fetched for it alone).
 // Where this kernel came from (before: a kernel with the same fragments under the same kind of magic
 // number that read its activations from shared memory for every tile and staged each tile's tables there behind barriers of the CTA; float32: the SIMT kernel), int4 group 64: 8 rows 28672 x 4096 27.1 -> 20.2 us (3.3 TB/s), 128256 x 4096
 // 99.5 -> 65.6 (4.5 TB/s), 4096 x 14336 26.8 -> 16.8, 16 rows 128256 x 4096 170 -> 128, 16 rows 4096 x 4096 12.2 -> 9.2; 8-bit 14336 x 4096 22.6
-// -> 15.5 (3.9 TB/s); float32 33 rows 4096 x 4096 323 -> 34.5. At the small end (2 rows 4096 x 4096 6.3 -> 7.1 us) it is the chain launch, activations,
+// -> 15.5 (3.9 TB/s); float32 33 rows 4096 x 4096 323 -> 34.5. At the small end (2 rows 4096 x 4096: 5.4 us) it is the chain launch, activations,
 // one tile, sum that counts, not a stream.
+// Rows of a table that are no multiple of 16 bytes are copied by words, and every such copy is a line a lane: a word more a row costs 4 to 20 % of a product (K of
+// 5376, 7936). MXFP4 against such K is 2 to 6 % slower than before the codes' chunks of 64 (8 rows of 37802 x 7936 56.0 -> 58.3 us), other kinds 1 to 5 % faster.
 //
 // Every wait on an mbarrier is bounded. The kernel is launched with programmatic stream
 // serialization: it lets the next kernel of the stream start early and touches only weights and
@@ -79,7 +81,7 @@ using namespace ptx;
 
 constexpr int kMaxWarps = 8;
 constexpr int kSliceK = 512;            // codes of K per warp
-constexpr int kBlockRows = 16;          // weight rows of an MMA; a tile is one or two blocks (see tile_blocks)
+constexpr int kBlockRows = 16;          // weight rows of an MMA; a tile is one or two blocks (see plan_rows)
 constexpr int kBoxBytes = 128;          // bytes of a weight row in a TMA box
 constexpr int kMaxRing = 6;
 constexpr int kMaxCluster = 8;
@@ -269,15 +271,15 @@ __device__ __forceinline__ void st_async4(uint32_t addr, uint32_t bar, const flo
 
 // Shared memory, from the (1024-byte aligned) start: barriers and small state, then per warp its ring, then
 // what the CTA shares. Fixed places first: an address that is a constant costs no register.
-constexpr int kFullAt = 0;                                             // [16 warps][kMaxRing] a box has landed
+constexpr int kFullAt = 0;                                             // [kMaxWarps][kMaxRing] a box has landed
 constexpr int kRedFullAt = kMaxWarps * kMaxRing * 8;                   // [4] every warp's share of a tile is there
 constexpr int kRedEmptyAt = kRedFullAt + 4 * 8;                        // [4] ... and has been added up
 constexpr int kXFullAt = kRedEmptyAt + 4 * 8;                          // [kExchangeSlots] the peers' sums of a tile this CTA leads
 constexpr int kXFreeAt = kXFullAt + kExchangeSlots * 8;                // [kMaxCluster][kExchangeSlots] leader r has read slot s
 constexpr int kAbortAt = kXFreeAt + kMaxCluster * kExchangeSlots * 8;  // the abort flag, the number of chunks of a grouped product
-constexpr int kStateAt = kAbortAt + 16;                                // [16 warps][2] where a warp's consumer is
+constexpr int kStateAt = kAbortAt + 16;                                // [kMaxWarps][2] where a warp's consumer is
 constexpr int kStateBytes = 32;
-constexpr int kAheadAt = kStateAt + kMaxWarps * 2 * kStateBytes;       // [16 warps] where its requests are: segment, chunk
+constexpr int kAheadAt = kStateAt + kMaxWarps * 2 * kStateBytes;       // [kMaxWarps] where its requests are: segment, chunk
 constexpr int kLedAt = kAheadAt + kMaxWarps * 8;                                   // [kExchangeSlots] where a tile that this CTA leads goes: element of y, rows, tile
 constexpr int kHeadBytes = (kLedAt + kExchangeSlots * 16 + 1023) / 1024 * 1024;
 
