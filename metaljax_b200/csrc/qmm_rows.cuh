@@ -361,6 +361,9 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   constexpr int kSums = sums_bytes(1, kTwice);                        // the columns' sums of a group
   constexpr int kTable = table_bytes(kTileRows, kGroups, TT, kQuads); // one table of a tile
   constexpr int kEight = table_at(8, kGroups, TT, kQuads);            // its next eight rows
+  // Rows of float32 entries in groups of 32 that do not start on 16 bytes: a word a lane. A word a copy of a row a lane is sixteen copies that touch 32 rows each (2 rows of 52352 x 5568 85.4 -> 69.0 us,
+  // 28672 x 3200 29.2 -> 21.9, float32 activations 52083 x 5760 216 -> 159). Shorter rows are left to that: MXFP4 and 8-bit codes were up to 4 % slower so.
+  constexpr bool kByWords = kRowBytes == 64;
   constexpr int kSlot = kStage + table_stage_bytes(R, kGroups, TT, kQuads);   // codes, scales, biases: a place of the ring
   constexpr float kUnit = QK == kMx4 ? 16384.0f : kNibbles && kCentred ? 64.0f : 1.0f;               // (the E2M1 fragments are the values times 2^-14)
 
@@ -517,38 +520,57 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
       }
     }
     {
-      // a lane's share of the tables: a weight row of one table, or (two blocks) of both. Entries past the end of a row are
-      // some other entry of it: what they multiply is zero.
-      const int64_t at = static_cast<int64_t>(min(ahead_row + (pair ? table_row & 15 : table_row), ahead_last)) * table_row_size + first_entry(slice) * kEntry;
-      const bool second = pair && lane >= 16;
-      const uint32_t dst = my_tables + ahead_slot * (kSlot - kStage);
-      auto copy = [&](const uint8_t* table, uint32_t to) {
-        const uint8_t* src = table + at;
-        constexpr int kWhole = kQuads ? 16 : 8;
-        if (p.table_unit >= kWhole && kRowBytes >= kWhole) {
+      // Entries past the end of a row are some other entry of it: what they multiply is zero.
+      const uint32_t stage_at = ahead_slot * (kSlot - kStage);
+      // a word a lane, the lanes of a row side by side
+      auto words = [&]() {
+        constexpr int kWords = kRowBytes / 4, kAtOnce = 32 / kWords, kStep = table_at(kAtOnce, kGroups, TT, kQuads);
+        const int row = lane / kWords, word = lane % kWords * 4, first = first_entry(slice) * kEntry;
+        const int from = first + (slice * kGroups * kEntry + word < table_row_size ? word : 0);
+        const uint32_t dst = tables_at + stage_at + table_at(row, kGroups, TT, kQuads) + word;
+        static_for<kTileRows / kAtOnce>([&](auto jc) {
+          constexpr int j = decltype(jc)::value;
+          const bool second = pair && j * kAtOnce >= kBlockRows;
+          const int64_t at = static_cast<int64_t>(min(ahead_row + row + (second ? j * kAtOnce - kBlockRows : j * kAtOnce), ahead_last)) * table_row_size + from;
+          cp_async4(dst + j * kStep, static_cast<const uint8_t*>(second ? p.scales2 : p.scales) + at);
+          cp_async4(dst + j * kStep + kTable, static_cast<const uint8_t*>(second ? p.biases2 : p.biases) + at);
+        });
+      };
+      // a lane's share: a weight row of one table, or (two blocks) of both
+      auto rows = [&]() {
+        const int64_t at = static_cast<int64_t>(min(ahead_row + (pair ? table_row & 15 : table_row), ahead_last)) * table_row_size + first_entry(slice) * kEntry;
+        const bool second = pair && lane >= 16;
+        const uint32_t dst = my_tables + stage_at;
+        auto copy = [&](const uint8_t* table, uint32_t to) {
+          const uint8_t* src = table + at;
+          constexpr int kWhole = kQuads ? 16 : 8;
+          if (kByWords || (p.table_unit >= kWhole && kRowBytes >= kWhole)) {
 #pragma unroll
-          for (int i = 0; i < kRowBytes; i += kWhole) {
-            if constexpr (kQuads) cp_async16(to + i, src + i);
-            else cp_async8(to + i, src + i);
+            for (int i = 0; i < kRowBytes; i += kWhole) {
+              if constexpr (kQuads) cp_async16(to + i, src + i);
+              else cp_async8(to + i, src + i);
+            }
+          } else if (kEntry == 4 || p.table_unit >= 4) {
+#pragma unroll
+            for (int i = 0; i < kRowBytes; i += 4) cp_async4(to + i, slice * kGroups * kEntry + i < table_row_size ? src + i : src);
+          } else {                         // from the word the first entry lies in; nothing past the table's end is read
+            const int skew = static_cast<int>(at & 3);
+#pragma unroll
+            for (int i = 0; i <= kRowBytes; i += 4) {
+              const int64_t room = p.table_bytes - (at - skew + i);
+              cp_async4(to + (i < kRowBytes ? i : spare), room > 0 ? src - skew + i : src - skew, room >= 4 ? 4 : room > 0 ? static_cast<int>(room) : 0);
+            }
           }
-        } else if (p.table_unit >= 4) {
-#pragma unroll
-          for (int i = 0; i < kRowBytes; i += 4) cp_async4(to + i, slice * kGroups * kEntry + i < table_row_size ? src + i : src);
-        } else {                         // from the word the first entry lies in; nothing past the table's end is read
-          const int skew = static_cast<int>(at & 3);
-#pragma unroll
-          for (int i = 0; i <= kRowBytes; i += 4) {
-            const int64_t room = p.table_bytes - (at - skew + i);
-            cp_async4(to + (i < kRowBytes ? i : spare), room > 0 ? src - skew + i : src - skew, room >= 4 ? 4 : room > 0 ? static_cast<int>(room) : 0);
-          }
+        };
+        if (kBothTables) {
+          if (kTileRows == 32 || lane < 16) copy(static_cast<const uint8_t*>(second ? p.scales2 : p.scales), dst);
+          if (TT != kTabE8) copy(static_cast<const uint8_t*>(second ? p.biases2 : p.biases), dst + kTable);
+        } else {
+          copy(my_table, dst);
         }
       };
-      if (kBothTables) {
-        if (kTileRows == 32 || lane < 16) copy(static_cast<const uint8_t*>(second ? p.scales2 : p.scales), dst);
-        if (TT != kTabE8) copy(static_cast<const uint8_t*>(second ? p.biases2 : p.biases), dst + kTable);
-      } else {
-        copy(my_table, dst);
-      }
+      if (kByWords && p.table_unit == 4) words();
+      else rows();
       cp_async_arrive(bar);
     }
     --ahead_left;

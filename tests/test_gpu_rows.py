@@ -354,3 +354,20 @@ def test_laps_of_leaders_with_8_bit_codes_and_with_experts(kind, gs, x, tdt, siz
         exact = torch.cat([rows @ e.T for rows, e in zip(xt.double().split(sizes), weights)])
     assert ((y.double() - exact).abs().max() / exact.abs().max()).item() <= 1e-2
     assert ((y.double() - exact).norm() / exact.norm()).item() <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("kind,x", [("int4", "bf16"), ("int4", "f32"), ("int8", "f16"), ("int8", "f32")])
+@pytest.mark.parametrize("m,k,n", [(2, 32, 1), (5, 288, 33), (8, 512, 300), (8, 3232, 700), (3, 4096, 129), (7, 14368, 48)])
+def test_rows_of_float32_entries_in_groups_of_32(kind, x, m, k, n):
+    """A word of one row's entries a lane where rows start on no 16 bytes (K no multiple of 128), 16 or 8 bytes where they do; one group, a slice that ends in the middle of its entries, clusters. The file's tolerances."""
+    rng = np.random.default_rng(m + k + n)
+    (w, s, b), kw = _case(rng, kind, n, k, 32, "f32")
+    xt = to_torch(activations(rng, (m, k), x), DEV).to(DT[x])
+    args = [to_torch(a, DEV) for a in (w, s, b)]
+    exact = xt.double() @ _dequantized(*args, kind, 32).T
+    if x == "f32":
+        y = qmm.quantized_matmul(xt, *args, **kw)
+    else:
+        with _lib.force_route("gemv_fmma"):
+            y = qmm.quantized_matmul(xt, *args, **kw)
+    assert ((y.double() - exact).abs().max() / exact.abs().max()).item() <= TOL[x]
