@@ -57,8 +57,8 @@
 // 99.5 -> 65.6 (4.5 TB/s), 4096 x 14336 26.8 -> 16.8, 16 rows 128256 x 4096 170 -> 128, 16 rows 4096 x 4096 12.2 -> 9.2; 8-bit 14336 x 4096 22.6
 // -> 15.5 (3.9 TB/s); float32 33 rows 4096 x 4096 323 -> 34.5. At the small end (2 rows 4096 x 4096: 5.4 us) it is the chain launch, activations,
 // one tile, sum that counts, not a stream.
-// Rows of a table that are no multiple of 16 bytes are copied by words, and every such copy is a line a lane: a word more a row costs 4 to 20 % of a product (K of
-// 5376, 7936). MXFP4 against such K is 2 to 6 % slower than before the codes' chunks of 64 (8 rows of 37802 x 7936 56.0 -> 58.3 us), other kinds 1 to 5 % faster.
+// Rows of a table that are no multiple of 16 bytes are copied by words, and every such copy but those of float32 entries in groups of 32 is a line a lane: a word more a row
+// costs 4 to 20 % of a product (K of 5376, 7936). MXFP4 against such K is 2 to 6 % slower than before the codes' chunks of 64 (8 rows of 37802 x 7936 56.0 -> 58.3 us), other kinds 1 to 5 % faster.
 //
 // Every wait on an mbarrier is bounded. The kernel is launched with programmatic stream
 // serialization: it lets the next kernel of the stream start early and touches only weights and
