@@ -25,7 +25,7 @@ namespace {
 
 size_t smem_of(const RowsPlan& pl, const RowsShape& sh, int segs) {
   const int qk = sh.tt == kTabE8 ? kMx4 : sh.stage == kBlockRows * kSliceK ? kAff8 : kAff4;
-  const bool quads = table_quads(sh.groups, sh.tt, sh.tokens), twice = sums_twice(qk, sh.groups, sh.tt, sh.exact || sh.tokens == 4);
+  const bool quads = table_quads(sh.groups, sh.tt), twice = sums_twice(qk, sh.groups, sh.tt, sh.exact || sh.tokens == 4);
   auto own = [&](bool q, bool t) { return pl.ring * (pl.blocks * sh.stage + table_stage_bytes(pl.blocks, sh.groups, sh.tt, q)) + sums_bytes(sh.groups, t); };
   // (at least what the plainest layout takes: a few hundred bytes decide between plans whose costs are close, and the costs were fitted with these)
   const size_t shares = static_cast<size_t>(pl.blocks) * 512, warp = std::max(own(quads, twice), own(false, false));

@@ -295,12 +295,13 @@ static_assert(sizeof(Place) <= kStateBytes, "");
 constexpr int kMaxBlocks = 2;
 
 // A tile's table entries travel with its codes: per weight row the slice's entries as they are in memory, so far apart that reads of a word of eight rows meet
-// all banks, with a word to spare for entries that do not start on a word. QUADS (affine tables of 16-bit activations): rows of 16 bytes and more lie on
-// multiples of 16, for one copy to take that many, every few rows another 16 bytes further on, and the spare words behind the rows. The others are copied by
-// eights at most: a fourth way to copy cost float32 and MXFP4 kernels registers. (A pitch of the row and 16 bytes for all of them took memory that rings and
-// plans were made of: steps of 2 sequences 251 -> 271 us, float32 against 8-bit codes 28480 x 2048 17.3 -> 25.7, 8 rows of 4096 x 28672 16.8 as now; with eights alone 17.4.)
+// all banks, with a word to spare for entries that do not start on a word. QUADS (affine tables): rows of 16 bytes and more lie on
+// multiples of 16, for one copy to take that many, every few rows another 16 bytes further on, and the spare words behind the rows. MXFP4's scales are copied by
+// eights at most (K of no multiple of 512 2 % slower else). (A pitch of the row and 16 bytes for all of them took memory that rings and
+// plans were made of: steps of 2 sequences 251 -> 271 us, float32 against 8-bit codes 28480 x 2048 17.3 -> 25.7. By eights alone 8 rows of 28672 x 4096 take
+// 17.4 us instead of 17.1, in groups of 32 with float32 tables 30.0 instead of 24.4, float32 activations there 17 % more.)
 constexpr int table_row_bytes(int groups, int tt) { return groups * entry_bytes(tt); }
-constexpr bool table_quads(int groups, int tt, int tokens) { return tokens == 8 && tt != kTabE8 && table_row_bytes(groups, tt) >= 16; }
+constexpr bool table_quads(int groups, int tt) { return tt != kTabE8 && table_row_bytes(groups, tt) >= 16; }
 constexpr int table_at(int row, int groups, int tt, bool quads) {
   const int bytes = table_row_bytes(groups, tt);
   return quads ? row * bytes + (bytes == 32 ? (row >> 2) * 16 : bytes == 64 ? (row >> 1) * 16 : 0) : row * (bytes == 8 ? 16 : bytes + 8);
@@ -357,7 +358,7 @@ qmm_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   constexpr int kBiasMmas = kGroups == 16 ? 3 : kGroups == 8 ? 2 : 1;
   constexpr int kEntry = entry_bytes(TT);
   constexpr int kRowBytes = table_row_bytes(kGroups, TT);             // a weight row's table entries in a slice
-  constexpr bool kQuads = table_quads(kGroups, TT, T), kTwice = sums_twice(QK, kGroups, TT, kCentred);
+  constexpr bool kQuads = table_quads(kGroups, TT), kTwice = sums_twice(QK, kGroups, TT, kCentred);
   constexpr int kSums = sums_bytes(1, kTwice);                        // the columns' sums of a group
   constexpr int kTable = table_bytes(kTileRows, kGroups, TT, kQuads); // one table of a tile
   constexpr int kEight = table_at(8, kGroups, TT, kQuads);            // its next eight rows
